@@ -149,6 +149,7 @@ bool resolve_reorder(const dfgpu_tensor& t, ScaleLayout& layout) {
 // ---- scale initialisation: every slot <- encode(1.0) = 0x7f --------------------
 
 __global__ void fill_bytes_kernel(uint8_t* data, int64_t count, uint8_t value) {
+    chain_begin();
     int64_t i = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 16;
     if (i + 16 <= count && (reinterpret_cast<uintptr_t>(data + i) & 15u) == 0) {
         uint32_t w = value * 0x01010101u;
@@ -159,6 +160,7 @@ __global__ void fill_bytes_kernel(uint8_t* data, int64_t count, uint8_t value) {
 }
 
 __global__ void fill_strided_kernel(uint8_t* data, View view, int64_t count, uint8_t value) {
+    chain_begin();
     int64_t flat = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (flat >= count) return;
     int64_t offset = 0;
@@ -173,6 +175,7 @@ __global__ void fill_strided_kernel(uint8_t* data, View view, int64_t count, uin
 
 __global__ void bsq_generic_kernel(const void* x, uint8_t* y, uint8_t* scale, View xv, View yv, View sv,
                                    ScaleLayout layout, int axis, int64_t block, int64_t block_total) {
+    chain_begin();
     int64_t flat = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (flat >= block_total) return;
     int64_t index[DFGPU_MAX_RANK];
@@ -718,6 +721,7 @@ struct BlockSizes {
 
 __global__ void bsd_generic_kernel(const uint8_t* x, const uint8_t* scale, void* y, View xv, View sv, View yv,
                                    ScaleLayout layout, int block_first_axis, BlockSizes sizes, int64_t total) {
+    chain_begin();
     int64_t flat = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (flat >= total) return;
     const int64_t* blocks = sizes.per_axis;  // 1 where unblocked
@@ -743,6 +747,9 @@ template <int OUT_DTYPE>
 __global__ void __launch_bounds__(256)
 bsd_packed_kernel(const uint8_t* __restrict__ x, const uint8_t* __restrict__ scale, void* __restrict__ y,
                   int64_t rows, int64_t cols, int64_t block_rows, int64_t block_cols) {
+    chain_begin();
+    x = after_chain(x);
+    scale = after_chain(scale);
     int64_t thread = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     int64_t element = thread * 16;
     if (element >= rows * cols) return;
@@ -945,9 +952,9 @@ extern "C" int dfgpu_block_scale_quantize(const dfgpu_bsq_params* p, void* const
         const uint8_t one = p->scale.dtype == DFGPU_E4M3 ? 0x38 : 0x7f;   // 1.0 as E4M3 (FP4 codes) or E8M0
         if (plan.layout.reordered || is_packed_row_major(p->scale)) {
             int64_t threads = (count + 15) / 16;
-            fill_bytes_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(scale, count, one);
+            launch_chained(fill_bytes_kernel, dim3(static_cast<unsigned>((threads + 255) / 256)), dim3(256), 0, stream, scale, count, one);
         } else {
-            fill_strided_kernel<<<static_cast<unsigned>((count + 255) / 256), 256, 0, stream>>>(
+            launch_chained(fill_strided_kernel, dim3(static_cast<unsigned>((count + 255) / 256)), dim3(256), 0, stream, 
                 scale, make_view(p->scale), count, one);
         }
     }
@@ -976,7 +983,7 @@ extern "C" int dfgpu_block_scale_quantize(const dfgpu_bsq_params* p, void* const
     } else {
         int64_t block_total = element_count(p->x) / p->block_size;
         unsigned grid = static_cast<unsigned>((block_total + 127) / 128);
-        bsq_generic_kernel<<<grid, 128, 0, stream>>>(x, y, scale, make_view(p->x), make_view(p->y),
+        launch_chained(bsq_generic_kernel, dim3(grid), dim3(128), 0, stream, x, y, scale, make_view(p->x), make_view(p->y),
                                                      make_view(p->scale), plan.layout, plan.axis, p->block_size,
                                                      block_total);
     }
@@ -1105,14 +1112,14 @@ extern "C" int dfgpu_block_scale_dequantize(const dfgpu_bsd_params* p, void* con
         int64_t threads = total / 16;
         unsigned grid = static_cast<unsigned>((threads + 255) / 256);
         int64_t rows = p->y.dim[0], cols = p->y.dim[1];
-        if (p->y.dtype == DFGPU_F32) bsd_packed_kernel<DFGPU_F32><<<grid, 256, 0, stream>>>(x, scale, y, rows, cols, plan.blocks[0], plan.blocks[1]);
-        else if (p->y.dtype == DFGPU_BF16) bsd_packed_kernel<DFGPU_BF16><<<grid, 256, 0, stream>>>(x, scale, y, rows, cols, plan.blocks[0], plan.blocks[1]);
-        else bsd_packed_kernel<DFGPU_F16><<<grid, 256, 0, stream>>>(x, scale, y, rows, cols, plan.blocks[0], plan.blocks[1]);
+        if (p->y.dtype == DFGPU_F32) launch_chained(bsd_packed_kernel<DFGPU_F32>, dim3(grid), dim3(256), 0, stream, x, scale, y, rows, cols, plan.blocks[0], plan.blocks[1]);
+        else if (p->y.dtype == DFGPU_BF16) launch_chained(bsd_packed_kernel<DFGPU_BF16>, dim3(grid), dim3(256), 0, stream, x, scale, y, rows, cols, plan.blocks[0], plan.blocks[1]);
+        else launch_chained(bsd_packed_kernel<DFGPU_F16>, dim3(grid), dim3(256), 0, stream, x, scale, y, rows, cols, plan.blocks[0], plan.blocks[1]);
     } else {
         unsigned grid = static_cast<unsigned>((total + 255) / 256);
         BlockSizes sizes;
         for (int i = 0; i < DFGPU_MAX_RANK; ++i) sizes.per_axis[i] = plan.blocks[i];
-        bsd_generic_kernel<<<grid, 256, 0, stream>>>(x, scale, y, make_view(p->x), make_view(p->scale),
+        launch_chained(bsd_generic_kernel, dim3(grid), dim3(256), 0, stream, x, scale, y, make_view(p->x), make_view(p->scale),
                                                      make_view(p->y), plan.layout, plan.first_axis, sizes, total);
     }
     return check_launch("BLOCK_SCALE_DEQUANTIZE");

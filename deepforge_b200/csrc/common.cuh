@@ -66,12 +66,29 @@ int sm_count();
 // draining: its CTAs take SMs as the earlier kernel's CTAs leave, run their private prologue (barrier
 // setup, tensor-memory allocation) and then block in chain_wait() until the earlier kernel has completed
 // and its writes are visible. Every kernel launched this way must call chain_wait() before its first
-// global-memory access; chain_release() at its top lets the kernel after it do the same. Both are no-ops
+// global-memory access; chain_release() lets the kernel after it do the same. Both are no-ops
 // when the kernel was launched the ordinary way. Captured into a CUDA graph the dependency becomes a
 // programmatic edge, so the gap between the kernels of one plan shrinks to the tail of the slowest CTA.
+// Every product kernel is launched this way: ordinary launches follow one another in a stream at multiples of
+// 2.05 us (a 2 us kernel every 4.1 us, a 5 us one every 8.2), chained ones at their own length plus 0.7 us.
+// A kernel that allocates tensor memory releases after the allocation: a later kernel's CTA on the same SM could
+// otherwise take the columns first and wait for this kernel, which waits for the columns. A convolution releases after
+// its wait: the convolution behind it may read its filter before it waits (dfgpu_conv_params.reserved bit 1), which
+// is safe only when nothing older than this kernel is still running.
 #ifdef __CUDACC__
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The pointer again, but known only from here on: a load through a const __restrict__ pointer counts as independent of
+// memory barriers, so only a data dependence keeps the compiler from moving it above the wait.
+template <typename T>
+__device__ __forceinline__ T* after_chain(T* pointer) {
+    asm volatile("" : "+l"(pointer) :: "memory");
+    return pointer;
+}
+__device__ __forceinline__ void chain_begin() {
+    chain_release();
+    chain_wait();
+}
 
 template <typename... Params, typename... Args>
 cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t dynamic_smem, cudaStream_t stream, Args&&... args) {

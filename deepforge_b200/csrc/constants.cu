@@ -12,6 +12,7 @@ struct ConstantTargets {
 };
 
 __global__ void constants_kernel(dfgpu_constants_params p, ConstantTargets targets) {
+    chain_begin();
     const int i = threadIdx.x;
     if (i >= p.count) return;
     void* target = targets.pointer[i];
@@ -56,6 +57,6 @@ extern "C" int dfgpu_constants(const dfgpu_constants_params* p, void* const* ten
             return fail(kInvalidArgument, "CONSTANTS: destination %d is null or not aligned to its %d bytes", i, p->bytes[i]);
         targets.pointer[i] = tensors[i];
     }
-    constants_kernel<<<1, 32, 0, as_stream(stream_handle)>>>(*p, targets);
+    launch_chained(constants_kernel, dim3(1), dim3(32), 0, as_stream(stream_handle), *p, targets);
     return check_launch("CONSTANTS");
 }

@@ -15,6 +15,8 @@ namespace dfgpu {
 namespace {
 
 __global__ void conv_direct_kernel(const void* x, const void* w, void* y, ConvArgs a, int64_t total) {
+    chain_wait();
+    chain_release();
     int64_t flat = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (flat >= total) return;
     int64_t q = flat % a.y.dim[3];
@@ -54,6 +56,10 @@ template <int BM, bool CHANNELS_LAST>
 __global__ void __launch_bounds__(256)
 conv_igemm_ffma_kernel(const void* __restrict__ x, const void* __restrict__ w, void* __restrict__ y, ConvArgs a,
                        int64_t m_total, int64_t k_total) {
+    chain_wait();
+    chain_release();
+    x = after_chain(x);
+    w = after_chain(w);
     constexpr int BN = 64, BK = 16, TM = BM / 16, TN = 4;
     constexpr int A_PER_THREAD = BM * BK / 256;
     constexpr int B_PER_THREAD = BN * BK / 256;
@@ -168,6 +174,12 @@ template <int BM>
 __global__ void __launch_bounds__(256)
 conv_nhwc_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, void* __restrict__ y, ConvArgs a, int m_total,
                      const int* __restrict__ run_if_any, int flag_count, const float* __restrict__ partial, int partial_count) {
+    chain_wait();
+    chain_release();
+    x = after_chain(x);
+    w = after_chain(w);
+    run_if_any = after_chain(run_if_any);
+    partial = after_chain(partial);
     constexpr int BN = 64, BK = 16, TM = BM / 16, TN = 4;
     __shared__ float as[2][BK][BM + 4];
     __shared__ float bs[2][BK][BN + 4];
@@ -526,16 +538,16 @@ extern "C" int dfgpu_conv_fprop(const dfgpu_conv_params* p, void* const* tensors
         unsigned grid_n = static_cast<unsigned>((p->y.dim[1] + 63) / 64);
         if ((m_total + 63) / 64 * grid_n < 2 * sm_count()) {
             dim3 grid(static_cast<unsigned>((m_total + 31) / 32), grid_n);
-            conv_nhwc_f32_kernel<32><<<grid, 256, 0, stream>>>(xf, wf, tensors[2], a, static_cast<int>(m_total), flags, split.flag_count, partial, k_split.splits);
+            launch_chained(conv_nhwc_f32_kernel<32>, dim3(grid), dim3(256), 0, stream, xf, wf, tensors[2], a, static_cast<int>(m_total), flags, split.flag_count, partial, k_split.splits);
         } else {
             dim3 grid(static_cast<unsigned>((m_total + 63) / 64), grid_n);
-            conv_nhwc_f32_kernel<64><<<grid, 256, 0, stream>>>(xf, wf, tensors[2], a, static_cast<int>(m_total), flags, split.flag_count, partial, k_split.splits);
+            launch_chained(conv_nhwc_f32_kernel<64>, dim3(grid), dim3(256), 0, stream, xf, wf, tensors[2], a, static_cast<int>(m_total), flags, split.flag_count, partial, k_split.splits);
         }
         return check_launch("CONV_FPROP");
     }
     if (kernel == DFGPU_CONV_DIRECT) {
         int64_t total = element_count(p->y);
-        conv_direct_kernel<<<static_cast<unsigned>((total + 127) / 128), 128, 0, stream>>>(tensors[0], tensors[1], tensors[2], a, total);
+        launch_chained(conv_direct_kernel, dim3(static_cast<unsigned>((total + 127) / 128)), dim3(128), 0, stream, tensors[0], tensors[1], tensors[2], a, total);
     } else {
         int64_t k_total = p->x.dim[1] * p->w.dim[2] * p->w.dim[3];
         bool channels_last = p->x.stride[1] == 1;
@@ -547,19 +559,19 @@ extern "C" int dfgpu_conv_fprop(const dfgpu_conv_params* p, void* const* tensors
             const float* wf = static_cast<const float*>(tensors[1]);
             if (small) {
                 dim3 grid(static_cast<unsigned>((m_total + 31) / 32), grid_n);
-                conv_nhwc_f32_kernel<32><<<grid, 256, 0, stream>>>(xf, wf, tensors[2], a, static_cast<int>(m_total), nullptr, 0, nullptr, 0);
+                launch_chained(conv_nhwc_f32_kernel<32>, dim3(grid), dim3(256), 0, stream, xf, wf, tensors[2], a, static_cast<int>(m_total), nullptr, 0, nullptr, 0);
             } else {
                 dim3 grid(static_cast<unsigned>((m_total + 63) / 64), grid_n);
-                conv_nhwc_f32_kernel<64><<<grid, 256, 0, stream>>>(xf, wf, tensors[2], a, static_cast<int>(m_total), nullptr, 0, nullptr, 0);
+                launch_chained(conv_nhwc_f32_kernel<64>, dim3(grid), dim3(256), 0, stream, xf, wf, tensors[2], a, static_cast<int>(m_total), nullptr, 0, nullptr, 0);
             }
         } else if (small) {
             dim3 grid(static_cast<unsigned>((m_total + 31) / 32), grid_n);
-            if (channels_last) conv_igemm_ffma_kernel<32, true><<<grid, 256, 0, stream>>>(tensors[0], tensors[1], tensors[2], a, m_total, k_total);
-            else conv_igemm_ffma_kernel<32, false><<<grid, 256, 0, stream>>>(tensors[0], tensors[1], tensors[2], a, m_total, k_total);
+            if (channels_last) launch_chained(conv_igemm_ffma_kernel<32, true>, dim3(grid), dim3(256), 0, stream, tensors[0], tensors[1], tensors[2], a, m_total, k_total);
+            else launch_chained(conv_igemm_ffma_kernel<32, false>, dim3(grid), dim3(256), 0, stream, tensors[0], tensors[1], tensors[2], a, m_total, k_total);
         } else {
             dim3 grid(static_cast<unsigned>((m_total + 63) / 64), grid_n);
-            if (channels_last) conv_igemm_ffma_kernel<64, true><<<grid, 256, 0, stream>>>(tensors[0], tensors[1], tensors[2], a, m_total, k_total);
-            else conv_igemm_ffma_kernel<64, false><<<grid, 256, 0, stream>>>(tensors[0], tensors[1], tensors[2], a, m_total, k_total);
+            if (channels_last) launch_chained(conv_igemm_ffma_kernel<64, true>, dim3(grid), dim3(256), 0, stream, tensors[0], tensors[1], tensors[2], a, m_total, k_total);
+            else launch_chained(conv_igemm_ffma_kernel<64, false>, dim3(grid), dim3(256), 0, stream, tensors[0], tensors[1], tensors[2], a, m_total, k_total);
         }
     }
     return check_launch("CONV_FPROP");

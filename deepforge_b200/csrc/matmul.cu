@@ -40,6 +40,10 @@ __device__ __forceinline__ void batch_offsets(const MatmulArgs& g, int64_t batch
 __global__ void __launch_bounds__(256)
 matmul_ffma_kernel(const void* __restrict__ a, const void* __restrict__ b, void* __restrict__ c, MatmulArgs g, const int* __restrict__ run_if_any,
                    int flag_count) {
+    chain_begin();
+    a = after_chain(a);
+    b = after_chain(b);
+    run_if_any = after_chain(run_if_any);
     constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
     __shared__ float as[BK][BM + 4];
     __shared__ float bs[BK][BN + 4];
@@ -337,7 +341,7 @@ extern "C" int dfgpu_matmul(const dfgpu_matmul_params* p, void* const* tensors, 
         status = launch_matmul_umma(split.bf16, bf16_tensors, DFGPU_MATMUL_UMMA_BF16, stream);
         if (status) return status;
         dim3 grid(static_cast<unsigned>((g.m + 63) / 64), static_cast<unsigned>((g.n + 63) / 64), 1);
-        matmul_ffma_kernel<<<grid, 256, 0, stream>>>(tensors[0], tensors[1], tensors[2], g, flags, split.flag_count);
+        launch_chained(matmul_ffma_kernel, dim3(grid), dim3(256), 0, stream, tensors[0], tensors[1], tensors[2], g, flags, split.flag_count);
         return check_launch("MATMUL");
     }
     if (kernel != DFGPU_MATMUL_FFMA) return launch_matmul_umma(*p, tensors, kernel, stream);
@@ -345,6 +349,6 @@ extern "C" int dfgpu_matmul(const dfgpu_matmul_params* p, void* const* tensors, 
     for (int i = 0; i < g.rank - 2; ++i) batches *= p->c.dim[i];
     if (batches > 65535) return fail(kUnsupported, "MATMUL: more than 65535 batch matrices");
     dim3 grid(static_cast<unsigned>((g.m + 63) / 64), static_cast<unsigned>((g.n + 63) / 64), static_cast<unsigned>(batches));
-    matmul_ffma_kernel<<<grid, 256, 0, stream>>>(tensors[0], tensors[1], tensors[2], g, nullptr, 0);
+    launch_chained(matmul_ffma_kernel, dim3(grid), dim3(256), 0, stream, tensors[0], tensors[1], tensors[2], g, nullptr, 0);
     return check_launch("MATMUL");
 }

@@ -5,7 +5,7 @@
 // over |value|, and C takes value * Scale_C through store_from_f32. The kernel here is the general one (any rank,
 // batch broadcast over extent-1 axes, any strides; one thread per output element, so the k order is the
 // reference's); large aligned problems go to the tcgen05 kernel in umma_mxf8.cu, whose f32 additions run in the
-// tensor core's order. Amax_C is cleared by a memset in the stream and folded with an atomic maximum on the bits of
+// tensor core's order. Amax_C is cleared by a one-word kernel in front and folded with an atomic maximum on the bits of
 // the non-negative f32 (NaN, made canonical, is the largest pattern, so it sticks like maximumf's).
 #include "common.cuh"
 #include "umma.cuh"
@@ -25,6 +25,9 @@ struct Fp8Args {
 
 __global__ void __launch_bounds__(256)
 matmul_fp8_scalar_kernel(const void* __restrict__ a, const void* __restrict__ b, void* __restrict__ c, Fp8Args g) {
+    chain_begin();
+    a = after_chain(a);
+    b = after_chain(b);
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     const int64_t im = static_cast<int64_t>(blockIdx.y) * 16 + ty;
     const int64_t in = static_cast<int64_t>(blockIdx.x) * 16 + tx;
@@ -56,6 +59,13 @@ matmul_fp8_scalar_kernel(const void* __restrict__ a, const void* __restrict__ b,
     unsigned int bits = magnitude != magnitude ? 0x7fc00000u : __float_as_uint(magnitude);
     bits = __reduce_max_sync(0xffffffffu, bits);
     if ((threadIdx.x & 31) == 0 && bits != 0u) atomicMax(g.amax_bits, bits);
+}
+
+// Amax_C <- +0. A kernel and not a memset: a memset in the stream would keep the matrix kernel from being chained.
+__global__ void clear_amax_kernel(unsigned int* amax_bits) {
+    chain_wait();
+    chain_release();
+    if (threadIdx.x == 0) *amax_bits = 0u;
 }
 
 int build_args(const dfgpu_matmul_fp8_params& p, void* const* tensors, Fp8Args& g) {
@@ -111,7 +121,7 @@ extern "C" int dfgpu_query_matmul_fp8(const dfgpu_matmul_fp8_params* p, dfgpu_pl
     status = choose_kernel(*p, kernel);
     if (status) return status;
     info->kernel = kernel;
-    info->launches = 1;  // plus the 4-byte memset that clears Amax_C
+    info->launches = 1;  // plus the one-word kernel that clears Amax_C
     info->scratch_bytes = 0;
     return kOk;
 }
@@ -130,13 +140,14 @@ extern "C" int dfgpu_matmul_fp8(const dfgpu_matmul_fp8_params* p, void* const* t
     status = choose_kernel(*p, kernel);
     if (status) return status;
     cudaStream_t stream = as_stream(stream_handle);
-    cudaError_t error = cudaMemsetAsync(tensors[3], 0, sizeof(float), stream);
-    if (error != cudaSuccess) return fail(kExecutionFailed, "MATMUL_FP8: clearing Amax_C failed: %s", cudaGetErrorString(error));
+    launch_chained(clear_amax_kernel, dim3(1), dim3(32), 0, stream, g.amax_bits);
+    status = check_launch("MATMUL_FP8: clearing Amax_C");
+    if (status) return status;
     if (kernel == DFGPU_MATMUL_FP8_UMMA) return launch_matmul_fp8_umma(*p, tensors, stream);
     int64_t batches = 1;
     for (int i = 0; i < g.rank - 2; ++i) batches *= p->c.dim[i];
     if (batches > 65535 || (g.m + 15) / 16 > 65535) return fail(kUnsupported, "MATMUL_FP8: more than 65535 batch matrices or row blocks");
     dim3 grid(static_cast<unsigned>((g.n + 15) / 16), static_cast<unsigned>((g.m + 15) / 16), static_cast<unsigned>(batches));
-    matmul_fp8_scalar_kernel<<<grid, 256, 0, stream>>>(tensors[0], tensors[1], tensors[2], g);
+    launch_chained(matmul_fp8_scalar_kernel, dim3(grid), dim3(256), 0, stream, tensors[0], tensors[1], tensors[2], g);
     return check_launch("MATMUL_FP8");
 }

@@ -125,6 +125,7 @@ __device__ __forceinline__ float pointwise_value(int mode, float x, float y, flo
 // Any mode, any strides and storage types: one thread per output element.
 __global__ void pointwise_general_kernel(const void* a, const void* b, const void* c, void* out, View av, View bv, View cv, View ov,
                                          int mode, PointwiseScalars s, int64_t total) {
+    chain_begin();
     int64_t flat = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (flat >= total) return;
     int64_t index[DFGPU_MAX_RANK];
@@ -144,6 +145,7 @@ __global__ void pointwise_general_kernel(const void* a, const void* b, const voi
 
 __global__ void pointwise_kernel(const void* a, const void* b, void* out, View av, View bv, View ov, int mode,
                                  float lower, float upper, float slope, int64_t total) {
+    chain_begin();
     int64_t flat = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (flat >= total) return;
     int64_t index[DFGPU_MAX_RANK];
@@ -264,6 +266,9 @@ static_assert(DFGPU_PW_MODE_COUNT == 50, "DFGPU_PW_EVERY_MODE lists every mode")
 template <typename T, int INPUTS>
 __global__ void __launch_bounds__(kPackedThreads, (sizeof(T) == 2 && INPUTS == 2) ? 5 : 2048 / kPackedThreads)
 pointwise_general_packed_kernel(const void* a, const void* b, void* out, int mode, PointwiseScalars s, int64_t total) {
+    chain_begin();
+    a = after_chain(a);
+    b = after_chain(b);
     switch (mode) {
 #define DFGPU_PW_CASE(M) case M: if constexpr (input_count(M) == INPUTS) packed_body<T, M>(a, b, out, s, total); break;
         DFGPU_PW_EVERY_MODE(DFGPU_PW_CASE)
@@ -274,8 +279,8 @@ pointwise_general_packed_kernel(const void* a, const void* b, void* out, int mod
 
 template <typename T>
 void launch_packed(int inputs, const void* a, const void* b, void* out, int mode, const PointwiseScalars& s, int64_t total, cudaStream_t stream) {
-    if (inputs == 1) pointwise_general_packed_kernel<T, 1><<<packed_grid<T>(total), kPackedThreads, 0, stream>>>(a, b, out, mode, s, total);
-    else pointwise_general_packed_kernel<T, 2><<<packed_grid<T>(total), kPackedThreads, 0, stream>>>(a, b, out, mode, s, total);
+    if (inputs == 1) launch_chained(pointwise_general_packed_kernel<T, 1>, dim3(packed_grid<T>(total)), dim3(kPackedThreads), 0, stream, a, b, out, mode, s, total);
+    else launch_chained(pointwise_general_packed_kernel<T, 2>, dim3(packed_grid<T>(total)), dim3(kPackedThreads), 0, stream, a, b, out, mode, s, total);
 }
 
 bool same_packed(const dfgpu_tensor& a, const dfgpu_tensor& b) {
@@ -354,13 +359,13 @@ extern "C" int dfgpu_pointwise(const dfgpu_pointwise_params* p, void* const* ten
         else launch_packed<__nv_bfloat16>(inputs, tensors[0], tensors[1], tensors[2], p->mode, s, total, stream);
     } else if (!simple_mode(p->mode)) {
         unsigned grid = static_cast<unsigned>((total + 255) / 256);
-        pointwise_general_kernel<<<grid, 256, 0, stream>>>(tensors[0], tensors[1], inputs >= 3 ? tensors[3] : nullptr, tensors[2],
+        launch_chained(pointwise_general_kernel, dim3(grid), dim3(256), 0, stream, tensors[0], tensors[1], inputs >= 3 ? tensors[3] : nullptr, tensors[2],
                                                            make_view(p->in0), inputs >= 2 ? make_view(p->in1) : make_view(p->in0),
                                                            inputs >= 3 ? make_view(p->in2) : make_view(p->in0), make_view(p->out),
                                                            p->mode, s, total);
     } else {
         unsigned grid = static_cast<unsigned>((total + 255) / 256);
-        pointwise_kernel<<<grid, 256, 0, stream>>>(tensors[0], tensors[1], tensors[2], make_view(p->in0),
+        launch_chained(pointwise_kernel, dim3(grid), dim3(256), 0, stream, tensors[0], tensors[1], tensors[2], make_view(p->in0),
                                                    binary ? make_view(p->in1) : make_view(p->in0), make_view(p->out),
                                                    p->mode, p->relu_lower, p->relu_upper, p->relu_slope, total);
     }

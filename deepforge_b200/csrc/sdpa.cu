@@ -141,6 +141,7 @@ __device__ int g_sdpa_status = 0;
 
 __global__ void __launch_bounds__(256)
 validate_page_prefix_kernel(SdpaArgs a, int* prefix_ok) {
+    chain_begin();
     const int which = blockIdx.x;
     const void* offsets = which ? a.offsets_v_data : a.offsets_k_data;
     if (!offsets) {
@@ -174,6 +175,7 @@ constexpr int kPrefixScratchBytes = 256;  // the two validation results of compa
 
 __global__ void __launch_bounds__(128)
 sdpa_rowwise_kernel(SdpaArgs a, int64_t rows) {
+    chain_begin();
     __shared__ float q_shared[4][kRowwiseMaxD];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int64_t row = static_cast<int64_t>(blockIdx.x) * 4 + warp;
@@ -326,6 +328,7 @@ __device__ __forceinline__ void unpack8(const uint4& raw, float (&out)[8]) {
 template <int G>
 __global__ void __launch_bounds__(256)
 sdpa_paged_decode_kernel(SdpaArgs a, float* __restrict__ partial, int max_chunks) {
+    chain_begin();
     __shared__ float scores[G][kDecodeChunk];
     __shared__ float reduce[8][G][kDecodeD / 4 + 1];  // staged in 4 passes of 32 columns
     __shared__ int64_t page_base_k[kDecodeChunk / 16];
@@ -504,6 +507,8 @@ sdpa_paged_decode_kernel(SdpaArgs a, float* __restrict__ partial, int max_chunks
 // One CTA of 128 threads per (batch, query head): combine the chunk partials.
 __global__ void __launch_bounds__(128)
 sdpa_decode_merge_kernel(SdpaArgs a, const float* __restrict__ partial, int max_chunks, int chunk_keys) {
+    chain_begin();
+    partial = after_chain(partial);
     const int64_t row = blockIdx.x;  // b * Hq + h
     const int64_t hq = a.q.dim[1];
     const int64_t ib = row / hq, ih = row % hq;
@@ -786,7 +791,7 @@ extern "C" int dfgpu_sdpa_forward(const dfgpu_sdpa_params* p, void* const* tenso
         if (!scratch || !aligned16(scratch)) return fail(kInvalidArgument, "SDPA: compact page tables need the 16-byte aligned scratch dfgpu_query_sdpa_forward reports");
         int* prefix_ok = static_cast<int*>(scratch);
         scratch = static_cast<uint8_t*>(scratch) + kPrefixScratchBytes;
-        validate_page_prefix_kernel<<<2, 256, 0, stream>>>(a, prefix_ok);
+        launch_chained(validate_page_prefix_kernel, dim3(2), dim3(256), 0, stream, a, prefix_ok);
         status = check_launch("SDPA page table prefix validation");
         if (status) return status;
         a.prefix_ok = prefix_ok;
@@ -797,7 +802,7 @@ extern "C" int dfgpu_sdpa_forward(const dfgpu_sdpa_params* p, void* const* tenso
         status = launch_decode_umma(*p, tensors, scratch, a.prefix_ok, stream);
         if (status) return status;
         const int chunks = decode_umma_chunks(*p);
-        sdpa_decode_merge_kernel<<<static_cast<unsigned>(p->q.dim[0] * p->q.dim[1]), kDecodeD, 0, stream>>>(a, static_cast<const float*>(scratch), chunks, 1024);
+        launch_chained(sdpa_decode_merge_kernel, dim3(static_cast<unsigned>(p->q.dim[0] * p->q.dim[1])), dim3(kDecodeD), 0, stream, a, static_cast<const float*>(scratch), chunks, 1024);
         return check_launch("SDPA decode merge");
     }
     if (kernel == DFGPU_SDPA_PAGED_DECODE) {
@@ -809,18 +814,18 @@ extern "C" int dfgpu_sdpa_forward(const dfgpu_sdpa_params* p, void* const* tenso
         dim3 grid(static_cast<unsigned>(chunks), static_cast<unsigned>(p->k.dim[1]), static_cast<unsigned>(p->q.dim[0]));
         float* partial = static_cast<float*>(scratch);
         switch (group) {
-            case 1: sdpa_paged_decode_kernel<1><<<grid, 256, 0, stream>>>(a, partial, chunks); break;
-            case 2: sdpa_paged_decode_kernel<2><<<grid, 256, 0, stream>>>(a, partial, chunks); break;
-            case 4: sdpa_paged_decode_kernel<4><<<grid, 256, 0, stream>>>(a, partial, chunks); break;
-            default: sdpa_paged_decode_kernel<8><<<grid, 256, 0, stream>>>(a, partial, chunks); break;
+            case 1: launch_chained(sdpa_paged_decode_kernel<1>, dim3(grid), dim3(256), 0, stream, a, partial, chunks); break;
+            case 2: launch_chained(sdpa_paged_decode_kernel<2>, dim3(grid), dim3(256), 0, stream, a, partial, chunks); break;
+            case 4: launch_chained(sdpa_paged_decode_kernel<4>, dim3(grid), dim3(256), 0, stream, a, partial, chunks); break;
+            default: launch_chained(sdpa_paged_decode_kernel<8>, dim3(grid), dim3(256), 0, stream, a, partial, chunks); break;
         }
         status = check_launch("SDPA paged decode");
         if (status) return status;
-        sdpa_decode_merge_kernel<<<static_cast<unsigned>(p->q.dim[0] * p->q.dim[1]), kDecodeD, 0, stream>>>(a, partial, chunks, kDecodeChunk);
+        launch_chained(sdpa_decode_merge_kernel, dim3(static_cast<unsigned>(p->q.dim[0] * p->q.dim[1])), dim3(kDecodeD), 0, stream, a, partial, chunks, kDecodeChunk);
         return check_launch("SDPA decode merge");
     }
     int64_t rows = p->q.dim[0] * p->q.dim[1] * p->q.dim[2];
-    sdpa_rowwise_kernel<<<static_cast<unsigned>((rows + 3) / 4), 128, 0, stream>>>(a, rows);
+    launch_chained(sdpa_rowwise_kernel, dim3(static_cast<unsigned>((rows + 3) / 4)), dim3(128), 0, stream, a, rows);
     return check_launch("SDPA");
 }
 
@@ -912,13 +917,13 @@ extern "C" int dfgpu_sdpa_paged_decode_static(const dfgpu_sdpa_params* p, void* 
     dim3 grid(static_cast<unsigned>(chunks), static_cast<unsigned>(p->k.dim[1]), static_cast<unsigned>(p->q.dim[0]));
     float* partial = static_cast<float*>(scratch);
     switch (group) {
-        case 1: sdpa_paged_decode_kernel<1><<<grid, 256, 0, stream>>>(a, partial, chunks); break;
-        case 2: sdpa_paged_decode_kernel<2><<<grid, 256, 0, stream>>>(a, partial, chunks); break;
-        case 4: sdpa_paged_decode_kernel<4><<<grid, 256, 0, stream>>>(a, partial, chunks); break;
-        default: sdpa_paged_decode_kernel<8><<<grid, 256, 0, stream>>>(a, partial, chunks); break;
+        case 1: launch_chained(sdpa_paged_decode_kernel<1>, dim3(grid), dim3(256), 0, stream, a, partial, chunks); break;
+        case 2: launch_chained(sdpa_paged_decode_kernel<2>, dim3(grid), dim3(256), 0, stream, a, partial, chunks); break;
+        case 4: launch_chained(sdpa_paged_decode_kernel<4>, dim3(grid), dim3(256), 0, stream, a, partial, chunks); break;
+        default: launch_chained(sdpa_paged_decode_kernel<8>, dim3(grid), dim3(256), 0, stream, a, partial, chunks); break;
     }
     status = check_launch("SDPA static decode");
     if (status) return status;
-    sdpa_decode_merge_kernel<<<static_cast<unsigned>(p->q.dim[0] * p->q.dim[1]), kDecodeD, 0, stream>>>(a, partial, chunks, kDecodeChunk);
+    launch_chained(sdpa_decode_merge_kernel, dim3(static_cast<unsigned>(p->q.dim[0] * p->q.dim[1])), dim3(kDecodeD), 0, stream, a, partial, chunks, kDecodeChunk);
     return check_launch("SDPA static decode merge");
 }

@@ -34,6 +34,10 @@ __device__ __forceinline__ bool split_f32(float v, uint32_t (&piece)[3]) {
 
 __global__ void __launch_bounds__(256)
 split6_f32_kernel(SplitOperand first, SplitOperand second, int* __restrict__ flags) {
+    chain_wait();
+    chain_release();
+    first.source = after_chain(first.source);
+    second.source = after_chain(second.source);
     bool finite = true;
     float4 v[4];
     bool live[4], in_second[4];
@@ -85,7 +89,7 @@ int split_flag_count(const SplitOperand& first, const SplitOperand& second) {
 }
 
 int launch_split6(const SplitOperand& first, const SplitOperand& second, int* flags, cudaStream_t stream) {
-    split6_f32_kernel<<<split_flag_count(first, second), 256, 0, stream>>>(first, second, flags);
+    launch_chained(split6_f32_kernel, dim3(split_flag_count(first, second)), dim3(256), 0, stream, first, second, flags);
     return check_launch("f32 operand split");
 }
 

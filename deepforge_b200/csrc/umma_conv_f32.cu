@@ -210,6 +210,8 @@ umma_conv_f32_kernel(const __grid_constant__ ClusterConvArgs g, const __grid_con
         v[1] = make_float4(value[4], value[5], value[6], value[7]);
     };
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const void* x_data = g.x;
+    const void* w_data = g.w;
     auto fetch = [&](int u, float4 (&xv)[2][2], float4 (&wv)[2]) {
         const int unit = first_unit + u;
         const int tap = static_cast<int>(fast_divide(unit, g.by_chunks)), c0 = (unit - tap * g.chunks) * kChunk;
@@ -222,10 +224,10 @@ umma_conv_f32_kernel(const __grid_constant__ ClusterConvArgs g, const __grid_con
             if (live[i] && ih >= 0 && ih < H && iw >= 0 && iw < W && (!volume || (id >= 0 && id < g.depth_in)) && c0 + x_unit[i] * 8 < C) {
                 const int source = x_image[i] + ih * g.x_h + iw * g.x_w + c0 * g.x_c + (volume ? id * g.x_d : 0);
                 if (x_quads) {
-                    xv[i][0] = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(g.x) + source));
-                    xv[i][1] = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(g.x) + source) + 1);
+                    xv[i][0] = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(x_data) + source));
+                    xv[i][1] = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(x_data) + source) + 1);
                 } else {
-                    eight(g.x, g.x_type, source, g.x_c, C - (c0 + x_unit[i] * 8), xv[i]);
+                    eight(x_data, g.x_type, source, g.x_c, C - (c0 + x_unit[i] * 8), xv[i]);
                 }
             }
         }
@@ -237,14 +239,17 @@ umma_conv_f32_kernel(const __grid_constant__ ClusterConvArgs g, const __grid_con
             const int source = w_row + (a.reverse ? R - 1 - r : r) * g.w_r + (a.reverse ? S - 1 - s : s) * g.w_s + c0 * g.w_c +
                                (volume ? (a.reverse ? g.depth_taps - 1 - t : t) * g.w_t : 0);
             if (w_quads) {
-                wv[0] = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(g.w) + source));
-                wv[1] = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(g.w) + source) + 1);
+                wv[0] = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(w_data) + source));
+                wv[1] = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(w_data) + source) + 1);
             } else {
-                eight(g.w, g.w_type, source, g.w_c, C - (c0 + w_unit * 8), wv);
+                eight(w_data, g.w_type, source, g.w_c, C - (c0 + w_unit * 8), wv);
             }
         }
     };
     float4 xv[2][2], wv[2];
+    chain_wait();
+    x_data = after_chain(x_data);
+    w_data = after_chain(w_data);
     if (tid < kLoaders && my_units > 0) fetch(0, xv, wv);   // in flight while the barriers and tensor memory are set up
 
     if (tid == 0) {
@@ -267,6 +272,7 @@ umma_conv_f32_kernel(const __grid_constant__ ClusterConvArgs g, const __grid_con
         tc_fence_before();
         __syncthreads();
         tc_fence_after();
+        chain_release();
     };
 
     bool ok = true, finite = true;
@@ -434,7 +440,7 @@ umma_conv_f32_kernel(const __grid_constant__ ClusterConvArgs g, const __grid_con
                         const int tap = filter + (a.reverse ? R - 1 - r : r) * g.w_r + (a.reverse ? S - 1 - s : s) * g.w_s +
                                         (a.reverse ? g.depth_taps - 1 - t : t) * g.w_t;
                         for (int c = 0; c < C; ++c)
-                            sum = fmaf(inside ? load_value(g.x, g.x_type, pixel + c * g.x_c) : 0.0f, load_value(g.w, g.w_type, tap + c * g.w_c), sum);
+                            sum = fmaf(inside ? load_value(x_data, g.x_type, pixel + c * g.x_c) : 0.0f, load_value(w_data, g.w_type, tap + c * g.w_c), sum);
                     }
             store_from_f32(g.y, g.y_type, n * g.y_n + p * g.y_p + q * g.y_q + k * g.y_k + d * g.y_d, apply_epilogue(sum, a, n, k, p, q, d));
         }
@@ -565,12 +571,14 @@ static int launch_clusters(ClusterForm form, ClusterConvArgs g, const ConvArgs& 
     config.blockDim = dim3(kThreads);
     config.dynamicSmemBytes = kSmemBytes;
     config.stream = stream;
-    cudaLaunchAttribute attribute{};
-    attribute.id = cudaLaunchAttributeClusterDimension;
-    attribute.val.clusterDim.x = form.ranks;
-    attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
-    config.attrs = &attribute;
-    config.numAttrs = 1;
+    cudaLaunchAttribute attribute[2]{};
+    attribute[0].id = cudaLaunchAttributeClusterDimension;
+    attribute[0].val.clusterDim.x = form.ranks;
+    attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
+    attribute[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attribute;
+    config.numAttrs = 2;
     const bool fast = g.x_quads && g.w_quads && g.y_quads && a.groups == 1 && g.tiles_per_image == 0 && g.depth_out * g.depth_in * g.depth_taps == 1;
     cudaError_t error = fast ? cudaLaunchKernelEx(&config, umma_conv_f32_kernel<true>, g, a) : cudaLaunchKernelEx(&config, umma_conv_f32_kernel<false>, g, a);
     if (error != cudaSuccess) return fail(kExecutionFailed, "%s: cluster launch failed: %s", what, cudaGetErrorString(error));

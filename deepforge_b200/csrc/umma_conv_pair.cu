@@ -139,7 +139,6 @@ umma_conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
     const bool leader = elect_one();
     const int issuers = args.split_in ? 2 : 1;
-    chain_release();
     if (threadIdx.x == 0) {
         prefetch_tensormap(&map_x);
         prefetch_tensormap(&map_wa);
@@ -213,6 +212,7 @@ umma_conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     }
     __syncthreads();
     tc_fence_after();
+    chain_release();
     const uint32_t tmem_base = *tmem_slot_ptr;
 
     if (warp == 0) {

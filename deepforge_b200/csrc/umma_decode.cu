@@ -143,6 +143,7 @@ sdpa_decode_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         prefetch_tensormap(&map_k);
         prefetch_tensormap(&map_v);
     }
+    chain_wait();
     const int chunk = blockIdx.x;
     const int kv_head = blockIdx.y;
     const int64_t batch = blockIdx.z;
@@ -213,6 +214,7 @@ sdpa_decode_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot_ptr;
+    chain_release();
     const uint32_t tmem_o = tmem_base + 32;  // S^T buffers at +0 and +16, O^T at +32
 
     if (warp == 0) {
@@ -527,7 +529,7 @@ int launch_decode_umma(const dfgpu_sdpa_params& p, void* const* tensors, void* s
     auto run = [&](auto kernel, int dynamic) -> int {
         cudaError_t error = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dynamic);
         if (error != cudaSuccess) return fail(kExecutionFailed, "SDPA decode: cannot reserve %d bytes of shared memory: %s", dynamic, cudaGetErrorString(error));
-        kernel<<<grid, kDecodeThreads, dynamic, stream>>>(map_q, map_k, map_v, args);
+        launch_chained(kernel, dim3(grid), dim3(kDecodeThreads), dynamic, stream, map_q, map_k, map_v, args);
         return check_launch("SDPA paged decode (tcgen05)");
     };
     // three ring slots: two CTAs per SM (about 219 KiB of shared memory together) hide each other's softmax latency

@@ -126,6 +126,8 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot_ptr;
+    chain_wait();
+    chain_release();
     if (warp == 0) {
         if (lane == 0) {
             const uint32_t a_bytes = args.is_conv ? static_cast<uint32_t>(args.rows_per_tile * args.out_q * kBlockK * 2) : L::kABytes;
@@ -352,7 +354,6 @@ umma_conv_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(generic_base + pargs.barrier_offset + 8 * (2 * kMaxRingStages + 17));
 
     const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
-    chain_release();  // the next kernel of the plan may start taking SMs as this one's CTAs leave
     if (threadIdx.x == 0) {
         prefetch_tensormap(&map_a);
         prefetch_tensormap(&map_b);
@@ -505,6 +506,7 @@ umma_conv_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     if (warp != 0 && pargs.early_static) chain_wait();  // the bias vectors above are static operands
     __syncthreads();
     tc_fence_after();
+    chain_release();  // the next kernel of the plan may start taking SMs as this one's CTAs leave
     const uint32_t tmem_base = *tmem_slot_ptr;
 
     if (warp == 0) {
@@ -729,7 +731,7 @@ umma_conv_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __g
 // ---- host side ----------------------------------------------------------------------------
 
 template <int BN, int STAGES>
-int launch(const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmArgs& args, dim3 grid, cudaStream_t stream, bool chained) {
+int launch(const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmArgs& args, dim3 grid, cudaStream_t stream) {
     using L = SmemLayout<BN, STAGES>;
     static bool configured = false;
     if (!configured) {
@@ -737,31 +739,27 @@ int launch(const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmArgs& a
         if (error != cudaSuccess) return fail(kExecutionFailed, "tcgen05 GEMM: cannot reserve %d bytes of shared memory: %s", L::kDynamic, cudaGetErrorString(error));
         configured = true;
     }
-    if (chained) {
-        cudaError_t error = launch_chained(umma_gemm_kernel<BN, STAGES>, grid, dim3(kThreads), L::kDynamic, stream, map_a, map_b, args);
-        if (error != cudaSuccess) return fail(kExecutionFailed, "tcgen05 GEMM: launch failed: %s", cudaGetErrorString(error));
-    } else {
-        umma_gemm_kernel<BN, STAGES><<<grid, kThreads, L::kDynamic, stream>>>(map_a, map_b, args);
-    }
+    cudaError_t error = launch_chained(umma_gemm_kernel<BN, STAGES>, grid, dim3(kThreads), L::kDynamic, stream, map_a, map_b, args);
+    if (error != cudaSuccess) return fail(kExecutionFailed, "tcgen05 GEMM: launch failed: %s", cudaGetErrorString(error));
     return check_launch("tcgen05 GEMM");
 }
 
 // Ring depth: shallow K loops (the 1x1 convolutions) get short rings so that several CTAs fit on
 // one SM and overlap each other's load / MMA / epilogue phases; deep K loops (matmul) get 4 stages.
-int dispatch(int bn, int k_blocks, const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmArgs& args, dim3 grid, cudaStream_t stream, bool chained = false) {
+int dispatch(int bn, int k_blocks, const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmArgs& args, dim3 grid, cudaStream_t stream) {
     const int stages = k_blocks <= 1 ? 1 : (k_blocks <= 12 ? 2 : 4);
     if (bn == 64) {
-        if (stages == 1) return launch<64, 1>(map_a, map_b, args, grid, stream, chained);
-        if (stages == 2) return launch<64, 2>(map_a, map_b, args, grid, stream, chained);
-        return launch<64, 4>(map_a, map_b, args, grid, stream, chained);
+        if (stages == 1) return launch<64, 1>(map_a, map_b, args, grid, stream);
+        if (stages == 2) return launch<64, 2>(map_a, map_b, args, grid, stream);
+        return launch<64, 4>(map_a, map_b, args, grid, stream);
     }
     if (bn == 128) {
-        if (stages == 1) return launch<128, 1>(map_a, map_b, args, grid, stream, chained);
-        if (stages == 2) return launch<128, 2>(map_a, map_b, args, grid, stream, chained);
-        return launch<128, 4>(map_a, map_b, args, grid, stream, chained);
+        if (stages == 1) return launch<128, 1>(map_a, map_b, args, grid, stream);
+        if (stages == 2) return launch<128, 2>(map_a, map_b, args, grid, stream);
+        return launch<128, 4>(map_a, map_b, args, grid, stream);
     }
-    if (stages <= 2) return launch<256, 2>(map_a, map_b, args, grid, stream, chained);
-    return launch<256, 4>(map_a, map_b, args, grid, stream, chained);
+    if (stages <= 2) return launch<256, 2>(map_a, map_b, args, grid, stream);
+    return launch<256, 4>(map_a, map_b, args, grid, stream);
 }
 
 constexpr int kSmemBudget = 227 * 1024;

@@ -218,7 +218,6 @@ umma_mxf8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             n0 += half * (BN / 2);
         }
     };
-    chain_release();
 
     if (warp == 0) {
         if (leader) {
@@ -240,6 +239,7 @@ umma_mxf8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot_ptr;
     chain_wait();  // barriers and tensor memory are set up; from here on the previous kernel's output is read
+    chain_release();
 
     if (warp == 0) {
         // ---- TMA loader ----

@@ -123,6 +123,8 @@ sdpa_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot_ptr;
+    chain_wait();
+    chain_release();
     const uint32_t tmem_o = tmem_base + 256;  // S0 at +0, S1 at +128, O at +256
 
     if (warp == 0) {
@@ -576,6 +578,8 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot_ptr;
+    chain_wait();
+    chain_release();
 
     if (warp == 16) {
         const bool leader = elect_one();
@@ -1041,11 +1045,11 @@ int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, void* scr
         const int64_t units = static_cast<int64_t>(args.causal ? (pairs + 1) / 2 : pairs) * batch * hq;
         args.batch_heads = static_cast<int>(batch * hq);
         const unsigned grid = static_cast<unsigned>(units < sm_count ? units : sm_count);
-        sdpa_umma_pair_kernel<<<grid, kPairThreads, PairSmem::kDynamic, stream>>>(map_q, map_k, map_v, map_o, args);
+        launch_chained(sdpa_umma_pair_kernel, dim3(grid), dim3(kPairThreads), PairSmem::kDynamic, stream, map_q, map_k, map_v, map_o, args);
         return check_launch("SDPA (tcgen05, two query tiles per CTA)");
     }
     dim3 grid(static_cast<unsigned>(args.q_tiles), static_cast<unsigned>(batch * hq));
-    sdpa_umma_kernel<<<grid, kSdpaThreads, Smem::kDynamic, stream>>>(map_q, map_k, map_v, map_o, args);
+    launch_chained(sdpa_umma_kernel, dim3(grid), dim3(kSdpaThreads), Smem::kDynamic, stream, map_q, map_k, map_v, map_o, args);
     return check_launch("SDPA (tcgen05)");
 }
 
