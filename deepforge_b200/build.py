@@ -1,11 +1,13 @@
-"""In-tree builds of the two native libraries (no JIT cache, no pip install).
+"""In-tree builds of the native libraries (no JIT cache, no pip install).
 
 libdfgpu.so         CUDA kernels + the C ABI of include/dfgpu.h, compiled for sm_100a only.
 libdeepforge_b200.so  C++20 host side (importer, graph analysis, workspace planner,
                     kernel-selection lowering, runtime) + the flat C API of
                     include/deepforge_b200.h. It links libdfgpu.so.
 
-Both land in deepforge_b200/_build/. nvcc cross-compiles without a GPU.
+_execute.so         the CPython entry to Executable.execute (host/python/execute_module.cpp).
+
+All land in deepforge_b200/_build/. nvcc cross-compiles without a GPU.
 """
 from __future__ import annotations
 
@@ -64,7 +66,7 @@ def nlohmann_include() -> Path:
 def build_kernels(force: bool = False, verbose: bool = False) -> Path:
     OUT.mkdir(exist_ok=True)
     sources = sorted((PKG / "csrc").glob("*.cu"))
-    headers = sorted((PKG / "csrc").glob("*.cuh")) + [ROOT / "include" / "dfgpu.h"]
+    headers = sorted((PKG / "csrc").glob("*.cuh")) + sorted((PKG / "csrc").glob("*.h")) + [ROOT / "include" / "dfgpu.h"]
     target = OUT / "libdfgpu.so"
     stamp = _stamp(sources + headers, " ".join(NVCC_FLAGS))
     if not force and _up_to_date(target, stamp):
@@ -95,7 +97,7 @@ def build_host(force: bool = False) -> Path:
     OUT.mkdir(exist_ok=True)
     kernels = build_kernels()
     sources = sorted((PKG / "host").glob("*.cpp"))
-    headers = sorted((ROOT / "include").rglob("*.h"))
+    headers = sorted((ROOT / "include").rglob("*.h")) + sorted((PKG / "csrc").glob("*.h")) + sorted((PKG / "host").glob("*.h"))
     target = OUT / "libdeepforge_b200.so"
     flags = ["-std=c++20", "-O2", "-fPIC", "-Wall", "-Wextra", "-Wno-unused-parameter"]
     stamp = _stamp(sources + headers, " ".join(flags))
@@ -106,6 +108,23 @@ def build_host(force: bool = False) -> Path:
     _run(command)
     target.with_suffix(".so.stamp").write_text(stamp)
     assert kernels.exists()
+    return target
+
+
+def build_python_entry(force: bool = False) -> Path:
+    """_execute.so (host/python/execute_module.cpp), linked against the host library beside it."""
+    library = build_host()
+    source = PKG / "host" / "python" / "execute_module.cpp"
+    target = OUT / "_execute.so"
+    include = sysconfig.get_paths()["include"]
+    flags = ["-std=c++20", "-O2", "-fPIC", "-Wall", "-Wextra"]
+    stamp = _stamp([source, ROOT / "include" / "deepforge_b200.h"], " ".join(flags) + include)
+    if not force and _up_to_date(target, stamp):
+        return target
+    _run(["g++", *flags, "-shared", "-I", str(ROOT / "include"), "-I", include, str(source), "-o", str(target), f"-L{OUT}", "-ldeepforge_b200", "-ldfgpu",
+          "-Wl,-rpath,$ORIGIN"])
+    target.with_suffix(".so.stamp").write_text(stamp)
+    assert library.exists()
     return target
 
 
@@ -154,6 +173,7 @@ def build_benchmark_tool(force: bool = False) -> Path:
 def build_all(force: bool = False) -> None:
     build_kernels(force)
     build_host(force)
+    build_python_entry(force)
     build_cli(force)
     build_benchmark_tool(force)
 

@@ -8,6 +8,8 @@
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <tuple>
+#include <utility>
 
 #include "dfgpu.h"
 
@@ -61,6 +63,10 @@ inline bool valid_tensor(const dfgpu_tensor& t) {
 
 int sm_count();
 
+// Sends one kernel off (chained, see below) and writes it down when the thread has a recorder open (launch_record.h).
+cudaError_t submit(const void* function, dim3 grid, dim3 block, unsigned cluster, size_t dynamic_smem, cudaStream_t stream, void** arguments,
+                   const size_t* sizes, size_t count);
+
 // ---- programmatic dependent launch ------------------------------------------------
 // A kernel launched with launch_chained() may start while the kernel before it in the stream is still
 // draining: its CTAs take SMs as the earlier kernel's CTAs leave, run their private prologue (barrier
@@ -90,19 +96,22 @@ __device__ __forceinline__ void chain_begin() {
     chain_wait();
 }
 
+template <typename... Params, std::size_t... I, typename... Args>
+cudaError_t launch_chained_clusters(std::index_sequence<I...>, void (*kernel)(Params...), dim3 grid, dim3 block, unsigned cluster, size_t dynamic_smem,
+                                    cudaStream_t stream, Args&&... args) {
+    std::tuple<std::remove_cv_t<Params>...> held(static_cast<Params>(args)...);
+    void* pointers[] = {static_cast<void*>(&std::get<I>(held))...};
+    constexpr size_t sizes[] = {sizeof(std::remove_cv_t<Params>)...};
+    return submit(reinterpret_cast<const void*>(kernel), grid, block, cluster, dynamic_smem, stream, pointers, sizes, sizeof...(Params));
+}
 template <typename... Params, typename... Args>
 cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t dynamic_smem, cudaStream_t stream, Args&&... args) {
-    cudaLaunchConfig_t config{};
-    config.gridDim = grid;
-    config.blockDim = block;
-    config.dynamicSmemBytes = dynamic_smem;
-    config.stream = stream;
-    cudaLaunchAttribute attribute[1];
-    attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute[0].val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = attribute;
-    config.numAttrs = 1;
-    return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+    return launch_chained_clusters(std::index_sequence_for<Params...>{}, kernel, grid, block, 0u, dynamic_smem, stream, std::forward<Args>(args)...);
+}
+// The same with `cluster` CTAs along x forming a thread-block cluster.
+template <typename... Params, typename... Args>
+cudaError_t launch_chained_cluster(void (*kernel)(Params...), dim3 grid, dim3 block, unsigned cluster, size_t dynamic_smem, cudaStream_t stream, Args&&... args) {
+    return launch_chained_clusters(std::index_sequence_for<Params...>{}, kernel, grid, block, cluster, dynamic_smem, stream, std::forward<Args>(args)...);
 }
 #endif
 

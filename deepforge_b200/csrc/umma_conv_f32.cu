@@ -566,21 +566,9 @@ static int launch_clusters(ClusterForm form, ClusterConvArgs g, const ConvArgs& 
     g.by_chunks = make_fast_divisor(static_cast<uint32_t>(form.chunks));
     g.by_s = make_fast_divisor(static_cast<uint32_t>(g.S));
     g.by_tiles = make_fast_divisor(static_cast<uint32_t>(std::max(1, g.tiles_per_image)));
-    cudaLaunchConfig_t config{};
-    config.gridDim = dim3(form.ranks, form.tiles_m, form.tiles_n);
-    config.blockDim = dim3(kThreads);
-    config.dynamicSmemBytes = kSmemBytes;
-    config.stream = stream;
-    cudaLaunchAttribute attribute[2]{};
-    attribute[0].id = cudaLaunchAttributeClusterDimension;
-    attribute[0].val.clusterDim.x = form.ranks;
-    attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
-    attribute[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute[1].val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = attribute;
-    config.numAttrs = 2;
     const bool fast = g.x_quads && g.w_quads && g.y_quads && a.groups == 1 && g.tiles_per_image == 0 && g.depth_out * g.depth_in * g.depth_taps == 1;
-    cudaError_t error = fast ? cudaLaunchKernelEx(&config, umma_conv_f32_kernel<true>, g, a) : cudaLaunchKernelEx(&config, umma_conv_f32_kernel<false>, g, a);
+    cudaError_t error = launch_chained_cluster(fast ? umma_conv_f32_kernel<true> : umma_conv_f32_kernel<false>, dim3(form.ranks, form.tiles_m, form.tiles_n), dim3(kThreads),
+                                               static_cast<unsigned>(form.ranks), kSmemBytes, stream, g, a);
     if (error != cudaSuccess) return fail(kExecutionFailed, "%s: cluster launch failed: %s", what, cudaGetErrorString(error));
     return check_launch(what);
 }

@@ -213,17 +213,12 @@ extern "C" int df_conv2d_metadata(const df_executable* executable, int32_t* adap
 extern "C" void df_set_stream(df_executable* executable, void* stream) { executable->result.executable->set_stream(stream); }
 
 extern "C" int df_execute(const df_executable* executable, void* handle, const int64_t* uids, void* const* pointers, size_t count, void* workspace) {
-    runtime::VariantPack pack;
-    pack.reserve(count);
-    for (size_t i = 0; i < count; ++i) pack[uids[i]] = pointers[i];
-    return report(executable->result.executable->execute(handle, pack, workspace));
+    (void)handle;
+    return report(executable->result.executable->execute_list(uids, pointers, count, workspace, nullptr, false));
 }
 
 extern "C" int df_execute_on(const df_executable* executable, void* stream, const int64_t* uids, void* const* pointers, size_t count, void* workspace) {
-    runtime::VariantPack pack;
-    pack.reserve(count);
-    for (size_t i = 0; i < count; ++i) pack[uids[i]] = pointers[i];
-    return report(executable->result.executable->execute_on(stream, pack, workspace));
+    return report(executable->result.executable->execute_list(uids, pointers, count, workspace, stream, true));
 }
 
 extern "C" int64_t df_step_count(const df_executable* executable) { return static_cast<int64_t>(executable->result.plan.steps.size()); }

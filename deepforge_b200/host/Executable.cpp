@@ -8,6 +8,10 @@
 // Pointers are device pointers: they are compared and offset, never dereferenced here.
 #include "Internal.h"
 
+#include "../csrc/launch_record.h"
+
+#include <algorithm>
+#include <array>
 #include <mutex>
 
 namespace deepforge::runtime {
@@ -19,6 +23,19 @@ using compiler::TensorBinding;
 using import::ErrorCode;
 using import::Status;
 
+namespace {
+// What one whole execute() sent off, for the pointers it was given: a host that runs the same buffers again (a training
+// or serving loop does) skips the validation and the launchers, which find the same answers from the same pointers
+// (2.2 us of a 5.4 us one-launch call, 3.4 us of two-launch ones). Kept per executable for the last kReplays pointer
+// sets, so that a host may rotate its buffers; recorded when a set comes by for the second time, so that a host whose
+// pointers are always new pays for the comparison only.
+constexpr std::size_t kReplays = 4;
+struct Replay {
+    std::vector<void*> pointers;   // in the order of the argument table, then the workspace
+    std::shared_ptr<dfgpu::LaunchRecord const> record;   // null: seen once
+};
+}  // namespace
+
 struct Executable::Impl {
     compiler::GraphCompileMetadata metadata;
     compiler::WorkspacePlan workspace;
@@ -26,7 +43,50 @@ struct Executable::Impl {
     void* stream = nullptr;
     std::int64_t launches = 0;
     mutable std::mutex mutex;
+    mutable std::mutex replay_mutex;
+    mutable std::array<Replay, kReplays> replays;
+    mutable std::size_t next_replay = 0, last_replay = 0;
+
+    std::shared_ptr<dfgpu::LaunchRecord const> find_replay(void* const* pointers, std::size_t count, void* workspace, bool& record) const;
+    void keep_replay(std::vector<void*> const& pointers, void* workspace, std::shared_ptr<dfgpu::LaunchRecord const> made) const;
 };
+
+namespace {
+bool same_pointers(Replay const& entry, void* const* pointers, std::size_t count, void* workspace) {
+    if (entry.pointers.size() != count + 1 || entry.pointers[count] != workspace) return false;
+    return std::equal(pointers, pointers + count, entry.pointers.begin());
+}
+}  // namespace
+
+// The record for these pointers, or null; `record` then says whether the call should be written down.
+std::shared_ptr<dfgpu::LaunchRecord const> Executable::Impl::find_replay(void* const* pointers, std::size_t count, void* workspace, bool& record) const {
+    std::lock_guard<std::mutex> lock(replay_mutex);
+    record = false;
+    for (std::size_t i = 0; i < kReplays; ++i) {
+        auto const slot = (last_replay + i) % kReplays;
+        auto const& entry = replays[slot];
+        if (!same_pointers(entry, pointers, count, workspace)) continue;
+        last_replay = slot;
+        if (entry.record && entry.record->device == dfgpu::current_device()) return entry.record;
+        record = true;
+        return nullptr;
+    }
+    auto& entry = replays[next_replay];
+    next_replay = (next_replay + 1) % kReplays;
+    entry.record.reset();
+    entry.pointers.assign(pointers, pointers + count);
+    entry.pointers.push_back(workspace);
+    return nullptr;
+}
+
+void Executable::Impl::keep_replay(std::vector<void*> const& pointers, void* workspace, std::shared_ptr<dfgpu::LaunchRecord const> made) const {
+    std::lock_guard<std::mutex> lock(replay_mutex);
+    for (auto& entry : replays)
+        if (same_pointers(entry, pointers.data(), pointers.size(), workspace)) {
+            entry.record = std::move(made);
+            return;
+        }
+}
 
 std::string_view cpu_variant_name(CpuVariant variant) noexcept {
     switch (variant) {
@@ -60,6 +120,10 @@ Status Executable::get_workspace_size(std::int64_t& workspace_size) const {
 }
 
 namespace {
+Status missing_uid(compiler::TensorArgumentMetadata const& argument) {
+    return Status::failure(ErrorCode::kInvalidVariantPack, argument.name, "UID " + std::to_string(argument.uid) + " is missing from the variant pack");
+}
+
 Status reject_overrides(OverrideUids const& uids, OverrideShapes const& shapes, OverrideStrides const& strides) {
     if (uids.empty() && shapes.empty() && strides.empty()) return Status::ok();
     return Status::failure(ErrorCode::kInvalidVariantPack, "override", "the graph was compiled without shape overrides");
@@ -117,7 +181,51 @@ Status Executable::execute_steps(std::int64_t first, std::int64_t last, VariantP
 }
 
 Status Executable::run_steps(std::int64_t first, std::int64_t last, VariantPack& pack, void* workspace, void* call_stream, bool own_stream) const {
+    auto const& arguments = impl_->metadata.arguments;
+    std::vector<void*> pointers(arguments.size());
+    for (std::size_t i = 0; i < arguments.size(); ++i) {
+        auto it = pack.find(arguments[i].uid);
+        if (it == pack.end()) return missing_uid(arguments[i]);
+        pointers[i] = it->second;
+    }
+    return run_bound(first, last, pointers.data(), workspace, call_stream, own_stream);
+}
+
+Status Executable::execute_list(std::int64_t const* uids, void* const* list, std::size_t count, void* workspace, void* call_stream, bool own_stream) const {
+    auto const& arguments = impl_->metadata.arguments;
+    constexpr std::size_t kFew = 32;   // (above, a map beats the scan)
+    if (count > kFew || arguments.size() > kFew) {
+        VariantPack pack;
+        pack.reserve(count);
+        for (std::size_t i = 0; i < count; ++i) pack[uids[i]] = list[i];
+        return run_steps(0, static_cast<std::int64_t>(impl_->plan.steps.size()), pack, workspace, call_stream, own_stream);
+    }
+    void* pointers[kFew];
+    for (std::size_t i = 0; i < arguments.size(); ++i) {
+        std::size_t at = count;
+        while (at > 0 && uids[at - 1] != arguments[i].uid) --at;   // from the end: the last entry of a UID counts, as in a map
+        if (at == 0) return missing_uid(arguments[i]);
+        pointers[i] = list[at - 1];
+    }
+    return run_bound(0, static_cast<std::int64_t>(impl_->plan.steps.size()), pointers, workspace, call_stream, own_stream);
+}
+
+// bound: one pointer per entry of the argument table, in its order.
+Status Executable::run_bound(std::int64_t first, std::int64_t last, void* const* bound, void* workspace, void* call_stream, bool own_stream) const {
     auto const& impl = *impl_;
+    auto const argument_count = impl.metadata.arguments.size();
+    bool const whole = first == 0 && last == static_cast<std::int64_t>(impl.plan.steps.size());
+    bool write_down = false;
+    if (whole)
+        if (auto record = impl.find_replay(bound, argument_count, workspace, write_down)) {
+            std::unique_lock<std::mutex> lock(impl.mutex, std::defer_lock);
+            if (!own_stream) {
+                lock.lock();
+                call_stream = impl.stream;
+            }
+            int const code = dfgpu::replay(*record, call_stream);
+            return code == 0 ? Status::ok() : Status::failure(static_cast<ErrorCode>(code), "execute", dfgpu_last_error());
+        }
     if (first < 0 || last > static_cast<std::int64_t>(impl.plan.steps.size()) || first > last)
         return Status::failure(ErrorCode::kInvalidArgument, "steps", "step range is outside the kernel plan");
 
@@ -128,11 +236,10 @@ Status Executable::run_steps(std::int64_t first, std::int64_t last, VariantPack&
     };
     std::vector<Range> ranges;
     ranges.reserve(impl.metadata.arguments.size());
-    for (auto const& argument : impl.metadata.arguments) {
-        auto it = pack.find(argument.uid);
-        if (it == pack.end()) return Status::failure(ErrorCode::kInvalidVariantPack, argument.name, "UID " + std::to_string(argument.uid) + " is missing from the variant pack");
-        if (it->second == nullptr) return Status::failure(ErrorCode::kInvalidVariantPack, argument.name, "pointer is null");
-        auto address = reinterpret_cast<std::uintptr_t>(it->second);
+    for (std::size_t i = 0; i < argument_count; ++i) {
+        auto const& argument = impl.metadata.arguments[i];
+        if (bound[i] == nullptr) return Status::failure(ErrorCode::kInvalidVariantPack, argument.name, "pointer is null");
+        auto address = reinterpret_cast<std::uintptr_t>(bound[i]);
         if (address % argument.alignment != 0) return Status::failure(ErrorCode::kInvalidVariantPack, argument.name, "pointer is not aligned to " + std::to_string(argument.alignment) + " bytes");
         ranges.push_back({address, address + argument.size_bytes, argument.access != TensorAccess::kRead, &argument.name});
     }
@@ -160,11 +267,22 @@ Status Executable::run_steps(std::int64_t first, std::int64_t last, VariantPack&
     }
     auto resolve = [&](TensorBinding const& binding) -> void* {
         switch (binding.kind) {
-            case TensorBinding::Kind::kArgument: return pack.at(binding.uid);
+            case TensorBinding::Kind::kArgument: {   // (the table is in ascending UID order, or X, W, Y for a single convolution)
+                auto const& arguments = impl.metadata.arguments;
+                for (std::size_t i = 0; i < argument_count; ++i)
+                    if (arguments[i].uid == binding.uid) return bound[i];
+                return nullptr;
+            }
             case TensorBinding::Kind::kWorkspace: return static_cast<char*>(workspace) + binding.offset;
             default: return nullptr;
         }
     };
+    dfgpu::LaunchRecord made;
+    struct Recorder {
+        bool open;
+        Recorder(bool wanted, dfgpu::LaunchRecord& record) : open(wanted) { if (open) dfgpu::open_recorder(&record); }
+        ~Recorder() { if (open) dfgpu::close_recorder(); }
+    } recorder(write_down, made);
     std::vector<void*> pointers;
     for (std::int64_t index = first; index < last; ++index) {
         auto const& step = impl.plan.steps[static_cast<std::size_t>(index)];
@@ -201,6 +319,8 @@ Status Executable::run_steps(std::int64_t first, std::int64_t last, VariantPack&
             return Status::failure(mapped, step.label, dfgpu_last_error());
         }
     }
+    if (write_down && made.device >= 0)
+        impl.keep_replay(std::vector<void*>(bound, bound + argument_count), workspace, std::make_shared<dfgpu::LaunchRecord const>(std::move(made)));
     return Status::ok();
 }
 

@@ -7,6 +7,8 @@ legacy default stream unless told otherwise); synchronisation is the caller's bu
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import json
 from pathlib import Path
 from typing import Dict, Mapping, Optional, Union
@@ -23,6 +25,7 @@ EXPORTS = [
 ]
 
 _LIB: Optional[C.CDLL] = None
+_execute = None  # set by load()
 
 
 class DeepForgeError(RuntimeError):
@@ -59,8 +62,21 @@ def load() -> C.CDLL:
         lib.df_argument_name.restype = C.c_size_t
         lib.df_argument_name.argtypes = [C.c_void_p, C.c_int64, C.c_char_p, C.c_size_t]
         lib.df_set_stream.argtypes = [C.c_void_p, C.c_void_p]
+        _load_execute()
         _LIB = lib
     return _LIB
+
+
+def _load_execute() -> None:
+    """Binds _execute, the native entry of Executable.execute / execute_on (host/python/execute_module.cpp)."""
+    global _execute
+    path = library_path().with_name("_execute.so")
+    if not path.exists():
+        raise RuntimeError(f"{path} is missing: run `python -m deepforge_b200.build` (or __graft_entry__.build())")
+    loader = importlib.machinery.ExtensionFileLoader("_execute", str(path))
+    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_execute", str(path), loader=loader))
+    loader.exec_module(module)
+    _execute = module.execute
 
 
 def _check(code: int) -> None:
@@ -97,6 +113,7 @@ def dump_graph(document: Union[str, bytes, dict], fmt: int = FORMAT_AUTO) -> str
 class Executable:
     def __init__(self, handle: int):
         self._handle = C.c_void_p(handle)
+        self._address = handle
 
     def __del__(self):
         if getattr(self, "_handle", None) and _LIB is not None:
@@ -174,18 +191,17 @@ class Executable:
         _check(load().df_execute_steps(self._handle, C.c_int64(first), C.c_int64(last), uids, pointers, C.c_size_t(count), C.c_void_p(workspace or None)))
 
     def execute(self, pack: Mapping[int, int], workspace: Optional[int] = None, handle: Optional[int] = None) -> None:
-        count = len(pack)
-        uids = (C.c_int64 * count)(*pack.keys())
-        pointers = (C.c_void_p * count)(*[C.c_void_p(p or None) for p in pack.values()])
-        _check(load().df_execute(self._handle, C.c_void_p(handle or None), uids, pointers, C.c_size_t(count), C.c_void_p(workspace or None)))
+        # (the handle is accepted and never looked at, as in the C++ call)
+        code = _execute(self._address, pack if type(pack) is dict else dict(pack), workspace, None, False)
+        if code:
+            _check(code)
 
     def execute_on(self, stream: int, pack: Mapping[int, int], workspace: Optional[int] = None) -> None:
         """execute() with the launches on `stream` (a cudaStream_t) for this call only; safe to call from several
         threads at once with different streams, workspaces and outputs (ctypes releases the GIL during the call)."""
-        count = len(pack)
-        uids = (C.c_int64 * count)(*pack.keys())
-        pointers = (C.c_void_p * count)(*[C.c_void_p(p or None) for p in pack.values()])
-        _check(load().df_execute_on(self._handle, C.c_void_p(stream or None), uids, pointers, C.c_size_t(count), C.c_void_p(workspace or None)))
+        code = _execute(self._address, pack if type(pack) is dict else dict(pack), workspace, stream, True)
+        if code:
+            _check(code)
 
 
 def compile_graph(document: Union[str, bytes, dict], fmt: int = FORMAT_AUTO, options: int = 0) -> Executable:

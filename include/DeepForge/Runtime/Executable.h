@@ -6,6 +6,7 @@
 
 #include "DeepForge/Import/Status.h"
 
+#include <cstddef>
 #include <cstdint>
 #include <memory>
 #include <string>
@@ -80,10 +81,14 @@ public:
     // Runs plan steps [first, last) only, after the same validation as execute().
     [[nodiscard]] import::Status execute_steps(std::int64_t first, std::int64_t last, VariantPack& uid_to_device_ptr, void* workspace) const;
 
+    // execute() / execute_on() for hosts that hold the pack as two arrays (of one UID given twice the last entry counts);
+    // `own_stream` false: the stream of set_stream().
+    [[nodiscard]] import::Status execute_list(std::int64_t const* uids, void* const* device_ptrs, std::size_t count, void* workspace, void* stream,
+                                              bool own_stream) const;
+
 private:
     import::Status run_steps(std::int64_t first, std::int64_t last, VariantPack& pack, void* workspace, void* stream, bool own_stream) const;
-
-public:
+    import::Status run_bound(std::int64_t first, std::int64_t last, void* const* bound, void* workspace, void* stream, bool own_stream) const;
 
 private:
     struct Impl;
