@@ -322,6 +322,10 @@ extern "C" int dfgpu_matmul(const dfgpu_matmul_params* p, void* const* tensors, 
     status = choose_kernel(*p, kernel);
     if (status) return status;
     cudaStream_t stream = as_stream(stream_handle);
+    // (AUTO: operands off the 16-byte boundary TMA needs are read by the CUDA-core kernel instead)
+    if (p->kernel == DFGPU_MATMUL_AUTO && (kernel == DFGPU_MATMUL_UMMA_BF16 || kernel == DFGPU_MATMUL_UMMA_MXF8) &&
+        ((reinterpret_cast<uintptr_t>(tensors[0]) | reinterpret_cast<uintptr_t>(tensors[1])) & 15u) != 0)
+        kernel = DFGPU_MATMUL_FFMA;
     if (kernel == DFGPU_MATMUL_UMMA_F32X3_CLUSTER) return launch_matmul_f32_cluster(*p, tensors, stream);  // (any f32 pointer: 4-byte alignment is enough)
     if (kernel == DFGPU_MATMUL_UMMA_F32X3) {
         SplitMatmul split;

@@ -4,7 +4,7 @@
 // 0.0 in k order, the two descales are separate multiplications, Amax_C folds maximumf (NaN-propagating) from 0.0
 // over |value|, and C takes value * Scale_C through store_from_f32. The kernel here is the general one (any rank,
 // batch broadcast over extent-1 axes, any strides; one thread per output element, so the k order is the
-// reference's); large aligned problems go to the tcgen05 kernel in umma_mxf8.cu, whose f32 additions run in the
+// reference's); problems whose rows start on 16-byte boundaries go to the tcgen05 kernel in umma_matmul.cu, whose f32 additions run in the
 // tensor core's order. Amax_C is cleared by a one-word kernel in front and folded with an atomic maximum on the bits of
 // the non-negative f32 (NaN, made canonical, is the largest pattern, so it sticks like maximumf's).
 #include "common.cuh"
@@ -143,6 +143,8 @@ extern "C" int dfgpu_matmul_fp8(const dfgpu_matmul_fp8_params* p, void* const* t
     launch_chained(clear_amax_kernel, dim3(1), dim3(32), 0, stream, g.amax_bits);
     status = check_launch("MATMUL_FP8: clearing Amax_C");
     if (status) return status;
+    // (AUTO: operands off the 16-byte boundary TMA needs are read by the general kernel instead)
+    if (p->kernel == DFGPU_MATMUL_FP8_AUTO && ((reinterpret_cast<uintptr_t>(tensors[0]) | reinterpret_cast<uintptr_t>(tensors[1])) & 15u) != 0) kernel = DFGPU_MATMUL_FP8_SCALAR;
     if (kernel == DFGPU_MATMUL_FP8_UMMA) return launch_matmul_fp8_umma(*p, tensors, stream);
     int64_t batches = 1;
     for (int i = 0; i < g.rank - 2; ++i) batches *= p->c.dim[i];

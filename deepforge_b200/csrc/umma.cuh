@@ -66,17 +66,14 @@ struct SplitOperand {
 int split_flag_count(const SplitOperand& first, const SplitOperand& second);
 int launch_split6(const SplitOperand& first, const SplitOperand& second, int* flags, cudaStream_t stream);
 
-// MATMUL on tcgen05: kernel is DFGPU_MATMUL_UMMA_BF16 or DFGPU_MATMUL_UMMA_MXF8.
+// MATMUL on tcgen05 (umma_matmul.cu): kernel is DFGPU_MATMUL_UMMA_BF16 (bf16 or f16 operands) or DFGPU_MATMUL_UMMA_MXF8 (codes
+// and E8M0 block scales, no dequantize pass). Any extents; rows on 16-byte boundaries.
 bool matmul_umma_supported(const dfgpu_matmul_params& p, int kernel);
 int launch_matmul_umma(const dfgpu_matmul_params& p, void* const* tensors, int kernel, cudaStream_t stream);
-
-// MATMUL on MXFP8 codes + E8M0 block scales (tcgen05 block-scaled kind), no dequantize pass.
-bool matmul_mxf8_supported(const dfgpu_matmul_params& p);
-int launch_matmul_mxf8(const dfgpu_matmul_params& p, void* const* tensors, cudaStream_t stream);
-// MATMUL_FP8 on the same kernel: unit block scales, the three scalars and Amax_C applied in the epilogue.
+// MATMUL_FP8: the three scalars and Amax_C applied in the epilogue.
 bool matmul_fp8_umma_supported(const dfgpu_matmul_fp8_params& p);
 int launch_matmul_fp8_umma(const dfgpu_matmul_fp8_params& p, void* const* tensors, cudaStream_t stream);
-int mxf8_device_status(int* status);
+int matmul_tiles_device_status(int* status);
 
 // SDPA forward on tcgen05 (bf16, head dim 128, contiguous K/V).
 bool sdpa_umma_supported(const dfgpu_sdpa_params& p);

@@ -1085,72 +1085,6 @@ ConvKSplit conv_umma_k_split(const dfgpu_conv_params& p) {
     return split;
 }
 
-bool matmul_umma_supported(const dfgpu_matmul_params& p, int kernel) {
-    if (kernel == DFGPU_MATMUL_UMMA_MXF8) return matmul_mxf8_supported(p);
-    if (kernel != DFGPU_MATMUL_UMMA_BF16) return false;
-    if (p.a_scale.rank || p.b_scale.rank) return false;
-    if (p.a.dtype != DFGPU_BF16 || p.b.dtype != DFGPU_BF16 || (p.c.dtype != DFGPU_BF16 && p.c.dtype != DFGPU_F32)) return false;
-    const int rank = p.c.rank;
-    if (rank < 2) return false;
-    for (int i = 0; i < rank - 2; ++i)
-        if (p.c.dim[i] != 1 || p.a.dim[i] != 1 || p.b.dim[i] != 1) return false;
-    const int64_t M = p.c.dim[rank - 2], N = p.c.dim[rank - 1], K = p.a.dim[rank - 1];
-    if (K % 64 != 0 || N % 64 != 0 || M < 1 || M > (1ll << 30)) return false;
-    if (p.a.stride[rank - 1] != 1 || p.a.stride[rank - 2] % 8 != 0 || p.a.stride[rank - 2] < K) return false;
-    const bool b_k_major = p.b.stride[rank - 2] == 1 && p.b.stride[rank - 1] % 8 == 0 && p.b.stride[rank - 1] >= K;
-    const bool b_n_major = p.b.stride[rank - 1] == 1 && p.b.stride[rank - 2] % 8 == 0 && p.b.stride[rank - 2] >= N;
-    if (!b_k_major && !b_n_major) return false;
-    if (p.c.stride[rank - 1] != 1 || p.c.stride[rank - 2] % 8 != 0 || p.c.stride[rank - 2] < N) return false;
-    return translate_epilogue(p.epilogue_count, p.epilogue, p.extra, p.c, rank - 1, true, p.c.stride[rank - 2], nullptr, nullptr);
-}
-
-int launch_matmul_umma(const dfgpu_matmul_params& p, void* const* tensors, int kernel, cudaStream_t stream) {
-    if (kernel == DFGPU_MATMUL_UMMA_MXF8) return launch_matmul_mxf8(p, tensors, stream);
-    const int rank = p.c.rank;
-    const int64_t M = p.c.dim[rank - 2], N = p.c.dim[rank - 1], K = p.a.dim[rank - 1];
-    if (!aligned16(tensors[0]) || !aligned16(tensors[1]) || !aligned16(tensors[2]))
-        return fail(kInvalidArgument, "MATMUL: the tcgen05 kernel needs 16-byte aligned A, B and C");
-    const int bn = pick_bn(N, K / kBlockK);
-    const bool b_k_major = p.b.stride[rank - 2] == 1 && p.b.stride[rank - 1] % 8 == 0 && p.b.stride[rank - 1] >= K;
-    const bool b_n_major = !b_k_major;
-    GemmArgs args{};
-    CUtensorMap map_a, map_b;
-    {
-        uint64_t dims[2] = {static_cast<uint64_t>(K), static_cast<uint64_t>(M)};
-        uint64_t strides[1] = {static_cast<uint64_t>(p.a.stride[rank - 2]) * 2};
-        uint32_t box[2] = {kBlockK, kTileM};
-        int status = make_map(&map_a, tensors[0], 2, dims, strides, box, "MATMUL A");
-        if (status) return status;
-    }
-    if (b_n_major) {
-        uint64_t dims[2] = {static_cast<uint64_t>(N), static_cast<uint64_t>(K)};
-        uint64_t strides[1] = {static_cast<uint64_t>(p.b.stride[rank - 2]) * 2};
-        uint32_t box[2] = {64, kBlockK};
-        int status = make_map(&map_b, tensors[1], 2, dims, strides, box, "MATMUL B");
-        if (status) return status;
-    } else {
-        uint64_t dims[2] = {static_cast<uint64_t>(K), static_cast<uint64_t>(N)};
-        uint64_t strides[1] = {static_cast<uint64_t>(p.b.stride[rank - 1]) * 2};
-        uint32_t box[2] = {kBlockK, static_cast<uint32_t>(bn)};
-        int status = make_map(&map_b, tensors[1], 2, dims, strides, box, "MATMUL B");
-        if (status) return status;
-    }
-    args.is_conv = 0;
-    args.m_total = M;
-    args.k_blocks_per_tap = static_cast<int>(K / kBlockK);
-    args.k_blocks = args.k_blocks_per_tap;
-    args.filter_s = 1;
-    args.b_mn_major = b_n_major ? 1 : 0;
-    args.n_total = N;
-    args.out = tensors[2];
-    args.out_ld = p.c.stride[rank - 2];
-    args.out_dtype = p.c.dtype;
-    if (!translate_epilogue(p.epilogue_count, p.epilogue, p.extra, p.c, rank - 1, true, args.out_ld, tensors + 5, &args))
-        return fail(kUnsupported, "MATMUL: the fused epilogue is not one the tcgen05 kernel applies");
-    dim3 grid(static_cast<unsigned>((M + kTileM - 1) / kTileM), static_cast<unsigned>(N / bn));
-    return dispatch(bn, args.k_blocks, map_a, map_b, args, grid, stream);
-}
-
 }  // namespace dfgpu
 
 // Reads and clears the device-side status words the bounded waits write (0 = none).
@@ -1158,7 +1092,7 @@ int launch_matmul_umma(const dfgpu_matmul_params& p, void* const* tensors, int k
 extern "C" int dfgpu_device_status(int* status) {
     using namespace dfgpu;
     if (!status) return fail(kInvalidArgument, "device_status: null pointer");
-    int gemm = 0, sdpa = 0, decode = 0, mxf8 = 0, pair = 0;
+    int gemm = 0, sdpa = 0, decode = 0, tiles = 0, pair = 0;
     int code = read_and_clear_device_status(&gemm);
     if (code) return code;
     code = conv_pair_device_status(&pair);
@@ -1168,9 +1102,9 @@ extern "C" int dfgpu_device_status(int* status) {
     code = conv_f32_device_status(&cluster);
     if (code) return code;
     if (!gemm) gemm = cluster;
-    code = mxf8_device_status(&mxf8);
+    code = matmul_tiles_device_status(&tiles);
     if (code) return code;
-    if (!gemm) gemm = mxf8;
+    if (!gemm) gemm = tiles;
     code = sdpa_umma_device_status(&sdpa);
     if (code) return code;
     code = decode_umma_device_status(&decode);

@@ -1,0 +1,922 @@
+// Matrix products on the 5th-generation tensor cores for every extent: C = steps(A B), A [M, K] with K contiguous, B with
+// K or N contiguous, 16-bit floats (bf16, f16), FP8 codes (MATMUL_FP8) or FP8 codes with E8M0 block scales (MXFP8).
+//
+// Extents are free because the copies are: TMA fills what lies outside a matrix with zeros and clips what would be stored
+// there, so a tile may hang over any edge. Only the rows' starts have to fall on 16-byte boundaries.
+//
+// Three shapes of work, one kernel body:
+//   CG = 2      two SMs (a cluster) on one 256 x bn tile: CTA r holds rows 128 r .. 128 r + 127 of A and half of the bn columns
+//               of B, and one thread of CTA 0 issues tcgen05.mma.cta_group::2, which reads both. Each operand byte is written
+//               to shared memory once and read once, and both go through the same 128 B per clock: a 128 x 256 x 64 step of
+//               ONE SM moves 2 x 48 KB = 768 clocks for 512 clocks of products, the pair moves 2 x 32 KB = 512 per SM.
+//   CG = 1      one SM per 128 x bn tile, for problems whose tiles are few.
+//   splits > 1  CG = 1, and a cluster of `splits` CTAs shares out the K blocks of ONE tile; the partial tiles meet through
+//               distributed shared memory and are added in rank order. For products with fewer tiles than SMs.
+// bn is 64, 128, 192 or 256 at run time; choose_shape() says which shape a product takes and why.
+//
+// Warps: 0 loads (TMA), 1 issues products, 4-11 are the epilogue (two groups of four, alternating 128-byte column boxes), and
+// with block scales 2, 3, 12 and 13 gather them. Two accumulators in tensor memory where they fit, so that a tile's epilogue
+// runs under the next tile's products. Finished boxes leave through a swizzled staging tile by TMA; a thread's own row of
+// 64 bytes at a row's distance would jam the load/store unit.
+#include <algorithm>
+
+#include "umma.cuh"
+#include "umma_ptx.cuh"
+
+namespace dfgpu {
+namespace {
+
+constexpr int kRows = 128;            // rows of A per CTA and tile
+constexpr int kRowBytes = 128;        // one swizzled shared-memory row: 64 16-bit values or 128 codes of K
+constexpr int kABytes = kRows * kRowBytes;
+constexpr int kStageBox = 128 * 128;  // one staging tile: 128 rows x 128 bytes of C
+constexpr int kMaxStages = 12;
+constexpr int kMaxSteps = DFGPU_MAX_EPILOGUE;
+constexpr int kSmemBudget = 227 * 1024 - 1024;   // (1 KB of slack aligns the tiles)
+
+enum Kind { kSixteen = 0, kCodes = 1, kScaled = 2 };
+enum { kStepRelu = 1, kStepBias = 2, kStepFull = 3 };
+
+struct TileArgs {
+    int32_t m_total, n_total;
+    int32_t m_tiles, n_tiles, k_blocks;
+    int32_t bn;                       // columns of a tile
+    int32_t splits, k_per_split;
+    int32_t stages, stage_bytes, accumulators;
+    int32_t load_bytes;               // what one CTA's copies of a stage write
+    int32_t b_boxes, b_box_bytes, b_box_columns;   // B of one CTA and stage
+    int32_t b_mn_major;
+    uint32_t idesc;
+    int32_t staging_offset, barrier_offset;
+    void* out;
+    int64_t out_ld;
+    int32_t out_dtype;
+    int32_t tma_store;                // C's rows start on 16-byte boundaries
+    int32_t step_count;
+    int32_t step_kind[kMaxSteps], step_dtype[kMaxSteps], step_vector[kMaxSteps];
+    float relu_lower[kMaxSteps], relu_upper[kMaxSteps], relu_slope[kMaxSteps];
+    const void* step_data[kMaxSteps];
+    int64_t step_ld[kMaxSteps];
+    // MATMUL_FP8: value = acc * *descale_a * *descale_b, *amax_bits = max |value| (bits of the non-negative f32, NaN
+    // canonical), C = value * *scale_c
+    const float* descale_a;
+    const float* descale_b;
+    const float* scale_c;
+    unsigned int* amax_bits;
+    // block scales: [M, K/32] and [K/32, N], one byte each
+    const uint8_t* sfa;
+    const uint8_t* sfb;
+    int64_t sfa_ld, sfb_ld;
+    int32_t scale_blocks, sfa_words;  // K / 32; sfa rows may be read as aligned words
+};
+
+// ---- cluster and pair forms of the PTX wrappers ------------------------------------------------------------
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t address_in(uint32_t own_address, uint32_t rank) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(own_address), "r"(rank));
+    return remote;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_address) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
+}
+__device__ __forceinline__ float4 load_from_rank(uint32_t cluster_address) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_address) : "memory");
+    return v;
+}
+template <int CG>
+__device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+    if constexpr (CG == 2)
+        asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                     ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar) : "memory");
+    else tma_load_2d(dst, map, c0, c1, bar);
+}
+// Arrival on a barrier of this CTA, and with CG = 2 on the same barrier of the other one.
+template <int CG>
+__device__ __forceinline__ void commit_to_all(uint32_t bar) {
+    if constexpr (CG == 2) {
+        const uint16_t both = 3;
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(both) : "memory");
+    } else {
+        umma_commit(bar);
+    }
+}
+template <int CG>
+__device__ __forceinline__ void alloc_columns(uint32_t slot) {
+    if constexpr (CG == 2) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+        tmem_alloc(slot, 512);
+        tmem_relinquish();
+    }
+}
+template <int CG>
+__device__ __forceinline__ void free_columns(uint32_t base) {
+    if constexpr (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(512u) : "memory");
+    else tmem_dealloc(base, 512);
+}
+template <int KIND, int CG>
+__device__ __forceinline__ void product(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate, uint32_t sfa, uint32_t sfb) {
+#define DFGPU_MMA(FORM)                                                                                                   \
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma." FORM " [%0], %1, %2, %3, p;\n\t}"          \
+                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory")
+    if constexpr (KIND == kSixteen && CG == 1) DFGPU_MMA("cta_group::1.kind::f16");
+    if constexpr (KIND == kSixteen && CG == 2) DFGPU_MMA("cta_group::2.kind::f16");
+    if constexpr (KIND == kCodes && CG == 1) DFGPU_MMA("cta_group::1.kind::f8f6f4");
+    if constexpr (KIND == kCodes && CG == 2) DFGPU_MMA("cta_group::2.kind::f8f6f4");
+#undef DFGPU_MMA
+#define DFGPU_MMA(FORM)                                                                                                   \
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma." FORM ".kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}" \
+                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb) : "memory")
+    if constexpr (KIND == kScaled && CG == 1) DFGPU_MMA("cta_group::1");
+    if constexpr (KIND == kScaled && CG == 2) DFGPU_MMA("cta_group::2");
+#undef DFGPU_MMA
+}
+// 32 rows x 16 bytes of shared memory -> 4 columns of tensor memory, replicated to the four lane quarters.
+template <int CG>
+__device__ __forceinline__ void copy_scales(uint32_t tmem_dst, uint32_t address) {
+    // an unswizzled K-major block: 8-row groups 128 bytes apart
+    const uint64_t desc = static_cast<uint64_t>((address & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(128u >> 4) << 32) | (1ull << 46);
+    if constexpr (CG == 2) asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem_dst), "l"(desc) : "memory");
+    else asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem_dst), "l"(desc) : "memory");
+}
+
+// ---- the fused steps on values of one row of C ---------------------------------------------------------------
+
+__device__ __forceinline__ void widen_pair(uint32_t word, int dtype, float& lo, float& hi) {
+    if (dtype == DFGPU_BF16) {
+        lo = __uint_as_float(word << 16);
+        hi = __uint_as_float(word & 0xffff0000u);
+    } else {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&word));
+        lo = f.x;
+        hi = f.y;
+    }
+}
+// v[i] += operand[first + i] for COUNT neighbouring columns, as far as the operand's row reaches (`live` of them).
+template <int COUNT>
+__device__ __forceinline__ void add_operand(float (&v)[COUNT], const void* data, int dtype, int64_t first, int live, bool vector) {
+    if (vector && live >= COUNT) {
+        if (dtype == DFGPU_F32) {
+            const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(data) + first);
+#pragma unroll
+            for (int j = 0; j < COUNT / 4; ++j) {
+                const float4 q = __ldg(p + j);
+                v[4 * j] = __fadd_rn(v[4 * j], q.x);
+                v[4 * j + 1] = __fadd_rn(v[4 * j + 1], q.y);
+                v[4 * j + 2] = __fadd_rn(v[4 * j + 2], q.z);
+                v[4 * j + 3] = __fadd_rn(v[4 * j + 3], q.w);
+            }
+        } else {
+            const uint2* p = reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(data) + first);
+#pragma unroll
+            for (int j = 0; j < COUNT / 4; ++j) {
+                const uint2 q = __ldg(p + j);
+                float f[4];
+                widen_pair(q.x, dtype, f[0], f[1]);
+                widen_pair(q.y, dtype, f[2], f[3]);
+#pragma unroll
+                for (int t = 0; t < 4; ++t) v[4 * j + t] = __fadd_rn(v[4 * j + t], f[t]);
+            }
+        }
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < COUNT; ++i)
+        if (i < live) v[i] = __fadd_rn(v[i], load_as_f32(data, dtype, first + i));
+}
+
+struct Scalars {
+    bool on;
+    float descale_a, descale_b, scale_c;
+    float magnitude;   // largest |value| of this thread so far (NaN sticks)
+};
+__device__ __forceinline__ Scalars load_scalars(const TileArgs& args) {
+    Scalars s{};
+    if (args.descale_a != nullptr) {
+        s.on = true;
+        s.descale_a = *args.descale_a;
+        s.descale_b = *args.descale_b;
+        s.scale_c = *args.scale_c;
+    }
+    return s;
+}
+__device__ __forceinline__ void fold_amax(const TileArgs& args, const Scalars& s, int lane, bool ok) {
+    if (!s.on) return;
+    unsigned int bits = s.magnitude != s.magnitude ? 0x7fc00000u : __float_as_uint(s.magnitude);
+    bits = __reduce_max_sync(0xffffffffu, bits);
+    if (lane == 0 && bits != 0u && ok) atomicMax(args.amax_bits, bits);
+}
+
+// COUNT neighbouring columns of one row: fused steps, then MATMUL_FP8's scalars. `row_live`: the row exists.
+template <int COUNT>
+__device__ __forceinline__ void apply_steps(const TileArgs& args, float (&v)[COUNT], int row, int col0, bool row_live, Scalars& scalars) {
+    const int live = args.n_total - col0;
+    for (int s = 0; s < args.step_count; ++s) {
+        const int kind = args.step_kind[s];
+        if (kind == kStepRelu) {
+            const float lower = args.relu_lower[s], upper = args.relu_upper[s], slope = args.relu_slope[s];
+#pragma unroll
+            for (int e = 0; e < COUNT; ++e) v[e] = relu_fast(v[e], lower, upper, slope);
+        } else if (kind == kStepBias || row_live) {
+            add_operand<COUNT>(v, args.step_data[s], args.step_dtype[s], (kind == kStepBias ? 0 : row * args.step_ld[s]) + col0, live, args.step_vector[s] != 0);
+        }
+    }
+    if (scalars.on) {
+        float top = scalars.magnitude;
+#pragma unroll
+        for (int e = 0; e < COUNT; ++e) {
+            // (+0.0 first: the reference's sum starts from +0.0 and so is never -0.0, the tensor core's can be)
+            const float value = __fmul_rn(__fmul_rn(__fadd_rn(v[e], 0.0f), scalars.descale_a), scalars.descale_b);
+            if (row_live && e < live) top = maximum_nan(top, fabsf(value));
+            v[e] = __fmul_rn(value, scalars.scale_c);
+        }
+        scalars.magnitude = top;
+    }
+}
+
+__device__ __forceinline__ uint32_t narrow_pair(float lo, float hi, int dtype) {
+    if (dtype == DFGPU_BF16) {
+        const __nv_bfloat162 pair = __floats2bfloat162_rn(lo, hi);
+        return *reinterpret_cast<const uint32_t*>(&pair);
+    }
+    const __half2 pair = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&pair);
+}
+__device__ __forceinline__ uint32_t encode_four_e4m3(const float* f) {
+    uint32_t lo = encode_e4m3_pair(f[0], f[1]), hi = encode_e4m3_pair(f[2], f[3]);
+    // NaN -> 0x7f whatever its sign (the hardware convert keeps the sign bit)
+    if (f[0] != f[0]) lo = (lo & 0xff00u) | 0x7fu;
+    if (f[1] != f[1]) lo = (lo & 0x00ffu) | 0x7f00u;
+    if (f[2] != f[2]) hi = (hi & 0xff00u) | 0x7fu;
+    if (f[3] != f[3]) hi = (hi & 0x00ffu) | 0x7f00u;
+    return lo | (hi << 16);
+}
+
+// Four neighbouring columns straight to C (the split form: neighbouring threads hold neighbouring columns).
+__device__ __forceinline__ void store_four(const TileArgs& args, const float (&v)[4], int row, int col) {
+    const int64_t at = row * args.out_ld + col;
+    const int live = args.n_total - col;
+    if (live >= 4 && args.tma_store) {
+        if (args.out_dtype == DFGPU_F32) *reinterpret_cast<float4*>(static_cast<float*>(args.out) + at) = make_float4(v[0], v[1], v[2], v[3]);
+        else if (args.out_dtype == DFGPU_E4M3) *reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(args.out) + at) = encode_four_e4m3(v);
+        else *reinterpret_cast<uint2*>(static_cast<uint16_t*>(args.out) + at) = make_uint2(narrow_pair(v[0], v[1], args.out_dtype), narrow_pair(v[2], v[3], args.out_dtype));
+        return;
+    }
+    for (int i = 0; i < 4; ++i)
+        if (i < live) store_from_f32(args.out, args.out_dtype, at + i, v[i]);
+}
+
+// A wait whose phase may be completed by the other CTA's threads: acquires at cluster scope. Bounded like mbar_wait().
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    return done != 0;
+}
+__device__ __noinline__ bool mbar_wait_cluster_slow(uint32_t bar, uint32_t parity, int code) {
+    const uint64_t start = global_timer_ns();
+    for (;;) {
+        for (int spin = 0; spin < 128; ++spin)
+            if (mbar_try_wait_cluster(bar, parity)) return true;
+        if (global_timer_ns() - start > 2000000000ull) {
+            atomicCAS(&g_device_status, 0, code);
+            return false;
+        }
+    }
+}
+template <bool CLUSTER>
+__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, int code) {
+    if constexpr (CLUSTER) {
+#pragma unroll 1
+        for (int spin = 0; spin < 64; ++spin)
+            if (__all_sync(0xffffffffu, mbar_try_wait_cluster(bar, parity))) return true;
+        return __all_sync(0xffffffffu, mbar_wait_cluster_slow(bar, parity, code)) != 0;
+    } else {
+        return mbar_wait_warp(bar, parity, code);
+    }
+}
+
+template <int KIND>
+constexpr int thread_count() { return KIND == kScaled ? 448 : 384; }
+
+// The four rows-of-32 words of scales of one 128-row (or 128-column) chunk, as tcgen05.cp wants them: byte j of a word is
+// the scale of K block j. Blocks, rows and columns past the end count as 2^0 (their codes are zeros).
+__device__ __forceinline__ void gather_row_scales(const TileArgs& args, int row0, int kb, int lane, uint32_t (&words)[4]) {
+    const int first = kb * 4, live = args.scale_blocks - first;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        const int row = row0 + g * 32 + lane;
+        words[g] = 0x7f7f7f7fu;
+        if (row >= args.m_total) continue;
+        const uint8_t* p = args.sfa + row * args.sfa_ld + first;
+        if (args.sfa_words && live >= 4) {
+            words[g] = __ldg(reinterpret_cast<const uint32_t*>(p));
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (j < live) words[g] = (words[g] & ~(0xffu << (8 * j))) | (static_cast<uint32_t>(__ldg(p + j)) << (8 * j));
+        }
+    }
+}
+__device__ __forceinline__ void gather_column_scales(const TileArgs& args, int col0, int kb, int lane, uint32_t (&words)[4]) {
+    const int first = kb * 4, live = args.scale_blocks - first;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        const int col = col0 + g * 32 + lane;
+        words[g] = 0x7f7f7f7fu;
+        if (col >= args.n_total) continue;
+        const uint8_t* p = args.sfb + first * args.sfb_ld + col;
+        uint32_t byte[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) byte[j] = j < live ? __ldg(p + j * args.sfb_ld) : 0x7fu;
+        words[g] = byte[0] | (byte[1] << 8) | (byte[2] << 16) | (byte[3] << 24);
+    }
+}
+
+template <int KIND, int CG>
+__global__ void __launch_bounds__(thread_count<KIND>(), 1)
+umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c,
+                   const __grid_constant__ TileArgs args) {
+    constexpr bool kClusterWaits = KIND == kScaled && CG == 2;
+    constexpr int kCode = KIND == kSixteen ? 0 : (KIND == kCodes ? 20 : 40);
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* generic_base = smem_raw + (smem_base - smem_u32(smem_raw));
+    const uint32_t bar_base = smem_base + args.barrier_offset;
+    auto full_bar = [&](int s) { return bar_base + 8u * s; };
+    auto empty_bar = [&](int s) { return bar_base + 8u * (kMaxStages + s); };
+    auto acc_full = [&](int a) { return bar_base + 8u * (2 * kMaxStages + a); };
+    auto acc_empty = [&](int a) { return bar_base + 8u * (2 * kMaxStages + 2 + a); };
+    const uint32_t tmem_slot = bar_base + 8u * (2 * kMaxStages + 4);
+    volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(generic_base + args.barrier_offset + 8 * (2 * kMaxStages + 4));
+
+    const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
+    const bool leader = elect_one();
+    const bool split = CG == 1 && args.splits > 1;
+    const int rank = CG == 2 || split ? static_cast<int>(cluster_rank()) : 0;
+    const int group = CG == 2 ? 2 : args.splits;            // CTAs that share a tile
+    const int first_tile = static_cast<int>(blockIdx.x) / group, tile_step = static_cast<int>(gridDim.x) / group;
+    const int tiles = args.m_tiles * args.n_tiles;
+    const int kb_begin = split ? rank * args.k_per_split : 0;
+    const int kb_end = split ? min(args.k_blocks, kb_begin + args.k_per_split) : args.k_blocks;
+    const int bn = args.bn;
+
+    if (threadIdx.x == 0) {
+        prefetch_tensormap(&map_a);
+        prefetch_tensormap(&map_b);
+        if (args.tma_store) prefetch_tensormap(&map_c);
+    }
+    if (warp == 0 && leader) {
+        for (int s = 0; s < args.stages; ++s) {
+            mbar_init(full_bar(s), KIND == kScaled ? 1 + CG : 1);   // the byte count, and one scale warp of each CTA
+            mbar_init(empty_bar(s), 1);
+        }
+        for (int a = 0; a < 2; ++a) {
+            mbar_init(acc_full(a), 1);
+            mbar_init(acc_empty(a), 8 * CG);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        alloc_columns<CG>(tmem_slot);
+        tc_fence_before();
+    }
+    __syncthreads();
+    if (CG == 2) cluster_sync_all();   // both CTAs' barriers exist before either touches the other's
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot_ptr;
+    chain_wait();
+    chain_release();
+
+    if (warp == 0) {
+        // ---- loader: this CTA's rows of A and share of B; with CG = 2 the bytes are counted on CTA 0's barrier ----
+        const uint32_t counted_on = CG == 2 ? address_in(bar_base, 0) : bar_base;
+        int stage = 0;
+        uint32_t phase = 1;
+        bool ok = true;
+        for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
+            const int m_tile = tile % args.m_tiles, n_tile = tile / args.m_tiles;
+            const int row0 = (m_tile * CG + (CG == 2 ? rank : 0)) * kRows, col0 = n_tile * bn + (CG == 2 ? rank * (bn / 2) : 0);
+            for (int kb = kb_begin; kb < kb_end; ++kb) {
+                ok = mbar_wait_warp(empty_bar(stage), phase, 501 + kCode);
+                if (!ok) break;
+                if (leader) {
+                    const uint32_t a_dst = smem_base + stage * args.stage_bytes, b_dst = a_dst + kABytes;
+                    const uint32_t bar = counted_on + 8u * stage;
+                    constexpr int kPerRow = KIND == kSixteen ? 64 : 128;   // elements of K per block
+                    if (CG == 1 || rank == 0) mbar_expect_tx(full_bar(stage), CG * args.load_bytes);
+                    load_tile<CG>(a_dst, &map_a, kb * kPerRow, row0, bar);
+                    for (int j = 0; j < args.b_boxes; ++j) {
+                        if (args.b_mn_major) load_tile<CG>(b_dst + j * args.b_box_bytes, &map_b, col0 + j * args.b_box_columns, kb * kPerRow, bar);
+                        else load_tile<CG>(b_dst + j * args.b_box_bytes, &map_b, kb * kPerRow, col0 + j * args.b_box_columns, bar);
+                    }
+                }
+                __syncwarp();
+                if (++stage == args.stages) { stage = 0; phase ^= 1; }
+            }
+        }
+    } else if (warp == 1) {
+        // ---- issuing warp (of CTA 0 in a pair) ----
+        if (CG == 1 || rank == 0) {
+            const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+            const uint32_t b_lbo = args.b_mn_major ? (KIND == kSixteen ? 64 * kRowBytes : 128 * kRowBytes) : 16;
+            const uint32_t b_step = args.b_mn_major ? (KIND == kSixteen ? 2048u >> 4 : 4096u >> 4) : 32u >> 4;
+            const int scale_columns = args.accumulators * bn;   // where the scales' tensor memory starts
+            int stage = 0, local = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int tile = first_tile; tile < tiles; tile += tile_step, ++local) {
+                const int acc = args.accumulators == 2 ? local & 1 : 0, use = args.accumulators == 2 ? local >> 1 : local;
+                if (ok) ok = wait_warp<CG == 2>(acc_empty(acc), (use & 1) ^ 1, 502 + kCode);
+                tc_fence_after();
+                const uint32_t d = tmem_u + acc * bn;
+                for (int kb = kb_begin; kb < kb_end && ok; ++kb) {
+                    ok = wait_warp<kClusterWaits>(full_bar(stage), phase, 503 + kCode);
+                    if (!ok) break;   // (operands by TMA, scales by generic stores + fence.proxy.async: no tcgen05 fence needed)
+                    if (leader) {
+                        const uint32_t a_src = smem_base + stage * args.stage_bytes, b_src = a_src + kABytes;
+                        const uint32_t a_lo = smem_desc_lo(a_src, 16), b_lo = smem_desc_lo(b_src, b_lbo);
+                        uint32_t sf = 0;
+                        if constexpr (KIND == kScaled) {
+                            const uint32_t scales = b_src + (CG == 2 ? bn / 2 : bn) * kRowBytes;
+                            sf = tmem_u + scale_columns + (stage & 1) * 16;   // A's at +0..3, B's at +4..11
+                            copy_scales<CG>(sf, scales);
+                            copy_scales<CG>(sf + 4, scales + 512);
+                            if (bn > 128) copy_scales<CG>(sf + 8, scales + 1024);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            uint32_t idesc = args.idesc;
+                            if constexpr (KIND == kScaled) idesc |= (static_cast<uint32_t>(j) << 29) | (static_cast<uint32_t>(j) << 4);   // the K block's byte of the scale words
+                            product<KIND, CG>(d, desc_words(a_lo + ((j * 32) >> 4), smem_desc_hi(1024)), desc_words(b_lo + j * b_step, smem_desc_hi(1024)), idesc,
+                                              kb != kb_begin || j != 0 ? 1u : 0u, sf, sf + 4);
+                        }
+                        commit_to_all<CG>(empty_bar(stage));
+                    }
+                    __syncwarp();
+                    if (++stage == args.stages) { stage = 0; phase ^= 1; }
+                }
+                if (leader) commit_to_all<CG>(acc_full(acc));   // arrives even after a failed wait, so that no epilogue hangs
+                __syncwarp();
+            }
+        }
+    } else if (warp >= 4 && warp < 12) {
+        // ---- epilogue: this CTA's 128 rows, group g the boxes g, g + 2, ... of 128 bytes of C each ----
+        const int quadrant = warp & 3, g = (warp - 4) >> 2, row = quadrant * 32 + lane;
+        const uint32_t lane_base = static_cast<uint32_t>(quadrant * 32) << 16;
+        bool ok = true;
+        if (split) {
+            // park the f32 partial tile where the operands were: rows of bn floats, 16-byte units swizzled by the row
+            ok = mbar_wait(acc_full(0), 0, 504 + kCode);
+            tc_fence_after();
+            uint8_t* parked = generic_base + row * bn * 4;
+            for (int c = g; c < bn / 32; c += 2) {
+                uint32_t raw[32];
+                tmem_load_32(tmem_base + lane_base + c * 32, raw);
+                tmem_load_wait();
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    *reinterpret_cast<uint4*>(parked + ((c * 8 + (j ^ (row & 7))) << 4)) = make_uint4(raw[4 * j], raw[4 * j + 1], raw[4 * j + 2], raw[4 * j + 3]);
+            }
+            tc_fence_before();
+        } else {
+            const uint32_t leader_bars = CG == 2 ? address_in(bar_base, 0) : bar_base;
+            uint8_t* staging = generic_base + args.staging_offset + g * kStageBox;
+            const int box_columns = !args.tma_store || args.out_dtype == DFGPU_F32 ? 32 : (args.out_dtype == DFGPU_E4M3 ? 128 : 64);
+            Scalars scalars = load_scalars(args);
+            bool stored = false;   // (this group has a store in flight)
+            int local = 0;
+            for (int tile = first_tile; tile < tiles; tile += tile_step, ++local) {
+                const int acc = args.accumulators == 2 ? local & 1 : 0, use = args.accumulators == 2 ? local >> 1 : local;
+                const int m_tile = tile % args.m_tiles, n_tile = tile / args.m_tiles;
+                const int row0 = (m_tile * CG + (CG == 2 ? rank : 0)) * kRows, out_row = row0 + row;
+                const bool row_live = out_row < args.m_total;
+                if (ok) ok = mbar_wait(acc_full(acc), use & 1, 505 + kCode);
+                tc_fence_after();
+                const bool healthy = ok && g_device_status == 0;
+                const uint32_t columns = tmem_base + lane_base + acc * bn;
+                for (int box = g; box < bn / box_columns; box += 2) {
+                    const int col0 = n_tile * bn + box * box_columns;
+                    if (args.tma_store && stored) {
+                        if (row == 0) tma_store_wait_read<0>();
+                        epilogue_barrier(1 + g);
+                    }
+                    for (int part = 0; part < box_columns / 32; ++part) {
+                        uint32_t raw[32];
+                        tmem_load_32(columns + box * box_columns + part * 32, raw);
+                        tmem_load_wait();
+                        float v[32];
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(raw[e]);
+                        const int col = col0 + part * 32;
+                        apply_steps<32>(args, v, out_row, col, row_live, scalars);
+                        if (args.tma_store) {
+                            uint8_t* target = staging + row * 128;
+                            if (args.out_dtype == DFGPU_F32) {
+#pragma unroll
+                                for (int j = 0; j < 8; ++j)
+                                    *reinterpret_cast<float4*>(target + ((j ^ (row & 7)) << 4)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                            } else if (args.out_dtype == DFGPU_E4M3) {
+#pragma unroll
+                                for (int j = 0; j < 2; ++j)
+                                    *reinterpret_cast<uint4*>(target + (((part * 2 + j) ^ (row & 7)) << 4)) =
+                                        make_uint4(encode_four_e4m3(v + 16 * j), encode_four_e4m3(v + 16 * j + 4), encode_four_e4m3(v + 16 * j + 8), encode_four_e4m3(v + 16 * j + 12));
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < 4; ++j)
+                                    *reinterpret_cast<uint4*>(target + (((part * 4 + j) ^ (row & 7)) << 4)) =
+                                        make_uint4(narrow_pair(v[8 * j], v[8 * j + 1], args.out_dtype), narrow_pair(v[8 * j + 2], v[8 * j + 3], args.out_dtype),
+                                                   narrow_pair(v[8 * j + 4], v[8 * j + 5], args.out_dtype), narrow_pair(v[8 * j + 6], v[8 * j + 7], args.out_dtype));
+                            }
+                        } else if (row_live && healthy) {
+                            const int64_t at = out_row * args.out_ld + col;
+#pragma unroll
+                            for (int e = 0; e < 32; ++e)
+                                if (col + e < args.n_total) store_from_f32(args.out, args.out_dtype, at + e, v[e]);
+                        }
+                    }
+                    if (args.tma_store) {
+                        fence_async_shared();
+                        epilogue_barrier(1 + g);
+                        if (row == 0) {
+                            if (healthy && row0 < args.m_total && col0 < args.n_total) tma_store_2d(&map_c, smem_base + args.staging_offset + g * kStageBox, col0, row0);
+                            tma_store_commit();
+                        }
+                        stored = true;
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if (CG == 2) mbar_arrive_cluster(leader_bars + 8u * (2 * kMaxStages + 2 + acc));
+                    else mbar_arrive(acc_empty(acc));
+                }
+            }
+            if (args.tma_store && row == 0) tma_store_wait_all();
+            __syncwarp();
+            fold_amax(args, scalars, lane, ok);
+        }
+    } else if (KIND == kScaled) {
+        // ---- scale loaders: warp i of the four fills the slots of every fourth block ----
+        const int me = warp < 4 ? warp - 2 : warp - 10;
+        const uint32_t counted_on = CG == 2 ? address_in(bar_base, 0) : bar_base;
+        int stage = 0, block = 0;
+        uint32_t phase = 1;
+        bool ok = true;
+        for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
+            const int m_tile = tile % args.m_tiles, n_tile = tile / args.m_tiles;
+            const int row0 = (m_tile * CG + (CG == 2 ? rank : 0)) * kRows;
+            for (int kb = kb_begin; kb < kb_end; ++kb, ++block) {
+                const int slot = stage;
+                const uint32_t slot_phase = phase;
+                if (++stage == args.stages) { stage = 0; phase ^= 1; }
+                if ((block & 3) != me) continue;
+                // the global loads do not wait for the slot
+                uint32_t a_words[4], b_words[2][4];
+                gather_row_scales(args, row0, kb, lane, a_words);
+                gather_column_scales(args, n_tile * bn, kb, lane, b_words[0]);
+                if (bn > 128) gather_column_scales(args, n_tile * bn + 128, kb, lane, b_words[1]);
+                ok = mbar_wait_warp(empty_bar(slot), slot_phase, 506 + kCode);
+                if (!ok) break;
+                uint8_t* scales = generic_base + slot * args.stage_bytes + kABytes + (CG == 2 ? bn / 2 : bn) * kRowBytes + lane * 16;
+                *reinterpret_cast<uint4*>(scales) = make_uint4(a_words[0], a_words[1], a_words[2], a_words[3]);
+                *reinterpret_cast<uint4*>(scales + 512) = make_uint4(b_words[0][0], b_words[0][1], b_words[0][2], b_words[0][3]);
+                if (bn > 128) *reinterpret_cast<uint4*>(scales + 1024) = make_uint4(b_words[1][0], b_words[1][1], b_words[1][2], b_words[1][3]);
+                fence_async_shared();
+                __syncwarp();
+                if (leader) {
+                    if (CG == 2) mbar_arrive_cluster(counted_on + 8u * slot);
+                    else mbar_arrive(full_bar(slot));
+                }
+            }
+        }
+    }
+
+    if (split) {
+        // ---- the cluster's partial tiles: every CTA adds its share of the live rows over all ranks, in rank order ----
+        __syncthreads();
+        cluster_sync_all();
+        const int m_tile = first_tile % args.m_tiles, n_tile = first_tile / args.m_tiles;
+        const int row0 = m_tile * kRows, live_rows = min(kRows, args.m_total - row0);
+        const int share = (live_rows + args.splits - 1) / args.splits, begin = rank * share, end = min(live_rows, begin + share);
+        const int quads = bn / 4;
+        Scalars scalars = load_scalars(args);
+        const bool healthy = g_device_status == 0;
+        for (int item = threadIdx.x; item < (end - begin) * quads; item += blockDim.x) {
+            const int row = begin + item / quads, unit = item % quads;
+            const int col = n_tile * bn + unit * 4;
+            if (col >= args.n_total) continue;
+            const uint32_t at = smem_base + row * bn * 4 + (((unit & ~7) | ((unit ^ row) & 7)) << 4);
+            constexpr int kMost = 8;
+            float4 part[kMost];
+#pragma unroll
+            for (int z = 0; z < kMost; ++z)   // every load in flight before the first sum
+                if (z < args.splits) part[z] = load_from_rank(address_in(at, z));
+            float v[4] = {part[0].x, part[0].y, part[0].z, part[0].w};
+#pragma unroll
+            for (int z = 1; z < kMost; ++z) {
+                if (z >= args.splits) break;
+                v[0] = __fadd_rn(v[0], part[z].x);
+                v[1] = __fadd_rn(v[1], part[z].y);
+                v[2] = __fadd_rn(v[2], part[z].z);
+                v[3] = __fadd_rn(v[3], part[z].w);
+            }
+            apply_steps<4>(args, v, row0 + row, col, true, scalars);
+            if (healthy) store_four(args, v, row0 + row, col);
+        }
+        __syncwarp();
+        fold_amax(args, scalars, lane, healthy);
+        cluster_sync_all();   // no CTA leaves while another still reads its partial tile
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (CG == 2) cluster_sync_all();   // ... or may still signal its barriers or read its operands
+    if (warp == 1) {
+        tc_fence_after();
+        free_columns<CG>(tmem_base);
+    }
+}
+
+// ---- host --------------------------------------------------------------------------------------------------
+
+bool on16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+int encode_map(CUtensorMap* map, CUtensorMapDataType type, const void* base, int64_t inner, int64_t outer, int64_t stride_bytes, uint32_t box_inner,
+               uint32_t box_outer, const char* what) {
+    EncodeTiled encode = encode_tiled();
+    if (!encode) return fail(kExecutionFailed, "%s: cuTensorMapEncodeTiled is unavailable", what);
+    cuuint64_t dims[2] = {static_cast<cuuint64_t>(inner), static_cast<cuuint64_t>(outer)}, strides[1] = {static_cast<cuuint64_t>(stride_bytes)};
+    cuuint32_t box[2] = {box_inner, box_outer}, element_strides[2] = {1, 1};
+    CUresult result = encode(map, type, 2, const_cast<void*>(base), dims, strides, box, element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (result != CUDA_SUCCESS) return fail(kExecutionFailed, "%s: tensor map encode failed (CUresult %d)", what, static_cast<int>(result));
+    return kOk;
+}
+
+// One product as the kernel sees it; the descriptors alone decide everything but the pointers.
+struct Problem {
+    int kind;
+    int64_t M, N, K;
+    int64_t a_ld, b_ld, c_ld;
+    bool b_mn_major;
+    int in_bytes, out_bytes, out_dtype;
+};
+
+bool row_ok(int64_t ld, int64_t extent, int bytes) { return ld >= extent && (ld * bytes) % 16 == 0 && ld * bytes < (1ll << 40); }
+
+// A and B must be readable by TMA: contiguous rows that start on 16-byte boundaries (a single row has no stride to mind).
+bool describe(const dfgpu_tensor& a, const dfgpu_tensor& b, const dfgpu_tensor& c, int kind, Problem& p) {
+    const int rank = c.rank;
+    if (rank < 2 || a.rank != rank || b.rank != rank) return false;
+    for (int i = 0; i < rank - 2; ++i)
+        if (a.dim[i] != 1 || b.dim[i] != 1 || c.dim[i] != 1) return false;
+    p.kind = kind;
+    p.M = c.dim[rank - 2];
+    p.N = c.dim[rank - 1];
+    p.K = a.dim[rank - 1];
+    if (a.dim[rank - 2] != p.M || b.dim[rank - 2] != p.K || b.dim[rank - 1] != p.N) return false;
+    if (p.M < 1 || p.N < 1 || p.K < 1 || p.M > (1ll << 28) || p.N > (1ll << 28) || p.K > (1ll << 28)) return false;
+    p.in_bytes = kind == kSixteen ? 2 : 1;
+    p.out_dtype = c.dtype;
+    p.out_bytes = dtype_bytes(c.dtype);
+    p.a_ld = a.stride[rank - 2];
+    if (p.M == 1) p.a_ld = (p.K * p.in_bytes + 15) / 16 * 16 / p.in_bytes;
+    if (a.stride[rank - 1] != 1 || !row_ok(p.a_ld, p.K, p.in_bytes)) return false;
+    const bool k_major = b.stride[rank - 2] == 1 && row_ok(b.stride[rank - 1], p.K, p.in_bytes);
+    p.b_mn_major = !k_major;
+    p.b_ld = k_major ? b.stride[rank - 1] : b.stride[rank - 2];
+    if (!k_major && (b.stride[rank - 1] != 1 || !row_ok(p.b_ld, p.N, p.in_bytes))) return false;
+    p.c_ld = c.stride[rank - 2];
+    return c.stride[rank - 1] == 1 && p.c_ld >= p.N;
+}
+
+struct Shape {
+    int cg, bn, splits, k_per_split;
+    int64_t tiles;
+    double clocks;
+};
+
+// The shape with the fewest estimated clocks. One K block of a CTA costs the longest of
+//   products       2 bn clocks (128 rows per SM, 16-bit and FP8 alike: a block is 128 bytes of K)
+//   shared memory  every operand byte written and read once at 128 B per clock: 2 (rows of A + columns of B)
+//   L2             the same bytes at about 48 per clock and SM when all SMs fetch
+// and a round over the SMs costs its blocks, a fill of ~2000 clocks and the last tile's epilogue. Splitting K divides the
+// blocks and adds ~2500 clocks of exchange; clusters of 4 and 8 leave some SMs of a GPC without a place.
+Shape choose_shape(const Problem& p) {
+    const int64_t blocks = (p.K * p.in_bytes + kRowBytes - 1) / kRowBytes;
+    const int sms = 148;   // (a function of the shape alone: the count this library is built for)
+    Shape best{0, 0, 0, 0, 0, 0.0};
+    for (int cg = 1; cg <= 2; ++cg)
+        for (int bn = 64; bn <= 256; bn += 64) {
+            const int chunk = p.kind == kSixteen ? 64 : 128;   // columns of one N-major copy
+            if (p.b_mn_major && (bn / cg) % chunk != 0) continue;
+            if (p.out_dtype == DFGPU_E4M3 && bn % 128 != 0) continue;   // (whole 128-byte boxes)
+            if (cg == 2 && bn < 128) continue;
+            if (bn > chunk && bn >= 2 * ((p.N + 63) / 64 * 64)) continue;  // (half the tile would be empty)
+            const int64_t m_tiles = (p.M + kRows * cg - 1) / (kRows * cg), n_tiles = (p.N + bn - 1) / bn, tiles = m_tiles * n_tiles;
+            const double rows = m_tiles == 1 && cg == 1 ? static_cast<double>(std::min<int64_t>(kRows, (p.M + 7) / 8 * 8)) : kRows;
+            for (int splits = 1; splits <= (cg == 1 ? 8 : 1); splits *= 2) {
+                if (splits > 1 && (bn > 128 || splits > blocks || tiles * splits > sms)) break;
+                const int64_t k_per_split = (blocks + splits - 1) / splits;
+                if (splits > 1 && k_per_split * (splits - 1) >= blocks) continue;   // (no CTA without a block)
+                const int64_t slots = splits == 8 ? 16 : (splits == 4 ? 35 : sms / (cg * splits));
+                const double rounds = static_cast<double>((tiles + slots - 1) / slots);
+                const double block = std::max({2.0 * bn, 2.0 * (rows + bn / cg), (rows + bn / cg) * kRowBytes / 48.0});
+                const double clocks = rounds * (k_per_split * block + (p.kind == kScaled && bn == 256 ? 1500.0 : 0.0)) + 2000.0 + bn * 6.0 + (splits > 1 ? 2500.0 : 0.0) + (cg == 2 ? 500.0 : 0.0);
+                if (best.cg == 0 || clocks < best.clocks) best = Shape{cg, bn, splits, static_cast<int>(k_per_split), tiles, clocks};
+            }
+        }
+    return best;
+}
+
+template <int KIND, int CG>
+int launch_kernel(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_c, const TileArgs& args, int grid, int dynamic, cudaStream_t stream, const char* what) {
+    cudaError_t error = cudaFuncSetAttribute(umma_matmul_kernel<KIND, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, dynamic);
+    if (error != cudaSuccess) return fail(kExecutionFailed, "%s: cannot reserve %d bytes of shared memory: %s", what, dynamic, cudaGetErrorString(error));
+    const unsigned cluster = CG == 2 ? 2u : (args.splits > 1 ? static_cast<unsigned>(args.splits) : 0u);
+    error = launch_chained_cluster(umma_matmul_kernel<KIND, CG>, dim3(static_cast<unsigned>(grid)), dim3(thread_count<KIND>()), cluster, static_cast<size_t>(dynamic), stream,
+                                   map_a, map_b, map_c, args);
+    if (error != cudaSuccess) return fail(kExecutionFailed, "%s: launch failed: %s", what, cudaGetErrorString(error));
+    return check_launch(what);
+}
+
+// Everything but the epilogue's operands and the operand formats, which the callers have put into `args`.
+int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* b, void* c, cudaStream_t stream, const char* what) {
+    const Shape shape = choose_shape(p);
+    const int chunk = p.kind == kSixteen ? 64 : 128;
+    args.m_total = static_cast<int>(p.M);
+    args.n_total = static_cast<int>(p.N);
+    args.bn = shape.bn;
+    args.m_tiles = static_cast<int>((p.M + kRows * shape.cg - 1) / (kRows * shape.cg));
+    args.n_tiles = static_cast<int>((p.N + shape.bn - 1) / shape.bn);
+    args.k_blocks = static_cast<int>((p.K * p.in_bytes + kRowBytes - 1) / kRowBytes);
+    args.splits = shape.splits;
+    args.k_per_split = shape.k_per_split;
+    args.b_mn_major = p.b_mn_major ? 1 : 0;
+    const int columns = shape.bn / shape.cg;   // of B per CTA
+    args.b_boxes = p.b_mn_major ? columns / chunk : 1;
+    args.b_box_columns = p.b_mn_major ? chunk : columns;
+    args.b_box_bytes = (p.b_mn_major ? kRowBytes / p.in_bytes : columns) * kRowBytes;   // N-major: one row of 128 bytes per element of K
+    const int a_rows = args.m_tiles == 1 && shape.cg == 1 ? static_cast<int>(std::min<int64_t>(kRows, (p.M + 7) / 8 * 8)) : kRows;
+    args.load_bytes = (a_rows + columns) * kRowBytes;
+    args.stage_bytes = kABytes + columns * kRowBytes + (p.kind == kScaled ? 2048 : 0);
+    args.out = c;
+    args.out_ld = p.c_ld;
+    args.out_dtype = p.out_dtype;
+    args.tma_store = on16(c) && (p.c_ld * p.out_bytes) % 16 == 0 && p.out_dtype != DFGPU_E5M2 ? 1 : 0;
+    args.accumulators = 2 * shape.bn + (p.kind == kScaled ? 32 : 0) <= 512 ? 2 : 1;
+    const int staging = shape.splits > 1 || !args.tma_store ? 0 : 2 * kStageBox, barriers = (2 * kMaxStages + 5) * 8;
+    args.stages = std::min(kMaxStages, (kSmemBudget - staging - barriers) / args.stage_bytes);
+    args.staging_offset = args.stages * args.stage_bytes;
+    args.barrier_offset = args.staging_offset + staging;
+    const int dynamic = args.barrier_offset + barriers + 1024;
+    // instruction descriptor: f32 accumulators (or E8M0 scales), the operand formats the caller has set, B's major, N, M
+    args.idesc |= (p.kind == kScaled ? 1u << 23 : 1u << 4) | (static_cast<uint32_t>(args.b_mn_major) << 16) | (static_cast<uint32_t>(shape.bn >> 3) << 17) |
+                  (static_cast<uint32_t>(kRows * shape.cg >> 4) << 24);
+    const CUtensorMapDataType in_type = p.kind == kSixteen ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;   // (copied, never computed on)
+    const uint32_t per_row = kRowBytes / p.in_bytes;
+    CUtensorMap map_a, map_b, map_c{};
+    int status = encode_map(&map_a, in_type, a, p.K, p.M, p.a_ld * p.in_bytes, per_row, a_rows, what);
+    if (!status) {
+        if (p.b_mn_major) status = encode_map(&map_b, in_type, b, p.N, p.K, p.b_ld * p.in_bytes, chunk, per_row, what);
+        else status = encode_map(&map_b, in_type, b, p.K, p.N, p.b_ld * p.in_bytes, per_row, columns, what);
+    }
+    if (!status && args.tma_store) {
+        const CUtensorMapDataType out_type = p.out_dtype == DFGPU_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : (p.out_dtype == DFGPU_E4M3 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
+        status = encode_map(&map_c, out_type, c, p.N, p.M, p.c_ld * p.out_bytes, kRowBytes / p.out_bytes, kRows, what);
+    }
+    if (status) return status;
+    const int64_t groups = shape.splits > 1 ? shape.tiles : std::min<int64_t>(shape.tiles, sm_count() / shape.cg);
+    const int grid = static_cast<int>(groups * (shape.cg == 2 ? 2 : shape.splits));
+    if (p.kind == kSixteen) return shape.cg == 2 ? launch_kernel<kSixteen, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kSixteen, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
+    if (p.kind == kCodes) return shape.cg == 2 ? launch_kernel<kCodes, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kCodes, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
+    return shape.cg == 2 ? launch_kernel<kScaled, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kScaled, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
+}
+
+// The fused steps the kernel applies: ReLU, a per-column ADD operand, a full [M, N] ADD operand with contiguous columns.
+bool translate_steps(const dfgpu_matmul_params& p, void* const* tensors, TileArgs* args) {
+    if (p.epilogue_count < 0 || p.epilogue_count > kMaxSteps) return false;
+    const int rank = p.c.rank;
+    if (args) args->step_count = p.epilogue_count;
+    for (int i = 0; i < p.epilogue_count; ++i) {
+        const dfgpu_epilogue_step& step = p.epilogue[i];
+        if (step.op == DFGPU_EPI_RELU) {
+            if (args) {
+                args->step_kind[i] = kStepRelu;
+                args->relu_lower[i] = step.relu_lower;
+                args->relu_upper[i] = step.relu_upper;
+                args->relu_slope[i] = step.relu_slope;
+            }
+            continue;
+        }
+        if (step.op != DFGPU_EPI_ADD || step.operand < 0 || step.operand > 1) return false;
+        const dfgpu_tensor& t = p.extra[step.operand];
+        if (t.rank < 1 || t.rank > rank || (t.dtype != DFGPU_BF16 && t.dtype != DFGPU_F16 && t.dtype != DFGPU_F32)) return false;
+        for (int axis = 0; axis < t.rank - 2; ++axis)
+            if (t.dim[axis] != 1) return false;
+        if (t.dim[t.rank - 1] != p.c.dim[rank - 1] || (t.stride[t.rank - 1] != 1 && t.dim[t.rank - 1] != 1)) return false;
+        const bool per_column = t.rank == 1 || t.dim[t.rank - 2] == 1;
+        if (!per_column && t.dim[t.rank - 2] != p.c.dim[rank - 2]) return false;
+        if (args) {
+            args->step_kind[i] = per_column ? kStepBias : kStepFull;
+            args->step_data[i] = tensors[5 + step.operand];
+            args->step_dtype[i] = t.dtype;
+            args->step_ld[i] = per_column ? 0 : t.stride[t.rank - 2];
+            args->step_vector[i] = on16(args->step_data[i]) && (args->step_ld[i] * dtype_bytes(t.dtype)) % 16 == 0 ? 1 : 0;
+        }
+    }
+    return true;
+}
+
+bool sixteen_problem(const dfgpu_matmul_params& p, Problem& problem) {
+    if (p.a_scale.rank || p.b_scale.rank) return false;
+    if ((p.a.dtype != DFGPU_BF16 && p.a.dtype != DFGPU_F16) || p.b.dtype != p.a.dtype) return false;   // (one kind of operand per instruction)
+    if (p.c.dtype != DFGPU_BF16 && p.c.dtype != DFGPU_F16 && p.c.dtype != DFGPU_F32) return false;
+    return describe(p.a, p.b, p.c, kSixteen, problem) && translate_steps(p, nullptr, nullptr);
+}
+
+bool scaled_problem(const dfgpu_matmul_params& p, Problem& problem) {
+    if (p.a.dtype != DFGPU_E4M3 || p.b.dtype != DFGPU_E4M3 || p.a_scale.dtype != DFGPU_E8M0 || p.b_scale.dtype != DFGPU_E8M0) return false;
+    if (p.c.dtype != DFGPU_BF16 && p.c.dtype != DFGPU_F16 && p.c.dtype != DFGPU_F32) return false;
+    const int rank = p.c.rank;
+    if (p.a_scale.rank != rank || p.b_scale.rank != rank || !describe(p.a, p.b, p.c, kScaled, problem)) return false;
+    for (int i = 0; i < rank - 2; ++i)
+        if (p.a_scale.dim[i] != 1 || p.b_scale.dim[i] != 1) return false;
+    if (problem.N <= 64) return false;   // (column scales come in chunks of 128: half of a tile would be empty; dequantized to bf16, N = 64 is a tile)
+    // scales: one per 32 elements along K, plain layout
+    if (problem.K % 32 != 0 || p.a_block[0] != 1 || p.a_block[1] != 32 || p.b_block[0] != 32 || p.b_block[1] != 1) return false;
+    if (p.a_scale.reorder != DFGPU_REORDER_NONE || p.b_scale.reorder != DFGPU_REORDER_NONE) return false;
+    if (p.a_scale.dim[rank - 2] != problem.M || p.a_scale.dim[rank - 1] != problem.K / 32 || p.a_scale.stride[rank - 1] != 1) return false;
+    if (p.b_scale.dim[rank - 2] != problem.K / 32 || p.b_scale.dim[rank - 1] != problem.N || p.b_scale.stride[rank - 1] != 1) return false;
+    return translate_steps(p, nullptr, nullptr);
+}
+
+}  // namespace
+
+bool matmul_umma_supported(const dfgpu_matmul_params& p, int kernel) {
+    Problem problem;
+    return kernel == DFGPU_MATMUL_UMMA_MXF8 ? scaled_problem(p, problem) : (kernel == DFGPU_MATMUL_UMMA_BF16 && sixteen_problem(p, problem));
+}
+
+int launch_matmul_umma(const dfgpu_matmul_params& p, void* const* tensors, int kernel, cudaStream_t stream) {
+    Problem problem;
+    TileArgs args{};
+    if (!on16(tensors[0]) || !on16(tensors[1])) return fail(kInvalidArgument, "MATMUL: the tcgen05 kernel needs 16-byte aligned A and B");
+    if (kernel == DFGPU_MATMUL_UMMA_MXF8) {
+        if (!scaled_problem(p, problem)) return fail(kUnsupported, "MATMUL: the tcgen05 kernel does not take these block-scaled operands");
+        const int rank = p.c.rank;
+        args.sfa = static_cast<const uint8_t*>(tensors[3]);
+        args.sfb = static_cast<const uint8_t*>(tensors[4]);
+        args.sfa_ld = p.a_scale.stride[rank - 2];
+        args.sfb_ld = p.b_scale.stride[rank - 2];
+        args.scale_blocks = static_cast<int>(problem.K / 32);
+        args.sfa_words = (reinterpret_cast<uintptr_t>(args.sfa) & 3u) == 0 && args.sfa_ld % 4 == 0 ? 1 : 0;
+    } else {
+        if (!sixteen_problem(p, problem)) return fail(kUnsupported, "MATMUL: the tcgen05 kernel does not take these operands");
+        if (p.a.dtype == DFGPU_BF16) args.idesc = (1u << 7) | (1u << 10);
+    }
+    translate_steps(p, tensors, &args);
+    return launch_problem(problem, args, tensors[0], tensors[1], tensors[2], stream, "MATMUL (tcgen05)");
+}
+
+bool fp8_problem(const dfgpu_matmul_fp8_params& p, Problem& problem) {
+    if ((p.a.dtype != DFGPU_E4M3 && p.a.dtype != DFGPU_E5M2) || (p.b.dtype != DFGPU_E4M3 && p.b.dtype != DFGPU_E5M2)) return false;
+    if (p.c.dtype != DFGPU_BF16 && p.c.dtype != DFGPU_F16 && p.c.dtype != DFGPU_F32 && p.c.dtype != DFGPU_E4M3 && p.c.dtype != DFGPU_E5M2) return false;
+    return describe(p.a, p.b, p.c, kCodes, problem);
+}
+
+bool matmul_fp8_umma_supported(const dfgpu_matmul_fp8_params& p) {
+    Problem problem;
+    return fp8_problem(p, problem);
+}
+
+int launch_matmul_fp8_umma(const dfgpu_matmul_fp8_params& p, void* const* tensors, cudaStream_t stream) {
+    Problem problem;
+    TileArgs args{};
+    if (!on16(tensors[0]) || !on16(tensors[1])) return fail(kInvalidArgument, "MATMUL_FP8: the tcgen05 kernel needs 16-byte aligned A and B");
+    if (!fp8_problem(p, problem)) return fail(kUnsupported, "MATMUL_FP8: the tcgen05 kernel does not take these operands");
+    args.idesc = (p.a.dtype == DFGPU_E5M2 ? 1u << 7 : 0u) | (p.b.dtype == DFGPU_E5M2 ? 1u << 10 : 0u);
+    args.amax_bits = static_cast<unsigned int*>(tensors[3]);
+    args.descale_a = static_cast<const float*>(tensors[4]);
+    args.descale_b = static_cast<const float*>(tensors[5]);
+    args.scale_c = static_cast<const float*>(tensors[6]);
+    return launch_problem(problem, args, tensors[0], tensors[1], tensors[2], stream, "MATMUL_FP8 (tcgen05)");
+}
+
+int matmul_tiles_device_status(int* status) { return read_and_clear_device_status(status); }
+
+}  // namespace dfgpu

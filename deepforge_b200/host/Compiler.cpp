@@ -359,6 +359,7 @@ bool matmul_fits_tensor_cores(Lowering const& low, OperationDesc const& node) {
     if (trial.b.dtype == DFGPU_F32 && !low.tensor(*b).is_virtual) return false;
     trial.a.dtype = trial.b.dtype = DFGPU_BF16;
     if (trial.c.dtype == DFGPU_F32 && low.tensor(*c).is_virtual) trial.c.dtype = DFGPU_BF16;
+    if (trial.a.dim[trial.a.rank - 1] % 64 != 0 || trial.c.dim[trial.c.rank - 1] % 64 != 0) return false;   // (whole 64-deep, 64-wide tiles only: a virtual tensor between others stays what the graph says)
     trial.kernel = DFGPU_MATMUL_UMMA_BF16;
     dfgpu_plan_info info{};
     return dfgpu_query_matmul(&trial, &info) == 0;
@@ -1099,17 +1100,26 @@ void materialise_constants(Lowering& low) {
 
 // Alignment the resolved kernel's launcher demands of the pointer in tensor slot `slot` (0: no demand of its own).
 // The TMA-fed kernels read and write 16-byte units and have no narrower fallback (the block-scale launchers do).
+// (A matrix product whose extents are whole tiles takes 16-byte aligned operands only; any other falls back to the CUDA
+// cores where a pointer is off that boundary, so its arguments keep the reference's alignment.)
+template <typename Params>
+bool whole_tiles(Params const& p, std::int64_t tile) {
+    auto const rank = p.c.rank;
+    return p.a.dim[rank - 1] % tile == 0 && p.c.dim[rank - 1] % tile == 0 && (tile == 64 || p.c.dim[rank - 2] % tile == 0);
+}
+
 std::uint64_t kernel_alignment(KernelStep const& step, std::size_t slot) {
     switch (step.op) {
         case KernelOp::kConvFprop: return step.kernel == DFGPU_CONV_UMMA_BF16 || step.kernel == DFGPU_CONV_UMMA_F32X3 ? 16 : 0;  // (the one-launch f32 form takes any pointer: see dfgpu_conv_fprop)
         case KernelOp::kMatmul:
             if (step.kernel != DFGPU_MATMUL_UMMA_BF16 && step.kernel != DFGPU_MATMUL_UMMA_MXF8 && step.kernel != DFGPU_MATMUL_UMMA_F32X3) return 0;
+            if (step.kernel != DFGPU_MATMUL_UMMA_F32X3 && !whole_tiles(std::get<dfgpu_matmul_params>(step.params), step.kernel == DFGPU_MATMUL_UMMA_MXF8 ? 128 : 64)) return 0;
             return slot == 3 || slot == 4 ? 4 : 16;  // the scale tensors are gathered with 4-byte loads
         case KernelOp::kSdpaForward:
             if (step.kernel == DFGPU_SDPA_UMMA) return slot <= 3 ? 16 : 0;
             if (step.kernel == DFGPU_SDPA_PAGED_DECODE_UMMA || step.kernel == DFGPU_SDPA_PAGED_DECODE) return slot <= 2 ? 16 : 0;
             return 0;
-        case KernelOp::kMatmulFp8: return step.kernel == DFGPU_MATMUL_FP8_UMMA && slot <= 2 ? 16 : 0;
+        case KernelOp::kMatmulFp8: return step.kernel == DFGPU_MATMUL_FP8_UMMA && slot <= 2 && whole_tiles(std::get<dfgpu_matmul_fp8_params>(step.params), 128) ? 16 : 0;
         case KernelOp::kConvFpropPair: return 16;
         case KernelOp::kBlockScaleQuantizePair: return slot % 3 == 0 ? 16 : 8;
         case KernelOp::kBlockScaleQuantize:   // packed FP4 codes are written a nibble at a time through their aligned word
