@@ -71,7 +71,8 @@ int launch_split6(const SplitOperand& first, const SplitOperand& second, int* fl
 bool matmul_umma_supported(const dfgpu_matmul_params& p, int kernel);
 int launch_matmul_umma(const dfgpu_matmul_params& p, void* const* tensors, int kernel, cudaStream_t stream);
 // MATMUL_FP8: the three scalars and Amax_C applied in the epilogue.
-bool matmul_fp8_umma_supported(const dfgpu_matmul_fp8_params& p);
+bool matmul_fp8_umma_supported(const dfgpu_matmul_fp8_params& p);   // whole tiles: the kernel id's promise
+bool matmul_fp8_tiles_supported(const dfgpu_matmul_fp8_params& p);  // everything launch_matmul_fp8_umma() takes
 int launch_matmul_fp8_umma(const dfgpu_matmul_fp8_params& p, void* const* tensors, cudaStream_t stream);
 int matmul_tiles_device_status(int* status);
 

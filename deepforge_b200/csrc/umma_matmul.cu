@@ -899,9 +899,15 @@ bool fp8_problem(const dfgpu_matmul_fp8_params& p, Problem& problem) {
     return describe(p.a, p.b, p.c, kCodes, problem);
 }
 
-bool matmul_fp8_umma_supported(const dfgpu_matmul_fp8_params& p) {
+bool matmul_fp8_tiles_supported(const dfgpu_matmul_fp8_params& p) {
     Problem problem;
     return fp8_problem(p, problem);
+}
+
+// What the kernel id DFGPU_MATMUL_FP8_UMMA promises: whole tiles and the outputs it names.
+bool matmul_fp8_umma_supported(const dfgpu_matmul_fp8_params& p) {
+    Problem problem;
+    return fp8_problem(p, problem) && problem.M % 128 == 0 && problem.N % 128 == 0 && problem.K % 128 == 0 && p.c.dtype != DFGPU_F16 && p.c.dtype != DFGPU_E5M2;
 }
 
 int launch_matmul_fp8_umma(const dfgpu_matmul_fp8_params& p, void* const* tensors, cudaStream_t stream) {
