@@ -571,20 +571,22 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             fold_amax(args, scalars, lane, ok);
         }
     } else if (KIND == kScaled) {
-        // ---- scale loaders: warp i of the four fills the slots of every fourth block ----
+        // ---- scale loaders: warp i of the four owns the slots i, i + 4, i + 8 ----
+        // (A slot has ONE owner: the parity of its barrier tells apart two rounds, not three, so a warp that came by a slot
+        // only every other round could fill it before its last round was read.)
         const int me = warp < 4 ? warp - 2 : warp - 10;
         const uint32_t counted_on = CG == 2 ? address_in(bar_base, 0) : bar_base;
-        int stage = 0, block = 0;
+        int stage = 0;
         uint32_t phase = 1;
         bool ok = true;
         for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
             const int m_tile = tile % args.m_tiles, n_tile = tile / args.m_tiles;
             const int row0 = (m_tile * CG + (CG == 2 ? rank : 0)) * kRows;
-            for (int kb = kb_begin; kb < kb_end; ++kb, ++block) {
+            for (int kb = kb_begin; kb < kb_end; ++kb) {
                 const int slot = stage;
                 const uint32_t slot_phase = phase;
                 if (++stage == args.stages) { stage = 0; phase ^= 1; }
-                if ((block & 3) != me) continue;
+                if ((slot & 3) != me) continue;
                 // the global loads do not wait for the slot
                 uint32_t a_words[4], b_words[2][4];
                 gather_row_scales(args, row0, kb, lane, a_words);
