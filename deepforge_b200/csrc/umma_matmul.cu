@@ -15,7 +15,7 @@
 // bn is 64, 128, 192 or 256 at run time; choose_shape() says which shape a product takes and why.
 //
 // Warps: 0 loads (TMA), 1 issues products, 4-11 are the epilogue (two groups of four, alternating 128-byte column boxes), and
-// with block scales 2, 3, 12 and 13 gather them. Two accumulators in tensor memory where they fit, so that a tile's epilogue
+// with block scales 2, 3 and 12-15 gather them. Two accumulators in tensor memory, so that a tile's epilogue
 // runs under the next tile's products. Finished boxes leave through a swizzled staging tile by TMA; a thread's own row of
 // 64 bytes at a row's distance would jam the load/store unit.
 #include <algorithm>
@@ -39,12 +39,14 @@ enum { kStepRelu = 1, kStepBias = 2, kStepFull = 3 };
 
 struct TileArgs {
     int32_t m_total, n_total;
-    int32_t m_tiles, n_tiles, k_blocks;
+    int32_t m_tiles, k_blocks;
     int32_t bn;                       // columns of a tile
+    int32_t whole_items, items;       // work items: whole tiles, and after them the halves of the tiles that are left for the last round
     int32_t splits, k_per_split;
-    int32_t stages, stage_bytes, accumulators;
-    int32_t load_bytes;               // what one CTA's copies of a stage write
-    int32_t b_boxes, b_box_bytes, b_box_columns;   // B of one CTA and stage
+    int32_t stages, stage_bytes;
+    int32_t acc_stride, scale_columns;   // tensor memory: see launch_problem()
+    int32_t a_bytes;                  // what one CTA's copy of A writes per stage
+    int32_t b_box_bytes, b_box_columns;   // B comes in boxes
     int32_t b_mn_major;
     uint32_t idesc;
     int32_t staging_offset, barrier_offset;
@@ -67,7 +69,7 @@ struct TileArgs {
     const uint8_t* sfa;
     const uint8_t* sfb;
     int64_t sfa_ld, sfb_ld;
-    int32_t scale_blocks, sfa_words;  // K / 32; sfa rows may be read as aligned words
+    int32_t scale_blocks, sfa_words;  // K / 32; sfa rows are whole aligned words
 };
 
 // ---- cluster and pair forms of the PTX wrappers ------------------------------------------------------------
@@ -138,17 +140,14 @@ __device__ __forceinline__ void product(uint32_t d, uint64_t a, uint64_t b, uint
 #define DFGPU_MMA(FORM)                                                                                                   \
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma." FORM ".kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}" \
                  ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb) : "memory")
-    if constexpr (KIND == kScaled && CG == 1) DFGPU_MMA("cta_group::1");
-    if constexpr (KIND == kScaled && CG == 2) DFGPU_MMA("cta_group::2");
+    if constexpr (KIND == kScaled) DFGPU_MMA("cta_group::1");
 #undef DFGPU_MMA
 }
 // 32 rows x 16 bytes of shared memory -> 4 columns of tensor memory, replicated to the four lane quarters.
-template <int CG>
 __device__ __forceinline__ void copy_scales(uint32_t tmem_dst, uint32_t address) {
     // an unswizzled K-major block: 8-row groups 128 bytes apart
     const uint64_t desc = static_cast<uint64_t>((address & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(128u >> 4) << 32) | (1ull << 46);
-    if constexpr (CG == 2) asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem_dst), "l"(desc) : "memory");
-    else asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem_dst), "l"(desc) : "memory");
+    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem_dst), "l"(desc) : "memory");
 }
 
 // ---- the fused steps on values of one row of C ---------------------------------------------------------------
@@ -298,9 +297,19 @@ __device__ __noinline__ bool mbar_wait_cluster_slow(uint32_t bar, uint32_t parit
         }
     }
 }
+__device__ __forceinline__ bool mbar_test_wait_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    return done != 0;
+}
 template <bool CLUSTER>
 __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, int code) {
     if constexpr (CLUSTER) {
+        if (__all_sync(0xffffffffu, mbar_test_wait_cluster(bar, parity))) return true;
 #pragma unroll 1
         for (int spin = 0; spin < 64; ++spin)
             if (__all_sync(0xffffffffu, mbar_try_wait_cluster(bar, parity))) return true;
@@ -311,47 +320,91 @@ __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, int cod
 }
 
 template <int KIND>
-constexpr int thread_count() { return KIND == kScaled ? 448 : 384; }
+constexpr int thread_count() { return KIND == kScaled ? 512 : 384; }
 
-// The four rows-of-32 words of scales of one 128-row (or 128-column) chunk, as tcgen05.cp wants them: byte j of a word is
-// the scale of K block j. Blocks, rows and columns past the end count as 2^0 (their codes are zeros).
-__device__ __forceinline__ void gather_row_scales(const TileArgs& args, int row0, int kb, int lane, uint32_t (&words)[4]) {
-    const int first = kb * 4, live = args.scale_blocks - first;
+// One K block's scales of a tile as a lane reads them from the plain tensors: 4 rows of A (rows lane, lane + 32, ... of 128)
+// and 4 or 8 columns of B, four K blocks each. Addresses are clamped, so that nothing branches around a load and all of
+// them are in flight together (with branches the gather took three times as long as the products); pack() selects. The
+// loads of a warp's next block are issued before it waits for its current slot, and packed after.
+struct RawScales {
+    uint32_t a[4];          // words, or bytes of block 0 when rows cannot be read as words
+    uint32_t a_more[4][3];  // bytes of blocks 1..3 then
+    uint32_t b[2][4][4];
+};
+__device__ __forceinline__ void load_scales(const TileArgs& args, int row0, int col0, int kb, int lane, RawScales& raw) {
+    const int first = kb * 4, last = args.scale_blocks - 1;
+    if (args.sfa_words) {
 #pragma unroll
-    for (int g = 0; g < 4; ++g) {
-        const int row = row0 + g * 32 + lane;
-        words[g] = 0x7f7f7f7fu;
-        if (row >= args.m_total) continue;
-        const uint8_t* p = args.sfa + row * args.sfa_ld + first;
-        if (args.sfa_words && live >= 4) {
-            words[g] = __ldg(reinterpret_cast<const uint32_t*>(p));
-        } else {
+        for (int g = 0; g < 4; ++g)
+            raw.a[g] = __ldg(reinterpret_cast<const uint32_t*>(args.sfa + min(row0 + g * 32 + lane, args.m_total - 1) * args.sfa_ld + first));
+    } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (j < live) words[g] = (words[g] & ~(0xffu << (8 * j))) | (static_cast<uint32_t>(__ldg(p + j)) << (8 * j));
+        for (int g = 0; g < 4; ++g) {
+            const uint8_t* p = args.sfa + min(row0 + g * 32 + lane, args.m_total - 1) * args.sfa_ld;
+            raw.a[g] = __ldg(p + first);
+#pragma unroll
+            for (int j = 1; j < 4; ++j) raw.a_more[g][j - 1] = __ldg(p + min(first + j, last));
+        }
+    }
+    const uint8_t* base[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) base[j] = args.sfb + min(first + j, last) * args.sfb_ld;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        if (c == 1 && args.bn <= 128) break;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            const int col = min(col0 + c * 128 + g * 32 + lane, args.n_total - 1);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) raw.b[c][g][j] = __ldg(base[j] + col);
         }
     }
 }
-__device__ __forceinline__ void gather_column_scales(const TileArgs& args, int col0, int kb, int lane, uint32_t (&words)[4]) {
-    const int first = kb * 4, live = args.scale_blocks - first;
+// The words tcgen05.cp wants: byte j the scale of K block j. Blocks, rows and columns past the end count as 2^0 (their codes
+// are zeros).
+__device__ __forceinline__ uint32_t pack_word(uint32_t b0, uint32_t b1, uint32_t b2, uint32_t b3, int live) {
+    return b0 | ((live > 1 ? b1 : 0x7fu) << 8) | ((live > 2 ? b2 : 0x7fu) << 16) | ((live > 3 ? b3 : 0x7fu) << 24);
+}
+__device__ __forceinline__ void pack_scales(const TileArgs& args, int row0, int col0, int kb, int lane, const RawScales& raw, uint32_t (&a)[4], uint32_t (&b)[2][4]) {
+    const int live = args.scale_blocks - kb * 4;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
-        const int col = col0 + g * 32 + lane;
-        words[g] = 0x7f7f7f7fu;
-        if (col >= args.n_total) continue;
-        const uint8_t* p = args.sfb + first * args.sfb_ld + col;
-        uint32_t byte[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) byte[j] = j < live ? __ldg(p + j * args.sfb_ld) : 0x7fu;
-        words[g] = byte[0] | (byte[1] << 8) | (byte[2] << 16) | (byte[3] << 24);
+        a[g] = args.sfa_words ? raw.a[g] : pack_word(raw.a[g], raw.a_more[g][0], raw.a_more[g][1], raw.a_more[g][2], live);
+        if (row0 + g * 32 + lane >= args.m_total) a[g] = 0x7f7f7f7fu;
     }
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            b[c][g] = pack_word(raw.b[c][g][0], raw.b[c][g][1], raw.b[c][g][2], raw.b[c][g][3], live);
+            if (col0 + c * 128 + g * 32 + lane >= args.n_total) b[c][g] = 0x7f7f7f7fu;
+        }
+}
+
+// A work item's tile, first column and width.
+struct Item {
+    int m_tile, col0, width;
+};
+__device__ __forceinline__ Item item_at(const TileArgs& args, int item) {
+    int tile = item, half = 0;
+    Item out;
+    out.width = args.bn;
+    if (item >= args.whole_items) {
+        tile = args.whole_items + ((item - args.whole_items) >> 1);
+        half = (item - args.whole_items) & 1;
+        out.width = args.bn >> 1;
+    }
+    const int n_tile = tile / args.m_tiles;
+    out.m_tile = tile - n_tile * args.m_tiles;
+    out.col0 = n_tile * args.bn + half * out.width;
+    return out;
 }
 
 template <int KIND, int CG>
 __global__ void __launch_bounds__(thread_count<KIND>(), 1)
 umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c,
                    const __grid_constant__ TileArgs args) {
-    constexpr bool kClusterWaits = KIND == kScaled && CG == 2;
+    static_assert(KIND != kScaled || CG == 1, "block scales: one SM per tile (see choose_shape())");
     constexpr int kCode = KIND == kSixteen ? 0 : (KIND == kCodes ? 20 : 40);
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -361,19 +414,20 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     auto empty_bar = [&](int s) { return bar_base + 8u * (kMaxStages + s); };
     auto acc_full = [&](int a) { return bar_base + 8u * (2 * kMaxStages + a); };
     auto acc_empty = [&](int a) { return bar_base + 8u * (2 * kMaxStages + 2 + a); };
-    const uint32_t tmem_slot = bar_base + 8u * (2 * kMaxStages + 4);
-    volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(generic_base + args.barrier_offset + 8 * (2 * kMaxStages + 4));
+    const uint32_t overlap_free = bar_base + 8u * (2 * kMaxStages + 4);
+    const uint32_t tmem_slot = bar_base + 8u * (2 * kMaxStages + 5);
+    volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(generic_base + args.barrier_offset + 8 * (2 * kMaxStages + 5));
 
     const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
     const bool leader = elect_one();
     const bool split = CG == 1 && args.splits > 1;
     const int rank = CG == 2 || split ? static_cast<int>(cluster_rank()) : 0;
     const int group = CG == 2 ? 2 : args.splits;            // CTAs that share a tile
-    const int first_tile = static_cast<int>(blockIdx.x) / group, tile_step = static_cast<int>(gridDim.x) / group;
-    const int tiles = args.m_tiles * args.n_tiles;
+    const int first_item = static_cast<int>(blockIdx.x) / group, item_step = static_cast<int>(gridDim.x) / group;
     const int kb_begin = split ? rank * args.k_per_split : 0;
     const int kb_end = split ? min(args.k_blocks, kb_begin + args.k_per_split) : args.k_blocks;
     const int bn = args.bn;
+    const bool overlapped = KIND == kScaled && args.acc_stride < bn;
 
     if (threadIdx.x == 0) {
         prefetch_tensormap(&map_a);
@@ -382,13 +436,14 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     }
     if (warp == 0 && leader) {
         for (int s = 0; s < args.stages; ++s) {
-            mbar_init(full_bar(s), KIND == kScaled ? 1 + CG : 1);   // the byte count, and one scale warp of each CTA
+            mbar_init(full_bar(s), KIND == kScaled ? 2 : 1);   // the byte count, and the slot's scale warp
             mbar_init(empty_bar(s), 1);
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(acc_full(a), 1);
             mbar_init(acc_empty(a), 8 * CG);
         }
+        mbar_init(overlap_free, 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -408,9 +463,10 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         int stage = 0;
         uint32_t phase = 1;
         bool ok = true;
-        for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
-            const int m_tile = tile % args.m_tiles, n_tile = tile / args.m_tiles;
-            const int row0 = (m_tile * CG + (CG == 2 ? rank : 0)) * kRows, col0 = n_tile * bn + (CG == 2 ? rank * (bn / 2) : 0);
+        for (int i = first_item; i < args.items && ok; i += item_step) {
+            const Item item = item_at(args, i);
+            const int columns = item.width / CG, boxes = columns / args.b_box_columns;
+            const int row0 = (item.m_tile * CG + (CG == 2 ? rank : 0)) * kRows, col0 = item.col0 + (CG == 2 ? rank * columns : 0);
             for (int kb = kb_begin; kb < kb_end; ++kb) {
                 ok = mbar_wait_warp(empty_bar(stage), phase, 501 + kCode);
                 if (!ok) break;
@@ -418,9 +474,9 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     const uint32_t a_dst = smem_base + stage * args.stage_bytes, b_dst = a_dst + kABytes;
                     const uint32_t bar = counted_on + 8u * stage;
                     constexpr int kPerRow = KIND == kSixteen ? 64 : 128;   // elements of K per block
-                    if (CG == 1 || rank == 0) mbar_expect_tx(full_bar(stage), CG * args.load_bytes);
+                    if (CG == 1 || rank == 0) mbar_expect_tx(full_bar(stage), CG * (args.a_bytes + columns * kRowBytes));
                     load_tile<CG>(a_dst, &map_a, kb * kPerRow, row0, bar);
-                    for (int j = 0; j < args.b_boxes; ++j) {
+                    for (int j = 0; j < boxes; ++j) {
                         if (args.b_mn_major) load_tile<CG>(b_dst + j * args.b_box_bytes, &map_b, col0 + j * args.b_box_columns, kb * kPerRow, bar);
                         else load_tile<CG>(b_dst + j * args.b_box_bytes, &map_b, kb * kPerRow, col0 + j * args.b_box_columns, bar);
                     }
@@ -435,32 +491,34 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
             const uint32_t b_lbo = args.b_mn_major ? (KIND == kSixteen ? 64 * kRowBytes : 128 * kRowBytes) : 16;
             const uint32_t b_step = args.b_mn_major ? (KIND == kSixteen ? 2048u >> 4 : 4096u >> 4) : 32u >> 4;
-            const int scale_columns = args.accumulators * bn;   // where the scales' tensor memory starts
             int stage = 0, local = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (int tile = first_tile; tile < tiles; tile += tile_step, ++local) {
-                const int acc = args.accumulators == 2 ? local & 1 : 0, use = args.accumulators == 2 ? local >> 1 : local;
+            for (int i = first_item; i < args.items; i += item_step, ++local) {
+                const int width = item_at(args, i).width, acc = local & 1, use = local >> 1;
+                const uint32_t idesc_wide = args.idesc | (static_cast<uint32_t>(width >> 3) << 17);
                 if (ok) ok = wait_warp<CG == 2>(acc_empty(acc), (use & 1) ^ 1, 502 + kCode);
+                // (where the accumulators overlap, the other one's shared columns must have been read out too)
+                if (overlapped && ok && local > 0) ok = mbar_wait_warp(overlap_free, (local - 1) & 1, 507 + kCode);
                 tc_fence_after();
-                const uint32_t d = tmem_u + acc * bn;
+                const uint32_t d = tmem_u + acc * args.acc_stride;
                 for (int kb = kb_begin; kb < kb_end && ok; ++kb) {
-                    ok = wait_warp<kClusterWaits>(full_bar(stage), phase, 503 + kCode);
+                    ok = mbar_wait_warp(full_bar(stage), phase, 503 + kCode);
                     if (!ok) break;   // (operands by TMA, scales by generic stores + fence.proxy.async: no tcgen05 fence needed)
                     if (leader) {
                         const uint32_t a_src = smem_base + stage * args.stage_bytes, b_src = a_src + kABytes;
                         const uint32_t a_lo = smem_desc_lo(a_src, 16), b_lo = smem_desc_lo(b_src, b_lbo);
                         uint32_t sf = 0;
                         if constexpr (KIND == kScaled) {
-                            const uint32_t scales = b_src + (CG == 2 ? bn / 2 : bn) * kRowBytes;
-                            sf = tmem_u + scale_columns + (stage & 1) * 16;   // A's at +0..3, B's at +4..11
-                            copy_scales<CG>(sf, scales);
-                            copy_scales<CG>(sf + 4, scales + 512);
-                            if (bn > 128) copy_scales<CG>(sf + 8, scales + 1024);
+                            const uint32_t scales = b_src + bn * kRowBytes;
+                            sf = tmem_u + args.scale_columns + (stage & 1) * 16;   // A's at +0..3, B's at +4..11
+                            copy_scales(sf, scales);
+                            copy_scales(sf + 4, scales + 512);
+                            if (width > 128) copy_scales(sf + 8, scales + 1024);
                         }
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
-                            uint32_t idesc = args.idesc;
+                            uint32_t idesc = idesc_wide;
                             if constexpr (KIND == kScaled) idesc |= (static_cast<uint32_t>(j) << 29) | (static_cast<uint32_t>(j) << 4);   // the K block's byte of the scale words
                             product<KIND, CG>(d, desc_words(a_lo + ((j * 32) >> 4), smem_desc_hi(1024)), desc_words(b_lo + j * b_step, smem_desc_hi(1024)), idesc,
                                               kb != kb_begin || j != 0 ? 1u : 0u, sf, sf + 4);
@@ -500,17 +558,20 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             Scalars scalars = load_scalars(args);
             bool stored = false;   // (this group has a store in flight)
             int local = 0;
-            for (int tile = first_tile; tile < tiles; tile += tile_step, ++local) {
-                const int acc = args.accumulators == 2 ? local & 1 : 0, use = args.accumulators == 2 ? local >> 1 : local;
-                const int m_tile = tile % args.m_tiles, n_tile = tile / args.m_tiles;
-                const int row0 = (m_tile * CG + (CG == 2 ? rank : 0)) * kRows, out_row = row0 + row;
+            for (int i = first_item; i < args.items; i += item_step, ++local) {
+                const int acc = local & 1, use = local >> 1;
+                const Item item = item_at(args, i);
+                const int row0 = (item.m_tile * CG + (CG == 2 ? rank : 0)) * kRows, out_row = row0 + row;
                 const bool row_live = out_row < args.m_total;
                 if (ok) ok = mbar_wait(acc_full(acc), use & 1, 505 + kCode);
                 tc_fence_after();
                 const bool healthy = ok && g_device_status == 0;
-                const uint32_t columns = tmem_base + lane_base + acc * bn;
-                for (int box = g; box < bn / box_columns; box += 2) {
-                    const int col0 = n_tile * bn + box * box_columns;
+                const uint32_t columns = tmem_base + lane_base + acc * args.acc_stride;
+                const int boxes = item.width / box_columns;
+                for (int b = g; b < boxes; b += 2) {
+                    // overlapping accumulators: the first one is read from its end, the second from its start
+                    const int box = overlapped && acc == 0 ? boxes - 2 + 2 * g - b : b;
+                    const int col0 = item.col0 + box * box_columns;
                     if (args.tma_store && stored) {
                         if (row == 0) tma_store_wait_read<0>();
                         epilogue_barrier(1 + g);
@@ -519,6 +580,11 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         uint32_t raw[32];
                         tmem_load_32(columns + box * box_columns + part * 32, raw);
                         tmem_load_wait();
+                        if (overlapped && b == g && g != acc && part == box_columns / 32 - 1) {   // the shared columns are in registers
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(overlap_free);
+                        }
                         float v[32];
 #pragma unroll
                         for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(raw[e]);
@@ -571,40 +637,46 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             fold_amax(args, scalars, lane, ok);
         }
     } else if (KIND == kScaled) {
-        // ---- scale loaders: warp i of the four owns the slots i, i + 4, i + 8 ----
+        // ---- scale loaders: warp i of the six owns the slots i and i + 6 ----
         // (A slot has ONE owner: the parity of its barrier tells apart two rounds, not three, so a warp that came by a slot
         // only every other round could fill it before its last round was read.)
         const int me = warp < 4 ? warp - 2 : warp - 10;
-        const uint32_t counted_on = CG == 2 ? address_in(bar_base, 0) : bar_base;
-        int stage = 0;
+        constexpr int kScaleWarps = 6;   // (no fewer than the slots of a 256-column ring: a warp with two slots set the pace)
+        // position in the list of (work item, K block) pairs this CTA walks, `stage` the slot of the pair
+        int at = first_item, kb = kb_begin, stage = 0;
         uint32_t phase = 1;
-        bool ok = true;
-        for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
-            const int m_tile = tile % args.m_tiles, n_tile = tile / args.m_tiles;
-            const int row0 = (m_tile * CG + (CG == 2 ? rank : 0)) * kRows;
-            for (int kb = kb_begin; kb < kb_end; ++kb) {
-                const int slot = stage;
-                const uint32_t slot_phase = phase;
-                if (++stage == args.stages) { stage = 0; phase ^= 1; }
-                if ((slot & 3) != me) continue;
-                // the global loads do not wait for the slot
-                uint32_t a_words[4], b_words[2][4];
-                gather_row_scales(args, row0, kb, lane, a_words);
-                gather_column_scales(args, n_tile * bn, kb, lane, b_words[0]);
-                if (bn > 128) gather_column_scales(args, n_tile * bn + 128, kb, lane, b_words[1]);
-                ok = mbar_wait_warp(empty_bar(slot), slot_phase, 506 + kCode);
-                if (!ok) break;
-                uint8_t* scales = generic_base + slot * args.stage_bytes + kABytes + (CG == 2 ? bn / 2 : bn) * kRowBytes + lane * 16;
-                *reinterpret_cast<uint4*>(scales) = make_uint4(a_words[0], a_words[1], a_words[2], a_words[3]);
-                *reinterpret_cast<uint4*>(scales + 512) = make_uint4(b_words[0][0], b_words[0][1], b_words[0][2], b_words[0][3]);
-                if (bn > 128) *reinterpret_cast<uint4*>(scales + 1024) = make_uint4(b_words[1][0], b_words[1][1], b_words[1][2], b_words[1][3]);
-                fence_async_shared();
-                __syncwarp();
-                if (leader) {
-                    if (CG == 2) mbar_arrive_cluster(counted_on + 8u * slot);
-                    else mbar_arrive(full_bar(slot));
-                }
-            }
+        auto advance = [&] {
+            if (++stage == args.stages) { stage = 0; phase ^= 1; }
+            if (++kb == kb_end) { kb = kb_begin; at += item_step; }
+        };
+        auto seek = [&] {   // the next pair in one of this warp's slots
+            while (at < args.items && stage % kScaleWarps != me) advance();
+            return at < args.items;
+        };
+        RawScales raw;
+        Item item = item_at(args, at);
+        auto load = [&] {
+            item = item_at(args, at);
+            load_scales(args, item.m_tile * kRows, item.col0, kb, lane, raw);
+        };
+        bool more = kb_begin < kb_end && seek();
+        if (more) load();
+        while (more) {
+            const int slot = stage;
+            const uint32_t slot_phase = phase;
+            uint32_t a_words[4], b_words[2][4];
+            pack_scales(args, item.m_tile * kRows, item.col0, kb, lane, raw, a_words, b_words);
+            advance();
+            more = seek();
+            if (more) load();
+            if (!mbar_wait_warp(empty_bar(slot), slot_phase, 506 + kCode)) break;
+            uint8_t* scales = generic_base + slot * args.stage_bytes + kABytes + bn * kRowBytes + lane * 16;
+            *reinterpret_cast<uint4*>(scales) = make_uint4(a_words[0], a_words[1], a_words[2], a_words[3]);
+            *reinterpret_cast<uint4*>(scales + 512) = make_uint4(b_words[0][0], b_words[0][1], b_words[0][2], b_words[0][3]);
+            if (bn > 128) *reinterpret_cast<uint4*>(scales + 1024) = make_uint4(b_words[1][0], b_words[1][1], b_words[1][2], b_words[1][3]);
+            fence_async_shared();
+            __syncwarp();
+            if (leader) mbar_arrive(full_bar(slot));
         }
     }
 
@@ -612,15 +684,15 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         // ---- the cluster's partial tiles: every CTA adds its share of the live rows over all ranks, in rank order ----
         __syncthreads();
         cluster_sync_all();
-        const int m_tile = first_tile % args.m_tiles, n_tile = first_tile / args.m_tiles;
-        const int row0 = m_tile * kRows, live_rows = min(kRows, args.m_total - row0);
+        const Item item = item_at(args, first_item);
+        const int row0 = item.m_tile * kRows, live_rows = min(kRows, args.m_total - row0);
         const int share = (live_rows + args.splits - 1) / args.splits, begin = rank * share, end = min(live_rows, begin + share);
         const int quads = bn / 4;
         Scalars scalars = load_scalars(args);
         const bool healthy = g_device_status == 0;
-        for (int item = threadIdx.x; item < (end - begin) * quads; item += blockDim.x) {
-            const int row = begin + item / quads, unit = item % quads;
-            const int col = n_tile * bn + unit * 4;
+        for (int i = threadIdx.x; i < (end - begin) * quads; i += blockDim.x) {
+            const int row = begin + i / quads, unit = i % quads;
+            const int col = item.col0 + unit * 4;
             if (col >= args.n_total) continue;
             const uint32_t at = smem_base + row * bn * 4 + (((unit & ~7) | ((unit ^ row) & 7)) << 4);
             constexpr int kMost = 8;
@@ -709,6 +781,7 @@ bool describe(const dfgpu_tensor& a, const dfgpu_tensor& b, const dfgpu_tensor& 
 struct Shape {
     int cg, bn, splits, k_per_split;
     int64_t tiles;
+    int64_t halved;   // tiles of the last round that are cut into halves
     double clocks;
 };
 
@@ -716,17 +789,19 @@ struct Shape {
 //   products       2 bn clocks (128 rows per SM, 16-bit and FP8 alike: a block is 128 bytes of K)
 //   shared memory  every operand byte written and read once at 128 B per clock: 2 (rows of A + columns of B)
 //   L2             the same bytes at about 48 per clock and SM when all SMs fetch
-// and a round over the SMs costs its blocks, a fill of ~2000 clocks and the last tile's epilogue. Splitting K divides the
-// blocks and adds ~2500 clocks of exchange; clusters of 4 and 8 leave some SMs of a GPC without a place.
+// and a round over the SMs costs its blocks (a last round that at most half fills the SMs is cut into half tiles: 4096^3 is 512
+// tiles of 128 x 256 on 148 SMs, three rounds and 68 tiles, which become 136 halves), a fill of ~2000 clocks and the last tile's epilogue. Splitting K divides the
+// blocks and adds ~2500 clocks of exchange; 33 clusters of 4 and 15 of 8 fit the chip at once (cudaOccupancyMaxActiveClusters).
 Shape choose_shape(const Problem& p) {
     const int64_t blocks = (p.K * p.in_bytes + kRowBytes - 1) / kRowBytes;
     const int sms = 148;   // (a function of the shape alone: the count this library is built for)
-    Shape best{0, 0, 0, 0, 0, 0.0};
-    for (int cg = 1; cg <= 2; ++cg)
+    Shape best{0, 0, 0, 0, 0, 0, 0.0};
+    for (int cg = 1; cg <= (p.kind == kScaled ? 1 : 2); ++cg)
         for (int bn = 64; bn <= 256; bn += 64) {
             const int chunk = p.kind == kSixteen ? 64 : 128;   // columns of one N-major copy
             if (p.b_mn_major && (bn / cg) % chunk != 0) continue;
             if (p.out_dtype == DFGPU_E4M3 && bn % 128 != 0) continue;   // (whole 128-byte boxes)
+            if (p.kind == kScaled && bn % 128 != 0) continue;           // (whole chunks of column scales)
             if (cg == 2 && bn < 128) continue;
             if (bn > chunk && bn >= 2 * ((p.N + 63) / 64 * 64)) continue;  // (half the tile would be empty)
             const int64_t m_tiles = (p.M + kRows * cg - 1) / (kRows * cg), n_tiles = (p.N + bn - 1) / bn, tiles = m_tiles * n_tiles;
@@ -735,11 +810,18 @@ Shape choose_shape(const Problem& p) {
                 if (splits > 1 && (bn > 128 || splits > blocks || tiles * splits > sms)) break;
                 const int64_t k_per_split = (blocks + splits - 1) / splits;
                 if (splits > 1 && k_per_split * (splits - 1) >= blocks) continue;   // (no CTA without a block)
-                const int64_t slots = splits == 8 ? 16 : (splits == 4 ? 35 : sms / (cg * splits));
-                const double rounds = static_cast<double>((tiles + slots - 1) / slots);
+                const int64_t slots = splits == 8 ? 15 : (splits == 4 ? 33 : sms / (cg * splits));
+                double rounds = static_cast<double>((tiles + slots - 1) / slots);
+                int64_t halved = 0;
+                const int half = bn / 2;
+                const bool halves = splits == 1 && half / cg >= 64 && (!p.b_mn_major || half / cg % chunk == 0) && half % (p.kind == kScaled || p.out_dtype == DFGPU_E4M3 ? 128 : 64) == 0;
+                if (halves && tiles > slots && tiles % slots != 0 && 2 * (tiles % slots) <= slots) {
+                    halved = tiles % slots;
+                    rounds -= 0.45;
+                }
                 const double block = std::max({2.0 * bn, 2.0 * (rows + bn / cg), (rows + bn / cg) * kRowBytes / 48.0});
-                const double clocks = rounds * (k_per_split * block + (p.kind == kScaled && bn == 256 ? 1500.0 : 0.0)) + 2000.0 + bn * 6.0 + (splits > 1 ? 2500.0 : 0.0) + (cg == 2 ? 500.0 : 0.0);
-                if (best.cg == 0 || clocks < best.clocks) best = Shape{cg, bn, splits, static_cast<int>(k_per_split), tiles, clocks};
+                const double clocks = rounds * (k_per_split * block) + 2000.0 + bn * 6.0 + (splits > 1 ? 2500.0 : 0.0) + (cg == 2 ? 500.0 : 0.0);
+                if (best.cg == 0 || clocks < best.clocks) best = Shape{cg, bn, splits, static_cast<int>(k_per_split), tiles, halved, clocks};
             }
         }
     return best;
@@ -764,30 +846,33 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     args.n_total = static_cast<int>(p.N);
     args.bn = shape.bn;
     args.m_tiles = static_cast<int>((p.M + kRows * shape.cg - 1) / (kRows * shape.cg));
-    args.n_tiles = static_cast<int>((p.N + shape.bn - 1) / shape.bn);
     args.k_blocks = static_cast<int>((p.K * p.in_bytes + kRowBytes - 1) / kRowBytes);
     args.splits = shape.splits;
     args.k_per_split = shape.k_per_split;
     args.b_mn_major = p.b_mn_major ? 1 : 0;
     const int columns = shape.bn / shape.cg;   // of B per CTA
-    args.b_boxes = p.b_mn_major ? columns / chunk : 1;
-    args.b_box_columns = p.b_mn_major ? chunk : columns;
-    args.b_box_bytes = (p.b_mn_major ? kRowBytes / p.in_bytes : columns) * kRowBytes;   // N-major: one row of 128 bytes per element of K
+    args.b_box_columns = p.b_mn_major ? chunk : (shape.halved > 0 ? columns / 2 : columns);
+    args.whole_items = static_cast<int>(shape.tiles - shape.halved);
+    args.items = static_cast<int>(shape.tiles + shape.halved);
+    args.b_box_bytes = (p.b_mn_major ? kRowBytes / p.in_bytes : args.b_box_columns) * kRowBytes;   // N-major: one row of 128 bytes per element of K
     const int a_rows = args.m_tiles == 1 && shape.cg == 1 ? static_cast<int>(std::min<int64_t>(kRows, (p.M + 7) / 8 * 8)) : kRows;
-    args.load_bytes = (a_rows + columns) * kRowBytes;
+    args.a_bytes = a_rows * kRowBytes;
     args.stage_bytes = kABytes + columns * kRowBytes + (p.kind == kScaled ? 2048 : 0);
     args.out = c;
     args.out_ld = p.c_ld;
     args.out_dtype = p.out_dtype;
     args.tma_store = on16(c) && (p.c_ld * p.out_bytes) % 16 == 0 && p.out_dtype != DFGPU_E5M2 ? 1 : 0;
-    args.accumulators = 2 * shape.bn + (p.kind == kScaled ? 32 : 0) <= 512 ? 2 : 1;
-    const int staging = shape.splits > 1 || !args.tma_store ? 0 : 2 * kStageBox, barriers = (2 * kMaxStages + 5) * 8;
+    // Tensor memory: two accumulators, and with block scales 32 columns of them at the end. At bn = 256 the accumulators then
+    // overlap by 32 columns, which the epilogue reads out first.
+    args.acc_stride = p.kind == kScaled && shape.bn == 256 ? 224 : shape.bn;
+    args.scale_columns = 480;
+    const int staging = shape.splits > 1 || !args.tma_store ? 0 : 2 * kStageBox, barriers = (2 * kMaxStages + 6) * 8;
     args.stages = std::min(kMaxStages, (kSmemBudget - staging - barriers) / args.stage_bytes);
     args.staging_offset = args.stages * args.stage_bytes;
     args.barrier_offset = args.staging_offset + staging;
     const int dynamic = args.barrier_offset + barriers + 1024;
-    // instruction descriptor: f32 accumulators (or E8M0 scales), the operand formats the caller has set, B's major, N, M
-    args.idesc |= (p.kind == kScaled ? 1u << 23 : 1u << 4) | (static_cast<uint32_t>(args.b_mn_major) << 16) | (static_cast<uint32_t>(shape.bn >> 3) << 17) |
+    // instruction descriptor: f32 accumulators (or E8M0 scales), the operand formats the caller has set, B's major, M (N is the item's)
+    args.idesc |= (p.kind == kScaled ? 1u << 23 : 1u << 4) | (static_cast<uint32_t>(args.b_mn_major) << 16) |
                   (static_cast<uint32_t>(kRows * shape.cg >> 4) << 24);
     const CUtensorMapDataType in_type = p.kind == kSixteen ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;   // (copied, never computed on)
     const uint32_t per_row = kRowBytes / p.in_bytes;
@@ -795,7 +880,7 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     int status = encode_map(&map_a, in_type, a, p.K, p.M, p.a_ld * p.in_bytes, per_row, a_rows, what);
     if (!status) {
         if (p.b_mn_major) status = encode_map(&map_b, in_type, b, p.N, p.K, p.b_ld * p.in_bytes, chunk, per_row, what);
-        else status = encode_map(&map_b, in_type, b, p.K, p.N, p.b_ld * p.in_bytes, per_row, columns, what);
+        else status = encode_map(&map_b, in_type, b, p.K, p.N, p.b_ld * p.in_bytes, per_row, static_cast<uint32_t>(args.b_box_columns), what);
     }
     if (!status && args.tma_store) {
         const CUtensorMapDataType out_type = p.out_dtype == DFGPU_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : (p.out_dtype == DFGPU_E4M3 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
@@ -806,7 +891,7 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     const int grid = static_cast<int>(groups * (shape.cg == 2 ? 2 : shape.splits));
     if (p.kind == kSixteen) return shape.cg == 2 ? launch_kernel<kSixteen, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kSixteen, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     if (p.kind == kCodes) return shape.cg == 2 ? launch_kernel<kCodes, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kCodes, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
-    return shape.cg == 2 ? launch_kernel<kScaled, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kScaled, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
+    return launch_kernel<kScaled, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
 }
 
 // The fused steps the kernel applies: ReLU, a per-column ADD operand, a full [M, N] ADD operand with contiguous columns.
@@ -886,7 +971,7 @@ int launch_matmul_umma(const dfgpu_matmul_params& p, void* const* tensors, int k
         args.sfa_ld = p.a_scale.stride[rank - 2];
         args.sfb_ld = p.b_scale.stride[rank - 2];
         args.scale_blocks = static_cast<int>(problem.K / 32);
-        args.sfa_words = (reinterpret_cast<uintptr_t>(args.sfa) & 3u) == 0 && args.sfa_ld % 4 == 0 ? 1 : 0;
+        args.sfa_words = (reinterpret_cast<uintptr_t>(args.sfa) & 3u) == 0 && args.sfa_ld % 4 == 0 && args.scale_blocks % 4 == 0 ? 1 : 0;
     } else {
         if (!sixteen_problem(p, problem)) return fail(kUnsupported, "MATMUL: the tcgen05 kernel does not take these operands");
         if (p.a.dtype == DFGPU_BF16) args.idesc = (1u << 7) | (1u << 10);
