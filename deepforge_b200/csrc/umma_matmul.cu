@@ -30,7 +30,7 @@ constexpr int kRows = 128;            // rows of A per CTA and tile
 constexpr int kRowBytes = 128;        // one swizzled shared-memory row: 64 16-bit values or 128 codes of K
 constexpr int kABytes = kRows * kRowBytes;
 constexpr int kStageBox = 128 * 128;  // one staging tile: 128 rows x 128 bytes of C
-constexpr int kMaxStages = 12;
+constexpr int kMaxStages = 16;
 constexpr int kMaxSteps = DFGPU_MAX_EPILOGUE;
 constexpr int kSmemBudget = 227 * 1024 - 1024;   // (1 KB of slack aligns the tiles)
 
@@ -45,7 +45,7 @@ struct TileArgs {
     int32_t splits, k_per_split;
     int32_t stages, stage_bytes;
     int32_t acc_stride, scale_columns;   // tensor memory: see launch_problem()
-    int32_t a_bytes;                  // what one CTA's copy of A writes per stage
+    int32_t a_bytes;                  // A of one CTA and stage; B lies behind it
     int32_t b_box_bytes, b_box_columns;   // B comes in boxes
     int32_t b_mn_major;
     uint32_t idesc;
@@ -471,7 +471,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 ok = mbar_wait_warp(empty_bar(stage), phase, 501 + kCode);
                 if (!ok) break;
                 if (leader) {
-                    const uint32_t a_dst = smem_base + stage * args.stage_bytes, b_dst = a_dst + kABytes;
+                    const uint32_t a_dst = smem_base + stage * args.stage_bytes, b_dst = a_dst + args.a_bytes;
                     const uint32_t bar = counted_on + 8u * stage;
                     constexpr int kPerRow = KIND == kSixteen ? 64 : 128;   // elements of K per block
                     if (CG == 1 || rank == 0) mbar_expect_tx(full_bar(stage), CG * (args.a_bytes + columns * kRowBytes));
@@ -506,7 +506,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     ok = mbar_wait_warp(full_bar(stage), phase, 503 + kCode);
                     if (!ok) break;   // (operands by TMA, scales by generic stores + fence.proxy.async: no tcgen05 fence needed)
                     if (leader) {
-                        const uint32_t a_src = smem_base + stage * args.stage_bytes, b_src = a_src + kABytes;
+                        const uint32_t a_src = smem_base + stage * args.stage_bytes, b_src = a_src + args.a_bytes;   // (with few rows the products read on into B: rows of C nobody stores)
                         const uint32_t a_lo = smem_desc_lo(a_src, 16), b_lo = smem_desc_lo(b_src, b_lbo);
                         uint32_t sf = 0;
                         if constexpr (KIND == kScaled) {
@@ -670,7 +670,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             more = seek();
             if (more) load();
             if (!mbar_wait_warp(empty_bar(slot), slot_phase, 506 + kCode)) break;
-            uint8_t* scales = generic_base + slot * args.stage_bytes + kABytes + bn * kRowBytes + lane * 16;
+            uint8_t* scales = generic_base + slot * args.stage_bytes + args.a_bytes + bn * kRowBytes + lane * 16;
             *reinterpret_cast<uint4*>(scales) = make_uint4(a_words[0], a_words[1], a_words[2], a_words[3]);
             *reinterpret_cast<uint4*>(scales + 512) = make_uint4(b_words[0][0], b_words[0][1], b_words[0][2], b_words[0][3]);
             if (bn > 128) *reinterpret_cast<uint4*>(scales + 1024) = make_uint4(b_words[1][0], b_words[1][1], b_words[1][2], b_words[1][3]);
@@ -778,6 +778,17 @@ bool describe(const dfgpu_tensor& a, const dfgpu_tensor& b, const dfgpu_tensor& 
     return c.stride[rank - 1] == 1 && p.c_ld >= p.N;
 }
 
+// Few rows take little of a stage, so that more stages fit. (A product still reads 128 rows: ring_bytes() keeps the last
+// stage's inside the allocation.)
+int rows_of_a(const Problem& p, int cg) { return cg == 1 && p.M < kRows ? static_cast<int>((p.M + 7) / 8 * 8) : kRows; }
+int stage_bytes(const Problem& p, int bn, int cg, int a_rows) { return (a_rows + bn / cg) * kRowBytes + (p.kind == kScaled ? 2048 : 0); }
+int ring_bytes(int stages, int stage_size) { return (stages - 1) * stage_size + std::max(stage_size, kABytes); }
+int stages_that_fit(int stage_size, int budget) {
+    int stages = std::min(kMaxStages, budget / stage_size);
+    while (stages > 2 && ring_bytes(stages, stage_size) > budget) --stages;
+    return stages;
+}
+
 struct Shape {
     int cg, bn, splits, k_per_split;
     int64_t tiles;
@@ -788,10 +799,10 @@ struct Shape {
 // The shape with the fewest estimated clocks. One K block of a CTA costs the longest of
 //   products       2 bn clocks (128 rows per SM, 16-bit and FP8 alike: a block is 128 bytes of K)
 //   shared memory  every operand byte written and read once at 128 B per clock: 2 (rows of A + columns of B)
-//   L2             the same bytes at about 48 per clock and SM when all SMs fetch
+//   L2             the same bytes at about 48 per clock and SM when all SMs fetch, or what the ring holds per ~2300 clocks of latency
 // and a round over the SMs costs its blocks (a last round that at most half fills the SMs is cut into half tiles: 4096^3 is 512
 // tiles of 128 x 256 on 148 SMs, three rounds and 68 tiles, which become 136 halves), a fill of ~2000 clocks and the last tile's epilogue. Splitting K divides the
-// blocks and adds ~2500 clocks of exchange; 33 clusters of 4 and 15 of 8 fit the chip at once (cudaOccupancyMaxActiveClusters).
+// blocks and adds ~2500 clocks of exchange (5000 with block scales); 33 clusters of 4 and 15 of 8 fit the chip at once (cudaOccupancyMaxActiveClusters).
 Shape choose_shape(const Problem& p) {
     const int64_t blocks = (p.K * p.in_bytes + kRowBytes - 1) / kRowBytes;
     const int sms = 148;   // (a function of the shape alone: the count this library is built for)
@@ -805,7 +816,7 @@ Shape choose_shape(const Problem& p) {
             if (cg == 2 && bn < 128) continue;
             if (bn > chunk && bn >= 2 * ((p.N + 63) / 64 * 64)) continue;  // (half the tile would be empty)
             const int64_t m_tiles = (p.M + kRows * cg - 1) / (kRows * cg), n_tiles = (p.N + bn - 1) / bn, tiles = m_tiles * n_tiles;
-            const double rows = m_tiles == 1 && cg == 1 ? static_cast<double>(std::min<int64_t>(kRows, (p.M + 7) / 8 * 8)) : kRows;
+            const int rows = rows_of_a(p, cg), stage_size = stage_bytes(p, bn, cg, rows);
             for (int splits = 1; splits <= (cg == 1 ? 8 : 1); splits *= 2) {
                 if (splits > 1 && (bn > 128 || splits > blocks || tiles * splits > sms)) break;
                 const int64_t k_per_split = (blocks + splits - 1) / splits;
@@ -819,8 +830,9 @@ Shape choose_shape(const Problem& p) {
                     halved = tiles % slots;
                     rounds -= 0.45;
                 }
-                const double block = std::max({2.0 * bn, 2.0 * (rows + bn / cg), (rows + bn / cg) * kRowBytes / 48.0});
-                const double clocks = rounds * (k_per_split * block) + 2000.0 + bn * 6.0 + (splits > 1 ? 2500.0 : 0.0) + (cg == 2 ? 500.0 : 0.0);
+                const double in_flight = static_cast<double>(stages_that_fit(stage_size, kSmemBudget - 2 * kStageBox)) * stage_size;
+                const double block = std::max({2.0 * bn, 2.0 * (rows + bn / cg), (rows + bn / cg) * kRowBytes / std::min(48.0, in_flight / 2300.0)});
+                const double clocks = rounds * (k_per_split * block) + 2000.0 + bn * 6.0 + (splits > 1 ? (p.kind == kScaled ? 5000.0 : 2500.0) : 0.0) + (cg == 2 ? 1500.0 : 0.0);
                 if (best.cg == 0 || clocks < best.clocks) best = Shape{cg, bn, splits, static_cast<int>(k_per_split), tiles, halved, clocks};
             }
         }
@@ -855,9 +867,9 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     args.whole_items = static_cast<int>(shape.tiles - shape.halved);
     args.items = static_cast<int>(shape.tiles + shape.halved);
     args.b_box_bytes = (p.b_mn_major ? kRowBytes / p.in_bytes : args.b_box_columns) * kRowBytes;   // N-major: one row of 128 bytes per element of K
-    const int a_rows = args.m_tiles == 1 && shape.cg == 1 ? static_cast<int>(std::min<int64_t>(kRows, (p.M + 7) / 8 * 8)) : kRows;
+    const int a_rows = rows_of_a(p, shape.cg);
     args.a_bytes = a_rows * kRowBytes;
-    args.stage_bytes = kABytes + columns * kRowBytes + (p.kind == kScaled ? 2048 : 0);
+    args.stage_bytes = stage_bytes(p, shape.bn, shape.cg, a_rows);
     args.out = c;
     args.out_ld = p.c_ld;
     args.out_dtype = p.out_dtype;
@@ -867,8 +879,8 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     args.acc_stride = p.kind == kScaled && shape.bn == 256 ? 224 : shape.bn;
     args.scale_columns = 480;
     const int staging = shape.splits > 1 || !args.tma_store ? 0 : 2 * kStageBox, barriers = (2 * kMaxStages + 6) * 8;
-    args.stages = std::min(kMaxStages, (kSmemBudget - staging - barriers) / args.stage_bytes);
-    args.staging_offset = args.stages * args.stage_bytes;
+    args.stages = stages_that_fit(args.stage_bytes, kSmemBudget - staging - barriers);
+    args.staging_offset = ring_bytes(args.stages, args.stage_bytes);   // (a split product parks its 128 x bn partial tile, at most 64 KB, in the ring)
     args.barrier_offset = args.staging_offset + staging;
     const int dynamic = args.barrier_offset + barriers + 1024;
     // instruction descriptor: f32 accumulators (or E8M0 scales), the operand formats the caller has set, B's major, M (N is the item's)

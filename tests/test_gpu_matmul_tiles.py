@@ -1,0 +1,96 @@
+"""The tensor-core matrix kernel at extents that fill no tile: one row or column past and short of the tile edges, one K block and
+remainders of it, each shape of work (two SMs per tile, one SM, clusters that share out K), both layouts of B, every operand
+type, fused steps. Compared with an f64 product of the same stored values.
+
+Tolerances: the products of stored values are exact in f32 and are added in f32, so an element is off by at most K 2^-24
+sum |a b| before C is rounded once: by half a unit in the last of 8 (bf16), 11 (f16) or 24 (f32) significant bits, that is 2^-8,
+2^-11 or 2^-24 relative."""
+import numpy as np
+import pytest
+
+from deepforge_b200 import dfgpu, graphs, runtime
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+TORCH = {"FLOAT": torch.float32, "BFLOAT16": torch.bfloat16, "HALF": torch.float16, "FP8_E4M3": torch.uint8, "FP8_E8M0": torch.uint8}
+ROUNDING = {"FLOAT": 2.0 ** -24, "BFLOAT16": 2.0 ** -8, "HALF": 2.0 ** -11}
+# M, K, N: K and N in 16-byte rows. Single rows; edges of 128 and 256 rows; 64 / 128 / 192 / 256 columns; K of one block, less, more
+EXTENTS = [(1, 16, 16), (1, 4096, 96), (7, 144, 272), (16, 4096, 4096), (64, 8192, 512), (127, 128, 112), (128, 4096, 256), (129, 272, 128), (255, 64, 192),
+           (257, 1040, 400), (777, 2064, 1552), (1500, 528, 3088), (2049, 256, 2064)]
+
+
+def run(doc, buffers):
+    for t in doc["tensors"].values():
+        if not t["is_virtual"] and t["uid"] not in buffers:
+            count, dtype = int(np.prod(t["dim"])), TORCH[t["data_type"]]
+            buffers[t["uid"]] = torch.full((count,), 0x5A if dtype == torch.uint8 else float("nan"), dtype=dtype, device="cuda")
+    exe = runtime.compile_graph(doc)
+    workspace = torch.empty(max(exe.workspace_size, 1), dtype=torch.uint8, device="cuda")
+    exe.execute({uid: b.data_ptr() for uid, b in buffers.items()}, workspace.data_ptr())
+    torch.cuda.synchronize()
+    assert dfgpu.device_status() == 0
+    return exe
+
+
+def close(got, a, b, after, out_type, k):
+    product, weight = a @ b, a.abs() @ b.abs()
+    want = after(product)
+    bound = ROUNDING[out_type] * want.abs() + k * 2.0 ** -24 * weight + 1e-30
+    assert torch.all((got.double() - want).abs() <= bound), float(((got.double() - want).abs() / bound).max())
+
+
+@pytest.mark.parametrize("m,k,n", EXTENTS)
+@pytest.mark.parametrize("io", ["BFLOAT16", "HALF"])
+@pytest.mark.parametrize("b_k_major", [False, True])
+def test_sixteen_bit_operands(m, k, n, io, b_k_major):
+    g = torch.Generator(device="cuda").manual_seed(m * 7 + n)
+    tensors = [graphs.tensor(1, "A", [m, k], io), graphs.tensor(2, "B", [k, n], io, [1, k] if b_k_major else [n, 1]), graphs.tensor(3, "bias", [1, n], io),
+               graphs.tensor(7, "addend", [m, n], io), graphs.tensor(4, "C", [m, n], io), graphs.tensor(5, "p", [m, n], virtual=True), graphs.tensor(6, "q", [m, n], virtual=True),
+               graphs.tensor(8, "r", [m, n], virtual=True)]
+    nodes = [graphs.matmul_node("matmul", 1, 2, 5), graphs.pointwise_node("bias", "ADD", 5, 6, 3), graphs.pointwise_node("relu", "RELU_FWD", 6, 8), graphs.pointwise_node("add", "ADD", 8, 4, 7)]
+    buffers = {uid: torch.randn(count, device="cuda", generator=g).to(TORCH[io]) for uid, count in ((1, m * k), (2, k * n), (3, n), (7, m * n))}
+    exe = run(graphs.document("tiles", nodes, tensors, io=io), buffers)
+    assert exe.launch_count == 1
+    a, b = buffers[1].view(m, k).double(), (buffers[2].view(n, k).t() if b_k_major else buffers[2].view(k, n)).double()
+    close(buffers[4].view(m, n), a, b, lambda p: torch.relu(p + buffers[3].double()) + buffers[7].view(m, n).double(), io, k)
+
+
+@pytest.mark.parametrize("m,k,n", EXTENTS)
+@pytest.mark.parametrize("c_type,b_k_major", [("BFLOAT16", True), ("FLOAT", False), ("HALF", True)])
+def test_fp8_codes(m, k, n, c_type, b_k_major):
+    g = torch.Generator(device="cuda").manual_seed(m * 11 + n)
+    codes = {uid: (torch.randn(count, device="cuda", generator=g) * 16).to(torch.float8_e4m3fn) for uid, count in ((21, m * k), (22, k * n))}
+    scalars = {23: 0.5, 24: 0.25, 25: 0.125}
+    buffers = {uid: c.view(torch.uint8) for uid, c in codes.items()}
+    buffers.update({uid: torch.full((1,), v, device="cuda") for uid, v in scalars.items()})
+    run(graphs.matmul_fp8(m, k, n, c_type, batch=(), b_k_major=b_k_major), buffers)
+    a, b = codes[21].double().view(m, k), (codes[22].double().view(n, k).t() if b_k_major else codes[22].double().view(k, n))
+    if c_type == "HALF":  # (values past the largest f16 become infinities on both sides)
+        assert float((a @ b).abs().max()) * (0.5 * 0.25 * 0.125) < 65504
+    close(buffers[26].view(m, n), a, b, lambda p: p * (0.5 * 0.25 * 0.125), c_type, k)
+    top = float((a @ b).abs().max()) * 0.125
+    assert abs(float(buffers[27][0]) - top) <= k * 2.0 ** -24 * float((a.abs() @ b.abs()).max())
+
+
+@pytest.mark.parametrize("m,k,n", [(m, (k + 31) // 32 * 32, n) for m, k, n in EXTENTS if n > 64])
+def test_block_scaled_codes(m, k, n):
+    g = torch.Generator(device="cuda").manual_seed(m * 13 + n)
+    buffers = {1: torch.randn(m * k, device="cuda", generator=g).to(torch.bfloat16), 2: torch.randn(k * n, device="cuda", generator=g).to(torch.bfloat16)}
+    exe = run(graphs.c3_quantize_matmul(m, k, n), buffers)
+    assert [s["kernel"] for s in exe.steps()][-1] == dfgpu.MATMUL_UMMA_MXF8
+    scale = lambda uid: torch.pow(2.0, buffers[uid].double() - 127)
+    a = buffers[3].view(torch.float8_e4m3fn).double().view(m, k) * scale(4).view(m, k // 32).repeat_interleave(32, 1)
+    b = buffers[5].view(torch.float8_e4m3fn).double().view(k, n) * scale(6).view(k // 32, n).repeat_interleave(32, 0)
+    close(buffers[9].view(m, n), a, b, lambda p: p, "BFLOAT16", k)
+
+
+def test_operands_off_the_sixteen_byte_boundary_fall_back():
+    """Extents that are no whole tiles keep the element's alignment: an operand TMA cannot read goes to the CUDA cores."""
+    m, k, n = 40, 72, 88
+    g = torch.Generator(device="cuda").manual_seed(5)
+    doc = graphs.document("tiles", [graphs.matmul_node("matmul", 1, 2, 4)], [graphs.tensor(1, "A", [m, k], "BFLOAT16"), graphs.tensor(2, "B", [k, n], "BFLOAT16"), graphs.tensor(4, "C", [m, n], "BFLOAT16")], io="BFLOAT16")
+    a, b = (torch.randn(count + 1, device="cuda", generator=g).to(torch.bfloat16)[1:] for count in (m * k, k * n))
+    buffers = {1: a, 2: b}
+    run(doc, buffers)
+    close(buffers[4].view(m, n), a.view(m, k).double(), b.view(k, n).double(), lambda p: p, "BFLOAT16", k)
