@@ -796,7 +796,9 @@ extern "C" int dfgpu_sdpa_forward(const dfgpu_sdpa_params* p, void* const* tenso
         if (status) return status;
         a.prefix_ok = prefix_ok;
     }
-    if (kernel == DFGPU_SDPA_UMMA) return launch_sdpa_umma(*p, tensors, scratch, stream);
+    // (AUTO: operands off the 16-byte boundary TMA needs go to the general kernel)
+    if (kernel == DFGPU_SDPA_UMMA && p->kernel == DFGPU_SDPA_AUTO && !(aligned16(a.q_data) && aligned16(a.k_data) && aligned16(a.v_data) && aligned16(a.o_data))) kernel = DFGPU_SDPA_ROWWISE;
+    if (kernel == DFGPU_SDPA_UMMA) return launch_sdpa_umma(*p, tensors, stream);
     if (kernel == DFGPU_SDPA_PAGED_DECODE_UMMA) {
         if (!scratch || !aligned16(scratch)) return fail(kInvalidArgument, "SDPA: the paged decode kernel needs its 16-byte aligned scratch buffer");
         status = launch_decode_umma(*p, tensors, scratch, a.prefix_ok, stream);

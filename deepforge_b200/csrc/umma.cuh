@@ -76,9 +76,9 @@ bool matmul_fp8_tiles_supported(const dfgpu_matmul_fp8_params& p);  // everythin
 int launch_matmul_fp8_umma(const dfgpu_matmul_fp8_params& p, void* const* tensors, cudaStream_t stream);
 int matmul_tiles_device_status(int* status);
 
-// SDPA forward on tcgen05 (bf16, head dim 128, contiguous K/V).
+// SDPA forward on tcgen05 (bf16 or f16, head dimension 64 or 128, any lengths, causal and padding masks).
 bool sdpa_umma_supported(const dfgpu_sdpa_params& p);
-int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, void* scratch, cudaStream_t stream);
+int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, cudaStream_t stream);
 int sdpa_umma_device_status(int* status);  // reads and clears that unit's status word
 
 // Paged-KV decode on TMA + tcgen05 (bf16, head dim 128, Sq = 1); partials go to `scratch`, the

@@ -1,18 +1,20 @@
-// SDPA forward on the 5th-generation tensor cores (bf16, head dim 128, contiguous K/V).
+// SDPA forward on the 5th-generation tensor cores: bf16 or f16, head dimension 64 or 128, any sequence lengths, grouped heads,
+// causal (top-left) and padding masks.
 //
-// One CTA owns a 128-row query tile of one (batch, head) and walks the key/value tiles of 128:
-//   warp 0     TMA producer: Q once, then K_0, V_0, K_1, V_1, ... into a ring of 32 KiB slots
-//   warp 1     one lane issues S_j = Q K_j^T into one of two TMEM score buffers (so S_{j+1} is
-//              multiplied while the softmax warps work on S_j) and O += P_j V_j into the TMEM
-//              output accumulator
-//   warps 2-5  softmax, one query row per thread: tcgen05.ld the scores, running max / sum in the
-//              exp2 domain, P_j as bf16 into a swizzled shared-memory tile (the A operand of the
-//              second product), final 1/sum, O and Stats stores.
 // The running maximum is only raised when it grows by more than 2^8 (the accumulator is rescaled
 // in TMEM then, which is rare); Stats = ln2 * (m + log2(l)) is exact whichever reference m is
 // in use. Causal graphs skip tiles above the diagonal and mask inside the diagonal tile.
 // Scores are scaled after the f32 dot product, invalid positions are -inf, as in the reference's
 // emit_sdpa_forward (lib/Compiler/SequenceGraph.cpp:2135-2341).
+//
+// Lengths are free because the copies are: Q, K, V and O are rank-4 tensor maps (channel, position, head, batch), so TMA fills
+// the positions past the end with zeros and clips them on the store, and what is left is a mask on the last key tile. With
+// SEQ_LEN_Q / SEQ_LEN_KV a batch's key tiles end at its own length, V rows behind it are cleared in shared memory (a zero
+// probability times an infinity in the padding would be NaN), and rows past SEQ_LEN_Q store 0 and -inf. 4 x 16 heads of 1000
+// padded positions, causal: 9.7 ms on the row-at-a-time kernel.
+#include <algorithm>
+#include <cmath>
+
 #include "umma_ptx.cuh"
 
 namespace dfgpu {
@@ -20,37 +22,26 @@ namespace {
 
 constexpr int kRows = 128;      // query rows per CTA
 constexpr int kKeys = 128;      // keys per tile
-constexpr int kHeadDim = 128;
-constexpr int kTileBytes = kRows * kHeadDim * 2;  // 32 KiB: one Q / K / V / P tile (two 64-column halves)
-constexpr int kHalfBytes = kTileBytes / 2;
-constexpr int kSlots = 3;       // K/V ring
-constexpr int kSdpaThreads = 192;
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 
 struct SdpaUmmaArgs {
     int32_t heads_q, heads_kv, seq_q, seq_kv;
-    int32_t q_tiles;
+    int32_t q_tiles, pairs;   // 128-row query tiles and pairs of them, the last one perhaps partly past the end
     int32_t causal;
-    float scale_log2;  // attn_scale * log2(e)
+    int32_t paired_units;     // causal: a unit of work is a heavy and a light pair (see PairWalker)
+    float scale_log2;  // |attn_scale| * log2(e); a negative scale negates Q in the products
+    uint32_t negate_q; // ... through this bit of the instruction descriptor
+    const int32_t* len_q;   // SEQ_LEN_Q and SEQ_LEN_KV by batch, or null
+    const int32_t* len_kv;
+    int64_t len_q_stride, len_kv_stride;
     float* stats;      // [B, Hq, Sq] or null
     int64_t stats_batch_stride, stats_head_stride, stats_row_stride;
-    // Max and Sum_exp rows (two-tile kernel only), or null; element strides like Stats
+    // Max and Sum_exp rows, or null; element strides like Stats
     float* row_max;
     float* row_sum;
     int64_t max_stride[3], sum_stride[3];
-    float attn_scale;  // natural-log units: Max = attn_scale * largest dot product
-    int32_t batch_heads;  // two-tile kernel: batch * query heads
-};
-
-struct Smem {
-    static constexpr int kQ = 0;
-    static constexpr int kRing = kTileBytes;
-    static constexpr int kP = kRing + kSlots * kTileBytes;
-    static constexpr int kBarriers = kP + 2 * kTileBytes;
-    // q_full, kv_full[3], kv_empty[3], s_full[2], s_empty[2], p_full[2], pv_done[2]
-    static constexpr int kBarrierCount = 1 + 2 * kSlots + 8;
-    static constexpr int kTotal = kBarriers + kBarrierCount * 8 + 16;
-    static constexpr int kDynamic = kTotal + 1024;
+    float attn_scale;  // |attn_scale|, natural-log units: Max = attn_scale * largest dot product
+    int32_t batch_heads;  // batch * query heads
 };
 
 __device__ __forceinline__ void tmem_store_32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -73,248 +64,6 @@ __device__ __forceinline__ void tmem_store_16(uint32_t taddr, const uint32_t (&r
 }
 __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-__global__ void __launch_bounds__(kSdpaThreads, 1)
-sdpa_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                 const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o, SdpaUmmaArgs args) {
-    extern __shared__ uint8_t smem_raw[];
-    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    uint8_t* generic_base = smem_raw + (smem_base - smem_u32(smem_raw));
-    const uint32_t bar_base = smem_base + Smem::kBarriers;
-    const uint32_t q_full = bar_base;
-    auto kv_full = [&](int s) { return bar_base + 8u * (1 + s); };
-    auto kv_empty = [&](int s) { return bar_base + 8u * (1 + kSlots + s); };
-    auto s_full = [&](int b) { return bar_base + 8u * (1 + 2 * kSlots + b); };
-    auto s_empty = [&](int b) { return bar_base + 8u * (3 + 2 * kSlots + b); };
-    auto p_full = [&](int b) { return bar_base + 8u * (5 + 2 * kSlots + b); };
-    auto pv_done = [&](int b) { return bar_base + 8u * (7 + 2 * kSlots + b); };
-    const uint32_t tmem_slot = bar_base + 8u * Smem::kBarrierCount;
-    volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(generic_base + Smem::kBarriers + 8 * Smem::kBarrierCount);
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // heavy (late) causal tiles first
-    const int q_tile = args.q_tiles - 1 - static_cast<int>(blockIdx.x);
-    const int bh = blockIdx.y;
-    const int batch = bh / args.heads_q, head = bh - batch * args.heads_q;
-    const int kv_head = head / (args.heads_q / args.heads_kv);
-    const int q_row0 = (batch * args.heads_q + head) * args.seq_q + q_tile * kRows;
-    const int kv_row0 = (batch * args.heads_kv + kv_head) * args.seq_kv;
-    const int total_kv_tiles = args.seq_kv / kKeys;
-    const int kv_tiles = args.causal ? min(total_kv_tiles, q_tile + 1) : total_kv_tiles;
-
-    if (threadIdx.x == 0) {
-        mbar_init(q_full, 1);
-        for (int s = 0; s < kSlots; ++s) {
-            mbar_init(kv_full(s), 1);
-            mbar_init(kv_empty(s), 1);
-        }
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(s_full(b), 1);
-            mbar_init(s_empty(b), 4);
-            mbar_init(p_full(b), 4);
-            mbar_init(pv_done(b), 1);
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 1) {
-        tmem_alloc(tmem_slot, 512);
-        tmem_relinquish();
-        tc_fence_before();
-    }
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot_ptr;
-    chain_wait();
-    chain_release();
-    const uint32_t tmem_o = tmem_base + 256;  // S0 at +0, S1 at +128, O at +256
-
-    if (warp == 0) {
-        if (lane == 0) {
-            mbar_expect_tx(q_full, kTileBytes);
-            tma_load_2d(smem_base + Smem::kQ, &map_q, 0, q_row0, q_full);
-            tma_load_2d(smem_base + Smem::kQ + kHalfBytes, &map_q, 64, q_row0, q_full);
-            for (int t = 0; t < 2 * kv_tiles; ++t) {
-                const int slot = t % kSlots;
-                if (!mbar_wait(kv_empty(slot), ((t / kSlots) & 1) ^ 1, 201)) break;
-                const CUtensorMap* map = (t & 1) ? &map_v : &map_k;
-                const int row = kv_row0 + (t >> 1) * kKeys;
-                const uint32_t dst = smem_base + Smem::kRing + slot * kTileBytes;
-                mbar_expect_tx(kv_full(slot), kTileBytes);
-                tma_load_2d(dst, map, 0, row, kv_full(slot));
-                tma_load_2d(dst + kHalfBytes, map, 64, row, kv_full(slot));
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            // D f32, A/B bf16, M = 128, N = 128; the second product reads V as an MN-major B operand
-            const uint32_t idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kKeys >> 3) << 17) | (static_cast<uint32_t>(kRows >> 4) << 24);
-            const uint32_t idesc_pv = idesc_qk | (1u << 16);
-            const uint32_t q_smem = smem_base + Smem::kQ;
-            bool ok = mbar_wait(q_full, 0, 202);
-            auto issue_scores = [&](int j) {
-                const int t = 2 * j, slot = t % kSlots, b = j & 1;
-                if (ok) ok = mbar_wait(kv_full(slot), (t / kSlots) & 1, 203);
-                if (ok) ok = mbar_wait(s_empty(b), ((j >> 1) & 1) ^ 1, 204);
-                tc_fence_after();
-                if (ok) {
-                    const uint32_t q_lo = smem_desc_lo(q_smem, 16), k_lo = smem_desc_lo(smem_base + Smem::kRing + slot * kTileBytes, 16);
-#pragma unroll
-                    for (int k = 0; k < kHeadDim / 16; ++k) {
-                        const uint32_t offset = ((k >> 2) * kHalfBytes + (k & 3) * 32) >> 4;
-                        umma_bf16(tmem_base + b * 128, desc_words(q_lo + offset, smem_desc_hi(1024)), desc_words(k_lo + offset, smem_desc_hi(1024)), idesc_qk, k != 0 ? 1u : 0u);
-                    }
-                }
-                umma_commit(kv_empty(slot));
-                umma_commit(s_full(b));
-            };
-            issue_scores(0);
-            for (int j = 0; j < kv_tiles; ++j) {
-                if (j + 1 < kv_tiles) issue_scores(j + 1);
-                const int t = 2 * j + 1, slot = t % kSlots, b = j & 1;
-                if (ok) ok = mbar_wait(p_full(b), (j >> 1) & 1, 205);
-                if (ok) ok = mbar_wait(kv_full(slot), (t / kSlots) & 1, 206);
-                tc_fence_after();
-                if (ok) {
-                    const uint32_t p_lo = smem_desc_lo(smem_base + Smem::kP + b * kTileBytes, 16);
-                    const uint32_t v_lo = smem_desc_lo(smem_base + Smem::kRing + slot * kTileBytes, kHalfBytes);
-#pragma unroll
-                    for (int k = 0; k < kKeys / 16; ++k)
-                        umma_bf16(tmem_o, desc_words(p_lo + (((k >> 2) * kHalfBytes + (k & 3) * 32) >> 4), smem_desc_hi(1024)),
-                                  desc_words(v_lo + ((k * 2048) >> 4), smem_desc_hi(1024)), idesc_pv, (j | k) != 0 ? 1u : 0u);
-                }
-                umma_commit(kv_empty(slot));
-                umma_commit(pv_done(b));
-            }
-        }
-    } else {
-        const int quadrant = warp & 3;
-        const int row = quadrant * 32 + lane;
-        const uint32_t lane_base = static_cast<uint32_t>(quadrant * 32) << 16;
-        const int q_index = q_tile * kRows + row;  // query position inside the sequence
-        float m_ref = -INFINITY;  // reference maximum (scaled, log2 domain)
-        float l_sum = 0.0f;
-        bool ok = true;
-        for (int j = 0; j < kv_tiles; ++j) {
-            const int b = j & 1;
-            if (ok) ok = mbar_wait(s_full(b), (j >> 1) & 1, 207);
-            tc_fence_after();
-            float s[128];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                uint32_t raw[32];
-                tmem_load_32(tmem_base + lane_base + b * 128 + c * 32, raw);
-                tmem_load_wait();
-#pragma unroll
-                for (int e = 0; e < 32; ++e) s[c * 32 + e] = __uint_as_float(raw[e]) * args.scale_log2;
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(s_empty(b));
-            if (args.causal && j == q_tile) {
-                const int limit = q_index - j * kKeys;  // keys 0..limit of this tile are visible
-#pragma unroll
-                for (int e = 0; e < 128; ++e)
-                    if (e > limit) s[e] = -INFINITY;
-            }
-            float tile_max = s[0];
-#pragma unroll
-            for (int e = 1; e < 128; ++e) tile_max = fmaxf(tile_max, s[e]);
-            // raise the reference only when it would grow by more than the threshold (or on the first tile)
-            const bool raise = tile_max > m_ref + kRescaleThreshold;
-            const bool any_raise = __any_sync(0xffffffffu, raise) != 0;
-            if (any_raise) {
-                const float m_new = fmaxf(m_ref, tile_max);
-                const float alpha = m_ref == -INFINITY ? 0.0f : exp2f(m_ref - m_new);
-                l_sum *= alpha;
-                m_ref = m_new;
-                if (j > 0) {
-                    // the accumulator holds P V up to tile j-1: wait for that product, then rescale it in TMEM
-                    if (ok) ok = mbar_wait(pv_done((j - 1) & 1), ((j - 1) >> 1) & 1, 208);
-                    tc_fence_after();
-#pragma unroll 1
-                    for (int c = 0; c < 4; ++c) {
-                        uint32_t raw[32];
-                        tmem_load_32(tmem_o + lane_base + c * 32, raw);
-                        tmem_load_wait();
-#pragma unroll
-                        for (int e = 0; e < 32; ++e) raw[e] = __float_as_uint(__uint_as_float(raw[e]) * alpha);
-                        tmem_store_32(tmem_o + lane_base + c * 32, raw);
-                    }
-                    tmem_store_wait();
-                    tc_fence_before();
-                }
-            }
-            // P buffer b was last read by the product of tile j-2
-            if (ok) ok = mbar_wait(pv_done(b), ((j >> 1) & 1) ^ 1, 209);
-            uint8_t* p_row = generic_base + Smem::kP + b * kTileBytes + row * 128;
-            float tile_sum = 0.0f;
-#pragma unroll
-            for (int c = 0; c < 16; ++c) {  // 16-byte units: 8 keys each
-                uint32_t w[4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const float p0 = exp2f(s[c * 8 + 2 * t] - m_ref);
-                    const float p1 = exp2f(s[c * 8 + 2 * t + 1] - m_ref);
-                    tile_sum += p0 + p1;
-                    __nv_bfloat162 pair = __floats2bfloat162_rn(p0, p1);
-                    w[t] = *reinterpret_cast<uint32_t*>(&pair);
-                }
-                const int half = c >> 3, unit = c & 7;
-                *reinterpret_cast<uint4*>(p_row + half * kHalfBytes + ((unit ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-            }
-            l_sum += tile_sum;
-            fence_async_shared();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(p_full(b));
-        }
-        // last product done -> normalise, store O through shared memory and the TMA unit
-        const int last = kv_tiles - 1;
-        if (ok) ok = mbar_wait(pv_done(last & 1), (last >> 1) & 1, 210);
-        tc_fence_after();
-        const float inverse = l_sum > 0.0f ? 1.0f / l_sum : 0.0f;
-        uint8_t* o_row = generic_base + Smem::kP + row * 128;  // P buffer 0 doubles as the output staging tile
-        // P buffer 0 may still be the operand of the last product only if last is even: that product is done (waited above)
-#pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-            uint32_t raw[32];
-            tmem_load_32(tmem_o + lane_base + c * 32, raw);
-            tmem_load_wait();
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                uint32_t w[4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    __nv_bfloat162 pair = __floats2bfloat162_rn(__uint_as_float(raw[u * 8 + 2 * t]) * inverse, __uint_as_float(raw[u * 8 + 2 * t + 1]) * inverse);
-                    w[t] = *reinterpret_cast<uint32_t*>(&pair);
-                }
-                const int unit16 = c * 4 + u;  // 16-byte unit inside the 256-byte output row
-                const int half = unit16 >> 3, unit = unit16 & 7;
-                *reinterpret_cast<uint4*>(o_row + half * kHalfBytes + ((unit ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-            }
-        }
-        if (args.stats != nullptr && ok)
-            args.stats[batch * args.stats_batch_stride + head * args.stats_head_stride + static_cast<int64_t>(q_index) * args.stats_row_stride] =
-                l_sum > 0.0f ? 0.6931471805599453f * (m_ref + log2f(l_sum)) : -INFINITY;
-        tc_fence_before();
-        fence_async_shared();
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (warp == 2 && lane == 0) {
-            if (ok && g_device_status == 0) {
-                tma_store_2d(&map_o, smem_base + Smem::kP, 0, q_row0);
-                tma_store_2d(&map_o, smem_base + Smem::kP + kHalfBytes, 64, q_row0);
-            }
-            tma_store_commit();
-            tma_store_wait_all();
-        }
-    }
-
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 1) {
-        tc_fence_after();
-        tmem_dealloc(tmem_base, 512);
-    }
-}
-
 // ---- two query tiles per CTA ------------------------------------------------------
 // The softmax of one tile costs about as many cycles as its two products, so a CTA that owns two
 // 128-row query tiles (A and B) lets the tensor pipe work on one while the other is in its softmax:
@@ -324,7 +73,7 @@ sdpa_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 //   warps 0-7   softmax of tile A, warps 8-15 softmax of tile B (four whole warpgroups, which take the registers the
 //               loader and issuing warps give up): two threads per query row, each with 64 of the
 //               tile's 128 keys (the two warps that share a lane quarter trade row maxima through shared memory)
-// TMEM: S_A at +0, S_B at +128, O_A at +256, O_B at +384. P never goes through shared memory: each
+// (D is the head dimension.) TMEM: S_A at +0, S_B at +128, O_A at +256, O_B at +384. P never goes through shared memory: each
 // thread overwrites the front of its own score row with the bf16 probabilities (two per 32-bit
 // column) and the second product takes its A operand from tensor memory. The tensor pipe runs the
 // products of one CTA in issue order, so S_X(j+1) may be issued right behind the product that reads P_X(j).
@@ -334,19 +83,27 @@ constexpr int kPairSlots = 4;
 constexpr int kPolyEvery = 4;  // one pair of exponentials in kPolyEvery goes to the FMA pipe (0: none)
 constexpr int kPairThreads = 608;  // 2 x 8 softmax warps (two threads per query row), loader, issuer and output-store warps
 
+template <int D>
 struct PairSmem {
+    static constexpr int kTile = kRows * D * 2;         // one Q / K / V / O tile: D / 64 boxes of 128 rows x 64 channels
     static constexpr int kQ = 0;                       // Q_A, Q_B
-    static constexpr int kRing = 2 * kTileBytes;
-    static constexpr int kStage = kRing + kPairSlots * kTileBytes;  // one output tile on its way to global memory
+    static constexpr int kRing = 2 * kTile;
+    static constexpr int kStage = kRing + kPairSlots * kTile;  // one output tile on its way to global memory
     // 128 bytes per (tile, lane quarter): during the key loop the half-row maxima [half][lane] as bf16, after it the row sum
     // [lane] as f32. 1 KiB in all: with two Q tiles, four 32 KiB ring slots and the output tile this is what the 227 KiB leave.
-    static constexpr int kExchange = kStage + kTileBytes;
+    static constexpr int kExchange = kStage + kTile;
     static constexpr int kBarriers = kExchange + 1024;
     // stage_free, q_full[2], q_empty[2], kv_full[S], kv_empty[S], s_full[2], p_full[2], o_full[2], o_empty[2], staged[2]
     static constexpr int kBarrierCount = 5 + 2 * kPairSlots + 10;
     static constexpr int kTotal = kBarriers + kBarrierCount * 8 + 16;
     static constexpr int kDynamic = kTotal + 1024;
 };
+constexpr int kHalfBytes = kRows * 128;   // one box
+
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+                 ::"l"(map), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
 
 // D[tmem] (+)= A[tmem] * B[smem]: the A operand (bf16 pairs, one row per lane) is read from tensor memory.
 __device__ __forceinline__ void umma_bf16_a_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
@@ -442,7 +199,18 @@ __device__ __forceinline__ float max_of_16(const uint32_t (&raw)[16], float runn
         part[g] = max3(__uint_as_float(raw[4 * g]), __uint_as_float(raw[4 * g + 1]), max3(__uint_as_float(raw[4 * g + 2]), __uint_as_float(raw[4 * g + 3]), running));
     return fmaxf(fmaxf(part[0], part[1]), fmaxf(part[2], part[3]));
 }
-// Sixteen scores -> probabilities 2^(s * scale + bias) as eight bf16 pairs, their sum added to two packed partial sums.
+template <bool F16>
+__device__ __forceinline__ uint32_t pack_pair(float lo, float hi) {
+    if constexpr (F16) {
+        const __half2 two = __floats2half2_rn(lo, hi);
+        return *reinterpret_cast<const uint32_t*>(&two);
+    } else {
+        const __nv_bfloat162 two = __floats2bfloat162_rn(lo, hi);
+        return *reinterpret_cast<const uint32_t*>(&two);
+    }
+}
+// Sixteen scores -> probabilities 2^(s * scale + bias) as eight bf16 or f16 pairs, their sum added to two packed partial sums.
+template <bool F16>
 __device__ __forceinline__ void probabilities_of_16(const uint32_t (&raw)[16], uint64_t scale2, uint64_t bias2, uint64_t (&sums)[2], uint32_t* packed) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
@@ -457,43 +225,53 @@ __device__ __forceinline__ void probabilities_of_16(const uint32_t (&raw)[16], u
             p1 = ex2_fast(x1);
         }
         sums[e & 1] = add2(sums[e & 1], pack2(p0, p1));
-        __nv_bfloat162 two = __floats2bfloat162_rn(p0, p1);
-        packed[e] = *reinterpret_cast<uint32_t*>(&two);
+        packed[e] = pack_pair<F16>(p0, p1);
     }
 }
 
-// One (batch, head, query pair) of the two-tile kernel's work list.
+// One (batch, head, query pair) of the work list.
 struct PairItem {
-    int batch, head;
+    int batch, head, kv_head;
     int q_tile_a;        // index of the first of the two 128-row query tiles
-    int q_row_a;         // its first row in the [B * Hq * Sq, D] view of Q and O
-    int kv_row0;         // first row of this head in the [B * Hkv * Skv, D] view of K and V
-    int tiles_a, tiles_b;  // key tiles the two query tiles walk (causal: up to their diagonals)
+    int tiles_a, tiles_b;  // key tiles the two query tiles walk (up to their diagonals and the batch's length), at least one
+    int tiles;           // ... the larger of them: key tiles that are loaded
+    int kv_len;          // keys of this batch, at least one
+    int live_q;          // query rows before this one have keys; the others store 0 and -inf
 };
 
 __device__ __forceinline__ PairItem pair_item(const SdpaUmmaArgs& args, int bh, int pair) {
     PairItem item;
     item.batch = bh / args.heads_q;
     item.head = bh - item.batch * args.heads_q;
-    const int kv_head = item.head / (args.heads_q / args.heads_kv);
+    item.kv_head = item.head / (args.heads_q / args.heads_kv);
     item.q_tile_a = 2 * pair;
-    item.q_row_a = bh * args.seq_q + item.q_tile_a * kRows;
-    item.kv_row0 = (item.batch * args.heads_kv + kv_head) * args.seq_kv;
-    const int total_kv_tiles = args.seq_kv / kKeys;
-    item.tiles_a = args.causal ? min(total_kv_tiles, item.q_tile_a + 1) : total_kv_tiles;
-    item.tiles_b = args.causal ? min(total_kv_tiles, item.q_tile_a + 2) : total_kv_tiles;
+    item.kv_len = args.seq_kv;
+    item.live_q = args.seq_q;
+    if (args.len_q != nullptr) {
+        const int len_kv = __ldg(args.len_kv + item.batch * args.len_kv_stride);
+        item.live_q = len_kv > 0 ? min(item.live_q, __ldg(args.len_q + item.batch * args.len_q_stride)) : 0;
+        item.kv_len = max(1, min(item.kv_len, len_kv));
+    }
+    const int kv_tiles = (item.kv_len + kKeys - 1) / kKeys;
+    auto tiles_of = [&](int q_tile) {
+        if (q_tile * kRows >= item.live_q) return 1;
+        return args.causal ? min(kv_tiles, q_tile + 1) : kv_tiles;
+    };
+    item.tiles_a = tiles_of(item.q_tile_a);
+    item.tiles_b = tiles_of(item.q_tile_a + 1);
+    item.tiles = max(item.tiles_a, item.tiles_b);
     return item;
 }
 
 // The work list of one CTA, the same in every warp role. A head's P query pairs form units: under a causal mask unit i
 // is the heavy pair P-1-i followed by the light pair i, so that every unit walks 2P+2 key tiles and equal numbers of
-// units are equal work; otherwise each pair is a unit. CTA c takes units c, c + gridDim.x, ...; neighbouring CTAs
-// thus work on the same head at the same time and share its K and V in L2. `body(bh, pair)` returns false to stop.
+// units are equal work; otherwise, or when the single pairs fit the SMs at once, each pair is a unit. CTA c takes units c,
+// c + gridDim.x, ...; neighbouring CTAs thus work on the same head at the same time and share its K and V in L2.
 struct PairWalker {
     int k = 0;
     __device__ __forceinline__ bool next(const SdpaUmmaArgs& args, int& bh, int& pair) {
-        const int pairs = args.q_tiles >> 1;
-        const int units_per_head = args.causal ? (pairs + 1) >> 1 : pairs;
+        const int pairs = args.pairs;
+        const int units_per_head = args.paired_units ? (pairs + 1) >> 1 : pairs;
         const int units = units_per_head * args.batch_heads;
         for (;; ++k) {
             const int unit = static_cast<int>(blockIdx.x) + (k >> 1) * static_cast<int>(gridDim.x);
@@ -501,7 +279,7 @@ struct PairWalker {
             bh = unit / units_per_head;
             const int i = unit - bh * units_per_head;
             pair = i;
-            if (args.causal) {
+            if (args.paired_units) {
                 pair = (k & 1) ? i : pairs - 1 - i;
                 if ((k & 1) && 2 * i == pairs - 1) continue;  // the middle pair of an odd count stands alone
             } else if (k & 1) {
@@ -528,13 +306,16 @@ __device__ __forceinline__ void for_each_pair_item(const SdpaUmmaArgs& args, Bod
 //   warp 17     issues the products; one elected lane issues, all lanes walk the schedule
 //   warp 18     sends staged output tiles to global memory by TMA (row-per-thread global stores of 16 bytes at a
 //               256-byte stride kept the load/store unit busy for ~5000 cycles per tile)
+template <int D, bool F16>
 __global__ void __launch_bounds__(kPairThreads, 1)
 sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o, SdpaUmmaArgs args) {
+    using Smem = PairSmem<D>;
+    constexpr int kTileBytes = Smem::kTile;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* generic_base = smem_raw + (smem_base - smem_u32(smem_raw));
-    const uint32_t bar_base = smem_base + PairSmem::kBarriers;
+    const uint32_t bar_base = smem_base + Smem::kBarriers;
     const uint32_t stage_free = bar_base;
     auto q_full = [&](int x) { return bar_base + 8u * (1 + x); };
     auto q_empty = [&](int x) { return bar_base + 8u * (3 + x); };
@@ -545,8 +326,8 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     auto o_full = [&](int x) { return bar_base + 8u * (9 + 2 * kPairSlots + x); };
     auto o_empty = [&](int x) { return bar_base + 8u * (11 + 2 * kPairSlots + x); };
     auto staged = [&](int x) { return bar_base + 8u * (13 + 2 * kPairSlots + x); };
-    const uint32_t tmem_slot = bar_base + 8u * PairSmem::kBarrierCount;
-    volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(generic_base + PairSmem::kBarriers + 8 * PairSmem::kBarrierCount);
+    const uint32_t tmem_slot = bar_base + 8u * Smem::kBarrierCount;
+    volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(generic_base + Smem::kBarriers + 8 * Smem::kBarrierCount);
 
     const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -588,6 +369,10 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         uint32_t n = 0;      // items started
         for_each_pair_item(args, [&](int bh, int pair) {
             const PairItem item = pair_item(args, bh, pair);
+            auto load_box = [&](uint32_t dst, const CUtensorMap* map, int row, int head, uint32_t bar) {
+#pragma unroll
+                for (int h = 0; h < D / 64; ++h) tma_load_4d(dst + h * kHalfBytes, map, 64 * h, row, head, item.batch, bar);
+            };
             // a Q buffer is free once the previous item's last score product of that query tile has completed; tile A's
             // (which under a causal mask ends a key tile earlier) and the first K tile go first, so that the issuing warp
             // can start this item's tile A under the previous item's last round
@@ -595,22 +380,18 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 if (!mbar_wait_warp(q_empty(x), (n & 1) ^ 1, 220 + x)) return false;
                 if (leader) {
                     mbar_expect_tx(q_full(x), kTileBytes);
-                    tma_load_2d(smem_base + PairSmem::kQ + x * kTileBytes, &map_q, 0, item.q_row_a + x * kRows, q_full(x));
-                    tma_load_2d(smem_base + PairSmem::kQ + x * kTileBytes + kHalfBytes, &map_q, 64, item.q_row_a + x * kRows, q_full(x));
+                    load_box(smem_base + Smem::kQ + x * kTileBytes, &map_q, (item.q_tile_a + x) * kRows, item.head, q_full(x));
                 }
                 return true;
             };
             if (!load_q(0)) return false;
-            for (int t = 0; t < 2 * item.tiles_b; ++t) {
+            for (int t = 0; t < 2 * item.tiles; ++t) {
                 if (t == 1 && !load_q(1)) return false;
                 if (!mbar_wait_warp(kv_empty(slot), phase, 215)) return false;
-                const int row = item.kv_row0 + (t >> 1) * kKeys;
-                const uint32_t dst = smem_base + PairSmem::kRing + slot * kTileBytes;
+                const uint32_t dst = smem_base + Smem::kRing + slot * kTileBytes;
                 if (leader) {
-                    const CUtensorMap* map = (t & 1) ? &map_v : &map_k;
                     mbar_expect_tx(kv_full(slot), kTileBytes);
-                    tma_load_2d(dst, map, 0, row, kv_full(slot));
-                    tma_load_2d(dst + kHalfBytes, map, 64, row, kv_full(slot));
+                    load_box(dst, (t & 1) ? &map_v : &map_k, (t >> 1) * kKeys, item.kv_head, kv_full(slot));
                 }
                 if (++slot == kPairSlots) { slot = 0; phase ^= 1; }
             }
@@ -620,8 +401,10 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     } else if (warp == 17) {
         // All 32 lanes walk the schedule; the elected lane issues the products and their commits.
         const bool leader = elect_one();
-        const uint32_t idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kKeys >> 3) << 17) | (static_cast<uint32_t>(kRows >> 4) << 24);
-        const uint32_t idesc_pv = idesc_qk | (1u << 16);  // B = V read MN-major
+        // f32 accumulators, bf16 (1) or f16 (0) operands, N, M; the second product reads V MN-major
+        constexpr uint32_t kFormats = (1u << 4) | (F16 ? 0u : (1u << 7) | (1u << 10)) | (static_cast<uint32_t>(kRows >> 4) << 24);
+        const uint32_t idesc_qk = kFormats | (static_cast<uint32_t>(kKeys >> 3) << 17) | args.negate_q;
+        constexpr uint32_t idesc_pv = kFormats | (static_cast<uint32_t>(D >> 3) << 17) | (1u << 16);
         const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
         bool ok = true;
         int slot = 0;         // ring slot of the next K or V tile to consume
@@ -637,12 +420,12 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         constexpr uint32_t kDescHi = smem_desc_hi(1024);
         auto scores = [&](int x, int k_slot) {  // S_x = Q_x K^T
             if (!ok) return;
-            const uint32_t q_lo = smem_desc_lo(smem_base + PairSmem::kQ + x * kTileBytes, 16);
-            const uint32_t k_lo = smem_desc_lo(smem_base + PairSmem::kRing + k_slot * kTileBytes, 16);
+            const uint32_t q_lo = smem_desc_lo(smem_base + Smem::kQ + x * kTileBytes, 16);
+            const uint32_t k_lo = smem_desc_lo(smem_base + Smem::kRing + k_slot * kTileBytes, 16);
             const uint32_t d_tmem = tmem_u + x * 128;
             if (leader) {
 #pragma unroll
-                for (int k = 0; k < kHeadDim / 16; ++k) {
+                for (int k = 0; k < D / 16; ++k) {
                     const uint32_t offset = ((k >> 2) * kHalfBytes + (k & 3) * 32) >> 4;  // in 16-byte units
                     umma_bf16(d_tmem, desc_words(q_lo + offset, kDescHi), desc_words(k_lo + offset, kDescHi), idesc_qk, k != 0 ? 1u : 0u);
                 }
@@ -657,7 +440,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             ++p_count[x];
             tc_fence_after();
             if (!ok) return;
-            const uint32_t v_lo = smem_desc_lo(smem_base + PairSmem::kRing + v_slot * kTileBytes, kHalfBytes);
+            const uint32_t v_lo = smem_desc_lo(smem_base + Smem::kRing + v_slot * kTileBytes, kHalfBytes);
             const uint32_t d_tmem = tmem_u + 256 + x * 128, p_tmem = tmem_u + x * 128;
             if (leader) {
 #pragma unroll
@@ -672,7 +455,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         int early_slot = 0;  // the ring slot of its K tile
         while (have && ok) {
             const PairItem item = pair_item(args, bh, pair);
-            const int tiles_a = item.tiles_a, tiles_b = item.tiles_b;
+            const int tiles_a = item.tiles_a, tiles_b = item.tiles_b, tiles = item.tiles;
             const bool have_next = walker.next(args, next_bh, next_pair);
             const int next_tiles_a = have_next ? pair_item(args, next_bh, next_pair).tiles_a : 0;
             int k0_slot = early_slot;
@@ -691,14 +474,14 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             commit(s_full(1));
             commit(kv_empty(k0_slot));
             if (tiles_b == 1) commit(q_empty(1));
-            for (int j = 0; j < tiles_b; ++j) {
+            for (int j = 0; j < tiles; ++j) {
                 wait_slot(226);
                 const int v_slot = slot;
                 next_slot();
                 if (j < tiles_a) {
                     product(0, j, v_slot);
                     if (j == tiles_a - 1) commit(o_full(0));
-                } else if (have_next && ok && j == tiles_b - 1) {
+                } else if (have_next && ok && j == tiles - 1) {
                     // Tile A has no key tile in this item's last round (causal mask): if the next item's Q_A and first K
                     // tile have landed, its first scores go out now and its softmax runs under tile B's last round.
                     const bool landed = __all_sync(0xffffffffu, mbar_test_wait(q_full(0), (n + 1) & 1)) && __all_sync(0xffffffffu, mbar_test_wait(kv_full(slot), phase));
@@ -711,7 +494,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                         if (next_tiles_a == 1) commit(q_empty(0));
                     }
                 }
-                const bool more = j + 1 < tiles_b;
+                const bool more = j + 1 < tiles;
                 int k_slot = 0;
                 if (more) {
                     wait_slot(227);
@@ -723,16 +506,18 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     commit(s_full(0));
                     if (j + 2 == tiles_a) commit(q_empty(0));  // the item's last read of Q_A
                 }
-                product(1, j, v_slot);
+                if (j < tiles_b) {
+                    product(1, j, v_slot);
+                    if (j == tiles_b - 1) commit(o_full(1));
+                }
                 commit(kv_empty(v_slot));
-                if (more) {
+                if (j + 1 < tiles_b) {
                     scores(1, k_slot);
                     commit(s_full(1));
-                    commit(kv_empty(k_slot));
                     if (j + 2 == tiles_b) commit(q_empty(1));  // the item's last read of Q_B
                 }
+                if (more) commit(kv_empty(k_slot));
             }
-            commit(o_full(1));
             ++n;
             bh = next_bh;
             pair = next_pair;
@@ -750,8 +535,11 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 if (ok) ok = mbar_wait_warp(staged(x), n & 1, 216 + x);
                 if (leader) {
                     if (ok && g_device_status == 0) {
-                        tma_store_2d(&map_o, smem_base + PairSmem::kStage, 0, item.q_row_a + x * kRows);
-                        tma_store_2d(&map_o, smem_base + PairSmem::kStage + kHalfBytes, 64, item.q_row_a + x * kRows);
+                        const int row = (item.q_tile_a + x) * kRows;
+                        if (row < args.seq_q) {
+#pragma unroll
+                            for (int h = 0; h < D / 64; ++h) tma_store_4d(&map_o, smem_base + Smem::kStage + h * kHalfBytes, 64 * h, row, item.head, item.batch);
+                        }
                     }
                     tma_store_commit();
                     tma_store_wait_read<0>();
@@ -771,15 +559,15 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         const int row = quadrant * 32 + lane;
         const uint32_t lane_base = static_cast<uint32_t>(quadrant * 32) << 16;
         const uint32_t tmem_s = tmem_base + lane_base + x * 128;
-        const uint32_t tmem_o = tmem_base + lane_base + 256 + x * 128 + half * 64;
+        constexpr int kColumns = D / 2;  // of O per thread
+        const uint32_t tmem_o = tmem_base + lane_base + 256 + x * 128 + half * kColumns;
         const float scale = args.scale_log2;
         const int pair_barrier = 1 + x * 4 + quadrant;  // the 64 threads that share these 32 rows
-        uint16_t* exchange = reinterpret_cast<uint16_t*>(generic_base + PairSmem::kExchange) + ((x * 4 + quadrant) * 2) * 32;  // [half][lane]
-        float* sum_exchange = reinterpret_cast<float*>(generic_base + PairSmem::kExchange) + (x * 4 + quadrant) * 32;
-        const bool stamp = blockIdx.x == 0 && (threadIdx.x & 255) == 0;
-        (void)stamp;
+        uint16_t* exchange = reinterpret_cast<uint16_t*>(generic_base + Smem::kExchange) + ((x * 4 + quadrant) * 2) * 32;  // [half][lane]
+        float* sum_exchange = reinterpret_cast<float*>(generic_base + Smem::kExchange) + (x * 4 + quadrant) * 32;
         uint32_t n = 0;        // items started
         uint32_t s_count = 0;  // score tiles consumed (parity of s_full)
+        uint32_t ring_base = 0;  // ring slots of the items before this one
         bool ok = true;
         for_each_pair_item(args, [&](int bh, int pair) {
         const PairItem item = pair_item(args, bh, pair);
@@ -795,8 +583,10 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             // One pass over this thread's 64 scores, 16 at a time with the next load in flight: each chunk gives its part
             // of the half-row maximum and, from the second key tile on, its probabilities against the reference maximum
             // of the earlier tiles. Only a tile that raises the reference (rare after the first) is read a second time.
-            const bool diagonal = args.causal && j == q_tile;
-            const int limit = q_index - j * kKeys - half * 64;  // diagonal tile: keys 0..limit of this thread's 64 are visible
+            // keys 0..limit of this thread's 64 are visible; only a tile at the diagonal or at the batch's end has others
+            const int last_key = args.causal ? min(q_index, item.kv_len - 1) : item.kv_len - 1;
+            const int limit = last_key - j * kKeys - half * 64;
+            const bool diagonal = (args.causal && j >= q_tile) || (j + 1) * kKeys > item.kv_len;
             const bool speculative = j > 0;
             const uint64_t scale2 = pack2(scale, scale);
             uint64_t bias2 = pack2(-m_ref, -m_ref);
@@ -816,7 +606,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                             if (c * 16 + e > limit) raw[c][e] = 0xff800000u;  // -inf
                     }
                     mine = max_of_16(raw[c], mine);
-                    if (speculative) probabilities_of_16(raw[c], scale2, bias2, sums, packed + c * 8);
+                    if (speculative) probabilities_of_16<F16>(raw[c], scale2, bias2, sums, packed + c * 8);
                 }
             }
             raw_max = fmaxf(raw_max, mine);
@@ -843,9 +633,9 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 m_ref = m_new;
                 if (j > 0) {
                     // O_x holds P V up to tile j-1; that product was issued ahead of S_x(j), which has completed.
-                    // This thread rescales its 64 columns of the row.
+                    // This thread rescales its columns of the row.
 #pragma unroll 1
-                    for (int c = 0; c < 2; ++c) {
+                    for (int c = 0; c < kColumns / 32; ++c) {
                         uint32_t acc[32];
                         tmem_load_32(tmem_o + c * 32, acc);
                         tmem_load_wait();
@@ -870,8 +660,20 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                         for (int e = 0; e < 16; ++e)
                             if (c * 16 + e > limit) raw[e] = 0xff800000u;
                     }
-                    probabilities_of_16(raw, scale2, bias2, sums, packed + c * 8);
+                    probabilities_of_16<F16>(raw, scale2, bias2, sums, packed + c * 8);
                 }
+            }
+            if (args.len_q != nullptr && (j + 1) * kKeys > item.kv_len && (D == 128 || half == 0)) {
+                // V rows past the batch's length are not this sequence's: cleared before the product (by either tile's
+                // warps, which write the same zeros). The slot is V_j's place in the ring.
+                const uint32_t place = ring_base + 2 * j + 1, v_slot = place % kPairSlots;
+                if (ok) ok = mbar_wait(kv_full(v_slot), (place / kPairSlots) & 1, 234 + x);
+                if (j * kKeys + row >= item.kv_len) {
+                    uint8_t* v_row = generic_base + Smem::kRing + v_slot * kTileBytes + half * kHalfBytes + row * 128;
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) *reinterpret_cast<uint4*>(v_row + u * 16) = make_uint4(0, 0, 0, 0);
+                }
+                fence_async_shared();
             }
             tmem_store_32(tmem_s + half * 64, packed);
             {
@@ -905,28 +707,31 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             if (half == 0) {
                 const float row_raw_max = fmaxf(raw_max, sum_exchange[lane]);
                 const int64_t b64 = item.batch, h64 = item.head, q64 = q_index;
-                const bool any = total > 0.0f;
-                if (ok && args.row_max != nullptr)
+                const bool any = q_index < item.live_q;
+                const bool inside = ok && q_index < args.seq_q;
+                if (inside && args.row_max != nullptr)
                     args.row_max[b64 * args.max_stride[0] + h64 * args.max_stride[1] + q64 * args.max_stride[2]] = any ? row_raw_max * args.attn_scale : -INFINITY;
-                if (ok && args.row_sum != nullptr)  // the sum was accumulated against m_ref; re-express it against the true maximum
+                if (inside && args.row_sum != nullptr)  // the sum was accumulated against m_ref; re-express it against the true maximum
                     args.row_sum[b64 * args.sum_stride[0] + h64 * args.sum_stride[1] + q64 * args.sum_stride[2]] = any ? total * exp2f(m_ref - row_raw_max * scale) : 0.0f;
             }
         }
         // the hand-over words double as the next item's maxima: every read above must precede those writes
         asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
-        const float inverse = total > 0.0f ? 1.0f / total : 0.0f;
+        const bool live = q_index < item.live_q;
+        const float inverse = live ? 1.0f / total : 0.0f;
         // the staging tile serves the query tiles in turn: A, B, the next item's A, ...
         {
             const uint32_t turn = 2 * n + x;
             if (ok) ok = mbar_wait(stage_free, (turn & 1) ^ 1, 232 + x);
         }
-        uint8_t* o_row = generic_base + PairSmem::kStage + half * kHalfBytes + row * 128;  // this thread's 64 output columns
+        uint8_t* o_row = generic_base + Smem::kStage + (D == 128 ? half * kHalfBytes : 0) + row * 128;  // this thread's output columns: 16-byte units from first_unit on
+        const int first_unit = D == 128 ? 0 : half * 4;
 #pragma unroll 1
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < kColumns / 32; ++c) {
             uint32_t acc[32];
             tmem_load_32(tmem_o + c * 32, acc);
             tmem_load_wait();
-            if (c == 1) {
+            if (c == kColumns / 32 - 1) {
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(o_empty(x));
@@ -935,20 +740,19 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             for (int u = 0; u < 4; ++u) {
                 uint32_t w[4];
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    __nv_bfloat162 two = __floats2bfloat162_rn(__uint_as_float(acc[u * 8 + 2 * t]) * inverse, __uint_as_float(acc[u * 8 + 2 * t + 1]) * inverse);
-                    w[t] = *reinterpret_cast<uint32_t*>(&two);
-                }
-                const int unit = c * 4 + u;  // 16-byte unit inside this thread's 128 bytes of the output row
+                for (int t = 0; t < 4; ++t)   // (selected, not multiplied: a dead row's accumulator may hold anything)
+                    w[t] = live ? pack_pair<F16>(__uint_as_float(acc[u * 8 + 2 * t]) * inverse, __uint_as_float(acc[u * 8 + 2 * t + 1]) * inverse) : 0u;
+                const int unit = first_unit + c * 4 + u;
                 *reinterpret_cast<uint4*>(o_row + ((unit ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
             }
         }
         fence_async_shared();
         __syncwarp();
         if (lane == 0) mbar_arrive(staged(x));
-        if (args.stats != nullptr && ok && half == 0)
+        if (args.stats != nullptr && ok && half == 0 && q_index < args.seq_q)
             args.stats[item.batch * args.stats_batch_stride + item.head * args.stats_head_stride + static_cast<int64_t>(q_index) * args.stats_row_stride] =
-                total > 0.0f ? 0.6931471805599453f * (m_ref + log2f(total)) : -INFINITY;
+                live ? 0.6931471805599453f * (m_ref + log2f(total)) : -INFINITY;
+        ring_base += 2 * item.tiles;
         ++n;
         return true;  // also after a wait gave up: the two warps of a row pair must meet at the same barriers to the end
         });
@@ -962,95 +766,98 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     }
 }
 
-bool packed_bhsd(const dfgpu_tensor& t) {
-    return t.rank == 4 && t.stride[3] == 1 && t.stride[2] == t.dim[3] && t.stride[1] == t.dim[2] * t.dim[3] &&
-           t.stride[0] == t.dim[1] * t.dim[2] * t.dim[3];
+// Channel-contiguous [B, H, S, D] whose rows TMA can read: every other stride a positive multiple of 16 bytes.
+bool rows_for_tma(const dfgpu_tensor& t) {
+    if (t.rank != 4 || t.stride[3] != 1) return false;
+    for (int i = 0; i < 3; ++i)
+        if (t.dim[i] != 1 && (t.stride[i] <= 0 || t.stride[i] % 8 != 0 || t.stride[i] >= (1ll << 38))) return false;
+    return t.dim[0] < (1ll << 31) && t.dim[1] < (1ll << 31) && t.dim[2] < (1ll << 30);
+}
+
+int sdpa_map(CUtensorMap* map, const dfgpu_tensor& t, const void* data, const char* what) {
+    uint64_t dims[4] = {static_cast<uint64_t>(t.dim[3]), static_cast<uint64_t>(t.dim[2]), static_cast<uint64_t>(t.dim[1]), static_cast<uint64_t>(t.dim[0])};
+    uint64_t strides[3];
+    for (int i = 0; i < 3; ++i) strides[i] = static_cast<uint64_t>(t.dim[2 - i] == 1 ? t.dim[3] : t.stride[2 - i]) * 2;   // (an axis of one position has no stride to mind)
+    uint32_t box[4] = {64, kRows, 1, 1};
+    return make_map(map, data, 4, dims, strides, box, what);
+}
+
+template <int D, bool F16>
+int launch_pair(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_o, const SdpaUmmaArgs& args, unsigned grid, cudaStream_t stream) {
+    cudaError_t error = cudaFuncSetAttribute(sdpa_umma_pair_kernel<D, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<D>::kDynamic);
+    if (error != cudaSuccess) return fail(kExecutionFailed, "SDPA: cannot reserve %d bytes of shared memory: %s", PairSmem<D>::kDynamic, cudaGetErrorString(error));
+    launch_chained(sdpa_umma_pair_kernel<D, F16>, dim3(grid), dim3(kPairThreads), PairSmem<D>::kDynamic, stream, map_q, map_k, map_v, map_o, args);
+    return check_launch("SDPA (tcgen05, two query tiles per CTA)");
 }
 
 }  // namespace
 
 bool sdpa_umma_supported(const dfgpu_sdpa_params& p) {
-    if (p.q.dtype != DFGPU_BF16 || p.k.dtype != DFGPU_BF16 || p.v.dtype != DFGPU_BF16 || p.o.dtype != DFGPU_BF16) return false;
+    if (p.q.dtype != DFGPU_BF16 && p.q.dtype != DFGPU_F16) return false;
+    if (p.k.dtype != p.q.dtype || p.v.dtype != p.q.dtype || p.o.dtype != p.q.dtype) return false;
     if (p.q.rank != 4 || p.k.rank != 4 || p.v.rank != 4 || p.o.rank != 4) return false;
-    if (p.q.dim[3] != kHeadDim || p.v.dim[3] != kHeadDim || p.k.dim[3] != kHeadDim) return false;
-    if (p.page_table_k.rank || p.page_table_v.rank || p.padding_mask || p.has_left_bound || p.bottom_right) return false;
-    if ((p.max.rank || p.sum_exp.rank) && (p.q.dim[2] % (2 * kRows) != 0 || !(p.attn_scale > 0.0f) || !(p.attn_scale < INFINITY))) return false;  // only the two-tile kernel writes them
-    if ((p.max.rank && p.max.dtype != DFGPU_F32) || (p.sum_exp.rank && p.sum_exp.dtype != DFGPU_F32)) return false;
-    if (!packed_bhsd(p.q) || !packed_bhsd(p.k) || !packed_bhsd(p.v) || !packed_bhsd(p.o)) return false;
+    const int64_t d = p.q.dim[3];
+    if ((d != 64 && d != 128) || p.v.dim[3] != d || p.k.dim[3] != d || p.o.dim[3] != d) return false;
+    if (p.page_table_k.rank || p.page_table_v.rank || p.has_left_bound || p.bottom_right) return false;
+    if (!rows_for_tma(p.q) || !rows_for_tma(p.k) || !rows_for_tma(p.v) || !rows_for_tma(p.o)) return false;
     const int64_t sq = p.q.dim[2], skv = p.k.dim[2];
     if (p.s_kv != skv || p.v.dim[2] != skv || p.k.dim[1] != p.v.dim[1]) return false;
-    if (sq % kRows != 0 || skv % kKeys != 0 || sq < kRows || skv < kKeys) return false;
-    if (p.has_right_bound && (p.right_bound != 0 || sq != skv)) return false;  // causal, top-left aligned, square
-    if (p.stats.rank && p.stats.dtype != DFGPU_F32) return false;
-    const int64_t rows_q = p.q.dim[0] * p.q.dim[1] * sq, rows_kv = p.k.dim[0] * p.k.dim[1] * skv;
-    if (rows_q >= (1ll << 31) || rows_kv >= (1ll << 31) || p.q.dim[0] * p.q.dim[1] > 65535) return false;
-    return true;
+    if (p.has_right_bound && p.right_bound != 0) return false;  // causal, top-left aligned
+    if (!(p.attn_scale > -INFINITY && p.attn_scale < INFINITY)) return false;
+    for (const dfgpu_tensor* row : {&p.stats, &p.max, &p.sum_exp})
+        if (row->rank && row->dtype != DFGPU_F32) return false;
+    return p.q.dim[0] * p.q.dim[1] * ((sq + 2 * kRows - 1) / (2 * kRows)) < (1ll << 30);
 }
 
-int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, void* scratch, cudaStream_t stream) {
-    (void)scratch;
+int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, cudaStream_t stream) {
     for (int i = 0; i < 4; ++i)
         if ((reinterpret_cast<uintptr_t>(tensors[i]) & 15u) != 0) return fail(kInvalidArgument, "SDPA: the tcgen05 kernel needs 16-byte aligned Q, K, V and O");
-    const int64_t batch = p.q.dim[0], hq = p.q.dim[1], hkv = p.k.dim[1], sq = p.q.dim[2], skv = p.k.dim[2];
     CUtensorMap map_q, map_k, map_v, map_o;
-    uint32_t box[2] = {64, kRows};
-    uint64_t strides[1] = {kHeadDim * 2};
-    uint64_t dims_q[2] = {kHeadDim, static_cast<uint64_t>(batch * hq * sq)};
-    uint64_t dims_kv[2] = {kHeadDim, static_cast<uint64_t>(batch * hkv * skv)};
-    int status = make_map(&map_q, tensors[0], 2, dims_q, strides, box, "SDPA Q");
-    if (!status) status = make_map(&map_k, tensors[1], 2, dims_kv, strides, box, "SDPA K");
-    if (!status) status = make_map(&map_v, tensors[2], 2, dims_kv, strides, box, "SDPA V");
-    if (!status) status = make_map(&map_o, tensors[3], 2, dims_q, strides, box, "SDPA O");
+    int status = sdpa_map(&map_q, p.q, tensors[0], "SDPA Q");
+    if (!status) status = sdpa_map(&map_k, p.k, tensors[1], "SDPA K");
+    if (!status) status = sdpa_map(&map_v, p.v, tensors[2], "SDPA V");
+    if (!status) status = sdpa_map(&map_o, p.o, tensors[3], "SDPA O");
     if (status) return status;
     SdpaUmmaArgs args{};
-    args.heads_q = static_cast<int>(hq);
-    args.heads_kv = static_cast<int>(hkv);
-    args.seq_q = static_cast<int>(sq);
-    args.seq_kv = static_cast<int>(skv);
-    args.q_tiles = static_cast<int>(sq / kRows);
+    args.heads_q = static_cast<int>(p.q.dim[1]);
+    args.heads_kv = static_cast<int>(p.k.dim[1]);
+    args.seq_q = static_cast<int>(p.q.dim[2]);
+    args.seq_kv = static_cast<int>(p.k.dim[2]);
+    args.q_tiles = (args.seq_q + kRows - 1) / kRows;
+    args.pairs = (args.q_tiles + 1) / 2;
+    args.batch_heads = static_cast<int>(p.q.dim[0] * p.q.dim[1]);
     args.causal = p.has_right_bound ? 1 : 0;
-    args.scale_log2 = p.attn_scale * 1.4426950408889634f;
-    args.stats = p.stats.rank ? static_cast<float*>(tensors[4]) : nullptr;
+    // (a scale of zero weighs every key alike; the smallest normal one does too, and keeps scale * -inf at -inf)
+    args.attn_scale = std::max(std::fabs(p.attn_scale), 1e-37f);
+    args.scale_log2 = args.attn_scale * 1.4426950408889634f;
+    args.negate_q = p.attn_scale < 0.0f ? 1u << 13 : 0u;
+    if (p.padding_mask) {
+        args.len_q = static_cast<const int32_t*>(tensors[7]);
+        args.len_kv = static_cast<const int32_t*>(tensors[8]);
+        args.len_q_stride = p.seq_q.stride[0];
+        args.len_kv_stride = p.seq_kv.stride[0];
+    }
     if (p.stats.rank) {
+        args.stats = static_cast<float*>(tensors[4]);
         args.stats_batch_stride = p.stats.stride[0];
         args.stats_head_stride = p.stats.stride[1];
         args.stats_row_stride = p.stats.stride[2];
     }
-    args.attn_scale = p.attn_scale;
     args.row_max = p.max.rank ? static_cast<float*>(tensors[5]) : nullptr;
     args.row_sum = p.sum_exp.rank ? static_cast<float*>(tensors[6]) : nullptr;
     for (int i = 0; i < 3; ++i) {
         args.max_stride[i] = p.max.rank ? p.max.stride[i] : 0;
         args.sum_stride[i] = p.sum_exp.rank ? p.sum_exp.stride[i] : 0;
     }
-    const bool pair_form = sq % (2 * kRows) == 0 && p.attn_scale > 0.0f && p.attn_scale < INFINITY;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t error = cudaFuncSetAttribute(sdpa_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::kDynamic);
-        if (error == cudaSuccess) error = cudaFuncSetAttribute(sdpa_umma_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem::kDynamic);
-        if (error != cudaSuccess) return fail(kExecutionFailed, "SDPA: cannot reserve %d bytes of shared memory: %s", PairSmem::kDynamic, cudaGetErrorString(error));
-        configured = true;
-    }
-    if (pair_form) {
-        // persistent: one CTA per SM over the work list (see for_each_pair_item)
-        static int sm_count = 0;
-        if (sm_count == 0) {
-            int device = 0;
-            if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sm_count <= 0) {
-                sm_count = 0;
-                return fail(kExecutionFailed, "SDPA: cannot read the number of multiprocessors");
-            }
-        }
-        const int pairs = args.q_tiles / 2;
-        const int64_t units = static_cast<int64_t>(args.causal ? (pairs + 1) / 2 : pairs) * batch * hq;
-        args.batch_heads = static_cast<int>(batch * hq);
-        const unsigned grid = static_cast<unsigned>(units < sm_count ? units : sm_count);
-        launch_chained(sdpa_umma_pair_kernel, dim3(grid), dim3(kPairThreads), PairSmem::kDynamic, stream, map_q, map_k, map_v, map_o, args);
-        return check_launch("SDPA (tcgen05, two query tiles per CTA)");
-    }
-    dim3 grid(static_cast<unsigned>(args.q_tiles), static_cast<unsigned>(batch * hq));
-    launch_chained(sdpa_umma_kernel, dim3(grid), dim3(kSdpaThreads), Smem::kDynamic, stream, map_q, map_k, map_v, map_o, args);
-    return check_launch("SDPA (tcgen05)");
+    // persistent: one CTA per SM over the work list (see PairWalker)
+    const int sms = sm_count();
+    const int64_t single = static_cast<int64_t>(args.pairs) * args.batch_heads;
+    args.paired_units = args.causal && single > sms ? 1 : 0;
+    const int64_t units = args.paired_units ? static_cast<int64_t>((args.pairs + 1) / 2) * args.batch_heads : single;
+    const unsigned grid = static_cast<unsigned>(units < sms ? units : sms);
+    const bool f16 = p.q.dtype == DFGPU_F16;
+    if (p.q.dim[3] == 64) return f16 ? launch_pair<64, true>(map_q, map_k, map_v, map_o, args, grid, stream) : launch_pair<64, false>(map_q, map_k, map_v, map_o, args, grid, stream);
+    return f16 ? launch_pair<128, true>(map_q, map_k, map_v, map_o, args, grid, stream) : launch_pair<128, false>(map_q, map_k, map_v, map_o, args, grid, stream);
 }
 
 int sdpa_umma_device_status(int* status) { return read_and_clear_device_status(status); }

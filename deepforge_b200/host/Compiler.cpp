@@ -1116,7 +1116,11 @@ std::uint64_t kernel_alignment(KernelStep const& step, std::size_t slot) {
             if (step.kernel != DFGPU_MATMUL_UMMA_F32X3 && !whole_tiles(std::get<dfgpu_matmul_params>(step.params), step.kernel == DFGPU_MATMUL_UMMA_MXF8 ? 128 : 64)) return 0;
             return slot == 3 || slot == 4 ? 4 : 16;  // the scale tensors are gathered with 4-byte loads
         case KernelOp::kSdpaForward:
-            if (step.kernel == DFGPU_SDPA_UMMA) return slot <= 3 ? 16 : 0;
+            if (step.kernel == DFGPU_SDPA_UMMA) {   // (lengths that are no whole tiles fall back where a pointer is off the boundary, as above)
+                auto const& p = std::get<dfgpu_sdpa_params>(step.params);
+                bool const whole = p.q.dtype == DFGPU_BF16 && p.q.dim[3] == 128 && p.q.dim[2] % 128 == 0 && p.k.dim[2] % 128 == 0 && !p.padding_mask;
+                return slot <= 3 && whole ? 16 : 0;
+            }
             if (step.kernel == DFGPU_SDPA_PAGED_DECODE_UMMA || step.kernel == DFGPU_SDPA_PAGED_DECODE) return slot <= 2 ? 16 : 0;
             return 0;
         case KernelOp::kMatmulFp8: return step.kernel == DFGPU_MATMUL_FP8_UMMA && slot <= 2 && whole_tiles(std::get<dfgpu_matmul_fp8_params>(step.params), 128) ? 16 : 0;

@@ -1,0 +1,90 @@
+"""SDPA on the tensor cores at lengths that fill no tile: one row past and short of the 128-row tiles, single rows, more and fewer
+keys than queries, grouped heads, padding masks with short and empty sequences (NaN in the padding must not leak), causal or
+not, both 16-bit types and head dimensions, strided layouts, a negative scale. Compared with an f64 softmax of the stored values.
+
+Tolerances: a probability is rounded to the operands' type before it weighs V (u = 2^-8 for bf16, 2^-11 for f16, relative) and
+exponentials are within 2^-13, so O is off by at most (u + 2^-12) sum p |v| before it is rounded once by u; subnormal f16
+probabilities (up to 2^-24 of the largest) add 2^-24 sum |v|. Stats carry the exponentials' error and f32 scores."""
+import pytest
+
+from deepforge_b200 import dfgpu, graphs, runtime
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+TORCH = {"BFLOAT16": torch.bfloat16, "HALF": torch.float16}
+ROUNDING = {"BFLOAT16": 2.0 ** -8, "HALF": 2.0 ** -11}
+
+
+def attention(q, k, v, scale, causal, len_q=None, len_kv=None):
+    b, h, sq, _ = q.shape
+    group, skv = h // k.shape[1], k.shape[2]
+    k, v = k.double().repeat_interleave(group, 1), v.double().repeat_interleave(group, 1)
+    keys, rows = torch.arange(skv, device="cuda"), torch.arange(sq, device="cuda")
+    valid = torch.ones(b, 1, sq, skv, dtype=torch.bool, device="cuda")
+    if causal:
+        valid = valid & (keys[None, :] <= rows[:, None])
+    if len_q is not None:
+        valid = valid & (keys[None, None, None, :] < len_kv[:, None, None, None]) & (rows[None, None, :, None] < len_q[:, None, None, None])
+        v = torch.where(keys[None, None, :, None] < len_kv[:, None, None, None], v, 0.0)
+        k = torch.where(keys[None, None, :, None] < len_kv[:, None, None, None], k, 0.0)
+        q = torch.where(rows[None, None, :, None] < len_q[:, None, None, None], q, 0.0)
+    s = (q.double() @ k.transpose(-1, -2) * scale).masked_fill(~valid, -float("inf"))
+    stats = torch.logsumexp(s, -1)
+    p = torch.where(valid, torch.exp(s - torch.where(torch.isinf(stats), 0.0, stats)[..., None]), 0.0)
+    return p @ v, p @ v.abs(), v.abs().sum(-2, keepdim=True), stats
+
+
+def check(b, h, hkv, sq, skv, d, io, causal, padding=None, scale=None, strided=False, seed=3):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    scale = d ** -0.5 if scale is None else scale
+    def operand(heads, length):
+        x = torch.randn(b, length, heads, d, device="cuda", generator=g).to(TORCH[io])   # [B, S, H, D]
+        return x.transpose(1, 2) if strided else x.transpose(1, 2).contiguous()
+    q, k, v = operand(h, sq), operand(hkv, skv), operand(hkv, skv)
+    o = torch.full_like(q, float("nan"))
+    stats = torch.full((b, h, sq), float("nan"), device="cuda")
+    tensors = [graphs.tensor(uid, name, list(x.shape), io, list(x.stride())) for uid, name, x in ((1, "Q", q), (2, "K", k), (3, "V", v), (4, "O", o))]
+    tensors.append(graphs.tensor(5, "Stats", [b, h, sq, 1], "FLOAT"))
+    inputs, pack, len_q, len_kv = {"Q": 1, "K": 2, "V": 3}, {1: q, 2: k, 3: v, 4: o, 5: stats}, None, None
+    if padding is not None:
+        len_q, len_kv = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in padding)
+        for i in range(b):
+            q[i, :, len_q[i]:], k[i, :, len_kv[i]:], v[i, :, len_kv[i]:] = float("nan"), float("nan"), float("inf")
+        tensors += [graphs.tensor(6, "SEQ_LEN_Q", [b, 1, 1, 1], "INT32"), graphs.tensor(7, "SEQ_LEN_KV", [b, 1, 1, 1], "INT32")]
+        inputs.update(SEQ_LEN_Q=6, SEQ_LEN_KV=7)
+        pack.update({6: len_q, 7: len_kv})
+    node = graphs.sdpa_node("sdpa", inputs, {"O": 4, "Stats": 5}, scale, padding is not None, True, right_bound=0 if causal else None)
+    exe = runtime.compile_graph(graphs.document("ragged", [node], tensors, io=io))
+    assert exe.steps()[0]["kernel"] == dfgpu.SDPA_UMMA and exe.workspace_size == 0
+    exe.execute({uid: x.data_ptr() for uid, x in pack.items()})
+    torch.cuda.synchronize()
+    assert dfgpu.device_status() == 0
+    want, weight, every, want_stats = attention(q, k, v, scale, causal, len_q, len_kv)
+    u = ROUNDING[io]
+    bound = (u + 2.0 ** -12) * weight + u * want.abs() + (2.0 ** -24 * every if io == "HALF" else 0.0) + 1e-30
+    error = (o.double() - want).abs()
+    assert bool(torch.all(error <= bound)), float((error / bound).nan_to_num(1e9).max())
+    dead = torch.isinf(want_stats)
+    assert bool(torch.all(torch.isneginf(stats[dead]))) and bool(torch.all((stats.double() - want_stats)[~dead].abs() <= 1e-3))
+
+
+@pytest.mark.parametrize("io,d", [("BFLOAT16", 128), ("HALF", 128), ("BFLOAT16", 64), ("HALF", 64)])
+@pytest.mark.parametrize("b,h,hkv,sq,skv,causal", [(1, 2, 1, 1, 1, False), (2, 4, 2, 19, 301, False), (1, 4, 4, 127, 127, True), (1, 2, 2, 128, 129, False), (2, 2, 1, 129, 129, True),
+                                                   (3, 8, 2, 257, 64, False), (1, 3, 1, 300, 1000, True), (2, 40, 8, 641, 641, True), (1, 2, 2, 1000, 130, True)])
+def test_any_lengths(io, d, b, h, hkv, sq, skv, causal):
+    check(b, h, hkv, sq, skv, d, io, causal)
+
+
+@pytest.mark.parametrize("io,d", [("BFLOAT16", 128), ("HALF", 64)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_padded_lengths(io, d, causal):
+    check(5, 4, 2, 300, 300, d, io, causal, padding=([300, 130, 1, 0, 257], [300, 130, 1, 200, 0]))
+    check(3, 40, 8, 513, 400, d, io, causal, padding=([513, 400, 128], [128, 129, 400]))
+
+
+def test_strides_scale_and_misalignment():
+    check(2, 4, 2, 200, 200, 128, "BFLOAT16", True, strided=True)
+    check(1, 2, 2, 200, 300, 64, "HALF", False, scale=-0.2)
+    check(1, 2, 1, 150, 260, 128, "BFLOAT16", False, scale=0.0)
+    check(1, 2, 2, 384, 384, 128, "BFLOAT16", True, scale=1.5)   # (the running maximum jumps: O is rescaled)
