@@ -239,6 +239,9 @@ struct PairItem {
     int live_q;          // query rows before this one have keys; the others store 0 and -inf
 };
 
+// EDGES: a batch's keys may end inside a key tile (padding masks, or a key length that is no multiple of 128). Without them
+// the masks of the last tile, the clearing of V rows and the dead rows are not compiled in: they cost 5 % of 8 x 32 x 2048 causal.
+template <bool EDGES>
 __device__ __forceinline__ PairItem pair_item(const SdpaUmmaArgs& args, int bh, int pair) {
     PairItem item;
     item.batch = bh / args.heads_q;
@@ -247,7 +250,7 @@ __device__ __forceinline__ PairItem pair_item(const SdpaUmmaArgs& args, int bh, 
     item.q_tile_a = 2 * pair;
     item.kv_len = args.seq_kv;
     item.live_q = args.seq_q;
-    if (args.len_q != nullptr) {
+    if (EDGES && args.len_q != nullptr) {
         const int len_kv = __ldg(args.len_kv + item.batch * args.len_kv_stride);
         item.live_q = len_kv > 0 ? min(item.live_q, __ldg(args.len_q + item.batch * args.len_q_stride)) : 0;
         item.kv_len = max(1, min(item.kv_len, len_kv));
@@ -306,7 +309,7 @@ __device__ __forceinline__ void for_each_pair_item(const SdpaUmmaArgs& args, Bod
 //   warp 17     issues the products; one elected lane issues, all lanes walk the schedule
 //   warp 18     sends staged output tiles to global memory by TMA (row-per-thread global stores of 16 bytes at a
 //               256-byte stride kept the load/store unit busy for ~5000 cycles per tile)
-template <int D, bool F16>
+template <int D, bool F16, bool EDGES>
 __global__ void __launch_bounds__(kPairThreads, 1)
 sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o, SdpaUmmaArgs args) {
@@ -368,7 +371,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         uint32_t phase = 1;  // parity of the "slot is free" wait
         uint32_t n = 0;      // items started
         for_each_pair_item(args, [&](int bh, int pair) {
-            const PairItem item = pair_item(args, bh, pair);
+            const PairItem item = pair_item<EDGES>(args, bh, pair);
             auto load_box = [&](uint32_t dst, const CUtensorMap* map, int row, int head, uint32_t bar) {
 #pragma unroll
                 for (int h = 0; h < D / 64; ++h) tma_load_4d(dst + h * kHalfBytes, map, 64 * h, row, head, item.batch, bar);
@@ -454,10 +457,10 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         bool early = false;  // S_A of the current item was issued in the previous item's last round
         int early_slot = 0;  // the ring slot of its K tile
         while (have && ok) {
-            const PairItem item = pair_item(args, bh, pair);
+            const PairItem item = pair_item<EDGES>(args, bh, pair);
             const int tiles_a = item.tiles_a, tiles_b = item.tiles_b, tiles = item.tiles;
             const bool have_next = walker.next(args, next_bh, next_pair);
-            const int next_tiles_a = have_next ? pair_item(args, next_bh, next_pair).tiles_a : 0;
+            const int next_tiles_a = have_next ? pair_item<EDGES>(args, next_bh, next_pair).tiles_a : 0;
             int k0_slot = early_slot;
             if (!early) {
                 if (ok) ok = mbar_wait_warp(q_full(0), n & 1, 222);
@@ -530,7 +533,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         uint32_t n = 0;
         bool ok = true;
         for_each_pair_item(args, [&](int bh, int pair) {
-            const PairItem item = pair_item(args, bh, pair);
+            const PairItem item = pair_item<EDGES>(args, bh, pair);
             for (int x = 0; x < 2; ++x) {
                 if (ok) ok = mbar_wait_warp(staged(x), n & 1, 216 + x);
                 if (leader) {
@@ -570,7 +573,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         uint32_t ring_base = 0;  // ring slots of the items before this one
         bool ok = true;
         for_each_pair_item(args, [&](int bh, int pair) {
-        const PairItem item = pair_item(args, bh, pair);
+        const PairItem item = pair_item<EDGES>(args, bh, pair);
         const int q_tile = item.q_tile_a + x;
         const int q_index = q_tile * kRows + row;
         const int my_tiles = x ? item.tiles_b : item.tiles_a;
@@ -584,9 +587,9 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             // of the half-row maximum and, from the second key tile on, its probabilities against the reference maximum
             // of the earlier tiles. Only a tile that raises the reference (rare after the first) is read a second time.
             // keys 0..limit of this thread's 64 are visible; only a tile at the diagonal or at the batch's end has others
-            const int last_key = args.causal ? min(q_index, item.kv_len - 1) : item.kv_len - 1;
+            const int last_key = !EDGES ? q_index : (args.causal ? min(q_index, item.kv_len - 1) : item.kv_len - 1);
             const int limit = last_key - j * kKeys - half * 64;
-            const bool diagonal = (args.causal && j >= q_tile) || (j + 1) * kKeys > item.kv_len;
+            const bool diagonal = (args.causal && j == q_tile) || (EDGES && (j + 1) * kKeys > item.kv_len);
             const bool speculative = j > 0;
             const uint64_t scale2 = pack2(scale, scale);
             uint64_t bias2 = pack2(-m_ref, -m_ref);
@@ -663,7 +666,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     probabilities_of_16<F16>(raw, scale2, bias2, sums, packed + c * 8);
                 }
             }
-            if (args.len_q != nullptr && (j + 1) * kKeys > item.kv_len && (D == 128 || half == 0)) {
+            if (EDGES && args.len_q != nullptr && (j + 1) * kKeys > item.kv_len && (D == 128 || half == 0)) {
                 // V rows past the batch's length are not this sequence's: cleared before the product (by either tile's
                 // warps, which write the same zeros). The slot is V_j's place in the ring.
                 const uint32_t place = ring_base + 2 * j + 1, v_slot = place % kPairSlots;
@@ -707,7 +710,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             if (half == 0) {
                 const float row_raw_max = fmaxf(raw_max, sum_exchange[lane]);
                 const int64_t b64 = item.batch, h64 = item.head, q64 = q_index;
-                const bool any = q_index < item.live_q;
+                const bool any = !EDGES || q_index < item.live_q;
                 const bool inside = ok && q_index < args.seq_q;
                 if (inside && args.row_max != nullptr)
                     args.row_max[b64 * args.max_stride[0] + h64 * args.max_stride[1] + q64 * args.max_stride[2]] = any ? row_raw_max * args.attn_scale : -INFINITY;
@@ -717,7 +720,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         }
         // the hand-over words double as the next item's maxima: every read above must precede those writes
         asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
-        const bool live = q_index < item.live_q;
+        const bool live = !EDGES || q_index < item.live_q;
         const float inverse = live ? 1.0f / total : 0.0f;
         // the staging tile serves the query tiles in turn: A, B, the next item's A, ...
         {
@@ -752,7 +755,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         if (args.stats != nullptr && ok && half == 0 && q_index < args.seq_q)
             args.stats[item.batch * args.stats_batch_stride + item.head * args.stats_head_stride + static_cast<int64_t>(q_index) * args.stats_row_stride] =
                 live ? 0.6931471805599453f * (m_ref + log2f(total)) : -INFINITY;
-        ring_base += 2 * item.tiles;
+        if (EDGES) ring_base += 2 * item.tiles;
         ++n;
         return true;  // also after a wait gave up: the two warps of a row pair must meet at the same barriers to the end
         });
@@ -782,12 +785,17 @@ int sdpa_map(CUtensorMap* map, const dfgpu_tensor& t, const void* data, const ch
     return make_map(map, data, 4, dims, strides, box, what);
 }
 
+template <int D, bool F16, bool EDGES>
+int launch_edges(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_o, const SdpaUmmaArgs& args, unsigned grid, cudaStream_t stream) {
+    cudaError_t error = cudaFuncSetAttribute(sdpa_umma_pair_kernel<D, F16, EDGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<D>::kDynamic);
+    if (error != cudaSuccess) return fail(kExecutionFailed, "SDPA: cannot reserve %d bytes of shared memory: %s", PairSmem<D>::kDynamic, cudaGetErrorString(error));
+    launch_chained(sdpa_umma_pair_kernel<D, F16, EDGES>, dim3(grid), dim3(kPairThreads), PairSmem<D>::kDynamic, stream, map_q, map_k, map_v, map_o, args);
+    return check_launch("SDPA (tcgen05, two query tiles per CTA)");
+}
 template <int D, bool F16>
 int launch_pair(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_o, const SdpaUmmaArgs& args, unsigned grid, cudaStream_t stream) {
-    cudaError_t error = cudaFuncSetAttribute(sdpa_umma_pair_kernel<D, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<D>::kDynamic);
-    if (error != cudaSuccess) return fail(kExecutionFailed, "SDPA: cannot reserve %d bytes of shared memory: %s", PairSmem<D>::kDynamic, cudaGetErrorString(error));
-    launch_chained(sdpa_umma_pair_kernel<D, F16>, dim3(grid), dim3(kPairThreads), PairSmem<D>::kDynamic, stream, map_q, map_k, map_v, map_o, args);
-    return check_launch("SDPA (tcgen05, two query tiles per CTA)");
+    if (args.len_q != nullptr || args.seq_kv % kKeys != 0) return launch_edges<D, F16, true>(map_q, map_k, map_v, map_o, args, grid, stream);
+    return launch_edges<D, F16, false>(map_q, map_k, map_v, map_o, args, grid, stream);
 }
 
 }  // namespace
