@@ -3,9 +3,13 @@
 //
 // Every mode of the reference's pointwise_result (lib/Compiler/FoundationalGraph.cpp:2581-2955) goes through
 // pointwise_value below: the same expression, one separately rounded f32 operation per step, with CUDA's full-precision
-// math functions (no fast-math intrinsics). Packed tensors of equal shape (f32, f16 or bf16) take the kernel of four values per
-// load; anything else (broadcast, strides, mixed storage types, three inputs, GEN_INDEX) one element per thread, where
-// ADD / MUL / SUB / RELU_FWD / IDENTITY keep a kernel with nothing else in it.
+// math functions where the result is stored as f32 (see Math for the 16-bit types). Dense tensors of one storage type take the kernel of four
+// values per load, also where an operand is broadcast along the leading or the trailing axes (a bias, a mask by rows, a
+// scalar); anything else (gaps, other broadcasts, mixed storage types, three inputs, GEN_INDEX) one element per thread,
+// where ADD / MUL / SUB / RELU_FWD / IDENTITY keep a kernel with nothing else in it.
+#include <algorithm>
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace dfgpu {
@@ -40,11 +44,50 @@ __host__ __device__ constexpr int input_count(int mode) {
 
 inline bool simple_mode(int mode) { return mode >= DFGPU_PW_ADD && mode <= DFGPU_PW_SUB; }
 
+// The functions of the math library. EXACT: CUDA's full-precision ones, for results stored as f32. Otherwise (results rounded
+// to 8 or 11 significant bits) forms within a few 2^-22 relative, a thousandth of that rounding, because the bytes are half and the
+// instructions set the pace: GELU_BWD on 33.5 M bf16 values is 60 instructions a value with erff and expf, 55.8 us against
+// 30.7 for its bytes.
+template <bool EXACT>
+struct Math {
+    static __device__ __forceinline__ float exp(float v) { return EXACT ? expf(v) : __expf(v); }
+    static __device__ __forceinline__ float divide(float a, float b) { return EXACT ? __fdiv_rn(a, b) : __fdividef(a, b); }
+    static __device__ __forceinline__ float tanh(float v) {
+        if constexpr (EXACT) return tanhf(v);
+        // 1 - 2 / (1 + e^2v); near zero, where that cancels, the first two terms of the series (4e-8 relative at 0.02)
+        const float far = 1.0f - __fdividef(2.0f, 1.0f + __expf(2.0f * v));
+        return fabsf(v) < 0.02f ? v * fmaf(v * v, -0.33333334f, 1.0f) : far;
+    }
+    // 1 - tanh^2
+    static __device__ __forceinline__ float tanh_slope(float v, float t) {
+        if constexpr (EXACT) return __fsub_rn(1.0f, __fmul_rn(t, t));
+        const float e = __expf(-2.0f * fabsf(v)), d = 1.0f + e;   // (4e / (1 + e)^2 does not cancel)
+        return fabsf(v) <= 3.4e38f ? __fdividef(4.0f * e, d * d) : (v != v ? v : 0.0f);
+    }
+    // The normal distribution function and exp(-v^2 / 2), which gives it.
+    static __device__ __forceinline__ float normal_cdf(float v, float& bell) {
+        if constexpr (EXACT) {
+            bell = expf(__fmul_rn(-0.5f, __fmul_rn(v, v)));
+            return __fmul_rn(0.5f, __fadd_rn(1.0f, erff(__fmul_rn(v, 0.7071067811865475f))));
+        }
+        // 1 - erf(z) = (a1 t + ... + a5 t^5) e^-z^2, t = 1 / (1 + p z), z = |v| / sqrt 2, within 1.5e-7 (Abramowitz and Stegun,
+        // Handbook of Mathematical Functions, 7.1.26): half of it is the smaller tail.
+        bell = __expf(-0.5f * v * v);
+        const float k = __fdividef(1.0f, fmaf(0.3275911f * 0.70710678f, fabsf(v), 1.0f));
+        const float sum = fmaf(fmaf(fmaf(fmaf(1.061405429f, k, -1.453152027f), k, 1.421413741f), k, -0.284496736f), k, 0.254829592f);
+        const float tail = 0.5f * sum * k * bell;
+        return v >= 0.0f ? 1.0f - tail : tail;
+    }
+};
+
 // 1 / (1 + exp(-v)) (FoundationalGraph.cpp:2569-2579)
-__device__ __forceinline__ float sigmoid_value(float v) { return __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-v))); }
+template <bool EXACT>
+__device__ __forceinline__ float sigmoid_value(float v) { return Math<EXACT>::divide(1.0f, __fadd_rn(1.0f, Math<EXACT>::exp(-v))); }
 
 // x, y, z: IN_0, IN_1, IN_2 (0 where the mode has none). u: the activation's input (IN_1 of a _BWD mode, else IN_0).
+template <bool EXACT>
 __device__ __forceinline__ float pointwise_value(int mode, float x, float y, float z, const PointwiseScalars& s, int64_t position) {
+    using M = Math<EXACT>;
     const float u = (mode >= DFGPU_PW_RELU_BWD && input_count(mode) == 2) ? y : x;
     switch (mode) {
         case DFGPU_PW_ADD: return __fadd_rn(x, y);
@@ -58,7 +101,7 @@ __device__ __forceinline__ float pointwise_value(int mode, float x, float y, flo
         case DFGPU_PW_POW: return powf(x, y);
         case DFGPU_PW_SQRT: return __fsqrt_rn(x);
         case DFGPU_PW_RSQRT: return __fdiv_rn(1.0f, __fsqrt_rn(x));
-        case DFGPU_PW_EXP: return expf(x);
+        case DFGPU_PW_EXP: return M::exp(x);
         case DFGPU_PW_LOG: return logf(x);
         case DFGPU_PW_NEG: return -x;
         case DFGPU_PW_ABS: return fabsf(x);
@@ -83,39 +126,40 @@ __device__ __forceinline__ float pointwise_value(int mode, float x, float y, flo
         case DFGPU_PW_CMP_LE: return x <= y ? 1.0f : 0.0f;
         case DFGPU_PW_RELU_FWD: return relu_forward(x, s.relu_lower, s.relu_upper, s.relu_slope);
         case DFGPU_PW_RELU_BWD: return __fmul_rn(x, y < s.relu_lower ? s.relu_slope : (y > s.relu_upper ? 0.0f : 1.0f));
-        case DFGPU_PW_TANH_FWD: return tanhf(u);
-        case DFGPU_PW_TANH_BWD: { float t = tanhf(u); return __fmul_rn(x, __fsub_rn(1.0f, __fmul_rn(t, t))); }
-        case DFGPU_PW_SIGMOID_FWD: return sigmoid_value(u);
-        case DFGPU_PW_SIGMOID_BWD: { float v = sigmoid_value(u); return __fmul_rn(x, __fmul_rn(v, __fsub_rn(1.0f, v))); }
+        case DFGPU_PW_TANH_FWD: return M::tanh(u);
+        case DFGPU_PW_TANH_BWD: return __fmul_rn(x, M::tanh_slope(u, EXACT ? M::tanh(u) : 0.0f));
+        case DFGPU_PW_SIGMOID_FWD: return sigmoid_value<EXACT>(u);
+        case DFGPU_PW_SIGMOID_BWD: { float v = sigmoid_value<EXACT>(u); return __fmul_rn(x, __fmul_rn(v, __fsub_rn(1.0f, v))); }
         case DFGPU_PW_ELU_FWD: { float e = expf(u); return u >= 0.0f ? u : __fmul_rn(s.elu_alpha, __fsub_rn(e, 1.0f)); }
-        case DFGPU_PW_ELU_BWD: { float e = expf(u); return __fmul_rn(x, u >= 0.0f ? 1.0f : __fmul_rn(s.elu_alpha, e)); }
+        case DFGPU_PW_ELU_BWD: { float e = M::exp(u); return __fmul_rn(x, u >= 0.0f ? 1.0f : __fmul_rn(s.elu_alpha, e)); }
         case DFGPU_PW_SOFTPLUS_FWD: {
             float scaled = __fmul_rn(s.softplus_beta, u);
             float logarithm = logf(__fadd_rn(1.0f, expf(-fabsf(scaled))));
             return __fdiv_rn(__fadd_rn(maximum_nan(scaled, 0.0f), logarithm), s.softplus_beta);
         }
-        case DFGPU_PW_SOFTPLUS_BWD: return __fmul_rn(x, sigmoid_value(__fmul_rn(s.softplus_beta, u)));
-        case DFGPU_PW_SWISH_FWD: return __fmul_rn(u, sigmoid_value(__fmul_rn(s.swish_beta, u)));
+        case DFGPU_PW_SOFTPLUS_BWD: return __fmul_rn(x, sigmoid_value<EXACT>(__fmul_rn(s.softplus_beta, u)));
+        case DFGPU_PW_SWISH_FWD: return __fmul_rn(u, sigmoid_value<EXACT>(__fmul_rn(s.swish_beta, u)));
         case DFGPU_PW_SWISH_BWD: {
             float scaled = __fmul_rn(s.swish_beta, u);
-            float v = sigmoid_value(scaled);
+            float v = sigmoid_value<EXACT>(scaled);
             return __fmul_rn(x, __fadd_rn(v, __fmul_rn(scaled, __fmul_rn(v, __fsub_rn(1.0f, v)))));
         }
         case DFGPU_PW_GELU_FWD: case DFGPU_PW_GELU_BWD: {
-            float cdf = __fmul_rn(0.5f, __fadd_rn(1.0f, erff(__fmul_rn(u, 0.7071067811865475f))));
+            float bell;
+            float cdf = M::normal_cdf(u, bell);
             if (mode == DFGPU_PW_GELU_FWD) return __fmul_rn(u, cdf);
-            float density = __fmul_rn(0.3989422804014327f, expf(__fmul_rn(-0.5f, __fmul_rn(u, u))));
+            float density = __fmul_rn(0.3989422804014327f, bell);
             return __fmul_rn(x, __fadd_rn(cdf, __fmul_rn(u, density)));
         }
         case DFGPU_PW_GELU_APPROX_TANH_FWD: case DFGPU_PW_GELU_APPROX_TANH_BWD: {
             float square = __fmul_rn(u, u);
             float cubic = __fmul_rn(square, u);
             float inner = __fmul_rn(0.7978845608028654f, __fadd_rn(u, __fmul_rn(0.044715f, cubic)));
-            float t = tanhf(inner);
+            float t = M::tanh(inner);
             float cdf = __fmul_rn(0.5f, __fadd_rn(1.0f, t));
             if (mode == DFGPU_PW_GELU_APPROX_TANH_FWD) return __fmul_rn(u, cdf);
             float inner_derivative = __fmul_rn(0.7978845608028654f, __fadd_rn(1.0f, __fmul_rn(0.134145f, square)));
-            float tanh_derivative = __fsub_rn(1.0f, __fmul_rn(t, t));
+            float tanh_derivative = M::tanh_slope(inner, t);
             return __fmul_rn(x, __fadd_rn(cdf, __fmul_rn(0.5f, __fmul_rn(u, __fmul_rn(tanh_derivative, inner_derivative)))));
         }
         default: return x;
@@ -140,7 +184,7 @@ __global__ void pointwise_general_kernel(const void* a, const void* b, const voi
     float y = inputs >= 2 ? load_as_f32(b, bv.dtype, broadcast_offset(bv, ov.rank, index)) : 0.0f;
     float z = inputs >= 3 ? load_as_f32(c, cv.dtype, broadcast_offset(cv, ov.rank, index)) : 0.0f;
     int64_t position = mode == DFGPU_PW_GEN_INDEX ? index[s.axis] : 0;
-    store_from_f32(out, ov.dtype, out_offset, pointwise_value(mode, x, y, z, s, position));
+    store_from_f32(out, ov.dtype, out_offset, pointwise_value<true>(mode, x, y, z, s, position));
 }
 
 __global__ void pointwise_kernel(const void* a, const void* b, void* out, View av, View bv, View ov, int mode,
@@ -249,7 +293,7 @@ __device__ __forceinline__ void packed_body(const void* a, const void* b, void* 
         widen(raw_x[u], x);
         if (binary) widen(raw_y[u], y);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) r[j] = pointwise_value(MODE, x[j], y[j], 0.0f, s, 0);
+        for (int j = 0; j < 4; ++j) r[j] = pointwise_value<sizeof(T) == 4>(MODE, x[j], y[j], 0.0f, s, 0);
         store4<T>(out, i, r);
     }
 }
@@ -275,6 +319,149 @@ pointwise_general_packed_kernel(const void* a, const void* b, void* out, int mod
 #undef DFGPU_PW_CASE
         default: break;
     }
+}
+
+// ---- dense tensors with broadcast operands, any count and pointer ------------------------------------------------
+// The output is dense in some order of its axes; an operand has the same order (FULL), only the innermost axes (PERIOD: a bias
+// along the channels), only the outermost ones (REPEAT: a value per row, or one for all), and is indexed by one division per
+// quad. Where rows or pointers do not fall on quads the same kernel goes value by value. 4096 x 3072 bf16 + bias: 118 us
+// with an index computation per value and axis.
+enum { kFull = 0, kPeriod = 1, kRepeat = 2 };
+struct DenseOperand {
+    const void* data;
+    int32_t kind;
+    int32_t vector;       // quads of this operand (or the value a quad repeats) may be read at once
+    FastDivisor by;       // PERIOD: values before it starts again; REPEAT: outputs per value
+};
+
+template <typename T>
+__device__ __forceinline__ float one_value(const void* p, uint32_t i) {
+    if constexpr (sizeof(T) == 4) return __ldg(static_cast<const float*>(p) + i);
+    const uint16_t bits = __ldg(static_cast<const uint16_t*>(p) + i);
+    if constexpr (std::is_same_v<T, __nv_bfloat16>) return __uint_as_float(static_cast<uint32_t>(bits) << 16);
+    return __half2float(__ushort_as_half(bits));
+}
+__device__ __forceinline__ uint32_t dense_index(const DenseOperand& o, uint32_t i) {
+    if (o.kind == kFull) return i;
+    const uint32_t q = fast_divide(i, o.by);
+    return o.kind == kRepeat ? q : i - q * o.by.divisor;
+}
+template <typename T>
+__device__ __forceinline__ void load_dense(const DenseOperand& o, uint32_t i, uint32_t total, float (&v)[4]) {
+    if (o.vector && i + 4 <= total) {
+        const uint32_t at = dense_index(o, i);
+        if (o.kind == kRepeat) v[0] = v[1] = v[2] = v[3] = one_value<T>(o.data, at);
+        else widen(load_quad<T>(o.data, at), v);
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = i + j < total ? one_value<T>(o.data, dense_index(o, i + j)) : 0.0f;
+}
+
+template <typename T, int MODE>
+__device__ __forceinline__ void dense_body(const DenseOperand& a, const DenseOperand& b, void* out, bool out_vector, const PointwiseScalars& s, uint32_t total) {
+    constexpr int U = QuadsInFlight<T>::value;
+    constexpr bool binary = input_count(MODE) == 2;
+    const uint32_t first = (blockIdx.x * U * kPackedThreads + threadIdx.x) * 4;
+    float x[U][4], y[U][4];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const uint32_t i = first + u * kPackedThreads * 4;
+        if (i >= total) break;
+        load_dense<T>(a, i, total, x[u]);
+        if (binary) load_dense<T>(b, i, total, y[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const uint32_t i = first + u * kPackedThreads * 4;
+        if (i >= total) break;
+        float r[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) r[j] = pointwise_value<sizeof(T) == 4>(MODE, x[u][j], binary ? y[u][j] : 0.0f, 0.0f, s, 0);
+        if (out_vector && i + 4 <= total) {
+            store4<T>(out, i, r);
+        } else {
+            for (int j = 0; j < 4; ++j) {
+                if (i + j >= total) break;
+                if constexpr (sizeof(T) == 4) static_cast<float*>(out)[i + j] = r[j];
+                else if constexpr (std::is_same_v<T, __nv_bfloat16>) static_cast<uint16_t*>(out)[i + j] = f32_to_bf16_bits(r[j]);
+                else static_cast<__half*>(out)[i + j] = __float2half_rn(r[j]);
+            }
+        }
+    }
+}
+
+template <typename T, int INPUTS>
+__global__ void __launch_bounds__(kPackedThreads)
+pointwise_dense_kernel(DenseOperand a, DenseOperand b, void* out, int out_vector, int mode, PointwiseScalars s, uint32_t total) {
+    chain_begin();
+    a.data = after_chain(a.data);
+    b.data = after_chain(b.data);
+    switch (mode) {
+#define DFGPU_PW_CASE(M) case M: if constexpr (input_count(M) == INPUTS) dense_body<T, M>(a, b, out, out_vector != 0, s, total); break;
+        DFGPU_PW_EVERY_MODE(DFGPU_PW_CASE)
+#undef DFGPU_PW_CASE
+        default: break;
+    }
+}
+
+// The output's axes from the outermost to the innermost as they lie in memory, or false when there are gaps between them.
+bool dense_order(const dfgpu_tensor& out, int (&order)[DFGPU_MAX_RANK], int& count) {
+    count = 0;
+    for (int i = 0; i < out.rank; ++i)
+        if (out.dim[i] != 1) order[count++] = i;
+    std::stable_sort(order, order + count, [&](int a, int b) { return out.stride[a] > out.stride[b]; });
+    int64_t expected = 1;
+    for (int i = count - 1; i >= 0; --i) {
+        if (out.stride[order[i]] != expected) return false;
+        expected *= out.dim[order[i]];
+    }
+    return expected < (1ll << 31) - 65536;
+}
+
+bool dense_operand(const dfgpu_tensor& t, const dfgpu_tensor& out, const int (&order)[DFGPU_MAX_RANK], int count, const void* data, DenseOperand& o) {
+    const int shift = out.rank - t.rank;
+    int64_t inner = 1, own = 1, held = 1;   // outputs and own values so far, from the innermost axis; outputs per own value
+    int64_t period = 0;                     // set where the operand's axes end
+    for (int i = count - 1; i >= 0; --i) {
+        const int axis = order[i] - shift;
+        const int64_t extent = out.dim[order[i]];
+        if (axis >= 0 && t.dim[axis] == extent && t.stride[axis] == own) {
+            if (period != 0) return false;   // (a broadcast axis between its own)
+            own *= extent;
+        } else if (axis < 0 || t.dim[axis] == 1) {
+            if (own == 1) held *= extent;    // a trailing broadcast axis
+            else if (period == 0) period = inner;
+        } else {
+            return false;
+        }
+        inner *= extent;
+    }
+    const int bytes = dtype_bytes(t.dtype);
+    const bool on_quads = reinterpret_cast<uintptr_t>(data) % (4 * bytes) == 0;
+    o.data = data;
+    o.by = make_fast_divisor(1);
+    if (held > 1) {
+        if (period != 0) return false;
+        o.kind = kRepeat;
+        o.by = make_fast_divisor(static_cast<uint32_t>(held));
+        o.vector = held % 4 == 0;
+    } else if (period != 0) {
+        o.kind = kPeriod;
+        o.by = make_fast_divisor(static_cast<uint32_t>(period));
+        o.vector = period % 4 == 0 && on_quads;
+    } else {
+        o.kind = kFull;
+        o.vector = on_quads;
+    }
+    return true;
+}
+
+template <typename T>
+void launch_dense(int inputs, const DenseOperand& a, const DenseOperand& b, void* out, int mode, const PointwiseScalars& s, int64_t total, cudaStream_t stream) {
+    const int out_vector = reinterpret_cast<uintptr_t>(out) % (4 * sizeof(T)) == 0;
+    if (inputs == 1) launch_chained(pointwise_dense_kernel<T, 1>, dim3(packed_grid<T>(total)), dim3(kPackedThreads), 0, stream, a, b, out, out_vector, mode, s, static_cast<uint32_t>(total));
+    else launch_chained(pointwise_dense_kernel<T, 2>, dim3(packed_grid<T>(total)), dim3(kPackedThreads), 0, stream, a, b, out, out_vector, mode, s, static_cast<uint32_t>(total));
 }
 
 template <typename T>
@@ -357,7 +544,20 @@ extern "C" int dfgpu_pointwise(const dfgpu_pointwise_params* p, void* const* ten
         if (f32_all) launch_packed<float>(inputs, tensors[0], tensors[1], tensors[2], p->mode, s, total, stream);
         else if (f16_all) launch_packed<__half>(inputs, tensors[0], tensors[1], tensors[2], p->mode, s, total, stream);
         else launch_packed<__nv_bfloat16>(inputs, tensors[0], tensors[1], tensors[2], p->mode, s, total, stream);
-    } else if (!simple_mode(p->mode)) {
+        return check_launch("POINTWISE");
+    }
+    if ((f32_all || bf16_all || f16_all) && inputs <= 2 && p->mode != DFGPU_PW_GEN_INDEX) {
+        int order[DFGPU_MAX_RANK], count = 0;
+        DenseOperand a{}, b{};
+        if (dense_order(p->out, order, count) && dense_operand(p->in0, p->out, order, count, tensors[0], a) &&
+            dense_operand(binary ? p->in1 : p->in0, p->out, order, count, binary ? tensors[1] : tensors[0], b)) {
+            if (f32_all) launch_dense<float>(inputs, a, b, tensors[2], p->mode, s, total, stream);
+            else if (f16_all) launch_dense<__half>(inputs, a, b, tensors[2], p->mode, s, total, stream);
+            else launch_dense<__nv_bfloat16>(inputs, a, b, tensors[2], p->mode, s, total, stream);
+            return check_launch("POINTWISE");
+        }
+    }
+    if (!simple_mode(p->mode)) {
         unsigned grid = static_cast<unsigned>((total + 255) / 256);
         launch_chained(pointwise_general_kernel, dim3(grid), dim3(256), 0, stream, tensors[0], tensors[1], inputs >= 3 ? tensors[3] : nullptr, tensors[2],
                                                            make_view(p->in0), inputs >= 2 ? make_view(p->in1) : make_view(p->in0),
