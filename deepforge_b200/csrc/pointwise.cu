@@ -48,21 +48,37 @@ inline bool simple_mode(int mode) { return mode >= DFGPU_PW_ADD && mode <= DFGPU
 // to 8 or 11 significant bits) forms within a few 2^-22 relative, a thousandth of that rounding, because the bytes are half and the
 // instructions set the pace: GELU_BWD on 33.5 M bf16 values is 60 instructions a value with erff and expf, 55.8 us against
 // 30.7 for its bytes.
+// The approximate instructions flush subnormals, which a 16-bit result inside one of these formulas cannot show (EXP itself
+// keeps __expf).
+__device__ __forceinline__ float quick_exp(float v) {
+    float e;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(v * 1.4426950408889634f));
+    return e;
+}
+__device__ __forceinline__ float quick_reciprocal(float v) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
 template <bool EXACT>
 struct Math {
     static __device__ __forceinline__ float exp(float v) { return EXACT ? expf(v) : __expf(v); }
-    static __device__ __forceinline__ float divide(float a, float b) { return EXACT ? __fdiv_rn(a, b) : __fdividef(a, b); }
+    // 1 / (1 + exp(-v)) (FoundationalGraph.cpp:2569-2579)
+    static __device__ __forceinline__ float sigmoid(float v) {
+        if constexpr (EXACT) return __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-v)));
+        return quick_reciprocal(1.0f + quick_exp(-v));
+    }
     static __device__ __forceinline__ float tanh(float v) {
         if constexpr (EXACT) return tanhf(v);
         // 1 - 2 / (1 + e^2v); near zero, where that cancels, the first two terms of the series (4e-8 relative at 0.02)
-        const float far = 1.0f - __fdividef(2.0f, 1.0f + __expf(2.0f * v));
+        const float far = fmaf(-2.0f, quick_reciprocal(1.0f + quick_exp(2.0f * v)), 1.0f);
         return fabsf(v) < 0.02f ? v * fmaf(v * v, -0.33333334f, 1.0f) : far;
     }
     // 1 - tanh^2
     static __device__ __forceinline__ float tanh_slope(float v, float t) {
         if constexpr (EXACT) return __fsub_rn(1.0f, __fmul_rn(t, t));
-        const float e = __expf(-2.0f * fabsf(v)), d = 1.0f + e;   // (4e / (1 + e)^2 does not cancel)
-        return fabsf(v) <= 3.4e38f ? __fdividef(4.0f * e, d * d) : (v != v ? v : 0.0f);
+        const float e = quick_exp(-2.0f * fabsf(v)), r = quick_reciprocal(1.0f + e);   // (4e / (1 + e)^2 does not cancel)
+        return 4.0f * e * r * r;
     }
     // The normal distribution function and exp(-v^2 / 2), which gives it.
     static __device__ __forceinline__ float normal_cdf(float v, float& bell) {
@@ -71,18 +87,14 @@ struct Math {
             return __fmul_rn(0.5f, __fadd_rn(1.0f, erff(__fmul_rn(v, 0.7071067811865475f))));
         }
         // 1 - erf(z) = (a1 t + ... + a5 t^5) e^-z^2, t = 1 / (1 + p z), z = |v| / sqrt 2, within 1.5e-7 (Abramowitz and Stegun,
-        // Handbook of Mathematical Functions, 7.1.26): half of it is the smaller tail.
-        bell = __expf(-0.5f * v * v);
-        const float k = __fdividef(1.0f, fmaf(0.3275911f * 0.70710678f, fabsf(v), 1.0f));
-        const float sum = fmaf(fmaf(fmaf(fmaf(1.061405429f, k, -1.453152027f), k, 1.421413741f), k, -0.284496736f), k, 0.254829592f);
-        const float tail = 0.5f * sum * k * bell;
+        // Handbook of Mathematical Functions, 7.1.26): half of it is the smaller tail, so the coefficients here are halved.
+        bell = quick_exp(-0.5f * v * v);
+        const float k = quick_reciprocal(fmaf(0.3275911f * 0.70710678f, fabsf(v), 1.0f));
+        const float sum = fmaf(fmaf(fmaf(fmaf(0.5f * 1.061405429f, k, 0.5f * -1.453152027f), k, 0.5f * 1.421413741f), k, 0.5f * -0.284496736f), k, 0.5f * 0.254829592f);
+        const float tail = sum * k * bell;
         return v >= 0.0f ? 1.0f - tail : tail;
     }
 };
-
-// 1 / (1 + exp(-v)) (FoundationalGraph.cpp:2569-2579)
-template <bool EXACT>
-__device__ __forceinline__ float sigmoid_value(float v) { return Math<EXACT>::divide(1.0f, __fadd_rn(1.0f, Math<EXACT>::exp(-v))); }
 
 // x, y, z: IN_0, IN_1, IN_2 (0 where the mode has none). u: the activation's input (IN_1 of a _BWD mode, else IN_0).
 template <bool EXACT>
@@ -128,8 +140,8 @@ __device__ __forceinline__ float pointwise_value(int mode, float x, float y, flo
         case DFGPU_PW_RELU_BWD: return __fmul_rn(x, y < s.relu_lower ? s.relu_slope : (y > s.relu_upper ? 0.0f : 1.0f));
         case DFGPU_PW_TANH_FWD: return M::tanh(u);
         case DFGPU_PW_TANH_BWD: return __fmul_rn(x, M::tanh_slope(u, EXACT ? M::tanh(u) : 0.0f));
-        case DFGPU_PW_SIGMOID_FWD: return sigmoid_value<EXACT>(u);
-        case DFGPU_PW_SIGMOID_BWD: { float v = sigmoid_value<EXACT>(u); return __fmul_rn(x, __fmul_rn(v, __fsub_rn(1.0f, v))); }
+        case DFGPU_PW_SIGMOID_FWD: return M::sigmoid(u);
+        case DFGPU_PW_SIGMOID_BWD: { float v = M::sigmoid(u); return __fmul_rn(x, __fmul_rn(v, __fsub_rn(1.0f, v))); }
         case DFGPU_PW_ELU_FWD: { float e = expf(u); return u >= 0.0f ? u : __fmul_rn(s.elu_alpha, __fsub_rn(e, 1.0f)); }
         case DFGPU_PW_ELU_BWD: { float e = M::exp(u); return __fmul_rn(x, u >= 0.0f ? 1.0f : __fmul_rn(s.elu_alpha, e)); }
         case DFGPU_PW_SOFTPLUS_FWD: {
@@ -137,11 +149,11 @@ __device__ __forceinline__ float pointwise_value(int mode, float x, float y, flo
             float logarithm = logf(__fadd_rn(1.0f, expf(-fabsf(scaled))));
             return __fdiv_rn(__fadd_rn(maximum_nan(scaled, 0.0f), logarithm), s.softplus_beta);
         }
-        case DFGPU_PW_SOFTPLUS_BWD: return __fmul_rn(x, sigmoid_value<EXACT>(__fmul_rn(s.softplus_beta, u)));
-        case DFGPU_PW_SWISH_FWD: return __fmul_rn(u, sigmoid_value<EXACT>(__fmul_rn(s.swish_beta, u)));
+        case DFGPU_PW_SOFTPLUS_BWD: return __fmul_rn(x, M::sigmoid(__fmul_rn(s.softplus_beta, u)));
+        case DFGPU_PW_SWISH_FWD: return __fmul_rn(u, M::sigmoid(__fmul_rn(s.swish_beta, u)));
         case DFGPU_PW_SWISH_BWD: {
             float scaled = __fmul_rn(s.swish_beta, u);
-            float v = sigmoid_value<EXACT>(scaled);
+            float v = M::sigmoid(scaled);
             return __fmul_rn(x, __fadd_rn(v, __fmul_rn(scaled, __fmul_rn(v, __fsub_rn(1.0f, v)))));
         }
         case DFGPU_PW_GELU_FWD: case DFGPU_PW_GELU_BWD: {
@@ -346,6 +358,22 @@ __device__ __forceinline__ uint32_t dense_index(const DenseOperand& o, uint32_t 
     const uint32_t q = fast_divide(i, o.by);
     return o.kind == kRepeat ? q : i - q * o.by.divisor;
 }
+// A quad, or the one value it repeats, as it is stored: nothing waits for it before widen_raw().
+template <typename T>
+__device__ __forceinline__ typename Quad<T>::type load_raw(const DenseOperand& o, uint32_t i) {
+    if (o.kind == kRepeat) {
+        typename Quad<T>::type raw{};
+        if constexpr (sizeof(T) == 4) raw.x = __ldg(static_cast<const float*>(o.data) + dense_index(o, i));
+        else raw.x = __ldg(static_cast<const uint16_t*>(o.data) + dense_index(o, i));
+        return raw;
+    }
+    return load_quad<T>(o.data, dense_index(o, i));
+}
+template <typename T>
+__device__ __forceinline__ void widen_raw(const DenseOperand& o, const typename Quad<T>::type& raw, float (&v)[4]) {
+    widen(raw, v);
+    if (o.kind == kRepeat) v[1] = v[2] = v[3] = v[0];
+}
 template <typename T>
 __device__ __forceinline__ void load_dense(const DenseOperand& o, uint32_t i, uint32_t total, float (&v)[4]) {
     if (o.vector && i + 4 <= total) {
@@ -363,21 +391,33 @@ __device__ __forceinline__ void dense_body(const DenseOperand& a, const DenseOpe
     constexpr int U = QuadsInFlight<T>::value;
     constexpr bool binary = input_count(MODE) == 2;
     const uint32_t first = (blockIdx.x * U * kPackedThreads + threadIdx.x) * 4;
-    float x[U][4], y[U][4];
+    if (a.vector && (!binary || b.vector) && out_vector && (blockIdx.x + 1) * U * kPackedThreads * 4 <= total) {
+        typename Quad<T>::type raw_x[U], raw_y[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-        const uint32_t i = first + u * kPackedThreads * 4;
-        if (i >= total) break;
-        load_dense<T>(a, i, total, x[u]);
-        if (binary) load_dense<T>(b, i, total, y[u]);
+        for (int u = 0; u < U; ++u) {   // every load in flight before the first value is used
+            raw_x[u] = load_raw<T>(a, first + u * kPackedThreads * 4);
+            if (binary) raw_y[u] = load_raw<T>(b, first + u * kPackedThreads * 4);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            float x[4], y[4] = {0.0f, 0.0f, 0.0f, 0.0f}, r[4];
+            widen_raw<T>(a, raw_x[u], x);
+            if (binary) widen_raw<T>(b, raw_y[u], y);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) r[j] = pointwise_value<sizeof(T) == 4>(MODE, x[j], y[j], 0.0f, s, 0);
+            store4<T>(out, first + u * kPackedThreads * 4, r);
+        }
+        return;
     }
-#pragma unroll
+#pragma unroll 1
     for (int u = 0; u < U; ++u) {
         const uint32_t i = first + u * kPackedThreads * 4;
         if (i >= total) break;
-        float r[4];
+        float x[4], y[4] = {0.0f, 0.0f, 0.0f, 0.0f}, r[4];
+        load_dense<T>(a, i, total, x);
+        if (binary) load_dense<T>(b, i, total, y);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) r[j] = pointwise_value<sizeof(T) == 4>(MODE, x[u][j], binary ? y[u][j] : 0.0f, 0.0f, s, 0);
+        for (int j = 0; j < 4; ++j) r[j] = pointwise_value<sizeof(T) == 4>(MODE, x[j], y[j], 0.0f, s, 0);
         if (out_vector && i + 4 <= total) {
             store4<T>(out, i, r);
         } else {
