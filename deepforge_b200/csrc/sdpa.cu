@@ -504,30 +504,52 @@ sdpa_paged_decode_kernel(SdpaArgs a, float* __restrict__ partial, int max_chunks
     }
 }
 
-// One CTA of 128 threads per (batch, query head): combine the chunk partials.
+// One CTA of 128 threads per (batch, query head): combine the chunk partials. Latency-bound (a few KB per CTA): the chunks'
+// maxima and sums are read side by side, one chunk per thread, and the weighted sum over chunks has eight loads in flight.
 __global__ void __launch_bounds__(128)
 sdpa_decode_merge_kernel(SdpaArgs a, const float* __restrict__ partial, int max_chunks, int chunk_keys) {
+    __shared__ float weights[128], reduce[8];
     chain_begin();
     partial = after_chain(partial);
     const int64_t row = blockIdx.x;  // b * Hq + h
     const int64_t hq = a.q.dim[1];
     const int64_t ib = row / hq, ih = row % hq;
-    const int d = threadIdx.x;
+    const int d = threadIdx.x, warp = d >> 5, lane = d & 31;
     int64_t lo, hi;
     valid_range(a, ib, 0, lo, hi);
     int chunks = hi > 0 ? static_cast<int>((hi + chunk_keys - 1) / chunk_keys) : 0;
     if (chunks > max_chunks) chunks = max_chunks;
     const float* base = partial + row * max_chunks * kPartialStride;
     float total_max = -INFINITY;
-    for (int c = 0; c < chunks; ++c) total_max = fmaxf(total_max, base[c * kPartialStride + kDecodeD]);
+    for (int c = d; c < chunks; c += 128) total_max = fmaxf(total_max, base[c * kPartialStride + kDecodeD]);
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) total_max = fmaxf(total_max, __shfl_xor_sync(0xffffffffu, total_max, s));
+    if (lane == 0) reduce[warp] = total_max;
+    __syncthreads();
+    total_max = fmaxf(fmaxf(reduce[0], reduce[1]), fmaxf(reduce[2], reduce[3]));
     float total_sum = 0.0f, value = 0.0f;
-    for (int c = 0; c < chunks; ++c) {
-        float m = base[c * kPartialStride + kDecodeD];
-        if (m == -INFINITY) continue;
-        float weight = expf(m - total_max);
-        total_sum = fmaf(base[c * kPartialStride + kDecodeD + 1], weight, total_sum);
-        value = fmaf(base[c * kPartialStride + d], weight, value);
+    for (int first = 0; first < chunks; first += 128) {
+        const int count = min(128, chunks - first);
+        __syncthreads();   // (the weights of the chunks before have been read)
+        if (d < count) {
+            const float* own = base + (first + d) * kPartialStride + kDecodeD;
+            const float m = own[0];
+            const float weight = m == -INFINITY ? 0.0f : expf(m - total_max);
+            weights[d] = weight;
+            total_sum = fmaf(weight == 0.0f ? 0.0f : own[1], weight, total_sum);
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int c = 0; c < count; ++c) {
+            const float o = base[(first + c) * kPartialStride + d];   // (an empty chunk's is never written: not counted)
+            value = weights[c] == 0.0f ? value : fmaf(o, weights[c], value);
+        }
     }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) total_sum += __shfl_xor_sync(0xffffffffu, total_sum, s);
+    if (lane == 0) reduce[4 + warp] = total_sum;
+    __syncthreads();
+    total_sum = reduce[4] + reduce[5] + reduce[6] + reduce[7];
     float result = total_sum > 0.0f ? value / total_sum : 0.0f;
     store_from_f32(a.o_data, a.o.dtype, off4(a.o, ib, ih, 0, d), result);
     if (d == 0) {
@@ -804,7 +826,7 @@ extern "C" int dfgpu_sdpa_forward(const dfgpu_sdpa_params* p, void* const* tenso
         status = launch_decode_umma(*p, tensors, scratch, a.prefix_ok, stream);
         if (status) return status;
         const int chunks = decode_umma_chunks(*p);
-        launch_chained(sdpa_decode_merge_kernel, dim3(static_cast<unsigned>(p->q.dim[0] * p->q.dim[1])), dim3(kDecodeD), 0, stream, a, static_cast<const float*>(scratch), chunks, 1024);
+        launch_chained(sdpa_decode_merge_kernel, dim3(static_cast<unsigned>(p->q.dim[0] * p->q.dim[1])), dim3(kDecodeD), 0, stream, a, static_cast<const float*>(scratch), chunks, decode_umma_chunk_keys(*p));
         return check_launch("SDPA decode merge");
     }
     if (kernel == DFGPU_SDPA_PAGED_DECODE) {

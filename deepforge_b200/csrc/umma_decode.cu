@@ -6,11 +6,11 @@
 // the 128 TMEM lanes (one key per softmax thread) and the GQA group's query heads to columns:
 //     S^T[key, head] = K_tile[key, :] . Q[head, :]          M = 128 keys,  N = 16, K = 128
 //     O^T[d,   head] += V_tile^T[d, key] . P[key, head]     M = 128 (d),   N = 16, K = 128 keys
-// One CTA handles one (sequence, KV head) and up to kTilesPerCta key tiles; a second kernel (the
+// One CTA handles one (sequence, KV head) and up to tiles_per_cta key tiles; a second kernel (the
 // same merge the CUDA-core decode path uses) combines the per-CTA (max, sum, partial O) triples.
 // Two CTAs share an SM (three 32 KiB ring slots each): one CTA's softmax and barrier latencies are
 // covered by the other's loads, which measured 1.6x the bandwidth of one CTA with a five-slot ring.
-// The page ids of a CTA's 1024 keys are fetched once into shared memory.
+// The page ids of a CTA's keys (at most 1024) are fetched once into shared memory.
 // Semantics as the reference (lib/Compiler/SequenceGraph.cpp:1839-1889, 1988-2341): a key is
 // valid iff it lies inside the sequence's [lo, hi) window; a page id outside [0, pages) reads as
 // zeros (its keys score 0 and add nothing to O) and is never dereferenced.
@@ -22,7 +22,7 @@ namespace {
 constexpr int kTileKeys = 128;
 constexpr int kDim = 128;
 constexpr int kHeadsPadded = 16;              // N of both products (GQA group padded)
-constexpr int kTilesPerCta = 8;               // 1024 keys per CTA
+constexpr int kMaxTilesPerCta = 8;            // 1024 keys per CTA, fewer when the CTAs are few (tiles_per_cta())
 constexpr int kKvTileBytes = kTileKeys * kDim * 2;  // 32 KiB
 constexpr int kKvHalfBytes = kKvTileBytes / 2;
 constexpr int kDecodeThreads = 192;
@@ -35,7 +35,7 @@ struct DecodeArgs {
     int32_t pages_per_tile;   // 128 / block
     int32_t table_len_k, table_len_v;
     int32_t num_pages;
-    int32_t max_chunks;
+    int32_t max_chunks, tiles_per_cta;
     int32_t has_left, has_right, bottom_right, padding;
     int64_t left, right, s_kv;
     float scale_log2;
@@ -143,29 +143,7 @@ sdpa_decode_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         prefetch_tensormap(&map_k);
         prefetch_tensormap(&map_v);
     }
-    chain_wait();
-    const int chunk = blockIdx.x;
-    const int kv_head = blockIdx.y;
-    const int64_t batch = blockIdx.z;
-
-    int64_t lo, hi;
-    key_window(args, batch, lo, hi);
-    const int64_t chunk_begin = static_cast<int64_t>(chunk) * kTilesPerCta * kTileKeys;
-    const int64_t chunk_end_all = chunk_begin + kTilesPerCta * kTileKeys;
-    float* my_partial = args.partial + ((batch * args.heads_q + static_cast<int64_t>(kv_head) * G) * args.max_chunks + chunk) * kPartialStride;
-    if (chunk_begin >= hi || chunk_end_all <= lo) {
-        if (threadIdx.x < G) {
-            float* p = my_partial + static_cast<int64_t>(threadIdx.x) * args.max_chunks * kPartialStride;
-            p[kDim] = -INFINITY;
-            p[kDim + 1] = 0.0f;
-        }
-        return;
-    }
-    // tiles of this CTA that intersect the window
-    const int first_tile = lo > chunk_begin ? static_cast<int>((lo - chunk_begin) / kTileKeys) : 0;
-    const int64_t last_key = (hi < chunk_end_all ? hi : chunk_end_all) - 1;
-    const int tiles = static_cast<int>((last_key - chunk_begin) / kTileKeys) + 1 - first_tile;
-
+    // Barriers and tensor memory need nothing of the kernel before: they are ready when it ends.
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
         for (int s = 0; s < kRingSlots; ++s) {
@@ -180,37 +158,58 @@ sdpa_decode_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // Page ids of the (at most 64 + 64) table slots this CTA's 1024 keys map to, fetched once and side by side:
-    // the loader and the softmax threads then read them from shared memory instead of paying a dependent
-    // global load per tile. An id outside the container is stored as -1 (its rows read as zeros).
-    int32_t* page_ids = reinterpret_cast<int32_t*>(generic_base + DecodeSmem::kPages);
-    if (threadIdx.x < 128) {
-        const bool is_v = threadIdx.x >= 64;
-        const int entry = threadIdx.x & 63;
-        const int64_t table_slot = chunk_begin / args.block + entry;
-        int64_t page = -1;
-        const void* offsets = is_v ? args.offsets_v : args.offsets_k;
-        if (entry < kTilesPerCta * args.pages_per_tile && table_slot < (is_v ? args.table_len_v : args.table_len_k)) {
-            if (!offsets) {
-                page = is_v ? args.table_v[batch * args.table_v_stride + table_slot * args.table_v_slot_stride]
-                            : args.table_k[batch * args.table_k_stride + table_slot * args.table_k_slot_stride];
-            } else if (args.prefix_ok[is_v ? 1 : 0]) {
-                const int64_t length = args.seq_kv[batch * args.seq_kv_stride];
-                if (table_slot < (length + args.block - 1) / args.block) {
-                    const int64_t at = batch * (is_v ? args.offsets_v_stride : args.offsets_k_stride);
-                    const int64_t base = (is_v ? args.offsets_v_wide : args.offsets_k_wide) ? static_cast<const int64_t*>(offsets)[at]
-                                                                                          : static_cast<int64_t>(static_cast<const int32_t*>(offsets)[at]);
-                    page = is_v ? args.table_v[base + table_slot * args.table_v_slot_stride] : args.table_k[base + table_slot * args.table_k_slot_stride];
-                }
-            }
-        }
-        page_ids[threadIdx.x] = (page >= 0 && page < args.num_pages) ? static_cast<int32_t>(page) : -1;
-    }
     if (warp == 1) {
         tmem_alloc(tmem_slot, 64);
         tmem_relinquish();
         tc_fence_before();
     }
+    const int chunk = blockIdx.x;
+    const int kv_head = blockIdx.y;
+    const int64_t batch = blockIdx.z;
+    chain_wait();
+
+    // Page ids of the (at most 64 + 64) table slots this CTA's keys map to, fetched once and side by side, and in a strided
+    // table before the sequence length is known: the loader and the softmax threads then read them from shared memory instead of
+    // paying a dependent global load per tile. An id outside the container is stored as -1 (its rows read as zeros).
+    int32_t* page_ids = reinterpret_cast<int32_t*>(generic_base + DecodeSmem::kPages);
+    const bool is_v = threadIdx.x >= 64;
+    const int entry = threadIdx.x & 63, table_slot = chunk * args.tiles_per_cta * args.pages_per_tile + entry;
+    const void* offsets = is_v ? args.offsets_v : args.offsets_k;
+    const bool in_table = threadIdx.x < 128 && entry < args.tiles_per_cta * args.pages_per_tile && table_slot < (is_v ? args.table_len_v : args.table_len_k);
+    int64_t page = -1;
+    if (in_table && !offsets)
+        page = is_v ? args.table_v[batch * args.table_v_stride + table_slot * args.table_v_slot_stride]
+                    : args.table_k[batch * args.table_k_stride + table_slot * args.table_k_slot_stride];
+
+    int64_t lo, hi;
+    key_window(args, batch, lo, hi);
+    const int64_t chunk_begin = static_cast<int64_t>(chunk) * args.tiles_per_cta * kTileKeys;
+    const int64_t chunk_end_all = chunk_begin + args.tiles_per_cta * kTileKeys;
+    float* my_partial = args.partial + ((batch * args.heads_q + static_cast<int64_t>(kv_head) * G) * args.max_chunks + chunk) * kPartialStride;
+    if (chunk_begin >= hi || chunk_end_all <= lo) {
+        if (threadIdx.x < G) {
+            float* p = my_partial + static_cast<int64_t>(threadIdx.x) * args.max_chunks * kPartialStride;
+            p[kDim] = -INFINITY;
+            p[kDim + 1] = 0.0f;
+        }
+        if (warp == 1) tmem_dealloc(*tmem_slot_ptr, 64);
+        return;
+    }
+    // tiles of this CTA that intersect the window
+    const int first_tile = lo > chunk_begin ? static_cast<int>((lo - chunk_begin) / kTileKeys) : 0;
+    const int64_t last_key = (hi < chunk_end_all ? hi : chunk_end_all) - 1;
+    const int tiles = static_cast<int>((last_key - chunk_begin) / kTileKeys) + 1 - first_tile;
+
+    if (in_table && offsets && args.prefix_ok[is_v ? 1 : 0]) {
+        const int64_t length = args.seq_kv[batch * args.seq_kv_stride];
+        if (table_slot < (length + args.block - 1) / args.block) {
+            const int64_t at = batch * (is_v ? args.offsets_v_stride : args.offsets_k_stride);
+            const int64_t base = (is_v ? args.offsets_v_wide : args.offsets_k_wide) ? static_cast<const int64_t*>(offsets)[at]
+                                                                                  : static_cast<int64_t>(static_cast<const int32_t*>(offsets)[at]);
+            page = is_v ? args.table_v[base + table_slot * args.table_v_slot_stride] : args.table_k[base + table_slot * args.table_k_slot_stride];
+        }
+    }
+    if (threadIdx.x < 128) page_ids[threadIdx.x] = (page >= 0 && page < args.num_pages) ? static_cast<int32_t>(page) : -1;
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot_ptr;
@@ -448,7 +447,17 @@ sdpa_decode_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 
 }  // namespace
 
-int decode_umma_chunks(const dfgpu_sdpa_params& p) { return static_cast<int>((p.s_kv + kTilesPerCta * kTileKeys - 1) / (kTilesPerCta * kTileKeys)); }
+// Key tiles per CTA: 8 where that makes three CTAs for every two SMs (148 SMs: a function of the shape alone, as the scratch is), else
+// as many fewer as it takes. A CTA walks its tiles one after the other, ~1.2 us each, so short chunks are what a small batch
+// gains from; with many CTAs long ones save partial results and prologues.
+static int tiles_per_cta(const dfgpu_sdpa_params& p) {
+    const int64_t tiles = (p.s_kv + kTileKeys - 1) / kTileKeys, lists = p.q.dim[0] * p.k.dim[1];
+    int per_cta = kMaxTilesPerCta;
+    while (per_cta > 1 && 2 * lists * ((tiles + per_cta - 1) / per_cta) < 3 * 148) per_cta /= 2;
+    return per_cta;
+}
+int decode_umma_chunk_keys(const dfgpu_sdpa_params& p) { return tiles_per_cta(p) * kTileKeys; }
+int decode_umma_chunks(const dfgpu_sdpa_params& p) { return static_cast<int>((p.s_kv + decode_umma_chunk_keys(p) - 1) / decode_umma_chunk_keys(p)); }
 
 bool decode_umma_supported(const dfgpu_sdpa_params& p) {
     if (p.q.rank != 4 || p.k.rank != 4 || p.v.rank != 4) return false;
@@ -499,6 +508,7 @@ int launch_decode_umma(const dfgpu_sdpa_params& p, void* const* tensors, void* s
     args.table_len_v = static_cast<int>(p.page_table_v.dim[2]);
     args.num_pages = static_cast<int>(pages);
     args.max_chunks = decode_umma_chunks(p);
+    args.tiles_per_cta = tiles_per_cta(p);
     args.has_left = p.has_left_bound;
     args.has_right = p.has_right_bound;
     args.bottom_right = p.bottom_right;
