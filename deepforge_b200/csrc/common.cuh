@@ -85,11 +85,13 @@ cudaError_t submit(const void* function, dim3 grid, dim3 block, unsigned cluster
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The pointer again, but known only from here on: a load through a const __restrict__ pointer counts as independent of
-// memory barriers, so only a data dependence keeps the compiler from moving it above the wait.
+// memory barriers, so only a data dependence keeps the compiler from moving it above the wait. The address passes through
+// as a global one: a pointer of unknown space would make generic loads of what were global ones (22 % on the CUDA-core MATMUL).
 template <typename T>
 __device__ __forceinline__ T* after_chain(T* pointer) {
-    asm volatile("" : "+l"(pointer) :: "memory");
-    return pointer;
+    size_t address = __cvta_generic_to_global(pointer);
+    asm volatile("" : "+l"(address) :: "memory");
+    return static_cast<T*>(__cvta_global_to_generic(address));
 }
 __device__ __forceinline__ void chain_begin() {
     chain_release();

@@ -510,6 +510,8 @@ extern "C" int dfgpu_conv_fprop(const dfgpu_conv_params* p, void* const* tensors
     status = choose_kernel(*p, a, kernel);
     if (status) return status;
     cudaStream_t stream = as_stream(stream_handle);
+    if (p->kernel == DFGPU_CONV_AUTO && kernel == DFGPU_CONV_IGEMM_FFMA && conv_f32_flat(*p, tensors))
+        kernel = DFGPU_CONV_UMMA_F32X3_CLUSTER;
     if (kernel == DFGPU_CONV_UMMA_BF16) return launch_conv_umma(*p, tensors, stream);
     if (kernel == DFGPU_CONV_UMMA_F32X3_CLUSTER) return launch_conv_f32_cluster(*p, a, tensors, stream);  // (any f32 pointer: 4-byte alignment is enough)
     int64_t m_total = p->y.dim[0] * p->y.dim[2] * p->y.dim[3];

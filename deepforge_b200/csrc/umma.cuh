@@ -41,6 +41,11 @@ int conv_f32_device_status(int* status);
 // The same kernel for an unbatched f32 MATMUL (the 1 x 1 convolution of M pixels; B with N or K contiguous).
 bool matmul_f32_cluster_supported(const dfgpu_matmul_params& p);
 int launch_matmul_f32_cluster(const dfgpu_matmul_params& p, void* const* tensors, cudaStream_t stream);
+// Channels-last tensors (row-major matrices) whose reduction the kernel walks flat, 64 (tap, channel) pairs a unit. AUTO takes
+// these at any depth: 7 us where the CUDA-core forms take 8 (16 deep) to 30 (100 deep). Their kernel id stays the
+// CUDA-core one, whose form still takes what is not aligned for this.
+bool conv_f32_flat(const dfgpu_conv_params& p, void* const* tensors);
+bool matmul_f32_flat(const dfgpu_matmul_params& p, void* const* tensors);
 constexpr int64_t kClusterFormMinDepth = 128;  // AUTO takes the one-launch form from this reduction depth (C R S, or K) on: the CUDA-core kernels walk the depth 16 at a time at ~0.8 us a step, the cluster launch costs 7-9 us whatever the depth
 
 // A wide-filter convolution and the 1 x 1 convolution that consumes it, in one persistent kernel (the intermediate
@@ -65,6 +70,28 @@ struct SplitOperand {
 };
 int split_flag_count(const SplitOperand& first, const SplitOperand& second);
 int launch_split6(const SplitOperand& first, const SplitOperand& second, int* flags, cudaStream_t stream);
+
+// The three pieces of an f32 matrix [rows][row_length] as bf16 [3][rows][out_ld], out_ld a multiple of 8 (rows on 16-byte
+// boundaries). `groups` = rows * row_groups groups of four values, below 2^30. The last values of a padded row may be
+// anything: nobody reads past row_length.
+struct PieceOperand {
+    const float* source;
+    uint16_t* pieces;
+    int32_t groups, row_groups, row_length, vector;   // vector: float4 loads
+    FastDivisor by_row;                               // row_groups
+    int64_t source_ld, out_ld, piece_stride;
+};
+int piece_flag_count(const PieceOperand& first, const PieceOperand& second);
+int launch_split3(const PieceOperand& first, const PieceOperand& second, int* flags, cudaStream_t stream);
+// The product of two such matrices (p describes the f32 MATMUL; A's pieces are [3][M][a_ld], B's [3][N][b_ld] or, N-major, [3][K][b_ld]).
+struct PieceMatmul {
+    const uint16_t* a;
+    const uint16_t* b;
+    int64_t a_ld, b_ld;
+    bool b_n_major;
+};
+bool matmul_pieces_supported(const dfgpu_matmul_params& p);
+int launch_matmul_pieces(const dfgpu_matmul_params& p, const PieceMatmul& pieces, void* const* tensors, cudaStream_t stream);
 
 // MATMUL on tcgen05 (umma_matmul.cu): kernel is DFGPU_MATMUL_UMMA_BF16 (bf16 or f16 operands) or DFGPU_MATMUL_UMMA_MXF8 (codes
 // and E8M0 block scales, no dequantize pass). Any extents; rows on 16-byte boundaries.

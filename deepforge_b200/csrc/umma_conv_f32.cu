@@ -54,7 +54,7 @@ constexpr int kInboxBytes = (kTileM + kMaxRanks) * kRowBytes + kMaxRanks * 16;  
 static_assert(kInboxBytes <= kUnitBytes, "the outgoing chunks are parked in the first operand buffer");
 constexpr int kControlOffset = kInboxOffset + kInboxBytes;
 constexpr int kSmemBytes = kControlOffset + 128 + 1024;                    // (+ the slack that aligns the tiles to 1024 bytes)
-constexpr int kAccumulatorColumns = 64;
+constexpr int kAccumulatorColumns = 128;                                   // 64 for the products of the leading pieces, 64 for the others
 
 struct ClusterConvArgs {
     const void* x;
@@ -76,6 +76,8 @@ struct ClusterConvArgs {
     int x_quads, w_quads, y_quads;                // channels are contiguous and every other stride and the pointer a multiple of 16 bytes: float4 accesses
     int w_along_k;                                // output channels are contiguous in the filter (a MATMUL's row-major B): neighbouring threads take neighbouring output channels
     FastDivisor by_q, by_p, by_chunks, by_s;      // output width and height, chunks, filter width
+    int flat_depth;                               // FAST: R * S * C, the length of a filter's row of (tap, channel) pairs
+    FastDivisor by_c;                             // FAST: input channels
 };
 
 __device__ __forceinline__ uint32_t map_to_rank(uint32_t cta_address, uint32_t rank) {
@@ -135,12 +137,15 @@ __device__ __forceinline__ bool split_eight(const float4& a, const float4& b, ui
     return finite;
 }
 
-// FAST: X, W and Y all take float4 accesses (the flags in the arguments are then not looked at).
+// FAST: X, W and Y all take float4 accesses (the flags in the arguments are then not looked at), and a unit is 64 consecutive
+// (tap, channel) pairs of the flat reduction index tap * C + channel instead of 64 channels of one tap: with channels in
+// fours a float4 lies in one tap, and filters with few channels fill their units (5 x 5 over 76 channels: 30 units, not 50).
+// A MATMUL's row-major B (w_along_k) is read value by value, neighbouring threads on neighbouring columns.
 template <bool FAST>
 __global__ void __launch_bounds__(kThreads, 1)
 umma_conv_f32_kernel(const __grid_constant__ ClusterConvArgs g, const __grid_constant__ ConvArgs a) {
     const bool x_quads = FAST || g.x_quads != 0, w_quads = FAST || g.w_quads != 0, y_quads = FAST || g.y_quads != 0;
-    const bool w_along_k = !FAST && g.w_along_k != 0;
+    const bool w_along_k = g.w_along_k != 0;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     cg::cluster_group cluster = cg::this_cluster();
@@ -195,13 +200,21 @@ umma_conv_f32_kernel(const __grid_constant__ ClusterConvArgs g, const __grid_con
         ih0[i] = p * a.stride_h - a.pad_h;
         iw0[i] = q * a.stride_w - a.pad_w;
         id0[i] = volume ? (plane - n * g.depth_out) * a.stride_d - a.pad_d : 0;
-        x_image[i] = n * g.x_n + x_group + x_unit[i] * 8 * g.x_c;
+        x_image[i] = n * g.x_n + x_group + (FAST ? 0 : x_unit[i] * 8 * g.x_c);
     }
     // The filter tile: 64 output channels x 8 groups of 8 input channels. Stored with input channels contiguous, a thread
     // reads its group as two quads; stored with output channels contiguous, neighbouring threads take neighbouring output
     // channels and each reads its 8 input channels one by one.
     const int w_channel = w_along_k ? tid & 63 : tid >> 3, w_unit = w_along_k ? (tid >> 6) & 7 : tid & 7;
     const int w_row = filter_first + (n0 + w_channel < K ? (n0 + w_channel) * g.w_k + w_unit * 8 * g.w_c : 0);   // (rows past the last filter are never read)
+    // One tap: every unit reads the same pixel, whose offset and presence are known here.
+    const bool one_tap = FAST && R * S == 1;
+    if (one_tap)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            live[i] = live[i] && ih0[i] >= 0 && ih0[i] < H && iw0[i] >= 0 && iw0[i] < W;
+            x_image[i] += ih0[i] * g.x_h + iw0[i] * g.x_w;
+        }
     auto eight = [](const void* data, int type, int first, int stride, int count, float4 (&v)[2]) {   // `count` (of eight) values `stride` elements apart, zeros behind them
         float value[8];
 #pragma unroll
@@ -214,6 +227,39 @@ umma_conv_f32_kernel(const __grid_constant__ ClusterConvArgs g, const __grid_con
     const void* w_data = g.w;
     auto fetch = [&](int u, float4 (&xv)[2][2], float4 (&wv)[2]) {
         const int unit = first_unit + u;
+        if constexpr (FAST) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int at = unit * kChunk + x_unit[0] * 8 + 4 * q;
+                if (one_tap) {   // (a matrix product or a 1 x 1 filter: nothing to divide)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+                        xv[i][q] = live[i] && at < g.flat_depth ? __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(x_data) + x_image[i] + at)) : zero;
+                    continue;
+                }
+                const int tap = static_cast<int>(fast_divide(at, g.by_c)), c = at - tap * C;
+                const int r = static_cast<int>(fast_divide(tap, g.by_s)), s = tap - r * S;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int ih = ih0[i] + r * a.dilation_h, iw = iw0[i] + s * a.dilation_w;
+                    xv[i][q] = zero;
+                    if (live[i] && at < g.flat_depth && ih >= 0 && ih < H && iw >= 0 && iw < W)
+                        xv[i][q] = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(x_data) + x_image[i] + ih * g.x_h + iw * g.x_w + c));
+                }
+            }
+            wv[0] = wv[1] = zero;
+            const int first = unit * kChunk + w_unit * 8;
+            if (n0 + w_channel < K && first < g.flat_depth) {
+                if (w_along_k) {
+                    eight(w_data, DFGPU_F32, w_row + unit * kChunk * g.w_c, g.w_c, g.flat_depth - first, wv);
+                } else {
+                    const float4* source = reinterpret_cast<const float4*>(static_cast<const float*>(w_data) + w_row + unit * kChunk);
+                    wv[0] = __ldg(source);
+                    if (first + 4 < g.flat_depth) wv[1] = __ldg(source + 1);
+                }
+            }
+            return;
+        }
         const int tap = static_cast<int>(fast_divide(unit, g.by_chunks)), c0 = (unit - tap * g.chunks) * kChunk;
         const int t = volume ? static_cast<int>(fast_divide(tap, g.by_plane)) : 0, in_plane = tap - t * R * S;
         const int r = static_cast<int>(fast_divide(in_plane, g.by_s)), s = in_plane - r * S;
@@ -322,14 +368,16 @@ umma_conv_f32_kernel(const __grid_constant__ ClusterConvArgs g, const __grid_con
                 const uint32_t a_lo = smem_desc_lo(smem_base + buffer * kUnitBytes, 16);
                 const uint32_t b_lo = smem_desc_lo(smem_base + buffer * kUnitBytes + 3 * kPieceBytesA, 16);
                 if (elect_one()) {
-                    // smallest products first: middle*middle, low*high, high*low, middle*high, high*middle, high*high
+                    // middle*middle, low*high, high*low, middle*high, high*middle meet in an accumulator of their own: the tensor cores
+                    // cut off what a sum does not hold, and beside high*high (2^8 times larger) each would lose as much as it does
+                    // (largest error at 2544 x 120 x 512: 16 units of 2^-24 sum |x w| in one accumulator, 3 in two)
                     constexpr int piece_a[6] = {1, 2, 0, 1, 0, 0}, piece_b[6] = {1, 0, 2, 0, 1, 0};
 #pragma unroll
                     for (int product = 0; product < 6; ++product)
 #pragma unroll
                         for (int k = 0; k < kChunk / 16; ++k)
-                            umma_bf16(tmem_u, desc_words(a_lo + ((piece_a[product] * kPieceBytesA + k * 32) >> 4), smem_desc_hi(1024)),
-                                      desc_words(b_lo + ((piece_b[product] * kPieceBytesB + k * 32) >> 4), smem_desc_hi(1024)), idesc, (u | product | k) != 0 ? 1u : 0u);
+                            umma_bf16(product == 5 ? tmem_u : tmem_u + kTileN, desc_words(a_lo + ((piece_a[product] * kPieceBytesA + k * 32) >> 4), smem_desc_hi(1024)),
+                                      desc_words(b_lo + ((piece_b[product] * kPieceBytesB + k * 32) >> 4), smem_desc_hi(1024)), idesc, (u | k) != 0 || (product != 0 && product != 5) ? 1u : 0u);
                     umma_commit(empty_bar + 8 * buffer);
                 }
                 __syncwarp();
@@ -347,8 +395,13 @@ umma_conv_f32_kernel(const __grid_constant__ ClusterConvArgs g, const __grid_con
         if (my_units > 0) {
             ok = mbar_wait(empty_bar + 8 * ((my_units - 1) & 1), ((my_units - 1) >> 1) & 1, 133) && ok;   // the last commit covers every product
             tc_fence_after();
-            tmem_load_32(*tmem_slot + (static_cast<uint32_t>(quadrant * 32) << 16) + half * 32, r);
+            uint32_t small[32];
+            const uint32_t columns = *tmem_slot + (static_cast<uint32_t>(quadrant * 32) << 16) + half * 32;
+            tmem_load_32(columns, r);
+            tmem_load_32(columns + kTileN, small);
             tmem_load_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__fadd_rn(__uint_as_float(r[i]), __uint_as_float(small[i])));
             tc_fence_before();
         } else {
 #pragma unroll
@@ -541,12 +594,20 @@ const ClusterCapacity& cluster_capacity() {
 
 // The launch itself: all tiles' clusters at once, with fewer ranks per tile when the device cannot co-schedule that many
 // clusters of the first size.
+static bool flat_form(const ClusterConvArgs& g, const ConvArgs& a, bool& w_flat) {
+    auto quads = [](const void* pointer, int type, int64_t channels, int32_t channel_stride, int32_t s0, int32_t s1, int32_t s2) {
+        return type == DFGPU_F32 && channels % 4 == 0 && channel_stride == 1 && s0 % 4 == 0 && s1 % 4 == 0 && s2 % 4 == 0 && (reinterpret_cast<uintptr_t>(pointer) & 15u) == 0;
+    };
+    const int64_t channels = a.c_per_group;
+    // a filter's taps and channels in one row, or the row-major B of a MATMUL
+    w_flat = quads(g.w, g.w_type, channels * g.R * g.S, g.w_c, g.w_k, 0, 0) && (g.S == 1 || g.w_s == channels) && (g.R == 1 || g.w_r == g.S * channels);
+    const bool w_columns = g.w_type == DFGPU_F32 && g.R * g.S == 1 && g.w_k == 1;
+    return quads(g.x, g.x_type, channels, g.x_c, g.x_n, g.x_h, g.x_w) && (w_flat || w_columns) && !a.reverse && a.groups == 1 && g.tiles_per_image == 0 &&
+           g.depth_out * g.depth_in * g.depth_taps == 1 && quads(g.y, g.y_type, a.k_per_group, g.y_k, g.y_n, g.y_p, g.y_q);
+}
 static int launch_clusters(ClusterForm form, ClusterConvArgs g, const ConvArgs& a, const char* what, cudaStream_t stream) {
     const ClusterCapacity& capacity = cluster_capacity();
     if (capacity.error != cudaSuccess) return fail(kExecutionFailed, "%s: cluster launch set-up failed: %s", what, cudaGetErrorString(capacity.error));
-    const int tiles = form.tiles_m * form.tiles_n;
-    while (form.ranks > 1 && capacity.clusters[form.ranks] < tiles) share_units(form, form.ranks - 1);
-    if (capacity.clusters[form.ranks] < 1) return fail(kExecutionFailed, "%s: the device cannot run a cluster of %d CTAs with %d bytes of shared memory", what, form.ranks, kSmemBytes);
     // float4 accesses where the channels are contiguous and everything else falls on 16-byte boundaries
     auto quads = [](const void* pointer, int type, int64_t channels, int group, int32_t channel_stride, int32_t s0, int32_t s1, int32_t s2, int32_t s3) {
         return type == DFGPU_F32 && channels % group == 0 && channel_stride == 1 && s0 % 4 == 0 && s1 % 4 == 0 && s2 % 4 == 0 && s3 % 4 == 0 &&
@@ -554,8 +615,20 @@ static int launch_clusters(ClusterForm form, ClusterConvArgs g, const ConvArgs& 
     };
     g.x_quads = quads(g.x, g.x_type, a.c_per_group, 8, g.x_c, g.x_n, g.x_h, g.x_w, 0);
     g.w_quads = quads(g.w, g.w_type, a.c_per_group, 8, g.w_c, g.w_k, g.w_r, g.w_s, g.w_n);
+    bool w_flat = false;
+    const bool fast = flat_form(g, a, w_flat);
+    const int channels = static_cast<int>(a.c_per_group);
     g.y_quads = quads(g.y, g.y_type, a.k_per_group, 4, g.y_k, g.y_n, g.y_p, g.y_q, 0);
-    g.w_along_k = !g.w_quads && g.w_k == 1;
+    const int tiles = form.tiles_m * form.tiles_n;
+    if (fast) {
+        form.units = (channels * g.R * g.S + kChunk - 1) / kChunk;
+        share_units(form, std::min(std::min(kMaxRanks, form.units), std::max(1, 148 / tiles)));
+    }
+    while (form.ranks > 1 && capacity.clusters[form.ranks] < tiles) share_units(form, form.ranks - 1);
+    if (capacity.clusters[form.ranks] < 1) return fail(kExecutionFailed, "%s: the device cannot run a cluster of %d CTAs with %d bytes of shared memory", what, form.ranks, kSmemBytes);
+    g.w_along_k = fast ? !w_flat : !g.w_quads && g.w_k == 1;
+    g.flat_depth = channels * g.R * g.S;
+    g.by_c = make_fast_divisor(static_cast<uint32_t>(channels));
     g.units = form.units;
     g.units_per_rank = form.units_per_rank;
     g.chunks = form.chunks;
@@ -566,7 +639,6 @@ static int launch_clusters(ClusterForm form, ClusterConvArgs g, const ConvArgs& 
     g.by_chunks = make_fast_divisor(static_cast<uint32_t>(form.chunks));
     g.by_s = make_fast_divisor(static_cast<uint32_t>(g.S));
     g.by_tiles = make_fast_divisor(static_cast<uint32_t>(std::max(1, g.tiles_per_image)));
-    const bool fast = g.x_quads && g.w_quads && g.y_quads && a.groups == 1 && g.tiles_per_image == 0 && g.depth_out * g.depth_in * g.depth_taps == 1;
     cudaError_t error = launch_chained_cluster(fast ? umma_conv_f32_kernel<true> : umma_conv_f32_kernel<false>, dim3(form.ranks, form.tiles_m, form.tiles_n), dim3(kThreads),
                                                static_cast<unsigned>(form.ranks), kSmemBytes, stream, g, a);
     if (error != cudaSuccess) return fail(kExecutionFailed, "%s: cluster launch failed: %s", what, cudaGetErrorString(error));
@@ -578,9 +650,7 @@ bool conv_f32_cluster_supported(const dfgpu_conv_params& p) {
     return cluster_form(p, form);
 }
 
-int launch_conv_f32_cluster(const dfgpu_conv_params& p, const ConvArgs& a, void* const* tensors, cudaStream_t stream) {
-    ClusterForm form;
-    if (!cluster_form(p, form)) return fail(kUnsupported, "CONV_FPROP: the one-launch tcgen05 form needs FLOAT, HALF or BFLOAT16 X, W and Y and at most 64 reduction units (64 channels x one tap) per CTA");
+static ClusterConvArgs conv_cluster_args(const dfgpu_conv_params& p, void* const* tensors) {
     ClusterConvArgs g{};
     g.x = tensors[0], g.w = tensors[1], g.y = tensors[2];
     g.x_type = p.x.dtype, g.w_type = p.w.dtype, g.y_type = p.y.dtype;
@@ -598,7 +668,25 @@ int launch_conv_f32_cluster(const dfgpu_conv_params& p, const ConvArgs& a, void*
     g.x_n = stride(p.x, 0), g.x_c = stride(p.x, 1), g.x_h = stride(p.x, rows), g.x_w = stride(p.x, columns);
     g.w_k = stride(p.w, 0), g.w_c = stride(p.w, 1), g.w_r = stride(p.w, rows), g.w_s = stride(p.w, columns);
     g.y_n = stride(p.y, 0), g.y_k = stride(p.y, 1), g.y_p = stride(p.y, rows), g.y_q = stride(p.y, columns);
-    return launch_clusters(form, g, a, "CONV_FPROP", stream);
+    return g;
+}
+
+int launch_conv_f32_cluster(const dfgpu_conv_params& p, const ConvArgs& a, void* const* tensors, cudaStream_t stream) {
+    ClusterForm form;
+    if (!cluster_form(p, form)) return fail(kUnsupported, "CONV_FPROP: the one-launch tcgen05 form needs FLOAT, HALF or BFLOAT16 X, W and Y and at most 64 reduction units (64 channels x one tap) per CTA");
+    return launch_clusters(form, conv_cluster_args(p, tensors), a, "CONV_FPROP", stream);
+}
+
+bool conv_f32_flat(const dfgpu_conv_params& p, void* const* tensors) {
+    ClusterForm form;
+    if (p.x.rank != 4 || !cluster_form(p, form)) return false;
+    ConvArgs a{};
+    a.groups = static_cast<int32_t>(p.x.dim[1] / p.w.dim[1]);
+    a.c_per_group = p.w.dim[1];
+    a.k_per_group = p.y.dim[1] / a.groups;
+    a.reverse = p.reverse_filter;
+    bool w_flat;
+    return flat_form(conv_cluster_args(p, tensors), a, w_flat);
 }
 
 // ---- MATMUL through the same kernel: C[M, N] = A[M, K] B[K, N] is the 1 x 1 convolution of M pixels with K input and N
@@ -655,12 +743,10 @@ bool matmul_f32_cluster_supported(const dfgpu_matmul_params& p) {
     return matmul_cluster_form(p, f);
 }
 
-int launch_matmul_f32_cluster(const dfgpu_matmul_params& p, void* const* tensors, cudaStream_t stream) {
-    MatmulAsConv f;
-    if (!matmul_cluster_form(p, f)) return fail(kUnsupported, "MATMUL: the one-launch tcgen05 form needs FLOAT, HALF or BFLOAT16 A, B and C and at most one batch axis");
+static ClusterConvArgs matmul_cluster_args(const dfgpu_matmul_params& p, const MatmulAsConv& f, void* const* tensors, ConvArgs& a) {
     // The convolution's view of the problem: one image of 1 x M pixels with K channels in and N out; an epilogue operand
     // [.., M, N] becomes [1, N, 1, M].
-    ConvArgs a{};
+    a = ConvArgs{};
     auto image = [](int64_t channels, int64_t pixels) {
         View v{};
         v.dtype = DFGPU_F32;
@@ -706,8 +792,25 @@ int launch_matmul_f32_cluster(const dfgpu_matmul_params& p, void* const* tensors
     g.x_w = stride(f.m, f.a_m), g.x_c = stride(f.k, f.a_k);   // (one image, one row of pixels: the other strides are never multiplied by anything but 0)
     g.w_k = stride(f.n, f.b_n), g.w_c = stride(f.k, f.b_k);
     g.y_q = stride(f.m, f.c_m), g.y_k = stride(f.n, f.c_n);
+    return g;
+}
+
+int launch_matmul_f32_cluster(const dfgpu_matmul_params& p, void* const* tensors, cudaStream_t stream) {
+    MatmulAsConv f;
+    if (!matmul_cluster_form(p, f)) return fail(kUnsupported, "MATMUL: the one-launch tcgen05 form needs FLOAT, HALF or BFLOAT16 A, B and C and at most one batch axis");
+    ConvArgs a;
+    const ClusterConvArgs g = matmul_cluster_args(p, f, tensors, a);
     return launch_clusters(f.form, g, a, "MATMUL", stream);
 }
+
+bool matmul_f32_flat(const dfgpu_matmul_params& p, void* const* tensors) {
+    MatmulAsConv f;
+    if (!matmul_cluster_form(p, f)) return false;
+    ConvArgs a;
+    bool w_flat;
+    return flat_form(matmul_cluster_args(p, f, tensors, a), a, w_flat);
+}
+
 
 int conv_f32_device_status(int* status) { return read_and_clear_device_status(status); }
 
