@@ -1,4 +1,4 @@
-// f32 operands of a contraction as six-piece bf16 copies for the bf16 tensor cores.
+// f32 operands of a contraction as bf16 pieces for the bf16 tensor cores: six-piece copies, or the three pieces once each.
 //
 // x = xh + xm + xl and w = wh + wm + wl with bf16 pieces (the leading 8 significant bits, the next 8, the last 8; every
 // subtraction that forms them is exact), so x * w = xh*wh + xh*wm + xm*wh + xh*wl + xl*wh + xm*wm up to 2^-24 relative:
@@ -8,6 +8,8 @@
 // A product with an infinite or NaN factor does not survive the split (inf * 0 where the other factor's lower pieces
 // are zero), so every CTA of the split kernel also records whether it saw such a value; the caller launches its
 // CUDA-core kernel behind the tensor-core one, which redoes the contraction when any CTA did.
+#include <algorithm>
+
 #include "common.cuh"
 #include "umma.cuh"
 
@@ -82,7 +84,70 @@ split6_f32_kernel(SplitOperand first, SplitOperand second, int* __restrict__ fla
     if (threadIdx.x == 0) flags[blockIdx.x] = any;
 }
 
+// The three pieces themselves, [3][rows][out_ld], for a kernel that multiplies them pair by pair (umma_matmul.cu). 10 bytes
+// of traffic an f32 value against 16 with the six copies. Every thread keeps four float4 groups in flight; a row's last group
+// may be short, and the groups of an operand off the 16-byte boundaries are read value by value.
+__global__ void __launch_bounds__(256)
+split3_f32_kernel(PieceOperand first, PieceOperand second, int* __restrict__ flags) {
+    chain_wait();
+    chain_release();
+    first.source = after_chain(first.source);
+    second.source = after_chain(second.source);
+    const int total = first.groups + second.groups, step = static_cast<int>(gridDim.x) * 256;
+    bool finite = true;
+    for (int base = blockIdx.x * 256 + threadIdx.x; base < total; base += 4 * step) {
+        float4 v[4];
+        int64_t target[4];   // -1: nothing there
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int64_t at = static_cast<int64_t>(base) + static_cast<int64_t>(i) * step;
+            target[i] = -1;
+            v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (at >= total) continue;
+            const PieceOperand& operand = at < first.groups ? first : second;
+            const int group = static_cast<int>(at < first.groups ? at : at - first.groups);
+            const int row = static_cast<int>(fast_divide(static_cast<uint32_t>(group), operand.by_row)), column = (group - row * operand.row_groups) * 4;
+            const float* source = operand.source + row * operand.source_ld + column;
+            const int live = operand.row_length - column;
+            target[i] = row * operand.out_ld + column;
+            if (operand.vector && live >= 4) {
+                v[i] = __ldg(reinterpret_cast<const float4*>(source));
+            } else {
+                v[i].x = __ldg(source);
+                if (live > 1) v[i].y = __ldg(source + 1);
+                if (live > 2) v[i].z = __ldg(source + 2);
+                if (live > 3) v[i].w = __ldg(source + 3);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (target[i] < 0) continue;
+            const bool in_first = static_cast<int64_t>(base) + static_cast<int64_t>(i) * step < first.groups;
+            uint32_t p0[3], p1[3], p2[3], p3[3];
+            finite = split_f32(v[i].x, p0) && finite;
+            finite = split_f32(v[i].y, p1) && finite;
+            finite = split_f32(v[i].z, p2) && finite;
+            finite = split_f32(v[i].w, p3) && finite;
+            uint16_t* out = (in_first ? first.pieces : second.pieces) + target[i];
+            const int64_t piece = in_first ? first.piece_stride : second.piece_stride;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(out + j * piece) = make_uint2(p0[j] | (p1[j] << 16), p2[j] | (p3[j] << 16));
+        }
+    }
+    const int any = __syncthreads_or(finite ? 0 : 1);
+    if (threadIdx.x == 0) flags[blockIdx.x] = any;
+}
+
 }  // namespace
+
+int piece_flag_count(const PieceOperand& first, const PieceOperand& second) {
+    return static_cast<int>(std::min<int64_t>((static_cast<int64_t>(first.groups) + second.groups + 1023) / 1024, 148 * 6));
+}
+
+int launch_split3(const PieceOperand& first, const PieceOperand& second, int* flags, cudaStream_t stream) {
+    launch_chained(split3_f32_kernel, dim3(piece_flag_count(first, second)), dim3(256), 0, stream, first, second, flags);
+    return check_launch("f32 operand split");
+}
 
 int split_flag_count(const SplitOperand& first, const SplitOperand& second) {
     return static_cast<int>((first.quads + second.quads + kSplitQuadsPerCta - 1) / kSplitQuadsPerCta);

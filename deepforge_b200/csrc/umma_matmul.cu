@@ -1,6 +1,10 @@
 // Matrix products on the 5th-generation tensor cores for every extent: C = steps(A B), A [M, K] with K contiguous, B with
 // K or N contiguous, 16-bit floats (bf16, f16), FP8 codes (MATMUL_FP8) or FP8 codes with E8M0 block scales (MXFP8).
 //
+// kPieces: f32 operands as three bf16 pieces each (split_f32.cu), six products of a K block's tiles per stage: every piece is copied
+// once for two products (six-fold deep copies moved and stored twice as much: 1183 x 1888 x 5360 154 us then, 128 now, 87 of
+// products; 4096^3 586 of 500).
+//
 // Extents are free because the copies are: TMA fills what lies outside a matrix with zeros and clips what would be stored
 // there, so a tile may hang over any edge. Only the rows' starts have to fall on 16-byte boundaries.
 //
@@ -34,7 +38,7 @@ constexpr int kMaxStages = 16;
 constexpr int kMaxSteps = DFGPU_MAX_EPILOGUE;
 constexpr int kSmemBudget = 227 * 1024 - 1024;   // (1 KB of slack aligns the tiles)
 
-enum Kind { kSixteen = 0, kCodes = 1, kScaled = 2 };
+enum Kind { kSixteen = 0, kCodes = 1, kScaled = 2, kPieces = 3 };
 enum { kStepRelu = 1, kStepBias = 2, kStepFull = 3 };
 
 struct TileArgs {
@@ -44,10 +48,11 @@ struct TileArgs {
     int32_t whole_items, items;       // work items: whole tiles, and after them the halves of the tiles that are left for the last round
     int32_t splits, k_per_split;
     int32_t stages, stage_bytes;
-    int32_t acc_stride, scale_columns;   // tensor memory: see launch_problem()
+    int32_t acc_stride, acc_shift, scale_columns;   // tensor memory: see launch_problem(); 1 << acc_shift accumulators
     int32_t a_bytes;                  // A of one CTA and stage; B lies behind it
     int32_t b_box_bytes, b_box_columns;   // B comes in boxes
     int32_t b_mn_major;
+    int32_t a_piece_rows, b_piece_rows;   // kPieces: rows of the maps from one piece to the next
     uint32_t idesc;
     int32_t staging_offset, barrier_offset;
     void* out;
@@ -132,8 +137,9 @@ __device__ __forceinline__ void product(uint32_t d, uint64_t a, uint64_t b, uint
 #define DFGPU_MMA(FORM)                                                                                                   \
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma." FORM " [%0], %1, %2, %3, p;\n\t}"          \
                  ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory")
-    if constexpr (KIND == kSixteen && CG == 1) DFGPU_MMA("cta_group::1.kind::f16");
-    if constexpr (KIND == kSixteen && CG == 2) DFGPU_MMA("cta_group::2.kind::f16");
+    constexpr bool sixteen = KIND == kSixteen || KIND == kPieces;
+    if constexpr (sixteen && CG == 1) DFGPU_MMA("cta_group::1.kind::f16");
+    if constexpr (sixteen && CG == 2) DFGPU_MMA("cta_group::2.kind::f16");
     if constexpr (KIND == kCodes && CG == 1) DFGPU_MMA("cta_group::1.kind::f8f6f4");
     if constexpr (KIND == kCodes && CG == 2) DFGPU_MMA("cta_group::2.kind::f8f6f4");
 #undef DFGPU_MMA
@@ -319,6 +325,15 @@ __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, int cod
     }
 }
 
+// kPieces: 32 columns of the products of the lower pieces onto those of the leading ones.
+__device__ __forceinline__ void add_small_products(uint32_t address, uint32_t (&sum)[32]) {
+    uint32_t small[32];
+    tmem_load_32(address, small);
+    tmem_load_wait();
+#pragma unroll
+    for (int e = 0; e < 32; ++e) sum[e] = __float_as_uint(__fadd_rn(__uint_as_float(sum[e]), __uint_as_float(small[e])));
+}
+
 template <int KIND>
 constexpr int thread_count() { return KIND == kScaled ? 512 : 384; }
 
@@ -405,7 +420,9 @@ __global__ void __launch_bounds__(thread_count<KIND>(), 1)
 umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c,
                    const __grid_constant__ TileArgs args) {
     static_assert(KIND != kScaled || CG == 1, "block scales: one SM per tile (see choose_shape())");
-    constexpr int kCode = KIND == kSixteen ? 0 : (KIND == kCodes ? 20 : 40);
+    constexpr int kCode = KIND == kSixteen ? 0 : (KIND == kCodes ? 20 : (KIND == kScaled ? 40 : 60));
+    constexpr bool kSixteenBits = KIND == kSixteen || KIND == kPieces;
+    constexpr int kPieceCount = KIND == kPieces ? 3 : 1;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* generic_base = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -471,14 +488,20 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 ok = mbar_wait_warp(empty_bar(stage), phase, 501 + kCode);
                 if (!ok) break;
                 if (leader) {
-                    const uint32_t a_dst = smem_base + stage * args.stage_bytes, b_dst = a_dst + args.a_bytes;
                     const uint32_t bar = counted_on + 8u * stage;
-                    constexpr int kPerRow = KIND == kSixteen ? 64 : 128;   // elements of K per block
-                    if (CG == 1 || rank == 0) mbar_expect_tx(full_bar(stage), CG * (args.a_bytes + columns * kRowBytes));
-                    load_tile<CG>(a_dst, &map_a, kb * kPerRow, row0, bar);
-                    for (int j = 0; j < boxes; ++j) {
-                        if (args.b_mn_major) load_tile<CG>(b_dst + j * args.b_box_bytes, &map_b, col0 + j * args.b_box_columns, kb * kPerRow, bar);
-                        else load_tile<CG>(b_dst + j * args.b_box_bytes, &map_b, kb * kPerRow, col0 + j * args.b_box_columns, bar);
+                    constexpr int kPerRow = kSixteenBits ? 64 : 128;   // elements of K per block
+                    if (CG == 1 || rank == 0) mbar_expect_tx(full_bar(stage), CG * kPieceCount * (args.a_bytes + columns * kRowBytes));
+                    // (pieces: the rows of one follow those of the one before in the same map. A tile that hangs over the end of a
+                    // piece reads the next one's first rows, for rows and columns of C that are not stored; past the end of K it is A that holds zeros.)
+#pragma unroll
+                    for (int piece = 0; piece < kPieceCount; ++piece) {
+                        const uint32_t a_dst = smem_base + stage * args.stage_bytes + piece * args.a_bytes;
+                        const uint32_t b_dst = smem_base + stage * args.stage_bytes + kPieceCount * args.a_bytes + piece * (bn / CG) * kRowBytes;
+                        load_tile<CG>(a_dst, &map_a, kb * kPerRow, row0 + piece * args.a_piece_rows, bar);
+                        for (int j = 0; j < boxes; ++j) {
+                            if (args.b_mn_major) load_tile<CG>(b_dst + j * args.b_box_bytes, &map_b, col0 + j * args.b_box_columns, kb * kPerRow + piece * args.b_piece_rows, bar);
+                            else load_tile<CG>(b_dst + j * args.b_box_bytes, &map_b, kb * kPerRow, col0 + j * args.b_box_columns + piece * args.b_piece_rows, bar);
+                        }
                     }
                 }
                 __syncwarp();
@@ -489,13 +512,13 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         // ---- issuing warp (of CTA 0 in a pair) ----
         if (CG == 1 || rank == 0) {
             const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
-            const uint32_t b_lbo = args.b_mn_major ? (KIND == kSixteen ? 64 * kRowBytes : 128 * kRowBytes) : 16;
-            const uint32_t b_step = args.b_mn_major ? (KIND == kSixteen ? 2048u >> 4 : 4096u >> 4) : 32u >> 4;
+            const uint32_t b_lbo = args.b_mn_major ? (kSixteenBits ? 64 * kRowBytes : 128 * kRowBytes) : 16;
+            const uint32_t b_step = args.b_mn_major ? (kSixteenBits ? 2048u >> 4 : 4096u >> 4) : 32u >> 4;
             int stage = 0, local = 0;
             uint32_t phase = 0;
             bool ok = true;
             for (int i = first_item; i < args.items; i += item_step, ++local) {
-                const int width = item_at(args, i).width, acc = local & 1, use = local >> 1;
+                const int width = item_at(args, i).width, acc = local & args.acc_shift, use = local >> args.acc_shift;
                 const uint32_t idesc_wide = args.idesc | (static_cast<uint32_t>(width >> 3) << 17);
                 if (ok) ok = wait_warp<CG == 2>(acc_empty(acc), (use & 1) ^ 1, 502 + kCode);
                 // (where the accumulators overlap, the other one's shared columns must have been read out too)
@@ -506,7 +529,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     ok = mbar_wait_warp(full_bar(stage), phase, 503 + kCode);
                     if (!ok) break;   // (operands by TMA, scales by generic stores + fence.proxy.async: no tcgen05 fence needed)
                     if (leader) {
-                        const uint32_t a_src = smem_base + stage * args.stage_bytes, b_src = a_src + args.a_bytes;   // (with few rows the products read on into B: rows of C nobody stores)
+                        const uint32_t a_src = smem_base + stage * args.stage_bytes, b_src = a_src + kPieceCount * args.a_bytes;   // (with few rows the products read on into B: rows of C nobody stores)
                         const uint32_t a_lo = smem_desc_lo(a_src, 16), b_lo = smem_desc_lo(b_src, b_lbo);
                         uint32_t sf = 0;
                         if constexpr (KIND == kScaled) {
@@ -516,6 +539,19 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                             copy_scales(sf + 4, scales + 512);
                             if (width > 128) copy_scales(sf + 8, scales + 1024);
                         }
+                        if constexpr (KIND == kPieces) {
+                            // middle*middle, low*high, high*low, middle*high, high*middle meet in an accumulator of their own: the tensor
+                            // cores cut off what a sum does not hold, and beside high*high (2^8 times larger) every one of them would lose as much as it does.
+                            constexpr int piece_a[6] = {1, 2, 0, 1, 0, 0}, piece_b[6] = {1, 0, 2, 0, 1, 0};
+                            const uint32_t a_piece = static_cast<uint32_t>(args.a_bytes) >> 4, b_piece = static_cast<uint32_t>(bn / CG * kRowBytes) >> 4;
+#pragma unroll
+                            for (int pair = 0; pair < 6; ++pair)
+#pragma unroll
+                                for (int j = 0; j < 4; ++j)
+                                    product<KIND, CG>(pair == 5 ? d : d + bn, desc_words(a_lo + piece_a[pair] * a_piece + ((j * 32) >> 4), smem_desc_hi(1024)),
+                                                      desc_words(b_lo + piece_b[pair] * b_piece + j * b_step, smem_desc_hi(1024)), idesc_wide,
+                                                      kb != kb_begin || j != 0 || (pair != 0 && pair != 5) ? 1u : 0u, 0u, 0u);
+                        } else
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             uint32_t idesc = idesc_wide;
@@ -546,6 +582,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 uint32_t raw[32];
                 tmem_load_32(tmem_base + lane_base + c * 32, raw);
                 tmem_load_wait();
+                if constexpr (KIND == kPieces) add_small_products(tmem_base + lane_base + bn + c * 32, raw);
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
                     *reinterpret_cast<uint4*>(parked + ((c * 8 + (j ^ (row & 7))) << 4)) = make_uint4(raw[4 * j], raw[4 * j + 1], raw[4 * j + 2], raw[4 * j + 3]);
@@ -559,7 +596,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             bool stored = false;   // (this group has a store in flight)
             int local = 0;
             for (int i = first_item; i < args.items; i += item_step, ++local) {
-                const int acc = local & 1, use = local >> 1;
+                const int acc = local & args.acc_shift, use = local >> args.acc_shift;
                 const Item item = item_at(args, i);
                 const int row0 = (item.m_tile * CG + (CG == 2 ? rank : 0)) * kRows, out_row = row0 + row;
                 const bool row_live = out_row < args.m_total;
@@ -580,6 +617,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         uint32_t raw[32];
                         tmem_load_32(columns + box * box_columns + part * 32, raw);
                         tmem_load_wait();
+                        if constexpr (KIND == kPieces) add_small_products(columns + bn + box * box_columns + part * 32, raw);
                         if (overlapped && b == g && g != acc && part == box_columns / 32 - 1) {   // the shared columns are in registers
                             tc_fence_before();
                             __syncwarp();
@@ -748,6 +786,7 @@ struct Problem {
     int64_t a_ld, b_ld, c_ld;
     bool b_mn_major;
     int in_bytes, out_bytes, out_dtype;
+    int64_t a_rows, b_rows;   // rows the maps span (pieces: three matrices on top of one another)
 };
 
 bool row_ok(int64_t ld, int64_t extent, int bytes) { return ld >= extent && (ld * bytes) % 16 == 0 && ld * bytes < (1ll << 40); }
@@ -765,6 +804,7 @@ bool describe(const dfgpu_tensor& a, const dfgpu_tensor& b, const dfgpu_tensor& 
     if (a.dim[rank - 2] != p.M || b.dim[rank - 2] != p.K || b.dim[rank - 1] != p.N) return false;
     if (p.M < 1 || p.N < 1 || p.K < 1 || p.M > (1ll << 28) || p.N > (1ll << 28) || p.K > (1ll << 28)) return false;
     p.in_bytes = kind == kSixteen ? 2 : 1;
+    p.a_rows = p.M;
     p.out_dtype = c.dtype;
     p.out_bytes = dtype_bytes(c.dtype);
     p.a_ld = a.stride[rank - 2];
@@ -774,6 +814,7 @@ bool describe(const dfgpu_tensor& a, const dfgpu_tensor& b, const dfgpu_tensor& 
     p.b_mn_major = !k_major;
     p.b_ld = k_major ? b.stride[rank - 1] : b.stride[rank - 2];
     if (!k_major && (b.stride[rank - 1] != 1 || !row_ok(p.b_ld, p.N, p.in_bytes))) return false;
+    p.b_rows = k_major ? p.N : p.K;
     p.c_ld = c.stride[rank - 2];
     return c.stride[rank - 1] == 1 && p.c_ld >= p.N;
 }
@@ -781,7 +822,8 @@ bool describe(const dfgpu_tensor& a, const dfgpu_tensor& b, const dfgpu_tensor& 
 // Few rows take little of a stage, so that more stages fit. (A product still reads 128 rows: ring_bytes() keeps the last
 // stage's inside the allocation.)
 int rows_of_a(const Problem& p, int cg) { return cg == 1 && p.M < kRows ? static_cast<int>((p.M + 7) / 8 * 8) : kRows; }
-int stage_bytes(const Problem& p, int bn, int cg, int a_rows) { return (a_rows + bn / cg) * kRowBytes + (p.kind == kScaled ? 2048 : 0); }
+int stage_bytes(const Problem& p, int bn, int cg, int a_rows) { return (a_rows + bn / cg) * kRowBytes * (p.kind == kPieces ? 3 : 1) + (p.kind == kScaled ? 2048 : 0); }
+bool sixteen_bits(const Problem& p) { return p.kind == kSixteen || p.kind == kPieces; }
 int ring_bytes(int stages, int stage_size) { return (stages - 1) * stage_size + std::max(stage_size, kABytes); }
 int stages_that_fit(int stage_size, int budget) {
     int stages = std::min(kMaxStages, budget / stage_size);
@@ -802,14 +844,15 @@ struct Shape {
 //   L2             the same bytes at about 48 per clock and SM when all SMs fetch, or what the ring holds per ~2300 clocks of latency
 // and a round over the SMs costs its blocks (a last round that at most half fills the SMs is cut into half tiles: 4096^3 is 512
 // tiles of 128 x 256 on 148 SMs, three rounds and 68 tiles, which become 136 halves), a fill of ~2000 clocks and the last tile's epilogue. Splitting K divides the
-// blocks and adds ~2500 clocks of exchange (5000 with block scales); 33 clusters of 4 and 15 of 8 fit the chip at once (cudaOccupancyMaxActiveClusters).
+// blocks and adds ~2500 clocks of exchange (5000 with block scales).
 Shape choose_shape(const Problem& p) {
     const int64_t blocks = (p.K * p.in_bytes + kRowBytes - 1) / kRowBytes;
+    constexpr int clusters_at_once[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};   // (cudaOccupancyMaxActiveClusters, by CTAs per cluster)
     const int sms = 148;   // (a function of the shape alone: the count this library is built for)
     Shape best{0, 0, 0, 0, 0, 0, 0.0};
     for (int cg = 1; cg <= (p.kind == kScaled ? 1 : 2); ++cg)
         for (int bn = 64; bn <= 256; bn += 64) {
-            const int chunk = p.kind == kSixteen ? 64 : 128;   // columns of one N-major copy
+            const int chunk = sixteen_bits(p) ? 64 : 128;   // columns of one N-major copy
             if (p.b_mn_major && (bn / cg) % chunk != 0) continue;
             if (p.out_dtype == DFGPU_E4M3 && bn % 128 != 0) continue;   // (whole 128-byte boxes)
             if (p.kind == kScaled && bn % 128 != 0) continue;           // (whole chunks of column scales)
@@ -817,11 +860,12 @@ Shape choose_shape(const Problem& p) {
             if (bn > chunk && bn >= 2 * ((p.N + 63) / 64 * 64)) continue;  // (half the tile would be empty)
             const int64_t m_tiles = (p.M + kRows * cg - 1) / (kRows * cg), n_tiles = (p.N + bn - 1) / bn, tiles = m_tiles * n_tiles;
             const int rows = rows_of_a(p, cg), stage_size = stage_bytes(p, bn, cg, rows);
-            for (int splits = 1; splits <= (cg == 1 ? 8 : 1); splits *= 2) {
+            if (2 * stage_size > kSmemBudget - 2 * kStageBox - 1024) continue;   // (pieces: a second stage has to fit)
+            for (int splits = 1; splits <= (cg == 1 ? 8 : 1); ++splits) {
                 if (splits > 1 && (bn > 128 || splits > blocks || tiles * splits > sms)) break;
                 const int64_t k_per_split = (blocks + splits - 1) / splits;
                 if (splits > 1 && k_per_split * (splits - 1) >= blocks) continue;   // (no CTA without a block)
-                const int64_t slots = splits == 8 ? 15 : (splits == 4 ? 33 : sms / (cg * splits));
+                const int64_t slots = cg == 2 ? sms / 2 : clusters_at_once[splits];
                 double rounds = static_cast<double>((tiles + slots - 1) / slots);
                 int64_t halved = 0;
                 const int half = bn / 2;
@@ -831,7 +875,8 @@ Shape choose_shape(const Problem& p) {
                     rounds -= 0.45;
                 }
                 const double in_flight = static_cast<double>(stages_that_fit(stage_size, kSmemBudget - 2 * kStageBox)) * stage_size;
-                const double block = std::max({2.0 * bn, 2.0 * (rows + bn / cg), (rows + bn / cg) * kRowBytes / std::min(48.0, in_flight / 2300.0)});
+                const double products = p.kind == kPieces ? 6.0 : 1.0, pieces = p.kind == kPieces ? 3.0 : 1.0;
+                const double block = std::max({products * 2.0 * bn, (products + pieces) * (rows + bn / cg), pieces * (rows + bn / cg) * kRowBytes / std::min(48.0, in_flight / 2300.0)});
                 const double clocks = rounds * (k_per_split * block) + 2000.0 + bn * 6.0 + (splits > 1 ? (p.kind == kScaled ? 5000.0 : 2500.0) : 0.0) + (cg == 2 ? 1500.0 : 0.0);
                 if (best.cg == 0 || clocks < best.clocks) best = Shape{cg, bn, splits, static_cast<int>(k_per_split), tiles, halved, clocks};
             }
@@ -853,7 +898,7 @@ int launch_kernel(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUte
 // Everything but the epilogue's operands and the operand formats, which the callers have put into `args`.
 int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* b, void* c, cudaStream_t stream, const char* what) {
     const Shape shape = choose_shape(p);
-    const int chunk = p.kind == kSixteen ? 64 : 128;
+    const int chunk = sixteen_bits(p) ? 64 : 128;
     args.m_total = static_cast<int>(p.M);
     args.n_total = static_cast<int>(p.N);
     args.bn = shape.bn;
@@ -876,7 +921,10 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     args.tma_store = on16(c) && (p.c_ld * p.out_bytes) % 16 == 0 && p.out_dtype != DFGPU_E5M2 ? 1 : 0;
     // Tensor memory: two accumulators, and with block scales 32 columns of them at the end. At bn = 256 the accumulators then
     // overlap by 32 columns, which the epilogue reads out first.
-    args.acc_stride = p.kind == kScaled && shape.bn == 256 ? 224 : shape.bn;
+    // Pieces: an accumulator is two of bn columns (leading and lower products), so that 192 and 256 columns leave room for one: the
+    // epilogue of a tile then runs alone, a few percent of its 6 x K / 64 product steps.
+    args.acc_stride = p.kind == kScaled && shape.bn == 256 ? 224 : (p.kind == kPieces ? 2 * shape.bn : shape.bn);
+    args.acc_shift = p.kind == kPieces && shape.bn > 128 ? 0 : 1;
     args.scale_columns = 480;
     const int staging = shape.splits > 1 || !args.tma_store ? 0 : 2 * kStageBox, barriers = (2 * kMaxStages + 6) * 8;
     args.stages = stages_that_fit(args.stage_bytes, kSmemBudget - staging - barriers);
@@ -886,13 +934,13 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     // instruction descriptor: f32 accumulators (or E8M0 scales), the operand formats the caller has set, B's major, M (N is the item's)
     args.idesc |= (p.kind == kScaled ? 1u << 23 : 1u << 4) | (static_cast<uint32_t>(args.b_mn_major) << 16) |
                   (static_cast<uint32_t>(kRows * shape.cg >> 4) << 24);
-    const CUtensorMapDataType in_type = p.kind == kSixteen ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;   // (copied, never computed on)
+    const CUtensorMapDataType in_type = sixteen_bits(p) ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;   // (copied, never computed on)
     const uint32_t per_row = kRowBytes / p.in_bytes;
     CUtensorMap map_a, map_b, map_c{};
-    int status = encode_map(&map_a, in_type, a, p.K, p.M, p.a_ld * p.in_bytes, per_row, a_rows, what);
+    int status = encode_map(&map_a, in_type, a, p.K, p.a_rows, p.a_ld * p.in_bytes, per_row, a_rows, what);
     if (!status) {
-        if (p.b_mn_major) status = encode_map(&map_b, in_type, b, p.N, p.K, p.b_ld * p.in_bytes, chunk, per_row, what);
-        else status = encode_map(&map_b, in_type, b, p.K, p.N, p.b_ld * p.in_bytes, per_row, static_cast<uint32_t>(args.b_box_columns), what);
+        if (p.b_mn_major) status = encode_map(&map_b, in_type, b, p.N, p.b_rows, p.b_ld * p.in_bytes, chunk, per_row, what);
+        else status = encode_map(&map_b, in_type, b, p.K, p.b_rows, p.b_ld * p.in_bytes, per_row, static_cast<uint32_t>(args.b_box_columns), what);
     }
     if (!status && args.tma_store) {
         const CUtensorMapDataType out_type = p.out_dtype == DFGPU_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : (p.out_dtype == DFGPU_E4M3 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
@@ -903,6 +951,7 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     const int grid = static_cast<int>(groups * (shape.cg == 2 ? 2 : shape.splits));
     if (p.kind == kSixteen) return shape.cg == 2 ? launch_kernel<kSixteen, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kSixteen, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     if (p.kind == kCodes) return shape.cg == 2 ? launch_kernel<kCodes, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kCodes, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
+    if (p.kind == kPieces) return shape.cg == 2 ? launch_kernel<kPieces, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kPieces, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     return launch_kernel<kScaled, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
 }
 
@@ -969,6 +1018,30 @@ bool scaled_problem(const dfgpu_matmul_params& p, Problem& problem) {
 bool matmul_umma_supported(const dfgpu_matmul_params& p, int kernel) {
     Problem problem;
     return kernel == DFGPU_MATMUL_UMMA_MXF8 ? scaled_problem(p, problem) : (kernel == DFGPU_MATMUL_UMMA_BF16 && sixteen_problem(p, problem));
+}
+
+// The pieces' own matrices take the place of A and B: only C and the fused steps have to suit the kernel.
+bool matmul_pieces_supported(const dfgpu_matmul_params& p) {
+    const int rank = p.c.rank;
+    return p.c.stride[rank - 1] == 1 && p.c.stride[rank - 2] >= p.c.dim[rank - 1] && (p.c.dtype == DFGPU_BF16 || p.c.dtype == DFGPU_F16 || p.c.dtype == DFGPU_F32) && translate_steps(p, nullptr, nullptr);
+}
+
+int launch_matmul_pieces(const dfgpu_matmul_params& p, const PieceMatmul& pieces, void* const* tensors, cudaStream_t stream) {
+    const int rank = p.c.rank;
+    Problem problem{};
+    problem.kind = kPieces;
+    problem.M = p.c.dim[rank - 2], problem.N = p.c.dim[rank - 1], problem.K = p.a.dim[rank - 1];
+    problem.a_ld = pieces.a_ld, problem.b_ld = pieces.b_ld, problem.c_ld = p.c.stride[rank - 2];
+    problem.b_mn_major = pieces.b_n_major;
+    problem.in_bytes = 2, problem.out_bytes = dtype_bytes(p.c.dtype), problem.out_dtype = p.c.dtype;
+    problem.a_rows = 3 * problem.M;
+    problem.b_rows = 3 * (pieces.b_n_major ? problem.K : problem.N);
+    TileArgs args{};
+    args.idesc = (1u << 7) | (1u << 10);
+    args.a_piece_rows = static_cast<int>(problem.M);
+    args.b_piece_rows = static_cast<int>(problem.b_rows / 3);
+    translate_steps(p, tensors, &args);
+    return launch_problem(problem, args, pieces.a, pieces.b, tensors[2], stream, "MATMUL (tcgen05)");
 }
 
 int launch_matmul_umma(const dfgpu_matmul_params& p, void* const* tensors, int kernel, cudaStream_t stream) {

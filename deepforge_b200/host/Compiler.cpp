@@ -1112,8 +1112,8 @@ std::uint64_t kernel_alignment(KernelStep const& step, std::size_t slot) {
     switch (step.op) {
         case KernelOp::kConvFprop: return step.kernel == DFGPU_CONV_UMMA_BF16 || step.kernel == DFGPU_CONV_UMMA_F32X3 ? 16 : 0;  // (the one-launch f32 form takes any pointer: see dfgpu_conv_fprop)
         case KernelOp::kMatmul:
-            if (step.kernel != DFGPU_MATMUL_UMMA_BF16 && step.kernel != DFGPU_MATMUL_UMMA_MXF8 && step.kernel != DFGPU_MATMUL_UMMA_F32X3) return 0;
-            if (step.kernel != DFGPU_MATMUL_UMMA_F32X3 && !whole_tiles(std::get<dfgpu_matmul_params>(step.params), step.kernel == DFGPU_MATMUL_UMMA_MXF8 ? 128 : 64)) return 0;
+            if (step.kernel != DFGPU_MATMUL_UMMA_BF16 && step.kernel != DFGPU_MATMUL_UMMA_MXF8) return 0;
+            if (!whole_tiles(std::get<dfgpu_matmul_params>(step.params), step.kernel == DFGPU_MATMUL_UMMA_MXF8 ? 128 : 64)) return 0;
             return slot == 3 || slot == 4 ? 4 : 16;  // the scale tensors are gathered with 4-byte loads
         case KernelOp::kSdpaForward:
             if (step.kernel == DFGPU_SDPA_UMMA) {   // (lengths that are no whole tiles fall back where a pointer is off the boundary, as above)

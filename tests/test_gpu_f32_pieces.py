@@ -1,0 +1,74 @@
+"""The f32 contractions that AUTO picks by size: the flat reduction of the one-launch tensor-core kernel (channels in fours, 1 x 1 to
+5 x 5 filters, either layout of B), three bf16 pieces multiplied pair by pair (large matrix products) and the kernel for
+few rows. Compared with f64.
+
+Tolerances: a tensor-core sum cuts off what an f32 does not hold, at most 2^-23 of sum |x w| for each 16-deep step (twice:
+among a step's products and against what has been summed up), and the pieces leave out products below 2^-23; on the CUDA cores every one of
+K additions and products rounds by at most 2^-24."""
+import numpy as np
+import pytest
+
+from deepforge_b200 import dfgpu, graphs, runtime
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def pieces_bound(depth):
+    return (2 * (-(-depth // 16) + 12) + 8) * 2.0 ** -23   # (12: a rank's last unit is padded to 64, and eight ranks are added)
+
+
+def run(doc, buffers, out):
+    exe = runtime.compile_graph(doc)
+    workspace = torch.empty(max(exe.workspace_size, 1), dtype=torch.uint8, device="cuda")
+    exe.execute({uid: b.data_ptr() for uid, b in {**buffers, **out}.items()}, workspace.data_ptr())
+    torch.cuda.synchronize()
+    assert dfgpu.device_status() == 0
+    return exe
+
+
+@pytest.mark.parametrize("n,c,k,h,w,r", [(1, 4, 4, 8, 8, 1), (1, 12, 20, 9, 11, 3), (2, 8, 28, 17, 13, 3), (1, 76, 68, 10, 9, 5), (3, 16, 64, 8, 16, 1), (1, 60, 128, 15, 15, 1),
+                                         (2, 124, 12, 30, 30, 5), (4, 20, 64, 32, 32, 3), (1, 64, 64, 56, 56, 3)])
+def test_conv_flat_reduction(n, c, k, h, w, r):
+    g = torch.Generator(device="cuda").manual_seed(c * 131 + r)
+    x, f = torch.randn(n, h, w, c, device="cuda", generator=g), torch.randn(k, r, r, c, device="cuda", generator=g)
+    y = torch.full((n, h, w, k), float("nan"), device="cuda")
+    doc = graphs.c1_conv("nhwc", n, c, h, w, k, r, r // 2)
+    uid = {t["name"]: t["uid"] for t in doc["tensors"].values()}
+    names = sorted(uid.values())
+    run(doc, {names[0]: x, names[1]: f}, {names[2]: y})
+    conv = lambda a, b: torch.nn.functional.conv2d(a.double().cpu().permute(0, 3, 1, 2), b.double().cpu().permute(0, 3, 1, 2), padding=r // 2).permute(0, 2, 3, 1)
+    assert torch.all((y.double().cpu() - conv(x, f)).abs() <= pieces_bound(c * r * r) * conv(x.abs(), f.abs()))
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 4, 4), (1, 4232, 1688), (2, 132, 36), (3, 128, 32), (4, 1000, 64), (5, 127, 100), (8, 130, 2052), (9, 8192, 48), (16, 260, 4096),   # few rows
+                                   (17, 64, 64), (100, 120, 68), (131, 100, 76), (500, 8, 1024),                                                                       # flat, shallow
+                                   (129, 516, 4100), (1000, 130, 2052), (2047, 100, 257), (255, 4100, 640), (4097, 68, 130)])                                          # pieces
+@pytest.mark.parametrize("b_k_major", [False, True])
+def test_matmul(m, k, n, b_k_major):
+    g = torch.Generator(device="cuda").manual_seed(m * 7 + n)
+    tensors = [graphs.tensor(1, "A", [m, k]), graphs.tensor(2, "B", [k, n], strides=[1, k] if b_k_major else [n, 1]), graphs.tensor(3, "bias", [1, n]), graphs.tensor(4, "C", [m, n]),
+               graphs.tensor(5, "p", [m, n], virtual=True), graphs.tensor(6, "q", [m, n], virtual=True)]
+    nodes = [graphs.matmul_node("matmul", 1, 2, 5), graphs.pointwise_node("bias", "ADD", 5, 6, 3), graphs.pointwise_node("relu", "RELU_FWD", 6, 4)]
+    a, b, bias = (torch.randn(count, device="cuda", generator=g) for count in (m * k, k * n, n))
+    for shift in (0, 1):   # operands on and off the 16-byte boundaries
+        held = [torch.empty(t.numel() + 4, device="cuda")[shift:shift + t.numel()].copy_(t) for t in (a, b)]
+        c = torch.full((m * n,), float("nan"), device="cuda")
+        run(graphs.document("f32", nodes, tensors), {1: held[0], 2: held[1], 3: bias}, {4: c})
+        fa, fb = a.view(m, k).double(), (b.view(n, k).t() if b_k_major else b.view(k, n)).double()
+        want, weight = torch.relu(fa @ fb + bias.double()), fa.abs() @ fb.abs()
+        bound = max(pieces_bound(k), k * 2.0 ** -24) * weight + 2.0 ** -23 * (weight + bias.abs().double())
+        assert torch.all((c.view(m, n).double() - want).abs() <= bound), float(((c.view(m, n).double() - want).abs() / bound).max())
+
+
+@pytest.mark.parametrize("m,k,n", [(3, 300, 64), (200, 100, 64), (1000, 130, 2052)])
+def test_matmul_with_an_infinity(m, k, n):
+    """inf and NaN come out where an f32 product puts them."""
+    a, b = torch.ones(m, k, device="cuda"), torch.ones(k, n, device="cuda")
+    a[1, k - 1], b[5, 7] = float("inf"), float("nan")
+    c = torch.zeros(m, n, device="cuda")
+    tensors = [graphs.tensor(1, "A", [m, k]), graphs.tensor(2, "B", [k, n]), graphs.tensor(4, "C", [m, n])]
+    run(graphs.document("f32", [graphs.matmul_node("matmul", 1, 2, 4)], tensors), {1: a, 2: b}, {4: c})
+    want = np.full((m, n), float(k), np.float32)
+    want[1, :], want[:, 7] = np.inf, np.nan
+    assert np.array_equal(c.cpu().numpy(), want, equal_nan=True)
