@@ -93,7 +93,8 @@ __device__ __forceinline__ uint32_t address_in(uint32_t own_address, uint32_t ra
     return remote;
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_address) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
+    // (nothing but tensor memory is handed over, which the tcgen05 fences order; released to the cluster, it would wait for all stores)
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
 }
 __device__ __forceinline__ float4 load_from_rank(uint32_t cluster_address) {
     float4 v;

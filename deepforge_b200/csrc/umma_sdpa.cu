@@ -28,7 +28,7 @@ struct SdpaUmmaArgs {
     int32_t heads_q, heads_kv, seq_q, seq_kv;
     int32_t q_tiles, pairs;   // 128-row query tiles and pairs of them, the last one perhaps partly past the end
     int32_t causal;
-    int32_t paired_units;     // causal: a unit of work is a heavy and a light pair (see PairWalker)
+    int32_t order;            // of the work list: kAsStored, kHeavyWithLight or kHeaviestFirst (see PairWalker)
     float scale_log2;  // |attn_scale| * log2(e); a negative scale negates Q in the products
     uint32_t negate_q; // ... through this bit of the instruction descriptor
     const int32_t* len_q;   // SEQ_LEN_Q and SEQ_LEN_KV by batch, or null
@@ -61,6 +61,11 @@ __device__ __forceinline__ void tmem_store_16(uint32_t taddr, const uint32_t (&r
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
           "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
+}
+__device__ __forceinline__ void tmem_store_8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
 }
 __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
@@ -266,23 +271,42 @@ __device__ __forceinline__ PairItem pair_item(const SdpaUmmaArgs& args, int bh, 
     return item;
 }
 
-// The work list of one CTA, the same in every warp role. A head's P query pairs form units: under a causal mask unit i
-// is the heavy pair P-1-i followed by the light pair i, so that every unit walks 2P+2 key tiles and equal numbers of
-// units are equal work; otherwise, or when the single pairs fit the SMs at once, each pair is a unit. CTA c takes units c,
-// c + gridDim.x, ...; neighbouring CTAs thus work on the same head at the same time and share its K and V in L2.
+// The work list of one CTA (or cluster), the same in every warp role.
+//   kAsStored        every query pair of a head is a unit
+//   kHeavyWithLight  causal, many pairs: unit i of a head is the heavy pair P-1-i followed by the light pair i, so that every unit
+//                    walks 2P+2 key tiles and equal numbers of units are equal work
+//   kHeaviestFirst   causal, pairs for a few rounds at most: the pairs of all heads by falling length, and every other round
+//                    in reverse, so that the CTA with the longest pair of one round gets the shortest of the next
+// CTA c takes units c, c + gridDim.x, ...; but for the last order neighbouring CTAs thus work on the same head at the same
+// time and share its K and V in L2.
+enum { kAsStored = 0, kHeavyWithLight = 1, kHeaviestFirst = 2 };
 struct PairWalker {
+    int ctas;   // that walk one list together
     int k = 0;
+    __device__ __forceinline__ explicit PairWalker(int group = 1) : ctas(group) {}
     __device__ __forceinline__ bool next(const SdpaUmmaArgs& args, int& bh, int& pair) {
         const int pairs = args.pairs;
-        const int units_per_head = args.paired_units ? (pairs + 1) >> 1 : pairs;
+        const int places = static_cast<int>(gridDim.x) / ctas, place = static_cast<int>(blockIdx.x) / ctas;   // (the grid is a multiple of ctas)
+        if (args.order == kHeaviestFirst) {
+            const int unit = k * places + ((k & 1) ? places - 1 - place : place);
+            ++k;
+            if (unit >= pairs * args.batch_heads) {   // (a reversed last round may miss this place's unit only, and nothing follows it)
+                return false;
+            }
+            pair = unit / args.batch_heads;
+            bh = unit - pair * args.batch_heads;
+            pair = pairs - 1 - pair;
+            return true;
+        }
+        const int units_per_head = args.order == kHeavyWithLight ? (pairs + 1) >> 1 : pairs;
         const int units = units_per_head * args.batch_heads;
         for (;; ++k) {
-            const int unit = static_cast<int>(blockIdx.x) + (k >> 1) * static_cast<int>(gridDim.x);
+            const int unit = place + (k >> 1) * places;
             if (unit >= units) return false;
             bh = unit / units_per_head;
             const int i = unit - bh * units_per_head;
             pair = i;
-            if (args.paired_units) {
+            if (args.order == kHeavyWithLight) {
                 pair = (k & 1) ? i : pairs - 1 - i;
                 if ((k & 1) && 2 * i == pairs - 1) continue;  // the middle pair of an odd count stands alone
             } else if (k & 1) {
@@ -294,8 +318,8 @@ struct PairWalker {
     }
 };
 template <class Body>
-__device__ __forceinline__ void for_each_pair_item(const SdpaUmmaArgs& args, Body&& body) {
-    PairWalker walker;
+__device__ __forceinline__ void for_each_pair_item(const SdpaUmmaArgs& args, int ctas, Body&& body) {
+    PairWalker walker(ctas);
     int bh, pair;
     while (walker.next(args, bh, pair))  // one call site of the body: it is a whole warp role
         if (!body(bh, pair)) return;
@@ -370,7 +394,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         int slot = 0;
         uint32_t phase = 1;  // parity of the "slot is free" wait
         uint32_t n = 0;      // items started
-        for_each_pair_item(args, [&](int bh, int pair) {
+        for_each_pair_item(args, 1, [&](int bh, int pair) {
             const PairItem item = pair_item<EDGES>(args, bh, pair);
             auto load_box = [&](uint32_t dst, const CUtensorMap* map, int row, int head, uint32_t bar) {
 #pragma unroll
@@ -532,7 +556,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         const bool leader = elect_one();
         uint32_t n = 0;
         bool ok = true;
-        for_each_pair_item(args, [&](int bh, int pair) {
+        for_each_pair_item(args, 1, [&](int bh, int pair) {
             const PairItem item = pair_item<EDGES>(args, bh, pair);
             for (int x = 0; x < 2; ++x) {
                 if (ok) ok = mbar_wait_warp(staged(x), n & 1, 216 + x);
@@ -572,7 +596,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         uint32_t s_count = 0;  // score tiles consumed (parity of s_full)
         uint32_t ring_base = 0;  // ring slots of the items before this one
         bool ok = true;
-        for_each_pair_item(args, [&](int bh, int pair) {
+        for_each_pair_item(args, 1, [&](int bh, int pair) {
         const PairItem item = pair_item<EDGES>(args, bh, pair);
         const int q_tile = item.q_tile_a + x;
         const int q_index = q_tile * kRows + row;
@@ -769,6 +793,536 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     }
 }
 
+// ---- head dimension 128, few pairs: two SMs on a pair of query tiles ----------------------------
+// A score tile lives in tensor memory from the product that writes it to the product that reads its probabilities: 512
+// clocks of Q K^T, some 2600 of softmax and hand-overs, 512 of P V. With room for two tiles (two query tiles of one SM, each
+// with a 128-column accumulator of its own) one tile leaves every ~1840 clocks whatever the order. Here an SM takes
+// ONE query tile, whose accumulator leaves room for THREE score tiles of successive keys, and two SMs (a cluster) share
+// the keys: rows 0-127 on CTA 0, rows 128-255 on CTA 1, one tcgen05.mma.cta_group::2 per step for both, each holding
+// half of the K rows and half of the V columns, so that K and V are fetched and stored once per pair of query tiles as before.
+//   warps 0-7, 8-15  softmax of the even and of the odd key tiles, two threads per query row
+//   warp 16          TMA: own Q rows, own half of every K and V tile, in the order they are read: K0 K1 K2 V0 K3 V1 K4 ...
+//   warp 17          of CTA 0 issues S(0) S(1) S(2) PV(0) S(3) PV(1) S(4) ..., on across items
+//   warp 18          output tiles to global memory by TMA
+// The reference maximum of a row goes from tile to tile: each group passes it on as soon as it has seen its own tile's
+// maximum, before its exponentials. Tensor memory: S(t) and P(t) at 128 (t mod 3), O at 384.
+constexpr int kDuoSlots = 6;
+constexpr int kDuoBuffers = 3;
+struct DuoSmem {
+    static constexpr int kTile = kRows * 128 * 2;
+    static constexpr int kSlot = kTile / 2;             // half a K or V tile
+    static constexpr int kQ = 0;                        // this item's and the next one's
+    static constexpr int kRing = 2 * kTile;
+    static constexpr int kStage = kRing + kDuoSlots * kSlot;
+    static constexpr int kMaxima = kStage + kTile;      // half-row maxima, bf16 [turn 2][group][quarter][half][lane]
+    static constexpr int kReference = kMaxima + 2048;   // f32 [turn 2][group][half][quarter][lane]
+    static constexpr int kSums = kReference + 4096;     // f32 {row sum, its reference, largest dot product} [group][half][row]
+    static constexpr int kBarriers = kSums + 3 * 2048;
+    // stage_free, staged, o_empty, sums_ready, sums_free, v_edge, edge_done, (one spare), q_full[2], q_empty[2], kv_full[S],
+    // kv_empty[S], s_full[3], p_full[3], pv_done[3], passed_on[group][half][quarter]
+    static constexpr int kBarrierCount = 12 + 2 * kDuoSlots + 3 * kDuoBuffers + 16;
+    static constexpr int kTotal = kBarriers + kBarrierCount * 8 + 16;
+    static constexpr int kDynamic = kTotal + 1024;
+};
+
+__device__ __forceinline__ uint32_t duo_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void duo_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t address_in_first(uint32_t own_address) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote) : "r"(own_address));
+    return remote;
+}
+__device__ __forceinline__ void arrive_in_cluster(uint32_t cluster_address) {
+    // (of this CTA's scope, as is the wait: what the waiter's products read is tensor memory, ordered by the tcgen05 fences, and shared
+    // memory behind a proxy fence. Released to the cluster, the arrival waits for every store on its way, and a wait that
+    // acquires from the cluster takes 250 clocks even when it is over at once.)
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
+}
+__device__ __forceinline__ void commit_to_both(uint32_t bar) {
+    const uint16_t both = 3;
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(both) : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+                 ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void duo_scores(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void duo_product(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+// The key tiles of a cluster's work list, one after the other.
+template <bool EDGES>
+struct TileCursor {
+    PairWalker walker;
+    PairItem item;
+    int j;        // key tile of the item
+    uint32_t n;   // items before this one
+    uint32_t t;   // key tiles before this one
+    bool live;
+    __device__ __forceinline__ void take(const SdpaUmmaArgs& args) {
+        int bh, pair;
+        live = walker.next(args, bh, pair);
+        if (live) item = pair_item<EDGES>(args, bh, pair);
+        j = 0;
+    }
+    __device__ __forceinline__ void start(const SdpaUmmaArgs& args) {
+        walker = PairWalker(2);
+        n = t = 0;
+        take(args);
+    }
+    __device__ __forceinline__ bool last() const { return j + 1 == item.tiles; }
+    __device__ __forceinline__ void step(const SdpaUmmaArgs& args) {
+        ++t;
+        if (++j == item.tiles) {
+            ++n;
+            take(args);
+        }
+    }
+};
+// The item's last key tile ends behind the batch's own length: V rows there are cleared.
+__device__ __forceinline__ bool clears_v(const SdpaUmmaArgs& args, const PairItem& item) { return args.len_q != nullptr && item.tiles * kKeys > item.kv_len; }
+
+template <bool F16, bool EDGES>
+__global__ void __launch_bounds__(kPairThreads, 1)
+sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
+                     const __grid_constant__ CUtensorMap map_o, SdpaUmmaArgs args) {
+    using Smem = DuoSmem;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* generic_base = smem_raw + (smem_base - smem_u32(smem_raw));
+    const uint32_t bar_base = smem_base + Smem::kBarriers;
+    const uint32_t stage_free = bar_base, staged = bar_base + 8, o_empty = bar_base + 16, sums_ready = bar_base + 24, sums_free = bar_base + 32, v_edge = bar_base + 40,
+                   edge_done = bar_base + 48;
+    auto q_full = [&](int i) { return bar_base + 8u * (8 + i); };
+    auto q_empty = [&](int i) { return bar_base + 8u * (10 + i); };
+    auto kv_full = [&](int s) { return bar_base + 8u * (12 + s); };
+    auto kv_empty = [&](int s) { return bar_base + 8u * (12 + kDuoSlots + s); };
+    auto s_full = [&](int b) { return bar_base + 8u * (12 + 2 * kDuoSlots + b); };
+    auto p_full = [&](int b) { return bar_base + 8u * (12 + 2 * kDuoSlots + kDuoBuffers + b); };
+    auto pv_done = [&](int b) { return bar_base + 8u * (12 + 2 * kDuoSlots + 2 * kDuoBuffers + b); };
+    auto passed_on = [&](int group, int half, int quarter) { return bar_base + 8u * (12 + 2 * kDuoSlots + 3 * kDuoBuffers + group * 8 + half * 4 + quarter); };
+    const uint32_t tmem_slot = bar_base + 8u * Smem::kBarrierCount;
+    volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(generic_base + Smem::kBarriers + 8 * Smem::kBarrierCount);
+    volatile int* edge_slot = reinterpret_cast<volatile int*>(generic_base + Smem::kBarriers + 8 * Smem::kBarrierCount + 4);
+
+    const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
+    const int rank = static_cast<int>(duo_rank());
+    if (threadIdx.x == 0) {
+        prefetch_tensormap(&map_q);
+        prefetch_tensormap(&map_k);
+        prefetch_tensormap(&map_v);
+        prefetch_tensormap(&map_o);
+        mbar_init(stage_free, 1);
+        mbar_init(staged, 8);
+        mbar_init(o_empty, 16);
+        mbar_init(sums_ready, 8);
+        mbar_init(sums_free, 8);
+        mbar_init(v_edge, 1);
+        mbar_init(edge_done, 8);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(q_full(i), 1);
+            mbar_init(q_empty(i), 1);
+        }
+        for (int s = 0; s < kDuoSlots; ++s) {
+            mbar_init(kv_full(s), 1);
+            mbar_init(kv_empty(s), 1);
+        }
+        for (int b = 0; b < kDuoBuffers; ++b) {
+            mbar_init(s_full(b), 1);
+            mbar_init(p_full(b), 16);
+            mbar_init(pv_done(b), 1);
+        }
+        for (int i = 0; i < 16; ++i) mbar_init(passed_on(0, 0, 0) + 8u * i, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 17) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        tc_fence_before();
+    }
+    __syncthreads();
+    duo_sync();   // both CTAs' barriers exist before either touches the other's
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot_ptr;
+    chain_wait();
+    chain_release();
+
+    if (warp == 16) {
+        const bool leader = elect_one();
+        const uint32_t counted_on = address_in_first(bar_base);   // CTA 0's barriers count both CTAs' bytes
+        TileCursor<EDGES> k, v;
+        k.start(args);
+        v.start(args);
+        int slot = 0;
+        uint32_t phase = 1, edges = 0;
+        bool ok = true;
+        auto next_slot = [&] { if (++slot == kDuoSlots) { slot = 0; phase ^= 1; } };
+        auto put_k = [&] {
+            if (!k.live || !ok) return;
+            if (k.j == 0) {
+                const int buffer = k.n & 1;
+                ok = mbar_wait_warp(q_empty(buffer), ((k.n >> 1) & 1) ^ 1, 240);
+                if (leader && ok) {
+                    if (rank == 0) mbar_expect_tx(q_full(buffer), 2 * Smem::kTile);
+                    for (int h = 0; h < 2; ++h)
+                        tma_load_4d_pair(smem_base + Smem::kQ + buffer * Smem::kTile + h * kHalfBytes, &map_q, 64 * h, (k.item.q_tile_a + rank) * kRows, k.item.head, k.item.batch,
+                                         counted_on + (q_full(buffer) - bar_base));
+                }
+            }
+            if (ok) ok = mbar_wait_warp(kv_empty(slot), phase, 241);
+            if (leader && ok) {
+                if (rank == 0) mbar_expect_tx(kv_full(slot), 2 * Smem::kSlot);
+                for (int h = 0; h < 2; ++h)
+                    tma_load_4d_pair(smem_base + Smem::kRing + slot * Smem::kSlot + h * (Smem::kSlot / 2), &map_k, 64 * h, k.j * kKeys + rank * 64, k.item.kv_head, k.item.batch,
+                                     counted_on + (kv_full(slot) - bar_base));
+            }
+            __syncwarp();
+            next_slot();
+            k.step(args);
+        };
+        for (int i = 0; i < kDuoBuffers; ++i) put_k();
+        while (v.live && ok) {
+            const bool edge = EDGES && v.last() && clears_v(args, v.item);
+            ok = mbar_wait_warp(kv_empty(slot), phase, 242);
+            // (a tile whose end is cleared is counted on a barrier of its own CTA, where the clearing warps wait for it)
+            if (edge && ok) ok = mbar_wait_warp(edge_done, (edges & 1) ^ 1, 243);
+            if (leader && ok) {
+                const uint32_t dst = smem_base + Smem::kRing + slot * Smem::kSlot;
+                if (edge) {
+                    *edge_slot = slot;
+                    if (rank == 0) mbar_arrive(kv_full(slot));
+                    mbar_expect_tx(v_edge, Smem::kSlot);
+                    tma_load_4d(dst, &map_v, 64 * rank, v.j * kKeys, v.item.kv_head, v.item.batch, v_edge);
+                } else {
+                    if (rank == 0) mbar_expect_tx(kv_full(slot), 2 * Smem::kSlot);
+                    tma_load_4d_pair(dst, &map_v, 64 * rank, v.j * kKeys, v.item.kv_head, v.item.batch, counted_on + (kv_full(slot) - bar_base));
+                }
+            }
+            __syncwarp();
+            edges += edge ? 1 : 0;
+            next_slot();
+            v.step(args);
+            put_k();
+        }
+    } else if (warp == 17) {
+        if (rank == 0) {
+            const bool leader = elect_one();
+            constexpr uint32_t kFormats = (1u << 4) | (F16 ? 0u : (1u << 7) | (1u << 10)) | (static_cast<uint32_t>(2 * kRows >> 4) << 24);
+            const uint32_t idesc_qk = kFormats | (static_cast<uint32_t>(kKeys >> 3) << 17) | args.negate_q;
+            constexpr uint32_t idesc_pv = kFormats | (static_cast<uint32_t>(128 >> 3) << 17) | (1u << 16);   // (V is read MN-major)
+            constexpr uint32_t kDescHi = smem_desc_hi(1024);
+            const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+            TileCursor<EDGES> s, p;
+            s.start(args);
+            p.start(args);
+            int slot = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            auto next_slot = [&] { if (++slot == kDuoSlots) { slot = 0; phase ^= 1; } };
+            auto put_scores = [&] {
+                if (!s.live || !ok) return;
+                const int q = s.n & 1, b = static_cast<int>(s.t % kDuoBuffers);
+                if (s.j == 0) ok = mbar_wait_warp(q_full(q), (s.n >> 1) & 1, 244);
+                if (ok) ok = mbar_wait_warp(kv_full(slot), phase, 245);
+                tc_fence_after();
+                if (leader && ok) {
+                    const uint32_t q_lo = smem_desc_lo(smem_base + Smem::kQ + q * Smem::kTile, 16), k_lo = smem_desc_lo(smem_base + Smem::kRing + slot * Smem::kSlot, 16);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        duo_scores(tmem_u + b * 128, desc_words(q_lo + (((k >> 2) * kHalfBytes + (k & 3) * 32) >> 4), kDescHi),
+                                   desc_words(k_lo + (((k >> 2) * (Smem::kSlot / 2) + (k & 3) * 32) >> 4), kDescHi), idesc_qk, k != 0 ? 1u : 0u);
+                    commit_to_both(s_full(b));
+                    commit_to_both(kv_empty(slot));
+                    if (s.last()) commit_to_both(q_empty(q));
+                }
+                __syncwarp();
+                next_slot();
+                s.step(args);
+            };
+            for (int i = 0; i < kDuoBuffers; ++i) put_scores();
+            while (p.live && ok) {
+                const int b = static_cast<int>(p.t % kDuoBuffers);
+                if (p.j == 0) ok = mbar_wait_warp(o_empty, (p.n & 1) ^ 1, 246);
+                if (ok) ok = mbar_wait_warp(kv_full(slot), phase, 247);
+                if (ok) ok = mbar_wait_warp(p_full(b), (p.t / kDuoBuffers) & 1, 248);
+                tc_fence_after();
+                if (leader && ok) {
+                    const uint32_t v_lo = smem_desc_lo(smem_base + Smem::kRing + slot * Smem::kSlot, kHalfBytes), p_tmem = tmem_u + b * 128;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        duo_product(tmem_u + 384, p_tmem + (k >> 2) * 64 + (k & 3) * 8, desc_words(v_lo + ((k * 2048) >> 4), kDescHi), idesc_pv, (p.j | k) != 0 ? 1u : 0u);
+                    commit_to_both(pv_done(b));
+                    commit_to_both(kv_empty(slot));
+                }
+                __syncwarp();
+                next_slot();
+                p.step(args);
+                put_scores();   // (into the buffer just read: the products of one thread run in order)
+            }
+        }
+    } else if (warp == 18) {
+        const bool leader = elect_one();
+        uint32_t n = 0;
+        bool ok = true;
+        for_each_pair_item(args, 2, [&](int bh, int pair) {
+            const PairItem item = pair_item<EDGES>(args, bh, pair);
+            if (ok) ok = mbar_wait_warp(staged, n & 1, 249);
+            if (leader) {
+                const int row = (item.q_tile_a + rank) * kRows;
+                if (ok && g_device_status == 0 && row < args.seq_q)
+                    for (int h = 0; h < 2; ++h) tma_store_4d(&map_o, smem_base + Smem::kStage + h * kHalfBytes, 64 * h, row, item.head, item.batch);
+                tma_store_commit();
+                tma_store_wait_read<0>();
+                mbar_arrive(stage_free);
+            }
+            __syncwarp();
+            ++n;
+            return true;
+        });
+        if (leader) tma_store_wait_all();
+    } else {
+        const int group = warp >> 3, half = (warp >> 2) & 1, quarter = warp & 3;
+        const int row = quarter * 32 + lane;
+        const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
+        const uint32_t tmem_o = tmem_base + lane_base + 384 + half * 64;
+        const float scale = args.scale_log2;
+        const uint64_t scale2 = pack2(scale, scale);
+        const int pair_barrier = 1 + group * 4 + quarter;   // the 64 threads of this group that share these 32 rows
+        uint16_t* maxima = reinterpret_cast<uint16_t*>(generic_base + Smem::kMaxima) + (group * 4 + quarter) * 64 + lane;          // + turn * 512 + half * 32
+        float* reference = reinterpret_cast<float*>(generic_base + Smem::kReference) + (half * 4 + quarter) * 32 + lane;           // + turn * 512 + group * 256
+        float* sums_of = reinterpret_cast<float*>(generic_base + Smem::kSums) + row;   // + 512 * {sum, reference, largest} + (group * 2 + half) * 128
+        const uint32_t p_full_first = address_in_first(p_full(0)), o_empty_first = address_in_first(o_empty);
+        uint32_t n = 0, t0 = 0, edges = 0;
+        uint32_t mine_done = 0;   // key tiles this group has finished (parity of its maxima and references)
+        bool ok = true;
+        for_each_pair_item(args, 2, [&](int bh, int pair) {
+            const PairItem item = pair_item<EDGES>(args, bh, pair);
+            const int q_tile = item.q_tile_a + rank, q_index = q_tile * kRows + row;
+            const bool idle_tile = q_tile * kRows >= item.live_q;   // no row of this CTA's has keys
+            float m_ref = -INFINITY, l_sum = 0.0f, raw_max = -INFINITY;
+            // The reference after key tile t, as the other group passed it on. That group's own count of tiles gives buffer and phase:
+            // tiles of its parity before t.
+            auto passed = [&](uint32_t t) {
+                const uint32_t turn = t >> 1;   // (tile t is the turn-th of its group)
+                if (ok) ok = mbar_wait(passed_on(group ^ 1, half, quarter), turn & 1, 250);
+                return reference[(turn & 1) * 512 + (group ^ 1) * 256];
+            };
+            for (int j = static_cast<int>((t0 ^ group) & 1); j < item.tiles; j += 2, ++mine_done) {
+                const uint32_t t = t0 + j;
+                const int b = static_cast<int>(t % kDuoBuffers);
+                const uint32_t tmem_s = tmem_base + lane_base + b * 128 + half * 64;
+                // (S(t) follows PV(t - 3): what this tile's turn of the buffers held before has been read, and no barrier below is more than one phase behind)
+                if (ok) ok = mbar_wait(s_full(b), (t / kDuoBuffers) & 1, 251);
+                tc_fence_after();
+                const bool empty = idle_tile || (args.causal && j > q_tile);   // nothing to see for any row: all probabilities are zero
+                const int last_key = !EDGES ? q_index : (args.causal ? min(q_index, item.kv_len - 1) : item.kv_len - 1);
+                const int limit = last_key - j * kKeys - half * 64;
+                const bool diagonal = (args.causal && j == q_tile) || (EDGES && (j + 1) * kKeys > item.kv_len);
+                // The tile's maximum first, then the reference, then the exponentials: nothing is formed twice. (The scores are read
+                // twice, which costs next to nothing; 64 of them held in registers would spill.)
+                float mine = -INFINITY;
+                auto masked = [&](uint32_t (&raw)[16], int c) {
+                    if (diagonal) {
+#pragma unroll
+                        for (int e = 0; e < 16; ++e)
+                            if (c * 16 + e > limit) raw[e] = 0xff800000u;  // -inf
+                    }
+                };
+                if (!empty) {
+                    uint32_t raw[4][16];
+                    tmem_load_16(tmem_s, raw[0]);
+                    tmem_load_16(tmem_s + 16, raw[1]);
+#pragma unroll
+                    for (int c = 0; c < 4; c += 2) {
+                        tmem_load_wait_for(raw[c]);
+                        tmem_load_wait_for(raw[c + 1]);
+                        if (c < 2) {
+                            tmem_load_16(tmem_s + 32, raw[2]);
+                            tmem_load_16(tmem_s + 48, raw[3]);
+                        }
+                        masked(raw[c], c);
+                        masked(raw[c + 1], c + 1);
+                        mine = max_of_16(raw[c + 1], max_of_16(raw[c], mine));
+                    }
+                }
+                raw_max = fmaxf(raw_max, mine);
+                // Half-row maxima as bf16 rounded towards +inf: any reference not below the true maximum by more than the threshold
+                // serves, and both threads must arrive at the same value. (Two buffers: the other warp may still be reading the
+                // last tile's when this one writes.)
+                const uint32_t turn = mine_done & 1;
+                const uint32_t mine_bits = __float_as_uint(mine);
+                const uint32_t mine_up = (mine_bits & 0x80000000u) ? (mine_bits & 0xffff0000u) : ((mine_bits + 0xffffu) & 0xffff0000u);
+                maxima[turn * 512 + half * 32] = static_cast<uint16_t>(mine_up >> 16);
+                asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
+                const float other = __uint_as_float(static_cast<uint32_t>(maxima[turn * 512 + (half ^ 1) * 32]) << 16);
+                const float tile_max = fmaxf(__uint_as_float(mine_up), other) * scale;
+                float before = t > 0 ? passed(t - 1) : -INFINITY;   // (at an item's start for the order alone: the other group has taken what this one passed on last)
+                if (j == 0) before = -INFINITY;
+                // raise the reference only when it would grow by more than the threshold (or on the first tile)
+                const bool raise = __any_sync(0xffffffffu, tile_max > before + kRescaleThreshold) != 0;
+                const float m_new = raise ? fmaxf(before, tile_max) : before;
+                reference[turn * 512 + group * 256] = m_new;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(passed_on(group, half, quarter));
+                if (__any_sync(0xffffffffu, m_new != m_ref)) {
+                    l_sum *= m_ref == -INFINITY ? 0.0f : ex2_fast(m_ref - m_new);
+                    m_ref = m_new;
+                }
+                uint64_t sums[2] = {0, 0};
+                if (!empty) {
+                    // (probabilities go over columns whose scores have been read: 8 columns for every 16)
+                    const uint64_t bias2 = pack2(-m_ref, -m_ref);
+                    uint32_t raw[4][16];
+                    tmem_load_16(tmem_s, raw[0]);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        tmem_load_wait_for(raw[c]);
+                        if (c < 3) tmem_load_16(tmem_s + (c + 1) * 16, raw[c + 1]);
+                        masked(raw[c], c);
+                        uint32_t packed[8];
+                        probabilities_of_16<F16>(raw[c], scale2, bias2, sums, packed);
+                        tmem_store_8(tmem_s + c * 8, packed);
+                    }
+                } else {
+                    const uint32_t zeros[8] = {};
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) tmem_store_8(tmem_s + c * 8, zeros);
+                }
+                {
+                    float lo, hi;
+                    unpack2(add2(sums[0], sums[1]), lo, hi);
+                    l_sum += lo + hi;
+                }
+                if (raise && j > 0) {
+                    // O holds P V up to the tile before once that product is done; this tile's waits for these probabilities.
+                    const float alpha = before == -INFINITY ? 0.0f : ex2_fast(before - m_new);
+                    if (ok) ok = mbar_wait(pv_done((t - 1) % kDuoBuffers), ((t - 1) / kDuoBuffers) & 1, 252);
+                    tc_fence_after();
+#pragma unroll 1
+                    for (int c = 0; c < 4; ++c) {
+                        uint32_t acc[16];
+                        tmem_load_16(tmem_o + c * 16, acc);
+                        tmem_load_wait_for(acc);
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) acc[e] = __float_as_uint(__uint_as_float(acc[e]) * alpha);
+                        tmem_store_16(tmem_o + c * 16, acc);
+                    }
+                }
+                if (EDGES && half == 0 && j + 1 == item.tiles && clears_v(args, item)) {
+                    // V rows past the batch's length are not this sequence's: this CTA's channels of them, a row per thread
+                    if (ok) ok = mbar_wait(v_edge, edges & 1, 253);
+                    if (j * kKeys + row >= item.kv_len) {
+                        uint8_t* v_row = generic_base + Smem::kRing + *edge_slot * Smem::kSlot + row * 128;
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) *reinterpret_cast<uint4*>(v_row + u * 16) = make_uint4(0, 0, 0, 0);
+                    }
+                    fence_async_shared();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(edge_done);
+                }
+                tmem_store_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) arrive_in_cluster(p_full_first + 8u * b);
+            }
+            const uint32_t last = t0 + item.tiles - 1;
+            if (EDGES && clears_v(args, item)) {
+                // (the group that does not clear waits and arrives as well: a barrier's phases are told apart by their parity, so nobody may
+                // be more than one behind or ahead)
+                if (half == 0 && (last & 1) != static_cast<uint32_t>(group)) {
+                    if (ok) ok = mbar_wait(v_edge, edges & 1, 258);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(edge_done);
+                }
+                ++edges;
+            }
+            // ---- the item's end: the group without the last tile leaves its sums, the other one finishes the rows ----
+            t0 += item.tiles;
+            float* own = sums_of + (group * 2 + half) * 128;
+            if (ok) ok = mbar_wait(sums_free, (n & 1) ^ 1, 254);   // (the last item's sums have been read)
+            if ((last & 1) != static_cast<uint32_t>(group)) {
+                own[0] = l_sum;
+                own[512] = m_ref;
+                own[1024] = raw_max;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(sums_ready);
+            } else {
+                if (ok) ok = mbar_wait(sums_ready, n & 1, 255);
+                own[0] = l_sum;
+                own[1024] = raw_max;
+                asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
+                float total = sums_of[group * 256] + sums_of[group * 256 + 128], row_raw_max = fmaxf(sums_of[group * 256 + 1024], sums_of[group * 256 + 128 + 1024]);
+                const float other_ref = sums_of[512 + (group ^ 1) * 256];   // (both halves of a row know the same reference)
+                if (other_ref != -INFINITY) {
+                    total += (sums_of[(group ^ 1) * 256] + sums_of[(group ^ 1) * 256 + 128]) * ex2_fast(other_ref - m_ref);
+                    row_raw_max = fmaxf(row_raw_max, fmaxf(sums_of[(group ^ 1) * 256 + 1024], sums_of[(group ^ 1) * 256 + 128 + 1024]));
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(sums_free);
+                const bool live = !EDGES ? true : q_index < item.live_q;
+                if (half == 0 && ok && q_index < args.seq_q) {
+                    const int64_t b64 = item.batch, h64 = item.head, q64 = q_index;
+                    if (args.row_max != nullptr)
+                        args.row_max[b64 * args.max_stride[0] + h64 * args.max_stride[1] + q64 * args.max_stride[2]] = live ? row_raw_max * args.attn_scale : -INFINITY;
+                    if (args.row_sum != nullptr)  // the sum was accumulated against m_ref; re-express it against the true maximum
+                        args.row_sum[b64 * args.sum_stride[0] + h64 * args.sum_stride[1] + q64 * args.sum_stride[2]] = live ? total * exp2f(m_ref - row_raw_max * scale) : 0.0f;
+                    if (args.stats != nullptr)
+                        args.stats[b64 * args.stats_batch_stride + h64 * args.stats_head_stride + q64 * args.stats_row_stride] =
+                            live ? 0.6931471805599453f * (m_ref + log2f(total)) : -INFINITY;
+                }
+                const float inverse = live ? 1.0f / total : 0.0f;
+                if (ok) ok = mbar_wait(stage_free, (n & 1) ^ 1, 256);
+                if (ok) ok = mbar_wait(pv_done(last % kDuoBuffers), (last / kDuoBuffers) & 1, 257);
+                tc_fence_after();
+                uint8_t* o_row = generic_base + Smem::kStage + half * kHalfBytes + row * 128;
+#pragma unroll 1
+                for (int c = 0; c < 2; ++c) {
+                    uint32_t acc[32];
+                    tmem_load_32(tmem_o + c * 32, acc);
+                    tmem_load_wait();
+                    if (c == 1) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) arrive_in_cluster(o_empty_first);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        uint32_t w[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)   // (selected, not multiplied: a dead row's accumulator may hold anything)
+                            w[i] = live ? pack_pair<F16>(__uint_as_float(acc[u * 8 + 2 * i]) * inverse, __uint_as_float(acc[u * 8 + 2 * i + 1]) * inverse) : 0u;
+                        *reinterpret_cast<uint4*>(o_row + (((c * 4 + u) ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+                }
+                fence_async_shared();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(staged);
+            }
+            ++n;
+            return true;  // also after a wait gave up: the warps of a row must meet at the same barriers to the end
+        });
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    duo_sync();   // no CTA leaves while the other may still signal its barriers or read its operands
+    if (warp == 17) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    }
+}
+
 // Channel-contiguous [B, H, S, D] whose rows TMA can read: every other stride a positive multiple of 16 bytes.
 bool rows_for_tma(const dfgpu_tensor& t) {
     if (t.rank != 4 || t.stride[3] != 1) return false;
@@ -777,11 +1331,11 @@ bool rows_for_tma(const dfgpu_tensor& t) {
     return t.dim[0] < (1ll << 31) && t.dim[1] < (1ll << 31) && t.dim[2] < (1ll << 30);
 }
 
-int sdpa_map(CUtensorMap* map, const dfgpu_tensor& t, const void* data, const char* what) {
+int sdpa_map(CUtensorMap* map, const dfgpu_tensor& t, const void* data, uint32_t rows, const char* what) {
     uint64_t dims[4] = {static_cast<uint64_t>(t.dim[3]), static_cast<uint64_t>(t.dim[2]), static_cast<uint64_t>(t.dim[1]), static_cast<uint64_t>(t.dim[0])};
     uint64_t strides[3];
     for (int i = 0; i < 3; ++i) strides[i] = static_cast<uint64_t>(t.dim[2 - i] == 1 ? t.dim[3] : t.stride[2 - i]) * 2;   // (an axis of one position has no stride to mind)
-    uint32_t box[4] = {64, kRows, 1, 1};
+    uint32_t box[4] = {64, rows, 1, 1};
     return make_map(map, data, 4, dims, strides, box, what);
 }
 
@@ -792,10 +1346,20 @@ int launch_edges(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUten
     launch_chained(sdpa_umma_pair_kernel<D, F16, EDGES>, dim3(grid), dim3(kPairThreads), PairSmem<D>::kDynamic, stream, map_q, map_k, map_v, map_o, args);
     return check_launch("SDPA (tcgen05, two query tiles per CTA)");
 }
+template <bool F16, bool EDGES>
+int launch_duo(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_o, const SdpaUmmaArgs& args, unsigned clusters, cudaStream_t stream) {
+    cudaError_t error = cudaFuncSetAttribute(sdpa_umma_duo_kernel<F16, EDGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, DuoSmem::kDynamic);
+    if (error != cudaSuccess) return fail(kExecutionFailed, "SDPA: cannot reserve %d bytes of shared memory: %s", DuoSmem::kDynamic, cudaGetErrorString(error));
+    error = launch_chained_cluster(sdpa_umma_duo_kernel<F16, EDGES>, dim3(2 * clusters), dim3(kPairThreads), 2u, static_cast<size_t>(DuoSmem::kDynamic), stream, map_q, map_k, map_v, map_o, args);
+    if (error != cudaSuccess) return fail(kExecutionFailed, "SDPA: launch failed: %s", cudaGetErrorString(error));
+    return check_launch("SDPA (tcgen05, two SMs per pair of query tiles)");
+}
 template <int D, bool F16>
-int launch_pair(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_o, const SdpaUmmaArgs& args, unsigned grid, cudaStream_t stream) {
-    if (args.len_q != nullptr || args.seq_kv % kKeys != 0) return launch_edges<D, F16, true>(map_q, map_k, map_v, map_o, args, grid, stream);
-    return launch_edges<D, F16, false>(map_q, map_k, map_v, map_o, args, grid, stream);
+int launch_shape(bool duo, const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_o, const SdpaUmmaArgs& args, unsigned grid, cudaStream_t stream) {
+    const bool edges = args.len_q != nullptr || args.seq_kv % kKeys != 0;
+    if constexpr (D == 128)
+        if (duo) return edges ? launch_duo<F16, true>(map_q, map_k, map_v, map_o, args, grid, stream) : launch_duo<F16, false>(map_q, map_k, map_v, map_o, args, grid, stream);
+    return edges ? launch_edges<D, F16, true>(map_q, map_k, map_v, map_o, args, grid, stream) : launch_edges<D, F16, false>(map_q, map_k, map_v, map_o, args, grid, stream);
 }
 
 }  // namespace
@@ -820,11 +1384,31 @@ bool sdpa_umma_supported(const dfgpu_sdpa_params& p) {
 int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, cudaStream_t stream) {
     for (int i = 0; i < 4; ++i)
         if ((reinterpret_cast<uintptr_t>(tensors[i]) & 15u) != 0) return fail(kInvalidArgument, "SDPA: the tcgen05 kernel needs 16-byte aligned Q, K, V and O");
+    // One SM or two per pair of query tiles: the longest list of key tiles any of them walks, times what a tile step costs (two
+    // tiles in 3670 clocks on one SM, one in 1620 on each of two; the latter count for 12 % more, since they draw more and a chip that is
+    // full has to lower its clocks), and 4500 clocks a pair. A causal pair's last tile is all masked for the first query tile, which
+    // one SM skips; so it does a second query tile that does not exist.
+    //   64 pairs, 2048 causal: 37 us on one SM each, 22 on two. 96: 38 / 27. 16 x 2171 causal: 39 / 29. 8 x 32 x 2048 causal: 329 / 351.
+    //   192 x 1538 queries on 190 keys: 61 / 73.
+    const int64_t pairs = (p.q.dim[2] + 2 * kRows - 1) / (2 * kRows), heads = p.q.dim[0] * p.q.dim[1], kv_tiles = (p.k.dim[2] + kKeys - 1) / kKeys;
+    int64_t longest = 0, all = 0;
+    for (int64_t i = 0; i < pairs; ++i) {
+        const int64_t tiles = p.has_right_bound ? std::min(kv_tiles, 2 * i + 2) : kv_tiles;
+        longest = std::max(longest, tiles);
+        all += tiles * heads;
+    }
+    auto clocks = [&](int64_t places, double step) {
+        constexpr double kPerPair = 4500.0;
+        if (p.has_right_bound) return std::max(longest * step + kPerPair, (all * step + pairs * heads * kPerPair) / places);
+        return static_cast<double>((pairs * heads + places - 1) / places) * (kv_tiles * step + kPerPair);
+    };
+    const double one = clocks(sm_count(), 3670.0 * (p.has_right_bound ? 0.94 : 1.0) * (p.q.dim[2] <= kRows ? 0.75 : 1.0)), two = clocks(sm_count() / 2, 1620.0 * 1.12);
+    const bool duo = p.q.dim[3] == 128 && two < one;
     CUtensorMap map_q, map_k, map_v, map_o;
-    int status = sdpa_map(&map_q, p.q, tensors[0], "SDPA Q");
-    if (!status) status = sdpa_map(&map_k, p.k, tensors[1], "SDPA K");
-    if (!status) status = sdpa_map(&map_v, p.v, tensors[2], "SDPA V");
-    if (!status) status = sdpa_map(&map_o, p.o, tensors[3], "SDPA O");
+    int status = sdpa_map(&map_q, p.q, tensors[0], kRows, "SDPA Q");
+    if (!status) status = sdpa_map(&map_k, p.k, tensors[1], duo ? kKeys / 2 : kKeys, "SDPA K");
+    if (!status) status = sdpa_map(&map_v, p.v, tensors[2], kRows, "SDPA V");
+    if (!status) status = sdpa_map(&map_o, p.o, tensors[3], kRows, "SDPA O");
     if (status) return status;
     SdpaUmmaArgs args{};
     args.heads_q = static_cast<int>(p.q.dim[1]);
@@ -857,15 +1441,15 @@ int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, cudaStrea
         args.max_stride[i] = p.max.rank ? p.max.stride[i] : 0;
         args.sum_stride[i] = p.sum_exp.rank ? p.sum_exp.stride[i] : 0;
     }
-    // persistent: one CTA per SM over the work list (see PairWalker)
-    const int sms = sm_count();
-    const int64_t single = static_cast<int64_t>(args.pairs) * args.batch_heads;
-    args.paired_units = args.causal && single > sms ? 1 : 0;
-    const int64_t units = args.paired_units ? static_cast<int64_t>((args.pairs + 1) / 2) * args.batch_heads : single;
-    const unsigned grid = static_cast<unsigned>(units < sms ? units : sms);
+    // persistent: one CTA (or cluster of two) per SM (or two) over the work list (see PairWalker)
+    const int places = duo ? sm_count() / 2 : sm_count();
+    const int64_t single = pairs * heads;
+    args.order = !args.causal || single <= places ? kAsStored : (single <= 4 * places ? kHeaviestFirst : kHeavyWithLight);
+    const int64_t units = args.order == kHeavyWithLight ? (pairs + 1) / 2 * heads : single;
+    const unsigned grid = static_cast<unsigned>(std::min<int64_t>(units, places));
     const bool f16 = p.q.dtype == DFGPU_F16;
-    if (p.q.dim[3] == 64) return f16 ? launch_pair<64, true>(map_q, map_k, map_v, map_o, args, grid, stream) : launch_pair<64, false>(map_q, map_k, map_v, map_o, args, grid, stream);
-    return f16 ? launch_pair<128, true>(map_q, map_k, map_v, map_o, args, grid, stream) : launch_pair<128, false>(map_q, map_k, map_v, map_o, args, grid, stream);
+    if (p.q.dim[3] == 64) return f16 ? launch_shape<64, true>(duo, map_q, map_k, map_v, map_o, args, grid, stream) : launch_shape<64, false>(duo, map_q, map_k, map_v, map_o, args, grid, stream);
+    return f16 ? launch_shape<128, true>(duo, map_q, map_k, map_v, map_o, args, grid, stream) : launch_shape<128, false>(duo, map_q, map_k, map_v, map_o, args, grid, stream);
 }
 
 int sdpa_umma_device_status(int* status) { return read_and_clear_device_status(status); }

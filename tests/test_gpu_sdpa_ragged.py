@@ -88,3 +88,18 @@ def test_strides_scale_and_misalignment():
     check(1, 2, 2, 200, 300, 64, "HALF", False, scale=-0.2)
     check(1, 2, 1, 150, 260, 128, "BFLOAT16", False, scale=0.0)
     check(1, 2, 2, 384, 384, 128, "BFLOAT16", True, scale=1.5)   # (the running maximum jumps: O is rescaled)
+
+
+@pytest.mark.parametrize("io", ["BFLOAT16", "HALF"])
+@pytest.mark.parametrize("b,h,hkv,sq,skv,causal,scale", [(1, 37, 37, 1000, 1000, True, None), (1, 40, 8, 700, 700, True, 1.5), (2, 60, 12, 256, 1500, False, 1.5), (1, 148, 4, 200, 129, False, None),
+                                                         (1, 16, 8, 2171, 2171, True, None), (2, 96, 96, 300, 300, True, 1.5)])
+def test_several_items_per_place(io, b, h, hkv, sq, skv, causal, scale):
+    """More work items than SMs or pairs of SMs, which walk them one after another, with maxima that jump."""
+    check(b, h, hkv, sq, skv, 128, io, causal, scale=scale)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("h,sq,skv", [(6, 390, 400), (24, 23, 23), (12, 130, 260)])
+def test_several_padded_items_per_place(causal, h, sq, skv):
+    lengths = [(i * 97) % (skv + 1) for i in range(12)]
+    check(12, h, 2, sq, skv, 128, "BFLOAT16", causal, padding=([min(sq, n + 30) for n in lengths], lengths))
