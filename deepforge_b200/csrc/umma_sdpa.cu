@@ -607,33 +607,37 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         for (int j = 0; j < my_tiles; ++j, ++s_count) {
             if (ok) ok = mbar_wait(s_full(x), s_count & 1, 228 + x);
             tc_fence_after();
-            // One pass over this thread's 64 scores, 16 at a time with the next load in flight: each chunk gives its part
-            // of the half-row maximum and, from the second key tile on, its probabilities against the reference maximum
-            // of the earlier tiles. Only a tile that raises the reference (rare after the first) is read a second time.
+            // This thread's 64 scores are read twice: for the maximum, and against the reference that follows from it. (Formed in one
+            // pass against the last tile's reference, probabilities wait for the exchange in registers: 2650 clocks from scores to
+            // probabilities, 2270 this way.)
             // keys 0..limit of this thread's 64 are visible; only a tile at the diagonal or at the batch's end has others
             const int last_key = !EDGES ? q_index : (args.causal ? min(q_index, item.kv_len - 1) : item.kv_len - 1);
             const int limit = last_key - j * kKeys - half * 64;
             const bool diagonal = (args.causal && j == q_tile) || (EDGES && (j + 1) * kKeys > item.kv_len);
-            const bool speculative = j > 0;
-            const uint64_t scale2 = pack2(scale, scale);
-            uint64_t bias2 = pack2(-m_ref, -m_ref);
-            uint64_t sums[2] = {0, 0};  // two independent chains of packed partial sums
-            uint32_t packed[32];        // this thread's 64 probabilities as bf16 pairs
+            const uint32_t scores_at = tmem_s + half * 64;
+            auto masked = [&](uint32_t (&raw)[16], int c) {
+                if (diagonal) {
+#pragma unroll
+                    for (int e = 0; e < 16; ++e)
+                        if (c * 16 + e > limit) raw[e] = 0xff800000u;  // -inf
+                }
+            };
             float mine = -INFINITY;
             {
                 uint32_t raw[4][16];
-                tmem_load_16(tmem_s + half * 64, raw[0]);
+                tmem_load_16(scores_at, raw[0]);
+                tmem_load_16(scores_at + 16, raw[1]);
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
+                for (int c = 0; c < 4; c += 2) {
                     tmem_load_wait_for(raw[c]);
-                    if (c < 3) tmem_load_16(tmem_s + half * 64 + (c + 1) * 16, raw[c + 1]);
-                    if (diagonal) {
-#pragma unroll
-                        for (int e = 0; e < 16; ++e)
-                            if (c * 16 + e > limit) raw[c][e] = 0xff800000u;  // -inf
+                    tmem_load_wait_for(raw[c + 1]);
+                    if (c < 2) {
+                        tmem_load_16(scores_at + 32, raw[2]);
+                        tmem_load_16(scores_at + 48, raw[3]);
                     }
-                    mine = max_of_16(raw[c], mine);
-                    if (speculative) probabilities_of_16<F16>(raw[c], scale2, bias2, sums, packed + c * 8);
+                    masked(raw[c], c);
+                    masked(raw[c + 1], c + 1);
+                    mine = max_of_16(raw[c + 1], max_of_16(raw[c], mine));
                 }
             }
             raw_max = fmaxf(raw_max, mine);
@@ -650,44 +654,44 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             const float tile_max = fmaxf(__uint_as_float(mine_up), other) * scale;
             // raise the reference only when it would grow by more than the threshold (or on the first tile); the two
             // warps of these rows see the same maxima, so they take the same branches
-            const bool raise = tile_max > m_ref + kRescaleThreshold;
-            bool again = !speculative;
-            if (__any_sync(0xffffffffu, raise)) {
-                again = true;
+            float alpha = 1.0f;
+            const bool raise = __any_sync(0xffffffffu, tile_max > m_ref + kRescaleThreshold) != 0;
+            if (raise) {
                 const float m_new = fmaxf(m_ref, tile_max);
-                const float alpha = m_ref == -INFINITY ? 0.0f : ex2_fast(m_ref - m_new);
+                alpha = m_ref == -INFINITY ? 0.0f : ex2_fast(m_ref - m_new);
                 l_sum *= alpha;
                 m_ref = m_new;
-                if (j > 0) {
-                    // O_x holds P V up to tile j-1; that product was issued ahead of S_x(j), which has completed.
-                    // This thread rescales its columns of the row.
-#pragma unroll 1
-                    for (int c = 0; c < kColumns / 32; ++c) {
-                        uint32_t acc[32];
-                        tmem_load_32(tmem_o + c * 32, acc);
-                        tmem_load_wait();
-#pragma unroll
-                        for (int e = 0; e < 32; ++e) acc[e] = __float_as_uint(__uint_as_float(acc[e]) * alpha);
-                        tmem_store_32(tmem_o + c * 32, acc);
-                    }
-                }
             }
-            if (again) {
-                // the scores are still in place (no probabilities stored yet): form them against the new reference
-                bias2 = pack2(-m_ref, -m_ref);
-#pragma unroll
-                for (int g = 0; g < 2; ++g) sums[g] = 0;
+            {
+                // (probabilities go over columns whose scores have been read: 8 columns for every 16)
+                const uint64_t scale2 = pack2(scale, scale), bias2 = pack2(-m_ref, -m_ref);
+                uint64_t sums[2] = {0, 0};  // two independent chains of packed partial sums
+                uint32_t raw[4][16];
+                tmem_load_16(scores_at, raw[0]);
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    uint32_t raw[16];
-                    tmem_load_16(tmem_s + half * 64 + c * 16, raw);
-                    tmem_load_wait_for(raw);
-                    if (diagonal) {
+                    tmem_load_wait_for(raw[c]);
+                    if (c < 3) tmem_load_16(scores_at + (c + 1) * 16, raw[c + 1]);
+                    masked(raw[c], c);
+                    uint32_t packed[8];
+                    probabilities_of_16<F16>(raw[c], scale2, bias2, sums, packed);
+                    tmem_store_8(scores_at + c * 8, packed);
+                }
+                float lo, hi;
+                unpack2(add2(sums[0], sums[1]), lo, hi);
+                l_sum += lo + hi;
+            }
+            if (raise && j > 0) {
+                // O_x holds P V up to tile j-1; that product was issued ahead of S_x(j), which has completed.
+                // This thread rescales its columns of the row.
+#pragma unroll 1
+                for (int c = 0; c < kColumns / 16; ++c) {
+                    uint32_t acc[16];
+                    tmem_load_16(tmem_o + c * 16, acc);
+                    tmem_load_wait_for(acc);
 #pragma unroll
-                        for (int e = 0; e < 16; ++e)
-                            if (c * 16 + e > limit) raw[e] = 0xff800000u;
-                    }
-                    probabilities_of_16<F16>(raw, scale2, bias2, sums, packed + c * 8);
+                    for (int e = 0; e < 16; ++e) acc[e] = __float_as_uint(__uint_as_float(acc[e]) * alpha);
+                    tmem_store_16(tmem_o + c * 16, acc);
                 }
             }
             if (EDGES && args.len_q != nullptr && (j + 1) * kKeys > item.kv_len && (D == 128 || half == 0)) {
@@ -701,12 +705,6 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     for (int u = 0; u < 8; ++u) *reinterpret_cast<uint4*>(v_row + u * 16) = make_uint4(0, 0, 0, 0);
                 }
                 fence_async_shared();
-            }
-            tmem_store_32(tmem_s + half * 64, packed);
-            {
-                float lo, hi;
-                unpack2(add2(sums[0], sums[1]), lo, hi);
-                l_sum += lo + hi;
             }
             tmem_store_wait();
             tc_fence_before();
