@@ -147,14 +147,18 @@ __device__ __forceinline__ void product(uint32_t d, uint64_t a, uint64_t b, uint
 #define DFGPU_MMA(FORM)                                                                                                   \
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma." FORM ".kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}" \
                  ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb) : "memory")
-    if constexpr (KIND == kScaled) DFGPU_MMA("cta_group::1");
+    if constexpr (KIND == kScaled && CG == 1) DFGPU_MMA("cta_group::1");
+    if constexpr (KIND == kScaled && CG == 2) DFGPU_MMA("cta_group::2");
 #undef DFGPU_MMA
 }
 // 32 rows x 16 bytes of shared memory -> 4 columns of tensor memory, replicated to the four lane quarters.
+// (CG = 2: each CTA's from its own shared memory.)
+template <int CG>
 __device__ __forceinline__ void copy_scales(uint32_t tmem_dst, uint32_t address) {
     // an unswizzled K-major block: 8-row groups 128 bytes apart
     const uint64_t desc = static_cast<uint64_t>((address & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(128u >> 4) << 32) | (1ull << 46);
-    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem_dst), "l"(desc) : "memory");
+    if constexpr (CG == 2) asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem_dst), "l"(desc) : "memory");
+    else asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem_dst), "l"(desc) : "memory");
 }
 
 // ---- the fused steps on values of one row of C ---------------------------------------------------------------
@@ -420,7 +424,6 @@ template <int KIND, int CG>
 __global__ void __launch_bounds__(thread_count<KIND>(), 1)
 umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c,
                    const __grid_constant__ TileArgs args) {
-    static_assert(KIND != kScaled || CG == 1, "block scales: one SM per tile (see choose_shape())");
     constexpr int kCode = KIND == kSixteen ? 0 : (KIND == kCodes ? 20 : (KIND == kScaled ? 40 : 60));
     constexpr bool kSixteenBits = KIND == kSixteen || KIND == kPieces;
     constexpr int kPieceCount = KIND == kPieces ? 3 : 1;
@@ -454,14 +457,14 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     }
     if (warp == 0 && leader) {
         for (int s = 0; s < args.stages; ++s) {
-            mbar_init(full_bar(s), KIND == kScaled ? 2 : 1);   // the byte count, and the slot's scale warp
+            mbar_init(full_bar(s), KIND == kScaled ? 1 + CG : 1);   // the byte count, and the slot's scale warp of each CTA
             mbar_init(empty_bar(s), 1);
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(acc_full(a), 1);
             mbar_init(acc_empty(a), 8 * CG);
         }
-        mbar_init(overlap_free, 4);
+        mbar_init(overlap_free, 4 * CG);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -534,11 +537,11 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         const uint32_t a_lo = smem_desc_lo(a_src, 16), b_lo = smem_desc_lo(b_src, b_lbo);
                         uint32_t sf = 0;
                         if constexpr (KIND == kScaled) {
-                            const uint32_t scales = b_src + bn * kRowBytes;
+                            const uint32_t scales = b_src + bn / CG * kRowBytes;
                             sf = tmem_u + args.scale_columns + (stage & 1) * 16;   // A's at +0..3, B's at +4..11
-                            copy_scales(sf, scales);
-                            copy_scales(sf + 4, scales + 512);
-                            if (width > 128) copy_scales(sf + 8, scales + 1024);
+                            copy_scales<CG>(sf, scales);
+                            copy_scales<CG>(sf + 4, scales + 512);
+                            if (width > 128) copy_scales<CG>(sf + 8, scales + 1024);
                         }
                         if constexpr (KIND == kPieces) {
                             // middle*middle, low*high, high*low, middle*high, high*middle meet in an accumulator of their own: the tensor
@@ -622,7 +625,10 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         if (overlapped && b == g && g != acc && part == box_columns / 32 - 1) {   // the shared columns are in registers
                             tc_fence_before();
                             __syncwarp();
-                            if (lane == 0) mbar_arrive(overlap_free);
+                            if (lane == 0) {
+                                if (CG == 2) mbar_arrive_cluster(leader_bars + (overlap_free - bar_base));
+                                else mbar_arrive(overlap_free);
+                            }
                         }
                         float v[32];
 #pragma unroll
@@ -696,7 +702,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         Item item = item_at(args, at);
         auto load = [&] {
             item = item_at(args, at);
-            load_scales(args, item.m_tile * kRows, item.col0, kb, lane, raw);
+            load_scales(args, (item.m_tile * CG + (CG == 2 ? rank : 0)) * kRows, item.col0, kb, lane, raw);
         };
         bool more = kb_begin < kb_end && seek();
         if (more) load();
@@ -704,18 +710,21 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             const int slot = stage;
             const uint32_t slot_phase = phase;
             uint32_t a_words[4], b_words[2][4];
-            pack_scales(args, item.m_tile * kRows, item.col0, kb, lane, raw, a_words, b_words);
+            pack_scales(args, (item.m_tile * CG + (CG == 2 ? rank : 0)) * kRows, item.col0, kb, lane, raw, a_words, b_words);
             advance();
             more = seek();
             if (more) load();
             if (!mbar_wait_warp(empty_bar(slot), slot_phase, 506 + kCode)) break;
-            uint8_t* scales = generic_base + slot * args.stage_bytes + args.a_bytes + bn * kRowBytes + lane * 16;
+            uint8_t* scales = generic_base + slot * args.stage_bytes + args.a_bytes + bn / CG * kRowBytes + lane * 16;
             *reinterpret_cast<uint4*>(scales) = make_uint4(a_words[0], a_words[1], a_words[2], a_words[3]);
             *reinterpret_cast<uint4*>(scales + 512) = make_uint4(b_words[0][0], b_words[0][1], b_words[0][2], b_words[0][3]);
             if (bn > 128) *reinterpret_cast<uint4*>(scales + 1024) = make_uint4(b_words[1][0], b_words[1][1], b_words[1][2], b_words[1][3]);
             fence_async_shared();
             __syncwarp();
-            if (leader) mbar_arrive(full_bar(slot));
+            if (leader) {
+                if (CG == 2) mbar_arrive_cluster(address_in(full_bar(slot), 0));   // (CTA 0's product reads both CTAs' scales)
+                else mbar_arrive(full_bar(slot));
+            }
         }
     }
 
@@ -851,7 +860,7 @@ Shape choose_shape(const Problem& p) {
     constexpr int clusters_at_once[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};   // (cudaOccupancyMaxActiveClusters, by CTAs per cluster)
     const int sms = 148;   // (a function of the shape alone: the count this library is built for)
     Shape best{0, 0, 0, 0, 0, 0, 0.0};
-    for (int cg = 1; cg <= (p.kind == kScaled ? 1 : 2); ++cg)
+    for (int cg = 1; cg <= 2; ++cg)
         for (int bn = 64; bn <= 256; bn += 64) {
             const int chunk = sixteen_bits(p) ? 64 : 128;   // columns of one N-major copy
             if (p.b_mn_major && (bn / cg) % chunk != 0) continue;
@@ -953,7 +962,7 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     if (p.kind == kSixteen) return shape.cg == 2 ? launch_kernel<kSixteen, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kSixteen, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     if (p.kind == kCodes) return shape.cg == 2 ? launch_kernel<kCodes, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kCodes, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     if (p.kind == kPieces) return shape.cg == 2 ? launch_kernel<kPieces, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kPieces, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
-    return launch_kernel<kScaled, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
+    return shape.cg == 2 ? launch_kernel<kScaled, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kScaled, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
 }
 
 // The fused steps the kernel applies: ReLU, a per-column ADD operand, a full [M, N] ADD operand with contiguous columns.
