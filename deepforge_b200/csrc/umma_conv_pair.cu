@@ -111,6 +111,8 @@ __device__ __forceinline__ float relu_step(float x, float lower, float upper, fl
     return x < lower ? fmaf(slope, x - lower, lower) : clipped;
 }
 
+// CLIPPED: the last tile of an image hangs over its end (map_out and map_res have rank 4).
+template <bool CLIPPED>
 __global__ void __launch_bounds__(kPairThreads, 1)
 umma_conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_wa, const __grid_constant__ CUtensorMap map_wb,
                       const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_res, PairArgs args) {
@@ -419,13 +421,13 @@ umma_conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         const float* bias_smem = reinterpret_cast<const float*>(generic_base + args.bias_offset);
         int bias_a_floats = 0;
         for (int e = 0; e < args.steps_a.count; ++e) bias_a_floats += args.steps_a.kind[e] == kStepBias ? kK1 : 0;
-        int image, h0, out_row0, next_row0 = 0;
-        if (my_tiles > 0) tile_origin(blockIdx.x, image, h0, next_row0);
+        int image, h0, out_row0, next_image = 0, next_h0 = 0, next_row0 = 0;
+        if (my_tiles > 0) tile_origin(blockIdx.x, next_image, next_h0, next_row0);
         bool ok = true;
         int n = 0;  // chunks handled: chunk n uses box n & 1 of the group
         for (int j = 0, tile = blockIdx.x; j < my_tiles; ++j, tile += gridDim.x) {
-            out_row0 = next_row0;
-            if (j + 1 < my_tiles) tile_origin(tile + gridDim.x, image, h0, next_row0);
+            out_row0 = next_row0, image = next_image, h0 = next_h0;
+            if (j + 1 < my_tiles) tile_origin(tile + gridDim.x, next_image, next_h0, next_row0);
             for (int c = 0; c < chunks; ++c, ++n) {
                 const int col0 = group * (args.k2 / 2) + c * 64;
                 const int box_index = 2 * group + (n & 1);
@@ -500,7 +502,10 @@ umma_conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 }
                 group_barrier();
                 if (store_thread) {
-                    if (healthy) tma_store_2d(&map_out, stage_base + box_index * args.box_bytes, col0, out_row0);
+                    if (healthy) {
+                        if constexpr (CLIPPED) tma_store_4d(&map_out, stage_base + box_index * args.box_bytes, col0, 0, h0, image);
+                        else tma_store_2d(&map_out, stage_base + box_index * args.box_bytes, col0, out_row0);
+                    }
                     tma_store_commit();
                 }
             }
@@ -523,7 +528,8 @@ umma_conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                     if (!ok) break;
                     if (leader) {
                         mbar_expect_tx(res_full(box), static_cast<uint32_t>(args.box_rows) * 128u);
-                        tma_load_2d(stage_base + box * args.box_bytes, &map_res, g * (args.k2 / 2) + c * 64, out_row0, res_full(box));
+                        if constexpr (CLIPPED) tma_load_4d(stage_base + box * args.box_bytes, &map_res, g * (args.k2 / 2) + c * 64, 0, h0, image, res_full(box));
+                        else tma_load_2d(stage_base + box * args.box_bytes, &map_res, g * (args.k2 / 2) + c * 64, out_row0, res_full(box));
                     }
                 }
         }
@@ -669,7 +675,7 @@ int launch_conv_pair_umma(const dfgpu_conv_params& first, const dfgpu_conv_param
     args.pad_w = static_cast<int>(first.pre_pad[1]);
     args.rows_per_tile = a.halo_rows;
     args.window_rows = f.window_rows;
-    args.tiles_per_image = static_cast<int>(a.P / a.halo_rows);
+    args.tiles_per_image = static_cast<int>((a.P + a.halo_rows - 1) / a.halo_rows);
     args.out_p = static_cast<int>(a.P);
     args.out_q = static_cast<int>(a.Q);
     args.pitch = static_cast<int>(a.Q + a.S - 1);
@@ -700,6 +706,7 @@ int launch_conv_pair_umma(const dfgpu_conv_params& first, const dfgpu_conv_param
     const int dynamic = args.bias_offset + f.bias_bytes + 1024;
     if (dynamic > kPairSmemBudget) return fail(kUnsupported, "CONV_FPROP pair: shared-memory layout does not fit");
 
+    const bool clipped = a.P % a.halo_rows != 0;
     CUtensorMap map_x, map_wa, map_wb, map_out, map_res;
     int status;
     {
@@ -721,20 +728,23 @@ int launch_conv_pair_umma(const dfgpu_conv_params& first, const dfgpu_conv_param
         if ((status = make_map(&map_wb, tensors[2], 2, dims, strides, box, "CONV_FPROP pair W (second)"))) return status;
     }
     {
-        uint64_t dims[2] = {static_cast<uint64_t>(f.k2), static_cast<uint64_t>(a.N * a.P * a.Q)};
-        uint64_t strides[1] = {static_cast<uint64_t>(f.k2) * 2};
-        uint32_t box[2] = {64, static_cast<uint32_t>(f.box_rows)};
-        if ((status = make_map(&map_out, tensors[3], 2, dims, strides, box, "CONV_FPROP pair Y"))) return status;
+        // rows of one image where the last tile hangs over its end (loads read zeros there and stores are clipped), else pixels of all images
+        const int rank = clipped ? 4 : 2;
+        uint64_t dims[4] = {static_cast<uint64_t>(f.k2), static_cast<uint64_t>(clipped ? a.Q : a.N * a.P * a.Q), static_cast<uint64_t>(a.P), static_cast<uint64_t>(a.N)};
+        uint64_t strides[3] = {static_cast<uint64_t>(f.k2) * 2, static_cast<uint64_t>(a.Q * f.k2) * 2, static_cast<uint64_t>(a.P * a.Q * f.k2) * 2};
+        uint32_t box[4] = {64, static_cast<uint32_t>(clipped ? a.Q : f.box_rows), static_cast<uint32_t>(a.halo_rows), 1};
+        if ((status = make_map(&map_out, tensors[3], rank, dims, strides, box, "CONV_FPROP pair Y"))) return status;
         const void* residual = tensors[3];
         for (int e = 0; e < args.steps_b.count; ++e)
             if (args.steps_b.kind[e] == kStepFull) residual = args.steps_b.data[e];
-        if ((status = make_map(&map_res, residual, 2, dims, strides, box, "CONV_FPROP pair residual"))) return status;
+        if ((status = make_map(&map_res, residual, rank, dims, strides, box, "CONV_FPROP pair residual"))) return status;
     }
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t error = cudaFuncSetAttribute(umma_conv_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBudget);
+    auto kernel = clipped ? umma_conv_pair_kernel<true> : umma_conv_pair_kernel<false>;
+    static bool configured[2] = {false, false};
+    if (!configured[clipped]) {
+        cudaError_t error = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBudget);
         if (error != cudaSuccess) return fail(kExecutionFailed, "CONV_FPROP pair: cannot reserve %d bytes of shared memory: %s", kPairSmemBudget, cudaGetErrorString(error));
-        configured = true;
+        configured[clipped] = true;
     }
     // even shares of the tile list (see launch_persistent in umma_gemm.cu)
     const int sms = sm_count();
@@ -743,7 +753,7 @@ int launch_conv_pair_umma(const dfgpu_conv_params& first, const dfgpu_conv_param
         const int rounds = (args.total_tiles + sms - 1) / sms;
         grid = (args.total_tiles + rounds - 1) / rounds;
     }
-    cudaError_t launched = launch_chained(umma_conv_pair_kernel, dim3(grid), dim3(kPairThreads), dynamic, stream, map_x, map_wa, map_wb, map_out, map_res, args);
+    cudaError_t launched = launch_chained(kernel, dim3(grid), dim3(kPairThreads), dynamic, stream, map_x, map_wa, map_wb, map_out, map_res, args);
     if (launched != cudaSuccess) return fail(kExecutionFailed, "CONV_FPROP pair: launch failed: %s", cudaGetErrorString(launched));
     return check_launch("CONV_FPROP pair");
 }

@@ -325,7 +325,9 @@ __device__ __forceinline__ float split_remainder(float x, uint32_t hi_bits) {
     return (hi_bits & 0x7f800000u) == 0x7f800000u ? 0.0f : x - __uint_as_float(hi_bits);
 }
 
-template <int BN, bool HAS_RES>
+// CLIPPED: the last tile of an image hangs over its end (map_out and map_res have rank 4). Compiled in: a branch around the stores cost
+// the bottleneck 5 %.
+template <int BN, bool HAS_RES, bool CLIPPED>
 __global__ void __launch_bounds__(kPersistentThreads, 1)
 umma_conv_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                             const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_res,
@@ -410,7 +412,8 @@ umma_conv_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __g
                         mbar_expect_tx(res_full_bar(b), res_bytes);
 #pragma unroll
                         for (int j = 0; j < BN / 64; ++j)
-                            tma_load_2d(epi_base + b * pargs.epi_bytes + j * (kTileM * 128), &map_res, ld.n_tile * BN + 64 * j, static_cast<int>(ld.out_row0), res_full_bar(b));
+                            if constexpr (CLIPPED) tma_load_4d(epi_base + b * pargs.epi_bytes + j * (kTileM * 128), &map_res, ld.n_tile * BN + 64 * j, 0, ld.h0, ld.image, res_full_bar(b));
+                            else tma_load_2d(epi_base + b * pargs.epi_bytes + j * (kTileM * 128), &map_res, ld.n_tile * BN + 64 * j, static_cast<int>(ld.out_row0), res_full_bar(b));
                     }
                 }
                 ld.open = true;
@@ -705,13 +708,16 @@ umma_conv_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __g
             epilogue_barrier(1 + group);
             if (store_thread) {
                 if (healthy) {
+                    auto store = [&](int box, int col0) {
+                        const uint32_t source = epi_base + buf * pargs.epi_bytes + box * (kTileM * 128);
+                        if constexpr (CLIPPED) tma_store_4d(&map_out, source, col0, 0, h0, image);
+                        else tma_store_2d(&map_out, source, col0, static_cast<int>(out_row0));
+                    };
 #pragma unroll
-                    for (int q = 0; q < BN / 64; ++q)
-                        tma_store_2d(&map_out, epi_base + buf * pargs.epi_bytes + q * (kTileM * 128), n0 + 64 * q, static_cast<int>(out_row0));
+                    for (int q = 0; q < BN / 64; ++q) store(q, n0 + 64 * q);
                     if (!HAS_RES && pargs.split_out) {
 #pragma unroll
-                        for (int q = 0; q < BN / 64; ++q)
-                            tma_store_2d(&map_out, epi_base + buf * pargs.epi_bytes + (BN / 64 + q) * (kTileM * 128), static_cast<int>(args.n_total) + n0 + 64 * q, static_cast<int>(out_row0));
+                        for (int q = 0; q < BN / 64; ++q) store(BN / 64 + q, static_cast<int>(args.n_total) + n0 + 64 * q);
                     }
                 }
                 tma_store_commit();
@@ -764,7 +770,7 @@ int dispatch(int bn, int k_blocks, const CUtensorMap& map_a, const CUtensorMap& 
 
 constexpr int kSmemBudget = 227 * 1024;
 
-template <int BN, bool HAS_RES>
+template <int BN, bool HAS_RES, bool CLIPPED>
 int launch_persistent(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_out, const CUtensorMap& map_res,
                       PersistentArgs args, cudaStream_t stream) {
     constexpr int kBarrierBytes = (2 * kMaxRingStages + 18) * 8;
@@ -804,7 +810,7 @@ int launch_persistent(const CUtensorMap& map_a, const CUtensorMap& map_b, const 
     args.issuers = (args.halo && args.gemm.k_blocks / args.gemm.filter_s + 2 <= stages) ? 2 : 1;
     static int configured = 0;
     if (configured < dynamic) {
-        cudaError_t error = cudaFuncSetAttribute(umma_conv_persistent_kernel<BN, HAS_RES>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget);
+        cudaError_t error = cudaFuncSetAttribute(umma_conv_persistent_kernel<BN, HAS_RES, CLIPPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget);
         if (error != cudaSuccess) return fail(kExecutionFailed, "tcgen05 conv: cannot reserve %d bytes of shared memory: %s", kSmemBudget, cudaGetErrorString(error));
         configured = kSmemBudget;
     }
@@ -816,7 +822,7 @@ int launch_persistent(const CUtensorMap& map_a, const CUtensorMap& map_b, const 
         const int rounds = (args.total_tiles + sms - 1) / sms;
         grid = (args.total_tiles + rounds - 1) / rounds;
     }
-    cudaError_t launched = launch_chained(umma_conv_persistent_kernel<BN, HAS_RES>, dim3(grid), dim3(kPersistentThreads), dynamic, stream, map_a, map_b, map_out, map_res, args);
+    cudaError_t launched = launch_chained(umma_conv_persistent_kernel<BN, HAS_RES, CLIPPED>, dim3(grid), dim3(kPersistentThreads), dynamic, stream, map_a, map_b, map_out, map_res, args);
     if (launched != cudaSuccess) return fail(kExecutionFailed, "tcgen05 conv (persistent): launch failed: %s", cudaGetErrorString(launched));
     return check_launch("tcgen05 conv (persistent)");
 }
@@ -919,15 +925,21 @@ bool conv_umma_form(const dfgpu_conv_params& p, ConvForm& f) {
             residual_bf16 = residual_bf16 && t.dtype == DFGPU_BF16;
         }
     }
-    // halo form: a tile is `halo_rows` output rows with their padded columns, halo_rows the largest divisor of P that fits
+    // halo form: a tile is `halo_rows` output rows with their padded columns, as many as fit 128 GEMM rows, evened out over the
+    // image's tiles. The last tile may hang over the image: its loads read zeros there and its stores are clipped (rows that had to
+    // divide P left 13 of 128 GEMM rows in use for 11 or 13 output rows).
     f.halo = false;
     f.halo_rows = 0;
     const int64_t pitch = f.Q + f.S - 1;
     if (!f.pointwise && f.S > 1 && f.S <= 8 && pitch <= kTileM) {
-        int halo_rows = static_cast<int>(kTileM / pitch);
-        while (halo_rows > 1 && f.P % halo_rows != 0) --halo_rows;
+        const int64_t most = kTileM / pitch, tiles = (f.P + most - 1) / most;
         f.halo = true;
-        f.halo_rows = halo_rows;
+        f.halo_rows = static_cast<int>((f.P + tiles - 1) / tiles);
+        // Rows that divide P evenly where they are nearly as many (no clipping), or where one row a tile already leaves SMs idle and is
+        // wide enough for the two-convolution kernel (130 + 2 pitch rows read, window and staging behind it rows (pitch + 4 Q)): 1 x 23 x 23 15.9 us, 16.6 with 5 rows.
+        int even = static_cast<int>(most);
+        while (even > 1 && f.P % even != 0) --even;
+        if (3 * even >= 2 * f.halo_rows || (f.N * f.P <= 148 && (5 * f.Q + 2) * even >= 114)) f.halo_rows = even;
     }
     const bool whole_tiles = f.pointwise || f.halo || f.P % f.rows_per_tile == 0;
     const bool residual_ok = full_steps == 0 || (full_steps == 1 && residual_bf16 && !f.split_out);
@@ -1026,7 +1038,7 @@ int launch_conv_umma(const dfgpu_conv_params& p, void* const* tensors, cudaStrea
             pargs.halo = 1;
             pargs.pitch = static_cast<int>(pitch);
             pargs.gemm.rows_per_tile = f.halo_rows;
-            pargs.gemm.tiles_per_image = static_cast<int>(P / f.halo_rows);
+            pargs.gemm.tiles_per_image = static_cast<int>((P + f.halo_rows - 1) / f.halo_rows);
             m_tiles = N * pargs.gemm.tiles_per_image;
             uint64_t dims4[4] = {static_cast<uint64_t>(Ca), static_cast<uint64_t>(W), static_cast<uint64_t>(H), static_cast<uint64_t>(N)};
             uint64_t strides3[3] = {static_cast<uint64_t>(Ca) * 2, static_cast<uint64_t>(W * Ca) * 2, static_cast<uint64_t>(H * W * Ca) * 2};
@@ -1041,20 +1053,25 @@ int launch_conv_umma(const dfgpu_conv_params& p, void* const* tensors, cudaStrea
         pargs.filter_bytes = static_cast<int>(K * R * S * C * 2);
         pargs.bias_stride = static_cast<int>(K);
         CUtensorMap map_out, map_res;
-        uint64_t dims[2] = {static_cast<uint64_t>(Kout), static_cast<uint64_t>(N * P * Q)};
-        uint64_t strides[1] = {static_cast<uint64_t>(Kout) * 2};
-        uint32_t box[2] = {64, static_cast<uint32_t>(out_box_rows)};
-        status = make_map(&map_out, tensors[2], 2, dims, strides, box, "CONV_FPROP Y");
+        // rows of one image where a tile hangs over its end, so that it is clipped; else pixels of all images (2 % faster)
+        const bool clipped = f.halo && P % f.halo_rows != 0;
+        const int rank = clipped ? 4 : 2;
+        uint64_t dims[4] = {static_cast<uint64_t>(Kout), static_cast<uint64_t>(clipped ? Q : N * P * Q), static_cast<uint64_t>(P), static_cast<uint64_t>(N)};
+        uint64_t strides[3] = {static_cast<uint64_t>(Kout) * 2, static_cast<uint64_t>(Q * Kout) * 2, static_cast<uint64_t>(P * Q * Kout) * 2};
+        uint32_t box[4] = {64, static_cast<uint32_t>(clipped ? Q : out_box_rows), static_cast<uint32_t>(f.halo_rows), 1};
+        status = make_map(&map_out, tensors[2], rank, dims, strides, box, "CONV_FPROP Y");
         if (status) return status;
         const void* residual = full_steps ? args.epi_data[residual_step] : tensors[2];
-        status = make_map(&map_res, residual, 2, dims, strides, box, "CONV_FPROP residual");
+        status = make_map(&map_res, residual, rank, dims, strides, box, "CONV_FPROP residual");
         if (status) return status;
-        if (bn == 64) {
-            if (full_steps) return launch_persistent<64, true>(map_a, map_b, map_out, map_res, pargs, stream);
-            return launch_persistent<64, false>(map_a, map_b, map_out, map_res, pargs, stream);
-        }
-        if (full_steps) return launch_persistent<128, true>(map_a, map_b, map_out, map_res, pargs, stream);
-        return launch_persistent<128, false>(map_a, map_b, map_out, map_res, pargs, stream);
+        auto launch = [&](auto width, auto clip) {
+            constexpr int BN = decltype(width)::value;
+            constexpr bool CLIPPED = decltype(clip)::value;
+            if (full_steps) return launch_persistent<BN, true, CLIPPED>(map_a, map_b, map_out, map_res, pargs, stream);
+            return launch_persistent<BN, false, CLIPPED>(map_a, map_b, map_out, map_res, pargs, stream);
+        };
+        auto by_width = [&](auto clip) { return bn == 64 ? launch(std::integral_constant<int, 64>{}, clip) : launch(std::integral_constant<int, 128>{}, clip); };
+        return clipped ? by_width(std::true_type{}) : by_width(std::false_type{});
     }
     dim3 grid(static_cast<unsigned>(m_tiles), static_cast<unsigned>(K / bn));
     if (k_split && k_split->splits > 1) {

@@ -105,10 +105,6 @@ struct PairSmem {
 };
 constexpr int kHalfBytes = kRows * 128;   // one box
 
-__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {
-    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
-                 ::"l"(map), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
-}
 
 // D[tmem] (+)= A[tmem] * B[smem]: the A operand (bf16 pairs, one row per lane) is read from tensor memory.
 __device__ __forceinline__ void umma_bf16_a_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
