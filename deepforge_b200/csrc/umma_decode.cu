@@ -217,34 +217,37 @@ sdpa_decode_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     const uint32_t tmem_o = tmem_base + 32;  // S^T buffers at +0 and +16, O^T at +32
 
     if (warp == 0) {
-        if (lane == 0) {
+        // The whole warp walks the tiles, lane l with the id of a tile's page l: with one lane reading ids and issuing, a tile of eight
+        // 16-token pages took it 16 dependent shared-memory loads.
+        const bool leader = elect_one();
+        if (leader) {
             // Q rows of this GQA group (the box holds 16 rows; rows past the group are other heads or zero fill and are ignored)
             mbar_expect_tx(q_full, 2 * kHeadsPadded * 128);
             const int q_row = static_cast<int>(batch * args.heads_q + kv_head * G);
             tma_load_2d(smem_base + DecodeSmem::kQ, &map_q, 0, q_row, q_full);
             tma_load_2d(smem_base + DecodeSmem::kQ + kHeadsPadded * 128, &map_q, 64, q_row, q_full);
-            const uint32_t page_bytes = static_cast<uint32_t>(args.block) * 128u;  // one page, one 64-column half
-            for (int t = 0; t < 2 * tiles; ++t) {
-                const int slot = t % kRingSlots;
-                if (!mbar_wait(kv_empty(slot), ((t / kRingSlots) & 1) ^ 1, 301)) break;
-                const bool is_v = (t & 1) != 0;
-                const CUtensorMap* map = is_v ? &map_v : &map_k;
-                const int32_t* ids = page_ids + (is_v ? 64 : 0) + (first_tile + (t >> 1)) * args.pages_per_tile;
-                const uint32_t dst = smem_base + DecodeSmem::kRing + slot * kKvTileBytes;
-                uint32_t expected = 0;
-                for (int pg = 0; pg < args.pages_per_tile; ++pg)
-                    if (ids[pg] >= 0) expected += 2 * page_bytes;
-                mbar_expect_tx(kv_full(slot), expected);  // also the arrival; 0 bytes when every page is invalid
-                for (int pg = 0; pg < args.pages_per_tile; ++pg) {
-                    const int64_t page = ids[pg];
-                    const uint32_t page_dst = dst + pg * page_bytes;
-                    if (page >= 0) {
-                        const int row = static_cast<int>((page * args.heads_kv + kv_head) * args.block);
-                        tma_load_2d(page_dst, map, 0, row, kv_full(slot));
-                        tma_load_2d(page_dst + kKvHalfBytes, map, 64, row, kv_full(slot));
-                    }
+        }
+        __syncwarp();
+        const uint32_t page_bytes = static_cast<uint32_t>(args.block) * 128u;  // one page, one 64-column half
+        for (int t = 0; t < 2 * tiles; ++t) {
+            const int slot = t % kRingSlots;
+            const bool is_v = (t & 1) != 0;
+            const int id = lane < args.pages_per_tile ? page_ids[(is_v ? 64 : 0) + (first_tile + (t >> 1)) * args.pages_per_tile + lane] : -1;
+            const uint32_t valid = __ballot_sync(0xffffffffu, id >= 0);
+            const int row = static_cast<int>((static_cast<int64_t>(id) * args.heads_kv + kv_head) * args.block);
+            if (!mbar_wait_warp(kv_empty(slot), ((t / kRingSlots) & 1) ^ 1, 301)) break;
+            const CUtensorMap* map = is_v ? &map_v : &map_k;
+            const uint32_t dst = smem_base + DecodeSmem::kRing + slot * kKvTileBytes;
+            if (leader) mbar_expect_tx(kv_full(slot), 2 * page_bytes * static_cast<uint32_t>(__popc(valid)));  // also the arrival; 0 bytes when every page is invalid
+            for (int pg = 0; pg < args.pages_per_tile; ++pg) {
+                const int page_row = __shfl_sync(0xffffffffu, row, pg);
+                const uint32_t page_dst = dst + pg * page_bytes;
+                if (leader && (valid >> pg & 1u) != 0) {
+                    tma_load_2d(page_dst, map, 0, page_row, kv_full(slot));
+                    tma_load_2d(page_dst + kKvHalfBytes, map, 64, page_row, kv_full(slot));
                 }
             }
+            __syncwarp();
         }
     } else if (warp == 1) {
         if (lane == 0) {
