@@ -250,47 +250,53 @@ sdpa_decode_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             __syncwarp();
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // S^T: A = K tile (K-major), B = Q (K-major). O^T: A = V tile read MN-major (M = d), B = P (K-major).
-            const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kHeadsPadded >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
-            const uint32_t idesc_o = idesc_s | (1u << 15);
-            const uint32_t q_smem = smem_base + DecodeSmem::kQ;
-            bool ok = mbar_wait(q_full, 0, 302);
-            auto issue_scores = [&](int j) {
-                const int t = 2 * j, slot = t % kRingSlots, b = j & 1;
-                if (ok) ok = mbar_wait(kv_full(slot), (t / kRingSlots) & 1, 303);
-                if (ok) ok = mbar_wait(s_empty(b), ((j >> 1) & 1) ^ 1, 304);
-                tc_fence_after();
-                if (ok) {
-                    const uint32_t k_smem = smem_base + DecodeSmem::kRing + slot * kKvTileBytes;
-                    const uint32_t k_lo = smem_desc_lo(k_smem, 16), q_lo = smem_desc_lo(q_smem, 16);
+        const bool leader = elect_one();   // all lanes walk the schedule, so that descriptors and addresses are uniform values, and one issues (196 us -> 192 with 64 sequences)
+        // S^T: A = K tile (K-major), B = Q (K-major). O^T: A = V tile read MN-major (M = d), B = P (K-major).
+        const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kHeadsPadded >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
+        const uint32_t idesc_o = idesc_s | (1u << 15);
+        const uint32_t q_smem = smem_base + DecodeSmem::kQ;
+        const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+        bool ok = mbar_wait_warp(q_full, 0, 302);
+        auto issue_scores = [&](int j) {
+            const int t = 2 * j, slot = t % kRingSlots, b = j & 1;
+            if (ok) ok = mbar_wait_warp(kv_full(slot), (t / kRingSlots) & 1, 303);
+            if (ok) ok = mbar_wait_warp(s_empty(b), ((j >> 1) & 1) ^ 1, 304);
+            tc_fence_after();
+            if (leader && ok) {
+                const uint32_t k_smem = smem_base + DecodeSmem::kRing + slot * kKvTileBytes;
+                const uint32_t k_lo = smem_desc_lo(k_smem, 16), q_lo = smem_desc_lo(q_smem, 16);
 #pragma unroll
-                    for (int k = 0; k < kDim / 16; ++k)
-                        umma_bf16(tmem_base + b * 16, desc_words(k_lo + (((k >> 2) * kKvHalfBytes + (k & 3) * 32) >> 4), smem_desc_hi(1024)),
-                                  desc_words(q_lo + (((k >> 2) * (kHeadsPadded * 128) + (k & 3) * 32) >> 4), smem_desc_hi(1024)), idesc_s, k != 0 ? 1u : 0u);
-                }
+                for (int k = 0; k < kDim / 16; ++k)
+                    umma_bf16(tmem_u + b * 16, desc_words(k_lo + (((k >> 2) * kKvHalfBytes + (k & 3) * 32) >> 4), smem_desc_hi(1024)),
+                              desc_words(q_lo + (((k >> 2) * (kHeadsPadded * 128) + (k & 3) * 32) >> 4), smem_desc_hi(1024)), idesc_s, k != 0 ? 1u : 0u);
+            }
+            if (leader) {
                 umma_commit(kv_empty(slot));
                 umma_commit(s_full(b));
-            };
-            issue_scores(0);
-            for (int j = 0; j < tiles; ++j) {
-                if (j + 1 < tiles) issue_scores(j + 1);
-                const int t = 2 * j + 1, slot = t % kRingSlots, b = j & 1;
-                if (ok) ok = mbar_wait(p_full(b), (j >> 1) & 1, 305);
-                if (ok) ok = mbar_wait(kv_full(slot), (t / kRingSlots) & 1, 306);
-                tc_fence_after();
-                if (ok) {
-                    const uint32_t v_smem = smem_base + DecodeSmem::kRing + slot * kKvTileBytes;
-                    const uint32_t p_smem = smem_base + DecodeSmem::kP + b * 4096;
-                    const uint32_t v_lo = smem_desc_lo(v_smem, kKvHalfBytes), p_lo = smem_desc_lo(p_smem, 16);
+            }
+            __syncwarp();
+        };
+        issue_scores(0);
+        for (int j = 0; j < tiles; ++j) {
+            if (j + 1 < tiles) issue_scores(j + 1);
+            const int t = 2 * j + 1, slot = t % kRingSlots, b = j & 1;
+            if (ok) ok = mbar_wait_warp(p_full(b), (j >> 1) & 1, 305);
+            if (ok) ok = mbar_wait_warp(kv_full(slot), (t / kRingSlots) & 1, 306);
+            tc_fence_after();
+            if (leader && ok) {
+                const uint32_t v_smem = smem_base + DecodeSmem::kRing + slot * kKvTileBytes;
+                const uint32_t p_smem = smem_base + DecodeSmem::kP + b * 4096;
+                const uint32_t v_lo = smem_desc_lo(v_smem, kKvHalfBytes), p_lo = smem_desc_lo(p_smem, 16);
 #pragma unroll
-                    for (int k = 0; k < kTileKeys / 16; ++k)
-                        umma_bf16(tmem_o, desc_words(v_lo + ((k * 2048) >> 4), smem_desc_hi(1024)),
-                                  desc_words(p_lo + (((k >> 2) * (kHeadsPadded * 128) + (k & 3) * 32) >> 4), smem_desc_hi(1024)), idesc_o, (j | k) != 0 ? 1u : 0u);
-                }
+                for (int k = 0; k < kTileKeys / 16; ++k)
+                    umma_bf16(tmem_u + 32, desc_words(v_lo + ((k * 2048) >> 4), smem_desc_hi(1024)),
+                              desc_words(p_lo + (((k >> 2) * (kHeadsPadded * 128) + (k & 3) * 32) >> 4), smem_desc_hi(1024)), idesc_o, (j | k) != 0 ? 1u : 0u);
+            }
+            if (leader) {
                 umma_commit(kv_empty(slot));
                 umma_commit(pv_done(b));
             }
+            __syncwarp();
         }
     } else {
         const int quadrant = warp & 3;
