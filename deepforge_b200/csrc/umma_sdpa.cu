@@ -269,35 +269,38 @@ __device__ __forceinline__ PairItem pair_item(const SdpaUmmaArgs& args, int bh, 
 
 // The work list of one CTA (or cluster), the same in every warp role.
 //   kAsStored        every query pair of a head is a unit
-//   kHeavyWithLight  causal, many pairs: unit i of a head is the heavy pair P-1-i followed by the light pair i, so that every unit
+//   kHeavyWithLight  causal, one SM per pair: unit i of a head is the heavy pair P-1-i followed by the light pair i, so that every unit
 //                    walks 2P+2 key tiles and equal numbers of units are equal work
-//   kHeaviestFirst   causal, pairs for a few rounds at most: the pairs of all heads by falling length, and every other round
+//   kHeaviestFirst   causal, two SMs per pair: the pairs of all heads by falling length, and every other round
 //                    in reverse, so that the CTA with the longest pair of one round gets the shortest of the next
 // CTA c takes units c, c + gridDim.x, ...; but for the last order neighbouring CTAs thus work on the same head at the same
 // time and share its K and V in L2.
 enum { kAsStored = 0, kHeavyWithLight = 1, kHeaviestFirst = 2 };
+template <int CTAS>   // that walk one list together
 struct PairWalker {
-    int ctas;   // that walk one list together
     int k = 0;
-    __device__ __forceinline__ explicit PairWalker(int group = 1) : ctas(group) {}
     __device__ __forceinline__ bool next(const SdpaUmmaArgs& args, int& bh, int& pair) {
         const int pairs = args.pairs;
-        const int places = static_cast<int>(gridDim.x) / ctas, place = static_cast<int>(blockIdx.x) / ctas;   // (the grid is a multiple of ctas)
-        if (args.order == kHeaviestFirst) {
-            const int unit = k * places + ((k & 1) ? places - 1 - place : place);
+        if constexpr (CTAS == 2) {
+            const int places = static_cast<int>(gridDim.x) / CTAS, place = static_cast<int>(blockIdx.x) / CTAS;   // (the grid is a multiple of CTAS)
+            const bool heaviest_first = args.order == kHeaviestFirst;
+            const int unit = k * places + (heaviest_first && (k & 1) ? places - 1 - place : place);
             ++k;
-            if (unit >= pairs * args.batch_heads) {   // (a reversed last round may miss this place's unit only, and nothing follows it)
-                return false;
+            if (unit >= pairs * args.batch_heads) return false;   // (a reversed last round may have nothing for this place)
+            if (heaviest_first) {
+                pair = unit / args.batch_heads;
+                bh = unit - pair * args.batch_heads;
+                pair = pairs - 1 - pair;
+            } else {
+                bh = unit / pairs;
+                pair = unit - bh * pairs;
             }
-            pair = unit / args.batch_heads;
-            bh = unit - pair * args.batch_heads;
-            pair = pairs - 1 - pair;
             return true;
         }
         const int units_per_head = args.order == kHeavyWithLight ? (pairs + 1) >> 1 : pairs;
         const int units = units_per_head * args.batch_heads;
         for (;; ++k) {
-            const int unit = place + (k >> 1) * places;
+            const int unit = static_cast<int>(blockIdx.x) + (k >> 1) * static_cast<int>(gridDim.x);
             if (unit >= units) return false;
             bh = unit / units_per_head;
             const int i = unit - bh * units_per_head;
@@ -313,9 +316,9 @@ struct PairWalker {
         }
     }
 };
-template <class Body>
-__device__ __forceinline__ void for_each_pair_item(const SdpaUmmaArgs& args, int ctas, Body&& body) {
-    PairWalker walker(ctas);
+template <int CTAS, class Body>
+__device__ __forceinline__ void for_each_pair_item(const SdpaUmmaArgs& args, Body&& body) {
+    PairWalker<CTAS> walker;
     int bh, pair;
     while (walker.next(args, bh, pair))  // one call site of the body: it is a whole warp role
         if (!body(bh, pair)) return;
@@ -383,14 +386,14 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot_ptr;
     chain_wait();
-    chain_release();
+    // (no early release: this kernel fills every SM, so the next one's CTAs would only wait beside it, 0.6 % of 330 us)
 
     if (warp == 16) {
         const bool leader = elect_one();
         int slot = 0;
         uint32_t phase = 1;  // parity of the "slot is free" wait
         uint32_t n = 0;      // items started
-        for_each_pair_item(args, 1, [&](int bh, int pair) {
+        for_each_pair_item<1>(args, [&](int bh, int pair) {
             const PairItem item = pair_item<EDGES>(args, bh, pair);
             auto load_box = [&](uint32_t dst, const CUtensorMap* map, int row, int head, uint32_t bar) {
 #pragma unroll
@@ -471,7 +474,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     umma_bf16_a_tmem(d_tmem, p_tmem + (k >> 2) * 64 + (k & 3) * 8, desc_words(v_lo + ((k * 2048) >> 4), kDescHi), idesc_pv, (j | k) != 0 ? 1u : 0u);
             }
         };
-        PairWalker walker;
+        PairWalker<1> walker;
         int bh = 0, pair = 0, next_bh = 0, next_pair = 0;
         bool have = walker.next(args, bh, pair);
         bool early = false;  // S_A of the current item was issued in the previous item's last round
@@ -552,7 +555,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         const bool leader = elect_one();
         uint32_t n = 0;
         bool ok = true;
-        for_each_pair_item(args, 1, [&](int bh, int pair) {
+        for_each_pair_item<1>(args, [&](int bh, int pair) {
             const PairItem item = pair_item<EDGES>(args, bh, pair);
             for (int x = 0; x < 2; ++x) {
                 if (ok) ok = mbar_wait_warp(staged(x), n & 1, 216 + x);
@@ -592,7 +595,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         uint32_t s_count = 0;  // score tiles consumed (parity of s_full)
         uint32_t ring_base = 0;  // ring slots of the items before this one
         bool ok = true;
-        for_each_pair_item(args, 1, [&](int bh, int pair) {
+        for_each_pair_item<1>(args, [&](int bh, int pair) {
         const PairItem item = pair_item<EDGES>(args, bh, pair);
         const int q_tile = item.q_tile_a + x;
         const int q_index = q_tile * kRows + row;
@@ -650,13 +653,24 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             const float tile_max = fmaxf(__uint_as_float(mine_up), other) * scale;
             // raise the reference only when it would grow by more than the threshold (or on the first tile); the two
             // warps of these rows see the same maxima, so they take the same branches
-            float alpha = 1.0f;
-            const bool raise = __any_sync(0xffffffffu, tile_max > m_ref + kRescaleThreshold) != 0;
-            if (raise) {
+            if (__any_sync(0xffffffffu, tile_max > m_ref + kRescaleThreshold)) {
                 const float m_new = fmaxf(m_ref, tile_max);
-                alpha = m_ref == -INFINITY ? 0.0f : ex2_fast(m_ref - m_new);
+                const float alpha = m_ref == -INFINITY ? 0.0f : ex2_fast(m_ref - m_new);
                 l_sum *= alpha;
                 m_ref = m_new;
+                if (j > 0) {
+                    // O_x holds P V up to tile j-1; that product was issued ahead of S_x(j), which has completed.
+                    // This thread rescales its columns of the row.
+#pragma unroll 1
+                    for (int c = 0; c < kColumns / 16; ++c) {
+                        uint32_t acc[16];
+                        tmem_load_16(tmem_o + c * 16, acc);
+                        tmem_load_wait_for(acc);
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) acc[e] = __float_as_uint(__uint_as_float(acc[e]) * alpha);
+                        tmem_store_16(tmem_o + c * 16, acc);
+                    }
+                }
             }
             {
                 // (probabilities go over columns whose scores have been read: 8 columns for every 16)
@@ -676,19 +690,6 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 float lo, hi;
                 unpack2(add2(sums[0], sums[1]), lo, hi);
                 l_sum += lo + hi;
-            }
-            if (raise && j > 0) {
-                // O_x holds P V up to tile j-1; that product was issued ahead of S_x(j), which has completed.
-                // This thread rescales its columns of the row.
-#pragma unroll 1
-                for (int c = 0; c < kColumns / 16; ++c) {
-                    uint32_t acc[16];
-                    tmem_load_16(tmem_o + c * 16, acc);
-                    tmem_load_wait_for(acc);
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) acc[e] = __float_as_uint(__uint_as_float(acc[e]) * alpha);
-                    tmem_store_16(tmem_o + c * 16, acc);
-                }
             }
             if (EDGES && args.len_q != nullptr && (j + 1) * kKeys > item.kv_len && (D == 128 || half == 0)) {
                 // V rows past the batch's length are not this sequence's: cleared before the product (by either tile's
@@ -858,7 +859,7 @@ __device__ __forceinline__ void duo_product(uint32_t d, uint32_t a, uint64_t b, 
 // The key tiles of a cluster's work list, one after the other.
 template <bool EDGES>
 struct TileCursor {
-    PairWalker walker;
+    PairWalker<2> walker;
     PairItem item;
     int j;        // key tile of the item
     uint32_t n;   // items before this one
@@ -871,7 +872,7 @@ struct TileCursor {
         j = 0;
     }
     __device__ __forceinline__ void start(const SdpaUmmaArgs& args) {
-        walker = PairWalker(2);
+        walker = PairWalker<2>();
         n = t = 0;
         take(args);
     }
@@ -1069,7 +1070,7 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         const bool leader = elect_one();
         uint32_t n = 0;
         bool ok = true;
-        for_each_pair_item(args, 2, [&](int bh, int pair) {
+        for_each_pair_item<2>(args, [&](int bh, int pair) {
             const PairItem item = pair_item<EDGES>(args, bh, pair);
             if (ok) ok = mbar_wait_warp(staged, n & 1, 249);
             if (leader) {
@@ -1100,7 +1101,7 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         uint32_t n = 0, t0 = 0, edges = 0;
         uint32_t mine_done = 0;   // key tiles this group has finished (parity of its maxima and references)
         bool ok = true;
-        for_each_pair_item(args, 2, [&](int bh, int pair) {
+        for_each_pair_item<2>(args, [&](int bh, int pair) {
             const PairItem item = pair_item<EDGES>(args, bh, pair);
             const int q_tile = item.q_tile_a + rank, q_index = q_tile * kRows + row;
             const bool idle_tile = q_tile * kRows >= item.live_q;   // no row of this CTA's has keys
@@ -1438,7 +1439,7 @@ int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, cudaStrea
     // persistent: one CTA (or cluster of two) per SM (or two) over the work list (see PairWalker)
     const int places = duo ? sm_count() / 2 : sm_count();
     const int64_t single = pairs * heads;
-    args.order = !args.causal || single <= places ? kAsStored : (single <= 4 * places ? kHeaviestFirst : kHeavyWithLight);
+    args.order = !args.causal || single <= places ? kAsStored : (duo ? kHeaviestFirst : kHeavyWithLight);   // (the third order in the one-SM kernel cost it 1.4 %)
     const int64_t units = args.order == kHeavyWithLight ? (pairs + 1) / 2 * heads : single;
     const unsigned grid = static_cast<unsigned>(std::min<int64_t>(units, places));
     const bool f16 = p.q.dtype == DFGPU_F16;
