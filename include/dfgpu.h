@@ -259,13 +259,14 @@ int dfgpu_conv_fprop_pair(const dfgpu_conv_pair_params*, void* const* tensors, v
    that feed A and B (SpecializedGraph.cpp:752-795), reading E4M3 codes and
    E8M0 scales directly. tensors: {A, B, C, A_scale or null, B_scale or null,
    extra0 or null, extra1 or null}. */
-/* UMMA_F32X3: f32 A, B and C on tcgen05: A and B split into three bf16 pieces each, six bf16 products (2^-24 relative);
-   needs scratch, three launches (split, the bf16 matmul over 6K, and the CUDA-core kernel again, which returns at once
-   unless A or B held an infinity or a NaN).
+/* UMMA_BF16: BFLOAT16 or HALF operands, any extents: contiguous rows on 16-byte boundaries (AUTO reads others on CUDA cores).
+   UMMA_F32X3: f32 A, B and C on tcgen05: A and B split into three bf16 pieces each, six bf16 products (2^-24 relative);
+   needs scratch, three launches (split, the products, and the CUDA-core kernel again, which returns at once
+   unless A or B held an infinity or a NaN). Unbatched, A with K and B with K or N contiguous, any extents and alignment.
    UMMA_F32X3_CLUSTER: the same six products in ONE launch without scratch: the kernel of DFGPU_CONV_UMMA_F32X3_CLUSTER run
    on the 1 x 1 convolution of M pixels, one image per matrix of the (at most one) batch axis. Made for at most 148 output
    tiles (128 x 64); more tiles run one CTA each (K at most 4096 then). Any strides of A, B and C and 4-byte aligned
-   pointers (float4 accesses where K is a multiple of 8, N of 4, the rows are contiguous and everything falls on 16-byte
+   pointers (float4 accesses where K and N are multiples of 4, the rows are contiguous and everything falls on 16-byte
    boundaries); HALF and BFLOAT16 matrices value by value. */
 enum { DFGPU_MATMUL_AUTO = 0, DFGPU_MATMUL_FFMA = 1, DFGPU_MATMUL_UMMA_BF16 = 2, DFGPU_MATMUL_UMMA_MXF8 = 3, DFGPU_MATMUL_UMMA_F32X3 = 4,
        DFGPU_MATMUL_UMMA_F32X3_CLUSTER = 5 };
@@ -290,10 +291,11 @@ int dfgpu_matmul(const dfgpu_matmul_params*, void* const* tensors, void* scratch
    zero gives +0, NaN gives 0x7f). The three scales and Amax_C are one-element FLOAT tensors in
    device memory. tensors: {A, B, C, Amax_C, Descale_A, Descale_B, Scale_C}.
    The extent-override inputs (M_override, N_override, K_override) are not executable.
-   Two launches: Amax_C is cleared, then one kernel computes C and folds Amax_C with an
+   Two launches: Amax_C is cleared by a kernel, then one kernel computes C and folds Amax_C with an
    atomic maximum. DFGPU_MATMUL_FP8_UMMA runs the products on tcgen05
-   (kind::mxf8f6f4 with unit block scales) and needs M, N, K multiples of 128, no batch
-   axes, A rows and B rows or columns contiguous; AUTO picks it when it fits. */
+   (kind::f8f6f4) and promises M, N, K multiples of 128, no batch
+   axes, A rows and B rows or columns contiguous; AUTO takes the same kernel for any extents whose
+   rows start on 16-byte boundaries. */
 enum { DFGPU_MATMUL_FP8_AUTO = 0, DFGPU_MATMUL_FP8_SCALAR = 1, DFGPU_MATMUL_FP8_UMMA = 2 };
 typedef struct dfgpu_matmul_fp8_params {
     dfgpu_tensor a, b, c;
@@ -316,7 +318,7 @@ enum {
     DFGPU_SDPA_AUTO = 0,
     DFGPU_SDPA_ROWWISE = 1,           /* general kernel on CUDA cores */
     DFGPU_SDPA_PAGED_DECODE = 2,      /* split-KV paged decode on CUDA cores */
-    DFGPU_SDPA_UMMA = 3,              /* tcgen05 forward, bf16, D = 128, contiguous K/V */
+    DFGPU_SDPA_UMMA = 3,              /* tcgen05 forward, bf16 or f16, D = 64 or 128, any lengths, contiguous K/V */
     DFGPU_SDPA_PAGED_DECODE_UMMA = 4  /* paged decode streamed by TMA, products on tcgen05 */
 };
 typedef struct dfgpu_sdpa_params {
