@@ -370,7 +370,7 @@ umma_conv_f32_kernel(const __grid_constant__ ClusterConvArgs g, const __grid_con
                 if (elect_one()) {
                     // middle*middle, low*high, high*low, middle*high, high*middle meet in an accumulator of their own: the tensor cores
                     // cut off what a sum does not hold, and beside high*high (2^8 times larger) each would lose as much as it does
-                    // (largest error at 2544 x 120 x 512: 16 units of 2^-24 sum |x w| in one accumulator, 3 in two)
+                    // (largest error at 2544 x 120 x 512: 16 units of 2^-24 sum |x w| in one accumulator, 4 in two)
                     constexpr int piece_a[6] = {1, 2, 0, 1, 0, 0}, piece_b[6] = {1, 0, 2, 0, 1, 0};
 #pragma unroll
                     for (int product = 0; product < 6; ++product)

@@ -44,17 +44,6 @@ struct SdpaUmmaArgs {
     int32_t batch_heads;  // batch * query heads
 };
 
-__device__ __forceinline__ void tmem_store_32(uint32_t taddr, const uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-          "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
-          "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]),
-          "r"(r[30]), "r"(r[31])
-        : "memory");
-}
 __device__ __forceinline__ void tmem_store_16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
@@ -143,17 +132,8 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
 // cubic for 2^(x - n) on [-0.5, 0.5] (relative error 7.5e-5, far below the bf16 rounding of P) and add n
 // to the exponent field. The special-function unit runs 16 ex2 per clock per SM: 1024 cycles for a 128 x 128
 // score tile, as long as its two tensor-core products take, so part of the exponentials go this way.
-__device__ __forceinline__ float exp2_poly(float x) {
-    x = fmaxf(x, -125.0f);  // masked scores (-inf) end as 2^-125: nothing in a sum that holds a term >= 2^-8
-    const float magic = 12582912.0f;
-    const float t = x + magic;
-    const float f = x - (t - magic);
-    const float p = fmaf(fmaf(fmaf(0.0551716685f, f, 0.2426111251f), f, 0.6932609677f), f, 0.9999280572f);
-    return __int_as_float(__float_as_int(p) + (__float_as_int(t) << 23));
-}
-
-// The same on a packed pair: the range reduction and the cubic run as f32x2 instructions (6 per pair), only the clamp
-// and the exponent insertion are per element.
+// On a packed pair: the range reduction and the cubic run as f32x2 instructions (6 per pair), only the clamp and the
+// exponent insertion are per element. Masked scores (-inf) end as 2^-125: nothing in a sum that holds a term >= 2^-8.
 __device__ __forceinline__ void exp2_poly_pair(uint64_t x2, float& p0, float& p1) {
     float x0, x1;
     unpack2(x2, x0, x1);
