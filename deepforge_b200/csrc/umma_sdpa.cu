@@ -11,7 +11,7 @@
 // the positions past the end with zeros and clips them on the store, and what is left is a mask on the last key tile. With
 // SEQ_LEN_Q / SEQ_LEN_KV a batch's key tiles end at its own length, V rows behind it are cleared in shared memory (a zero
 // probability times an infinity in the padding would be NaN), and rows past SEQ_LEN_Q store 0 and -inf. 4 x 16 heads of 1000
-// padded positions, causal: 9.7 ms on the row-at-a-time kernel.
+// padded positions, causal: 9.7 ms on the row-at-a-time kernel, 36 us here (31 with P in one 16-bit piece, and O 1.33 times as far from 64 bits).
 #include <algorithm>
 #include <cmath>
 
@@ -26,7 +26,7 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 units
 
 struct SdpaUmmaArgs {
     int32_t heads_q, heads_kv, seq_q, seq_kv;
-    int32_t q_tiles, pairs;   // 128-row query tiles and pairs of them, the last one perhaps partly past the end
+    int32_t pairs;            // of 128-row query tiles, the last one perhaps partly past the end
     int32_t causal;
     int32_t order;            // of the work list: kAsStored, kHeavyWithLight or kHeaviestFirst (see PairWalker)
     float scale_log2;  // |attn_scale| * log2(e); a negative scale negates Q in the products
@@ -41,6 +41,7 @@ struct SdpaUmmaArgs {
     float* row_sum;
     int64_t max_stride[3], sum_stride[3];
     float attn_scale;  // |attn_scale|, natural-log units: Max = attn_scale * largest dot product
+    float to_natural[2];  // attn_scale / scale_log2 as a sum: what takes m_ref to natural-log units
     int32_t batch_heads;  // batch * query heads
 };
 
@@ -56,6 +57,9 @@ __device__ __forceinline__ void tmem_store_8(uint32_t taddr, const uint32_t (&r)
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                  : "memory");
 }
+__device__ __forceinline__ void tmem_store_4(uint32_t taddr, const uint32_t (&r)[4]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
+}
 __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ---- two query tiles per CTA ------------------------------------------------------
@@ -64,11 +68,10 @@ __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::
 //   warp 16     TMA: Q_A, Q_B once, then K_0, V_0, K_1, ... into a ring of 32 KiB slots
 //   warp 17     one lane issues, per key tile j:  O_A += P_A(j) V_j ; S_A(j+1) = Q_A K_{j+1}^T ;
 //                                                 O_B += P_B(j) V_j ; S_B(j+1) = Q_B K_{j+1}^T
-//   warps 0-7   softmax of tile A, warps 8-15 softmax of tile B (four whole warpgroups, which take the registers the
-//               loader and issuing warps give up): two threads per query row, each with 64 of the
+//   warps 0-7   softmax of tile A, warps 8-15 softmax of tile B: two threads per query row, each with 64 of the
 //               tile's 128 keys (the two warps that share a lane quarter trade row maxima through shared memory)
 // (D is the head dimension.) TMEM: S_A at +0, S_B at +128, O_A at +256, O_B at +384. P never goes through shared memory: each
-// thread overwrites the front of its own score row with the bf16 probabilities (two per 32-bit
+// thread overwrites its own score row with the 16-bit probabilities (two per 32-bit
 // column) and the second product takes its A operand from tensor memory. The tensor pipe runs the
 // products of one CTA in issue order, so S_X(j+1) may be issued right behind the product that reads P_X(j).
 // Under a causal mask tile A (the earlier rows) has one key tile fewer than tile B.
@@ -190,25 +193,65 @@ __device__ __forceinline__ uint32_t pack_pair(float lo, float hi) {
         return *reinterpret_cast<const uint32_t*>(&two);
     }
 }
-// Sixteen scores -> probabilities 2^(s * scale + bias) as eight bf16 or f16 pairs, their sum added to two packed partial sums.
 template <bool F16>
-__device__ __forceinline__ void probabilities_of_16(const uint32_t (&raw)[16], uint64_t scale2, uint64_t bias2, uint64_t (&sums)[2], uint32_t* packed) {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        const uint64_t v = fma2(pack2(__uint_as_float(raw[2 * e]), __uint_as_float(raw[2 * e + 1])), scale2, bias2);
-        float p0, p1;
-        if (kPolyEvery > 0 && e % (kPolyEvery > 0 ? kPolyEvery : 1) == 0) {
-            exp2_poly_pair(v, p0, p1);  // this pair on the FMA pipe
-        } else {
-            float x0, x1;
-            unpack2(v, x0, x1);
-            p0 = ex2_fast(x0);
-            p1 = ex2_fast(x1);
-        }
-        sums[e & 1] = add2(sums[e & 1], pack2(p0, p1));
-        packed[e] = pack_pair<F16>(p0, p1);
+__device__ __forceinline__ void unpack_pair(uint32_t two, float& lo, float& hi) {
+    if constexpr (F16) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&two));
+        lo = f.x;
+        hi = f.y;
+    } else {
+        lo = __uint_as_float(two << 16);
+        hi = __uint_as_float(two & 0xffff0000u);
     }
 }
+// Sixteen scores -> probabilities 2^(s * scale + bias) as bf16 or f16 pairs in tensor memory, their sum added to two packed partial
+// sums. GENERAL: every exponential by the special-function unit (2^-22), and eight columns behind each pair what its rounding left
+// over, eight scores at a time (sixteen at once spilled).
+template <bool F16, bool GENERAL>
+__device__ __forceinline__ void put_probabilities(const uint32_t (&raw)[16], uint64_t scale2, uint64_t bias2, uint64_t (&sums)[2], uint32_t address) {
+    constexpr int kParts = GENERAL ? 2 : 1, kPairs = 8 / kParts;
+#pragma unroll
+    for (int part = 0; part < kParts; ++part) {
+        uint32_t packed[kPairs], left[kPairs];
+#pragma unroll
+        for (int e = 0; e < kPairs; ++e) {
+            const int i = part * kPairs + e;
+            const uint64_t v = fma2(pack2(__uint_as_float(raw[2 * i]), __uint_as_float(raw[2 * i + 1])), scale2, bias2);
+            float p0, p1;
+            if (!GENERAL && kPolyEvery > 0 && i % (kPolyEvery > 0 ? kPolyEvery : 1) == 0) {
+                exp2_poly_pair(v, p0, p1);  // this pair on the FMA pipe
+            } else {
+                float x0, x1;
+                unpack2(v, x0, x1);
+                p0 = ex2_fast(x0);
+                p1 = ex2_fast(x1);
+            }
+            sums[i & 1] = add2(sums[i & 1], pack2(p0, p1));
+            packed[e] = pack_pair<F16>(p0, p1);
+            if constexpr (GENERAL) {
+                float head0, head1;
+                unpack_pair<F16>(packed[e], head0, head1);
+                left[e] = pack_pair<F16>(p0 - head0, p1 - head1);
+            }
+        }
+        if constexpr (GENERAL) {
+            tmem_store_4(address + part * 4, packed);
+            tmem_store_4(address + 8 + part * 4, left);
+        } else {
+            tmem_store_8(address, packed);
+        }
+    }
+}
+// Stats of a row whose probabilities were formed against m_ref.
+template <bool GENERAL>
+__device__ __forceinline__ float natural_log_sum(const SdpaUmmaArgs& args, float m_ref, float total) {
+    // (rounded once behind the logarithm, as the row-at-a-time kernel's)
+    if constexpr (GENERAL) return fmaf(m_ref, args.to_natural[0], fmaf(m_ref, args.to_natural[1], logf(total)));
+    return 0.6931471805599453f * (m_ref + log2f(total));
+}
+// Columns that put_probabilities() fills for 16 keys.
+template <bool GENERAL>
+constexpr int kProbabilityColumns = GENERAL ? 16 : 8;
 
 // One (batch, head, query pair) of the work list.
 struct PairItem {
@@ -220,9 +263,12 @@ struct PairItem {
     int live_q;          // query rows before this one have keys; the others store 0 and -inf
 };
 
-// EDGES: a batch's keys may end inside a key tile (padding masks, or a key length that is no multiple of 128). Without them
-// the masks of the last tile, the clearing of V rows and the dead rows are not compiled in: they cost 5 % of 8 x 32 x 2048 causal.
-template <bool EDGES>
+// GENERAL: what the kernels take beyond whole tiles of packed bf16 rows of 128 (plain_tiles()): a batch's keys may end inside a key
+// tile (padding masks, or a key length that is no multiple of 128), and probabilities are held to f32's accuracy: O += P V runs
+// twice, on P rounded to the operands' type and on what that left over (16 or 22 bits in all), as O and Stats of these graphs are
+// those of f32 probabilities (sdpa_rowwise_kernel's) to the rounding of O. Without it the masks of the last tile, the clearing of V
+// rows and the dead rows are not compiled in: they cost 5 % of 8 x 32 x 2048 causal.
+template <bool GENERAL>
 __device__ __forceinline__ PairItem pair_item(const SdpaUmmaArgs& args, int bh, int pair) {
     PairItem item;
     item.batch = bh / args.heads_q;
@@ -231,7 +277,7 @@ __device__ __forceinline__ PairItem pair_item(const SdpaUmmaArgs& args, int bh, 
     item.q_tile_a = 2 * pair;
     item.kv_len = args.seq_kv;
     item.live_q = args.seq_q;
-    if (EDGES && args.len_q != nullptr) {
+    if (GENERAL && args.len_q != nullptr) {
         const int len_kv = __ldg(args.len_kv + item.batch * args.len_kv_stride);
         item.live_q = len_kv > 0 ? min(item.live_q, __ldg(args.len_q + item.batch * args.len_q_stride)) : 0;
         item.kv_len = max(1, min(item.kv_len, len_kv));
@@ -312,7 +358,7 @@ __device__ __forceinline__ void for_each_pair_item(const SdpaUmmaArgs& args, Bod
 //   warp 17     issues the products; one elected lane issues, all lanes walk the schedule
 //   warp 18     sends staged output tiles to global memory by TMA (row-per-thread global stores of 16 bytes at a
 //               256-byte stride kept the load/store unit busy for ~5000 cycles per tile)
-template <int D, bool F16, bool EDGES>
+template <int D, bool F16, bool GENERAL>
 __global__ void __launch_bounds__(kPairThreads, 1)
 sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o, SdpaUmmaArgs args) {
@@ -374,7 +420,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         uint32_t phase = 1;  // parity of the "slot is free" wait
         uint32_t n = 0;      // items started
         for_each_pair_item<1>(args, [&](int bh, int pair) {
-            const PairItem item = pair_item<EDGES>(args, bh, pair);
+            const PairItem item = pair_item<GENERAL>(args, bh, pair);
             auto load_box = [&](uint32_t dst, const CUtensorMap* map, int row, int head, uint32_t bar) {
 #pragma unroll
                 for (int h = 0; h < D / 64; ++h) tma_load_4d(dst + h * kHalfBytes, map, 64 * h, row, head, item.batch, bar);
@@ -437,8 +483,9 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 }
             }
         };
-        // O_x += P_x V_j. P_x lies as bf16 pairs over the scores: keys 0..63 in columns 0..31 of S_x, keys 64..127 in columns
-        // 64..95 (each softmax thread overwrites columns that held its own scores only). The first product of an item
+        // O_x += P_x V_j. P_x lies as 16-bit pairs over the scores: keys 0..63 in columns 0..31 of S_x, keys 64..127 in columns
+        // 64..95 (each softmax thread overwrites columns that held its own scores only); GENERAL: every 16 keys' pairs and then
+        // their left-overs over those keys' 16 scores, so columns 0..63 and 64..127. The first product of an item
         // overwrites O_x, which the softmax warps must have read out for the previous item.
         auto product = [&](int x, int j, int v_slot) {
             if (ok && j == 0) ok = mbar_wait_warp(o_empty(x), (n & 1) ^ 1, 218 + x);
@@ -450,8 +497,11 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             const uint32_t d_tmem = tmem_u + 256 + x * 128, p_tmem = tmem_u + x * 128;
             if (leader) {
 #pragma unroll
-                for (int k = 0; k < kKeys / 16; ++k)
-                    umma_bf16_a_tmem(d_tmem, p_tmem + (k >> 2) * 64 + (k & 3) * 8, desc_words(v_lo + ((k * 2048) >> 4), kDescHi), idesc_pv, (j | k) != 0 ? 1u : 0u);
+                for (int k = 0; k < kKeys / 16; ++k) {
+                    const uint32_t p_at = p_tmem + (k >> 2) * 64 + (k & 3) * kProbabilityColumns<GENERAL>;
+                    umma_bf16_a_tmem(d_tmem, p_at, desc_words(v_lo + ((k * 2048) >> 4), kDescHi), idesc_pv, (j | k) != 0 ? 1u : 0u);
+                    if constexpr (GENERAL) umma_bf16_a_tmem(d_tmem, p_at + 8, desc_words(v_lo + ((k * 2048) >> 4), kDescHi), idesc_pv, 1u);
+                }
             }
         };
         PairWalker<1> walker;
@@ -460,10 +510,10 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         bool early = false;  // S_A of the current item was issued in the previous item's last round
         int early_slot = 0;  // the ring slot of its K tile
         while (have && ok) {
-            const PairItem item = pair_item<EDGES>(args, bh, pair);
+            const PairItem item = pair_item<GENERAL>(args, bh, pair);
             const int tiles_a = item.tiles_a, tiles_b = item.tiles_b, tiles = item.tiles;
             const bool have_next = walker.next(args, next_bh, next_pair);
-            const int next_tiles_a = have_next ? pair_item<EDGES>(args, next_bh, next_pair).tiles_a : 0;
+            const int next_tiles_a = have_next ? pair_item<GENERAL>(args, next_bh, next_pair).tiles_a : 0;
             int k0_slot = early_slot;
             if (!early) {
                 if (ok) ok = mbar_wait_warp(q_full(0), n & 1, 222);
@@ -536,7 +586,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         uint32_t n = 0;
         bool ok = true;
         for_each_pair_item<1>(args, [&](int bh, int pair) {
-            const PairItem item = pair_item<EDGES>(args, bh, pair);
+            const PairItem item = pair_item<GENERAL>(args, bh, pair);
             for (int x = 0; x < 2; ++x) {
                 if (ok) ok = mbar_wait_warp(staged(x), n & 1, 216 + x);
                 if (leader) {
@@ -576,7 +626,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         uint32_t ring_base = 0;  // ring slots of the items before this one
         bool ok = true;
         for_each_pair_item<1>(args, [&](int bh, int pair) {
-        const PairItem item = pair_item<EDGES>(args, bh, pair);
+        const PairItem item = pair_item<GENERAL>(args, bh, pair);
         const int q_tile = item.q_tile_a + x;
         const int q_index = q_tile * kRows + row;
         const int my_tiles = x ? item.tiles_b : item.tiles_a;
@@ -590,9 +640,9 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             // pass against the last tile's reference, probabilities wait for the exchange in registers: 2650 clocks from scores to
             // probabilities, 2270 this way.)
             // keys 0..limit of this thread's 64 are visible; only a tile at the diagonal or at the batch's end has others
-            const int last_key = !EDGES ? q_index : (args.causal ? min(q_index, item.kv_len - 1) : item.kv_len - 1);
+            const int last_key = !GENERAL ? q_index : (args.causal ? min(q_index, item.kv_len - 1) : item.kv_len - 1);
             const int limit = last_key - j * kKeys - half * 64;
-            const bool diagonal = (args.causal && j == q_tile) || (EDGES && (j + 1) * kKeys > item.kv_len);
+            const bool diagonal = (args.causal && j == q_tile) || (GENERAL && (j + 1) * kKeys > item.kv_len);
             const uint32_t scores_at = tmem_s + half * 64;
             auto masked = [&](uint32_t (&raw)[16], int c) {
                 if (diagonal) {
@@ -653,7 +703,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 }
             }
             {
-                // (probabilities go over columns whose scores have been read: 8 columns for every 16)
+                // (probabilities go over columns whose scores have been read: 8 columns for every 16, or all 16)
                 const uint64_t scale2 = pack2(scale, scale), bias2 = pack2(-m_ref, -m_ref);
                 uint64_t sums[2] = {0, 0};  // two independent chains of packed partial sums
                 uint32_t raw[4][16];
@@ -663,15 +713,13 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     tmem_load_wait_for(raw[c]);
                     if (c < 3) tmem_load_16(scores_at + (c + 1) * 16, raw[c + 1]);
                     masked(raw[c], c);
-                    uint32_t packed[8];
-                    probabilities_of_16<F16>(raw[c], scale2, bias2, sums, packed);
-                    tmem_store_8(scores_at + c * 8, packed);
+                    put_probabilities<F16, GENERAL>(raw[c], scale2, bias2, sums, scores_at + c * kProbabilityColumns<GENERAL>);
                 }
                 float lo, hi;
                 unpack2(add2(sums[0], sums[1]), lo, hi);
                 l_sum += lo + hi;
             }
-            if (EDGES && args.len_q != nullptr && (j + 1) * kKeys > item.kv_len && (D == 128 || half == 0)) {
+            if (GENERAL && args.len_q != nullptr && (j + 1) * kKeys > item.kv_len && (D == 128 || half == 0)) {
                 // V rows past the batch's length are not this sequence's: cleared before the product (by either tile's
                 // warps, which write the same zeros). The slot is V_j's place in the ring.
                 const uint32_t place = ring_base + 2 * j + 1, v_slot = place % kPairSlots;
@@ -709,7 +757,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             if (half == 0) {
                 const float row_raw_max = fmaxf(raw_max, sum_exchange[lane]);
                 const int64_t b64 = item.batch, h64 = item.head, q64 = q_index;
-                const bool any = !EDGES || q_index < item.live_q;
+                const bool any = !GENERAL || q_index < item.live_q;
                 const bool inside = ok && q_index < args.seq_q;
                 if (inside && args.row_max != nullptr)
                     args.row_max[b64 * args.max_stride[0] + h64 * args.max_stride[1] + q64 * args.max_stride[2]] = any ? row_raw_max * args.attn_scale : -INFINITY;
@@ -719,7 +767,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         }
         // the hand-over words double as the next item's maxima: every read above must precede those writes
         asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
-        const bool live = !EDGES || q_index < item.live_q;
+        const bool live = !GENERAL || q_index < item.live_q;
         const float inverse = live ? 1.0f / total : 0.0f;
         // the staging tile serves the query tiles in turn: A, B, the next item's A, ...
         {
@@ -753,8 +801,8 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         if (lane == 0) mbar_arrive(staged(x));
         if (args.stats != nullptr && ok && half == 0 && q_index < args.seq_q)
             args.stats[item.batch * args.stats_batch_stride + item.head * args.stats_head_stride + static_cast<int64_t>(q_index) * args.stats_row_stride] =
-                live ? 0.6931471805599453f * (m_ref + log2f(total)) : -INFINITY;
-        if (EDGES) ring_base += 2 * item.tiles;
+                live ? natural_log_sum<GENERAL>(args, m_ref, total) : -INFINITY;
+        if (GENERAL) ring_base += 2 * item.tiles;
         ++n;
         return true;  // also after a wait gave up: the two warps of a row pair must meet at the same barriers to the end
         });
@@ -837,7 +885,7 @@ __device__ __forceinline__ void duo_product(uint32_t d, uint32_t a, uint64_t b, 
 }
 
 // The key tiles of a cluster's work list, one after the other.
-template <bool EDGES>
+template <bool GENERAL>
 struct TileCursor {
     PairWalker<2> walker;
     PairItem item;
@@ -848,7 +896,7 @@ struct TileCursor {
     __device__ __forceinline__ void take(const SdpaUmmaArgs& args) {
         int bh, pair;
         live = walker.next(args, bh, pair);
-        if (live) item = pair_item<EDGES>(args, bh, pair);
+        if (live) item = pair_item<GENERAL>(args, bh, pair);
         j = 0;
     }
     __device__ __forceinline__ void start(const SdpaUmmaArgs& args) {
@@ -868,7 +916,7 @@ struct TileCursor {
 // The item's last key tile ends behind the batch's own length: V rows there are cleared.
 __device__ __forceinline__ bool clears_v(const SdpaUmmaArgs& args, const PairItem& item) { return args.len_q != nullptr && item.tiles * kKeys > item.kv_len; }
 
-template <bool F16, bool EDGES>
+template <bool F16, bool GENERAL>
 __global__ void __launch_bounds__(kPairThreads, 1)
 sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                      const __grid_constant__ CUtensorMap map_o, SdpaUmmaArgs args) {
@@ -936,7 +984,7 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     if (warp == 16) {
         const bool leader = elect_one();
         const uint32_t counted_on = address_in_first(bar_base);   // CTA 0's barriers count both CTAs' bytes
-        TileCursor<EDGES> k, v;
+        TileCursor<GENERAL> k, v;
         k.start(args);
         v.start(args);
         int slot = 0;
@@ -968,7 +1016,7 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         };
         for (int i = 0; i < kDuoBuffers; ++i) put_k();
         while (v.live && ok) {
-            const bool edge = EDGES && v.last() && clears_v(args, v.item);
+            const bool edge = GENERAL && v.last() && clears_v(args, v.item);
             ok = mbar_wait_warp(kv_empty(slot), phase, 242);
             // (a tile whose end is cleared is counted on a barrier of its own CTA, where the clearing warps wait for it)
             if (edge && ok) ok = mbar_wait_warp(edge_done, (edges & 1) ^ 1, 243);
@@ -998,7 +1046,7 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             constexpr uint32_t idesc_pv = kFormats | (static_cast<uint32_t>(128 >> 3) << 17) | (1u << 16);   // (V is read MN-major)
             constexpr uint32_t kDescHi = smem_desc_hi(1024);
             const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
-            TileCursor<EDGES> s, p;
+            TileCursor<GENERAL> s, p;
             s.start(args);
             p.start(args);
             int slot = 0;
@@ -1035,8 +1083,11 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 if (leader && ok) {
                     const uint32_t v_lo = smem_desc_lo(smem_base + Smem::kRing + slot * Smem::kSlot, kHalfBytes), p_tmem = tmem_u + b * 128;
 #pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        duo_product(tmem_u + 384, p_tmem + (k >> 2) * 64 + (k & 3) * 8, desc_words(v_lo + ((k * 2048) >> 4), kDescHi), idesc_pv, (p.j | k) != 0 ? 1u : 0u);
+                    for (int k = 0; k < 8; ++k) {
+                        const uint32_t p_at = p_tmem + (k >> 2) * 64 + (k & 3) * kProbabilityColumns<GENERAL>;
+                        duo_product(tmem_u + 384, p_at, desc_words(v_lo + ((k * 2048) >> 4), kDescHi), idesc_pv, (p.j | k) != 0 ? 1u : 0u);
+                        if constexpr (GENERAL) duo_product(tmem_u + 384, p_at + 8, desc_words(v_lo + ((k * 2048) >> 4), kDescHi), idesc_pv, 1u);
+                    }
                     commit_to_both(pv_done(b));
                     commit_to_both(kv_empty(slot));
                 }
@@ -1051,7 +1102,7 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         uint32_t n = 0;
         bool ok = true;
         for_each_pair_item<2>(args, [&](int bh, int pair) {
-            const PairItem item = pair_item<EDGES>(args, bh, pair);
+            const PairItem item = pair_item<GENERAL>(args, bh, pair);
             if (ok) ok = mbar_wait_warp(staged, n & 1, 249);
             if (leader) {
                 const int row = (item.q_tile_a + rank) * kRows;
@@ -1082,7 +1133,7 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         uint32_t mine_done = 0;   // key tiles this group has finished (parity of its maxima and references)
         bool ok = true;
         for_each_pair_item<2>(args, [&](int bh, int pair) {
-            const PairItem item = pair_item<EDGES>(args, bh, pair);
+            const PairItem item = pair_item<GENERAL>(args, bh, pair);
             const int q_tile = item.q_tile_a + rank, q_index = q_tile * kRows + row;
             const bool idle_tile = q_tile * kRows >= item.live_q;   // no row of this CTA's has keys
             float m_ref = -INFINITY, l_sum = 0.0f, raw_max = -INFINITY;
@@ -1101,9 +1152,9 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 if (ok) ok = mbar_wait(s_full(b), (t / kDuoBuffers) & 1, 251);
                 tc_fence_after();
                 const bool empty = idle_tile || (args.causal && j > q_tile);   // nothing to see for any row: all probabilities are zero
-                const int last_key = !EDGES ? q_index : (args.causal ? min(q_index, item.kv_len - 1) : item.kv_len - 1);
+                const int last_key = !GENERAL ? q_index : (args.causal ? min(q_index, item.kv_len - 1) : item.kv_len - 1);
                 const int limit = last_key - j * kKeys - half * 64;
-                const bool diagonal = (args.causal && j == q_tile) || (EDGES && (j + 1) * kKeys > item.kv_len);
+                const bool diagonal = (args.causal && j == q_tile) || (GENERAL && (j + 1) * kKeys > item.kv_len);
                 // The tile's maximum first, then the reference, then the exponentials: nothing is formed twice. (The scores are read
                 // twice, which costs next to nothing; 64 of them held in registers would spill.)
                 float mine = -INFINITY;
@@ -1156,7 +1207,7 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 }
                 uint64_t sums[2] = {0, 0};
                 if (!empty) {
-                    // (probabilities go over columns whose scores have been read: 8 columns for every 16)
+                    // (probabilities go over columns whose scores have been read: 8 columns for every 16, or all 16)
                     const uint64_t bias2 = pack2(-m_ref, -m_ref);
                     uint32_t raw[4][16];
                     tmem_load_16(tmem_s, raw[0]);
@@ -1165,14 +1216,12 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                         tmem_load_wait_for(raw[c]);
                         if (c < 3) tmem_load_16(tmem_s + (c + 1) * 16, raw[c + 1]);
                         masked(raw[c], c);
-                        uint32_t packed[8];
-                        probabilities_of_16<F16>(raw[c], scale2, bias2, sums, packed);
-                        tmem_store_8(tmem_s + c * 8, packed);
+                        put_probabilities<F16, GENERAL>(raw[c], scale2, bias2, sums, tmem_s + c * kProbabilityColumns<GENERAL>);
                     }
                 } else {
                     const uint32_t zeros[8] = {};
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) tmem_store_8(tmem_s + c * 8, zeros);
+                    for (int c = 0; c < kProbabilityColumns<GENERAL> / 2; ++c) tmem_store_8(tmem_s + c * 8, zeros);
                 }
                 {
                     float lo, hi;
@@ -1194,7 +1243,7 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                         tmem_store_16(tmem_o + c * 16, acc);
                     }
                 }
-                if (EDGES && half == 0 && j + 1 == item.tiles && clears_v(args, item)) {
+                if (GENERAL && half == 0 && j + 1 == item.tiles && clears_v(args, item)) {
                     // V rows past the batch's length are not this sequence's: this CTA's channels of them, a row per thread
                     if (ok) ok = mbar_wait(v_edge, edges & 1, 253);
                     if (j * kKeys + row >= item.kv_len) {
@@ -1212,7 +1261,7 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 if (lane == 0) arrive_in_cluster(p_full_first + 8u * b);
             }
             const uint32_t last = t0 + item.tiles - 1;
-            if (EDGES && clears_v(args, item)) {
+            if (GENERAL && clears_v(args, item)) {
                 // (the group that does not clear waits and arrives as well: a barrier's phases are told apart by their parity, so nobody may
                 // be more than one behind or ahead)
                 if (half == 0 && (last & 1) != static_cast<uint32_t>(group)) {
@@ -1245,7 +1294,7 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(sums_free);
-                const bool live = !EDGES ? true : q_index < item.live_q;
+                const bool live = !GENERAL ? true : q_index < item.live_q;
                 if (half == 0 && ok && q_index < args.seq_q) {
                     const int64_t b64 = item.batch, h64 = item.head, q64 = q_index;
                     if (args.row_max != nullptr)
@@ -1254,7 +1303,7 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                         args.row_sum[b64 * args.sum_stride[0] + h64 * args.sum_stride[1] + q64 * args.sum_stride[2]] = live ? total * exp2f(m_ref - row_raw_max * scale) : 0.0f;
                     if (args.stats != nullptr)
                         args.stats[b64 * args.stats_batch_stride + h64 * args.stats_head_stride + q64 * args.stats_row_stride] =
-                            live ? 0.6931471805599453f * (m_ref + log2f(total)) : -INFINITY;
+                            live ? natural_log_sum<GENERAL>(args, m_ref, total) : -INFINITY;
                 }
                 const float inverse = live ? 1.0f / total : 0.0f;
                 if (ok) ok = mbar_wait(stage_free, (n & 1) ^ 1, 256);
@@ -1314,27 +1363,37 @@ int sdpa_map(CUtensorMap* map, const dfgpu_tensor& t, const void* data, uint32_t
     return make_map(map, data, 4, dims, strides, box, what);
 }
 
-template <int D, bool F16, bool EDGES>
-int launch_edges(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_o, const SdpaUmmaArgs& args, unsigned grid, cudaStream_t stream) {
-    cudaError_t error = cudaFuncSetAttribute(sdpa_umma_pair_kernel<D, F16, EDGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<D>::kDynamic);
+template <int D, bool F16, bool GENERAL>
+int launch_pair(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_o, const SdpaUmmaArgs& args, unsigned grid, cudaStream_t stream) {
+    cudaError_t error = cudaFuncSetAttribute(sdpa_umma_pair_kernel<D, F16, GENERAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<D>::kDynamic);
     if (error != cudaSuccess) return fail(kExecutionFailed, "SDPA: cannot reserve %d bytes of shared memory: %s", PairSmem<D>::kDynamic, cudaGetErrorString(error));
-    launch_chained(sdpa_umma_pair_kernel<D, F16, EDGES>, dim3(grid), dim3(kPairThreads), PairSmem<D>::kDynamic, stream, map_q, map_k, map_v, map_o, args);
+    launch_chained(sdpa_umma_pair_kernel<D, F16, GENERAL>, dim3(grid), dim3(kPairThreads), PairSmem<D>::kDynamic, stream, map_q, map_k, map_v, map_o, args);
     return check_launch("SDPA (tcgen05, two query tiles per CTA)");
 }
-template <bool F16, bool EDGES>
+template <bool F16, bool GENERAL>
 int launch_duo(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_o, const SdpaUmmaArgs& args, unsigned clusters, cudaStream_t stream) {
-    cudaError_t error = cudaFuncSetAttribute(sdpa_umma_duo_kernel<F16, EDGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, DuoSmem::kDynamic);
+    cudaError_t error = cudaFuncSetAttribute(sdpa_umma_duo_kernel<F16, GENERAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, DuoSmem::kDynamic);
     if (error != cudaSuccess) return fail(kExecutionFailed, "SDPA: cannot reserve %d bytes of shared memory: %s", DuoSmem::kDynamic, cudaGetErrorString(error));
-    error = launch_chained_cluster(sdpa_umma_duo_kernel<F16, EDGES>, dim3(2 * clusters), dim3(kPairThreads), 2u, static_cast<size_t>(DuoSmem::kDynamic), stream, map_q, map_k, map_v, map_o, args);
+    error = launch_chained_cluster(sdpa_umma_duo_kernel<F16, GENERAL>, dim3(2 * clusters), dim3(kPairThreads), 2u, static_cast<size_t>(DuoSmem::kDynamic), stream, map_q, map_k, map_v, map_o, args);
     if (error != cudaSuccess) return fail(kExecutionFailed, "SDPA: launch failed: %s", cudaGetErrorString(error));
     return check_launch("SDPA (tcgen05, two SMs per pair of query tiles)");
 }
 template <int D, bool F16>
-int launch_shape(bool duo, const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_o, const SdpaUmmaArgs& args, unsigned grid, cudaStream_t stream) {
-    const bool edges = args.len_q != nullptr || args.seq_kv % kKeys != 0;
+int launch_general(bool duo, const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_o, const SdpaUmmaArgs& args, unsigned grid, cudaStream_t stream) {
     if constexpr (D == 128)
-        if (duo) return edges ? launch_duo<F16, true>(map_q, map_k, map_v, map_o, args, grid, stream) : launch_duo<F16, false>(map_q, map_k, map_v, map_o, args, grid, stream);
-    return edges ? launch_edges<D, F16, true>(map_q, map_k, map_v, map_o, args, grid, stream) : launch_edges<D, F16, false>(map_q, map_k, map_v, map_o, args, grid, stream);
+        if (duo) return launch_duo<F16, true>(map_q, map_k, map_v, map_o, args, grid, stream);
+    return launch_pair<D, F16, true>(map_q, map_k, map_v, map_o, args, grid, stream);
+}
+
+bool packed_rows(const dfgpu_tensor& t) {
+    return t.stride[3] == 1 && t.stride[2] == t.dim[3] && t.stride[1] == t.dim[2] * t.stride[2] && t.stride[0] == t.dim[1] * t.stride[1];
+}
+// Whole 128-row tiles of packed bf16 rows of 128, no padding, a causal mask on square scores only: P V on P rounded to bf16.
+bool plain_tiles(const dfgpu_sdpa_params& p) {
+    const int64_t sq = p.q.dim[2], skv = p.k.dim[2];
+    return p.q.dtype == DFGPU_BF16 && p.q.dim[3] == 128 && !p.padding_mask && sq % kRows == 0 && skv % kKeys == 0 && (!p.has_right_bound || sq == skv) &&
+           packed_rows(p.q) && packed_rows(p.k) && packed_rows(p.v) && packed_rows(p.o) &&
+           ((p.max.rank == 0 && p.sum_exp.rank == 0) || (sq % (2 * kRows) == 0 && p.attn_scale > 0.0f)) && p.q.dim[0] * p.q.dim[1] <= 65535;
 }
 
 }  // namespace
@@ -1390,13 +1449,15 @@ int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, cudaStrea
     args.heads_kv = static_cast<int>(p.k.dim[1]);
     args.seq_q = static_cast<int>(p.q.dim[2]);
     args.seq_kv = static_cast<int>(p.k.dim[2]);
-    args.q_tiles = (args.seq_q + kRows - 1) / kRows;
-    args.pairs = (args.q_tiles + 1) / 2;
+    args.pairs = static_cast<int>(pairs);
     args.batch_heads = static_cast<int>(p.q.dim[0] * p.q.dim[1]);
     args.causal = p.has_right_bound ? 1 : 0;
     // (a scale of zero weighs every key alike; the smallest normal one does too, and keeps scale * -inf at -inf)
     args.attn_scale = std::max(std::fabs(p.attn_scale), 1e-37f);
     args.scale_log2 = args.attn_scale * 1.4426950408889634f;
+    const double to_natural = static_cast<double>(args.attn_scale) / args.scale_log2;
+    args.to_natural[0] = static_cast<float>(to_natural);
+    args.to_natural[1] = static_cast<float>(to_natural - args.to_natural[0]);
     args.negate_q = p.attn_scale < 0.0f ? 1u << 13 : 0u;
     if (p.padding_mask) {
         args.len_q = static_cast<const int32_t*>(tensors[7]);
@@ -1422,9 +1483,10 @@ int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, cudaStrea
     args.order = !args.causal || single <= places ? kAsStored : (duo ? kHeaviestFirst : kHeavyWithLight);   // (the third order in the one-SM kernel cost it 1.4 %)
     const int64_t units = args.order == kHeavyWithLight ? (pairs + 1) / 2 * heads : single;
     const unsigned grid = static_cast<unsigned>(std::min<int64_t>(units, places));
+    if (plain_tiles(p)) return duo ? launch_duo<false, false>(map_q, map_k, map_v, map_o, args, grid, stream) : launch_pair<128, false, false>(map_q, map_k, map_v, map_o, args, grid, stream);
     const bool f16 = p.q.dtype == DFGPU_F16;
-    if (p.q.dim[3] == 64) return f16 ? launch_shape<64, true>(duo, map_q, map_k, map_v, map_o, args, grid, stream) : launch_shape<64, false>(duo, map_q, map_k, map_v, map_o, args, grid, stream);
-    return f16 ? launch_shape<128, true>(duo, map_q, map_k, map_v, map_o, args, grid, stream) : launch_shape<128, false>(duo, map_q, map_k, map_v, map_o, args, grid, stream);
+    if (p.q.dim[3] == 64) return f16 ? launch_general<64, true>(duo, map_q, map_k, map_v, map_o, args, grid, stream) : launch_general<64, false>(duo, map_q, map_k, map_v, map_o, args, grid, stream);
+    return f16 ? launch_general<128, true>(duo, map_q, map_k, map_v, map_o, args, grid, stream) : launch_general<128, false>(duo, map_q, map_k, map_v, map_o, args, grid, stream);
 }
 
 int sdpa_umma_device_status(int* status) { return read_and_clear_device_status(status); }

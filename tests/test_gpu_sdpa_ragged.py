@@ -2,9 +2,11 @@
 keys than queries, grouped heads, padding masks with short and empty sequences (NaN in the padding must not leak), causal or
 not, both 16-bit types and head dimensions, strided layouts, a negative scale. Compared with an f64 softmax of the stored values.
 
-Tolerances: a probability is rounded to the operands' type before it weighs V (u = 2^-8 for bf16, 2^-11 for f16, relative) and
-exponentials are within 2^-13, so O is off by at most (u + 2^-12) sum p |v| before it is rounded once by u; subnormal f16
-probabilities (up to 2^-24 of the largest) add 2^-24 sum |v|. Stats carry the exponentials' error and f32 scores."""
+Tolerances of check(): a probability within u of its value (u = 2^-8 for bf16, 2^-11 for f16, relative) and exponentials within
+2^-13, so O is off by at most (u + 2^-12) sum p |v| before it is rounded once by u; subnormal f16 probabilities (up to 2^-24 of
+the largest) add 2^-24 sum |v|. Stats carry the exponentials' error and f32 scores. `fine` is what forms that are not whole bf16
+tiles of 128 channels promise: probabilities of 16 bits or more (2^-17), exponentials within 2^-22 and scores whose f32 sums over 128
+channels are off by at most 2^-20 sum |q k| (below 2^-16 here), 2^-14 sum p |v| in all, and Stats within 2^-16."""
 import pytest
 
 from deepforge_b200 import dfgpu, graphs, runtime
@@ -35,7 +37,7 @@ def attention(q, k, v, scale, causal, len_q=None, len_kv=None):
     return p @ v, p @ v.abs(), v.abs().sum(-2, keepdim=True), stats
 
 
-def check(b, h, hkv, sq, skv, d, io, causal, padding=None, scale=None, strided=False, seed=3):
+def check(b, h, hkv, sq, skv, d, io, causal, padding=None, scale=None, strided=False, seed=3, fine=False):
     g = torch.Generator(device="cuda").manual_seed(seed)
     scale = d ** -0.5 if scale is None else scale
     def operand(heads, length):
@@ -62,11 +64,11 @@ def check(b, h, hkv, sq, skv, d, io, causal, padding=None, scale=None, strided=F
     assert dfgpu.device_status() == 0
     want, weight, every, want_stats = attention(q, k, v, scale, causal, len_q, len_kv)
     u = ROUNDING[io]
-    bound = (u + 2.0 ** -12) * weight + u * want.abs() + (2.0 ** -24 * every if io == "HALF" else 0.0) + 1e-30
+    bound = (2.0 ** -14 if fine else u + 2.0 ** -12) * weight + u * want.abs() + (2.0 ** -24 * every if io == "HALF" else 0.0) + 1e-30
     error = (o.double() - want).abs()
     assert bool(torch.all(error <= bound)), float((error / bound).nan_to_num(1e9).max())
     dead = torch.isinf(want_stats)
-    assert bool(torch.all(torch.isneginf(stats[dead]))) and bool(torch.all((stats.double() - want_stats)[~dead].abs() <= 1e-3))
+    assert bool(torch.all(torch.isneginf(stats[dead]))) and bool(torch.all((stats.double() - want_stats)[~dead].abs() <= (2.0 ** -16 if fine else 1e-3)))
 
 
 @pytest.mark.parametrize("io,d", [("BFLOAT16", 128), ("HALF", 128), ("BFLOAT16", 64), ("HALF", 64)])
@@ -103,3 +105,17 @@ def test_several_items_per_place(io, b, h, hkv, sq, skv, causal, scale):
 def test_several_padded_items_per_place(causal, h, sq, skv):
     lengths = [(i * 97) % (skv + 1) for i in range(12)]
     check(12, h, 2, sq, skv, 128, "BFLOAT16", causal, padding=([min(sq, n + 30) for n in lengths], lengths))
+
+
+@pytest.mark.parametrize("io,d", [("BFLOAT16", 128), ("HALF", 128), ("BFLOAT16", 64), ("HALF", 64)])
+@pytest.mark.parametrize("b,h,hkv,sq,skv,causal", [(3, 1, 1, 17, 17, True), (5, 4, 1, 75, 89, False), (1, 37, 37, 1000, 1000, True), (2, 96, 96, 300, 300, True), (2, 60, 12, 256, 1500, False)])
+def test_probabilities_as_accurate_as_f32_ones(io, d, b, h, hkv, sq, skv, causal):
+    """On one SM and on two per pair of query tiles, short lists and long."""
+    check(b, h, hkv, sq, skv, d, io, causal, fine=True)
+
+
+def test_padded_and_strided_probabilities_as_accurate_as_f32_ones():
+    check(5, 4, 2, 300, 300, 128, "BFLOAT16", True, padding=([300, 130, 1, 0, 257], [300, 130, 1, 200, 0]), fine=True)
+    check(2, 4, 2, 256, 256, 128, "BFLOAT16", True, strided=True, fine=True)      # (whole tiles, rows that are not packed)
+    check(2, 4, 2, 128, 384, 128, "BFLOAT16", True, fine=True)                    # (whole tiles, more keys than queries under a causal mask)
+    check(2, 4, 2, 256, 256, 128, "HALF", False, fine=True)
