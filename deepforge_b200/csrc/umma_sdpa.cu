@@ -87,9 +87,10 @@ struct PairSmem {
     static constexpr int kRing = 2 * kTile;
     static constexpr int kStage = kRing + kPairSlots * kTile;  // one output tile on its way to global memory
     // 128 bytes per (tile, lane quarter): during the key loop the half-row maxima [half][lane] as bf16, after it the row sum
-    // [lane] as f32. 1 KiB in all: with two Q tiles, four 32 KiB ring slots and the output tile this is what the 227 KiB leave.
+    // [lane] as f32; GENERAL: behind them the maxima's third bytes (f32 maxima would not fit beside two Q tiles, four 32 KiB ring
+    // slots and the output tile).
     static constexpr int kExchange = kStage + kTile;
-    static constexpr int kBarriers = kExchange + 1024;
+    static constexpr int kBarriers = kExchange + 1024 + 512;
     // stage_free, q_full[2], q_empty[2], kv_full[S], kv_empty[S], s_full[2], p_full[2], o_full[2], o_empty[2], staged[2]
     static constexpr int kBarrierCount = 5 + 2 * kPairSlots + 10;
     static constexpr int kTotal = kBarriers + kBarrierCount * 8 + 16;
@@ -242,11 +243,26 @@ __device__ __forceinline__ void put_probabilities(const uint32_t (&raw)[16], uin
         }
     }
 }
+// The upper BITS bits of a float, rounded towards +inf.
+template <int BITS>
+__device__ __forceinline__ uint32_t round_up(float value) {
+    constexpr uint32_t kDropped = (1u << (32 - BITS)) - 1u;
+    const uint32_t bits = __float_as_uint(value);
+    return (bits & 0x80000000u) ? bits & ~kDropped : (bits + kDropped) & ~kDropped;
+}
+// What is added to the scaled scores of a row. (GENERAL: scores that are all -inf are probabilities of zero, not NaN.)
+template <bool GENERAL>
+__device__ __forceinline__ float bias_of(float m_ref) { return GENERAL && m_ref == -INFINITY ? 0.0f : -m_ref; }
+template <bool GENERAL>
+__device__ __forceinline__ float inverse_of(float total) { return GENERAL && !(total > 0.0f) ? 0.0f : 1.0f / total; }
+// Sum_exp: the sum was accumulated against m_ref; re-express it against the true maximum.
+template <bool GENERAL>
+__device__ __forceinline__ float sum_against(float total, float m_ref, float row_max) { return GENERAL && total == 0.0f ? 0.0f : total * exp2f(m_ref - row_max); }
 // Stats of a row whose probabilities were formed against m_ref.
 template <bool GENERAL>
 __device__ __forceinline__ float natural_log_sum(const SdpaUmmaArgs& args, float m_ref, float total) {
     // (rounded once behind the logarithm, as the row-at-a-time kernel's)
-    if constexpr (GENERAL) return fmaf(m_ref, args.to_natural[0], fmaf(m_ref, args.to_natural[1], logf(total)));
+    if constexpr (GENERAL) return m_ref == -INFINITY ? m_ref : fmaf(m_ref, args.to_natural[0], fmaf(m_ref, args.to_natural[1], logf(total)));
     return 0.6931471805599453f * (m_ref + log2f(total));
 }
 // Columns that put_probabilities() fills for 16 keys.
@@ -620,6 +636,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         const float scale = args.scale_log2;
         const int pair_barrier = 1 + x * 4 + quadrant;  // the 64 threads that share these 32 rows
         uint16_t* exchange = reinterpret_cast<uint16_t*>(generic_base + Smem::kExchange) + ((x * 4 + quadrant) * 2) * 32;  // [half][lane]
+        uint8_t* exchange_low = generic_base + Smem::kExchange + 1024 + (x * 4 + quadrant) * 64;   // [half][lane]
         float* sum_exchange = reinterpret_cast<float*>(generic_base + Smem::kExchange) + (x * 4 + quadrant) * 32;
         uint32_t n = 0;        // items started
         uint32_t s_count = 0;  // score tiles consumed (parity of s_full)
@@ -675,12 +692,14 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             // arrive at the same value, so each uses the rounded form of its own half too. (One buffer suffices: the next
             // scores of this tile, which precede the next write, need the probabilities of all eight warps, and a warp
             // hands those over after this read.)
-            const uint32_t mine_bits = __float_as_uint(mine);
-            const uint32_t mine_up = (mine_bits & 0x80000000u) ? (mine_bits & 0xffff0000u) : ((mine_bits + 0xffffu) & 0xffff0000u);
+            // (GENERAL: as 24 bits, since against a reference 2^-7 above a maximum of thousands all probabilities would be zero)
+            const uint32_t mine_up = round_up<GENERAL ? 24 : 16>(mine);
             exchange[half * 32 + lane] = static_cast<uint16_t>(mine_up >> 16);
+            if (GENERAL) exchange_low[half * 32 + lane] = static_cast<uint8_t>(mine_up >> 8);
             asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
-            const float other = __uint_as_float(static_cast<uint32_t>(exchange[(half ^ 1) * 32 + lane]) << 16);
-            const float tile_max = fmaxf(__uint_as_float(mine_up), other) * scale;
+            uint32_t other_bits = static_cast<uint32_t>(exchange[(half ^ 1) * 32 + lane]) << 16;
+            if (GENERAL) other_bits |= static_cast<uint32_t>(exchange_low[(half ^ 1) * 32 + lane]) << 8;
+            const float tile_max = fmaxf(__uint_as_float(mine_up), __uint_as_float(other_bits)) * scale;
             // raise the reference only when it would grow by more than the threshold (or on the first tile); the two
             // warps of these rows see the same maxima, so they take the same branches
             if (__any_sync(0xffffffffu, tile_max > m_ref + kRescaleThreshold)) {
@@ -704,7 +723,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             }
             {
                 // (probabilities go over columns whose scores have been read: 8 columns for every 16, or all 16)
-                const uint64_t scale2 = pack2(scale, scale), bias2 = pack2(-m_ref, -m_ref);
+                const uint64_t scale2 = pack2(scale, scale), bias2 = pack2(bias_of<GENERAL>(m_ref), bias_of<GENERAL>(m_ref));
                 uint64_t sums[2] = {0, 0};  // two independent chains of packed partial sums
                 uint32_t raw[4][16];
                 tmem_load_16(scores_at, raw[0]);
@@ -761,14 +780,14 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 const bool inside = ok && q_index < args.seq_q;
                 if (inside && args.row_max != nullptr)
                     args.row_max[b64 * args.max_stride[0] + h64 * args.max_stride[1] + q64 * args.max_stride[2]] = any ? row_raw_max * args.attn_scale : -INFINITY;
-                if (inside && args.row_sum != nullptr)  // the sum was accumulated against m_ref; re-express it against the true maximum
-                    args.row_sum[b64 * args.sum_stride[0] + h64 * args.sum_stride[1] + q64 * args.sum_stride[2]] = any ? total * exp2f(m_ref - row_raw_max * scale) : 0.0f;
+                if (inside && args.row_sum != nullptr)
+                    args.row_sum[b64 * args.sum_stride[0] + h64 * args.sum_stride[1] + q64 * args.sum_stride[2]] = any ? sum_against<GENERAL>(total, m_ref, row_raw_max * scale) : 0.0f;
             }
         }
         // the hand-over words double as the next item's maxima: every read above must precede those writes
         asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
         const bool live = !GENERAL || q_index < item.live_q;
-        const float inverse = live ? 1.0f / total : 0.0f;
+        const float inverse = live ? inverse_of<GENERAL>(total) : 0.0f;
         // the staging tile serves the query tiles in turn: A, B, the next item's A, ...
         {
             const uint32_t turn = 2 * n + x;
@@ -837,13 +856,13 @@ struct DuoSmem {
     static constexpr int kQ = 0;                        // this item's and the next one's
     static constexpr int kRing = 2 * kTile;
     static constexpr int kStage = kRing + kDuoSlots * kSlot;
-    static constexpr int kMaxima = kStage + kTile;      // half-row maxima, bf16 [turn 2][group][quarter][half][lane]
-    static constexpr int kReference = kMaxima + 2048;   // f32 [turn 2][group][half][quarter][lane]
+    static constexpr int kMaxima = kStage + kTile;      // half-row maxima, bf16 (GENERAL: f32) [turn 2][group][quarter][half][lane]
+    static constexpr int kReference = kMaxima + 4096;   // f32 [turn 2][group][half][quarter][lane]
     static constexpr int kSums = kReference + 4096;     // f32 {row sum, its reference, largest dot product} [group][half][row]
     static constexpr int kBarriers = kSums + 3 * 2048;
-    // stage_free, staged, o_empty, sums_ready, sums_free, v_edge, edge_done, (one spare), q_full[2], q_empty[2], kv_full[S],
+    // stage_free, staged, o_empty, sums_ready, sums_free, v_edge, edge_done, q_full[2], q_empty[2], kv_full[S],
     // kv_empty[S], s_full[3], p_full[3], pv_done[3], passed_on[group][half][quarter]
-    static constexpr int kBarrierCount = 12 + 2 * kDuoSlots + 3 * kDuoBuffers + 16;
+    static constexpr int kBarrierCount = 11 + 2 * kDuoSlots + 3 * kDuoBuffers + 16;
     static constexpr int kTotal = kBarriers + kBarrierCount * 8 + 16;
     static constexpr int kDynamic = kTotal + 1024;
 };
@@ -927,14 +946,14 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     const uint32_t bar_base = smem_base + Smem::kBarriers;
     const uint32_t stage_free = bar_base, staged = bar_base + 8, o_empty = bar_base + 16, sums_ready = bar_base + 24, sums_free = bar_base + 32, v_edge = bar_base + 40,
                    edge_done = bar_base + 48;
-    auto q_full = [&](int i) { return bar_base + 8u * (8 + i); };
-    auto q_empty = [&](int i) { return bar_base + 8u * (10 + i); };
-    auto kv_full = [&](int s) { return bar_base + 8u * (12 + s); };
-    auto kv_empty = [&](int s) { return bar_base + 8u * (12 + kDuoSlots + s); };
-    auto s_full = [&](int b) { return bar_base + 8u * (12 + 2 * kDuoSlots + b); };
-    auto p_full = [&](int b) { return bar_base + 8u * (12 + 2 * kDuoSlots + kDuoBuffers + b); };
-    auto pv_done = [&](int b) { return bar_base + 8u * (12 + 2 * kDuoSlots + 2 * kDuoBuffers + b); };
-    auto passed_on = [&](int group, int half, int quarter) { return bar_base + 8u * (12 + 2 * kDuoSlots + 3 * kDuoBuffers + group * 8 + half * 4 + quarter); };
+    auto q_full = [&](int i) { return bar_base + 8u * (7 + i); };
+    auto q_empty = [&](int i) { return bar_base + 8u * (9 + i); };
+    auto kv_full = [&](int s) { return bar_base + 8u * (11 + s); };
+    auto kv_empty = [&](int s) { return bar_base + 8u * (11 + kDuoSlots + s); };
+    auto s_full = [&](int b) { return bar_base + 8u * (11 + 2 * kDuoSlots + b); };
+    auto p_full = [&](int b) { return bar_base + 8u * (11 + 2 * kDuoSlots + kDuoBuffers + b); };
+    auto pv_done = [&](int b) { return bar_base + 8u * (11 + 2 * kDuoSlots + 2 * kDuoBuffers + b); };
+    auto passed_on = [&](int group, int half, int quarter) { return bar_base + 8u * (11 + 2 * kDuoSlots + 3 * kDuoBuffers + group * 8 + half * 4 + quarter); };
     const uint32_t tmem_slot = bar_base + 8u * Smem::kBarrierCount;
     volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(generic_base + Smem::kBarriers + 8 * Smem::kBarrierCount);
     volatile int* edge_slot = reinterpret_cast<volatile int*>(generic_base + Smem::kBarriers + 8 * Smem::kBarrierCount + 4);
@@ -1187,12 +1206,18 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 // serves, and both threads must arrive at the same value. (Two buffers: the other warp may still be reading the
                 // last tile's when this one writes.)
                 const uint32_t turn = mine_done & 1;
-                const uint32_t mine_bits = __float_as_uint(mine);
-                const uint32_t mine_up = (mine_bits & 0x80000000u) ? (mine_bits & 0xffff0000u) : ((mine_bits + 0xffffu) & 0xffff0000u);
-                maxima[turn * 512 + half * 32] = static_cast<uint16_t>(mine_up >> 16);
-                asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
-                const float other = __uint_as_float(static_cast<uint32_t>(maxima[turn * 512 + (half ^ 1) * 32]) << 16);
-                const float tile_max = fmaxf(__uint_as_float(mine_up), other) * scale;
+                float tile_max;
+                if constexpr (GENERAL) {   // (exact: see the kernel above)
+                    float* exact = reinterpret_cast<float*>(generic_base + Smem::kMaxima) + (group * 4 + quarter) * 64 + lane;
+                    exact[turn * 512 + half * 32] = mine;
+                    asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
+                    tile_max = fmaxf(mine, exact[turn * 512 + (half ^ 1) * 32]) * scale;
+                } else {
+                    const uint32_t mine_up = round_up<16>(mine);
+                    maxima[turn * 512 + half * 32] = static_cast<uint16_t>(mine_up >> 16);
+                    asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
+                    tile_max = fmaxf(__uint_as_float(mine_up), __uint_as_float(static_cast<uint32_t>(maxima[turn * 512 + (half ^ 1) * 32]) << 16)) * scale;
+                }
                 float before = t > 0 ? passed(t - 1) : -INFINITY;   // (at an item's start for the order alone: the other group has taken what this one passed on last)
                 if (j == 0) before = -INFINITY;
                 // raise the reference only when it would grow by more than the threshold (or on the first tile)
@@ -1208,7 +1233,7 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 uint64_t sums[2] = {0, 0};
                 if (!empty) {
                     // (probabilities go over columns whose scores have been read: 8 columns for every 16, or all 16)
-                    const uint64_t bias2 = pack2(-m_ref, -m_ref);
+                    const uint64_t bias2 = pack2(bias_of<GENERAL>(m_ref), bias_of<GENERAL>(m_ref));
                     uint32_t raw[4][16];
                     tmem_load_16(tmem_s, raw[0]);
 #pragma unroll
@@ -1299,13 +1324,13 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                     const int64_t b64 = item.batch, h64 = item.head, q64 = q_index;
                     if (args.row_max != nullptr)
                         args.row_max[b64 * args.max_stride[0] + h64 * args.max_stride[1] + q64 * args.max_stride[2]] = live ? row_raw_max * args.attn_scale : -INFINITY;
-                    if (args.row_sum != nullptr)  // the sum was accumulated against m_ref; re-express it against the true maximum
-                        args.row_sum[b64 * args.sum_stride[0] + h64 * args.sum_stride[1] + q64 * args.sum_stride[2]] = live ? total * exp2f(m_ref - row_raw_max * scale) : 0.0f;
+                    if (args.row_sum != nullptr)
+                        args.row_sum[b64 * args.sum_stride[0] + h64 * args.sum_stride[1] + q64 * args.sum_stride[2]] = live ? sum_against<GENERAL>(total, m_ref, row_raw_max * scale) : 0.0f;
                     if (args.stats != nullptr)
                         args.stats[b64 * args.stats_batch_stride + h64 * args.stats_head_stride + q64 * args.stats_row_stride] =
                             live ? natural_log_sum<GENERAL>(args, m_ref, total) : -INFINITY;
                 }
-                const float inverse = live ? 1.0f / total : 0.0f;
+                const float inverse = live ? inverse_of<GENERAL>(total) : 0.0f;
                 if (ok) ok = mbar_wait(stage_free, (n & 1) ^ 1, 256);
                 if (ok) ok = mbar_wait(pv_done(last % kDuoBuffers), (last / kDuoBuffers) & 1, 257);
                 tc_fence_after();

@@ -6,7 +6,8 @@ Tolerances of check(): a probability within u of its value (u = 2^-8 for bf16, 2
 2^-13, so O is off by at most (u + 2^-12) sum p |v| before it is rounded once by u; subnormal f16 probabilities (up to 2^-24 of
 the largest) add 2^-24 sum |v|. Stats carry the exponentials' error and f32 scores. `fine` is what forms that are not whole bf16
 tiles of 128 channels promise: probabilities of 16 bits or more (2^-17), exponentials within 2^-22 and scores whose f32 sums over 128
-channels are off by at most 2^-20 sum |q k| (below 2^-16 here), 2^-14 sum p |v| in all, and Stats within 2^-16."""
+channels are off by at most 2^-20 sum |q k| (below 2^-16 here), 2^-14 sum p |v| in all, and Stats within 2^-16 (both times `amplify`, the
+factor by which Q and so the scores' errors are larger)."""
 import pytest
 
 from deepforge_b200 import dfgpu, graphs, runtime
@@ -37,13 +38,14 @@ def attention(q, k, v, scale, causal, len_q=None, len_kv=None):
     return p @ v, p @ v.abs(), v.abs().sum(-2, keepdim=True), stats
 
 
-def check(b, h, hkv, sq, skv, d, io, causal, padding=None, scale=None, strided=False, seed=3, fine=False):
+def check(b, h, hkv, sq, skv, d, io, causal, padding=None, scale=None, strided=False, seed=3, fine=False, amplify=1.0):
     g = torch.Generator(device="cuda").manual_seed(seed)
     scale = d ** -0.5 if scale is None else scale
     def operand(heads, length):
         x = torch.randn(b, length, heads, d, device="cuda", generator=g).to(TORCH[io])   # [B, S, H, D]
         return x.transpose(1, 2) if strided else x.transpose(1, 2).contiguous()
     q, k, v = operand(h, sq), operand(hkv, skv), operand(hkv, skv)
+    q = q * amplify
     o = torch.full_like(q, float("nan"))
     stats = torch.full((b, h, sq), float("nan"), device="cuda")
     tensors = [graphs.tensor(uid, name, list(x.shape), io, list(x.stride())) for uid, name, x in ((1, "Q", q), (2, "K", k), (3, "V", v), (4, "O", o))]
@@ -64,11 +66,11 @@ def check(b, h, hkv, sq, skv, d, io, causal, padding=None, scale=None, strided=F
     assert dfgpu.device_status() == 0
     want, weight, every, want_stats = attention(q, k, v, scale, causal, len_q, len_kv)
     u = ROUNDING[io]
-    bound = (2.0 ** -14 if fine else u + 2.0 ** -12) * weight + u * want.abs() + (2.0 ** -24 * every if io == "HALF" else 0.0) + 1e-30
+    bound = (amplify * 2.0 ** -14 if fine else u + 2.0 ** -12) * weight + u * want.abs() + (2.0 ** -24 * every if io == "HALF" else 0.0) + 1e-30
     error = (o.double() - want).abs()
     assert bool(torch.all(error <= bound)), float((error / bound).nan_to_num(1e9).max())
     dead = torch.isinf(want_stats)
-    assert bool(torch.all(torch.isneginf(stats[dead]))) and bool(torch.all((stats.double() - want_stats)[~dead].abs() <= (2.0 ** -16 if fine else 1e-3)))
+    assert bool(torch.all(torch.isneginf(stats[dead]))) and bool(torch.all((stats.double() - want_stats)[~dead].abs() <= (amplify * 2.0 ** -16 if fine else 1e-3)))
 
 
 @pytest.mark.parametrize("io,d", [("BFLOAT16", 128), ("HALF", 128), ("BFLOAT16", 64), ("HALF", 64)])
@@ -119,3 +121,31 @@ def test_padded_and_strided_probabilities_as_accurate_as_f32_ones():
     check(2, 4, 2, 256, 256, 128, "BFLOAT16", True, strided=True, fine=True)      # (whole tiles, rows that are not packed)
     check(2, 4, 2, 128, 384, 128, "BFLOAT16", True, fine=True)                    # (whole tiles, more keys than queries under a causal mask)
     check(2, 4, 2, 256, 256, 128, "HALF", False, fine=True)
+
+
+@pytest.mark.parametrize("io,d", [("BFLOAT16", 128), ("HALF", 128), ("BFLOAT16", 64), ("HALF", 64)])
+@pytest.mark.parametrize("b,h,sq,skv,causal", [(3, 1, 17, 17, True), (1, 37, 500, 500, True), (2, 96, 300, 300, False)])
+@pytest.mark.parametrize("amplify", [700.0, 9000.0])
+def test_large_scores(io, d, b, h, sq, skv, causal, amplify):
+    """Scores of thousands, as the row maximum: probabilities are formed against the maximum itself, not a rounded one."""
+    check(b, h, h, sq, skv, d, io, causal, fine=True, amplify=amplify)
+
+
+@pytest.mark.parametrize("h", [1, 90])
+def test_scores_that_are_all_minus_infinity(h):
+    b, s, d = 2, 200, 128
+    q, k, v = (torch.full((b, h, s, d), x, device="cuda", dtype=torch.bfloat16) for x in (1e30, -1e30, 1.0))
+    q[:, :, 1::2] = 0.0   # every other row: scores of zero
+    o = torch.empty_like(q)
+    outs = [torch.empty(b, h, s, 1, device="cuda") for _ in range(3)]
+    tensors = [graphs.tensor(uid, name, [b, h, s, d], "BFLOAT16") for uid, name in ((1, "Q"), (2, "K"), (3, "V"), (4, "O"))]
+    tensors += [graphs.tensor(uid, name, [b, h, s, 1], "FLOAT") for uid, name in ((5, "Stats"), (6, "Max"), (7, "Sum_exp"))]
+    node = graphs.sdpa_node("sdpa", {"Q": 1, "K": 2, "V": 3}, {"O": 4, "Stats": 5, "Max": 6, "Sum_exp": 7}, 0.5, False, True)
+    exe = runtime.compile_graph(graphs.document("infinite", [node], tensors, io="BFLOAT16"))
+    assert exe.steps()[0]["kernel"] == dfgpu.SDPA_UMMA
+    exe.execute({uid: x.data_ptr() for uid, x in enumerate([q, k, v, o] + outs, 1)})
+    torch.cuda.synchronize()
+    assert dfgpu.device_status() == 0
+    stats, largest, total = (x[:, :, 0::2] for x in outs)
+    assert bool(torch.all(o[:, :, 0::2] == 0)) and bool(torch.all(torch.isneginf(stats))) and bool(torch.all(torch.isneginf(largest))) and bool(torch.all(total == 0))
+    assert bool(torch.all(o[:, :, 1::2] == 1)) and bool(torch.all((outs[2][:, :, 1::2] - s).abs() <= 1e-3))
