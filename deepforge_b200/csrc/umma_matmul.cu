@@ -896,8 +896,12 @@ Shape choose_shape(const Problem& p) {
 
 template <int KIND, int CG>
 int launch_kernel(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_c, const TileArgs& args, int grid, int dynamic, cudaStream_t stream, const char* what) {
-    cudaError_t error = cudaFuncSetAttribute(umma_matmul_kernel<KIND, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, dynamic);
-    if (error != cudaSuccess) return fail(kExecutionFailed, "%s: cannot reserve %d bytes of shared memory: %s", what, dynamic, cudaGetErrorString(error));
+    // (the most that any shape takes, and not this one's need: the attribute belongs to the function, and a launch of a larger
+    // shape between this call and the next, on another thread or repeated without it, would be refused)
+    constexpr int kMostDynamic = kSmemBudget + 1024;
+    if (dynamic > kMostDynamic) return fail(kExecutionFailed, "%s: %d bytes of shared memory", what, dynamic);
+    cudaError_t error = cudaFuncSetAttribute(umma_matmul_kernel<KIND, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostDynamic);
+    if (error != cudaSuccess) return fail(kExecutionFailed, "%s: cannot reserve %d bytes of shared memory: %s", what, kMostDynamic, cudaGetErrorString(error));
     const unsigned cluster = CG == 2 ? 2u : (args.splits > 1 ? static_cast<unsigned>(args.splits) : 0u);
     error = launch_chained_cluster(umma_matmul_kernel<KIND, CG>, dim3(static_cast<unsigned>(grid)), dim3(thread_count<KIND>()), cluster, static_cast<size_t>(dynamic), stream,
                                    map_a, map_b, map_c, args);

@@ -1,6 +1,8 @@
 """Repeated execution: an Executable keeps the launches of its last few sets of pointers. Results follow the data, the pointers, the
 workspace and the stream of every call, also when more sets rotate than are kept, and a pack that would be refused still is.
 f32 sums of 64 products and three additions: 2^-17 of the magnitudes."""
+import threading
+
 import pytest
 
 from deepforge_b200 import dfgpu, graphs, runtime
@@ -80,3 +82,71 @@ def test_other_streams_and_refusals():
     exe.execute(pack, one.workspace.data_ptr())
     torch.cuda.synchronize()
     one.check()
+
+
+class Linear:
+    """bf16 A [m, k] B [k, n] chained through any number of further square matrices."""
+    def __init__(self, m, k, sizes):
+        g = torch.Generator(device="cuda").manual_seed(m)
+        tensors, nodes, last, width = [graphs.tensor(1, "A", [m, k], "BFLOAT16")], [], 1, k
+        self.pack = {1: torch.randn(m, k, device="cuda", generator=g).bfloat16()}
+        self.want = self.pack[1].double()
+        for i, n in enumerate(sizes):
+            weight = (torch.randn(width, n, device="cuda", generator=g) * width ** -0.5).bfloat16()
+            tensors += [graphs.tensor(10 + i, f"B{i}", [width, n], "BFLOAT16"), graphs.tensor(20 + i, f"C{i}", [m, n], "BFLOAT16")]
+            nodes.append(graphs.matmul_node(f"matmul{i}", last, 10 + i, 20 + i))
+            self.pack[10 + i], self.pack[20 + i] = weight, torch.empty(m, n, device="cuda", dtype=torch.bfloat16)
+            self.want = (self.want @ weight.double()).bfloat16().double()
+            last, width = 20 + i, n
+        self.exe = runtime.compile_graph(graphs.document("linear", nodes, tensors, io="BFLOAT16"))
+        assert all(step["kernel"] == dfgpu.MATMUL_UMMA_BF16 for step in self.exe.steps())
+        self.out = self.pack[last]
+
+    def call(self, stream=None):
+        pack = {uid: x.data_ptr() for uid, x in self.pack.items()}
+        if stream is None:
+            self.exe.execute(pack)
+        else:
+            self.exe.execute_on(stream.cuda_stream, pack)
+
+    def check(self):
+        torch.cuda.synchronize()
+        # (values of about 1 rounded to bf16 after each product; a rounding that falls the other way early on moves later ones)
+        assert bool(torch.all((self.out.double() - self.want).abs() <= 2.0 ** -5 * (1 + self.want.abs())))
+
+
+def test_shapes_that_share_a_kernel_and_need_different_shared_memory():
+    tall, single = Linear(64, 4096, [4096]), Linear(1, 4096, [4096])   # (222512 and 155952 bytes)
+    for _ in range(3):
+        tall.call()
+    single.call()
+    for one in (tall, single, tall):
+        one.out.zero_()
+        one.call()
+        one.check()
+    both = Linear(64, 4096, [4096, 192, 4096])
+    for _ in range(4):
+        both.out.zero_()
+        both.call()
+        both.check()
+
+
+def test_shapes_that_share_a_kernel_on_two_threads():
+    pairs = [(Linear(64, 4096, [4096]), torch.cuda.Stream()), (Linear(1, 4096, [4096]), torch.cuda.Stream())]
+    torch.cuda.synchronize()
+    failures = []
+
+    def work(one, stream):
+        try:
+            for _ in range(300):
+                one.call(stream)
+        except Exception as error:
+            failures.append(error)
+    threads = [threading.Thread(target=work, args=pair) for pair in pairs]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    assert not failures
+    for one, _ in pairs:
+        one.check()
