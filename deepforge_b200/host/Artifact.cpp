@@ -604,7 +604,8 @@ Status load_artifact_executable(std::span<std::uint8_t const> input, std::unique
     if (parsed.kernel_abi_version != dfgpu_abi_version())
         return Status::failure(ErrorCode::kInvalidValue, "artifact", "built against kernel ABI " + std::to_string(parsed.kernel_abi_version) + ", this library is ABI " +
                                                                          std::to_string(dfgpu_abi_version()) + ": recompile the graph");
-    for (auto const& step : parsed.plan.steps) {
+    for (std::size_t index = 0; index < parsed.plan.steps.size(); ++index) {
+        auto const& step = parsed.plan.steps[index];
         KernelStep probe = step;
         std::int64_t scratch = 0;
         if ((status = query_kernel_step(probe, scratch)).is_bad())
@@ -612,7 +613,13 @@ Status load_artifact_executable(std::span<std::uint8_t const> input, std::unique
         if (probe.kernel != step.kernel || probe.launches != step.launches)
             return Status::failure(ErrorCode::kInvalidValue, "artifact", "launch '" + step.label + "' resolves to another kernel in this library: recompile the graph");
         if (scratch > 0) {
-            if (step.scratch.kind != TensorBinding::Kind::kWorkspace || step.scratch.offset + static_cast<std::uint64_t>(scratch) > parsed.workspace.size_bytes)
+            // (its own allocation, not the workspace's end: a kernel that has come to need more than the plan gave it would write over what lies behind)
+            std::uint64_t held = 0;
+            if (step.scratch.kind == TensorBinding::Kind::kWorkspace)
+                for (auto const& allocation : parsed.workspace.allocations)
+                    if (allocation.name == "scratch." + std::to_string(index) && allocation.offset == step.scratch.offset && allocation.live_start <= index && index <= allocation.live_end)
+                        held = allocation.size_bytes;
+            if (static_cast<std::uint64_t>(scratch) > held)
                 return Status::failure(ErrorCode::kInvalidValue, "artifact", "launch '" + step.label + "' needs " + std::to_string(scratch) + " bytes of scratch that the workspace plan does not hold");
         }
     }

@@ -169,6 +169,22 @@ def test_plan_fields_are_validated_against_the_kernel_library():
     assert code_of(_patched(data, params_at, "<i", 77)) == PARSE_ERROR             # first tensor's data type
 
 
+def test_scratch_must_fit_its_own_allocation():
+    """A plan from a library whose kernel needed less scratch: another tensor lies where this one's would write."""
+    n = 2048
+    tensors = [graphs.tensor(1, "A", [n, n]), graphs.tensor(2, "B", [n, n]), graphs.tensor(3, "P", [n, n], virtual=True), graphs.tensor(4, "C", [n, n])]
+    nodes = [graphs.matmul_node("matmul", 1, 2, 3), graphs.pointwise_node("tanh", "TANH_FWD", 3, 4)]
+    exe = runtime.compile_graph(graphs.document("scratch", nodes, tensors))
+    data = exe.serialize()
+    name = b"scratch.0"
+    at = data.rindex(name) + len(name)   # u64 offset, size, alignment, live_start, live_end
+    offset, size = struct.unpack_from("<QQ", data, at)
+    assert size > 1 << 20 and offset + size < exe.workspace_size   # (P lies behind it)
+    assert code_of(_patched(data, at + 8, "<Q", size)) == 0
+    assert code_of(_patched(data, at + 8, "<Q", size - 4096)) == INVALID_VALUE
+    assert code_of(_patched(data, at + 24, "<Q", 1)) in (PARSE_ERROR, INVALID_VALUE)   # (not alive while its launch runs)
+
+
 def test_bindings_must_stay_inside_arguments_and_workspace():
     exe = runtime.compile_graph(DOCS["c2"])
     data = exe.serialize()
