@@ -286,6 +286,7 @@ bsq_row32_kernel(const void* __restrict__ x, uint8_t* __restrict__ y, uint8_t* _
     constexpr int kChunks = 4;
     chain_release();
     chain_wait();
+    x = after_chain(x);
     const int64_t total = rows * cols;
     const int64_t tile0 = static_cast<int64_t>(blockIdx.x) * (256 * 8 * kChunks);
     float v[kChunks][8];
@@ -401,6 +402,7 @@ bsq_col32_kernel(const void* __restrict__ x, uint8_t* __restrict__ y, uint8_t* _
     __shared__ uint32_t partial[4][VEC][32];
     chain_release();
     chain_wait();
+    x = after_chain(x);
     const int lane = threadIdx.x & 31, group = threadIdx.x >> 5;
     const int64_t column = (static_cast<int64_t>(blockIdx.x) * 32 + lane) * VEC;
     const bool live = column < n_extent;
@@ -709,7 +711,8 @@ bsq_tile_bf16_kernel(const BsqTask first, const BsqTask second) {
     chain_release();
     chain_wait();
     const bool in_first = blockIdx.x < first.tiles;
-    const BsqTask task = in_first ? first : second;
+    BsqTask task = in_first ? first : second;
+    task.x = after_chain(task.x);
     const uint32_t tile = in_first ? blockIdx.x : blockIdx.x - first.tiles;
     if (task.column_form) encode_column_tile(task, tile);
     else encode_row_tile(task, tile);

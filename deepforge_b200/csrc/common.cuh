@@ -87,6 +87,8 @@ __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait
 // The pointer again, but known only from here on: a load through a const __restrict__ pointer counts as independent of
 // memory barriers, so only a data dependence keeps the compiler from moving it above the wait. The address passes through
 // as a global one: a pointer of unknown space would make generic loads of what were global ones (22 % on the CUDA-core MATMUL).
+// The same holds for __ldg() through any pointer. Pointers that stay in a struct of arguments are read by plain loads instead, which
+// the wait's "memory" does hold back.
 template <typename T>
 __device__ __forceinline__ T* after_chain(T* pointer) {
     size_t address = __cvta_generic_to_global(pointer);

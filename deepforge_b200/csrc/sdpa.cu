@@ -233,7 +233,7 @@ sdpa_rowwise_kernel(SdpaArgs a, int64_t rows) {
                     (reinterpret_cast<uintptr_t>(a.k_data) & 15u) == 0) {
                     const uint4* p = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(a.k_data) + offset);
                     for (int d = 0; d < dqk; d += 8) {
-                        uint4 raw = __ldg(p + (d >> 3));
+                        uint4 raw = p[d >> 3];
                         uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
@@ -379,8 +379,8 @@ sdpa_paged_decode_kernel(SdpaArgs a, float* __restrict__ partial, int max_chunks
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         const uint16_t* qp = static_cast<const uint16_t*>(a.q_data) + off4(a.q, ib, hkv * G + g, 0, part * 16);
-        uint4 r0 = __ldg(reinterpret_cast<const uint4*>(qp));
-        uint4 r1 = __ldg(reinterpret_cast<const uint4*>(qp) + 1);
+        uint4 r0 = reinterpret_cast<const uint4*>(qp)[0];
+        uint4 r1 = reinterpret_cast<const uint4*>(qp)[1];
         float lo8[8], hi8[8];
         unpack8(r0, lo8);
         unpack8(r1, hi8);
@@ -401,7 +401,7 @@ sdpa_paged_decode_kernel(SdpaArgs a, float* __restrict__ partial, int max_chunks
         for (int g = 0; g < G; ++g) dot[g] = 0.0f;
         if (in_range && base >= 0) {
             const uint4* kp = reinterpret_cast<const uint4*>(kdata + base + (ikv % block) * a.k.stride[2] + part * 16);
-            uint4 r0 = __ldg(kp), r1 = __ldg(kp + 1);
+            uint4 r0 = kp[0], r1 = kp[1];
             float kv[16];
             {
                 float lo8[8], hi8[8];
@@ -463,7 +463,7 @@ sdpa_paged_decode_kernel(SdpaArgs a, float* __restrict__ partial, int max_chunks
         int64_t ikv = chunk_begin + token;
         int64_t base = page_base_v[token / block];
         if (ikv >= lo && ikv < hi && base >= 0) {
-            uint4 raw = __ldg(reinterpret_cast<const uint4*>(vdata + base + (ikv % block) * a.v.stride[2] + column));
+            uint4 raw = *reinterpret_cast<const uint4*>(vdata + base + (ikv % block) * a.v.stride[2] + column);
             float vv[8];
             unpack8(raw, vv);
 #pragma unroll

@@ -216,7 +216,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                             const uint4* p = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(args.epi_data[e]) + base);
 #pragma unroll
                             for (int j = 0; j < 4; ++j) {
-                                const uint4 q = __ldg(p + j);
+                                const uint4 q = p[j];
                                 const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
                                 for (int t = 0; t < 4; ++t) {
@@ -228,7 +228,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                             const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(args.epi_data[e]) + base);
 #pragma unroll
                             for (int j = 0; j < 8; ++j) {
-                                const float4 q = __ldg(p + j);
+                                const float4 q = p[j];
                                 v[4 * j] = __fadd_rn(v[4 * j], q.x);
                                 v[4 * j + 1] = __fadd_rn(v[4 * j + 1], q.y);
                                 v[4 * j + 2] = __fadd_rn(v[4 * j + 2], q.z);

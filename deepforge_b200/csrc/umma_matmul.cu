@@ -181,7 +181,7 @@ __device__ __forceinline__ void add_operand(float (&v)[COUNT], const void* data,
             const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(data) + first);
 #pragma unroll
             for (int j = 0; j < COUNT / 4; ++j) {
-                const float4 q = __ldg(p + j);
+                const float4 q = p[j];
                 v[4 * j] = __fadd_rn(v[4 * j], q.x);
                 v[4 * j + 1] = __fadd_rn(v[4 * j + 1], q.y);
                 v[4 * j + 2] = __fadd_rn(v[4 * j + 2], q.z);
@@ -191,7 +191,7 @@ __device__ __forceinline__ void add_operand(float (&v)[COUNT], const void* data,
             const uint2* p = reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(data) + first);
 #pragma unroll
             for (int j = 0; j < COUNT / 4; ++j) {
-                const uint2 q = __ldg(p + j);
+                const uint2 q = p[j];
                 float f[4];
                 widen_pair(q.x, dtype, f[0], f[1]);
                 widen_pair(q.y, dtype, f[2], f[3]);
@@ -356,14 +356,14 @@ __device__ __forceinline__ void load_scales(const TileArgs& args, int row0, int 
     if (args.sfa_words) {
 #pragma unroll
         for (int g = 0; g < 4; ++g)
-            raw.a[g] = __ldg(reinterpret_cast<const uint32_t*>(args.sfa + min(row0 + g * 32 + lane, args.m_total - 1) * args.sfa_ld + first));
+            raw.a[g] = *reinterpret_cast<const uint32_t*>(args.sfa + min(row0 + g * 32 + lane, args.m_total - 1) * args.sfa_ld + first);
     } else {
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
             const uint8_t* p = args.sfa + min(row0 + g * 32 + lane, args.m_total - 1) * args.sfa_ld;
-            raw.a[g] = __ldg(p + first);
+            raw.a[g] = p[first];
 #pragma unroll
-            for (int j = 1; j < 4; ++j) raw.a_more[g][j - 1] = __ldg(p + min(first + j, last));
+            for (int j = 1; j < 4; ++j) raw.a_more[g][j - 1] = p[min(first + j, last)];
         }
     }
     const uint8_t* base[4];
@@ -376,7 +376,7 @@ __device__ __forceinline__ void load_scales(const TileArgs& args, int row0, int 
         for (int g = 0; g < 4; ++g) {
             const int col = min(col0 + c * 128 + g * 32 + lane, args.n_total - 1);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) raw.b[c][g][j] = __ldg(base[j] + col);
+            for (int j = 0; j < 4; ++j) raw.b[c][g][j] = base[j][col];
         }
     }
 }

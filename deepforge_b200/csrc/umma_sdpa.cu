@@ -294,8 +294,8 @@ __device__ __forceinline__ PairItem pair_item(const SdpaUmmaArgs& args, int bh, 
     item.kv_len = args.seq_kv;
     item.live_q = args.seq_q;
     if (GENERAL && args.len_q != nullptr) {
-        const int len_kv = __ldg(args.len_kv + item.batch * args.len_kv_stride);
-        item.live_q = len_kv > 0 ? min(item.live_q, __ldg(args.len_q + item.batch * args.len_q_stride)) : 0;
+        const int len_kv = args.len_kv[item.batch * args.len_kv_stride];
+        item.live_q = len_kv > 0 ? min(item.live_q, args.len_q[item.batch * args.len_q_stride]) : 0;
         item.kv_len = max(1, min(item.kv_len, len_kv));
     }
     const int kv_tiles = (item.kv_len + kKeys - 1) / kKeys;
