@@ -93,7 +93,8 @@ __device__ __forceinline__ uint32_t address_in(uint32_t own_address, uint32_t ra
     return remote;
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_address) {
-    // (nothing but tensor memory is handed over, which the tcgen05 fences order; released to the cluster, it would wait for all stores)
+    // (tensor memory is handed over, which the tcgen05 fences order, or block scales behind a proxy fence: see the scale loaders; released to
+    // the cluster, it would wait for all stores)
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
 }
 __device__ __forceinline__ float4 load_from_rank(uint32_t cluster_address) {
@@ -287,47 +288,10 @@ __device__ __forceinline__ void store_four(const TileArgs& args, const float (&v
         if (i < live) store_from_f32(args.out, args.out_dtype, at + i, v[i]);
 }
 
-// A wait whose phase may be completed by the other CTA's threads: acquires at cluster scope. Bounded like mbar_wait().
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    return done != 0;
-}
-__device__ __noinline__ bool mbar_wait_cluster_slow(uint32_t bar, uint32_t parity, int code) {
-    const uint64_t start = global_timer_ns();
-    for (;;) {
-        for (int spin = 0; spin < 128; ++spin)
-            if (mbar_try_wait_cluster(bar, parity)) return true;
-        if (global_timer_ns() - start > 2000000000ull) {
-            atomicCAS(&g_device_status, 0, code);
-            return false;
-        }
-    }
-}
-__device__ __forceinline__ bool mbar_test_wait_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    return done != 0;
-}
 template <bool CLUSTER>
 __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, int code) {
-    if constexpr (CLUSTER) {
-        if (__all_sync(0xffffffffu, mbar_test_wait_cluster(bar, parity))) return true;
-#pragma unroll 1
-        for (int spin = 0; spin < 64; ++spin)
-            if (__all_sync(0xffffffffu, mbar_try_wait_cluster(bar, parity))) return true;
-        return __all_sync(0xffffffffu, mbar_wait_cluster_slow(bar, parity, code)) != 0;
-    } else {
-        return mbar_wait_warp(bar, parity, code);
-    }
+    if constexpr (CLUSTER) return mbar_wait_warp_cluster(bar, parity, code);
+    else return mbar_wait_warp(bar, parity, code);
 }
 
 // kPieces: 32 columns of the products of the lower pieces onto those of the leading ones.
@@ -722,7 +686,10 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             fence_async_shared();
             __syncwarp();
             if (leader) {
-                if (CG == 2) mbar_arrive_cluster(address_in(full_bar(slot), 0));   // (CTA 0's product reads both CTAs' scales)
+                // CTA 0's products read both CTAs' scales, each from its CTA's own shared memory and by the asynchronous proxy, to which
+                // fence.proxy.async has made every lane's stores visible before the warp met: no thread of CTA 0 reads them, so there is
+                // nothing that a release to the cluster would order besides (it waits for its round trip, 89 -> 100 us at 4096^3)
+                if (CG == 2) mbar_arrive_cluster(address_in(full_bar(slot), 0));
                 else mbar_arrive(full_bar(slot));
             }
         }

@@ -89,6 +89,47 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, in
         if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
     return __all_sync(0xffffffffu, mbar_wait_slow(bar, parity, code)) != 0;
 }
+// A wait for what another CTA's threads have written to shared memory: acquires at cluster scope, as mbar_arrive_cluster_release()
+// releases. Bounded like mbar_wait().
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    return done != 0;
+}
+__device__ __noinline__ bool mbar_wait_cluster_slow(uint32_t bar, uint32_t parity, int code) {
+    const uint64_t start = global_timer_ns();
+    for (;;) {
+        for (int spin = 0; spin < 128; ++spin)
+            if (mbar_try_wait_cluster(bar, parity)) return true;
+        if (global_timer_ns() - start > 2000000000ull) {
+            atomicCAS(&g_device_status, 0, code);
+            return false;
+        }
+    }
+}
+__device__ __forceinline__ bool mbar_test_wait_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    return done != 0;
+}
+__device__ __forceinline__ bool mbar_wait_warp_cluster(uint32_t bar, uint32_t parity, int code) {
+    if (__all_sync(0xffffffffu, mbar_test_wait_cluster(bar, parity))) return true;
+#pragma unroll 1
+    for (int spin = 0; spin < 64; ++spin)
+        if (__all_sync(0xffffffffu, mbar_try_wait_cluster(bar, parity))) return true;
+    return __all_sync(0xffffffffu, mbar_wait_cluster_slow(bar, parity, code)) != 0;
+}
+__device__ __forceinline__ void mbar_arrive_cluster_release(uint32_t cluster_address) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
+}
 __device__ __forceinline__ bool elect_one() {
     uint32_t elected;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));

@@ -881,9 +881,9 @@ __device__ __forceinline__ uint32_t address_in_first(uint32_t own_address) {
     return remote;
 }
 __device__ __forceinline__ void arrive_in_cluster(uint32_t cluster_address) {
-    // (of this CTA's scope, as is the wait: what the waiter's products read is tensor memory, ordered by the tcgen05 fences, and shared
-    // memory behind a proxy fence. Released to the cluster, the arrival waits for every store on its way, and a wait that
-    // acquires from the cluster takes 250 clocks even when it is over at once.)
+    // (for hand-overs of tensor memory alone, ordered by the tcgen05 fences. Released to the cluster, the arrival waits for every store
+    // on its way, and a wait that acquires from the cluster takes 250 clocks even when it is over at once: only the tile whose V rows
+    // are cleared in shared memory is handed over that way.)
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
 }
 __device__ __forceinline__ void commit_to_both(uint32_t bar) {
@@ -1097,7 +1097,11 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 const int b = static_cast<int>(p.t % kDuoBuffers);
                 if (p.j == 0) ok = mbar_wait_warp(o_empty, (p.n & 1) ^ 1, 246);
                 if (ok) ok = mbar_wait_warp(kv_full(slot), phase, 247);
-                if (ok) ok = mbar_wait_warp(p_full(b), (p.t / kDuoBuffers) & 1, 248);
+                if (GENERAL && p.last() && clears_v(args, p.item)) {   // (V rows that both CTAs' warps have cleared)
+                    if (ok) ok = mbar_wait_warp_cluster(p_full(b), (p.t / kDuoBuffers) & 1, 248);
+                } else {
+                    if (ok) ok = mbar_wait_warp(p_full(b), (p.t / kDuoBuffers) & 1, 248);
+                }
                 tc_fence_after();
                 if (leader && ok) {
                     const uint32_t v_lo = smem_desc_lo(smem_base + Smem::kRing + slot * Smem::kSlot, kHalfBytes), p_tmem = tmem_u + b * 128;
@@ -1268,7 +1272,8 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                         tmem_store_16(tmem_o + c * 16, acc);
                     }
                 }
-                if (GENERAL && half == 0 && j + 1 == item.tiles && clears_v(args, item)) {
+                const bool cleared = GENERAL && half == 0 && j + 1 == item.tiles && clears_v(args, item);
+                if (cleared) {
                     // V rows past the batch's length are not this sequence's: this CTA's channels of them, a row per thread
                     if (ok) ok = mbar_wait(v_edge, edges & 1, 253);
                     if (j * kKeys + row >= item.kv_len) {
@@ -1283,7 +1288,10 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 tmem_store_wait();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) arrive_in_cluster(p_full_first + 8u * b);
+                if (lane == 0) {
+                    if (cleared) mbar_arrive_cluster_release(p_full_first + 8u * b);
+                    else arrive_in_cluster(p_full_first + 8u * b);
+                }
             }
             const uint32_t last = t0 + item.tiles - 1;
             if (GENERAL && clears_v(args, item)) {
