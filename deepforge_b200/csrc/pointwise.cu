@@ -3,7 +3,7 @@
 //
 // Every mode of the reference's pointwise_result (lib/Compiler/FoundationalGraph.cpp:2581-2955) goes through
 // pointwise_value below: the same expression, one separately rounded f32 operation per step, with CUDA's full-precision
-// math functions where the result is stored as f32 (see Math for the 16-bit types). Dense tensors of one storage type take the kernel of four
+// math functions (see sixteen_bit_activation() for dense 16-bit tensors). Dense tensors of one storage type take the kernel of four
 // values per load, also where an operand is broadcast along the leading or the trailing axes (a bias, a mask by rows, a
 // scalar); anything else (gaps, other broadcasts, mixed storage types, three inputs, GEN_INDEX) one element per thread,
 // where ADD / MUL / SUB / RELU_FWD / IDENTITY keep a kernel with nothing else in it.
@@ -44,63 +44,128 @@ __host__ __device__ constexpr int input_count(int mode) {
 
 inline bool simple_mode(int mode) { return mode >= DFGPU_PW_ADD && mode <= DFGPU_PW_SUB; }
 
-// The functions of the math library. EXACT: CUDA's full-precision ones, for results stored as f32. Otherwise (results rounded
-// to 8 or 11 significant bits) forms within a few 2^-22 relative, a thousandth of that rounding, because the bytes are half and the
-// instructions set the pace: GELU_BWD on 33.5 M bf16 values is 60 instructions a value with erff and expf, 55.8 us against
-// 30.7 for its bytes.
-// The approximate instructions flush subnormals, which a 16-bit result inside one of these formulas cannot show (EXP itself
-// keeps __expf).
-__device__ __forceinline__ float quick_exp(float v) {
-    float e;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(v * 1.4426950408889634f));
-    return e;
-}
-__device__ __forceinline__ float quick_reciprocal(float v) {
+// 1 / (1 + exp(-v)) (FoundationalGraph.cpp:2569-2579)
+__device__ __forceinline__ float sigmoid_value(float v) { return __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-v))); }
+
+// ---- activations whose result is rounded to 16 bits ----------------------------------------------------------------
+// With erff, tanhf and divisions the instructions set the pace instead of the bytes (GELU_BWD on 33.5 M bf16 values: 55.8 us
+// against 30.7 for its bytes). The forms here are one expf and one reciprocal each, arranged so that nothing cancels: errors of a
+// few 2^-23 relative over the whole range, tails and zeros included, subnormal results kept. Against the full-precision
+// formulas every mode's largest error over all 16-bit inputs, in units of the result's rounding, is no larger.
+__device__ __forceinline__ float reciprocal_of_one_or_more(float v) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
     return r;
 }
-template <bool EXACT>
-struct Math {
-    static __device__ __forceinline__ float exp(float v) { return EXACT ? expf(v) : __expf(v); }
-    // 1 / (1 + exp(-v)) (FoundationalGraph.cpp:2569-2579)
-    static __device__ __forceinline__ float sigmoid(float v) {
-        if constexpr (EXACT) return __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-v)));
-        return quick_reciprocal(1.0f + quick_exp(-v));
-    }
-    static __device__ __forceinline__ float tanh(float v) {
-        if constexpr (EXACT) return tanhf(v);
-        // 1 - 2 / (1 + e^2v); near zero, where that cancels, the first two terms of the series (4e-8 relative at 0.02)
-        const float far = fmaf(-2.0f, quick_reciprocal(1.0f + quick_exp(2.0f * v)), 1.0f);
-        return fabsf(v) < 0.02f ? v * fmaf(v * v, -0.33333334f, 1.0f) : far;
-    }
-    // 1 - tanh^2
-    static __device__ __forceinline__ float tanh_slope(float v, float t) {
-        if constexpr (EXACT) return __fsub_rn(1.0f, __fmul_rn(t, t));
-        const float e = quick_exp(-2.0f * fabsf(v)), r = quick_reciprocal(1.0f + e);   // (4e / (1 + e)^2 does not cancel)
-        return 4.0f * e * r * r;
-    }
-    // The normal distribution function and exp(-v^2 / 2), which gives it.
-    static __device__ __forceinline__ float normal_cdf(float v, float& bell) {
-        if constexpr (EXACT) {
-            bell = expf(__fmul_rn(-0.5f, __fmul_rn(v, v)));
-            return __fmul_rn(0.5f, __fadd_rn(1.0f, erff(__fmul_rn(v, 0.7071067811865475f))));
+__device__ __forceinline__ float exp2_flushing(float v) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+// s = 1 / (1 + e^-z) and its complement c = 1 - s, both to f32's relative accuracy.
+__device__ __forceinline__ void logistic(float z, float& s, float& c) {
+    const float e = expf(-fabsf(z)), larger = reciprocal_of_one_or_more(1.0f + e), smaller = e * larger;
+    s = z < 0.0f ? smaller : larger;
+    c = z < 0.0f ? larger : smaller;
+}
+// u: the activation's input, x: the gradient of a _BWD mode. False: not one of these modes.
+__device__ __forceinline__ bool sixteen_bit_activation(int mode, float x, float u, const PointwiseScalars& s, float& result) {
+    float p, q;
+    switch (mode) {
+        case DFGPU_PW_SIGMOID_FWD: logistic(u, p, q); result = p; return true;
+        case DFGPU_PW_SIGMOID_BWD: logistic(u, p, q); result = x * (p * q); return true;
+        case DFGPU_PW_SOFTPLUS_BWD: logistic(s.softplus_beta * u, p, q); result = x * p; return true;
+        case DFGPU_PW_SWISH_FWD: logistic(s.swish_beta * u, p, q); result = u * p; return true;
+        case DFGPU_PW_SWISH_BWD: {
+            const float z = s.swish_beta * u;
+            logistic(z, p, q);
+            result = x * fmaf(z, p * q, p);
+            return true;
         }
-        // 1 - erf(z) = (a1 t + ... + a5 t^5) e^-z^2, t = 1 / (1 + p z), z = |v| / sqrt 2, within 1.5e-7 (Abramowitz and Stegun,
-        // Handbook of Mathematical Functions, 7.1.26): half of it is the smaller tail, so the coefficients here are halved.
-        bell = quick_exp(-0.5f * v * v);
-        const float k = quick_reciprocal(fmaf(0.3275911f * 0.70710678f, fabsf(v), 1.0f));
-        const float sum = fmaf(fmaf(fmaf(fmaf(0.5f * 1.061405429f, k, 0.5f * -1.453152027f), k, 0.5f * 1.421413741f), k, 0.5f * -0.284496736f), k, 0.5f * 0.254829592f);
-        const float tail = sum * k * bell;
-        return v >= 0.0f ? 1.0f - tail : tail;
+        case DFGPU_PW_TANH_FWD: {
+            // (1 - e) / (1 + e), e = e^-2|v| (beside 1, e may be flushed); where that cancels, an odd polynomial of least relative error
+            // (4e-8 up to 0.35)
+            const float e = exp2_flushing(-2.8853900817779268f * fabsf(u)), far = copysignf((1.0f - e) * reciprocal_of_one_or_more(1.0f + e), u), square = u * u;
+            const float near = u * fmaf(square, fmaf(square, fmaf(square, -0.0491485f, 0.13299825f), -0.33332663f), 1.0f);
+            result = fabsf(u) < 0.35f ? near : far;
+            return true;
+        }
+        case DFGPU_PW_TANH_BWD: logistic(2.0f * u, p, q); result = x * (4.0f * (p * q)); return true;   // 1 - tanh^2
+        case DFGPU_PW_GELU_APPROX_TANH_FWD: case DFGPU_PW_GELU_APPROX_TANH_BWD: {   // (1 + tanh t) / 2 = logistic(2 t)
+            const float square = u * u, twice = 1.5957691216057308f * fmaf(0.044715f * square, u, u);
+            logistic(twice, p, q);
+            if (mode == DFGPU_PW_GELU_APPROX_TANH_FWD) {
+                result = u * p;
+            } else {   // p + u p', p' = p (1 - p) (2 t)'
+                const float slope = 1.5957691216057308f * fmaf(0.134145f, square, 1.0f);
+                result = x * fmaf(u, slope * (p * q), p);
+            }
+            return true;
+        }
+        default: return false;
     }
-};
+}
+
+// GELU on two values at once: its polynomial makes it the longest, and the FMA pipe takes pairs of f32.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ uint64_t both(float v) { return pack2(v, v); }
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// The upper tail of the normal distribution at |v| over its bell e^(-v^2/2), half of erfc(z) e^(z^2) at z = |v| / sqrt 2, as a
+// polynomial in k = 1 / (1 + 0.27 |v|) without constant term: least relative error up to |v| = 14.6, where the bell ends (2.4e-8;
+// 3.5e-7 with the rounding of its evaluation).
+__device__ __forceinline__ uint64_t tail_over_bell(uint64_t magnitude) {
+    float lo, hi;
+    unpack2(fma2(both(0.27f), magnitude, both(1.0f)), lo, hi);
+    const uint64_t k = pack2(reciprocal_of_one_or_more(lo), reciprocal_of_one_or_more(hi));
+    uint64_t sum = both(0.0289688222f);
+    sum = fma2(sum, k, both(-0.126524672f));
+    sum = fma2(sum, k, both(0.169869289f));
+    sum = fma2(sum, k, both(-0.0693096891f));
+    sum = fma2(sum, k, both(0.107896969f));
+    sum = fma2(sum, k, both(0.0720177665f));
+    sum = fma2(sum, k, both(0.101819173f));
+    sum = fma2(sum, k, both(0.107541606f));
+    sum = fma2(sum, k, both(0.107720733f));
+    return mul2(sum, k);
+}
+template <bool BACKWARD>
+__device__ __forceinline__ void sixteen_bit_gelu(const float* x, const float* u, float* result) {
+    const uint64_t value = pack2(u[0], u[1]), magnitude = pack2(fabsf(u[0]), fabsf(u[1]));
+    float e0, e1;
+    unpack2(mul2(mul2(value, value), both(-0.72134752044448170f)), e0, e1);   // (squares of 16-bit values are exact)
+    asm("ex2.approx.f32 %0, %0;" : "+f"(e0));
+    asm("ex2.approx.f32 %0, %0;" : "+f"(e1));
+    const uint64_t bell = pack2(e0, e1), tail = tail_over_bell(magnitude);
+    // the distribution function, or its derivative's cdf + u pdf: below zero `below`, above it one less that
+    const uint64_t below = BACKWARD ? mul2(bell, fma2(both(-0.3989422804014327f), magnitude, tail)) : mul2(bell, tail);
+    float below0, below1, above0, above1;
+    unpack2(fma2(below, both(1.0f), both(0.0f)), below0, below1);   // (+0.0: the formula's sum is never -0.0)
+    unpack2(fma2(below, both(-1.0f), both(1.0f)), above0, above1);
+    unpack2(mul2(BACKWARD ? pack2(x[0], x[1]) : value, pack2(u[0] >= 0.0f ? above0 : below0, u[1] >= 0.0f ? above1 : below1)), result[0], result[1]);
+}
 
 // x, y, z: IN_0, IN_1, IN_2 (0 where the mode has none). u: the activation's input (IN_1 of a _BWD mode, else IN_0).
 template <bool EXACT>
 __device__ __forceinline__ float pointwise_value(int mode, float x, float y, float z, const PointwiseScalars& s, int64_t position) {
-    using M = Math<EXACT>;
     const float u = (mode >= DFGPU_PW_RELU_BWD && input_count(mode) == 2) ? y : x;
+    if constexpr (!EXACT) {
+        float result;
+        if (sixteen_bit_activation(mode, x, u, s, result)) return result;
+    }
     switch (mode) {
         case DFGPU_PW_ADD: return __fadd_rn(x, y);
         case DFGPU_PW_MUL: return __fmul_rn(x, y);
@@ -113,7 +178,7 @@ __device__ __forceinline__ float pointwise_value(int mode, float x, float y, flo
         case DFGPU_PW_POW: return powf(x, y);
         case DFGPU_PW_SQRT: return __fsqrt_rn(x);
         case DFGPU_PW_RSQRT: return __fdiv_rn(1.0f, __fsqrt_rn(x));
-        case DFGPU_PW_EXP: return M::exp(x);
+        case DFGPU_PW_EXP: return expf(x);
         case DFGPU_PW_LOG: return logf(x);
         case DFGPU_PW_NEG: return -x;
         case DFGPU_PW_ABS: return fabsf(x);
@@ -138,43 +203,54 @@ __device__ __forceinline__ float pointwise_value(int mode, float x, float y, flo
         case DFGPU_PW_CMP_LE: return x <= y ? 1.0f : 0.0f;
         case DFGPU_PW_RELU_FWD: return relu_forward(x, s.relu_lower, s.relu_upper, s.relu_slope);
         case DFGPU_PW_RELU_BWD: return __fmul_rn(x, y < s.relu_lower ? s.relu_slope : (y > s.relu_upper ? 0.0f : 1.0f));
-        case DFGPU_PW_TANH_FWD: return M::tanh(u);
-        case DFGPU_PW_TANH_BWD: return __fmul_rn(x, M::tanh_slope(u, EXACT ? M::tanh(u) : 0.0f));
-        case DFGPU_PW_SIGMOID_FWD: return M::sigmoid(u);
-        case DFGPU_PW_SIGMOID_BWD: { float v = M::sigmoid(u); return __fmul_rn(x, __fmul_rn(v, __fsub_rn(1.0f, v))); }
+        case DFGPU_PW_TANH_FWD: return tanhf(u);
+        case DFGPU_PW_TANH_BWD: { float t = tanhf(u); return __fmul_rn(x, __fsub_rn(1.0f, __fmul_rn(t, t))); }
+        case DFGPU_PW_SIGMOID_FWD: return sigmoid_value(u);
+        case DFGPU_PW_SIGMOID_BWD: { float v = sigmoid_value(u); return __fmul_rn(x, __fmul_rn(v, __fsub_rn(1.0f, v))); }
         case DFGPU_PW_ELU_FWD: { float e = expf(u); return u >= 0.0f ? u : __fmul_rn(s.elu_alpha, __fsub_rn(e, 1.0f)); }
-        case DFGPU_PW_ELU_BWD: { float e = M::exp(u); return __fmul_rn(x, u >= 0.0f ? 1.0f : __fmul_rn(s.elu_alpha, e)); }
+        case DFGPU_PW_ELU_BWD: { float e = expf(u); return __fmul_rn(x, u >= 0.0f ? 1.0f : __fmul_rn(s.elu_alpha, e)); }
         case DFGPU_PW_SOFTPLUS_FWD: {
             float scaled = __fmul_rn(s.softplus_beta, u);
             float logarithm = logf(__fadd_rn(1.0f, expf(-fabsf(scaled))));
             return __fdiv_rn(__fadd_rn(maximum_nan(scaled, 0.0f), logarithm), s.softplus_beta);
         }
-        case DFGPU_PW_SOFTPLUS_BWD: return __fmul_rn(x, M::sigmoid(__fmul_rn(s.softplus_beta, u)));
-        case DFGPU_PW_SWISH_FWD: return __fmul_rn(u, M::sigmoid(__fmul_rn(s.swish_beta, u)));
+        case DFGPU_PW_SOFTPLUS_BWD: return __fmul_rn(x, sigmoid_value(__fmul_rn(s.softplus_beta, u)));
+        case DFGPU_PW_SWISH_FWD: return __fmul_rn(u, sigmoid_value(__fmul_rn(s.swish_beta, u)));
         case DFGPU_PW_SWISH_BWD: {
             float scaled = __fmul_rn(s.swish_beta, u);
-            float v = M::sigmoid(scaled);
+            float v = sigmoid_value(scaled);
             return __fmul_rn(x, __fadd_rn(v, __fmul_rn(scaled, __fmul_rn(v, __fsub_rn(1.0f, v)))));
         }
         case DFGPU_PW_GELU_FWD: case DFGPU_PW_GELU_BWD: {
-            float bell;
-            float cdf = M::normal_cdf(u, bell);
+            float cdf = __fmul_rn(0.5f, __fadd_rn(1.0f, erff(__fmul_rn(u, 0.7071067811865475f))));
             if (mode == DFGPU_PW_GELU_FWD) return __fmul_rn(u, cdf);
-            float density = __fmul_rn(0.3989422804014327f, bell);
+            float density = __fmul_rn(0.3989422804014327f, expf(__fmul_rn(-0.5f, __fmul_rn(u, u))));
             return __fmul_rn(x, __fadd_rn(cdf, __fmul_rn(u, density)));
         }
         case DFGPU_PW_GELU_APPROX_TANH_FWD: case DFGPU_PW_GELU_APPROX_TANH_BWD: {
             float square = __fmul_rn(u, u);
             float cubic = __fmul_rn(square, u);
             float inner = __fmul_rn(0.7978845608028654f, __fadd_rn(u, __fmul_rn(0.044715f, cubic)));
-            float t = M::tanh(inner);
+            float t = tanhf(inner);
             float cdf = __fmul_rn(0.5f, __fadd_rn(1.0f, t));
             if (mode == DFGPU_PW_GELU_APPROX_TANH_FWD) return __fmul_rn(u, cdf);
             float inner_derivative = __fmul_rn(0.7978845608028654f, __fadd_rn(1.0f, __fmul_rn(0.134145f, square)));
-            float tanh_derivative = M::tanh_slope(inner, t);
+            float tanh_derivative = __fsub_rn(1.0f, __fmul_rn(t, t));
             return __fmul_rn(x, __fadd_rn(cdf, __fmul_rn(0.5f, __fmul_rn(u, __fmul_rn(tanh_derivative, inner_derivative)))));
         }
         default: return x;
+    }
+}
+
+// Four neighbouring values of a dense tensor of type T.
+template <typename T, int MODE>
+__device__ __forceinline__ void four_values(const float (&x)[4], const float (&y)[4], const PointwiseScalars& s, float (&r)[4]) {
+    if constexpr (sizeof(T) == 2 && (MODE == DFGPU_PW_GELU_FWD || MODE == DFGPU_PW_GELU_BWD)) {
+#pragma unroll
+        for (int j = 0; j < 4; j += 2) sixteen_bit_gelu<MODE == DFGPU_PW_GELU_BWD>(x + j, (MODE == DFGPU_PW_GELU_BWD ? y : x) + j, r + j);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) r[j] = pointwise_value<sizeof(T) == 4>(MODE, x[j], y[j], 0.0f, s, 0);
     }
 }
 
@@ -304,8 +380,7 @@ __device__ __forceinline__ void packed_body(const void* a, const void* b, void* 
         float x[4], y[4] = {0.0f, 0.0f, 0.0f, 0.0f}, r[4];
         widen(raw_x[u], x);
         if (binary) widen(raw_y[u], y);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) r[j] = pointwise_value<sizeof(T) == 4>(MODE, x[j], y[j], 0.0f, s, 0);
+        four_values<T, MODE>(x, y, s, r);
         store4<T>(out, i, r);
     }
 }
@@ -403,8 +478,7 @@ __device__ __forceinline__ void dense_body(const DenseOperand& a, const DenseOpe
             float x[4], y[4] = {0.0f, 0.0f, 0.0f, 0.0f}, r[4];
             widen_raw<T>(a, raw_x[u], x);
             if (binary) widen_raw<T>(b, raw_y[u], y);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) r[j] = pointwise_value<sizeof(T) == 4>(MODE, x[j], y[j], 0.0f, s, 0);
+            four_values<T, MODE>(x, y, s, r);
             store4<T>(out, first + u * kPackedThreads * 4, r);
         }
         return;
@@ -416,8 +490,7 @@ __device__ __forceinline__ void dense_body(const DenseOperand& a, const DenseOpe
         float x[4], y[4] = {0.0f, 0.0f, 0.0f, 0.0f}, r[4];
         load_dense<T>(a, i, total, x);
         if (binary) load_dense<T>(b, i, total, y);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) r[j] = pointwise_value<sizeof(T) == 4>(MODE, x[j], y[j], 0.0f, s, 0);
+        four_values<T, MODE>(x, y, s, r);
         if (out_vector && i + 4 <= total) {
             store4<T>(out, i, r);
         } else {
