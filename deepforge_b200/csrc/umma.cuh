@@ -42,7 +42,7 @@ int conv_f32_device_status(int* status);
 bool matmul_f32_cluster_supported(const dfgpu_matmul_params& p);
 int launch_matmul_f32_cluster(const dfgpu_matmul_params& p, void* const* tensors, cudaStream_t stream);
 // Channels-last tensors (row-major matrices) whose reduction the kernel walks flat, 64 (tap, channel) pairs a unit. AUTO takes
-// these at any depth: 7 us where the CUDA-core forms take 8 (16 deep) to 30 (100 deep). Their kernel id stays the
+// these from 12 pairs on: 7 us where the CUDA-core forms take 8 (16 deep) to 30 (100 deep). Their kernel id stays the
 // CUDA-core one, whose form still takes what is not aligned for this.
 bool conv_f32_flat(const dfgpu_conv_params& p, void* const* tensors);
 bool matmul_f32_flat(const dfgpu_matmul_params& p, void* const* tensors);

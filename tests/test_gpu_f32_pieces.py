@@ -72,3 +72,22 @@ def test_matmul_with_an_infinity(m, k, n):
     want = np.full((m, n), float(k), np.float32)
     want[1, :], want[:, 7] = np.inf, np.nan
     assert np.array_equal(c.cpu().numpy(), want, equal_nan=True)
+
+
+@pytest.mark.parametrize("depth", [4, 8])
+@pytest.mark.parametrize("conv", [True, False])
+def test_shallow_reductions_are_f32_additions(depth, conv):
+    """A handful of products: one rounding each, in order (a product and a sum in f64, rounded to f32, is that but for double roundings)."""
+    g = torch.Generator(device="cuda").manual_seed(depth)
+    rows, k = 400, 64
+    x, f = torch.randn(rows, depth, device="cuda", generator=g), torch.randn(k, depth, device="cuda", generator=g)
+    y = torch.full((rows, k), float("nan"), device="cuda")
+    if conv:
+        doc = graphs.c1_conv("nhwc", 1, depth, 20, 20, k, 1, 0)
+    else:
+        doc = graphs.document("f32", [graphs.matmul_node("matmul", 1, 2, 3)], [graphs.tensor(1, "A", [rows, depth]), graphs.tensor(2, "B", [depth, k], strides=[1, depth]), graphs.tensor(3, "C", [rows, k])])
+    run(doc, {1: x, 2: f}, {3: y})
+    want = torch.zeros(rows, k, device="cuda")
+    for i in range(depth):
+        want = (x[:, i : i + 1].double() * f[:, i].double() + want.double()).float()
+    assert float((y == want).float().mean()) > 0.999
