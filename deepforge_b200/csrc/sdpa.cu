@@ -534,15 +534,15 @@ sdpa_decode_merge_kernel(SdpaArgs a, const float* __restrict__ partial, int max_
         if (d < count) {
             const float* own = base + (first + d) * kPartialStride + kDecodeD;
             const float m = own[0];
-            const float weight = m == -INFINITY ? 0.0f : expf(m - total_max);
+            const float weight = m == -INFINITY ? -1.0f : expf(m - total_max);   // (an empty chunk's weight is negative: a zero may be a small one's)
             weights[d] = weight;
-            total_sum = fmaf(weight == 0.0f ? 0.0f : own[1], weight, total_sum);
+            if (!(weight < 0.0f)) total_sum = fmaf(own[1], weight, total_sum);
         }
         __syncthreads();
 #pragma unroll 8
         for (int c = 0; c < count; ++c) {
             const float o = base[(first + c) * kPartialStride + d];   // (an empty chunk's is never written: not counted)
-            value = weights[c] == 0.0f ? value : fmaf(o, weights[c], value);
+            value = weights[c] < 0.0f ? value : fmaf(o, weights[c], value);
         }
     }
 #pragma unroll
@@ -550,7 +550,7 @@ sdpa_decode_merge_kernel(SdpaArgs a, const float* __restrict__ partial, int max_
     if (lane == 0) reduce[4 + warp] = total_sum;
     __syncthreads();
     total_sum = reduce[4] + reduce[5] + reduce[6] + reduce[7];
-    float result = total_sum > 0.0f ? value / total_sum : 0.0f;
+    float result = total_sum == 0.0f ? 0.0f : value / total_sum;   // (a NaN sum is a NaN result)
     store_from_f32(a.o_data, a.o.dtype, off4(a.o, ib, ih, 0, d), result);
     if (d == 0) {
         if (a.stats.rank) store_from_f32(a.stats_data, a.stats.dtype, off4(a.stats, ib, ih, 0, 0), total_max + logf(total_sum));
