@@ -762,7 +762,7 @@ __device__ __forceinline__ void widen_e4m3_pair(uint32_t two, float& lo, float& 
 
 enum { kScalePerUnit = 0, kScalePerColumn = 1, kScaleAny = 2 };
 struct BsdShape {
-    uint32_t total, scale_cols;
+    uint32_t total, scale_cols, first_row;   // first_row: of the slice, within its block of rows
     FastDivisor by_cols, by_block_rows, by_block_cols;
     int32_t scale_form;   // one scale for all codes of a unit; one per column, read VEC at a time; anything else
 };
@@ -788,7 +788,7 @@ bsd_packed_kernel(const uint8_t* __restrict__ x, const uint8_t* __restrict__ sca
             codes[u][0] = __ldg(reinterpret_cast<const uint32_t*>(x + i));
         }
         const uint32_t row = fast_divide(i, g.by_cols), col = i - row * g.by_cols.divisor;
-        const uint8_t* scale_row = scale + fast_divide(row, g.by_block_rows) * g.scale_cols;
+        const uint8_t* scale_row = scale + static_cast<int64_t>(fast_divide(g.first_row + row, g.by_block_rows)) * g.scale_cols;
         if (g.scale_form == kScalePerUnit) {
             scales[u][0] = __ldg(scale_row + fast_divide(col, g.by_block_cols));
         } else if (g.scale_form == kScalePerColumn) {
@@ -1074,7 +1074,7 @@ int plan_bsd(const dfgpu_bsd_params& p, BsdPlan& plan) {
         is_packed_row_major(p.scale) && p.y.dim[1] % 16 == 0 && p.y.dim[0] % plan.blocks[0] == 0 &&
         p.y.dim[1] % plan.blocks[1] == 0 && p.scale.dim[0] == p.y.dim[0] / plan.blocks[0] &&
         p.scale.dim[1] == p.y.dim[1] / plan.blocks[1] && (plan.blocks[1] % 16 == 0 || plan.blocks[1] < 16) &&
-        p.y.dim[1] * plan.blocks[0] < (1ll << 31) - (1 << 20))
+        p.y.dim[1] < (1ll << 31) - (1 << 20) && p.y.dim[0] < (1ll << 31))
         kernel = DFGPU_BSD_PACKED;
     if (p.x.dtype != DFGPU_E4M3 || p.scale.dtype != DFGPU_E8M0) kernel = DFGPU_BSD_GENERIC;
     if (p.kernel != DFGPU_BSD_AUTO && p.kernel != kernel) {
@@ -1162,13 +1162,14 @@ extern "C" int dfgpu_block_scale_dequantize(const dfgpu_bsd_params* p, void* con
         shape.by_block_rows = make_fast_divisor(static_cast<uint32_t>(block_rows));
         shape.by_block_cols = make_fast_divisor(static_cast<uint32_t>(block_cols));
         shape.scale_form = block_cols % vec == 0 ? kScalePerUnit : (block_cols == 1 && aligned(scale, vec) ? kScalePerColumn : kScaleAny);
-        // (indices are 32-bit: a larger tensor goes in slices of whole block rows)
-        const int64_t slice = std::min(rows, std::max<int64_t>(1, ((1ll << 31) - (1 << 20)) / cols / block_rows) * block_rows);
+        // (indices are 32-bit: a larger tensor goes in slices of rows)
+        const int64_t slice = std::min<int64_t>(rows, ((1ll << 31) - (1 << 20)) / cols);
         for (int64_t row = 0; row < rows; row += slice) {
             shape.total = static_cast<uint32_t>(std::min(slice, rows - row) * cols);
             const unsigned grid = (shape.total + 1024 * vec - 1) / (1024 * vec);
             const uint8_t* codes = x + row * cols;
             const uint8_t* scales = scale + row / block_rows * shape.scale_cols;
+            shape.first_row = static_cast<uint32_t>(row % block_rows);
             if (p->y.dtype == DFGPU_F32) launch_chained(bsd_packed_kernel<DFGPU_F32>, dim3(grid), dim3(256), 0, stream, codes, scales, static_cast<float*>(y) + row * cols, shape);
             else if (p->y.dtype == DFGPU_BF16) launch_chained(bsd_packed_kernel<DFGPU_BF16>, dim3(grid), dim3(256), 0, stream, codes, scales, static_cast<uint16_t*>(y) + row * cols, shape);
             else launch_chained(bsd_packed_kernel<DFGPU_F16>, dim3(grid), dim3(256), 0, stream, codes, scales, static_cast<uint16_t*>(y) + row * cols, shape);

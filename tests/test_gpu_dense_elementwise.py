@@ -104,3 +104,23 @@ def test_dequantize(io, rows, cols, blocks, offset):
     want = (codes.view(torch.float8_e4m3fn).double().view(rows, cols) * factor).to(TORCH[io])
     assert torch.equal(torch.isnan(out.view(rows, cols)), torch.isnan(want))
     assert torch.equal(out.view(rows, cols).nan_to_num(0.0, 1e30, -1e30), want.nan_to_num(0.0, 1e30, -1e30))
+
+
+def test_dequantize_in_slices():
+    """Blocks of rows that hold more codes than 32-bit indices reach: slices that begin inside a block, under the kernel id that takes them."""
+    cols, rows = 1 << 20, 3000
+    blocks = [rows, 1]
+    p = dfgpu.BsdParams()
+    p.x, p.scale, p.y = dfgpu.tensor(dfgpu.E4M3, [rows, cols]), dfgpu.tensor(dfgpu.E8M0, [rows // blocks[0], cols]), dfgpu.tensor(dfgpu.BF16, [rows, cols])
+    p.block[0], p.block[1], p.block_count, p.kernel = blocks[0], 1, 2, dfgpu.BSD_PACKED
+    assert dfgpu.query("block_scale_dequantize", p).kernel == dfgpu.BSD_PACKED
+    g = torch.Generator(device="cuda").manual_seed(1)
+    codes = torch.randint(0, 120, (rows, cols), device="cuda", generator=g, dtype=torch.uint8)
+    scales = torch.randint(120, 131, (rows // blocks[0], cols), device="cuda", generator=g, dtype=torch.uint8)
+    out = torch.empty(rows, cols, device="cuda", dtype=torch.bfloat16)
+    dfgpu.block_scale_dequantize(p, codes.data_ptr(), scales.data_ptr(), out.data_ptr())
+    torch.cuda.synchronize()
+    for first in (0, 2040, 2047, 2048, rows - 8):   # (2047 rows of 2^20 codes are a slice)
+        some = slice(first, first + 8)
+        want = codes[some].view(torch.float8_e4m3fn).float() * torch.pow(2.0, scales[0].float() - 127)
+        assert torch.equal(out[some], want.bfloat16())
