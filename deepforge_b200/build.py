@@ -66,7 +66,7 @@ def nlohmann_include() -> Path:
 def build_kernels(force: bool = False, verbose: bool = False) -> Path:
     OUT.mkdir(exist_ok=True)
     sources = sorted((PKG / "csrc").glob("*.cu"))
-    headers = sorted((PKG / "csrc").glob("*.cuh")) + sorted((PKG / "csrc").glob("*.h")) + [ROOT / "include" / "dfgpu.h"]
+    headers = sorted((PKG / "csrc").glob("*.cuh")) + [ROOT / "include" / "dfgpu.h"]
     target = OUT / "libdfgpu.so"
     stamp = _stamp(sources + headers, " ".join(NVCC_FLAGS))
     if not force and _up_to_date(target, stamp):
@@ -97,7 +97,7 @@ def build_host(force: bool = False) -> Path:
     OUT.mkdir(exist_ok=True)
     kernels = build_kernels()
     sources = sorted((PKG / "host").glob("*.cpp"))
-    headers = sorted((ROOT / "include").rglob("*.h")) + sorted((PKG / "csrc").glob("*.h")) + sorted((PKG / "host").glob("*.h"))
+    headers = sorted((ROOT / "include").rglob("*.h")) + sorted((PKG / "host").glob("*.h"))
     target = OUT / "libdeepforge_b200.so"
     flags = ["-std=c++20", "-O2", "-fPIC", "-Wall", "-Wextra", "-Wno-unused-parameter"]
     stamp = _stamp(sources + headers, " ".join(flags))

@@ -1,6 +1,5 @@
 // Error reporting and small host utilities shared by every launcher.
 #include "common.cuh"
-#include "launch_record.h"
 
 #include <cstring>
 
@@ -24,10 +23,7 @@ int check_launch(const char* what) {
     return kOk;
 }
 
-namespace {
-thread_local LaunchRecord* g_recorder = nullptr;
-
-cudaError_t send(const void* function, dim3 grid, dim3 block, unsigned cluster, size_t dynamic_smem, cudaStream_t stream, void** arguments) {
+cudaError_t submit(const void* function, dim3 grid, dim3 block, unsigned cluster, size_t dynamic_smem, cudaStream_t stream, void** arguments) {
     cudaLaunchConfig_t config{};
     config.gridDim = grid;
     config.blockDim = block;
@@ -45,52 +41,6 @@ cudaError_t send(const void* function, dim3 grid, dim3 block, unsigned cluster, 
         config.numAttrs = 2;
     }
     return cudaLaunchKernelExC(&config, function, arguments);
-}
-}  // namespace
-
-int current_device() {
-    int device = -1;
-    return cudaGetDevice(&device) == cudaSuccess ? device : -1;
-}
-
-void open_recorder(LaunchRecord* record) {
-    record->device = current_device();
-    record->launches.clear();
-    g_recorder = record;
-}
-void close_recorder() { g_recorder = nullptr; }
-
-cudaError_t submit(const void* function, dim3 grid, dim3 block, unsigned cluster, size_t dynamic_smem, cudaStream_t stream, void** arguments,
-                   const size_t* sizes, size_t count) {
-    if (g_recorder) {
-        RecordedLaunch launch{function, {grid.x, grid.y, grid.z}, {block.x, block.y, block.z}, cluster, dynamic_smem, {}, nullptr};
-        size_t total = 0;
-        for (size_t i = 0; i < count; ++i) {
-            launch.offsets.push_back(total);
-            total += (sizes[i] + 63) / 64 * 64;
-        }
-        launch.arguments.reset(new unsigned char[total + 1]);
-        for (size_t i = 0; i < count; ++i) std::memcpy(launch.arguments.get() + launch.offsets[i], arguments[i], sizes[i]);
-        g_recorder->launches.push_back(std::move(launch));
-    }
-    return send(function, grid, block, cluster, dynamic_smem, stream, arguments);
-}
-
-int replay(const LaunchRecord& record, void* stream) {
-    constexpr size_t kMaxArguments = 24;
-    for (const RecordedLaunch& launch : record.launches) {
-        void* arguments[kMaxArguments];
-        const size_t count = launch.offsets.size();
-        if (count > kMaxArguments) return fail(kExecutionFailed, "replay: a kernel with %zu arguments", count);
-        for (size_t i = 0; i < count; ++i) arguments[i] = launch.arguments.get() + launch.offsets[i];
-        cudaError_t error = send(launch.function, dim3(launch.grid[0], launch.grid[1], launch.grid[2]), dim3(launch.block[0], launch.block[1], launch.block[2]),
-                                 launch.cluster, launch.shared_bytes, as_stream(stream), arguments);
-        if (error != cudaSuccess) {
-            (void)cudaGetLastError();
-            return fail(kExecutionFailed, "kernel launch failed: %s", cudaGetErrorString(error));
-        }
-    }
-    return kOk;
 }
 
 int sm_count() {

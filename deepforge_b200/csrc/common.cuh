@@ -63,9 +63,8 @@ inline bool valid_tensor(const dfgpu_tensor& t) {
 
 int sm_count();
 
-// Sends one kernel off (chained, see below) and writes it down when the thread has a recorder open (launch_record.h).
-cudaError_t submit(const void* function, dim3 grid, dim3 block, unsigned cluster, size_t dynamic_smem, cudaStream_t stream, void** arguments,
-                   const size_t* sizes, size_t count);
+// Sends one kernel off, chained (see below); cluster: CTAs per cluster along x (0: none).
+cudaError_t submit(const void* function, dim3 grid, dim3 block, unsigned cluster, size_t dynamic_smem, cudaStream_t stream, void** arguments);
 
 // ---- programmatic dependent launch ------------------------------------------------
 // A kernel launched with launch_chained() may start while the kernel before it in the stream is still
@@ -105,8 +104,7 @@ cudaError_t launch_chained_clusters(std::index_sequence<I...>, void (*kernel)(Pa
                                     cudaStream_t stream, Args&&... args) {
     std::tuple<std::remove_cv_t<Params>...> held(static_cast<Params>(args)...);
     void* pointers[] = {static_cast<void*>(&std::get<I>(held))...};
-    constexpr size_t sizes[] = {sizeof(std::remove_cv_t<Params>)...};
-    return submit(reinterpret_cast<const void*>(kernel), grid, block, cluster, dynamic_smem, stream, pointers, sizes, sizeof...(Params));
+    return submit(reinterpret_cast<const void*>(kernel), grid, block, cluster, dynamic_smem, stream, pointers);
 }
 template <typename... Params, typename... Args>
 cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t dynamic_smem, cudaStream_t stream, Args&&... args) {

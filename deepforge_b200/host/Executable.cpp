@@ -8,10 +8,6 @@
 // Pointers are device pointers: they are compared and offset, never dereferenced here.
 #include "Internal.h"
 
-#include "../csrc/launch_record.h"
-
-#include <algorithm>
-#include <array>
 #include <mutex>
 
 namespace deepforge::runtime {
@@ -24,15 +20,34 @@ using import::ErrorCode;
 using import::Status;
 
 namespace {
-// What one whole execute() sent off, for the pointers it was given: a host that runs the same buffers again (a training
-// or serving loop does) skips the validation and the launchers, which find the same answers from the same pointers
-// (2.2 us of a 5.4 us one-launch call, 3.4 us of two-launch ones). Kept per executable for the last kReplays pointer
-// sets, so that a host may rotate its buffers; recorded when a set comes by for the second time, so that a host whose
-// pointers are always new pays for the comparison only.
-constexpr std::size_t kReplays = 4;
-struct Replay {
-    std::vector<void*> pointers;   // in the order of the argument table, then the workspace
-    std::shared_ptr<dfgpu::LaunchRecord const> record;   // null: seen once
+// Where a launch finds one of its pointers: in the argument table, in the workspace, or nowhere (null).
+struct Source {
+    TensorBinding::Kind kind = TensorBinding::Kind::kAbsent;
+    std::size_t at = 0;   // index into the argument table, or byte offset in the workspace
+};
+struct StepSources {
+    std::vector<Source> tensors;
+    Source scratch;
+};
+
+// A few values on the stack, more on the heap: a call binds fewer than ten pointers as a rule.
+template <class T>
+class Few {
+public:
+    explicit Few(std::size_t count) : data_(few_) {
+        if (count > kFew) {
+            many_.resize(count);
+            data_ = many_.data();
+        }
+    }
+    T& operator[](std::size_t i) { return data_[i]; }
+    T* data() { return data_; }
+
+private:
+    static constexpr std::size_t kFew = 32;
+    T few_[kFew];
+    std::vector<T> many_;
+    T* data_;
 };
 }  // namespace
 
@@ -43,50 +58,8 @@ struct Executable::Impl {
     void* stream = nullptr;
     std::int64_t launches = 0;
     mutable std::mutex mutex;
-    mutable std::mutex replay_mutex;
-    mutable std::array<Replay, kReplays> replays;
-    mutable std::size_t next_replay = 0, last_replay = 0;
-
-    std::shared_ptr<dfgpu::LaunchRecord const> find_replay(void* const* pointers, std::size_t count, void* workspace, bool& record) const;
-    void keep_replay(std::vector<void*> const& pointers, void* workspace, std::shared_ptr<dfgpu::LaunchRecord const> made) const;
+    std::vector<StepSources> sources;   // of the plan's steps
 };
-
-namespace {
-bool same_pointers(Replay const& entry, void* const* pointers, std::size_t count, void* workspace) {
-    if (entry.pointers.size() != count + 1 || entry.pointers[count] != workspace) return false;
-    return std::equal(pointers, pointers + count, entry.pointers.begin());
-}
-}  // namespace
-
-// The record for these pointers, or null; `record` then says whether the call should be written down.
-std::shared_ptr<dfgpu::LaunchRecord const> Executable::Impl::find_replay(void* const* pointers, std::size_t count, void* workspace, bool& record) const {
-    std::lock_guard<std::mutex> lock(replay_mutex);
-    record = false;
-    for (std::size_t i = 0; i < kReplays; ++i) {
-        auto const slot = (last_replay + i) % kReplays;
-        auto const& entry = replays[slot];
-        if (!same_pointers(entry, pointers, count, workspace)) continue;
-        last_replay = slot;
-        if (entry.record && entry.record->device == dfgpu::current_device()) return entry.record;
-        record = true;
-        return nullptr;
-    }
-    auto& entry = replays[next_replay];
-    next_replay = (next_replay + 1) % kReplays;
-    entry.record.reset();
-    entry.pointers.assign(pointers, pointers + count);
-    entry.pointers.push_back(workspace);
-    return nullptr;
-}
-
-void Executable::Impl::keep_replay(std::vector<void*> const& pointers, void* workspace, std::shared_ptr<dfgpu::LaunchRecord const> made) const {
-    std::lock_guard<std::mutex> lock(replay_mutex);
-    for (auto& entry : replays)
-        if (same_pointers(entry, pointers.data(), pointers.size(), workspace)) {
-            entry.record = std::move(made);
-            return;
-        }
-}
 
 std::string_view cpu_variant_name(CpuVariant variant) noexcept {
     switch (variant) {
@@ -108,7 +81,22 @@ std::unique_ptr<Executable> ExecutableFactory::create(compiler::GraphCompileMeta
     impl->metadata = std::move(metadata);
     impl->workspace = std::move(workspace);
     impl->plan = std::move(plan);
-    for (auto const& step : impl->plan.steps) impl->launches += step.launches;
+    auto const& arguments = impl->metadata.arguments;
+    auto source = [&](TensorBinding const& binding) {
+        Source out;
+        if (binding.kind == TensorBinding::Kind::kWorkspace) out = {binding.kind, static_cast<std::size_t>(binding.offset)};
+        if (binding.kind == TensorBinding::Kind::kArgument)
+            for (std::size_t i = 0; i < arguments.size(); ++i)
+                if (arguments[i].uid == binding.uid) out = {binding.kind, i};
+        return out;
+    };
+    for (auto const& step : impl->plan.steps) {
+        impl->launches += step.launches;
+        StepSources sources;
+        for (auto const& binding : step.tensors) sources.tensors.push_back(source(binding));
+        sources.scratch = source(step.scratch);
+        impl->sources.push_back(std::move(sources));
+    }
     return std::unique_ptr<Executable>(new Executable(std::move(impl)));
 }
 
@@ -120,10 +108,6 @@ Status Executable::get_workspace_size(std::int64_t& workspace_size) const {
 }
 
 namespace {
-Status missing_uid(compiler::TensorArgumentMetadata const& argument) {
-    return Status::failure(ErrorCode::kInvalidVariantPack, argument.name, "UID " + std::to_string(argument.uid) + " is missing from the variant pack");
-}
-
 Status reject_overrides(OverrideUids const& uids, OverrideShapes const& shapes, OverrideStrides const& strides) {
     if (uids.empty() && shapes.empty() && strides.empty()) return Status::ok();
     return Status::failure(ErrorCode::kInvalidVariantPack, "override", "the graph was compiled without shape overrides");
@@ -181,80 +165,70 @@ Status Executable::execute_steps(std::int64_t first, std::int64_t last, VariantP
 }
 
 Status Executable::run_steps(std::int64_t first, std::int64_t last, VariantPack& pack, void* workspace, void* call_stream, bool own_stream) const {
-    auto const& arguments = impl_->metadata.arguments;
-    std::vector<void*> pointers(arguments.size());
-    for (std::size_t i = 0; i < arguments.size(); ++i) {
-        auto it = pack.find(arguments[i].uid);
-        if (it == pack.end()) return missing_uid(arguments[i]);
-        pointers[i] = it->second;
-    }
-    return run_bound(first, last, pointers.data(), workspace, call_stream, own_stream);
+    auto find = [&](std::int64_t uid, void*& pointer) {
+        auto it = pack.find(uid);
+        if (it == pack.end()) return false;
+        pointer = it->second;
+        return true;
+    };
+    return run(first, last, find, workspace, call_stream, own_stream);
 }
 
 Status Executable::execute_list(std::int64_t const* uids, void* const* list, std::size_t count, void* workspace, void* call_stream, bool own_stream) const {
-    auto const& arguments = impl_->metadata.arguments;
-    constexpr std::size_t kFew = 32;   // (above, a map beats the scan)
-    if (count > kFew || arguments.size() > kFew) {
+    auto const steps = static_cast<std::int64_t>(impl_->plan.steps.size());
+    constexpr std::size_t kFewEntries = 32;   // (above, a map beats the scan)
+    if (count > kFewEntries) {
         VariantPack pack;
         pack.reserve(count);
         for (std::size_t i = 0; i < count; ++i) pack[uids[i]] = list[i];
-        return run_steps(0, static_cast<std::int64_t>(impl_->plan.steps.size()), pack, workspace, call_stream, own_stream);
+        return run_steps(0, steps, pack, workspace, call_stream, own_stream);
     }
-    void* pointers[kFew];
-    for (std::size_t i = 0; i < arguments.size(); ++i) {
-        std::size_t at = count;
-        while (at > 0 && uids[at - 1] != arguments[i].uid) --at;   // from the end: the last entry of a UID counts, as in a map
-        if (at == 0) return missing_uid(arguments[i]);
-        pointers[i] = list[at - 1];
-    }
-    return run_bound(0, static_cast<std::int64_t>(impl_->plan.steps.size()), pointers, workspace, call_stream, own_stream);
+    auto find = [&](std::int64_t uid, void*& pointer) {
+        for (std::size_t at = count; at > 0; --at)   // from the end: the last entry of a UID counts, as in a map
+            if (uids[at - 1] == uid) {
+                pointer = list[at - 1];
+                return true;
+            }
+        return false;
+    };
+    return run(0, steps, find, workspace, call_stream, own_stream);
 }
 
-// bound: one pointer per entry of the argument table, in its order.
-Status Executable::run_bound(std::int64_t first, std::int64_t last, void* const* bound, void* workspace, void* call_stream, bool own_stream) const {
+template <class Find>
+Status Executable::run(std::int64_t first, std::int64_t last, Find const& find, void* workspace, void* call_stream, bool own_stream) const {
     auto const& impl = *impl_;
-    auto const argument_count = impl.metadata.arguments.size();
-    bool const whole = first == 0 && last == static_cast<std::int64_t>(impl.plan.steps.size());
-    bool write_down = false;
-    if (whole)
-        if (auto record = impl.find_replay(bound, argument_count, workspace, write_down)) {
-            std::unique_lock<std::mutex> lock(impl.mutex, std::defer_lock);
-            if (!own_stream) {
-                lock.lock();
-                call_stream = impl.stream;
-            }
-            int const code = dfgpu::replay(*record, call_stream);
-            return code == 0 ? Status::ok() : Status::failure(static_cast<ErrorCode>(code), "execute", dfgpu_last_error());
-        }
     if (first < 0 || last > static_cast<std::int64_t>(impl.plan.steps.size()) || first > last)
         return Status::failure(ErrorCode::kInvalidArgument, "steps", "step range is outside the kernel plan");
 
     struct Range {
         std::uintptr_t begin, end;
         bool written;
-        std::string const* name;
     };
-    std::vector<Range> ranges;
-    ranges.reserve(impl.metadata.arguments.size());
-    for (std::size_t i = 0; i < argument_count; ++i) {
-        auto const& argument = impl.metadata.arguments[i];
+    auto const& arguments = impl.metadata.arguments;
+    auto const count = arguments.size();
+    Few<void*> bound(count);
+    Few<Range> ranges(count);
+    for (std::size_t i = 0; i < count; ++i) {
+        auto const& argument = arguments[i];
+        if (!find(argument.uid, bound[i]))
+            return Status::failure(ErrorCode::kInvalidVariantPack, argument.name, "UID " + std::to_string(argument.uid) + " is missing from the variant pack");
         if (bound[i] == nullptr) return Status::failure(ErrorCode::kInvalidVariantPack, argument.name, "pointer is null");
         auto address = reinterpret_cast<std::uintptr_t>(bound[i]);
         if (address % argument.alignment != 0) return Status::failure(ErrorCode::kInvalidVariantPack, argument.name, "pointer is not aligned to " + std::to_string(argument.alignment) + " bytes");
-        ranges.push_back({address, address + argument.size_bytes, argument.access != TensorAccess::kRead, &argument.name});
+        ranges[i] = {address, address + argument.size_bytes, argument.access != TensorAccess::kRead};
     }
-    for (std::size_t i = 0; i < ranges.size(); ++i)
-        for (std::size_t j = i + 1; j < ranges.size(); ++j)
+    for (std::size_t i = 0; i < count; ++i)
+        for (std::size_t j = i + 1; j < count; ++j)
             if ((ranges[i].written || ranges[j].written) && ranges[i].begin < ranges[j].end && ranges[j].begin < ranges[i].end)
-                return Status::failure(ErrorCode::kInvalidVariantPack, *ranges[i].name, "storage overlaps '" + *ranges[j].name + "' and at least one of them is written");
+                return Status::failure(ErrorCode::kInvalidVariantPack, arguments[i].name, "storage overlaps '" + arguments[j].name + "' and at least one of them is written");
     auto const workspace_bytes = impl.workspace.size_bytes;
     if (workspace_bytes != 0) {
         if (workspace == nullptr) return Status::failure(ErrorCode::kInvalidVariantPack, "workspace", "pointer is null but " + std::to_string(workspace_bytes) + " bytes are required");
         auto address = reinterpret_cast<std::uintptr_t>(workspace);
         if (address % compiler::kWorkspaceAlignment != 0) return Status::failure(ErrorCode::kInvalidVariantPack, "workspace", "pointer is not aligned to 64 bytes");
-        for (auto const& range : ranges)
-            if (address < range.end && range.begin < address + workspace_bytes)
-                return Status::failure(ErrorCode::kInvalidVariantPack, "workspace", "storage overlaps '" + *range.name + "'");
+        for (std::size_t i = 0; i < count; ++i)
+            if (address < ranges[i].end && ranges[i].begin < address + workspace_bytes)
+                return Status::failure(ErrorCode::kInvalidVariantPack, "workspace", "storage overlaps '" + arguments[i].name + "'");
     }
 
     // The plan is immutable and the launchers keep no state between calls, so a call with its own stream needs no
@@ -265,30 +239,19 @@ Status Executable::run_bound(std::int64_t first, std::int64_t last, void* const*
         lock.lock();
         stream = impl.stream;
     }
-    auto resolve = [&](TensorBinding const& binding) -> void* {
-        switch (binding.kind) {
-            case TensorBinding::Kind::kArgument: {   // (the table is in ascending UID order, or X, W, Y for a single convolution)
-                auto const& arguments = impl.metadata.arguments;
-                for (std::size_t i = 0; i < argument_count; ++i)
-                    if (arguments[i].uid == binding.uid) return bound[i];
-                return nullptr;
-            }
-            case TensorBinding::Kind::kWorkspace: return static_cast<char*>(workspace) + binding.offset;
+    auto resolve = [&](Source const& source) -> void* {
+        switch (source.kind) {
+            case TensorBinding::Kind::kArgument: return bound[source.at];
+            case TensorBinding::Kind::kWorkspace: return static_cast<char*>(workspace) + source.at;
             default: return nullptr;
         }
     };
-    dfgpu::LaunchRecord made;
-    struct Recorder {
-        bool open;
-        Recorder(bool wanted, dfgpu::LaunchRecord& record) : open(wanted) { if (open) dfgpu::open_recorder(&record); }
-        ~Recorder() { if (open) dfgpu::close_recorder(); }
-    } recorder(write_down, made);
-    std::vector<void*> pointers;
     for (std::int64_t index = first; index < last; ++index) {
         auto const& step = impl.plan.steps[static_cast<std::size_t>(index)];
-        pointers.clear();
-        for (auto const& binding : step.tensors) pointers.push_back(resolve(binding));
-        void* scratch = resolve(step.scratch);
+        auto const& sources = impl.sources[static_cast<std::size_t>(index)];
+        Few<void*> pointers(sources.tensors.size());
+        for (std::size_t i = 0; i < sources.tensors.size(); ++i) pointers[i] = resolve(sources.tensors[i]);
+        void* scratch = resolve(sources.scratch);
         int code = 0;
         switch (step.op) {
             case KernelOp::kBlockScaleQuantize: code = dfgpu_block_scale_quantize(&std::get<dfgpu_bsq_params>(step.params), pointers.data(), scratch, stream); break;
@@ -319,8 +282,6 @@ Status Executable::run_bound(std::int64_t first, std::int64_t last, void* const*
             return Status::failure(mapped, step.label, dfgpu_last_error());
         }
     }
-    if (write_down && made.device >= 0)
-        impl.keep_replay(std::vector<void*>(bound, bound + argument_count), workspace, std::make_shared<dfgpu::LaunchRecord const>(std::move(made)));
     return Status::ok();
 }
 

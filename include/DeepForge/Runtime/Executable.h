@@ -88,9 +88,9 @@ public:
 
 private:
     import::Status run_steps(std::int64_t first, std::int64_t last, VariantPack& pack, void* workspace, void* stream, bool own_stream) const;
-    import::Status run_bound(std::int64_t first, std::int64_t last, void* const* bound, void* workspace, void* stream, bool own_stream) const;
-
-private:
+    // find(uid, pointer): the pack's pointer for a UID, false when it holds none.
+    template <class Find>
+    import::Status run(std::int64_t first, std::int64_t last, Find const& find, void* workspace, void* stream, bool own_stream) const;
     struct Impl;
     explicit Executable(std::unique_ptr<Impl> impl);
     friend struct ExecutableFactory;

@@ -1,5 +1,5 @@
-"""Repeated execution: an Executable keeps the launches of its last few sets of pointers. Results follow the data, the pointers, the
-workspace and the stream of every call, also when more sets rotate than are kept, and a pack that would be refused still is.
+"""Repeated execution: results follow the data, the pointers, the workspace and the stream of every call, however many sets of pointers
+rotate, and a pack that would be refused once it has run still is.
 f32 sums of 64 products and three additions: 2^-17 of the magnitudes."""
 import threading
 
