@@ -7,6 +7,7 @@
 #include "deepforge_b200.h"
 
 #include <memory>
+#include <new>
 
 namespace {
 
@@ -49,8 +50,9 @@ PyObject* execute(PyObject*, PyObject* const* arguments, Py_ssize_t count) {
     std::unique_ptr<void*[]> many_pointers;
     const Py_ssize_t size = PyDict_GET_SIZE(pack);
     if (size > kFew) {
-        many_uids.reset(new std::int64_t[size]);
-        many_pointers.reset(new void*[size]);
+        many_uids.reset(new (std::nothrow) std::int64_t[size]);
+        many_pointers.reset(new (std::nothrow) void*[size]);
+        if (!many_uids || !many_pointers) return PyErr_NoMemory();
         uids = many_uids.get();
         pointers = many_pointers.get();
     }
