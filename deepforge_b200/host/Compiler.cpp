@@ -1098,32 +1098,59 @@ void materialise_constants(Lowering& low) {
     low.plan.steps.insert(low.plan.steps.begin(), std::make_move_iterator(head.begin()), std::make_move_iterator(head.end()));
 }
 
-// Alignment the resolved kernel's launcher demands of the pointer in tensor slot `slot` (0: no demand of its own).
-// The TMA-fed kernels read and write 16-byte units and have no narrower fallback (the block-scale launchers do).
-// (A matrix product whose extents are whole tiles takes 16-byte aligned operands only; any other falls back to the CUDA
-// cores where a pointer is off that boundary, so its arguments keep the reference's alignment.)
+// Graphs that demand 16-byte aligned arguments of the matrix and SDPA kernels: whole tiles, and every row and fused operand in
+// whole 16-byte units. The kernels take more than that (HALF, ragged extents, strides of any length in C, layouts other than packed
+// B, H, S, D); those arguments keep the reference's alignment, and the launchers fall back to the CUDA cores where a pointer is off TMA's boundary.
+bool in_units(dfgpu_tensor const& t, std::int64_t elements) { return t.stride[t.rank - 1] == 1 && t.stride[t.rank - 2] % elements == 0; }
+
 template <typename Params>
 bool whole_tiles(Params const& p, std::int64_t tile) {
     auto const rank = p.c.rank;
     return p.a.dim[rank - 1] % tile == 0 && p.c.dim[rank - 1] % tile == 0 && (tile == 64 || p.c.dim[rank - 2] % tile == 0);
 }
 
+bool demands_units(dfgpu_matmul_params const& p, bool scaled) {
+    if (!whole_tiles(p, scaled ? 128 : 64) || p.a.dtype == DFGPU_F16 || p.c.dtype == DFGPU_F16) return false;
+    if (!in_units(p.a, scaled ? 16 : 8) || !in_units(p.c, 8) || (scaled && !in_units(p.a_scale, 4))) return false;
+    for (int i = 0; i < p.epilogue_count; ++i) {
+        if (p.epilogue[i].op != DFGPU_EPI_ADD) continue;
+        auto const& t = p.extra[p.epilogue[i].operand];
+        if (t.dtype == DFGPU_F16) return false;
+        bool const per_column = t.rank == 1 || t.dim[t.rank - 2] == 1;   // (the kernel's own rule; any other operand is a full one)
+        if (scaled || per_column) continue;
+        if (t.rank != p.c.rank) return false;
+        for (int axis = 0; axis < t.rank; ++axis)
+            if (t.dim[axis] != p.c.dim[axis] || t.stride[axis] != p.c.stride[axis]) return false;
+    }
+    return true;
+}
+
+bool demands_units(dfgpu_matmul_fp8_params const& p) {
+    return whole_tiles(p, 128) && in_units(p.c, p.c.dtype == DFGPU_E4M3 ? 16 : (p.c.dtype == DFGPU_BF16 ? 8 : 4));
+}
+
+bool demands_units(dfgpu_sdpa_params const& p) {
+    if (p.q.dtype != DFGPU_BF16 || p.q.dim[3] != 128 || p.q.dim[2] % 128 != 0 || p.k.dim[2] % 128 != 0 || p.padding_mask) return false;
+    for (auto const* t : {&p.q, &p.k, &p.v, &p.o})
+        if (t->stride[3] != 1 || t->stride[2] != t->dim[3] || t->stride[1] != t->dim[2] * t->dim[3] || t->stride[0] != t->dim[1] * t->dim[2] * t->dim[3]) return false;
+    if ((p.max.rank || p.sum_exp.rank) && (p.q.dim[2] % 256 != 0 || !(p.attn_scale > 0.0f))) return false;
+    return !p.has_right_bound || p.q.dim[2] == p.k.dim[2];
+}
+
+// Alignment the resolved kernel's launcher demands of the pointer in tensor slot `slot` (0: no demand of its own).
+// The convolutions' TMA-fed kernels read and write 16-byte units and have no narrower fallback (the block-scale launchers do).
 std::uint64_t kernel_alignment(KernelStep const& step, std::size_t slot) {
     switch (step.op) {
         case KernelOp::kConvFprop: return step.kernel == DFGPU_CONV_UMMA_BF16 || step.kernel == DFGPU_CONV_UMMA_F32X3 ? 16 : 0;  // (the one-launch f32 form takes any pointer: see dfgpu_conv_fprop)
         case KernelOp::kMatmul:
             if (step.kernel != DFGPU_MATMUL_UMMA_BF16 && step.kernel != DFGPU_MATMUL_UMMA_MXF8) return 0;
-            if (!whole_tiles(std::get<dfgpu_matmul_params>(step.params), step.kernel == DFGPU_MATMUL_UMMA_MXF8 ? 128 : 64)) return 0;
+            if (!demands_units(std::get<dfgpu_matmul_params>(step.params), step.kernel == DFGPU_MATMUL_UMMA_MXF8)) return 0;
             return slot == 3 || slot == 4 ? 4 : 16;  // the scale tensors are gathered with 4-byte loads
         case KernelOp::kSdpaForward:
-            if (step.kernel == DFGPU_SDPA_UMMA) {   // (lengths that are no whole tiles fall back where a pointer is off the boundary, as above)
-                auto const& p = std::get<dfgpu_sdpa_params>(step.params);
-                bool const whole = p.q.dtype == DFGPU_BF16 && p.q.dim[3] == 128 && p.q.dim[2] % 128 == 0 && p.k.dim[2] % 128 == 0 && !p.padding_mask;
-                return slot <= 3 && whole ? 16 : 0;
-            }
+            if (step.kernel == DFGPU_SDPA_UMMA) return slot <= 3 && demands_units(std::get<dfgpu_sdpa_params>(step.params)) ? 16 : 0;
             if (step.kernel == DFGPU_SDPA_PAGED_DECODE_UMMA || step.kernel == DFGPU_SDPA_PAGED_DECODE) return slot <= 2 ? 16 : 0;
             return 0;
-        case KernelOp::kMatmulFp8: return step.kernel == DFGPU_MATMUL_FP8_UMMA && slot <= 2 && whole_tiles(std::get<dfgpu_matmul_fp8_params>(step.params), 128) ? 16 : 0;
+        case KernelOp::kMatmulFp8: return step.kernel == DFGPU_MATMUL_FP8_UMMA && slot <= 2 && demands_units(std::get<dfgpu_matmul_fp8_params>(step.params)) ? 16 : 0;
         case KernelOp::kConvFpropPair: return 16;
         case KernelOp::kBlockScaleQuantizePair: return slot % 3 == 0 ? 16 : 8;
         case KernelOp::kBlockScaleQuantize:   // packed FP4 codes are written a nibble at a time through their aligned word

@@ -94,3 +94,15 @@ def test_operands_off_the_sixteen_byte_boundary_fall_back():
     buffers = {1: a, 2: b}
     run(doc, buffers)
     close(buffers[4].view(m, n), a.view(m, k).double(), b.view(k, n).double(), lambda p: p, "BFLOAT16", k)
+
+
+@pytest.mark.parametrize("io,c_ld", [("HALF", 128), ("BFLOAT16", 130)])
+def test_whole_tiles_off_the_boundary_fall_back(io, c_ld):
+    """Whole tiles in HALF, or with rows of C that are no whole 16-byte units, keep the element's alignment as well."""
+    m, k, n = 128, 64, 128
+    g = torch.Generator(device="cuda").manual_seed(6)
+    doc = graphs.document("tiles", [graphs.matmul_node("matmul", 1, 2, 4)], [graphs.tensor(1, "A", [m, k], io), graphs.tensor(2, "B", [k, n], io), graphs.tensor(4, "C", [m, n], io, [c_ld, 1])], io=io)
+    a, b = (torch.randn(count + 1, device="cuda", generator=g).to(TORCH[io])[1:] for count in (m * k, k * n))
+    buffers = {1: a, 2: b, 4: torch.zeros(m * c_ld, dtype=TORCH[io], device="cuda")}
+    run(doc, buffers)
+    close(buffers[4].view(m, c_ld)[:, :n], a.view(m, k).double(), b.view(k, n).double(), lambda p: p, io, k)

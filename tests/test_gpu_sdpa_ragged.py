@@ -149,3 +149,20 @@ def test_scores_that_are_all_minus_infinity(h):
     stats, largest, total = (x[:, :, 0::2] for x in outs)
     assert bool(torch.all(o[:, :, 0::2] == 0)) and bool(torch.all(torch.isneginf(stats))) and bool(torch.all(torch.isneginf(largest))) and bool(torch.all(total == 0))
     assert bool(torch.all(o[:, :, 1::2] == 1)) and bool(torch.all((outs[2][:, :, 1::2] - s).abs() <= 1e-3))
+
+
+@pytest.mark.parametrize("io,d,strided", [("HALF", 128, False), ("BFLOAT16", 128, True)])
+def test_whole_tiles_off_the_boundary_fall_back(io, d, strided):
+    """Whole tiles in HALF or in a layout other than packed B, H, S, D accept pointers on the element's boundary."""
+    g = torch.Generator(device="cuda").manual_seed(8)
+    shape = (1, 256, 2, d) if strided else (1, 2, 256, d)
+    q, k, v, o = (torch.randn(2 * 256 * d + 1, device="cuda", generator=g).to(TORCH[io])[1:].view(shape) for _ in range(4))
+    if strided:
+        q, k, v, o = (x.transpose(1, 2) for x in (q, k, v, o))
+    tensors = [graphs.tensor(uid, name, list(x.shape), io, list(x.stride())) for uid, name, x in ((1, "Q", q), (2, "K", k), (3, "V", v), (4, "O", o))]
+    exe = runtime.compile_graph(graphs.document("units", [graphs.sdpa_node("sdpa", {"Q": 1, "K": 2, "V": 3}, {"O": 4}, d ** -0.5, False, False)], tensors, io=io))
+    exe.execute({1: q.data_ptr(), 2: k.data_ptr(), 3: v.data_ptr(), 4: o.data_ptr()})
+    torch.cuda.synchronize()
+    want, weight, _, _ = attention(q, k, v, d ** -0.5, False)
+    u = ROUNDING[io]
+    assert bool(torch.all((o.double() - want).abs() <= 2.0 ** -14 * weight + u * want.abs() + 1e-30))   # (the general kernel: f32 throughout)

@@ -213,6 +213,39 @@ def test_argument_table_is_sorted_with_clamped_alignment():
     assert {a["uid"]: a["alignment"] for a in decode.arguments()}[5] == 4
 
 
+def _matmul(io="BFLOAT16", c_type="BFLOAT16", c_ld=128, m=128, a_ld=128, addend=None):
+    tensors = [graphs.tensor(1, "A", [m, 128], io, [a_ld, 1]), graphs.tensor(2, "B", [128, 128], io), graphs.tensor(9, "C", [m, 128], c_type, [c_ld, 1])]
+    nodes = [graphs.matmul_node("matmul", 1, 2, 9 if addend is None else 5)]
+    if addend is not None:
+        tensors += [graphs.tensor(3, "addend", [m, 128], *addend), graphs.tensor(5, "p", [m, 128], virtual=True)]
+        nodes.append(graphs.pointwise_node("add", "ADD", 5, 9, 3))
+    return graphs.document("units", nodes, tensors, io=io)
+
+
+def _sdpa(io="BFLOAT16", s=256, skv=256, d=128, strided=False, causal=False, padding=False):
+    def operand(uid, name, length):
+        return graphs.tensor(uid, name, [1, 2, length, d], io, [2 * length * d, d, 2 * d, 1] if strided else None)
+    tensors = [operand(1, "Q", s), operand(2, "K", skv), operand(3, "V", skv), operand(9, "O", s)]
+    inputs = {"Q": 1, "K": 2, "V": 3}
+    if padding:
+        tensors += [graphs.tensor(6, "SEQ_LEN_Q", [1, 1, 1, 1], "INT32"), graphs.tensor(7, "SEQ_LEN_KV", [1, 1, 1, 1], "INT32")]
+        inputs.update(SEQ_LEN_Q=6, SEQ_LEN_KV=7)
+    return graphs.document("units", [graphs.sdpa_node("sdpa", inputs, {"O": 9}, d ** -0.5, padding, False, right_bound=0 if causal else None)], tensors, io=io)
+
+
+@pytest.mark.parametrize("document,uids,alignment", [
+    (_matmul(), (1, 2, 9), 16), (_matmul(c_type="FLOAT"), (1, 2, 9), 16), (_matmul(m=1), (1, 2, 9), 16), (_matmul(addend=("BFLOAT16",)), (1, 2, 3, 9), 16),
+    (_matmul("HALF", "HALF"), (1, 2, 9), 2), (_matmul(c_type="HALF"), (1, 2, 9), 2), (_matmul(c_ld=130), (1, 2, 9), 2), (_matmul(m=1, a_ld=129), (1, 2, 9), 2),
+    (_matmul(addend=("HALF",)), (1, 2, 3, 9), 2), (_matmul(addend=("BFLOAT16", [136, 1])), (1, 2, 3, 9), 2),
+    (graphs.matmul_fp8(128, 128, 128), (21, 22, 26), 16), (graphs.matmul_fp8(128, 128, 128, "HALF"), (21, 22), 1), (graphs.matmul_fp8(64, 128, 128), (21, 22), 1),
+    (_sdpa(), (1, 2, 3, 9), 16), (_sdpa(causal=True), (1, 2, 3, 9), 16), (_sdpa("HALF"), (1, 2, 3, 9), 2), (_sdpa(strided=True), (1, 2, 3, 9), 2), (_sdpa(d=64), (1, 2, 3, 9), 2),
+    (_sdpa(skv=384, causal=True), (1, 2, 3, 9), 2), (_sdpa(s=200, skv=200), (1, 2, 3, 9), 2), (_sdpa(padding=True), (1, 2, 3, 9), 2)])
+def test_only_whole_units_demand_sixteen_bytes(document, uids, alignment):
+    """Forms that the tensor cores took over from the CUDA cores accept the pointers they always accepted."""
+    table = {a["uid"]: a["alignment"] for a in runtime.compile_graph(document).arguments()}
+    assert {table[uid] for uid in uids} == {alignment}
+
+
 @pytest.mark.parametrize("doc_fn,expected", [
     (lambda: graphs.c4_sdpa(1, 2, 16, 8, io="HALF"), 0),
     (lambda: _with(graphs.c4_sdpa(1, 2, 16, 8), lambda d: d["nodes"][0].update(alibi_mask=True)), 0),
