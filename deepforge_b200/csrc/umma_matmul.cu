@@ -5,6 +5,12 @@
 // once for two products (six-fold deep copies moved and stored twice as much: 1183 x 1888 x 5360 154 us then, 128 now, 87 of
 // products; 4096^3 586 of 500).
 //
+// kSummed: 16-bit operands, f32 C, the products of every K block in an accumulator of their own and the blocks added by the epilogue in
+// f32. The tensor cores cut off what a sum does not hold, toward zero, so that the error of one long accumulation grows with K:
+// 2050 x 8184 x 1040 bf16 to f32 is 9.1e-6 from 64 bits in one accumulator, 9.6e-7 by the CUDA cores' additions, 2.2e-7 this way. The
+// forms that ran there (or in the one-launch f32 kernel) keep an accuracy no worse than theirs. The epilogue's two loads and 64
+// additions a block set the pace: 4096 x 4104 x 4104 124 us in one accumulator, 234 this way, 9227 on the CUDA cores.
+//
 // Extents are free because the copies are: TMA fills what lies outside a matrix with zeros and clips what would be stored
 // there, so a tile may hang over any edge. Only the rows' starts have to fall on 16-byte boundaries.
 //
@@ -38,7 +44,7 @@ constexpr int kMaxStages = 16;
 constexpr int kMaxSteps = DFGPU_MAX_EPILOGUE;
 constexpr int kSmemBudget = 227 * 1024 - 1024;   // (1 KB of slack aligns the tiles)
 
-enum Kind { kSixteen = 0, kCodes = 1, kScaled = 2, kPieces = 3 };
+enum Kind { kSixteen = 0, kCodes = 1, kScaled = 2, kPieces = 3, kSummed = 4 };
 enum { kStepRelu = 1, kStepBias = 2, kStepFull = 3 };
 
 struct TileArgs {
@@ -139,7 +145,7 @@ __device__ __forceinline__ void product(uint32_t d, uint64_t a, uint64_t b, uint
 #define DFGPU_MMA(FORM)                                                                                                   \
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma." FORM " [%0], %1, %2, %3, p;\n\t}"          \
                  ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory")
-    constexpr bool sixteen = KIND == kSixteen || KIND == kPieces;
+    constexpr bool sixteen = KIND == kSixteen || KIND == kPieces || KIND == kSummed;
     if constexpr (sixteen && CG == 1) DFGPU_MMA("cta_group::1.kind::f16");
     if constexpr (sixteen && CG == 2) DFGPU_MMA("cta_group::2.kind::f16");
     if constexpr (KIND == kCodes && CG == 1) DFGPU_MMA("cta_group::1.kind::f8f6f4");
@@ -303,6 +309,35 @@ __device__ __forceinline__ void add_small_products(uint32_t address, uint32_t (&
     for (int e = 0; e < 32; ++e) sum[e] = __float_as_uint(__fadd_rn(__uint_as_float(sum[e]), __uint_as_float(small[e])));
 }
 
+// kSummed: this thread's row of a tile, the boxes g and g + 2 of 32 columns, summed over the K blocks of the walk. `local` counts
+// accumulators, as the issuing warp does; one is handed back as soon as it is in registers.
+template <int CG>
+__device__ __forceinline__ void sum_blocks(float (&sums)[2][32], uint32_t columns, int acc_stride, int boxes, int g, int blocks, int& local, uint32_t acc_full, uint32_t acc_empty,
+                                           int lane, bool& ok) {
+    for (int block = 0; block < blocks; ++block, ++local) {
+        const int acc = local & 1;
+        if (ok) ok = mbar_wait_warp(acc_full + 8u * acc, (local >> 1) & 1, 585);   // (the warp stays together)
+        tc_fence_after();
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if (q == 1 && g + 2 >= boxes) break;   // (two boxes at least: one for each group)
+            uint32_t raw[32];
+            tmem_load_32(columns + acc * acc_stride + (g + 2 * q) * 32, raw);
+            tmem_load_wait();
+#pragma unroll
+            for (int e = 0; e < 32; ++e) asm volatile("" : "+r"(raw[e]));   // (no use above the wait)
+#pragma unroll
+            for (int e = 0; e < 32; ++e) sums[q][e] = block == 0 ? __uint_as_float(raw[e]) : __fadd_rn(sums[q][e], __uint_as_float(raw[e]));
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+            if (CG == 2) mbar_arrive_cluster(acc_empty + 8u * acc);
+            else mbar_arrive(acc_empty + 8u * acc);
+        }
+    }
+}
+
 template <int KIND>
 constexpr int thread_count() { return KIND == kScaled ? 512 : 384; }
 
@@ -388,8 +423,8 @@ template <int KIND, int CG>
 __global__ void __launch_bounds__(thread_count<KIND>(), 1)
 umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c,
                    const __grid_constant__ TileArgs args) {
-    constexpr int kCode = KIND == kSixteen ? 0 : (KIND == kCodes ? 20 : (KIND == kScaled ? 40 : 60));
-    constexpr bool kSixteenBits = KIND == kSixteen || KIND == kPieces;
+    constexpr int kCode = KIND == kSixteen ? 0 : (KIND == kCodes ? 20 : (KIND == kScaled ? 40 : (KIND == kPieces ? 60 : 80)));
+    constexpr bool kSixteenBits = KIND == kSixteen || KIND == kPieces || KIND == kSummed;
     constexpr int kPieceCount = KIND == kPieces ? 3 : 1;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -485,15 +520,23 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             int stage = 0, local = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (int i = first_item; i < args.items; i += item_step, ++local) {
+            for (int i = first_item; i < args.items; i += item_step, local += KIND == kSummed ? 0 : 1) {
                 const int width = item_at(args, i).width, acc = local & args.acc_shift, use = local >> args.acc_shift;
                 const uint32_t idesc_wide = args.idesc | (static_cast<uint32_t>(width >> 3) << 17);
-                if (ok) ok = wait_warp<CG == 2>(acc_empty(acc), (use & 1) ^ 1, 502 + kCode);
+                if (KIND != kSummed && ok) ok = wait_warp<CG == 2>(acc_empty(acc), (use & 1) ^ 1, 502 + kCode);
                 // (where the accumulators overlap, the other one's shared columns must have been read out too)
                 if (overlapped && ok && local > 0) ok = mbar_wait_warp(overlap_free, (local - 1) & 1, 507 + kCode);
                 tc_fence_after();
-                const uint32_t d = tmem_u + acc * args.acc_stride;
+                uint32_t d = tmem_u + acc * args.acc_stride;
                 for (int kb = kb_begin; kb < kb_end && ok; ++kb) {
+                    const int block_acc = local & 1;
+                    if constexpr (KIND == kSummed) {   // (an accumulator per block)
+                        ok = wait_warp<CG == 2>(acc_empty(block_acc), ((local >> 1) & 1) ^ 1, 502 + kCode);
+                        if (!ok) break;
+                        tc_fence_after();
+                        d = tmem_u + block_acc * args.acc_stride;
+                        ++local;
+                    }
                     ok = mbar_wait_warp(full_bar(stage), phase, 503 + kCode);
                     if (!ok) break;   // (operands by TMA, scales by generic stores + fence.proxy.async: no tcgen05 fence needed)
                     if (leader) {
@@ -525,14 +568,15 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                             uint32_t idesc = idesc_wide;
                             if constexpr (KIND == kScaled) idesc |= (static_cast<uint32_t>(j) << 29) | (static_cast<uint32_t>(j) << 4);   // the K block's byte of the scale words
                             product<KIND, CG>(d, desc_words(a_lo + ((j * 32) >> 4), smem_desc_hi(1024)), desc_words(b_lo + j * b_step, smem_desc_hi(1024)), idesc,
-                                              kb != kb_begin || j != 0 ? 1u : 0u, sf, sf + 4);
+                                              (KIND != kSummed && kb != kb_begin) || j != 0 ? 1u : 0u, sf, sf + 4);
                         }
                         commit_to_all<CG>(empty_bar(stage));
+                        if constexpr (KIND == kSummed) commit_to_all<CG>(acc_full(block_acc));
                     }
                     __syncwarp();
                     if (++stage == args.stages) { stage = 0; phase ^= 1; }
                 }
-                if (leader) commit_to_all<CG>(acc_full(acc));   // arrives even after a failed wait, so that no epilogue hangs
+                if (KIND != kSummed && leader) commit_to_all<CG>(acc_full(acc));   // arrives even after a failed wait, so that no epilogue hangs
                 __syncwarp();
             }
         }
@@ -541,15 +585,29 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const int quadrant = warp & 3, g = (warp - 4) >> 2, row = quadrant * 32 + lane;
         const uint32_t lane_base = static_cast<uint32_t>(quadrant * 32) << 16;
         bool ok = true;
+        float sums[2][32];   // (kSummed)
         if (split) {
             // park the f32 partial tile where the operands were: rows of bn floats, 16-byte units swizzled by the row
-            ok = mbar_wait(acc_full(0), 0, 504 + kCode);
-            tc_fence_after();
+            if constexpr (KIND == kSummed) {
+                int local = 0;
+                sum_blocks<CG>(sums, tmem_base + lane_base, args.acc_stride, bn / 32, g, kb_end - kb_begin, local, acc_full(0), acc_empty(0), lane, ok);
+            } else {
+                ok = mbar_wait(acc_full(0), 0, 504 + kCode);
+                tc_fence_after();
+            }
             uint8_t* parked = generic_base + row * bn * 4;
             for (int c = g; c < bn / 32; c += 2) {
                 uint32_t raw[32];
-                tmem_load_32(tmem_base + lane_base + c * 32, raw);
-                tmem_load_wait();
+                if constexpr (KIND == kSummed) {
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) {
+                        raw[e] = __float_as_uint(sums[0][e]);
+                        sums[0][e] = sums[1][e];
+                    }
+                } else {
+                    tmem_load_32(tmem_base + lane_base + c * 32, raw);
+                    tmem_load_wait();
+                }
                 if constexpr (KIND == kPieces) add_small_products(tmem_base + lane_base + bn + c * 32, raw);
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
@@ -563,13 +621,17 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             Scalars scalars = load_scalars(args);
             bool stored = false;   // (this group has a store in flight)
             int local = 0;
-            for (int i = first_item; i < args.items; i += item_step, ++local) {
+            for (int i = first_item; i < args.items; i += item_step, local += KIND == kSummed ? 0 : 1) {
                 const int acc = local & args.acc_shift, use = local >> args.acc_shift;
                 const Item item = item_at(args, i);
                 const int row0 = (item.m_tile * CG + (CG == 2 ? rank : 0)) * kRows, out_row = row0 + row;
                 const bool row_live = out_row < args.m_total;
-                if (ok) ok = mbar_wait(acc_full(acc), use & 1, 505 + kCode);
-                tc_fence_after();
+                if constexpr (KIND == kSummed) {
+                    sum_blocks<CG>(sums, tmem_base + lane_base, args.acc_stride, item.width / 32, g, kb_end - kb_begin, local, acc_full(0), leader_bars + (acc_empty(0) - bar_base), lane, ok);
+                } else {
+                    if (ok) ok = mbar_wait(acc_full(acc), use & 1, 505 + kCode);
+                    tc_fence_after();
+                }
                 const bool healthy = ok && g_device_status == 0;
                 const uint32_t columns = tmem_base + lane_base + acc * args.acc_stride;
                 const int boxes = item.width / box_columns;
@@ -583,8 +645,16 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     }
                     for (int part = 0; part < box_columns / 32; ++part) {
                         uint32_t raw[32];
-                        tmem_load_32(columns + box * box_columns + part * 32, raw);
-                        tmem_load_wait();
+                        if constexpr (KIND == kSummed) {   // (f32 C: boxes of 32 columns)
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) {
+                                raw[e] = __float_as_uint(sums[0][e]);
+                                sums[0][e] = sums[1][e];   // (the group's second box is next)
+                            }
+                        } else {
+                            tmem_load_32(columns + box * box_columns + part * 32, raw);
+                            tmem_load_wait();
+                        }
                         if constexpr (KIND == kPieces) add_small_products(columns + bn + box * box_columns + part * 32, raw);
                         if (overlapped && b == g && g != acc && part == box_columns / 32 - 1) {   // the shared columns are in registers
                             tc_fence_before();
@@ -636,7 +706,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) {
+                if (KIND != kSummed && lane == 0) {
                     if (CG == 2) mbar_arrive_cluster(leader_bars + 8u * (2 * kMaxStages + 2 + acc));
                     else mbar_arrive(acc_empty(acc));
                 }
@@ -780,7 +850,7 @@ bool describe(const dfgpu_tensor& a, const dfgpu_tensor& b, const dfgpu_tensor& 
     p.K = a.dim[rank - 1];
     if (a.dim[rank - 2] != p.M || b.dim[rank - 2] != p.K || b.dim[rank - 1] != p.N) return false;
     if (p.M < 1 || p.N < 1 || p.K < 1 || p.M > (1ll << 28) || p.N > (1ll << 28) || p.K > (1ll << 28)) return false;
-    p.in_bytes = kind == kSixteen ? 2 : 1;
+    p.in_bytes = kind == kSixteen || kind == kSummed ? 2 : 1;
     p.a_rows = p.M;
     p.out_dtype = c.dtype;
     p.out_bytes = dtype_bytes(c.dtype);
@@ -800,7 +870,7 @@ bool describe(const dfgpu_tensor& a, const dfgpu_tensor& b, const dfgpu_tensor& 
 // stage's inside the allocation.)
 int rows_of_a(const Problem& p, int cg) { return cg == 1 && p.M < kRows ? static_cast<int>((p.M + 7) / 8 * 8) : kRows; }
 int stage_bytes(const Problem& p, int bn, int cg, int a_rows) { return (a_rows + bn / cg) * kRowBytes * (p.kind == kPieces ? 3 : 1) + (p.kind == kScaled ? 2048 : 0); }
-bool sixteen_bits(const Problem& p) { return p.kind == kSixteen || p.kind == kPieces; }
+bool sixteen_bits(const Problem& p) { return p.kind == kSixteen || p.kind == kPieces || p.kind == kSummed; }
 int ring_bytes(int stages, int stage_size) { return (stages - 1) * stage_size + std::max(stage_size, kABytes); }
 int stages_that_fit(int stage_size, int budget) {
     int stages = std::min(kMaxStages, budget / stage_size);
@@ -834,6 +904,7 @@ Shape choose_shape(const Problem& p) {
             if (p.out_dtype == DFGPU_E4M3 && bn % 128 != 0) continue;   // (whole 128-byte boxes)
             if (p.kind == kScaled && bn % 128 != 0) continue;           // (whole chunks of column scales)
             if (cg == 2 && bn < 128) continue;
+            if (p.kind == kSummed && bn > 128) continue;                // (a row's sums live in registers)
             if (bn > chunk && bn >= 2 * ((p.N + 63) / 64 * 64)) continue;  // (half the tile would be empty)
             const int64_t m_tiles = (p.M + kRows * cg - 1) / (kRows * cg), n_tiles = (p.N + bn - 1) / bn, tiles = m_tiles * n_tiles;
             const int rows = rows_of_a(p, cg), stage_size = stage_bytes(p, bn, cg, rows);
@@ -853,7 +924,8 @@ Shape choose_shape(const Problem& p) {
                 }
                 const double in_flight = static_cast<double>(stages_that_fit(stage_size, kSmemBudget - 2 * kStageBox)) * stage_size;
                 const double products = p.kind == kPieces ? 6.0 : 1.0, pieces = p.kind == kPieces ? 3.0 : 1.0;
-                const double block = std::max({products * 2.0 * bn, (products + pieces) * (rows + bn / cg), pieces * (rows + bn / cg) * kRowBytes / std::min(48.0, in_flight / 2300.0)});
+                const double summed = p.kind == kSummed ? 150.0 + 2.0 * bn : 0.0;   // the epilogue's loads and additions of a block
+                const double block = std::max({summed, products * 2.0 * bn, (products + pieces) * (rows + bn / cg), pieces * (rows + bn / cg) * kRowBytes / std::min(48.0, in_flight / 2300.0)});
                 const double clocks = rounds * (k_per_split * block) + 2000.0 + bn * 6.0 + (splits > 1 ? (p.kind == kScaled ? 5000.0 : 2500.0) : 0.0) + (cg == 2 ? 1500.0 : 0.0);
                 if (best.cg == 0 || clocks < best.clocks) best = Shape{cg, bn, splits, static_cast<int>(k_per_split), tiles, halved, clocks};
             }
@@ -932,6 +1004,7 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     const int grid = static_cast<int>(groups * (shape.cg == 2 ? 2 : shape.splits));
     if (p.kind == kSixteen) return shape.cg == 2 ? launch_kernel<kSixteen, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kSixteen, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     if (p.kind == kCodes) return shape.cg == 2 ? launch_kernel<kCodes, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kCodes, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
+    if (p.kind == kSummed) return shape.cg == 2 ? launch_kernel<kSummed, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kSummed, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     if (p.kind == kPieces) return shape.cg == 2 ? launch_kernel<kPieces, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kPieces, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     return shape.cg == 2 ? launch_kernel<kScaled, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kScaled, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
 }
@@ -971,11 +1044,29 @@ bool translate_steps(const dfgpu_matmul_params& p, void* const* tensors, TileArg
     return true;
 }
 
+// f32 results that are summed block by block (kSummed): all but those of whole bf16 tiles in whole 16-byte units, which always
+// came from one accumulator.
+bool sums_blocks(const dfgpu_matmul_params& p) {
+    const int rank = p.c.rank;
+    if (p.c.dtype != DFGPU_F32 || rank < 2 || p.a.rank != rank) return false;
+    if (p.a.dtype != DFGPU_BF16 || p.a.dim[rank - 1] % 64 != 0 || p.c.dim[rank - 1] % 64 != 0 || p.a.stride[rank - 2] % 8 != 0 || p.c.stride[rank - 2] % 8 != 0) return true;
+    for (int i = 0; i < p.epilogue_count; ++i) {
+        if (p.epilogue[i].op != DFGPU_EPI_ADD) continue;
+        const dfgpu_tensor& t = p.extra[p.epilogue[i].operand];
+        const bool per_column = t.rank == 1 || t.dim[t.rank - 2] == 1;
+        if (t.dtype == DFGPU_F16 || (!per_column && (t.rank != rank || t.stride[rank - 2] != p.c.stride[rank - 2]))) return true;
+    }
+    return false;
+}
+
 bool sixteen_problem(const dfgpu_matmul_params& p, Problem& problem) {
     if (p.a_scale.rank || p.b_scale.rank) return false;
     if ((p.a.dtype != DFGPU_BF16 && p.a.dtype != DFGPU_F16) || p.b.dtype != p.a.dtype) return false;   // (one kind of operand per instruction)
     if (p.c.dtype != DFGPU_BF16 && p.c.dtype != DFGPU_F16 && p.c.dtype != DFGPU_F32) return false;
-    return describe(p.a, p.b, p.c, kSixteen, problem) && translate_steps(p, nullptr, nullptr);
+    // (fewer products in bf16: the CUDA cores' additions are the more exact, 5.4e-8 from 64 bits for 6.3e-8 at 72, 6.0 / 6.4 at 88, 6.6 / 6.6 at 104)
+    constexpr int64_t kSummedMinDepth = 104;
+    if (p.a.dtype == DFGPU_BF16 && sums_blocks(p) && p.a.dim[p.a.rank - 1] < kSummedMinDepth) return false;
+    return translate_steps(p, nullptr, nullptr) && describe(p.a, p.b, p.c, sums_blocks(p) ? kSummed : kSixteen, problem);
 }
 
 bool scaled_problem(const dfgpu_matmul_params& p, Problem& problem) {

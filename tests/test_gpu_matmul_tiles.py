@@ -106,3 +106,21 @@ def test_whole_tiles_off_the_boundary_fall_back(io, c_ld):
     buffers = {1: a, 2: b, 4: torch.zeros(m * c_ld, dtype=TORCH[io], device="cuda")}
     run(doc, buffers)
     close(buffers[4].view(m, c_ld)[:, :n], a.view(m, k).double(), b.view(k, n).double(), lambda p: p, io, k)
+
+
+@pytest.mark.parametrize("m,k,n,c_ld", [(1, 72, 24, 24), (77, 64, 40, 40), (77, 256, 272, 272), (129, 104, 136, 136), (130, 520, 136, 139), (300, 4112, 528, 528), (2050, 264, 1040, 1040), (2050, 8184, 1040, 1040), (4096, 1032, 4104, 4104)])
+@pytest.mark.parametrize("io", ["BFLOAT16", "HALF"])
+@pytest.mark.parametrize("b_k_major", [False, True])
+def test_f32_results_do_not_lose_accuracy_with_depth(m, k, n, c_ld, io, b_k_major):
+    """A block of 64 is off by at most four cut-off sums of four ulps (2^-21 of its value), blocks of random sign add up as their values
+    do, and every addition of a block rounds the sum so far by 2^-25 in the mean."""
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    doc = graphs.document("tiles", [graphs.matmul_node("matmul", 1, 2, 4)], [graphs.tensor(1, "A", [m, k], io), graphs.tensor(2, "B", [k, n], io, [1, k] if b_k_major else [n, 1]), graphs.tensor(4, "C", [m, n], "FLOAT", [c_ld, 1])], io=io)
+    a, b = (torch.randn(count, device="cuda", generator=g).to(TORCH[io]) for count in (m * k, k * n))
+    buffers = {1: a, 2: b, 4: torch.zeros(m * c_ld, device="cuda")}
+    shallow = io == "BFLOAT16" and k < 104   # (the CUDA cores' additions are the more exact)
+    assert [s["kernel"] for s in run(doc, buffers).steps()] == [dfgpu.MATMUL_FFMA if shallow else dfgpu.MATMUL_UMMA_BF16]
+    b = b.view(n, k).t() if b_k_major else b.view(k, n)
+    want = a.view(m, k).double() @ b.double()
+    error = (buffers[4].view(m, c_ld)[:, :n].double() - want).norm() / want.norm()
+    assert float(error) <= 2.0 ** -21 + 2.0 ** -25 * (k / 64) ** 0.5
