@@ -10,6 +10,7 @@
 // 2050 x 8184 x 1040 bf16 to f32 is 9.1e-6 from 64 bits in one accumulator, 9.6e-7 by the CUDA cores' additions, 2.2e-7 this way. The
 // forms that ran there (or in the one-launch f32 kernel) keep an accuracy no worse than theirs. The epilogue's two loads and 64
 // additions a block set the pace: 4096 x 4104 x 4104 124 us in one accumulator, 234 this way, 9227 on the CUDA cores.
+// kScaledSummed: the same for block-scaled codes (1026 x 8160 x 1040 to f32: 1.2e-7 on the CUDA cores, 4.7e-7 in one accumulator).
 //
 // Extents are free because the copies are: TMA fills what lies outside a matrix with zeros and clips what would be stored
 // there, so a tile may hang over any edge. Only the rows' starts have to fall on 16-byte boundaries.
@@ -44,7 +45,9 @@ constexpr int kMaxStages = 16;
 constexpr int kMaxSteps = DFGPU_MAX_EPILOGUE;
 constexpr int kSmemBudget = 227 * 1024 - 1024;   // (1 KB of slack aligns the tiles)
 
-enum Kind { kSixteen = 0, kCodes = 1, kScaled = 2, kPieces = 3, kSummed = 4 };
+enum Kind { kSixteen = 0, kCodes = 1, kScaled = 2, kPieces = 3, kSummed = 4, kScaledSummed = 5 };
+template <int KIND> constexpr bool kHasScales = KIND == kScaled || KIND == kScaledSummed;
+template <int KIND> constexpr bool kInBlocks = KIND == kSummed || KIND == kScaledSummed;   // an accumulator per K block, summed by the epilogue
 enum { kStepRelu = 1, kStepBias = 2, kStepFull = 3 };
 
 struct TileArgs {
@@ -154,8 +157,8 @@ __device__ __forceinline__ void product(uint32_t d, uint64_t a, uint64_t b, uint
 #define DFGPU_MMA(FORM)                                                                                                   \
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma." FORM ".kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}" \
                  ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb) : "memory")
-    if constexpr (KIND == kScaled && CG == 1) DFGPU_MMA("cta_group::1");
-    if constexpr (KIND == kScaled && CG == 2) DFGPU_MMA("cta_group::2");
+    if constexpr (kHasScales<KIND> && CG == 1) DFGPU_MMA("cta_group::1");
+    if constexpr (kHasScales<KIND> && CG == 2) DFGPU_MMA("cta_group::2");
 #undef DFGPU_MMA
 }
 // 32 rows x 16 bytes of shared memory -> 4 columns of tensor memory, replicated to the four lane quarters.
@@ -309,6 +312,10 @@ __device__ __forceinline__ void add_small_products(uint32_t address, uint32_t (&
     for (int e = 0; e < 32; ++e) sum[e] = __float_as_uint(__fadd_rn(__uint_as_float(sum[e]), __uint_as_float(small[e])));
 }
 
+__device__ __forceinline__ void tmem_put_32(uint32_t address, const uint32_t (&r)[32]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+                 ::"r"(address), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
+}
 // kSummed: this thread's row of a tile, the boxes g and g + 2 of 32 columns, summed over the K blocks of the walk. `local` counts
 // accumulators, as the issuing warp does; one is handed back as soon as it is in registers.
 template <int CG>
@@ -338,8 +345,43 @@ __device__ __forceinline__ void sum_blocks(float (&sums)[2][32], uint32_t column
     }
 }
 
+// kScaledSummed: the same with the sums in tensor memory, behind the two accumulators: its 16 warps leave too few registers.
+template <int CG>
+__device__ __forceinline__ void sum_blocks_in_place(uint32_t columns, int acc_stride, int boxes, int g, int blocks, int& local, uint32_t acc_full, uint32_t acc_empty, int lane, bool& ok) {
+    for (int block = 0; block < blocks; ++block, ++local) {
+        const int acc = local & 1;
+        if (ok) ok = mbar_wait_warp(acc_full + 8u * acc, (local >> 1) & 1, 595);
+        tc_fence_after();
+        for (int box = g; box < boxes; box += 2) {
+            uint32_t raw[32];
+            tmem_load_32(columns + acc * acc_stride + box * 32, raw);
+            if (block > 0) {
+                uint32_t sum[32];
+                tmem_load_32(columns + 2 * acc_stride + box * 32, sum);
+                tmem_load_wait();
+#pragma unroll
+                for (int e = 0; e < 32; ++e) asm volatile("" : "+r"(raw[e]), "+r"(sum[e]));   // (no use above the wait)
+#pragma unroll
+                for (int e = 0; e < 32; ++e) raw[e] = __float_as_uint(__fadd_rn(__uint_as_float(sum[e]), __uint_as_float(raw[e])));
+            } else {
+                tmem_load_wait();
+#pragma unroll
+                for (int e = 0; e < 32; ++e) asm volatile("" : "+r"(raw[e]));
+            }
+            tmem_put_32(columns + 2 * acc_stride + box * 32, raw);
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+            if (CG == 2) mbar_arrive_cluster(acc_empty + 8u * acc);
+            else mbar_arrive(acc_empty + 8u * acc);
+        }
+    }
+}
+
 template <int KIND>
-constexpr int thread_count() { return KIND == kScaled ? 512 : 384; }
+constexpr int thread_count() { return kHasScales<KIND> ? 512 : 384; }
 
 // One K block's scales of a tile as a lane reads them from the plain tensors: 4 rows of A (rows lane, lane + 32, ... of 128)
 // and 4 or 8 columns of B, four K blocks each. Addresses are clamped, so that nothing branches around a load and all of
@@ -423,7 +465,7 @@ template <int KIND, int CG>
 __global__ void __launch_bounds__(thread_count<KIND>(), 1)
 umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c,
                    const __grid_constant__ TileArgs args) {
-    constexpr int kCode = KIND == kSixteen ? 0 : (KIND == kCodes ? 20 : (KIND == kScaled ? 40 : (KIND == kPieces ? 60 : 80)));
+    constexpr int kCode = KIND == kSixteen ? 0 : (KIND == kCodes ? 20 : (KIND == kScaled ? 40 : (KIND == kPieces ? 60 : (KIND == kSummed ? 80 : 90))));
     constexpr bool kSixteenBits = KIND == kSixteen || KIND == kPieces || KIND == kSummed;
     constexpr int kPieceCount = KIND == kPieces ? 3 : 1;
     extern __shared__ uint8_t smem_raw[];
@@ -456,7 +498,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     }
     if (warp == 0 && leader) {
         for (int s = 0; s < args.stages; ++s) {
-            mbar_init(full_bar(s), KIND == kScaled ? 1 + CG : 1);   // the byte count, and the slot's scale warp of each CTA
+            mbar_init(full_bar(s), kHasScales<KIND> ? 1 + CG : 1);   // the byte count, and the slot's scale warp of each CTA
             mbar_init(empty_bar(s), 1);
         }
         for (int a = 0; a < 2; ++a) {
@@ -520,17 +562,17 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             int stage = 0, local = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (int i = first_item; i < args.items; i += item_step, local += KIND == kSummed ? 0 : 1) {
+            for (int i = first_item; i < args.items; i += item_step, local += kInBlocks<KIND> ? 0 : 1) {
                 const int width = item_at(args, i).width, acc = local & args.acc_shift, use = local >> args.acc_shift;
                 const uint32_t idesc_wide = args.idesc | (static_cast<uint32_t>(width >> 3) << 17);
-                if (KIND != kSummed && ok) ok = wait_warp<CG == 2>(acc_empty(acc), (use & 1) ^ 1, 502 + kCode);
+                if (!kInBlocks<KIND> && ok) ok = wait_warp<CG == 2>(acc_empty(acc), (use & 1) ^ 1, 502 + kCode);
                 // (where the accumulators overlap, the other one's shared columns must have been read out too)
                 if (overlapped && ok && local > 0) ok = mbar_wait_warp(overlap_free, (local - 1) & 1, 507 + kCode);
                 tc_fence_after();
                 uint32_t d = tmem_u + acc * args.acc_stride;
                 for (int kb = kb_begin; kb < kb_end && ok; ++kb) {
                     const int block_acc = local & 1;
-                    if constexpr (KIND == kSummed) {   // (an accumulator per block)
+                    if constexpr (kInBlocks<KIND>) {   // (an accumulator per block)
                         ok = wait_warp<CG == 2>(acc_empty(block_acc), ((local >> 1) & 1) ^ 1, 502 + kCode);
                         if (!ok) break;
                         tc_fence_after();
@@ -543,7 +585,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         const uint32_t a_src = smem_base + stage * args.stage_bytes, b_src = a_src + kPieceCount * args.a_bytes;   // (with few rows the products read on into B: rows of C nobody stores)
                         const uint32_t a_lo = smem_desc_lo(a_src, 16), b_lo = smem_desc_lo(b_src, b_lbo);
                         uint32_t sf = 0;
-                        if constexpr (KIND == kScaled) {
+                        if constexpr (kHasScales<KIND>) {
                             const uint32_t scales = b_src + bn / CG * kRowBytes;
                             sf = tmem_u + args.scale_columns + (stage & 1) * 16;   // A's at +0..3, B's at +4..11
                             copy_scales<CG>(sf, scales);
@@ -566,17 +608,17 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             uint32_t idesc = idesc_wide;
-                            if constexpr (KIND == kScaled) idesc |= (static_cast<uint32_t>(j) << 29) | (static_cast<uint32_t>(j) << 4);   // the K block's byte of the scale words
+                            if constexpr (kHasScales<KIND>) idesc |= (static_cast<uint32_t>(j) << 29) | (static_cast<uint32_t>(j) << 4);   // the K block's byte of the scale words
                             product<KIND, CG>(d, desc_words(a_lo + ((j * 32) >> 4), smem_desc_hi(1024)), desc_words(b_lo + j * b_step, smem_desc_hi(1024)), idesc,
-                                              (KIND != kSummed && kb != kb_begin) || j != 0 ? 1u : 0u, sf, sf + 4);
+                                              (!kInBlocks<KIND> && kb != kb_begin) || j != 0 ? 1u : 0u, sf, sf + 4);
                         }
                         commit_to_all<CG>(empty_bar(stage));
-                        if constexpr (KIND == kSummed) commit_to_all<CG>(acc_full(block_acc));
+                        if constexpr (kInBlocks<KIND>) commit_to_all<CG>(acc_full(block_acc));
                     }
                     __syncwarp();
                     if (++stage == args.stages) { stage = 0; phase ^= 1; }
                 }
-                if (KIND != kSummed && leader) commit_to_all<CG>(acc_full(acc));   // arrives even after a failed wait, so that no epilogue hangs
+                if (!kInBlocks<KIND> && leader) commit_to_all<CG>(acc_full(acc));   // arrives even after a failed wait, so that no epilogue hangs
                 __syncwarp();
             }
         }
@@ -591,6 +633,9 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             if constexpr (KIND == kSummed) {
                 int local = 0;
                 sum_blocks<CG>(sums, tmem_base + lane_base, args.acc_stride, bn / 32, g, kb_end - kb_begin, local, acc_full(0), acc_empty(0), lane, ok);
+            } else if constexpr (KIND == kScaledSummed) {
+                int local = 0;
+                sum_blocks_in_place<CG>(tmem_base + lane_base, args.acc_stride, bn / 32, g, kb_end - kb_begin, local, acc_full(0), acc_empty(0), lane, ok);
             } else {
                 ok = mbar_wait(acc_full(0), 0, 504 + kCode);
                 tc_fence_after();
@@ -605,7 +650,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         sums[0][e] = sums[1][e];
                     }
                 } else {
-                    tmem_load_32(tmem_base + lane_base + c * 32, raw);
+                    tmem_load_32(tmem_base + lane_base + (KIND == kScaledSummed ? 2 * args.acc_stride : 0) + c * 32, raw);
                     tmem_load_wait();
                 }
                 if constexpr (KIND == kPieces) add_small_products(tmem_base + lane_base + bn + c * 32, raw);
@@ -621,19 +666,21 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             Scalars scalars = load_scalars(args);
             bool stored = false;   // (this group has a store in flight)
             int local = 0;
-            for (int i = first_item; i < args.items; i += item_step, local += KIND == kSummed ? 0 : 1) {
+            for (int i = first_item; i < args.items; i += item_step, local += kInBlocks<KIND> ? 0 : 1) {
                 const int acc = local & args.acc_shift, use = local >> args.acc_shift;
                 const Item item = item_at(args, i);
                 const int row0 = (item.m_tile * CG + (CG == 2 ? rank : 0)) * kRows, out_row = row0 + row;
                 const bool row_live = out_row < args.m_total;
                 if constexpr (KIND == kSummed) {
                     sum_blocks<CG>(sums, tmem_base + lane_base, args.acc_stride, item.width / 32, g, kb_end - kb_begin, local, acc_full(0), leader_bars + (acc_empty(0) - bar_base), lane, ok);
+                } else if constexpr (KIND == kScaledSummed) {
+                    sum_blocks_in_place<CG>(tmem_base + lane_base, args.acc_stride, item.width / 32, g, kb_end - kb_begin, local, acc_full(0), leader_bars + (acc_empty(0) - bar_base), lane, ok);
                 } else {
                     if (ok) ok = mbar_wait(acc_full(acc), use & 1, 505 + kCode);
                     tc_fence_after();
                 }
                 const bool healthy = ok && g_device_status == 0;
-                const uint32_t columns = tmem_base + lane_base + acc * args.acc_stride;
+                const uint32_t columns = tmem_base + lane_base + (KIND == kScaledSummed ? 2 : acc) * args.acc_stride;
                 const int boxes = item.width / box_columns;
                 for (int b = g; b < boxes; b += 2) {
                     // overlapping accumulators: the first one is read from its end, the second from its start
@@ -706,7 +753,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (KIND != kSummed && lane == 0) {
+                if (!kInBlocks<KIND> && lane == 0) {
                     if (CG == 2) mbar_arrive_cluster(leader_bars + 8u * (2 * kMaxStages + 2 + acc));
                     else mbar_arrive(acc_empty(acc));
                 }
@@ -715,7 +762,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             __syncwarp();
             fold_amax(args, scalars, lane, ok);
         }
-    } else if (KIND == kScaled) {
+    } else if (kHasScales<KIND>) {
         // ---- scale loaders: warp i of the six owns the slots i and i + 6 ----
         // (A slot has ONE owner: the parity of its barrier tells apart two rounds, not three, so a warp that came by a slot
         // only every other round could fill it before its last round was read.)
@@ -869,7 +916,8 @@ bool describe(const dfgpu_tensor& a, const dfgpu_tensor& b, const dfgpu_tensor& 
 // Few rows take little of a stage, so that more stages fit. (A product still reads 128 rows: ring_bytes() keeps the last
 // stage's inside the allocation.)
 int rows_of_a(const Problem& p, int cg) { return cg == 1 && p.M < kRows ? static_cast<int>((p.M + 7) / 8 * 8) : kRows; }
-int stage_bytes(const Problem& p, int bn, int cg, int a_rows) { return (a_rows + bn / cg) * kRowBytes * (p.kind == kPieces ? 3 : 1) + (p.kind == kScaled ? 2048 : 0); }
+bool scaled(const Problem& p) { return p.kind == kScaled || p.kind == kScaledSummed; }
+int stage_bytes(const Problem& p, int bn, int cg, int a_rows) { return (a_rows + bn / cg) * kRowBytes * (p.kind == kPieces ? 3 : 1) + (scaled(p) ? 2048 : 0); }
 bool sixteen_bits(const Problem& p) { return p.kind == kSixteen || p.kind == kPieces || p.kind == kSummed; }
 int ring_bytes(int stages, int stage_size) { return (stages - 1) * stage_size + std::max(stage_size, kABytes); }
 int stages_that_fit(int stage_size, int budget) {
@@ -902,9 +950,9 @@ Shape choose_shape(const Problem& p) {
             const int chunk = sixteen_bits(p) ? 64 : 128;   // columns of one N-major copy
             if (p.b_mn_major && (bn / cg) % chunk != 0) continue;
             if (p.out_dtype == DFGPU_E4M3 && bn % 128 != 0) continue;   // (whole 128-byte boxes)
-            if (p.kind == kScaled && bn % 128 != 0) continue;           // (whole chunks of column scales)
+            if (scaled(p) && bn % 128 != 0) continue;           // (whole chunks of column scales)
             if (cg == 2 && bn < 128) continue;
-            if (p.kind == kSummed && bn > 128) continue;                // (a row's sums live in registers)
+            if ((p.kind == kSummed || p.kind == kScaledSummed) && bn > 128) continue;   // (a row's sums live in registers, or beside two accumulators)
             if (bn > chunk && bn >= 2 * ((p.N + 63) / 64 * 64)) continue;  // (half the tile would be empty)
             const int64_t m_tiles = (p.M + kRows * cg - 1) / (kRows * cg), n_tiles = (p.N + bn - 1) / bn, tiles = m_tiles * n_tiles;
             const int rows = rows_of_a(p, cg), stage_size = stage_bytes(p, bn, cg, rows);
@@ -917,16 +965,16 @@ Shape choose_shape(const Problem& p) {
                 double rounds = static_cast<double>((tiles + slots - 1) / slots);
                 int64_t halved = 0;
                 const int half = bn / 2;
-                const bool halves = splits == 1 && half / cg >= 64 && (!p.b_mn_major || half / cg % chunk == 0) && half % (p.kind == kScaled || p.out_dtype == DFGPU_E4M3 ? 128 : 64) == 0;
+                const bool halves = splits == 1 && half / cg >= 64 && (!p.b_mn_major || half / cg % chunk == 0) && half % (scaled(p) || p.out_dtype == DFGPU_E4M3 ? 128 : 64) == 0;
                 if (halves && tiles > slots && tiles % slots != 0 && 2 * (tiles % slots) <= slots) {
                     halved = tiles % slots;
                     rounds -= 0.45;
                 }
                 const double in_flight = static_cast<double>(stages_that_fit(stage_size, kSmemBudget - 2 * kStageBox)) * stage_size;
                 const double products = p.kind == kPieces ? 6.0 : 1.0, pieces = p.kind == kPieces ? 3.0 : 1.0;
-                const double summed = p.kind == kSummed ? 150.0 + 2.0 * bn : 0.0;   // the epilogue's loads and additions of a block
+                const double summed = p.kind == kSummed ? 150.0 + 2.0 * bn : (p.kind == kScaledSummed ? 250.0 + 3.0 * bn : 0.0);   // the epilogue's loads and additions of a block
                 const double block = std::max({summed, products * 2.0 * bn, (products + pieces) * (rows + bn / cg), pieces * (rows + bn / cg) * kRowBytes / std::min(48.0, in_flight / 2300.0)});
-                const double clocks = rounds * (k_per_split * block) + 2000.0 + bn * 6.0 + (splits > 1 ? (p.kind == kScaled ? 5000.0 : 2500.0) : 0.0) + (cg == 2 ? 1500.0 : 0.0);
+                const double clocks = rounds * (k_per_split * block) + 2000.0 + bn * 6.0 + (splits > 1 ? (scaled(p) ? 5000.0 : 2500.0) : 0.0) + (cg == 2 ? 1500.0 : 0.0);
                 if (best.cg == 0 || clocks < best.clocks) best = Shape{cg, bn, splits, static_cast<int>(k_per_split), tiles, halved, clocks};
             }
         }
@@ -985,7 +1033,7 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     args.barrier_offset = args.staging_offset + staging;
     const int dynamic = args.barrier_offset + barriers + 1024;
     // instruction descriptor: f32 accumulators (or E8M0 scales), the operand formats the caller has set, B's major, M (N is the item's)
-    args.idesc |= (p.kind == kScaled ? 1u << 23 : 1u << 4) | (static_cast<uint32_t>(args.b_mn_major) << 16) |
+    args.idesc |= (scaled(p) ? 1u << 23 : 1u << 4) | (static_cast<uint32_t>(args.b_mn_major) << 16) |
                   (static_cast<uint32_t>(kRows * shape.cg >> 4) << 24);
     const CUtensorMapDataType in_type = sixteen_bits(p) ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;   // (copied, never computed on)
     const uint32_t per_row = kRowBytes / p.in_bytes;
@@ -1006,6 +1054,7 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     if (p.kind == kCodes) return shape.cg == 2 ? launch_kernel<kCodes, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kCodes, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     if (p.kind == kSummed) return shape.cg == 2 ? launch_kernel<kSummed, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kSummed, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     if (p.kind == kPieces) return shape.cg == 2 ? launch_kernel<kPieces, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kPieces, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
+    if (p.kind == kScaledSummed) return shape.cg == 2 ? launch_kernel<kScaledSummed, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kScaledSummed, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     return shape.cg == 2 ? launch_kernel<kScaled, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kScaled, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
 }
 
@@ -1044,17 +1093,21 @@ bool translate_steps(const dfgpu_matmul_params& p, void* const* tensors, TileArg
     return true;
 }
 
-// f32 results that are summed block by block (kSummed): all but those of whole bf16 tiles in whole 16-byte units, which always
-// came from one accumulator.
+// f32 results that are summed block by block: all but those of whole tiles in whole 16-byte units, which always came from one
+// accumulator.
 bool sums_blocks(const dfgpu_matmul_params& p) {
     const int rank = p.c.rank;
     if (p.c.dtype != DFGPU_F32 || rank < 2 || p.a.rank != rank) return false;
-    if (p.a.dtype != DFGPU_BF16 || p.a.dim[rank - 1] % 64 != 0 || p.c.dim[rank - 1] % 64 != 0 || p.a.stride[rank - 2] % 8 != 0 || p.c.stride[rank - 2] % 8 != 0) return true;
-    for (int i = 0; i < p.epilogue_count; ++i) {
-        if (p.epilogue[i].op != DFGPU_EPI_ADD) continue;
+    const bool has_scales = p.a.dtype == DFGPU_E4M3;
+    const int64_t M = p.c.dim[rank - 2], N = p.c.dim[rank - 1], K = p.a.dim[rank - 1], tile = has_scales ? 128 : 64;
+    if (p.a.dtype == DFGPU_F16 || K % tile != 0 || N % tile != 0 || p.a.stride[rank - 2] % 8 != 0 || p.c.stride[rank - 2] % 8 != 0) return true;
+    if (has_scales && (M % 128 != 0 || p.a_scale.stride[rank - 2] % 4 != 0)) return true;
+    for (int i = 0; i < std::min<int>(p.epilogue_count, kMaxSteps); ++i) {
+        if (p.epilogue[i].op != DFGPU_EPI_ADD || p.epilogue[i].operand < 0 || p.epilogue[i].operand > 1) continue;   // (translate_steps() refuses those)
         const dfgpu_tensor& t = p.extra[p.epilogue[i].operand];
+        if (t.rank < 1) continue;
         const bool per_column = t.rank == 1 || t.dim[t.rank - 2] == 1;
-        if (t.dtype == DFGPU_F16 || (!per_column && (t.rank != rank || t.stride[rank - 2] != p.c.stride[rank - 2]))) return true;
+        if (t.dtype == DFGPU_F16 || (!has_scales && !per_column && (t.rank != rank || t.stride[rank - 2] != p.c.stride[rank - 2]))) return true;
     }
     return false;
 }
@@ -1074,6 +1127,7 @@ bool scaled_problem(const dfgpu_matmul_params& p, Problem& problem) {
     if (p.c.dtype != DFGPU_BF16 && p.c.dtype != DFGPU_F16 && p.c.dtype != DFGPU_F32) return false;
     const int rank = p.c.rank;
     if (p.a_scale.rank != rank || p.b_scale.rank != rank || !describe(p.a, p.b, p.c, kScaled, problem)) return false;
+    if (sums_blocks(p)) problem.kind = kScaledSummed;
     for (int i = 0; i < rank - 2; ++i)
         if (p.a_scale.dim[i] != 1 || p.b_scale.dim[i] != 1) return false;
     if (problem.N <= 64) return false;   // (column scales come in chunks of 128: half of a tile would be empty; dequantized to bf16, N = 64 is a tile)

@@ -124,3 +124,18 @@ def test_f32_results_do_not_lose_accuracy_with_depth(m, k, n, c_ld, io, b_k_majo
     want = a.view(m, k).double() @ b.double()
     error = (buffers[4].view(m, c_ld)[:, :n].double() - want).norm() / want.norm()
     assert float(error) <= 2.0 ** -21 + 2.0 ** -25 * (k / 64) ** 0.5
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 32, 80), (77, 288, 272), (300, 544, 528), (129, 4128, 144), (2050, 288, 2064), (1026, 32736, 1040)])
+def test_f32_results_of_block_scaled_codes_do_not_lose_accuracy_with_depth(m, k, n):
+    """As above with blocks of 128 codes, whose products hold eight significant bits: half the bound of a block."""
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    buffers = {1: torch.randn(m * k, device="cuda", generator=g).to(torch.bfloat16), 2: torch.randn(k * n, device="cuda", generator=g).to(torch.bfloat16)}
+    exe = run(graphs.c3_quantize_matmul(m, k, n, c_type="FLOAT"), buffers)
+    assert [s["kernel"] for s in exe.steps()][-1] == dfgpu.MATMUL_UMMA_MXF8
+    scale = lambda uid: torch.pow(2.0, buffers[uid].double() - 127)
+    a = buffers[3].view(torch.float8_e4m3fn).double().view(m, k) * scale(4).view(m, k // 32).repeat_interleave(32, 1)
+    b = buffers[5].view(torch.float8_e4m3fn).double().view(k, n) * scale(6).view(k // 32, n).repeat_interleave(32, 0)
+    want = a @ b
+    error = (buffers[9].view(m, n).double() - want).norm() / want.norm()
+    assert float(error) <= 2.0 ** -22 + 2.0 ** -25 * (k / 128) ** 0.5
