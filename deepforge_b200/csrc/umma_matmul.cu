@@ -10,7 +10,7 @@
 // 2050 x 8184 x 1040 bf16 to f32 is 9.1e-6 from 64 bits in one accumulator, 9.6e-7 by the CUDA cores' additions, 2.2e-7 this way. The
 // forms that ran there (or in the one-launch f32 kernel) keep an accuracy no worse than theirs. The epilogue's two loads and 64
 // additions a block set the pace: 4096 x 4104 x 4104 124 us in one accumulator, 234 this way, 9227 on the CUDA cores.
-// kScaledSummed: the same for block-scaled codes (1026 x 8160 x 1040 to f32: 1.2e-7 on the CUDA cores, 4.7e-7 in one accumulator).
+// kCodesSummed: the same for FP8 codes. kScaledSummed: for block-scaled codes (1026 x 8160 x 1040 to f32: 1.2e-7 on the CUDA cores, 4.7e-7 in one accumulator).
 //
 // Extents are free because the copies are: TMA fills what lies outside a matrix with zeros and clips what would be stored
 // there, so a tile may hang over any edge. Only the rows' starts have to fall on 16-byte boundaries.
@@ -45,9 +45,10 @@ constexpr int kMaxStages = 16;
 constexpr int kMaxSteps = DFGPU_MAX_EPILOGUE;
 constexpr int kSmemBudget = 227 * 1024 - 1024;   // (1 KB of slack aligns the tiles)
 
-enum Kind { kSixteen = 0, kCodes = 1, kScaled = 2, kPieces = 3, kSummed = 4, kScaledSummed = 5 };
+enum Kind { kSixteen = 0, kCodes = 1, kScaled = 2, kPieces = 3, kSummed = 4, kScaledSummed = 5, kCodesSummed = 6 };
 template <int KIND> constexpr bool kHasScales = KIND == kScaled || KIND == kScaledSummed;
-template <int KIND> constexpr bool kInBlocks = KIND == kSummed || KIND == kScaledSummed;   // an accumulator per K block, summed by the epilogue
+template <int KIND> constexpr bool kInRegisters = KIND == kSummed || KIND == kCodesSummed;
+template <int KIND> constexpr bool kInBlocks = kInRegisters<KIND> || KIND == kScaledSummed;   // an accumulator per K block, summed by the epilogue
 enum { kStepRelu = 1, kStepBias = 2, kStepFull = 3 };
 
 struct TileArgs {
@@ -151,8 +152,8 @@ __device__ __forceinline__ void product(uint32_t d, uint64_t a, uint64_t b, uint
     constexpr bool sixteen = KIND == kSixteen || KIND == kPieces || KIND == kSummed;
     if constexpr (sixteen && CG == 1) DFGPU_MMA("cta_group::1.kind::f16");
     if constexpr (sixteen && CG == 2) DFGPU_MMA("cta_group::2.kind::f16");
-    if constexpr (KIND == kCodes && CG == 1) DFGPU_MMA("cta_group::1.kind::f8f6f4");
-    if constexpr (KIND == kCodes && CG == 2) DFGPU_MMA("cta_group::2.kind::f8f6f4");
+    if constexpr ((KIND == kCodes || KIND == kCodesSummed) && CG == 1) DFGPU_MMA("cta_group::1.kind::f8f6f4");
+    if constexpr ((KIND == kCodes || KIND == kCodesSummed) && CG == 2) DFGPU_MMA("cta_group::2.kind::f8f6f4");
 #undef DFGPU_MMA
 #define DFGPU_MMA(FORM)                                                                                                   \
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma." FORM ".kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}" \
@@ -316,7 +317,7 @@ __device__ __forceinline__ void tmem_put_32(uint32_t address, const uint32_t (&r
     asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
                  ::"r"(address), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
 }
-// kSummed: this thread's row of a tile, the boxes g and g + 2 of 32 columns, summed over the K blocks of the walk. `local` counts
+// kSummed, kCodesSummed: this thread's row of a tile, the boxes g and g + 2 of 32 columns, summed over the K blocks of the walk. `local` counts
 // accumulators, as the issuing warp does; one is handed back as soon as it is in registers.
 template <int CG>
 __device__ __forceinline__ void sum_blocks(float (&sums)[2][32], uint32_t columns, int acc_stride, int boxes, int g, int blocks, int& local, uint32_t acc_full, uint32_t acc_empty,
@@ -465,7 +466,7 @@ template <int KIND, int CG>
 __global__ void __launch_bounds__(thread_count<KIND>(), 1)
 umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c,
                    const __grid_constant__ TileArgs args) {
-    constexpr int kCode = KIND == kSixteen ? 0 : (KIND == kCodes ? 20 : (KIND == kScaled ? 40 : (KIND == kPieces ? 60 : (KIND == kSummed ? 80 : 90))));
+    constexpr int kCode = KIND == kSixteen ? 0 : (KIND == kCodes || KIND == kCodesSummed ? 20 : (KIND == kScaled ? 40 : (KIND == kPieces ? 60 : (KIND == kSummed ? 80 : 90))));
     constexpr bool kSixteenBits = KIND == kSixteen || KIND == kPieces || KIND == kSummed;
     constexpr int kPieceCount = KIND == kPieces ? 3 : 1;
     extern __shared__ uint8_t smem_raw[];
@@ -627,10 +628,10 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const int quadrant = warp & 3, g = (warp - 4) >> 2, row = quadrant * 32 + lane;
         const uint32_t lane_base = static_cast<uint32_t>(quadrant * 32) << 16;
         bool ok = true;
-        float sums[2][32];   // (kSummed)
+        float sums[2][32];   // (kInRegisters)
         if (split) {
             // park the f32 partial tile where the operands were: rows of bn floats, 16-byte units swizzled by the row
-            if constexpr (KIND == kSummed) {
+            if constexpr (kInRegisters<KIND>) {
                 int local = 0;
                 sum_blocks<CG>(sums, tmem_base + lane_base, args.acc_stride, bn / 32, g, kb_end - kb_begin, local, acc_full(0), acc_empty(0), lane, ok);
             } else if constexpr (KIND == kScaledSummed) {
@@ -643,7 +644,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             uint8_t* parked = generic_base + row * bn * 4;
             for (int c = g; c < bn / 32; c += 2) {
                 uint32_t raw[32];
-                if constexpr (KIND == kSummed) {
+                if constexpr (kInRegisters<KIND>) {
 #pragma unroll
                     for (int e = 0; e < 32; ++e) {
                         raw[e] = __float_as_uint(sums[0][e]);
@@ -671,7 +672,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 const Item item = item_at(args, i);
                 const int row0 = (item.m_tile * CG + (CG == 2 ? rank : 0)) * kRows, out_row = row0 + row;
                 const bool row_live = out_row < args.m_total;
-                if constexpr (KIND == kSummed) {
+                if constexpr (kInRegisters<KIND>) {
                     sum_blocks<CG>(sums, tmem_base + lane_base, args.acc_stride, item.width / 32, g, kb_end - kb_begin, local, acc_full(0), leader_bars + (acc_empty(0) - bar_base), lane, ok);
                 } else if constexpr (KIND == kScaledSummed) {
                     sum_blocks_in_place<CG>(tmem_base + lane_base, args.acc_stride, item.width / 32, g, kb_end - kb_begin, local, acc_full(0), leader_bars + (acc_empty(0) - bar_base), lane, ok);
@@ -692,7 +693,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     }
                     for (int part = 0; part < box_columns / 32; ++part) {
                         uint32_t raw[32];
-                        if constexpr (KIND == kSummed) {   // (f32 C: boxes of 32 columns)
+                        if constexpr (kInRegisters<KIND>) {   // (f32 C: boxes of 32 columns)
 #pragma unroll
                             for (int e = 0; e < 32; ++e) {
                                 raw[e] = __float_as_uint(sums[0][e]);
@@ -916,6 +917,7 @@ bool describe(const dfgpu_tensor& a, const dfgpu_tensor& b, const dfgpu_tensor& 
 // Few rows take little of a stage, so that more stages fit. (A product still reads 128 rows: ring_bytes() keeps the last
 // stage's inside the allocation.)
 int rows_of_a(const Problem& p, int cg) { return cg == 1 && p.M < kRows ? static_cast<int>((p.M + 7) / 8 * 8) : kRows; }
+bool in_registers(const Problem& p) { return p.kind == kSummed || p.kind == kCodesSummed; }
 bool scaled(const Problem& p) { return p.kind == kScaled || p.kind == kScaledSummed; }
 int stage_bytes(const Problem& p, int bn, int cg, int a_rows) { return (a_rows + bn / cg) * kRowBytes * (p.kind == kPieces ? 3 : 1) + (scaled(p) ? 2048 : 0); }
 bool sixteen_bits(const Problem& p) { return p.kind == kSixteen || p.kind == kPieces || p.kind == kSummed; }
@@ -952,7 +954,7 @@ Shape choose_shape(const Problem& p) {
             if (p.out_dtype == DFGPU_E4M3 && bn % 128 != 0) continue;   // (whole 128-byte boxes)
             if (scaled(p) && bn % 128 != 0) continue;           // (whole chunks of column scales)
             if (cg == 2 && bn < 128) continue;
-            if ((p.kind == kSummed || p.kind == kScaledSummed) && bn > 128) continue;   // (a row's sums live in registers, or beside two accumulators)
+            if ((in_registers(p) || p.kind == kScaledSummed) && bn > 128) continue;   // (a row's sums live in registers, or beside two accumulators)
             if (bn > chunk && bn >= 2 * ((p.N + 63) / 64 * 64)) continue;  // (half the tile would be empty)
             const int64_t m_tiles = (p.M + kRows * cg - 1) / (kRows * cg), n_tiles = (p.N + bn - 1) / bn, tiles = m_tiles * n_tiles;
             const int rows = rows_of_a(p, cg), stage_size = stage_bytes(p, bn, cg, rows);
@@ -972,7 +974,7 @@ Shape choose_shape(const Problem& p) {
                 }
                 const double in_flight = static_cast<double>(stages_that_fit(stage_size, kSmemBudget - 2 * kStageBox)) * stage_size;
                 const double products = p.kind == kPieces ? 6.0 : 1.0, pieces = p.kind == kPieces ? 3.0 : 1.0;
-                const double summed = p.kind == kSummed ? 150.0 + 2.0 * bn : (p.kind == kScaledSummed ? 250.0 + 3.0 * bn : 0.0);   // the epilogue's loads and additions of a block
+                const double summed = in_registers(p) ? 150.0 + 2.0 * bn : (p.kind == kScaledSummed ? 250.0 + 3.0 * bn : 0.0);   // the epilogue's loads and additions of a block
                 const double block = std::max({summed, products * 2.0 * bn, (products + pieces) * (rows + bn / cg), pieces * (rows + bn / cg) * kRowBytes / std::min(48.0, in_flight / 2300.0)});
                 const double clocks = rounds * (k_per_split * block) + 2000.0 + bn * 6.0 + (splits > 1 ? (scaled(p) ? 5000.0 : 2500.0) : 0.0) + (cg == 2 ? 1500.0 : 0.0);
                 if (best.cg == 0 || clocks < best.clocks) best = Shape{cg, bn, splits, static_cast<int>(k_per_split), tiles, halved, clocks};
@@ -1051,6 +1053,7 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     const int64_t groups = shape.splits > 1 ? shape.tiles : std::min<int64_t>(shape.tiles, sm_count() / shape.cg);
     const int grid = static_cast<int>(groups * (shape.cg == 2 ? 2 : shape.splits));
     if (p.kind == kSixteen) return shape.cg == 2 ? launch_kernel<kSixteen, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kSixteen, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
+    if (p.kind == kCodesSummed) return shape.cg == 2 ? launch_kernel<kCodesSummed, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kCodesSummed, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     if (p.kind == kCodes) return shape.cg == 2 ? launch_kernel<kCodes, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kCodes, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     if (p.kind == kSummed) return shape.cg == 2 ? launch_kernel<kSummed, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kSummed, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     if (p.kind == kPieces) return shape.cg == 2 ? launch_kernel<kPieces, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kPieces, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
@@ -1194,7 +1197,12 @@ int launch_matmul_umma(const dfgpu_matmul_params& p, void* const* tensors, int k
 bool fp8_problem(const dfgpu_matmul_fp8_params& p, Problem& problem) {
     if ((p.a.dtype != DFGPU_E4M3 && p.a.dtype != DFGPU_E5M2) || (p.b.dtype != DFGPU_E4M3 && p.b.dtype != DFGPU_E5M2)) return false;
     if (p.c.dtype != DFGPU_BF16 && p.c.dtype != DFGPU_F16 && p.c.dtype != DFGPU_F32 && p.c.dtype != DFGPU_E4M3 && p.c.dtype != DFGPU_E5M2) return false;
-    return describe(p.a, p.b, p.c, kCodes, problem);
+    if (!describe(p.a, p.b, p.c, kCodes, problem)) return false;
+    // f32 results, but for whole tiles in whole 16-byte units (which always came from one accumulator): the blocks summed in f32. Relative
+    // error at 2050 x 256 / 640 x 1040: 1.36 / 2.63e-8 by the CUDA cores' additions, 1.5 / 3.22e-8 in one accumulator, 1.27 / 2.2e-8 this way.
+    const bool whole = problem.M % 128 == 0 && problem.N % 128 == 0 && problem.K % 128 == 0 && problem.c_ld % 4 == 0;
+    if (p.c.dtype == DFGPU_F32 && !whole) problem.kind = kCodesSummed;
+    return true;
 }
 
 bool matmul_fp8_tiles_supported(const dfgpu_matmul_fp8_params& p) {
