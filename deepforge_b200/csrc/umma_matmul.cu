@@ -45,10 +45,12 @@ constexpr int kMaxStages = 16;
 constexpr int kMaxSteps = DFGPU_MAX_EPILOGUE;
 constexpr int kSmemBudget = 227 * 1024 - 1024;   // (1 KB of slack aligns the tiles)
 
-enum Kind { kSixteen = 0, kCodes = 1, kScaled = 2, kPieces = 3, kSummed = 4, kScaledSummed = 5, kCodesSummed = 6 };
+enum Kind { kSixteen = 0, kCodes = 1, kScaled = 2, kPieces = 3, kSummed = 4, kScaledSummed = 5, kCodesSummed = 6, kPiecesSummed = 7 };
 template <int KIND> constexpr bool kHasScales = KIND == kScaled || KIND == kScaledSummed;
 template <int KIND> constexpr bool kInRegisters = KIND == kSummed || KIND == kCodesSummed;
-template <int KIND> constexpr bool kInBlocks = kInRegisters<KIND> || KIND == kScaledSummed;   // an accumulator per K block, summed by the epilogue
+template <int KIND> constexpr bool kInPlace = KIND == kScaledSummed || KIND == kPiecesSummed;   // ... in tensor memory
+template <int KIND> constexpr bool kInBlocks = kInRegisters<KIND> || kInPlace<KIND>;
+template <int KIND> constexpr bool kHasPieces = KIND == kPieces || KIND == kPiecesSummed;   // an accumulator per K block, summed by the epilogue
 enum { kStepRelu = 1, kStepBias = 2, kStepFull = 3 };
 
 struct TileArgs {
@@ -58,6 +60,7 @@ struct TileArgs {
     int32_t whole_items, items;       // work items: whole tiles, and after them the halves of the tiles that are left for the last round
     int32_t splits, k_per_split;
     int32_t stages, stage_bytes;
+    int32_t blocks_per_sum, sums_column;             // kInBlocks: K blocks of an accumulator; kInPlace: tensor-memory column of the sums
     int32_t acc_stride, acc_shift, scale_columns;   // tensor memory: see launch_problem(); 1 << acc_shift accumulators
     int32_t a_bytes;                  // A of one CTA and stage; B lies behind it
     int32_t b_box_bytes, b_box_columns;   // B comes in boxes
@@ -149,7 +152,7 @@ __device__ __forceinline__ void product(uint32_t d, uint64_t a, uint64_t b, uint
 #define DFGPU_MMA(FORM)                                                                                                   \
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma." FORM " [%0], %1, %2, %3, p;\n\t}"          \
                  ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory")
-    constexpr bool sixteen = KIND == kSixteen || KIND == kPieces || KIND == kSummed;
+    constexpr bool sixteen = KIND == kSixteen || kHasPieces<KIND> || KIND == kSummed;
     if constexpr (sixteen && CG == 1) DFGPU_MMA("cta_group::1.kind::f16");
     if constexpr (sixteen && CG == 2) DFGPU_MMA("cta_group::2.kind::f16");
     if constexpr ((KIND == kCodes || KIND == kCodesSummed) && CG == 1) DFGPU_MMA("cta_group::1.kind::f8f6f4");
@@ -346,30 +349,24 @@ __device__ __forceinline__ void sum_blocks(float (&sums)[2][32], uint32_t column
     }
 }
 
-// kScaledSummed: the same with the sums in tensor memory, behind the two accumulators: its 16 warps leave too few registers.
-template <int CG>
-__device__ __forceinline__ void sum_blocks_in_place(uint32_t columns, int acc_stride, int boxes, int g, int blocks, int& local, uint32_t acc_full, uint32_t acc_empty, int lane, bool& ok) {
-    for (int block = 0; block < blocks; ++block, ++local) {
-        const int acc = local & 1;
-        if (ok) ok = mbar_wait_warp(acc_full + 8u * acc, (local >> 1) & 1, 595);
+// The same with the sums in tensor memory, behind the accumulators: kScaledSummed's 16 warps leave too few registers, and kPiecesSummed
+// adds the products of the lower pieces on the way.
+template <int KIND, int CG>
+__device__ __forceinline__ void sum_blocks_in_place(const TileArgs& args, uint32_t columns, int boxes, int g, int blocks, int& local, uint32_t acc_full, uint32_t acc_empty, int lane, bool& ok) {
+    for (int block = 0; block < blocks; block += args.blocks_per_sum, ++local) {
+        const int acc = local & args.acc_shift;
+        if (ok) ok = mbar_wait_warp(acc_full + 8u * acc, (local >> args.acc_shift) & 1, KIND == kPiecesSummed ? 565 : 595);
         tc_fence_after();
         for (int box = g; box < boxes; box += 2) {
+            const uint32_t own = columns + acc * args.acc_stride + box * 32, target = columns + args.sums_column + box * 32;
             uint32_t raw[32];
-            tmem_load_32(columns + acc * acc_stride + box * 32, raw);
-            if (block > 0) {
-                uint32_t sum[32];
-                tmem_load_32(columns + 2 * acc_stride + box * 32, sum);
-                tmem_load_wait();
+            tmem_load_32(own, raw);
+            tmem_load_wait();
 #pragma unroll
-                for (int e = 0; e < 32; ++e) asm volatile("" : "+r"(raw[e]), "+r"(sum[e]));   // (no use above the wait)
-#pragma unroll
-                for (int e = 0; e < 32; ++e) raw[e] = __float_as_uint(__fadd_rn(__uint_as_float(sum[e]), __uint_as_float(raw[e])));
-            } else {
-                tmem_load_wait();
-#pragma unroll
-                for (int e = 0; e < 32; ++e) asm volatile("" : "+r"(raw[e]));
-            }
-            tmem_put_32(columns + 2 * acc_stride + box * 32, raw);
+            for (int e = 0; e < 32; ++e) asm volatile("" : "+r"(raw[e]));   // (no use above the wait)
+            if constexpr (KIND == kPiecesSummed) add_small_products(own + args.bn, raw);
+            if (block > 0) add_small_products(target, raw);   // (the sum so far)
+            tmem_put_32(target, raw);
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         tc_fence_before();
@@ -466,9 +463,9 @@ template <int KIND, int CG>
 __global__ void __launch_bounds__(thread_count<KIND>(), 1)
 umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c,
                    const __grid_constant__ TileArgs args) {
-    constexpr int kCode = KIND == kSixteen ? 0 : (KIND == kCodes || KIND == kCodesSummed ? 20 : (KIND == kScaled ? 40 : (KIND == kPieces ? 60 : (KIND == kSummed ? 80 : 90))));
-    constexpr bool kSixteenBits = KIND == kSixteen || KIND == kPieces || KIND == kSummed;
-    constexpr int kPieceCount = KIND == kPieces ? 3 : 1;
+    constexpr int kCode = KIND == kSixteen ? 0 : (KIND == kCodes || KIND == kCodesSummed ? 20 : (KIND == kScaled ? 40 : (kHasPieces<KIND> ? 60 : (KIND == kSummed ? 80 : 90))));
+    constexpr bool kSixteenBits = KIND == kSixteen || kHasPieces<KIND> || KIND == kSummed;
+    constexpr int kPieceCount = kHasPieces<KIND> ? 3 : 1;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* generic_base = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -571,14 +568,14 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 if (overlapped && ok && local > 0) ok = mbar_wait_warp(overlap_free, (local - 1) & 1, 507 + kCode);
                 tc_fence_after();
                 uint32_t d = tmem_u + acc * args.acc_stride;
+                int in_sum = 0;
                 for (int kb = kb_begin; kb < kb_end && ok; ++kb) {
-                    const int block_acc = local & 1;
-                    if constexpr (kInBlocks<KIND>) {   // (an accumulator per block)
-                        ok = wait_warp<CG == 2>(acc_empty(block_acc), ((local >> 1) & 1) ^ 1, 502 + kCode);
+                    const int block_acc = local & args.acc_shift;
+                    if (kInBlocks<KIND> && in_sum == 0) {   // (an accumulator per blocks_per_sum blocks)
+                        ok = wait_warp<CG == 2>(acc_empty(block_acc), ((local >> args.acc_shift) & 1) ^ 1, 502 + kCode);
                         if (!ok) break;
                         tc_fence_after();
                         d = tmem_u + block_acc * args.acc_stride;
-                        ++local;
                     }
                     ok = mbar_wait_warp(full_bar(stage), phase, 503 + kCode);
                     if (!ok) break;   // (operands by TMA, scales by generic stores + fence.proxy.async: no tcgen05 fence needed)
@@ -593,7 +590,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                             copy_scales<CG>(sf + 4, scales + 512);
                             if (width > 128) copy_scales<CG>(sf + 8, scales + 1024);
                         }
-                        if constexpr (KIND == kPieces) {
+                        if constexpr (kHasPieces<KIND>) {
                             // middle*middle, low*high, high*low, middle*high, high*middle meet in an accumulator of their own: the tensor
                             // cores cut off what a sum does not hold, and beside high*high (2^8 times larger) every one of them would lose as much as it does.
                             constexpr int piece_a[6] = {1, 2, 0, 1, 0, 0}, piece_b[6] = {1, 0, 2, 0, 1, 0};
@@ -604,17 +601,21 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                                 for (int j = 0; j < 4; ++j)
                                     product<KIND, CG>(pair == 5 ? d : d + bn, desc_words(a_lo + piece_a[pair] * a_piece + ((j * 32) >> 4), smem_desc_hi(1024)),
                                                       desc_words(b_lo + piece_b[pair] * b_piece + j * b_step, smem_desc_hi(1024)), idesc_wide,
-                                                      kb != kb_begin || j != 0 || (pair != 0 && pair != 5) ? 1u : 0u, 0u, 0u);
+                                                      (kInBlocks<KIND> ? in_sum != 0 : kb != kb_begin) || j != 0 || (pair != 0 && pair != 5) ? 1u : 0u, 0u, 0u);
                         } else
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             uint32_t idesc = idesc_wide;
                             if constexpr (kHasScales<KIND>) idesc |= (static_cast<uint32_t>(j) << 29) | (static_cast<uint32_t>(j) << 4);   // the K block's byte of the scale words
                             product<KIND, CG>(d, desc_words(a_lo + ((j * 32) >> 4), smem_desc_hi(1024)), desc_words(b_lo + j * b_step, smem_desc_hi(1024)), idesc,
-                                              (!kInBlocks<KIND> && kb != kb_begin) || j != 0 ? 1u : 0u, sf, sf + 4);
+                                              (kInBlocks<KIND> ? in_sum != 0 : kb != kb_begin) || j != 0 ? 1u : 0u, sf, sf + 4);
                         }
                         commit_to_all<CG>(empty_bar(stage));
-                        if constexpr (kInBlocks<KIND>) commit_to_all<CG>(acc_full(block_acc));
+                        if (kInBlocks<KIND> && (in_sum + 1 == args.blocks_per_sum || kb + 1 == kb_end)) commit_to_all<CG>(acc_full(block_acc));
+                    }
+                    if (kInBlocks<KIND> && (++in_sum == args.blocks_per_sum || kb + 1 == kb_end)) {
+                        in_sum = 0;
+                        ++local;
                     }
                     __syncwarp();
                     if (++stage == args.stages) { stage = 0; phase ^= 1; }
@@ -634,9 +635,9 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             if constexpr (kInRegisters<KIND>) {
                 int local = 0;
                 sum_blocks<CG>(sums, tmem_base + lane_base, args.acc_stride, bn / 32, g, kb_end - kb_begin, local, acc_full(0), acc_empty(0), lane, ok);
-            } else if constexpr (KIND == kScaledSummed) {
+            } else if constexpr (kInPlace<KIND>) {
                 int local = 0;
-                sum_blocks_in_place<CG>(tmem_base + lane_base, args.acc_stride, bn / 32, g, kb_end - kb_begin, local, acc_full(0), acc_empty(0), lane, ok);
+                sum_blocks_in_place<KIND, CG>(args, tmem_base + lane_base, bn / 32, g, kb_end - kb_begin, local, acc_full(0), acc_empty(0), lane, ok);
             } else {
                 ok = mbar_wait(acc_full(0), 0, 504 + kCode);
                 tc_fence_after();
@@ -651,7 +652,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         sums[0][e] = sums[1][e];
                     }
                 } else {
-                    tmem_load_32(tmem_base + lane_base + (KIND == kScaledSummed ? 2 * args.acc_stride : 0) + c * 32, raw);
+                    tmem_load_32(tmem_base + lane_base + (kInPlace<KIND> ? args.sums_column : 0) + c * 32, raw);
                     tmem_load_wait();
                 }
                 if constexpr (KIND == kPieces) add_small_products(tmem_base + lane_base + bn + c * 32, raw);
@@ -674,14 +675,14 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 const bool row_live = out_row < args.m_total;
                 if constexpr (kInRegisters<KIND>) {
                     sum_blocks<CG>(sums, tmem_base + lane_base, args.acc_stride, item.width / 32, g, kb_end - kb_begin, local, acc_full(0), leader_bars + (acc_empty(0) - bar_base), lane, ok);
-                } else if constexpr (KIND == kScaledSummed) {
-                    sum_blocks_in_place<CG>(tmem_base + lane_base, args.acc_stride, item.width / 32, g, kb_end - kb_begin, local, acc_full(0), leader_bars + (acc_empty(0) - bar_base), lane, ok);
+                } else if constexpr (kInPlace<KIND>) {
+                    sum_blocks_in_place<KIND, CG>(args, tmem_base + lane_base, item.width / 32, g, kb_end - kb_begin, local, acc_full(0), leader_bars + (acc_empty(0) - bar_base), lane, ok);
                 } else {
                     if (ok) ok = mbar_wait(acc_full(acc), use & 1, 505 + kCode);
                     tc_fence_after();
                 }
                 const bool healthy = ok && g_device_status == 0;
-                const uint32_t columns = tmem_base + lane_base + (KIND == kScaledSummed ? 2 : acc) * args.acc_stride;
+                const uint32_t columns = tmem_base + lane_base + (kInPlace<KIND> ? args.sums_column : acc * args.acc_stride);
                 const int boxes = item.width / box_columns;
                 for (int b = g; b < boxes; b += 2) {
                     // overlapping accumulators: the first one is read from its end, the second from its start
@@ -917,10 +918,11 @@ bool describe(const dfgpu_tensor& a, const dfgpu_tensor& b, const dfgpu_tensor& 
 // Few rows take little of a stage, so that more stages fit. (A product still reads 128 rows: ring_bytes() keeps the last
 // stage's inside the allocation.)
 int rows_of_a(const Problem& p, int cg) { return cg == 1 && p.M < kRows ? static_cast<int>((p.M + 7) / 8 * 8) : kRows; }
+bool has_pieces(const Problem& p) { return p.kind == kPieces || p.kind == kPiecesSummed; }
 bool in_registers(const Problem& p) { return p.kind == kSummed || p.kind == kCodesSummed; }
 bool scaled(const Problem& p) { return p.kind == kScaled || p.kind == kScaledSummed; }
-int stage_bytes(const Problem& p, int bn, int cg, int a_rows) { return (a_rows + bn / cg) * kRowBytes * (p.kind == kPieces ? 3 : 1) + (scaled(p) ? 2048 : 0); }
-bool sixteen_bits(const Problem& p) { return p.kind == kSixteen || p.kind == kPieces || p.kind == kSummed; }
+int stage_bytes(const Problem& p, int bn, int cg, int a_rows) { return (a_rows + bn / cg) * kRowBytes * (has_pieces(p) ? 3 : 1) + (scaled(p) ? 2048 : 0); }
+bool sixteen_bits(const Problem& p) { return p.kind == kSixteen || has_pieces(p) || p.kind == kSummed; }
 int ring_bytes(int stages, int stage_size) { return (stages - 1) * stage_size + std::max(stage_size, kABytes); }
 int stages_that_fit(int stage_size, int budget) {
     int stages = std::min(kMaxStages, budget / stage_size);
@@ -954,7 +956,7 @@ Shape choose_shape(const Problem& p) {
             if (p.out_dtype == DFGPU_E4M3 && bn % 128 != 0) continue;   // (whole 128-byte boxes)
             if (scaled(p) && bn % 128 != 0) continue;           // (whole chunks of column scales)
             if (cg == 2 && bn < 128) continue;
-            if ((in_registers(p) || p.kind == kScaledSummed) && bn > 128) continue;   // (a row's sums live in registers, or beside two accumulators)
+            if ((in_registers(p) || p.kind == kScaledSummed || p.kind == kPiecesSummed) && bn > 128) continue;   // (a row's sums live in registers, or beside two accumulators)
             if (bn > chunk && bn >= 2 * ((p.N + 63) / 64 * 64)) continue;  // (half the tile would be empty)
             const int64_t m_tiles = (p.M + kRows * cg - 1) / (kRows * cg), n_tiles = (p.N + bn - 1) / bn, tiles = m_tiles * n_tiles;
             const int rows = rows_of_a(p, cg), stage_size = stage_bytes(p, bn, cg, rows);
@@ -973,7 +975,7 @@ Shape choose_shape(const Problem& p) {
                     rounds -= 0.45;
                 }
                 const double in_flight = static_cast<double>(stages_that_fit(stage_size, kSmemBudget - 2 * kStageBox)) * stage_size;
-                const double products = p.kind == kPieces ? 6.0 : 1.0, pieces = p.kind == kPieces ? 3.0 : 1.0;
+                const double products = has_pieces(p) ? 6.0 : 1.0, pieces = has_pieces(p) ? 3.0 : 1.0;
                 const double summed = in_registers(p) ? 150.0 + 2.0 * bn : (p.kind == kScaledSummed ? 250.0 + 3.0 * bn : 0.0);   // the epilogue's loads and additions of a block
                 const double block = std::max({summed, products * 2.0 * bn, (products + pieces) * (rows + bn / cg), pieces * (rows + bn / cg) * kRowBytes / std::min(48.0, in_flight / 2300.0)});
                 const double clocks = rounds * (k_per_split * block) + 2000.0 + bn * 6.0 + (splits > 1 ? (scaled(p) ? 5000.0 : 2500.0) : 0.0) + (cg == 2 ? 1500.0 : 0.0);
@@ -1026,8 +1028,12 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     // overlap by 32 columns, which the epilogue reads out first.
     // Pieces: an accumulator is two of bn columns (leading and lower products), so that 192 and 256 columns leave room for one: the
     // epilogue of a tile then runs alone, a few percent of its 6 x K / 64 product steps.
-    args.acc_stride = p.kind == kScaled && shape.bn == 256 ? 224 : (p.kind == kPieces ? 2 * shape.bn : shape.bn);
-    args.acc_shift = p.kind == kPieces && shape.bn > 128 ? 0 : 1;
+    args.acc_stride = p.kind == kScaled && shape.bn == 256 ? 224 : (has_pieces(p) ? 2 * shape.bn : shape.bn);
+    args.acc_shift = (has_pieces(p) && shape.bn > 128) || p.kind == kPiecesSummed ? 0 : 1;
+    // (kPiecesSummed: one accumulator of 2 bn columns and the sums behind it; eight blocks each, whose error is half that of f32 additions over
+    // 4096 products, so that reading them out costs little)
+    args.blocks_per_sum = p.kind == kPiecesSummed ? 8 : 1;
+    args.sums_column = (args.acc_shift + 1) * args.acc_stride;
     args.scale_columns = 480;
     const int staging = shape.splits > 1 || !args.tma_store ? 0 : 2 * kStageBox, barriers = (2 * kMaxStages + 6) * 8;
     args.stages = stages_that_fit(args.stage_bytes, kSmemBudget - staging - barriers);
@@ -1056,7 +1062,8 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     if (p.kind == kCodesSummed) return shape.cg == 2 ? launch_kernel<kCodesSummed, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kCodesSummed, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     if (p.kind == kCodes) return shape.cg == 2 ? launch_kernel<kCodes, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kCodes, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     if (p.kind == kSummed) return shape.cg == 2 ? launch_kernel<kSummed, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kSummed, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
-    if (p.kind == kPieces) return shape.cg == 2 ? launch_kernel<kPieces, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kPieces, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
+    if (p.kind == kPiecesSummed) return shape.cg == 2 ? launch_kernel<kPiecesSummed, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kPiecesSummed, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
+    if (has_pieces(p)) return shape.cg == 2 ? launch_kernel<kPieces, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kPieces, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     if (p.kind == kScaledSummed) return shape.cg == 2 ? launch_kernel<kScaledSummed, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kScaledSummed, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
     return shape.cg == 2 ? launch_kernel<kScaled, 2>(map_a, map_b, map_c, args, grid, dynamic, stream, what) : launch_kernel<kScaled, 1>(map_a, map_b, map_c, args, grid, dynamic, stream, what);
 }
@@ -1158,10 +1165,11 @@ bool matmul_pieces_supported(const dfgpu_matmul_params& p) {
 int launch_matmul_pieces(const dfgpu_matmul_params& p, const PieceMatmul& pieces, void* const* tensors, cudaStream_t stream) {
     const int rank = p.c.rank;
     Problem problem{};
-    problem.kind = kPieces;
     problem.M = p.c.dim[rank - 2], problem.N = p.c.dim[rank - 1], problem.K = p.a.dim[rank - 1];
     problem.a_ld = pieces.a_ld, problem.b_ld = pieces.b_ld, problem.c_ld = p.c.stride[rank - 2];
     problem.b_mn_major = pieces.b_n_major;
+    // depths beyond the one-launch f32 kernel's, which the CUDA cores summed unless the extents were whole tiles: no further from 64 bits
+    problem.kind = problem.K > 4096 && (problem.K % 64 != 0 || problem.N % 64 != 0) ? kPiecesSummed : kPieces;
     problem.in_bytes = 2, problem.out_bytes = dtype_bytes(p.c.dtype), problem.out_dtype = p.c.dtype;
     problem.a_rows = 3 * problem.M;
     problem.b_rows = 3 * (pieces.b_n_major ? problem.K : problem.N);

@@ -159,3 +159,22 @@ def test_f32_results_of_codes_are_as_exact_as_f32_additions(m, k, n, b_k_major):
         errors.append(float((buffers[26].view(m, n).double() - want).norm() / want.norm()))
         assert float(buffers[27]) == float(buffers[26].abs().max())
     assert errors[0] <= 1.02 * errors[1] + (1e-9 if m * n < 4096 else 0.0)
+
+
+@pytest.mark.parametrize("m,k,n", [(20, 4104, 136), (300, 4160, 520), (1030, 4104, 1040), (2050, 8184, 1040)])
+@pytest.mark.parametrize("b_k_major", [False, True])
+def test_f32_operands_beyond_the_one_launch_kernel_do_not_lose_accuracy_with_depth(m, k, n, b_k_major):
+    """Products are within 2^-23, a sum of eight blocks of 64 is off by at most 32 cut-off sums of four ulps that lean one way (2^-19 at the
+    worst, a quarter of that in the mean of a growing sum), and sums of random sign add up as their values do. (One accumulator: 9e-6
+    at 2050 x 8184 x 1040.)"""
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    doc = graphs.document("tiles", [graphs.matmul_node("matmul", 1, 2, 4)], [graphs.tensor(1, "A", [m, k]), graphs.tensor(2, "B", [k, n], "FLOAT", [1, k] if b_k_major else [n, 1]), graphs.tensor(4, "C", [m, n])])
+    a, b = (torch.randn(count, device="cuda", generator=g) for count in (m * k, k * n))
+    buffers = {1: a, 2: b}
+    exe = run(doc, buffers)
+    want = a.view(m, k).double() @ (b.view(n, k).t() if b_k_major else b.view(k, n)).double()
+    error = (buffers[4].view(m, n).double() - want).norm() / want.norm()
+    if [s["kernel"] for s in exe.steps()] == [dfgpu.MATMUL_UMMA_F32X3]:
+        assert float(error) <= 2.0 ** -21 + 2.0 ** -23
+    else:
+        assert m <= 300 and float(error) <= 2.0 ** -19
