@@ -594,9 +594,10 @@ const ClusterCapacity& cluster_capacity() {
 
 // The launch itself: all tiles' clusters at once, with fewer ranks per tile when the device cannot co-schedule that many
 // clusters of the first size.
-// From this reduction depth on AUTO takes the flat form: below it f32 additions are more exact than pieces (1 x 1 over 4 channels 4.0e-8
-// against 5.5e-8 from 64 bits, 8 channels 5.4 / 5.8, 12 channels 6.4 / 6.0, 16 channels 7.4 / 6.3), at 10.3 us against 6.8.
-constexpr int64_t kFlatFormMinDepth = 12;
+// From this reduction depth on AUTO takes the flat form; below it f32 additions are more exact than pieces. Relative error against 64
+// bits of a 1 x 1 filter, f32 additions / pieces, normal values: 4 channels 4.0e-8 / 5.5e-8, 8 channels 5.4 / 5.8, 12 channels 6.5 / 7.3,
+// 16 channels 7.5 / 7.7, 20 channels 8.0 / 8.3, 24 channels 8.7 / 8.5, 32 channels 10.2 / 9.0 (uniform values cross at 12), at 10.3 us against 6.8.
+constexpr int64_t kFlatFormMinDepth = 24;
 static bool flat_form(const ClusterConvArgs& g, const ConvArgs& a, bool& w_flat) {
     auto quads = [](const void* pointer, int type, int64_t channels, int32_t channel_stride, int32_t s0, int32_t s1, int32_t s2) {
         return type == DFGPU_F32 && channels % 4 == 0 && channel_stride == 1 && s0 % 4 == 0 && s1 % 4 == 0 && s2 % 4 == 0 && (reinterpret_cast<uintptr_t>(pointer) & 15u) == 0;

@@ -74,7 +74,7 @@ def test_matmul_with_an_infinity(m, k, n):
     assert np.array_equal(c.cpu().numpy(), want, equal_nan=True)
 
 
-@pytest.mark.parametrize("depth", [4, 8])
+@pytest.mark.parametrize("depth", [4, 8, 12, 20])
 @pytest.mark.parametrize("conv", [True, False])
 def test_shallow_reductions_are_f32_additions(depth, conv):
     """A handful of products: one rounding each, in order (a product and a sum in f64, rounded to f32, is that but for double roundings)."""
