@@ -646,9 +646,7 @@ umma_conv_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __g
                 for (int e = 0; e < args.epi_count; ++e) {
                     const int kind = args.epi_kind[e];
                     if (kind == kEpiRelu) {
-                        const float lower = args.epi_lower[e], upper = args.epi_upper[e], slope = args.epi_slope[e];
-#pragma unroll
-                        for (int t = 0; t < 32; ++t) v[t] = relu_fast(v[t], lower, upper, slope);
+                        relu_values(v, args.epi_lower[e], args.epi_upper[e], args.epi_slope[e]);
                     } else if (kind == kEpiBias) {
                         const float4* p = reinterpret_cast<const float4*>(bias_smem + bias_slot * pargs.bias_stride + n0 + chunk * 32);
                         ++bias_slot;

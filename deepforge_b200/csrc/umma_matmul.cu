@@ -68,6 +68,7 @@ struct TileArgs {
     int32_t a_piece_rows, b_piece_rows;   // kPieces: rows of the maps from one piece to the next
     uint32_t idesc;
     int32_t staging_offset, barrier_offset;
+    int32_t staging_boxes;            // per epilogue group, used in turn: 1 or 2
     void* out;
     int64_t out_ld;
     int32_t out_dtype;
@@ -187,37 +188,73 @@ __device__ __forceinline__ void widen_pair(uint32_t word, int dtype, float& lo, 
         hi = f.y;
     }
 }
-// v[i] += operand[first + i] for COUNT neighbouring columns, as far as the operand's row reaches (`live` of them).
+// The fused ADD operands: COUNT neighbouring columns from element `first` on, as far as the row reaches (`live` of them). Every load
+// is issued before the first use, whole rows in 16-byte units where COUNT allows: a load at a time, each behind a branch on the
+// type, took an epilogue part of 32 columns 8 (ragged edges: 32) trips to the L2 one after the other, 3 to 8 us of a launch with a
+// bias (238 x 312 x 304 bf16: 9.5 us that way, 3.8 without a bias).
 template <int COUNT>
-__device__ __forceinline__ void add_operand(float (&v)[COUNT], const void* data, int dtype, int64_t first, int live, bool vector) {
+__device__ __forceinline__ void load_words(uint32_t (&words)[COUNT / 2], const uint16_t* p, int live, bool vector) {   // 16-bit operands
     if (vector && live >= COUNT) {
-        if (dtype == DFGPU_F32) {
-            const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(data) + first);
+        if constexpr (COUNT % 8 == 0) {
 #pragma unroll
-            for (int j = 0; j < COUNT / 4; ++j) {
-                const float4 q = p[j];
-                v[4 * j] = __fadd_rn(v[4 * j], q.x);
-                v[4 * j + 1] = __fadd_rn(v[4 * j + 1], q.y);
-                v[4 * j + 2] = __fadd_rn(v[4 * j + 2], q.z);
-                v[4 * j + 3] = __fadd_rn(v[4 * j + 3], q.w);
+            for (int j = 0; j < COUNT / 8; ++j) {
+                const uint4 q = reinterpret_cast<const uint4*>(p)[j];
+                words[4 * j] = q.x;
+                words[4 * j + 1] = q.y;
+                words[4 * j + 2] = q.z;
+                words[4 * j + 3] = q.w;
             }
         } else {
-            const uint2* p = reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(data) + first);
 #pragma unroll
             for (int j = 0; j < COUNT / 4; ++j) {
-                const uint2 q = p[j];
-                float f[4];
-                widen_pair(q.x, dtype, f[0], f[1]);
-                widen_pair(q.y, dtype, f[2], f[3]);
-#pragma unroll
-                for (int t = 0; t < 4; ++t) v[4 * j + t] = __fadd_rn(v[4 * j + t], f[t]);
+                const uint2 q = reinterpret_cast<const uint2*>(p)[j];
+                words[2 * j] = q.x;
+                words[2 * j + 1] = q.y;
             }
         }
+    } else {
+        uint16_t halves[COUNT];
+#pragma unroll
+        for (int i = 0; i < COUNT; ++i) halves[i] = i < live ? p[i] : 0;
+#pragma unroll
+        for (int i = 0; i < COUNT / 2; ++i) words[i] = halves[2 * i] | (static_cast<uint32_t>(halves[2 * i + 1]) << 16);
+    }
+}
+template <int COUNT>
+__device__ __forceinline__ void add_words(float (&v)[COUNT], const uint32_t (&words)[COUNT / 2], int dtype) {
+#pragma unroll
+    for (int i = 0; i < COUNT / 2; ++i) {
+        float lo, hi;
+        widen_pair(words[i], dtype, lo, hi);
+        v[2 * i] = __fadd_rn(v[2 * i], lo);
+        v[2 * i + 1] = __fadd_rn(v[2 * i + 1], hi);
+    }
+}
+template <int COUNT>
+__device__ __forceinline__ void add_operand(float (&v)[COUNT], const void* data, int dtype, int64_t first, int live, bool vector) {
+    if (dtype != DFGPU_F32) {
+        uint32_t words[COUNT / 2];
+        load_words<COUNT>(words, static_cast<const uint16_t*>(data) + first, live, vector);
+        add_words<COUNT>(v, words, dtype);
         return;
     }
+    const float* p = static_cast<const float*>(data) + first;
+    float x[COUNT];
+    if (vector && live >= COUNT) {
 #pragma unroll
-    for (int i = 0; i < COUNT; ++i)
-        if (i < live) v[i] = __fadd_rn(v[i], load_as_f32(data, dtype, first + i));
+        for (int j = 0; j < COUNT / 4; ++j) {
+            const float4 q = reinterpret_cast<const float4*>(p)[j];
+            x[4 * j] = q.x;
+            x[4 * j + 1] = q.y;
+            x[4 * j + 2] = q.z;
+            x[4 * j + 3] = q.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < COUNT; ++i) x[i] = i < live ? p[i] : 0.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < COUNT; ++i) v[i] = __fadd_rn(v[i], x[i]);
 }
 
 struct Scalars {
@@ -242,16 +279,16 @@ __device__ __forceinline__ void fold_amax(const TileArgs& args, const Scalars& s
     if (lane == 0 && bits != 0u && ok) atomicMax(args.amax_bits, bits);
 }
 
-// COUNT neighbouring columns of one row: fused steps, then MATMUL_FP8's scalars. `row_live`: the row exists.
+// COUNT neighbouring columns of one row: fused steps, then MATMUL_FP8's scalars. `row_live`: the row exists. `ahead`: the first
+// step's operand, where it was loaded ahead.
 template <int COUNT>
-__device__ __forceinline__ void apply_steps(const TileArgs& args, float (&v)[COUNT], int row, int col0, bool row_live, Scalars& scalars) {
+__device__ __forceinline__ void apply_steps(const TileArgs& args, float (&v)[COUNT], int row, int col0, bool row_live, Scalars& scalars, const uint32_t (*ahead)[COUNT / 2] = nullptr) {
     const int live = args.n_total - col0;
-    for (int s = 0; s < args.step_count; ++s) {
+    if (ahead != nullptr) add_words<COUNT>(v, *ahead, args.step_dtype[0]);
+    for (int s = ahead != nullptr ? 1 : 0; s < args.step_count; ++s) {
         const int kind = args.step_kind[s];
         if (kind == kStepRelu) {
-            const float lower = args.relu_lower[s], upper = args.relu_upper[s], slope = args.relu_slope[s];
-#pragma unroll
-            for (int e = 0; e < COUNT; ++e) v[e] = relu_fast(v[e], lower, upper, slope);
+            relu_values(v, args.relu_lower[s], args.relu_upper[s], args.relu_slope[s]);
         } else if (kind == kStepBias || row_live) {
             add_operand<COUNT>(v, args.step_data[s], args.step_dtype[s], (kind == kStepBias ? 0 : row * args.step_ld[s]) + col0, live, args.step_vector[s] != 0);
         }
@@ -267,6 +304,13 @@ __device__ __forceinline__ void apply_steps(const TileArgs& args, float (&v)[COU
         }
         scalars.magnitude = top;
     }
+}
+
+// The first step's operand for 32 columns, where it is 16 bits wide.
+__device__ __forceinline__ void load_ahead(const TileArgs& args, uint32_t (&words)[16], int row, int col0, bool row_live) {
+    const bool per_column = args.step_kind[0] == kStepBias;
+    load_words<32>(words, static_cast<const uint16_t*>(args.step_data[0]) + (per_column ? 0 : row * args.step_ld[0]) + col0, per_column || row_live ? args.n_total - col0 : 0,
+                   args.step_vector[0] != 0);
 }
 
 __device__ __forceinline__ uint32_t narrow_pair(float lo, float hi, int dtype) {
@@ -663,16 +707,21 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             tc_fence_before();
         } else {
             const uint32_t leader_bars = CG == 2 ? address_in(bar_base, 0) : bar_base;
-            uint8_t* staging = generic_base + args.staging_offset + g * kStageBox;
+            const int staging0 = args.staging_offset + g * args.staging_boxes * kStageBox;
             const int box_columns = !args.tma_store || args.out_dtype == DFGPU_F32 ? 32 : (args.out_dtype == DFGPU_E4M3 ? 128 : 64);
             Scalars scalars = load_scalars(args);
-            bool stored = false;   // (this group has a store in flight)
+            int stored = 0;   // boxes this group has sent off
             int local = 0;
+            const bool ahead = (KIND == kSixteen || KIND == kPieces) && args.step_count > 0 && args.step_kind[0] != kStepRelu && args.step_dtype[0] != DFGPU_F32;
+            uint32_t first_operand[16];
             for (int i = first_item; i < args.items; i += item_step, local += kInBlocks<KIND> ? 0 : 1) {
                 const int acc = local & args.acc_shift, use = local >> args.acc_shift;
                 const Item item = item_at(args, i);
                 const int row0 = (item.m_tile * CG + (CG == 2 ? rank : 0)) * kRows, out_row = row0 + row;
                 const bool row_live = out_row < args.m_total;
+                // (the first operand of a part is loaded under the part before, of an item's first part under its products: waited for
+                // in its place it cost 700 clocks of every part's 2300)
+                if (ahead) load_ahead(args, first_operand, out_row, item.col0 + g * box_columns, row_live);
                 if constexpr (kInRegisters<KIND>) {
                     sum_blocks<CG>(sums, tmem_base + lane_base, args.acc_stride, item.width / 32, g, kb_end - kb_begin, local, acc_full(0), leader_bars + (acc_empty(0) - bar_base), lane, ok);
                 } else if constexpr (kInPlace<KIND>) {
@@ -688,8 +737,12 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     // overlapping accumulators: the first one is read from its end, the second from its start
                     const int box = overlapped && acc == 0 ? boxes - 2 + 2 * g - b : b;
                     const int col0 = item.col0 + box * box_columns;
-                    if (args.tma_store && stored) {
-                        if (row == 0) tma_store_wait_read<0>();
+                    const int staging = staging0 + (args.staging_boxes == 2 ? (stored & 1) * kStageBox : 0);
+                    if (args.tma_store && stored >= args.staging_boxes) {
+                        if (row == 0) {
+                            if (args.staging_boxes == 2) tma_store_wait_read<1>();
+                            else tma_store_wait_read<0>();
+                        }
                         epilogue_barrier(1 + g);
                     }
                     for (int part = 0; part < box_columns / 32; ++part) {
@@ -717,9 +770,18 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 #pragma unroll
                         for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(raw[e]);
                         const int col = col0 + part * 32;
-                        apply_steps<32>(args, v, out_row, col, row_live, scalars);
+                        if (ahead) {
+                            uint32_t operand[16];
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) operand[e] = first_operand[e];
+                            const bool same_box = part + 1 < box_columns / 32;
+                            if (same_box || b + 2 < boxes) load_ahead(args, first_operand, out_row, same_box ? col + 32 : item.col0 + (b + 2) * box_columns, row_live);
+                            apply_steps<32>(args, v, out_row, col, row_live, scalars, &operand);
+                        } else {
+                            apply_steps<32>(args, v, out_row, col, row_live, scalars);
+                        }
                         if (args.tma_store) {
-                            uint8_t* target = staging + row * 128;
+                            uint8_t* target = generic_base + staging + row * 128;
                             if (args.out_dtype == DFGPU_F32) {
 #pragma unroll
                                 for (int j = 0; j < 8; ++j)
@@ -747,10 +809,10 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         fence_async_shared();
                         epilogue_barrier(1 + g);
                         if (row == 0) {
-                            if (healthy && row0 < args.m_total && col0 < args.n_total) tma_store_2d(&map_c, smem_base + args.staging_offset + g * kStageBox, col0, row0);
+                            if (healthy && row0 < args.m_total && col0 < args.n_total) tma_store_2d(&map_c, smem_base + staging, col0, row0);
                             tma_store_commit();
                         }
-                        stored = true;
+                        ++stored;
                     }
                 }
                 tc_fence_before();
@@ -1035,7 +1097,14 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     args.blocks_per_sum = p.kind == kPiecesSummed ? 8 : 1;
     args.sums_column = (args.acc_shift + 1) * args.acc_stride;
     args.scale_columns = 480;
-    const int staging = shape.splits > 1 || !args.tma_store ? 0 : 2 * kStageBox, barriers = (2 * kMaxStages + 6) * 8;
+    const int barriers = (2 * kMaxStages + 6) * 8;
+    const int box_columns = kRowBytes / p.out_bytes;
+    // (two staging boxes a group where it fills more than one and they leave the ring five stages: a box is otherwise written only when
+    // the store before has been read, 400 clocks each. 2048 x 64 x 4096 bf16 with bias and ReLU, with the operands loaded ahead: 12.6 us -> 10.8; MXFP8 4096^3
+    // with four stages for five: 0.9 % slower.)
+    const bool many_boxes = shape.bn > 2 * box_columns || shape.tiles + shape.halved > sm_count() / shape.cg;
+    args.staging_boxes = many_boxes && stages_that_fit(args.stage_bytes, kSmemBudget - 4 * kStageBox - barriers) >= 5 ? 2 : 1;
+    const int staging = shape.splits > 1 || !args.tma_store ? 0 : 2 * args.staging_boxes * kStageBox;
     args.stages = stages_that_fit(args.stage_bytes, kSmemBudget - staging - barriers);
     args.staging_offset = ring_bytes(args.stages, args.stage_bytes);   // (a split product parks its 128 x bn partial tile, at most 64 KB, in the ring)
     args.barrier_offset = args.staging_offset + staging;

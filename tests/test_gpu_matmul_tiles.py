@@ -178,3 +178,29 @@ def test_f32_operands_beyond_the_one_launch_kernel_do_not_lose_accuracy_with_dep
         assert float(error) <= 2.0 ** -21 + 2.0 ** -23
     else:
         assert m <= 300 and float(error) <= 2.0 ** -19
+
+
+@pytest.mark.parametrize("m,k,n", [(77, 64, 88), (130, 192, 216), (300, 136, 600), (2049, 72, 2064)])
+@pytest.mark.parametrize("first", ["bias", "full"])
+@pytest.mark.parametrize("io,operand,shift", [("BFLOAT16", "BFLOAT16", 0), ("BFLOAT16", "BFLOAT16", 1), ("HALF", "HALF", 0), ("HALF", "FLOAT", 1), ("BFLOAT16", "FLOAT", 0)])
+def test_fused_operands_at_the_edges(m, k, n, first, io, operand, shift):
+    """Operands in 16-byte units and off them, short rows of them at the last columns, values that ReLU passes through its three ways:
+    infinities (x < 0 becomes 0 (x - 0) + 0, so NaN for -inf; above the largest f32 it clips), and the ordinary ones."""
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    dims = [1, n] if first == "bias" else [m, n]
+    tensors = [graphs.tensor(1, "A", [m, k], io), graphs.tensor(2, "B", [k, n], io), graphs.tensor(3, "x", dims, operand), graphs.tensor(4, "C", [m, n], io), graphs.tensor(5, "p", [m, n], virtual=True), graphs.tensor(6, "q", [m, n], virtual=True)]
+    nodes = [graphs.matmul_node("matmul", 1, 2, 5), graphs.pointwise_node("add", "ADD", 5, 6, 3), graphs.pointwise_node("relu", "RELU_FWD", 6, 4)]
+    buffers = {uid: torch.randn(count, device="cuda", generator=g).to(TORCH[io]) for uid, count in ((1, m * k), (2, k * n))}
+    x = torch.randn(dims, device="cuda", generator=g).to(TORCH[operand])
+    x[-1, n - 3], x[-1, 5] = -float("inf"), float("inf")
+    buffers[3] = torch.zeros(x.numel() + shift, dtype=x.dtype, device="cuda")[shift:]
+    buffers[3].copy_(x.reshape(-1))
+    exe = run(graphs.document("tiles", nodes, tensors, io=io), buffers)
+    assert exe.launch_count == 1
+    a, b = buffers[1].view(m, k).double(), buffers[2].view(k, n).double()
+    got, want = buffers[4].view(m, n).double(), a @ b + x.double()
+    bound = ROUNDING[io] * want.abs() + k * 2.0 ** -24 * (a.abs() @ b.abs()) + 1e-30
+    assert torch.equal(got.isnan(), want == -float("inf"))
+    assert torch.all(got[want == float("inf")] >= torch.finfo(TORCH[io]).max)
+    finite = want.isfinite()
+    assert torch.all((got - torch.relu(want)).abs()[finite] <= bound[finite])
