@@ -504,52 +504,67 @@ sdpa_paged_decode_kernel(SdpaArgs a, float* __restrict__ partial, int max_chunks
     }
 }
 
-// One CTA of 128 threads per (batch, query head): combine the chunk partials. Latency-bound (a few KB per CTA): the chunks'
-// maxima and sums are read side by side, one chunk per thread, and the weighted sum over chunks has eight loads in flight.
+// One CTA of 128 threads per (batch, query head): combine the chunk partials. Latency-bound (a few KB per CTA), so everything is
+// loaded at once, before the lengths say which chunks hold keys: every warp takes all maxima and sums, a chunk per lane and
+// group of 32, and each thread its channel of the first 32 chunks. (Maxima, then sums, then values took three trips to the L2 cache
+// and two barriers more.) Sums add up lane by lane, then group by group; values chunk by chunk.
 __global__ void __launch_bounds__(128)
 sdpa_decode_merge_kernel(SdpaArgs a, const float* __restrict__ partial, int max_chunks, int chunk_keys) {
-    __shared__ float weights[128], reduce[8];
+    constexpr int kAhead = 32, kGroups = 4;
     chain_begin();
     partial = after_chain(partial);
     const int64_t row = blockIdx.x;  // b * Hq + h
     const int64_t hq = a.q.dim[1];
     const int64_t ib = row / hq, ih = row % hq;
-    const int d = threadIdx.x, warp = d >> 5, lane = d & 31;
+    const int d = threadIdx.x, lane = d & 31;
+    const float* base = partial + row * max_chunks * kPartialStride;
+    float ahead[kAhead], maxima[kGroups], sums[kGroups];
+#pragma unroll
+    for (int g = 0; g < kGroups; ++g) {
+        const bool in = g * 32 + lane < max_chunks;
+        maxima[g] = in ? base[(g * 32 + lane) * kPartialStride + kDecodeD] : -INFINITY;
+        sums[g] = in ? base[(g * 32 + lane) * kPartialStride + kDecodeD + 1] : 0.0f;
+    }
+#pragma unroll
+    for (int c = 0; c < kAhead; ++c) ahead[c] = c < max_chunks ? base[c * kPartialStride + d] : 0.0f;
     int64_t lo, hi;
     valid_range(a, ib, 0, lo, hi);
     int chunks = hi > 0 ? static_cast<int>((hi + chunk_keys - 1) / chunk_keys) : 0;
     if (chunks > max_chunks) chunks = max_chunks;
-    const float* base = partial + row * max_chunks * kPartialStride;
     float total_max = -INFINITY;
-    for (int c = d; c < chunks; c += 128) total_max = fmaxf(total_max, base[c * kPartialStride + kDecodeD]);
+#pragma unroll
+    for (int g = 0; g < kGroups; ++g) {
+        if (g * 32 + lane >= chunks) maxima[g] = -INFINITY;   // (never written, as an empty chunk's values)
+        total_max = fmaxf(total_max, maxima[g]);
+    }
+    for (int c = kGroups * 32 + lane; c < chunks; c += 32) total_max = fmaxf(total_max, base[c * kPartialStride + kDecodeD]);
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) total_max = fmaxf(total_max, __shfl_xor_sync(0xffffffffu, total_max, s));
-    if (lane == 0) reduce[warp] = total_max;
-    __syncthreads();
-    total_max = fmaxf(fmaxf(reduce[0], reduce[1]), fmaxf(reduce[2], reduce[3]));
     float total_sum = 0.0f, value = 0.0f;
-    for (int first = 0; first < chunks; first += 128) {
-        const int count = min(128, chunks - first);
-        __syncthreads();   // (the weights of the chunks before have been read)
-        if (d < count) {
-            const float* own = base + (first + d) * kPartialStride + kDecodeD;
-            const float m = own[0];
-            const float weight = m == -INFINITY ? -1.0f : expf(m - total_max);   // (an empty chunk's weight is negative: a zero may be a small one's)
-            weights[d] = weight;
-            if (!(weight < 0.0f)) total_sum = fmaf(own[1], weight, total_sum);
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int c = 0; c < count; ++c) {
-            const float o = base[(first + c) * kPartialStride + d];   // (an empty chunk's is never written: not counted)
-            value = weights[c] < 0.0f ? value : fmaf(o, weights[c], value);
+    for (int first = 0; first < chunks; first += 32) {   // 32 chunks at a time, the next ones' values on their way
+        float next[kAhead];
+#pragma unroll
+        for (int c = 0; c < kAhead; ++c) next[c] = first + 32 + c < chunks ? base[(first + 32 + c) * kPartialStride + d] : 0.0f;
+        const int g = first / 32;
+        const bool in = first + lane < chunks;
+        const float* own = base + (first + lane) * kPartialStride + kDecodeD;
+        float m = -INFINITY, sum = 0.0f;
+        if (g >= kGroups && in) m = own[0], sum = own[1];
+#pragma unroll
+        for (int i = 0; i < kGroups; ++i)
+            if (g == i) m = maxima[i], sum = sums[i];
+        const float weight = m == -INFINITY ? -1.0f : expf(m - total_max);   // (an empty chunk's weight is negative: a zero may be a small one's)
+        float part = weight < 0.0f ? 0.0f : sum * weight;
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) part += __shfl_xor_sync(0xffffffffu, part, s);
+        total_sum += part;
+#pragma unroll
+        for (int c = 0; c < kAhead; ++c) {
+            const float factor = __shfl_sync(0xffffffffu, weight, c);   // (negative past the last chunk too)
+            value = factor < 0.0f ? value : fmaf(ahead[c], factor, value);
+            ahead[c] = next[c];
         }
     }
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) total_sum += __shfl_xor_sync(0xffffffffu, total_sum, s);
-    if (lane == 0) reduce[4 + warp] = total_sum;
-    __syncthreads();
-    total_sum = reduce[4] + reduce[5] + reduce[6] + reduce[7];
     float result = total_sum == 0.0f ? 0.0f : value / total_sum;   // (a NaN sum is a NaN result)
     store_from_f32(a.o_data, a.o.dtype, off4(a.o, ib, ih, 0, d), result);
     if (d == 0) {
