@@ -11,7 +11,8 @@
 // the positions past the end with zeros and clips them on the store, and what is left is a mask on the last key tile. With
 // SEQ_LEN_Q / SEQ_LEN_KV a batch's key tiles end at its own length, V rows behind it are cleared in shared memory (a zero
 // probability times an infinity in the padding would be NaN), and rows past SEQ_LEN_Q store 0 and -inf. 4 x 16 heads of 1000
-// padded positions, causal: 9.7 ms on the row-at-a-time kernel, 36 us here (31 with P in one 16-bit piece, and O 1.33 times as far from 64 bits).
+// padded positions, causal: 9.7 ms on the row-at-a-time kernel, 26 to 34 us here, by the lengths (before the halves and the order below 36;
+// 31 then with P in one 16-bit piece, and O 1.33 times as far from 64 bits).
 #include <algorithm>
 #include <cmath>
 
@@ -28,7 +29,7 @@ struct SdpaUmmaArgs {
     int32_t heads_q, heads_kv, seq_q, seq_kv;
     int32_t pairs;            // of 128-row query tiles, the last one perhaps partly past the end
     int32_t causal;
-    int32_t order;            // of the work list: kAsStored, kHeavyWithLight or kHeaviestFirst (see PairWalker)
+    int32_t order;            // of the work list: kAsStored, kHeavyWithLight, kHeaviestFirst or kLongestFirst (see PairWalker)
     float scale_log2;  // |attn_scale| * log2(e); a negative scale negates Q in the products
     uint32_t negate_q; // ... through this bit of the instruction descriptor
     const int32_t* len_q;   // SEQ_LEN_Q and SEQ_LEN_KV by batch, or null
@@ -70,6 +71,9 @@ __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::
 //                                                 O_B += P_B(j) V_j ; S_B(j+1) = Q_B K_{j+1}^T
 //   warps 0-7   softmax of tile A, warps 8-15 softmax of tile B: two threads per query row, each with 64 of the
 //               tile's 128 keys (the two warps that share a lane quarter trade row maxima through shared memory)
+// Probabilities are handed over in two halves, each thread's first 32 keys under the exponentials of its others: a tile's chain of score
+// product, softmax and second product is what a round waits for (8 x 32 x 2048 x 128 causal 334 -> 329 us, 12 heads of 2061 x 64 causal
+// 40.1 -> 37.3, 2 x 32 x 4000 x 64 padded 178 -> 167).
 // (D is the head dimension.) TMEM: S_A at +0, S_B at +128, O_A at +256, O_B at +384. P never goes through shared memory: each
 // thread overwrites its own score row with the 16-bit probabilities (two per 32-bit
 // column) and the second product takes its A operand from tensor memory. The tensor pipe runs the
@@ -91,10 +95,13 @@ struct PairSmem {
     // slots and the output tile).
     static constexpr int kExchange = kStage + kTile;
     static constexpr int kBarriers = kExchange + 1024 + 512;
-    // stage_free, q_full[2], q_empty[2], kv_full[S], kv_empty[S], s_full[2], p_full[2], o_full[2], o_empty[2], staged[2]
-    static constexpr int kBarrierCount = 5 + 2 * kPairSlots + 10;
-    static constexpr int kTotal = kBarriers + kBarrierCount * 8 + 16;
+    // stage_free, q_full[2], q_empty[2], kv_full[S], kv_empty[S], s_full[2], p_full[2], o_full[2], o_empty[2], staged[2], p_half[2]
+    static constexpr int kBarrierCount = 5 + 2 * kPairSlots + 12;
+    static constexpr int kList = kBarriers + kBarrierCount * 8 + 16;   // kLongestFirst: kMostPairs bytes
+    static constexpr int kMostPairs = 256;
+    static constexpr int kTotal = kList + kMostPairs;
     static constexpr int kDynamic = kTotal + 1024;
+    static_assert(kDynamic <= 227 * 1024, "the most a block may have");
 };
 constexpr int kHalfBytes = kRows * 128;   // one box
 
@@ -283,8 +290,8 @@ struct PairItem {
 // tile (padding masks, or a key length that is no multiple of 128), and probabilities are held to f32's accuracy: O += P V runs
 // twice, on P rounded to the operands' type and on what that left over (16 or 22 bits in all), as O and Stats of these graphs are
 // those of f32 probabilities (sdpa_rowwise_kernel's) to the rounding of O. Without it the masks of the last tile, the clearing of V
-// rows and the dead rows are not compiled in: they cost 5 % of 8 x 32 x 2048 causal.
-template <bool GENERAL>
+// rows and the dead rows are not compiled in: they cost 5 % of 8 x 32 x 2048 causal. (LENGTHS: the batches have lengths of their own.)
+template <bool LENGTHS>
 __device__ __forceinline__ PairItem pair_item(const SdpaUmmaArgs& args, int bh, int pair) {
     PairItem item;
     item.batch = bh / args.heads_q;
@@ -293,7 +300,7 @@ __device__ __forceinline__ PairItem pair_item(const SdpaUmmaArgs& args, int bh, 
     item.q_tile_a = 2 * pair;
     item.kv_len = args.seq_kv;
     item.live_q = args.seq_q;
-    if (GENERAL && args.len_q != nullptr) {
+    if (LENGTHS && args.len_q != nullptr) {
         const int len_kv = args.len_kv[item.batch * args.len_kv_stride];
         item.live_q = len_kv > 0 ? min(item.live_q, args.len_q[item.batch * args.len_q_stride]) : 0;
         item.kv_len = max(1, min(item.kv_len, len_kv));
@@ -315,12 +322,16 @@ __device__ __forceinline__ PairItem pair_item(const SdpaUmmaArgs& args, int bh, 
 //                    walks 2P+2 key tiles and equal numbers of units are equal work
 //   kHeaviestFirst   causal, two SMs per pair: the pairs of all heads by falling length, and every other round
 //                    in reverse, so that the CTA with the longest pair of one round gets the shortest of the next
+//   kLongestFirst    padded lengths, one SM per pair: the same by the key tiles that a batch's own lengths leave of its pairs, in an order
+//                    that each CTA works out for itself (longest_first()). 4 x 16 heads of 500 to 1000 positions causal: 8 key tiles on the
+//                    longest list instead of 10, 34.7 -> 26.2 us with the halves above; 2 x 32 x 4000 x 64 252 -> 178 by the order alone.
 // CTA c takes units c, c + gridDim.x, ...; but for the last order neighbouring CTAs thus work on the same head at the same
 // time and share its K and V in L2.
-enum { kAsStored = 0, kHeavyWithLight = 1, kHeaviestFirst = 2 };
-template <int CTAS>   // that walk one list together
+enum { kAsStored = 0, kHeavyWithLight = 1, kHeaviestFirst = 2, kLongestFirst = 3 };
+template <int CTAS, bool LISTED = false>   // CTAs that walk one list together; LISTED: kLongestFirst is compiled in (it cost the other orders 2 %)
 struct PairWalker {
     int k = 0;
+    const uint8_t* list = nullptr;   // kLongestFirst: (batch, pair) by falling length
     __device__ __forceinline__ bool next(const SdpaUmmaArgs& args, int& bh, int& pair) {
         const int pairs = args.pairs;
         if constexpr (CTAS == 2) {
@@ -337,6 +348,16 @@ struct PairWalker {
                 bh = unit / pairs;
                 pair = unit - bh * pairs;
             }
+            return true;
+        }
+        if (LISTED && args.order == kLongestFirst) {
+            const int places = static_cast<int>(gridDim.x), place = static_cast<int>(blockIdx.x);
+            const int unit = k * places + ((k & 1) ? places - 1 - place : place);
+            ++k;
+            if (unit >= pairs * args.batch_heads) return false;
+            const int at = unit / args.heads_q, entry = list[at], batch = entry / pairs;
+            bh = batch * args.heads_q + unit - at * args.heads_q;
+            pair = entry - batch * pairs;
             return true;
         }
         const int units_per_head = args.order == kHeavyWithLight ? (pairs + 1) >> 1 : pairs;
@@ -358,9 +379,28 @@ struct PairWalker {
         }
     }
 };
-template <int CTAS, class Body>
-__device__ __forceinline__ void for_each_pair_item(const SdpaUmmaArgs& args, Body&& body) {
-    PairWalker<CTAS> walker;
+// The (batch, pair)s, at most 256, by falling number of key tiles: every thread counts the ones ahead of its own.
+__device__ __forceinline__ void longest_first(const SdpaUmmaArgs& args, uint8_t* list, uint16_t* weights) {
+    const int count = args.batch_heads / args.heads_q * args.pairs, own = static_cast<int>(threadIdx.x);
+    int weight = 0;
+    if (own < count) {
+        const int batch = own / args.pairs;
+        const PairItem item = pair_item<true>(args, batch * args.heads_q, own - batch * args.pairs);
+        weight = item.tiles_a + item.tiles_b;
+        weights[own] = static_cast<uint16_t>(weight);
+    }
+    __syncthreads();
+    if (own < count) {
+        int ahead = 0;
+        for (int i = 0; i < count; ++i) ahead += weights[i] > weight || (weights[i] == weight && i < own) ? 1 : 0;
+        list[ahead] = static_cast<uint8_t>(own);
+    }
+    __syncthreads();
+}
+template <int CTAS, bool LISTED, class Body>
+__device__ __forceinline__ void for_each_pair_item(const SdpaUmmaArgs& args, const uint8_t* list, Body&& body) {
+    PairWalker<CTAS, LISTED> walker;
+    walker.list = list;
     int bh, pair;
     while (walker.next(args, bh, pair))  // one call site of the body: it is a whole warp role
         if (!body(bh, pair)) return;
@@ -374,7 +414,7 @@ __device__ __forceinline__ void for_each_pair_item(const SdpaUmmaArgs& args, Bod
 //   warp 17     issues the products; one elected lane issues, all lanes walk the schedule
 //   warp 18     sends staged output tiles to global memory by TMA (row-per-thread global stores of 16 bytes at a
 //               256-byte stride kept the load/store unit busy for ~5000 cycles per tile)
-template <int D, bool F16, bool GENERAL>
+template <int D, bool F16, bool GENERAL, bool PADDED>
 __global__ void __launch_bounds__(kPairThreads, 1)
 sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o, SdpaUmmaArgs args) {
@@ -394,6 +434,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     auto o_full = [&](int x) { return bar_base + 8u * (9 + 2 * kPairSlots + x); };
     auto o_empty = [&](int x) { return bar_base + 8u * (11 + 2 * kPairSlots + x); };
     auto staged = [&](int x) { return bar_base + 8u * (13 + 2 * kPairSlots + x); };
+    auto p_half = [&](int x) { return bar_base + 8u * (15 + 2 * kPairSlots + x); };
     const uint32_t tmem_slot = bar_base + 8u * Smem::kBarrierCount;
     volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(generic_base + Smem::kBarriers + 8 * Smem::kBarrierCount);
 
@@ -410,6 +451,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         }
         for (int x = 0; x < 2; ++x) {
             mbar_init(s_full(x), 1);
+            mbar_init(p_half(x), 8);
             mbar_init(p_full(x), 8);
             mbar_init(o_full(x), 1);
             mbar_init(q_full(x), 1);
@@ -428,6 +470,8 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot_ptr;
     chain_wait();
+    const uint8_t* list = PADDED ? generic_base + Smem::kList : nullptr;
+    if (PADDED && args.order == kLongestFirst) longest_first(args, generic_base + Smem::kList, reinterpret_cast<uint16_t*>(generic_base + Smem::kStage));
     // (no early release: this kernel fills every SM, so the next one's CTAs would only wait beside it, 0.6 % of 330 us)
 
     if (warp == 16) {
@@ -435,8 +479,8 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         int slot = 0;
         uint32_t phase = 1;  // parity of the "slot is free" wait
         uint32_t n = 0;      // items started
-        for_each_pair_item<1>(args, [&](int bh, int pair) {
-            const PairItem item = pair_item<GENERAL>(args, bh, pair);
+        for_each_pair_item<1, PADDED>(args, list, [&](int bh, int pair) {
+            const PairItem item = pair_item<PADDED>(args, bh, pair);
             auto load_box = [&](uint32_t dst, const CUtensorMap* map, int row, int head, uint32_t bar) {
 #pragma unroll
                 for (int h = 0; h < D / 64; ++h) tma_load_4d(dst + h * kHalfBytes, map, 64 * h, row, head, item.batch, bar);
@@ -505,31 +549,36 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         // overwrites O_x, which the softmax warps must have read out for the previous item.
         auto product = [&](int x, int j, int v_slot) {
             if (ok && j == 0) ok = mbar_wait_warp(o_empty(x), (n & 1) ^ 1, 218 + x);
-            if (ok) ok = mbar_wait_warp(p_full(x), p_count[x] & 1, 223 + x);
-            ++p_count[x];
-            tc_fence_after();
-            if (!ok) return;
+            // (in two halves: the first 32 of each thread's 64 keys are multiplied while the softmax warps form the others)
             const uint32_t v_lo = smem_desc_lo(smem_base + Smem::kRing + v_slot * kTileBytes, kHalfBytes);
             const uint32_t d_tmem = tmem_u + 256 + x * 128, p_tmem = tmem_u + x * 128;
-            if (leader) {
 #pragma unroll
-                for (int k = 0; k < kKeys / 16; ++k) {
-                    const uint32_t p_at = p_tmem + (k >> 2) * 64 + (k & 3) * kProbabilityColumns<GENERAL>;
-                    umma_bf16_a_tmem(d_tmem, p_at, desc_words(v_lo + ((k * 2048) >> 4), kDescHi), idesc_pv, (j | k) != 0 ? 1u : 0u);
-                    if constexpr (GENERAL) umma_bf16_a_tmem(d_tmem, p_at + 8, desc_words(v_lo + ((k * 2048) >> 4), kDescHi), idesc_pv, 1u);
+            for (int part = 0; part < 2; ++part) {
+                if (ok) ok = mbar_wait_warp(part == 0 ? p_half(x) : p_full(x), p_count[x] & 1, 223 + x);
+                tc_fence_after();
+                if (leader && ok) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int k = (i >> 1) * 4 + part * 2 + (i & 1);   // 16 keys
+                        const uint32_t p_at = p_tmem + (k >> 2) * 64 + (k & 3) * kProbabilityColumns<GENERAL>;
+                        umma_bf16_a_tmem(d_tmem, p_at, desc_words(v_lo + ((k * 2048) >> 4), kDescHi), idesc_pv, (j | k) != 0 ? 1u : 0u);
+                        if constexpr (GENERAL) umma_bf16_a_tmem(d_tmem, p_at + 8, desc_words(v_lo + ((k * 2048) >> 4), kDescHi), idesc_pv, 1u);
+                    }
                 }
             }
+            ++p_count[x];
         };
-        PairWalker<1> walker;
+        PairWalker<1, PADDED> walker;
+        walker.list = list;
         int bh = 0, pair = 0, next_bh = 0, next_pair = 0;
         bool have = walker.next(args, bh, pair);
         bool early = false;  // S_A of the current item was issued in the previous item's last round
         int early_slot = 0;  // the ring slot of its K tile
         while (have && ok) {
-            const PairItem item = pair_item<GENERAL>(args, bh, pair);
+            const PairItem item = pair_item<PADDED>(args, bh, pair);
             const int tiles_a = item.tiles_a, tiles_b = item.tiles_b, tiles = item.tiles;
             const bool have_next = walker.next(args, next_bh, next_pair);
-            const int next_tiles_a = have_next ? pair_item<GENERAL>(args, next_bh, next_pair).tiles_a : 0;
+            const int next_tiles_a = have_next ? pair_item<PADDED>(args, next_bh, next_pair).tiles_a : 0;
             int k0_slot = early_slot;
             if (!early) {
                 if (ok) ok = mbar_wait_warp(q_full(0), n & 1, 222);
@@ -601,8 +650,8 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         const bool leader = elect_one();
         uint32_t n = 0;
         bool ok = true;
-        for_each_pair_item<1>(args, [&](int bh, int pair) {
-            const PairItem item = pair_item<GENERAL>(args, bh, pair);
+        for_each_pair_item<1, PADDED>(args, list, [&](int bh, int pair) {
+            const PairItem item = pair_item<PADDED>(args, bh, pair);
             for (int x = 0; x < 2; ++x) {
                 if (ok) ok = mbar_wait_warp(staged(x), n & 1, 216 + x);
                 if (leader) {
@@ -642,8 +691,8 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         uint32_t s_count = 0;  // score tiles consumed (parity of s_full)
         uint32_t ring_base = 0;  // ring slots of the items before this one
         bool ok = true;
-        for_each_pair_item<1>(args, [&](int bh, int pair) {
-        const PairItem item = pair_item<GENERAL>(args, bh, pair);
+        for_each_pair_item<1, PADDED>(args, list, [&](int bh, int pair) {
+        const PairItem item = pair_item<PADDED>(args, bh, pair);
         const int q_tile = item.q_tile_a + x;
         const int q_index = q_tile * kRows + row;
         const int my_tiles = x ? item.tiles_b : item.tiles_a;
@@ -733,22 +782,28 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     if (c < 3) tmem_load_16(scores_at + (c + 1) * 16, raw[c + 1]);
                     masked(raw[c], c);
                     put_probabilities<F16, GENERAL>(raw[c], scale2, bias2, sums, scores_at + c * kProbabilityColumns<GENERAL>);
+                    if (c == 1) {
+                        if (PADDED && (j + 1) * kKeys > item.kv_len && (D == 128 || half == 0)) {
+                            // V rows past the batch's length are not this sequence's: cleared before the product (by either tile's
+                            // warps, which write the same zeros). The slot is V_j's place in the ring.
+                            const uint32_t place = ring_base + 2 * j + 1, v_slot = place % kPairSlots;
+                            if (ok) ok = mbar_wait(kv_full(v_slot), (place / kPairSlots) & 1, 234 + x);
+                            if (j * kKeys + row >= item.kv_len) {
+                                uint8_t* v_row = generic_base + Smem::kRing + v_slot * kTileBytes + half * kHalfBytes + row * 128;
+#pragma unroll
+                                for (int u = 0; u < 8; ++u) *reinterpret_cast<uint4*>(v_row + u * 16) = make_uint4(0, 0, 0, 0);
+                            }
+                            fence_async_shared();
+                        }
+                        tmem_store_wait();
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(p_half(x));
+                    }
                 }
                 float lo, hi;
                 unpack2(add2(sums[0], sums[1]), lo, hi);
                 l_sum += lo + hi;
-            }
-            if (GENERAL && args.len_q != nullptr && (j + 1) * kKeys > item.kv_len && (D == 128 || half == 0)) {
-                // V rows past the batch's length are not this sequence's: cleared before the product (by either tile's
-                // warps, which write the same zeros). The slot is V_j's place in the ring.
-                const uint32_t place = ring_base + 2 * j + 1, v_slot = place % kPairSlots;
-                if (ok) ok = mbar_wait(kv_full(v_slot), (place / kPairSlots) & 1, 234 + x);
-                if (j * kKeys + row >= item.kv_len) {
-                    uint8_t* v_row = generic_base + Smem::kRing + v_slot * kTileBytes + half * kHalfBytes + row * 128;
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) *reinterpret_cast<uint4*>(v_row + u * 16) = make_uint4(0, 0, 0, 0);
-                }
-                fence_async_shared();
             }
             tmem_store_wait();
             tc_fence_before();
@@ -821,7 +876,7 @@ sdpa_umma_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         if (args.stats != nullptr && ok && half == 0 && q_index < args.seq_q)
             args.stats[item.batch * args.stats_batch_stride + item.head * args.stats_head_stride + static_cast<int64_t>(q_index) * args.stats_row_stride] =
                 live ? natural_log_sum<GENERAL>(args, m_ref, total) : -INFINITY;
-        if (GENERAL) ring_base += 2 * item.tiles;
+        if (PADDED) ring_base += 2 * item.tiles;
         ++n;
         return true;  // also after a wait gave up: the two warps of a row pair must meet at the same barriers to the end
         });
@@ -1124,7 +1179,7 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         const bool leader = elect_one();
         uint32_t n = 0;
         bool ok = true;
-        for_each_pair_item<2>(args, [&](int bh, int pair) {
+        for_each_pair_item<2, false>(args, nullptr, [&](int bh, int pair) {
             const PairItem item = pair_item<GENERAL>(args, bh, pair);
             if (ok) ok = mbar_wait_warp(staged, n & 1, 249);
             if (leader) {
@@ -1155,7 +1210,7 @@ sdpa_umma_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         uint32_t n = 0, t0 = 0, edges = 0;
         uint32_t mine_done = 0;   // key tiles this group has finished (parity of its maxima and references)
         bool ok = true;
-        for_each_pair_item<2>(args, [&](int bh, int pair) {
+        for_each_pair_item<2, false>(args, nullptr, [&](int bh, int pair) {
             const PairItem item = pair_item<GENERAL>(args, bh, pair);
             const int q_tile = item.q_tile_a + rank, q_index = q_tile * kRows + row;
             const bool idle_tile = q_tile * kRows >= item.live_q;   // no row of this CTA's has keys
@@ -1396,11 +1451,11 @@ int sdpa_map(CUtensorMap* map, const dfgpu_tensor& t, const void* data, uint32_t
     return make_map(map, data, 4, dims, strides, box, what);
 }
 
-template <int D, bool F16, bool GENERAL>
+template <int D, bool F16, bool GENERAL, bool PADDED>
 int launch_pair(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_o, const SdpaUmmaArgs& args, unsigned grid, cudaStream_t stream) {
-    cudaError_t error = cudaFuncSetAttribute(sdpa_umma_pair_kernel<D, F16, GENERAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<D>::kDynamic);
+    cudaError_t error = cudaFuncSetAttribute(sdpa_umma_pair_kernel<D, F16, GENERAL, PADDED>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<D>::kDynamic);
     if (error != cudaSuccess) return fail(kExecutionFailed, "SDPA: cannot reserve %d bytes of shared memory: %s", PairSmem<D>::kDynamic, cudaGetErrorString(error));
-    launch_chained(sdpa_umma_pair_kernel<D, F16, GENERAL>, dim3(grid), dim3(kPairThreads), PairSmem<D>::kDynamic, stream, map_q, map_k, map_v, map_o, args);
+    launch_chained(sdpa_umma_pair_kernel<D, F16, GENERAL, PADDED>, dim3(grid), dim3(kPairThreads), PairSmem<D>::kDynamic, stream, map_q, map_k, map_v, map_o, args);
     return check_launch("SDPA (tcgen05, two query tiles per CTA)");
 }
 template <bool F16, bool GENERAL>
@@ -1415,7 +1470,8 @@ template <int D, bool F16>
 int launch_general(bool duo, const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_o, const SdpaUmmaArgs& args, unsigned grid, cudaStream_t stream) {
     if constexpr (D == 128)
         if (duo) return launch_duo<F16, true>(map_q, map_k, map_v, map_o, args, grid, stream);
-    return launch_pair<D, F16, true>(map_q, map_k, map_v, map_o, args, grid, stream);
+    return args.len_q != nullptr ? launch_pair<D, F16, true, true>(map_q, map_k, map_v, map_o, args, grid, stream)
+                                 : launch_pair<D, F16, true, false>(map_q, map_k, map_v, map_o, args, grid, stream);
 }
 
 bool packed_rows(const dfgpu_tensor& t) {
@@ -1514,9 +1570,12 @@ int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, cudaStrea
     const int places = duo ? sm_count() / 2 : sm_count();
     const int64_t single = pairs * heads;
     args.order = !args.causal || single <= places ? kAsStored : (duo ? kHeaviestFirst : kHeavyWithLight);   // (the third order in the one-SM kernel cost it 1.4 %)
+    // (CTAs that run side by side then read different heads' K and V: only where all of them stay in the L2 cache)
+    const int64_t kv_bytes = p.k.dim[0] * p.k.dim[1] * p.k.dim[2] * p.k.dim[3] * 4;
+    if (!duo && p.padding_mask && single > places && p.q.dim[0] * pairs <= PairSmem<128>::kMostPairs && kv_bytes <= (64 << 20)) args.order = kLongestFirst;
     const int64_t units = args.order == kHeavyWithLight ? (pairs + 1) / 2 * heads : single;
     const unsigned grid = static_cast<unsigned>(std::min<int64_t>(units, places));
-    if (plain_tiles(p)) return duo ? launch_duo<false, false>(map_q, map_k, map_v, map_o, args, grid, stream) : launch_pair<128, false, false>(map_q, map_k, map_v, map_o, args, grid, stream);
+    if (plain_tiles(p)) return duo ? launch_duo<false, false>(map_q, map_k, map_v, map_o, args, grid, stream) : launch_pair<128, false, false, false>(map_q, map_k, map_v, map_o, args, grid, stream);
     const bool f16 = p.q.dtype == DFGPU_F16;
     if (p.q.dim[3] == 64) return f16 ? launch_general<64, true>(duo, map_q, map_k, map_v, map_o, args, grid, stream) : launch_general<64, false>(duo, map_q, map_k, map_v, map_o, args, grid, stream);
     return f16 ? launch_general<128, true>(duo, map_q, map_k, map_v, map_o, args, grid, stream) : launch_general<128, false>(duo, map_q, map_k, map_v, map_o, args, grid, stream);

@@ -109,6 +109,15 @@ def test_several_padded_items_per_place(causal, h, sq, skv):
     check(12, h, 2, sq, skv, 128, "BFLOAT16", causal, padding=([min(sq, n + 30) for n in lengths], lengths))
 
 
+@pytest.mark.parametrize("io,d", [("BFLOAT16", 128), ("HALF", 64)])
+@pytest.mark.parametrize("b,h,sq,causal", [(128, 2, 300, True), (129, 2, 300, True), (40, 5, 513, False)])
+def test_padded_items_by_their_lengths(io, d, b, h, sq, causal):
+    """Items walked by falling length: the most (batch, pair)s that are put in order, one too many, and a list that ends inside a reversed
+    round; equal lengths, empty ones and all in between."""
+    lengths = [sq if i % 3 == 0 else (i * 97) % (sq + 1) for i in range(b)]
+    check(b, h, 1, sq, sq, d, io, causal, padding=(lengths[::-1], lengths), fine=True)
+
+
 @pytest.mark.parametrize("io,d", [("BFLOAT16", 128), ("HALF", 128), ("BFLOAT16", 64), ("HALF", 64)])
 @pytest.mark.parametrize("b,h,hkv,sq,skv,causal", [(3, 1, 1, 17, 17, True), (5, 4, 1, 75, 89, False), (1, 37, 37, 1000, 1000, True), (2, 96, 96, 300, 300, True), (2, 60, 12, 256, 1500, False)])
 def test_probabilities_as_accurate_as_f32_ones(io, d, b, h, hkv, sq, skv, causal):
