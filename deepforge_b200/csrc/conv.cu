@@ -166,6 +166,134 @@ conv_igemm_ffma_kernel(const void* __restrict__ x, const void* __restrict__ w, v
     }
 }
 
+// The implicit GEMM for reductions of at most kShallowDepth products (1 x 1 filters, few channels): the whole depth of a tile goes to
+// shared memory at once, so that a CTA waits for global memory once instead of once per 16 products, and indices are 32-bit with
+// multiply-shift divisions (64-bit ones, 30 to 60 instructions each and several per element, were the rest). T: float, or uint16_t for
+// f16 and bf16. From kChainDepth products on, eights are summed by themselves, four of them added up and those added to the total:
+// chains of 8, 4 and 4 roundings, where a chain of the whole depth would be further from 64 bits than three bf16 pieces on the tensor cores.
+constexpr int kShallowDepth = 128, kChainDepth = 24;
+struct ShallowArgs {
+    int m_total, k_total, k_padded;       // k_padded: a multiple of 8
+    int x_n, x_c, x_h, x_w, w_k, w_c, w_r, w_s;
+    int P, Q, H, W, K, R, S;
+    int y_quads;                          // f32 Y whose channels are contiguous and whose pixels start on 16-byte boundaries
+    FastDivisor by_q, by_p, by_inner, by_middle;   // channels last: by C and by S; else by S and by R
+};
+template <int BM, int BN, bool CHANNELS_LAST, typename T>
+__global__ void __launch_bounds__(256)
+conv_shallow_kernel(const T* __restrict__ x, const T* __restrict__ w, void* __restrict__ y, ConvArgs a, ShallowArgs g) {
+    constexpr int TM = BM / 16, TN = BN / 16, kSteps = kShallowDepth / 8;
+    extern __shared__ float shallow_smem[];
+    float* as = shallow_smem;                              // [k][BM + 4]
+    float* bs = shallow_smem + g.k_padded * (BM + 4);      // [k][BN + 4]
+    const int tid = threadIdx.x, m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    chain_wait();
+    chain_release();
+    x = after_chain(x);
+    w = after_chain(w);
+    auto widen = [&](T raw, int type) {
+        if constexpr (sizeof(T) == 4) return static_cast<float>(raw);
+        else return type == DFGPU_BF16 ? __uint_as_float(static_cast<uint32_t>(raw) << 16) : __half2float(__ushort_as_half(raw));
+    };
+    // (channel, filter row and column) of product k
+    auto decode = [&](int k, int& c, int& r, int& s) {
+        const int outer = static_cast<int>(fast_divide(k, g.by_inner)), inner = k - outer * static_cast<int>(g.by_inner.divisor);
+        const int last = static_cast<int>(fast_divide(outer, g.by_middle)), middle = outer - last * static_cast<int>(g.by_middle.divisor);
+        if (CHANNELS_LAST) c = inner, s = middle, r = last;
+        else s = inner, r = middle, c = last;
+    };
+    T raw[kSteps];
+    // neighbouring threads take neighbouring channels (channels last) or pixels
+    const int a_k = CHANNELS_LAST ? tid & 7 : tid >> 5, a_row = CHANNELS_LAST ? tid >> 3 : tid & 31;
+#pragma unroll
+    for (int part = 0; part < BM / 32; ++part) {
+        const int row = a_row + part * 32, m = m0 + row;
+        const int line = static_cast<int>(fast_divide(m, g.by_q)), q = m - line * g.Q, n = static_cast<int>(fast_divide(line, g.by_p)), p = line - n * g.P;
+        const int ih0 = p * a.stride_h - a.pad_h, iw0 = q * a.stride_w - a.pad_w;
+#pragma unroll
+        for (int i = 0; i < kSteps; ++i) {
+            const int k = a_k + 8 * i;
+            raw[i] = T(0);
+            if (8 * i >= g.k_padded) continue;
+            int c, r, s;
+            decode(k, c, r, s);
+            const int ih = ih0 + r * a.dilation_h, iw = iw0 + s * a.dilation_w;
+            if (m < g.m_total && k < g.k_total && ih >= 0 && ih < g.H && iw >= 0 && iw < g.W) raw[i] = x[n * g.x_n + c * g.x_c + ih * g.x_h + iw * g.x_w];
+        }
+#pragma unroll
+        for (int i = 0; i < kSteps; ++i)
+            if (8 * i < g.k_padded) as[(a_k + 8 * i) * (BM + 4) + row] = widen(raw[i], a.x.dtype);
+    }
+#pragma unroll
+    for (int part = 0; part < BN / 32; ++part) {
+        const int row = (tid >> 3) + part * 32, channel = n0 + row;
+#pragma unroll
+        for (int i = 0; i < kSteps; ++i) {
+            const int k = (tid & 7) + 8 * i;
+            raw[i] = T(0);
+            if (8 * i >= g.k_padded) continue;
+            int c, r, s;
+            decode(k, c, r, s);
+            if (a.reverse) r = g.R - 1 - r, s = g.S - 1 - s;
+            if (channel < g.K && k < g.k_total) raw[i] = w[channel * g.w_k + c * g.w_c + r * g.w_r + s * g.w_s];
+        }
+#pragma unroll
+        for (int i = 0; i < kSteps; ++i)
+            if (8 * i < g.k_padded) bs[((tid & 7) + 8 * i) * (BN + 4) + row] = widen(raw[i], a.w.dtype);
+    }
+    __syncthreads();
+    const int ty = tid / 16, tx = tid % 16;
+    float acc[TM][TN] = {}, four[TM][TN] = {}, total[TM][TN] = {};
+    const bool chain = g.k_total < kChainDepth;
+    for (int k0 = 0; k0 < g.k_padded; k0 += 8) {
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) {
+            float av[TM], bv[TN];
+#pragma unroll
+            for (int i = 0; i < TM; ++i) av[i] = as[(k0 + kk) * (BM + 4) + ty * TM + i];
+#pragma unroll
+            for (int j = 0; j < TN; ++j) bv[j] = bs[(k0 + kk) * (BN + 4) + tx * TN + j];
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+        }
+        if (chain) continue;
+        const bool fold = (k0 & 24) == 24 || k0 + 8 >= g.k_padded;
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                four[i][j] = __fadd_rn(four[i][j], acc[i][j]);
+                acc[i][j] = 0.0f;
+                if (fold) {
+                    total[i][j] = __fadd_rn(total[i][j], four[i][j]);
+                    four[i][j] = 0.0f;
+                }
+            }
+    }
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const int m = m0 + ty * TM + i, k = n0 + tx * TN;
+        if (m >= g.m_total || k >= g.K) continue;
+        const int line = static_cast<int>(fast_divide(m, g.by_q)), q = m - line * g.Q, n = static_cast<int>(fast_divide(line, g.by_p)), p = line - n * g.P;
+        float value[TN];
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            value[j] = chain ? acc[i][j] : total[i][j];
+            if (a.epilogue.count > 0 && k + j < g.K) value[j] = apply_epilogue(value[j], a, n, k + j, p, q);
+        }
+        const int64_t target = n * a.y.stride[0] + k * a.y.stride[1] + p * a.y.stride[2] + q * a.y.stride[3];
+        if (TN == 4 && g.y_quads && k + 3 < g.K) {
+            *reinterpret_cast<float4*>(static_cast<float*>(y) + target) = make_float4(value[0], value[1], value[TN - 2], value[TN - 1]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < TN; ++j)
+                if (k + j < g.K) store_from_f32(y, a.y.dtype, target + j * a.y.stride[1], value[j]);
+        }
+    }
+}
+
 // Fast form of the implicit GEMM for the common f32 case: channels-last X with C % 16 == 0, a packed KRSC filter,
 // one group, no filter reversal. A 16-deep K slice then lies inside one filter tap, so the tap is decoded once
 // per slice for the whole CTA (no per-element divisions), X and W come in as 16-byte loads, and the loads of
@@ -377,6 +505,55 @@ bool f32_split_form(const dfgpu_conv_params& p, SplitForm& form) {
     return true;
 }
 
+// One group, at most kShallowDepth products per output, X and W of one type, every element within 2^31 of the first.
+bool shallow_form(const dfgpu_conv_params& p, const ConvArgs& a, void* const* tensors, ShallowArgs& g) {
+    const int64_t depth = p.x.dim[1] * p.w.dim[2] * p.w.dim[3], m_total = p.y.dim[0] * p.y.dim[2] * p.y.dim[3];
+    if (p.x.rank != 4 || a.groups != 1 || depth > kShallowDepth || p.x.dtype != p.w.dtype || m_total >= (1ll << 31) - 64) return false;
+    for (const dfgpu_tensor* t : {&p.x, &p.w}) {
+        int64_t last = 0;
+        for (int i = 0; i < 4; ++i) {
+            if (t->stride[i] < 0 || t->stride[i] >= (1ll << 31)) return false;
+            last += (t->dim[i] - 1) * t->stride[i];
+        }
+        if (last >= (1ll << 31)) return false;
+    }
+    const int64_t far = 1ll << 20;   // (row and column arithmetic stays within 32 bits)
+    if (p.x.dim[2] >= far || p.x.dim[3] >= far || p.y.dim[1] >= far || p.y.dim[2] >= far || p.y.dim[3] >= far || p.pre_pad[0] >= far || p.pre_pad[1] >= far ||
+        p.stride[0] >= 512 || p.stride[1] >= 512 || p.dilation[0] >= 512 || p.dilation[1] >= 512)
+        return false;
+    g.m_total = static_cast<int>(m_total);
+    g.k_total = static_cast<int>(depth);
+    g.k_padded = (g.k_total + 7) / 8 * 8;
+    g.x_n = static_cast<int>(p.x.stride[0]), g.x_c = static_cast<int>(p.x.stride[1]), g.x_h = static_cast<int>(p.x.stride[2]), g.x_w = static_cast<int>(p.x.stride[3]);
+    g.w_k = static_cast<int>(p.w.stride[0]), g.w_c = static_cast<int>(p.w.stride[1]), g.w_r = static_cast<int>(p.w.stride[2]), g.w_s = static_cast<int>(p.w.stride[3]);
+    g.P = static_cast<int>(p.y.dim[2]), g.Q = static_cast<int>(p.y.dim[3]), g.H = static_cast<int>(p.x.dim[2]), g.W = static_cast<int>(p.x.dim[3]);
+    g.K = static_cast<int>(p.y.dim[1]), g.R = static_cast<int>(p.w.dim[2]), g.S = static_cast<int>(p.w.dim[3]);
+    g.y_quads = p.y.dtype == DFGPU_F32 && p.y.stride[1] == 1 && p.y.stride[0] % 4 == 0 && p.y.stride[2] % 4 == 0 && p.y.stride[3] % 4 == 0 &&
+                (reinterpret_cast<uintptr_t>(tensors[2]) & 15u) == 0 ? 1 : 0;
+    const bool channels_last = p.x.stride[1] == 1;
+    g.by_q = make_fast_divisor(static_cast<uint32_t>(g.Q));
+    g.by_p = make_fast_divisor(static_cast<uint32_t>(g.P));
+    g.by_inner = make_fast_divisor(static_cast<uint32_t>(channels_last ? p.x.dim[1] : g.S));
+    g.by_middle = make_fast_divisor(static_cast<uint32_t>(channels_last ? g.S : g.R));
+    return true;
+}
+template <int BM, int BN>
+int launch_shallow(const dfgpu_conv_params& p, const ConvArgs& a, const ShallowArgs& g, void* const* tensors, cudaStream_t stream) {
+    const size_t dynamic = static_cast<size_t>(g.k_padded) * (BM + 4 + BN + 4) * 4;
+    constexpr int kMost = kShallowDepth * (BM + 4 + BN + 4) * 4;
+    const dim3 grid(static_cast<unsigned>((g.m_total + BM - 1) / BM), static_cast<unsigned>((g.K + BN - 1) / BN));
+    auto run = [&](auto kernel, auto element) -> int {
+        using T = decltype(element);
+        cudaError_t error = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
+        if (error != cudaSuccess) return fail(kExecutionFailed, "CONV_FPROP: cannot reserve %d bytes of shared memory: %s", kMost, cudaGetErrorString(error));
+        launch_chained(kernel, dim3(grid), dim3(256), dynamic, stream, static_cast<const T*>(tensors[0]), static_cast<const T*>(tensors[1]), tensors[2], a, g);
+        return check_launch("CONV_FPROP");
+    };
+    const bool channels_last = p.x.stride[1] == 1;
+    if (p.x.dtype == DFGPU_F32) return channels_last ? run(conv_shallow_kernel<BM, BN, true, float>, float{}) : run(conv_shallow_kernel<BM, BN, false, float>, float{});
+    return channels_last ? run(conv_shallow_kernel<BM, BN, true, uint16_t>, uint16_t{}) : run(conv_shallow_kernel<BM, BN, false, uint16_t>, uint16_t{});
+}
+
 int build_args(const dfgpu_conv_params& p, void* const* tensors, ConvArgs& a) {
     if (!valid_tensor(p.x) || !valid_tensor(p.w) || !valid_tensor(p.y))
         return fail(kInvalidShape, "CONV_FPROP: tensor rank or extent out of range");
@@ -510,6 +687,15 @@ extern "C" int dfgpu_conv_fprop(const dfgpu_conv_params* p, void* const* tensors
     status = choose_kernel(*p, a, kernel);
     if (status) return status;
     cudaStream_t stream = as_stream(stream_handle);
+    if (ShallowArgs shallow; kernel == DFGPU_CONV_IGEMM_FFMA && shallow_form(*p, a, tensors, shallow)) {
+        // Wherever neither the tensor cores nor 16-byte loads take the convolution (4 x 20 x 64 x 64 pixels, 1 x 1 to 128 channels: 39.4 us by 16
+        // products at a time, 12.3 here), and up to 96 products where every SM has one tile at most, at 2.6 us and 0.036 for every product (324
+        // pixels x 116 channels of 48 products 4.4 us, 6.7 on the tensor cores; of 124 products 7.1 and 6.6; 640 tiles of 40 products 10.6 and 6.8).
+        const int64_t tiles = (static_cast<int64_t>(shallow.m_total) + 31) / 32 * ((p->y.dim[1] + 31) / 32);
+        const bool other = (p->kernel == DFGPU_CONV_AUTO && conv_f32_flat(*p, tensors)) || nhwc_f32_fast_form(*p, tensors);
+        if (!other || (tiles <= sm_count() && shallow.k_total <= 96))
+            return tiles <= 4 * sm_count() ? launch_shallow<32, 32>(*p, a, shallow, tensors, stream) : launch_shallow<64, 64>(*p, a, shallow, tensors, stream);
+    }
     if (p->kernel == DFGPU_CONV_AUTO && kernel == DFGPU_CONV_IGEMM_FFMA && conv_f32_flat(*p, tensors))
         kernel = DFGPU_CONV_UMMA_F32X3_CLUSTER;
     if (kernel == DFGPU_CONV_UMMA_BF16) return launch_conv_umma(*p, tensors, stream);

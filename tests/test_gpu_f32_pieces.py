@@ -91,3 +91,21 @@ def test_shallow_reductions_are_f32_additions(depth, conv):
     for i in range(depth):
         want = (x[:, i : i + 1].double() * f[:, i].double() + want.double()).float()
     assert float((y == want).float().mean()) > 0.999
+
+
+@pytest.mark.parametrize("n,c,k,h,w,r", [(1, 5, 3, 4, 5, 1), (2, 20, 24, 56, 12, 1), (1, 23, 33, 9, 11, 1), (1, 24, 44, 16, 10, 1), (1, 96, 31, 8, 8, 1), (4, 22, 100, 64, 64, 1), (1, 8, 40, 30, 41, 3),
+                                         (3, 14, 65, 33, 31, 3), (1, 3, 64, 65, 66, 5)])
+@pytest.mark.parametrize("layout", ["nhwc", "nchw"])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_conv_shallow_reduction(n, c, k, h, w, r, layout, shift):
+    """The whole depth at once: one chain below 24 products, else sums of eight, of four of them and of those. Depths that are no eights,
+    pixels and channels that are no tiles, operands off the 16-byte boundary."""
+    g = torch.Generator(device="cuda").manual_seed(c * 131 + r)
+    x, f = torch.randn(n, c, h, w, device="cuda", generator=g), torch.randn(k, c, r, r, device="cuda", generator=g)
+    place = lambda t: torch.zeros(t.numel() + shift, device="cuda")[shift:].copy_((t.permute(0, 2, 3, 1) if layout == "nhwc" else t).reshape(-1))
+    y = torch.full((n * k * h * w,), float("nan"), device="cuda")
+    doc = graphs.c1_conv(layout, n, c, h, w, k, r, r // 2)
+    run(doc, {1: place(x), 2: place(f)}, {3: y})
+    y = y.view(n, h, w, k).permute(0, 3, 1, 2) if layout == "nhwc" else y.view(n, k, h, w)
+    conv = lambda a, b: torch.nn.functional.conv2d(a.double().cpu(), b.double().cpu(), padding=r // 2)
+    assert torch.all((y.double().cpu() - conv(x, f)).abs() <= max(c * r * r * 2.0 ** -24, pieces_bound(c * r * r)) * conv(x.abs(), f.abs()))
