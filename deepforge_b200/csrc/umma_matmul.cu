@@ -569,7 +569,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         bool ok = true;
         for (int i = first_item; i < args.items && ok; i += item_step) {
             const Item item = item_at(args, i);
-            const int columns = item.width / CG, boxes = columns / args.b_box_columns;
+            const int columns = item.width / CG, boxes = (columns + args.b_box_columns - 1) / args.b_box_columns;
             const int row0 = (item.m_tile * CG + (CG == 2 ? rank : 0)) * kRows, col0 = item.col0 + (CG == 2 ? rank * columns : 0);
             for (int kb = kb_begin; kb < kb_end; ++kb) {
                 ok = mbar_wait_warp(empty_bar(stage), phase, 501 + kCode);
@@ -577,7 +577,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 if (leader) {
                     const uint32_t bar = counted_on + 8u * stage;
                     constexpr int kPerRow = kSixteenBits ? 64 : 128;   // elements of K per block
-                    if (CG == 1 || rank == 0) mbar_expect_tx(full_bar(stage), CG * kPieceCount * (args.a_bytes + columns * kRowBytes));
+                    if (CG == 1 || rank == 0) mbar_expect_tx(full_bar(stage), CG * kPieceCount * (args.a_bytes + boxes * args.b_box_bytes));
                     // (pieces: the rows of one follow those of the one before in the same map. A tile that hangs over the end of a
                     // piece reads the next one's first rows, for rows and columns of C that are not stored; past the end of K it is A that holds zeros.)
 #pragma unroll
@@ -983,8 +983,13 @@ int rows_of_a(const Problem& p, int cg) { return cg == 1 && p.M < kRows ? static
 bool has_pieces(const Problem& p) { return p.kind == kPieces || p.kind == kPiecesSummed; }
 bool in_registers(const Problem& p) { return p.kind == kSummed || p.kind == kCodesSummed; }
 bool scaled(const Problem& p) { return p.kind == kScaled || p.kind == kScaledSummed; }
-int stage_bytes(const Problem& p, int bn, int cg, int a_rows) { return (a_rows + bn / cg) * kRowBytes * (has_pieces(p) ? 3 : 1) + (scaled(p) ? 2048 : 0); }
 bool sixteen_bits(const Problem& p) { return p.kind == kSixteen || has_pieces(p) || p.kind == kSummed; }
+// Columns of B that a CTA loads for bn / cg of its own: N-major copies come in whole boxes, so that 96 columns cost 128.
+int loaded_columns(const Problem& p, int bn, int cg) {
+    const int chunk = sixteen_bits(p) ? 64 : 128;
+    return p.b_mn_major ? (bn / cg + chunk - 1) / chunk * chunk : bn / cg;
+}
+int stage_bytes(const Problem& p, int bn, int cg, int a_rows) { return (a_rows + loaded_columns(p, bn, cg)) * kRowBytes * (has_pieces(p) ? 3 : 1) + (scaled(p) ? 2048 : 0); }
 int ring_bytes(int stages, int stage_size) { return (stages - 1) * stage_size + std::max(stage_size, kABytes); }
 int stages_that_fit(int stage_size, int budget) {
     int stages = std::min(kMaxStages, budget / stage_size);
@@ -1000,12 +1005,16 @@ struct Shape {
 };
 
 // The shape with the fewest estimated clocks. One K block of a CTA costs the longest of
-//   products       2 bn clocks (128 rows per SM, 16-bit and FP8 alike: a block is 128 bytes of K)
-//   shared memory  every operand byte written and read once at 128 B per clock: 2 (rows of A + columns of B)
-//   L2             the same bytes at about 48 per clock and SM when all SMs fetch, or what the ring holds per ~2300 clocks of latency
+//   products       2.3 bn clocks (128 rows per SM, 16-bit and FP8 alike: a block is 128 bytes of K)
+//   shared memory  every operand byte written and read once: 1.8 (rows of A + columns of B)
+//   L2             the same bytes at 48 a clock and SM, 6300 for all SMs that fetch, or what the ring holds per 3400 clocks of latency
 // and a round over the SMs costs its blocks (a last round that at most half fills the SMs is cut into half tiles: 4096^3 is 512
-// tiles of 128 x 256 on 148 SMs, three rounds and 68 tiles, which become 136 halves), a fill of ~2000 clocks and the last tile's epilogue. Splitting K divides the
-// blocks and adds ~2500 clocks of exchange (5000 with block scales).
+// tiles of 128 x 256 on 148 SMs, three rounds and 68 tiles, which become 136 halves) and, where there are several, an epilogue of 12 bn.
+// Splitting K divides the blocks and adds an exchange that grows with the partial tile: 230 + 0.31 x rows x bn (800 more with block scales,
+// whose six loading warps also fall behind once they have more than a block each). The constants are a fit to the times of every
+// shape on 726 products of 1 to 8192 rows, 64 to 8192 columns and depths: the shape taken is 1.0 % slower than the best of
+// them in the mean, 3.5 % with 2 bn, 2 (rows + columns), 48 a clock and exchanges of 2500 and 5000 whatever the tile
+// (15 x 1632 x 816 MXFP8 12.1 -> 9.5 us, 1309 x 2496 x 648 bf16 13.4 -> 12.0).
 Shape choose_shape(const Problem& p) {
     const int64_t blocks = (p.K * p.in_bytes + kRowBytes - 1) / kRowBytes;
     constexpr int clusters_at_once[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};   // (cudaOccupancyMaxActiveClusters, by CTAs per cluster)
@@ -1014,7 +1023,7 @@ Shape choose_shape(const Problem& p) {
     for (int cg = 1; cg <= 2; ++cg)
         for (int bn = 64; bn <= 256; bn += 64) {
             const int chunk = sixteen_bits(p) ? 64 : 128;   // columns of one N-major copy
-            if (p.b_mn_major && (bn / cg) % chunk != 0) continue;
+            if (p.b_mn_major && (bn / cg) % chunk != 0 && !(cg == 2 && bn == 192 && !has_pieces(p) && !scaled(p))) continue;
             if (p.out_dtype == DFGPU_E4M3 && bn % 128 != 0) continue;   // (whole 128-byte boxes)
             if (scaled(p) && bn % 128 != 0) continue;           // (whole chunks of column scales)
             if (cg == 2 && bn < 128) continue;
@@ -1027,7 +1036,7 @@ Shape choose_shape(const Problem& p) {
                 if (splits > 1 && (bn > 128 || splits > blocks || tiles * splits > sms)) break;
                 const int64_t k_per_split = (blocks + splits - 1) / splits;
                 if (splits > 1 && k_per_split * (splits - 1) >= blocks) continue;   // (no CTA without a block)
-                const int64_t slots = cg == 2 ? sms / 2 : clusters_at_once[splits];
+                const int64_t slots = cg == 2 ? sms / 2 : clusters_at_once[splits] - (scaled(p) && splits > 1 ? 1 : 0);   // (behind a quantize launch the last cluster often waits)
                 double rounds = static_cast<double>((tiles + slots - 1) / slots);
                 int64_t halved = 0;
                 const int half = bn / 2;
@@ -1038,9 +1047,13 @@ Shape choose_shape(const Problem& p) {
                 }
                 const double in_flight = static_cast<double>(stages_that_fit(stage_size, kSmemBudget - 2 * kStageBox)) * stage_size;
                 const double products = has_pieces(p) ? 6.0 : 1.0, pieces = has_pieces(p) ? 3.0 : 1.0;
-                const double summed = in_registers(p) ? 150.0 + 2.0 * bn : (p.kind == kScaledSummed ? 250.0 + 3.0 * bn : 0.0);   // the epilogue's loads and additions of a block
-                const double block = std::max({summed, products * 2.0 * bn, (products + pieces) * (rows + bn / cg), pieces * (rows + bn / cg) * kRowBytes / std::min(48.0, in_flight / 2300.0)});
-                const double clocks = rounds * (k_per_split * block) + 2000.0 + bn * 6.0 + (splits > 1 ? (scaled(p) ? 5000.0 : 2500.0) : 0.0) + (cg == 2 ? 1500.0 : 0.0);
+                const double summed = in_registers(p) ? (cg == 2 ? 1.25 : 1.0) * (150.0 + 2.0 * bn) : (p.kind == kScaledSummed ? 250.0 + 3.0 * bn : 0.0);   // the epilogue's loads and additions of a block
+                const int columns = loaded_columns(p, bn, cg);
+                const double active = static_cast<double>(std::min<int64_t>(sms, tiles * cg * splits));
+                const double rate = std::min({48.0, 6300.0 / active, in_flight / 3400.0});
+                const double block = std::max({summed, products * 2.3 * bn, 0.9 * (products * (rows + bn / cg) + pieces * (rows + columns)), pieces * (rows + columns) * kRowBytes / rate});
+                const double exchange = splits > 1 ? 230.0 + 0.31 * std::min<double>(rows, static_cast<double>(p.M)) * bn + (scaled(p) ? 800.0 : 0.0) : 0.0;
+                const double clocks = rounds * (k_per_split * block + (rounds > 1.0 ? 12.0 * bn : 0.0)) + 2000.0 + exchange + (scaled(p) && k_per_split > 6 ? 450.0 : 0.0) + (cg == 2 ? 1480.0 : 0.0);
                 if (best.cg == 0 || clocks < best.clocks) best = Shape{cg, bn, splits, static_cast<int>(k_per_split), tiles, halved, clocks};
             }
         }
