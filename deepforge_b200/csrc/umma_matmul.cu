@@ -258,22 +258,22 @@ __device__ __forceinline__ void add_operand(float (&v)[COUNT], const void* data,
 }
 
 struct Scalars {
-    bool on;
     float descale_a, descale_b, scale_c;
     float magnitude;   // largest |value| of this thread so far (NaN sticks)
 };
+template <bool CODES>
 __device__ __forceinline__ Scalars load_scalars(const TileArgs& args) {
     Scalars s{};
-    if (args.descale_a != nullptr) {
-        s.on = true;
+    if constexpr (CODES) {
         s.descale_a = *args.descale_a;
         s.descale_b = *args.descale_b;
         s.scale_c = *args.scale_c;
     }
     return s;
 }
+template <bool CODES>
 __device__ __forceinline__ void fold_amax(const TileArgs& args, const Scalars& s, int lane, bool ok) {
-    if (!s.on) return;
+    if constexpr (!CODES) return;
     unsigned int bits = s.magnitude != s.magnitude ? 0x7fc00000u : __float_as_uint(s.magnitude);
     bits = __reduce_max_sync(0xffffffffu, bits);
     if (lane == 0 && bits != 0u && ok) atomicMax(args.amax_bits, bits);
@@ -281,19 +281,22 @@ __device__ __forceinline__ void fold_amax(const TileArgs& args, const Scalars& s
 
 // COUNT neighbouring columns of one row: fused steps, then MATMUL_FP8's scalars. `row_live`: the row exists. `ahead`: the first
 // step's operand, where it was loaded ahead.
-template <int COUNT>
+// CODES: MATMUL_FP8, which has the scalars and no steps; the others have none of the scalars (neither is compiled into the other's kernel).
+template <bool CODES, int COUNT>
 __device__ __forceinline__ void apply_steps(const TileArgs& args, float (&v)[COUNT], int row, int col0, bool row_live, Scalars& scalars, const uint32_t (*ahead)[COUNT / 2] = nullptr) {
     const int live = args.n_total - col0;
-    if (ahead != nullptr) add_words<COUNT>(v, *ahead, args.step_dtype[0]);
-    for (int s = ahead != nullptr ? 1 : 0; s < args.step_count; ++s) {
-        const int kind = args.step_kind[s];
-        if (kind == kStepRelu) {
-            relu_values(v, args.relu_lower[s], args.relu_upper[s], args.relu_slope[s]);
-        } else if (kind == kStepBias || row_live) {
-            add_operand<COUNT>(v, args.step_data[s], args.step_dtype[s], (kind == kStepBias ? 0 : row * args.step_ld[s]) + col0, live, args.step_vector[s] != 0);
+    if constexpr (!CODES) {
+        if (ahead != nullptr) add_words<COUNT>(v, *ahead, args.step_dtype[0]);
+        for (int s = ahead != nullptr ? 1 : 0; s < args.step_count; ++s) {
+            const int kind = args.step_kind[s];
+            if (kind == kStepRelu) {
+                relu_values(v, args.relu_lower[s], args.relu_upper[s], args.relu_slope[s]);
+            } else if (kind == kStepBias || row_live) {
+                add_operand<COUNT>(v, args.step_data[s], args.step_dtype[s], (kind == kStepBias ? 0 : row * args.step_ld[s]) + col0, live, args.step_vector[s] != 0);
+            }
         }
     }
-    if (scalars.on) {
+    if constexpr (CODES) {
         float top = scalars.magnitude;
 #pragma unroll
         for (int e = 0; e < COUNT; ++e) {
@@ -510,6 +513,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     constexpr int kCode = KIND == kSixteen ? 0 : (KIND == kCodes || KIND == kCodesSummed ? 20 : (KIND == kScaled ? 40 : (kHasPieces<KIND> ? 60 : (KIND == kSummed ? 80 : 90))));
     constexpr bool kSixteenBits = KIND == kSixteen || kHasPieces<KIND> || KIND == kSummed;
     constexpr int kPieceCount = kHasPieces<KIND> ? 3 : 1;
+    constexpr bool kCodesOnly = KIND == kCodes || KIND == kCodesSummed;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* generic_base = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -709,7 +713,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             const uint32_t leader_bars = CG == 2 ? address_in(bar_base, 0) : bar_base;
             const int staging0 = args.staging_offset + g * args.staging_boxes * kStageBox;
             const int box_columns = !args.tma_store || args.out_dtype == DFGPU_F32 ? 32 : (args.out_dtype == DFGPU_E4M3 ? 128 : 64);
-            Scalars scalars = load_scalars(args);
+            Scalars scalars = load_scalars<kCodesOnly>(args);
             int stored = 0;   // boxes this group has sent off
             int local = 0;
             const bool ahead = (KIND == kSixteen || KIND == kPieces) && args.step_count > 0 && args.step_kind[0] != kStepRelu && args.step_dtype[0] != DFGPU_F32;
@@ -776,9 +780,9 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                             for (int e = 0; e < 16; ++e) operand[e] = first_operand[e];
                             const bool same_box = part + 1 < box_columns / 32;
                             if (same_box || b + 2 < boxes) load_ahead(args, first_operand, out_row, same_box ? col + 32 : item.col0 + (b + 2) * box_columns, row_live);
-                            apply_steps<32>(args, v, out_row, col, row_live, scalars, &operand);
+                            apply_steps<kCodesOnly, 32>(args, v, out_row, col, row_live, scalars, &operand);
                         } else {
-                            apply_steps<32>(args, v, out_row, col, row_live, scalars);
+                            apply_steps<kCodesOnly, 32>(args, v, out_row, col, row_live, scalars);
                         }
                         if (args.tma_store) {
                             uint8_t* target = generic_base + staging + row * 128;
@@ -824,7 +828,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             }
             if (args.tma_store && row == 0) tma_store_wait_all();
             __syncwarp();
-            fold_amax(args, scalars, lane, ok);
+            fold_amax<kCodesOnly>(args, scalars, lane, ok);
         }
     } else if (kHasScales<KIND>) {
         // ---- scale loaders: warp i of the six owns the slots i and i + 6 ----
@@ -884,7 +888,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const int row0 = item.m_tile * kRows, live_rows = min(kRows, args.m_total - row0);
         const int share = (live_rows + args.splits - 1) / args.splits, begin = rank * share, end = min(live_rows, begin + share);
         const int quads = bn / 4;
-        Scalars scalars = load_scalars(args);
+        Scalars scalars = load_scalars<kCodesOnly>(args);
         const bool healthy = g_device_status == 0;
         for (int i = threadIdx.x; i < (end - begin) * quads; i += blockDim.x) {
             const int row = begin + i / quads, unit = i % quads;
@@ -905,11 +909,11 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 v[2] = __fadd_rn(v[2], part[z].z);
                 v[3] = __fadd_rn(v[3], part[z].w);
             }
-            apply_steps<4>(args, v, row0 + row, col, true, scalars);
+            apply_steps<kCodesOnly, 4>(args, v, row0 + row, col, true, scalars);
             if (healthy) store_four(args, v, row0 + row, col);
         }
         __syncwarp();
-        fold_amax(args, scalars, lane, healthy);
+        fold_amax<kCodesOnly>(args, scalars, lane, healthy);
         cluster_sync_all();   // no CTA leaves while another still reads its partial tile
     }
     tc_fence_before();
