@@ -508,9 +508,12 @@ sdpa_paged_decode_kernel(SdpaArgs a, float* __restrict__ partial, int max_chunks
 // loaded at once, before the lengths say which chunks hold keys: every warp takes all maxima and sums, a chunk per lane and
 // group of 32, and each thread its channel of the first 32 chunks. (Maxima, then sums, then values took three trips to the L2 cache
 // and two barriers more.) Sums add up lane by lane, then group by group; values chunk by chunk.
+// CHUNKS: up to 8, or 32 at a time. (Large batches have few chunks each and thousands of CTAs: 96 registers for 32 values and the next 32
+// let five CTAs on an SM, 32 registers for 8 sixteen: 89 sequences of two chunks 66.8 us in all and 64.7.)
+template <int CHUNKS>
 __global__ void __launch_bounds__(128)
 sdpa_decode_merge_kernel(SdpaArgs a, const float* __restrict__ partial, int max_chunks, int chunk_keys) {
-    constexpr int kAhead = 32, kGroups = 4;
+    constexpr int kAhead = CHUNKS, kGroups = CHUNKS == 8 ? 1 : 4;
     chain_begin();
     partial = after_chain(partial);
     const int64_t row = blockIdx.x;  // b * Hq + h
@@ -537,19 +540,23 @@ sdpa_decode_merge_kernel(SdpaArgs a, const float* __restrict__ partial, int max_
         if (g * 32 + lane >= chunks) maxima[g] = -INFINITY;   // (never written, as an empty chunk's values)
         total_max = fmaxf(total_max, maxima[g]);
     }
-    for (int c = kGroups * 32 + lane; c < chunks; c += 32) total_max = fmaxf(total_max, base[c * kPartialStride + kDecodeD]);
+    if (CHUNKS > 8)
+        for (int c = kGroups * 32 + lane; c < chunks; c += 32) total_max = fmaxf(total_max, base[c * kPartialStride + kDecodeD]);
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) total_max = fmaxf(total_max, __shfl_xor_sync(0xffffffffu, total_max, s));
     float total_sum = 0.0f, value = 0.0f;
     for (int first = 0; first < chunks; first += 32) {   // 32 chunks at a time, the next ones' values on their way
-        float next[kAhead];
+        float next[CHUNKS == 8 ? 1 : kAhead];
+        if constexpr (CHUNKS > 8) {
 #pragma unroll
-        for (int c = 0; c < kAhead; ++c) next[c] = first + 32 + c < chunks ? base[(first + 32 + c) * kPartialStride + d] : 0.0f;
+            for (int c = 0; c < kAhead; ++c) next[c] = first + 32 + c < chunks ? base[(first + 32 + c) * kPartialStride + d] : 0.0f;
+        }
         const int g = first / 32;
-        const bool in = first + lane < chunks;
-        const float* own = base + (first + lane) * kPartialStride + kDecodeD;
         float m = -INFINITY, sum = 0.0f;
-        if (g >= kGroups && in) m = own[0], sum = own[1];
+        if (CHUNKS > 8 && g >= kGroups && first + lane < chunks) {
+            const float* own = base + (first + lane) * kPartialStride + kDecodeD;
+            m = own[0], sum = own[1];
+        }
 #pragma unroll
         for (int i = 0; i < kGroups; ++i)
             if (g == i) m = maxima[i], sum = sums[i];
@@ -562,7 +569,7 @@ sdpa_decode_merge_kernel(SdpaArgs a, const float* __restrict__ partial, int max_
         for (int c = 0; c < kAhead; ++c) {
             const float factor = __shfl_sync(0xffffffffu, weight, c);   // (negative past the last chunk too)
             value = factor < 0.0f ? value : fmaf(ahead[c], factor, value);
-            ahead[c] = next[c];
+            if constexpr (CHUNKS > 8) ahead[c] = next[c];
         }
     }
     float result = total_sum == 0.0f ? 0.0f : value / total_sum;   // (a NaN sum is a NaN result)
@@ -841,7 +848,7 @@ extern "C" int dfgpu_sdpa_forward(const dfgpu_sdpa_params* p, void* const* tenso
         status = launch_decode_umma(*p, tensors, scratch, a.prefix_ok, stream);
         if (status) return status;
         const int chunks = decode_umma_chunks(*p);
-        launch_chained(sdpa_decode_merge_kernel, dim3(static_cast<unsigned>(p->q.dim[0] * p->q.dim[1])), dim3(kDecodeD), 0, stream, a, static_cast<const float*>(scratch), chunks, decode_umma_chunk_keys(*p));
+        launch_chained(chunks <= 8 ? sdpa_decode_merge_kernel<8> : sdpa_decode_merge_kernel<32>, dim3(static_cast<unsigned>(p->q.dim[0] * p->q.dim[1])), dim3(kDecodeD), 0, stream, a, static_cast<const float*>(scratch), chunks, decode_umma_chunk_keys(*p));
         return check_launch("SDPA decode merge");
     }
     if (kernel == DFGPU_SDPA_PAGED_DECODE) {
@@ -860,7 +867,7 @@ extern "C" int dfgpu_sdpa_forward(const dfgpu_sdpa_params* p, void* const* tenso
         }
         status = check_launch("SDPA paged decode");
         if (status) return status;
-        launch_chained(sdpa_decode_merge_kernel, dim3(static_cast<unsigned>(p->q.dim[0] * p->q.dim[1])), dim3(kDecodeD), 0, stream, a, partial, chunks, kDecodeChunk);
+        launch_chained(chunks <= 8 ? sdpa_decode_merge_kernel<8> : sdpa_decode_merge_kernel<32>, dim3(static_cast<unsigned>(p->q.dim[0] * p->q.dim[1])), dim3(kDecodeD), 0, stream, a, partial, chunks, kDecodeChunk);
         return check_launch("SDPA decode merge");
     }
     int64_t rows = p->q.dim[0] * p->q.dim[1] * p->q.dim[2];
@@ -963,6 +970,6 @@ extern "C" int dfgpu_sdpa_paged_decode_static(const dfgpu_sdpa_params* p, void* 
     }
     status = check_launch("SDPA static decode");
     if (status) return status;
-    launch_chained(sdpa_decode_merge_kernel, dim3(static_cast<unsigned>(p->q.dim[0] * p->q.dim[1])), dim3(kDecodeD), 0, stream, a, partial, chunks, kDecodeChunk);
+    launch_chained(chunks <= 8 ? sdpa_decode_merge_kernel<8> : sdpa_decode_merge_kernel<32>, dim3(static_cast<unsigned>(p->q.dim[0] * p->q.dim[1])), dim3(kDecodeD), 0, stream, a, partial, chunks, kDecodeChunk);
     return check_launch("SDPA static decode merge");
 }
