@@ -126,6 +126,21 @@ def test_f32_results_do_not_lose_accuracy_with_depth(m, k, n, c_ld, io, b_k_majo
     assert float(error) <= 2.0 ** -21 + 2.0 ** -25 * (k / 64) ** 0.5
 
 
+@pytest.mark.parametrize("m,k,n,blocks", [(128, 384, 1152, 1), (128, 640, 3840, 3), (128, 896, 3712, 4), (128, 2048, 2688, 6), (128, 3328, 1536, 7)])
+@pytest.mark.parametrize("b_k_major", [False, True])
+def test_f32_results_of_whole_tiles_keep_their_splits(m, k, n, blocks, b_k_major):
+    """An accumulator loses 2^-24 of its value for every block of 64 it takes (sums are cut off toward zero), and adding the splits of K as
+    much once more. With `blocks` of them; K in one or two accumulators is two to four times as far off."""
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    doc = graphs.document("tiles", [graphs.matmul_node("matmul", 1, 2, 4)], [graphs.tensor(1, "A", [m, k], "BFLOAT16"), graphs.tensor(2, "B", [k, n], "BFLOAT16", [1, k] if b_k_major else [n, 1]), graphs.tensor(4, "C", [m, n], "FLOAT")], io="BFLOAT16")
+    a, b = (torch.randn(count, device="cuda", generator=g).to(torch.bfloat16) for count in (m * k, k * n))
+    buffers = {1: a, 2: b}
+    assert [s["kernel"] for s in run(doc, buffers).steps()] == [dfgpu.MATMUL_UMMA_BF16]
+    want = a.view(m, k).double() @ (b.view(n, k).t() if b_k_major else b.view(k, n)).double()
+    error = (buffers[4].view(m, n).double() - want).norm() / want.norm()
+    assert float(error) <= (blocks + 1) * 2.0 ** -24
+
+
 @pytest.mark.parametrize("m,k,n", [(1, 32, 80), (77, 288, 272), (300, 544, 528), (129, 4128, 144), (2050, 288, 2064), (1026, 32736, 1040)])
 def test_f32_results_of_block_scaled_codes_do_not_lose_accuracy_with_depth(m, k, n):
     """As above with blocks of 128 codes, whose products hold eight significant bits: half the bound of a block."""
