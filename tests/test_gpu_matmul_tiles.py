@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 from deepforge_b200 import dfgpu, graphs, runtime
+from test_matmul_shape_cpu import CODES, N_MAJOR_192, SIXTEEN
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
@@ -71,6 +72,32 @@ def test_fp8_codes(m, k, n, c_type, b_k_major):
     close(buffers[26].view(m, n), a, b, lambda p: p * (0.5 * 0.25 * 0.125), c_type, k)
     top = float((a @ b).abs().max()) * 0.125
     assert abs(float(buffers[27][0]) - top) <= k * 2.0 ** -24 * float((a.abs() @ b.abs()).max())
+
+
+@pytest.mark.parametrize("m,k,n", N_MAJOR_192[SIXTEEN])
+@pytest.mark.parametrize("io", ["BFLOAT16", "HALF"])
+def test_sixteen_bit_columns_of_one_and_a_half_boxes(m, k, n, io):
+    """B [K, N] in shares of 96 columns: a box of 64 and half of the next, the other half not multiplied."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    doc = graphs.document("tiles", [graphs.matmul_node("matmul", 1, 2, 5), graphs.pointwise_node("bias", "ADD", 5, 4, 3)], [graphs.tensor(1, "A", [m, k], io), graphs.tensor(2, "B", [k, n], io), graphs.tensor(3, "bias", [1, n], io),
+                          graphs.tensor(4, "C", [m, n], io), graphs.tensor(5, "p", [m, n], virtual=True)], io=io)
+    buffers = {uid: torch.randn(count, device="cuda", generator=g).to(TORCH[io]) for uid, count in ((1, m * k), (2, k * n), (3, n))}
+    assert [s["kernel"] for s in run(doc, buffers).steps()] == [dfgpu.MATMUL_UMMA_BF16]
+    close(buffers[4].view(m, n), buffers[1].view(m, k).double(), buffers[2].view(k, n).double(), lambda p: p + buffers[3].double(), io, k)
+
+
+@pytest.mark.parametrize("m,k,n", N_MAJOR_192[CODES])
+@pytest.mark.parametrize("c_type", ["BFLOAT16", "HALF"])
+def test_fp8_columns_of_three_quarters_of_a_box(m, k, n, c_type):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    codes = {uid: (torch.randn(count, device="cuda", generator=g) * 16).to(torch.float8_e4m3fn) for uid, count in ((21, m * k), (22, k * n))}
+    buffers = {uid: c.view(torch.uint8) for uid, c in codes.items()}
+    buffers.update({uid: torch.full((1,), v, device="cuda") for uid, v in ((23, 0.5), (24, 0.25), (25, 0.125))})
+    run(graphs.matmul_fp8(m, k, n, c_type, batch=()), buffers)
+    a, b = codes[21].double().view(m, k), codes[22].double().view(k, n)
+    assert float((a @ b).abs().max()) * (0.5 * 0.25 * 0.125) < 65504
+    close(buffers[26].view(m, n), a, b, lambda p: p * (0.5 * 0.25 * 0.125), c_type, k)
+    assert abs(float(buffers[27][0]) - float((a @ b).abs().max()) * 0.125) <= k * 2.0 ** -24 * float((a.abs() @ b.abs()).max())
 
 
 @pytest.mark.parametrize("m,k,n", [(m, (k + 31) // 32 * 32, n) for m, k, n in EXTENTS if n > 64])

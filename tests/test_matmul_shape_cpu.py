@@ -1,0 +1,55 @@
+"""What choose_shape() (csrc/matmul_shape.cuh) takes, as compiled for the host: the shapes of work that the GPU tests mean to run, and
+the splits of K on which the accuracy of f32 results rests."""
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parent.parent
+SIXTEEN, CODES = 0, 1
+TYPES = {"FLOAT": (0, 4), "HALF": (1, 2), "BFLOAT16": (2, 2)}
+# M, K, N with B [K, N] that two SMs take as tiles of 192 columns, 96 of them a CTA's. The last tile has all of them, 16 (none left for the
+# second CTA), 80, 96 (the first CTA's all), 112 and 144; a second round of tiles; rows past 256 and K with a remainder throughout.
+N_MAJOR_192 = {kind: [(1030, 1040, 2112), (1030, 528, 2128), (1030, 528, 2192), (1030, 528, 2208), (1030, 528, 2224), (1030, 1040, 2064), several]
+               for kind, several in ((SIXTEEN, (3333, 528, 1808)), (CODES, (2050, 528, 4432)))}
+
+
+@pytest.fixture(scope="module")
+def shapes(tmp_path_factory):
+    if not shutil.which("g++"):
+        pytest.skip("no C++ compiler")
+    folder = tmp_path_factory.mktemp("shape")
+    source = folder / "shape.cpp"
+    source.write_text("""#include <cstdio>
+#include "matmul_shape.cuh"
+int main() {
+    dfgpu::Problem p{};
+    int n_major;
+    while (scanf("%d %ld %ld %ld %d %d %d", &p.kind, &p.M, &p.K, &p.N, &n_major, &p.out_dtype, &p.out_bytes) == 7) {
+        p.b_mn_major = n_major != 0;
+        p.in_bytes = dfgpu::sixteen_bits(p) ? 2 : 1;
+        const dfgpu::Shape s = dfgpu::choose_shape(p);
+        printf("%d %d %d %d\\n", s.cg, s.bn, s.splits, s.k_per_split);
+    }
+}
+""")
+    subprocess.run(["g++", "-std=c++17", "-I", str(ROOT / "include"), "-I", str(ROOT / "deepforge_b200" / "csrc"), str(source), "-o", str(folder / "shape")], check=True)
+
+    def ask(kind, m, k, n, n_major, c_type):
+        dtype, size = TYPES[c_type]
+        line = f"{kind} {m} {k} {n} {int(n_major)} {dtype} {size}\n"
+        return tuple(int(v) for v in subprocess.run([str(folder / "shape")], input=line, check=True, capture_output=True, text=True).stdout.split())
+    return ask
+
+
+@pytest.mark.parametrize("kind", sorted(N_MAJOR_192))
+@pytest.mark.parametrize("c_type", ["BFLOAT16", "HALF"])
+def test_n_major_columns_of_one_and_a_half_boxes(shapes, kind, c_type):
+    for m, k, n in N_MAJOR_192[kind]:
+        assert shapes(kind, m, k, n, True, c_type)[:3] == (2, 192, 1), (m, k, n)
+
+
+@pytest.mark.parametrize("m,k,n,blocks", [(128, 384, 1152, 1), (128, 640, 3840, 3), (128, 896, 3712, 4), (128, 2048, 2688, 6), (128, 3328, 1536, 7)])
+def test_f32_results_split_k(shapes, m, k, n, blocks):
+    assert shapes(SIXTEEN, m, k, n, True, "FLOAT")[3] == blocks
