@@ -63,24 +63,25 @@ struct Shape {
 //   L2             the same bytes at 48 a clock and SM, 6300 for all SMs that fetch, or what the ring holds per 3400 clocks of latency
 // and a round over the SMs costs its blocks (a last round that at most half fills the SMs is cut into half tiles: 4096^3 is 512
 // tiles of 128 x 256 on 148 SMs, three rounds and 68 tiles, which become 136 halves) and, where there are several, an epilogue of 12 bn.
-// Splitting K divides the blocks and adds an exchange that grows with the partial tile: 230 + 0.31 x rows x bn (800 more with block scales,
-// whose six loading warps also fall behind once they have more than a block each). The constants are a fit to the times of every
-// shape on 726 products of 1 to 8192 rows, 64 to 8192 columns and depths: the shape taken is 1.0 % slower than the best of
-// them in the mean, 3.5 % with 2 bn, 2 (rows + columns), 48 a clock and exchanges of 2500 and 5000 whatever the tile
-// (15 x 1632 x 816 MXFP8 12.1 -> 9.5 us, 1309 x 2496 x 648 bf16 13.4 -> 12.0).
-// f32 results keep those costs, which split K more often: an accumulator is off by 2^-24 of its value for every block it takes, which
-// a 16-bit result does not show and an f32 result does (128 x 640 x 3840 bf16 to f32: 1.7e-7 from 64 bits in four splits, 5.9e-7 in one;
-// 128 x 3328 x 1536 4.0e-7 and 6.4e-7).
-inline Shape choose_shape(const Problem& p) {
+// Splitting K divides the blocks and adds an exchange that grows with the partial tile, 800 + 0.31 x rows x bn (1000 more with block
+// scales, whose six loading warps also fall behind once they have more than a block each), and shares out the epilogue, which counts
+// where it waits for a full f32 operand (`f32_operands` of them): 14 clocks for every column that a group of its warps takes.
+// Former costs -> these, in us: 777 x 4096 x 3072 bf16 [K, N] 26.9 (256 columns) -> 21.6 (192), 2050 x 1040 x 1040 13.0 -> 11.5, MXFP8
+// 15 x 1632 x 816 7.7 -> 6.3 (more splits). Where an exchange of 230 split K: 1 x 136 x 3648 bf16 4.0 whole, 5.0 in two. With bias, ReLU and a
+// full f32 operand, 128 x 384 x 384 f16: 6.0 in six, 7.5 whole.
+// f32 results and f32 operands (pieces) keep the former costs. Those split K more often, and an accumulator is off by 2^-24 of its value
+// for every block it takes, which a 16-bit result does not show and an f32 result does (128 x 640 x 3840 bf16 to f32: 1.7e-7 from
+// 64 bits in four splits, 5.9e-7 in one; 128 x 3328 x 1536 4.0e-7 and 6.4e-7). For pieces they are the quicker too (25 x 6312 x 6632 165 us, 196).
+inline Shape choose_shape(const Problem& p, int f32_operands) {
     const int64_t blocks = (p.K * p.in_bytes + kRowBytes - 1) / kRowBytes;
     constexpr int clusters_at_once[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};   // (cudaOccupancyMaxActiveClusters, by CTAs per cluster)
     const int sms = 148;   // (a function of the shape alone: the count this library is built for)
-    const bool exact = p.out_dtype == DFGPU_F32;
+    const bool former = p.out_dtype == DFGPU_F32 || has_pieces(p);
     Shape best{0, 0, 0, 0, 0, 0, 0.0};
     for (int cg = 1; cg <= 2; ++cg)
         for (int bn = 64; bn <= 256; bn += 64) {
             const int chunk = sixteen_bits(p) ? 64 : 128;   // columns of one N-major copy
-            if (p.b_mn_major && (bn / cg) % chunk != 0 && !(cg == 2 && bn == 192 && !has_pieces(p) && !scaled(p) && !exact)) continue;
+            if (p.b_mn_major && (bn / cg) % chunk != 0 && !(cg == 2 && bn == 192 && !scaled(p) && !former)) continue;
             if (p.out_dtype == DFGPU_E4M3 && bn % 128 != 0) continue;   // (whole 128-byte boxes)
             if (scaled(p) && bn % 128 != 0) continue;           // (whole chunks of column scales)
             if (cg == 2 && bn < 128) continue;
@@ -93,7 +94,7 @@ inline Shape choose_shape(const Problem& p) {
                 if (splits > 1 && (bn > 128 || splits > blocks || tiles * splits > sms)) break;
                 const int64_t k_per_split = (blocks + splits - 1) / splits;
                 if (splits > 1 && k_per_split * (splits - 1) >= blocks) continue;   // (no CTA without a block)
-                const int64_t slots = cg == 2 ? sms / 2 : clusters_at_once[splits] - (scaled(p) && splits > 1 && !exact ? 1 : 0);   // (behind a quantize launch the last cluster often waits)
+                const int64_t slots = cg == 2 ? sms / 2 : clusters_at_once[splits];
                 double rounds = static_cast<double>((tiles + slots - 1) / slots);
                 int64_t halved = 0;
                 const int half = bn / 2;
@@ -103,19 +104,21 @@ inline Shape choose_shape(const Problem& p) {
                     rounds -= 0.45;
                 }
                 const double in_flight = static_cast<double>(stages_that_fit(stage_size, kSmemBudget - 2 * kStageBox)) * stage_size;
-                const double products = has_pieces(p) ? 6.0 : 1.0, pieces = has_pieces(p) ? 3.0 : 1.0;
-                const int columns = loaded_columns(p, bn, cg);
                 double clocks;
-                if (exact) {
+                if (former) {
+                    const double products = has_pieces(p) ? 6.0 : 1.0, pieces = has_pieces(p) ? 3.0 : 1.0;
                     const double summed = in_registers(p) ? 150.0 + 2.0 * bn : (p.kind == kScaledSummed ? 250.0 + 3.0 * bn : 0.0);   // the epilogue's loads and additions of a block
                     const double block = std::max({summed, products * 2.0 * bn, (products + pieces) * (rows + bn / cg), pieces * (rows + bn / cg) * kRowBytes / std::min(48.0, in_flight / 2300.0)});
                     clocks = rounds * (k_per_split * block) + 2000.0 + bn * 6.0 + (splits > 1 ? (scaled(p) ? 5000.0 : 2500.0) : 0.0) + (cg == 2 ? 1500.0 : 0.0);
                 } else {
+                    const int columns = loaded_columns(p, bn, cg);
                     const double active = static_cast<double>(std::min<int64_t>(sms, tiles * cg * splits));
                     const double rate = std::min({48.0, 6300.0 / active, in_flight / 3400.0});
-                    const double block = std::max({products * 2.3 * bn, 0.9 * (products * (rows + bn / cg) + pieces * (rows + columns)), pieces * (rows + columns) * kRowBytes / rate});
-                    const double exchange = splits > 1 ? 230.0 + 0.31 * std::min<double>(rows, static_cast<double>(p.M)) * bn + (scaled(p) ? 800.0 : 0.0) : 0.0;
-                    clocks = rounds * (k_per_split * block + (rounds > 1.0 ? 12.0 * bn : 0.0)) + 2000.0 + exchange + (scaled(p) && k_per_split > 6 ? 450.0 : 0.0) + (cg == 2 ? 1480.0 : 0.0);
+                    const double block = std::max({2.3 * bn, 0.9 * (2 * rows + bn / cg + columns), (rows + columns) * kRowBytes / rate});
+                    const int box = kRowBytes / p.out_bytes, serial = std::min(bn, (bn / box + 1) / 2 * box);   // (columns that one epilogue group takes)
+                    const double exchange = splits > 1 ? 800.0 + 0.31 * std::min<double>(rows, static_cast<double>(p.M)) * bn + (scaled(p) ? 1000.0 : 0.0) : 0.0;
+                    const double operands = splits > 1 ? 0.0 : 14.0 * f32_operands * serial;
+                    clocks = rounds * (k_per_split * block + (rounds > 1.0 ? 12.0 * bn : 0.0)) + 2000.0 + exchange + operands + (scaled(p) && k_per_split > 6 ? 450.0 : 0.0) + (cg == 2 ? 1480.0 : 0.0);
                 }
                 if (best.cg == 0 || clocks < best.clocks) best = Shape{cg, bn, splits, static_cast<int>(k_per_split), tiles, halved, clocks};
             }

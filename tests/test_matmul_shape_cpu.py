@@ -7,7 +7,7 @@ from pathlib import Path
 import pytest
 
 ROOT = Path(__file__).resolve().parent.parent
-SIXTEEN, CODES = 0, 1
+SIXTEEN, CODES, SCALED = 0, 1, 2
 TYPES = {"FLOAT": (0, 4), "HALF": (1, 2), "BFLOAT16": (2, 2)}
 # M, K, N with B [K, N] that two SMs take as tiles of 192 columns, 96 of them a CTA's. The last tile has all of them, 16 (none left for the
 # second CTA), 80, 96 (the first CTA's all), 112 and 144; a second round of tiles; rows past 256 and K with a remainder throughout.
@@ -25,20 +25,20 @@ def shapes(tmp_path_factory):
 #include "matmul_shape.cuh"
 int main() {
     dfgpu::Problem p{};
-    int n_major;
-    while (scanf("%d %ld %ld %ld %d %d %d", &p.kind, &p.M, &p.K, &p.N, &n_major, &p.out_dtype, &p.out_bytes) == 7) {
+    int n_major, f32_operands;
+    while (scanf("%d %ld %ld %ld %d %d %d %d", &p.kind, &p.M, &p.K, &p.N, &n_major, &p.out_dtype, &p.out_bytes, &f32_operands) == 8) {
         p.b_mn_major = n_major != 0;
         p.in_bytes = dfgpu::sixteen_bits(p) ? 2 : 1;
-        const dfgpu::Shape s = dfgpu::choose_shape(p);
+        const dfgpu::Shape s = dfgpu::choose_shape(p, f32_operands);
         printf("%d %d %d %d\\n", s.cg, s.bn, s.splits, s.k_per_split);
     }
 }
 """)
     subprocess.run(["g++", "-std=c++17", "-I", str(ROOT / "include"), "-I", str(ROOT / "deepforge_b200" / "csrc"), str(source), "-o", str(folder / "shape")], check=True)
 
-    def ask(kind, m, k, n, n_major, c_type):
+    def ask(kind, m, k, n, n_major, c_type, f32_operands=0):
         dtype, size = TYPES[c_type]
-        line = f"{kind} {m} {k} {n} {int(n_major)} {dtype} {size}\n"
+        line = f"{kind} {m} {k} {n} {int(n_major)} {dtype} {size} {f32_operands}\n"
         return tuple(int(v) for v in subprocess.run([str(folder / "shape")], input=line, check=True, capture_output=True, text=True).stdout.split())
     return ask
 
@@ -53,3 +53,12 @@ def test_n_major_columns_of_one_and_a_half_boxes(shapes, kind, c_type):
 @pytest.mark.parametrize("m,k,n,blocks", [(128, 384, 1152, 1), (128, 640, 3840, 3), (128, 896, 3712, 4), (128, 2048, 2688, 6), (128, 3328, 1536, 7)])
 def test_f32_results_split_k(shapes, m, k, n, blocks):
     assert shapes(SIXTEEN, m, k, n, True, "FLOAT")[3] == blocks
+
+
+@pytest.mark.parametrize("kind,m,k,n", [(SIXTEEN, 1, 136, 3648), (SIXTEEN, 2, 240, 3680), (SIXTEEN, 4, 184, 224), (SIXTEEN, 22, 288, 192), (SCALED, 7, 736, 2624), (SCALED, 15, 704, 2448)])
+def test_few_blocks_are_not_worth_an_exchange(shapes, kind, m, k, n):
+    assert shapes(kind, m, k, n, True, "BFLOAT16")[2] == 1
+
+
+def test_a_full_f32_operand_is_shared_out(shapes):
+    assert [shapes(SIXTEEN, 128, 384, 384, True, "HALF", operands)[2] for operands in (0, 1)] == [1, 6]
