@@ -282,7 +282,7 @@ __device__ __forceinline__ void apply_steps(const TileArgs& args, float (&v)[COU
         for (int s = ahead != nullptr ? 1 : 0; s < args.step_count; ++s) {
             const int kind = args.step_kind[s];
             if (kind == kStepRelu) {
-                relu_values(v, args.relu_lower[s], args.relu_upper[s], args.relu_slope[s]);
+                relu_values(v, args.relu_lower[s], args.relu_upper[s], args.relu_slope[s], row_live);
             } else if (kind == kStepBias || row_live) {
                 add_operand<COUNT>(v, args.step_data[s], args.step_dtype[s], (kind == kStepBias ? 0 : row * args.step_ld[s]) + col0, live, args.step_vector[s] != 0);
             }

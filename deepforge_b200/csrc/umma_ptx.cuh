@@ -171,13 +171,14 @@ __device__ __forceinline__ void epilogue_barrier(int id) { asm volatile("bar.syn
 // RELU_FWD with the same result as relu_forward(): NaN in -> NaN out, x < lower takes the sloped branch (NaN for -inf with slope 0,
 // as the separate multiply and add give), otherwise clip to [lower, upper]. Eight epilogue warps apply it to every value of a tile,
 // so the ReLU without clips is two instructions a value, and half a one for the minimum that tells whether some value is -inf.
+// `live`: a row that is not stored holds whatever lay behind the operands, infinities among it, and takes the short way all the same.
 template <int COUNT>   // a multiple of 4
-__device__ __forceinline__ void relu_values(float (&v)[COUNT], float lower, float upper, float slope) {
+__device__ __forceinline__ void relu_values(float (&v)[COUNT], float lower, float upper, float slope, bool live = true) {
     if (lower == 0.0f && slope == 0.0f && upper >= 0.0f) {
         float least[4] = {v[0], v[1], v[2], v[3]};   // (four chains)
 #pragma unroll
         for (int e = 4; e + 1 < COUNT; e += 2) asm("min.f32 %0, %0, %1, %2;" : "+f"(least[(e >> 1) & 3]) : "f"(v[e]), "f"(v[e + 1]));
-        if (fminf(fminf(least[0], least[1]), fminf(least[2], least[3])) != -INFINITY) {
+        if (!live || fminf(fminf(least[0], least[1]), fminf(least[2], least[3])) != -INFINITY) {
 #pragma unroll
             for (int e = 0; e < COUNT; ++e) asm("max.NaN.f32 %0, %0, 0f00000000;\n\tmin.NaN.f32 %0, %0, %1;" : "+f"(v[e]) : "f"(upper));
             return;
