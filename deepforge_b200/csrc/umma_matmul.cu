@@ -222,7 +222,8 @@ __device__ __forceinline__ void add_words(float (&v)[COUNT], const uint32_t (&wo
         v[2 * i + 1] = __fadd_rn(v[2 * i + 1], hi);
     }
 }
-template <int COUNT>
+// (32-bit operands BATCH loads at a time: where a row's sums are in registers too, 32 more spill)
+template <int COUNT, int BATCH>
 __device__ __forceinline__ void add_operand(float (&v)[COUNT], const void* data, int dtype, int64_t first, int live, bool vector) {
     if (dtype != DFGPU_F32) {
         uint32_t words[COUNT / 2];
@@ -231,22 +232,25 @@ __device__ __forceinline__ void add_operand(float (&v)[COUNT], const void* data,
         return;
     }
     const float* p = static_cast<const float*>(data) + first;
-    float x[COUNT];
-    if (vector && live >= COUNT) {
 #pragma unroll
-        for (int j = 0; j < COUNT / 4; ++j) {
-            const float4 q = reinterpret_cast<const float4*>(p)[j];
-            x[4 * j] = q.x;
-            x[4 * j + 1] = q.y;
-            x[4 * j + 2] = q.z;
-            x[4 * j + 3] = q.w;
+    for (int at = 0; at < COUNT; at += BATCH) {
+        float x[BATCH];
+        if (vector && live >= COUNT) {
+#pragma unroll
+            for (int j = 0; j < BATCH / 4; ++j) {
+                const float4 q = reinterpret_cast<const float4*>(p + at)[j];
+                x[4 * j] = q.x;
+                x[4 * j + 1] = q.y;
+                x[4 * j + 2] = q.z;
+                x[4 * j + 3] = q.w;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) x[i] = at + i < live ? p[at + i] : 0.0f;
         }
-    } else {
 #pragma unroll
-        for (int i = 0; i < COUNT; ++i) x[i] = i < live ? p[i] : 0.0f;
+        for (int i = 0; i < BATCH; ++i) v[at + i] = __fadd_rn(v[at + i], x[i]);
     }
-#pragma unroll
-    for (int i = 0; i < COUNT; ++i) v[i] = __fadd_rn(v[i], x[i]);
 }
 
 struct Scalars {
@@ -274,7 +278,7 @@ __device__ __forceinline__ void fold_amax(const TileArgs& args, const Scalars& s
 // COUNT neighbouring columns of one row: fused steps, then MATMUL_FP8's scalars. `row_live`: the row exists. `ahead`: the first
 // step's operand, where it was loaded ahead.
 // CODES: MATMUL_FP8, which has the scalars and no steps; the others have none of the scalars (neither is compiled into the other's kernel).
-template <bool CODES, int COUNT>
+template <bool CODES, int BATCH, int COUNT>
 __device__ __forceinline__ void apply_steps(const TileArgs& args, float (&v)[COUNT], int row, int col0, bool row_live, Scalars& scalars, const uint32_t (*ahead)[COUNT / 2] = nullptr) {
     const int live = args.n_total - col0;
     if constexpr (!CODES) {
@@ -284,7 +288,7 @@ __device__ __forceinline__ void apply_steps(const TileArgs& args, float (&v)[COU
             if (kind == kStepRelu) {
                 relu_values(v, args.relu_lower[s], args.relu_upper[s], args.relu_slope[s], row_live);
             } else if (kind == kStepBias || row_live) {
-                add_operand<COUNT>(v, args.step_data[s], args.step_dtype[s], (kind == kStepBias ? 0 : row * args.step_ld[s]) + col0, live, args.step_vector[s] != 0);
+                add_operand<COUNT, BATCH>(v, args.step_data[s], args.step_dtype[s], (kind == kStepBias ? 0 : row * args.step_ld[s]) + col0, live, args.step_vector[s] != 0);
             }
         }
     }
@@ -506,6 +510,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     constexpr bool kSixteenBits = KIND == kSixteen || kHasPieces<KIND> || KIND == kSummed;
     constexpr int kPieceCount = kHasPieces<KIND> ? 3 : 1;
     constexpr bool kCodesOnly = KIND == kCodes || KIND == kCodesSummed;
+    constexpr int kBatch = KIND == kSummed ? 16 : 32;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* generic_base = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -772,9 +777,9 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                             for (int e = 0; e < 16; ++e) operand[e] = first_operand[e];
                             const bool same_box = part + 1 < box_columns / 32;
                             if (same_box || b + 2 < boxes) load_ahead(args, first_operand, out_row, same_box ? col + 32 : item.col0 + (b + 2) * box_columns, row_live);
-                            apply_steps<kCodesOnly, 32>(args, v, out_row, col, row_live, scalars, &operand);
+                            apply_steps<kCodesOnly, kBatch, 32>(args, v, out_row, col, row_live, scalars, &operand);
                         } else {
-                            apply_steps<kCodesOnly, 32>(args, v, out_row, col, row_live, scalars);
+                            apply_steps<kCodesOnly, kBatch, 32>(args, v, out_row, col, row_live, scalars);
                         }
                         if (args.tma_store) {
                             uint8_t* target = generic_base + staging + row * 128;
@@ -901,7 +906,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 v[2] = __fadd_rn(v[2], part[z].z);
                 v[3] = __fadd_rn(v[3], part[z].w);
             }
-            apply_steps<kCodesOnly, 4>(args, v, row0 + row, col, true, scalars);
+            apply_steps<kCodesOnly, 4, 4>(args, v, row0 + row, col, true, scalars);
             if (healthy) store_four(args, v, row0 + row, col);
         }
         __syncwarp();
