@@ -689,12 +689,18 @@ extern "C" int dfgpu_conv_fprop(const dfgpu_conv_params* p, void* const* tensors
     cudaStream_t stream = as_stream(stream_handle);
     if (ShallowArgs shallow; kernel == DFGPU_CONV_IGEMM_FFMA && shallow_form(*p, a, tensors, shallow)) {
         // Wherever neither the tensor cores nor 16-byte loads take the convolution (4 x 20 x 64 x 64 pixels, 1 x 1 to 128 channels: 39.4 us by 16
-        // products at a time, 12.3 here), and up to 96 products where every SM has one tile at most, at 2.6 us and 0.036 for every product (324
-        // pixels x 116 channels of 48 products 4.4 us, 6.7 on the tensor cores; of 124 products 7.1 and 6.6; 640 tiles of 40 products 10.6 and 6.8).
-        const int64_t tiles = (static_cast<int64_t>(shallow.m_total) + 31) / 32 * ((p->y.dim[1] + 31) / 32);
+        // products at a time, 12.0 here), and up to 96 products where every SM has one tile at most, at 2.6 us and 0.036 for every product (324
+        // pixels x 116 channels of 48 products 4.4 us, 6.7 on the tensor cores; of 124 products 7.1 and 6.6; 640 tiles of 40 products 10.6 and 6.8),
+        // but for one or two channels of so few products that 16-byte loads, two or four a pixel, are as many (16 products to one channel 3.1 us, 3.6 here;
+        // 32 to two 4.2 both).
+        // Tiles of 32 x 32 up to twelve per SM, as their CTAs stand side by side there (9744 pixels of 8 products to 43 channels in f16 5.7 us, 10.9 in
+        // tiles of 64 x 64; 13923 of 4 to 106 in bf16 12.9 and 19.5; 15552 of 73 to 128 are more than that, 34.5 and 25.6), and where tiles of 64 x 64
+        // would be more than a third of their number, half empty (43687 pixels of 27 products to one channel 13.0 us and 21.8).
+        const int64_t m_total = shallow.m_total, channels = p->y.dim[1];
+        const int64_t tiles = (m_total + 31) / 32 * ((channels + 31) / 32), large = (m_total + 63) / 64 * ((channels + 63) / 64);
         const bool other = (p->kernel == DFGPU_CONV_AUTO && conv_f32_flat(*p, tensors)) || nhwc_f32_fast_form(*p, tensors);
-        if (!other || (tiles <= sm_count() && shallow.k_total <= 96))
-            return tiles <= 4 * sm_count() ? launch_shallow<32, 32>(*p, a, shallow, tensors, stream) : launch_shallow<64, 64>(*p, a, shallow, tensors, stream);
+        if (!other || (tiles <= sm_count() && shallow.k_total <= 96 && channels * shallow.k_total > 32))
+            return tiles <= 12 * sm_count() || tiles < 3 * large ? launch_shallow<32, 32>(*p, a, shallow, tensors, stream) : launch_shallow<64, 64>(*p, a, shallow, tensors, stream);
     }
     if (p->kernel == DFGPU_CONV_AUTO && kernel == DFGPU_CONV_IGEMM_FFMA && conv_f32_flat(*p, tensors))
         kernel = DFGPU_CONV_UMMA_F32X3_CLUSTER;

@@ -109,3 +109,31 @@ def test_conv_shallow_reduction(n, c, k, h, w, r, layout, shift):
     y = y.view(n, h, w, k).permute(0, 3, 1, 2) if layout == "nhwc" else y.view(n, k, h, w)
     conv = lambda a, b: torch.nn.functional.conv2d(a.double().cpu(), b.double().cpu(), padding=r // 2)
     assert torch.all((y.double().cpu() - conv(x, f)).abs() <= max(c * r * r * 2.0 ** -24, pieces_bound(c * r * r)) * conv(x.abs(), f.abs()))
+
+
+@pytest.mark.parametrize("n,c,k,h,w,r,stride,dilation,reverse", [(1, 5, 3, 4, 5, 1, 1, 1, False), (2, 20, 24, 28, 12, 1, 1, 1, False), (1, 5, 33, 19, 21, 3, 2, 1, False), (1, 7, 40, 17, 13, 3, 1, 2, True), (3, 13, 65, 40, 41, 3, 1, 1, False),
+                                                                 (2, 8, 43, 87, 56, 1, 1, 1, False), (4, 3, 100, 96, 97, 3, 1, 1, False), (9, 3, 7, 80, 83, 3, 1, 1, True)])
+@pytest.mark.parametrize("layout", ["nhwc", "nchw"])
+@pytest.mark.parametrize("io", ["FLOAT", "HALF", "BFLOAT16"])
+def test_conv_shallow_fused_and_in_sixteen_bits(n, c, k, h, w, r, stride, dilation, reverse, layout, io):
+    """Bias, ReLU and a residual behind it, every element type, tiles of 32 and of 64 (the last but one), of 32 for few channels (the last).
+    Products of 16-bit values are exact in f32; C of them are added up in f32 and the operands behind, and Y is rounded once."""
+    dtype, rounding = {"FLOAT": (torch.float32, 2.0 ** -24), "HALF": (torch.float16, 2.0 ** -11), "BFLOAT16": (torch.bfloat16, 2.0 ** -8)}[io]
+    g = torch.Generator(device="cuda").manual_seed(c * 131 + k)
+    pad, strides = dilation * (r // 2), graphs.nhwc if layout == "nhwc" else graphs.contiguous
+    p, q = ((size + 2 * pad - dilation * (r - 1) - 1) // stride + 1 for size in (h, w))
+    dims = {1: [n, c, h, w], 2: [k, c, r, r], 3: [1, k, 1, 1], 4: [n, k, p, q], 5: [n, k, p, q]}
+    tensors = [graphs.tensor(uid, f"t{uid}", d, io, strides(d)) for uid, d in dims.items()] + [graphs.tensor(uid, f"v{uid}", dims[5], "FLOAT", strides(dims[5]), virtual=True) for uid in (6, 7, 8)]
+    nodes = [graphs.conv_node("conv", 1, 2, 6, (pad, pad), stride=(stride, stride), dilation=(dilation, dilation), mode="CONVOLUTION" if reverse else "CROSS_CORRELATION"), graphs.pointwise_node("bias", "ADD", 6, 7, 3),
+             graphs.pointwise_node("relu", "RELU_FWD", 7, 8), graphs.pointwise_node("residual", "ADD", 8, 5, 4)]
+    values = {uid: torch.randn(dims[uid], device="cuda", generator=g).to(dtype) for uid in (1, 2, 3, 4)}
+    place = lambda t: (t.permute(0, 2, 3, 1) if layout == "nhwc" else t).contiguous().reshape(-1)
+    y = torch.full((n * k * p * q,), float("nan"), device="cuda", dtype=dtype)
+    run(graphs.document("conv", nodes, tensors, io=io), {uid: place(t) for uid, t in values.items()}, {5: y})
+    y = (y.view(n, p, q, k).permute(0, 3, 1, 2) if layout == "nhwc" else y.view(n, k, p, q)).double().cpu()
+    x, f, bias, residual = (t.double().cpu() for t in values.values())
+    f = f.flip(2, 3) if reverse else f
+    conv = lambda a, b: torch.nn.functional.conv2d(a, b, padding=pad, stride=stride, dilation=dilation)
+    want, weight = torch.relu(conv(x, f) + bias) + residual, conv(x.abs(), f.abs()) + bias.abs() + residual.abs()
+    depth = c * r * r
+    assert torch.all((y - want).abs() <= rounding * want.abs() + max((depth + 3) * 2.0 ** -24, pieces_bound(depth)) * weight)
