@@ -1570,9 +1570,14 @@ int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, cudaStrea
     const int places = duo ? sm_count() / 2 : sm_count();
     const int64_t single = pairs * heads;
     args.order = !args.causal || single <= places ? kAsStored : (duo ? kHeaviestFirst : kHeavyWithLight);   // (the third order in the one-SM kernel cost it 1.4 %)
-    // (CTAs that run side by side then read different heads' K and V: only where all of them stay in the L2 cache)
+    // By length where lengths can differ: with one key tile all pairs are alike, and with one pair a sequence that sees all keys nearly so up to
+    // three tiles. Making the list costs each CTA 0.3 to 2 us there (5 x 32 x 108 causal 16.3 us without, 18.5 with; 15 x 2 x 2326 on 101 keys 21.0 and
+    // 22.8; 32 x 8 x 101 on 290 16.3 and 17.1). From two tiles on it gains (20 x 32 x 298 on 146 keys 102 and 85; 29 x 8 x 154 causal 16.9 and 15.2).
+    // CTAs that run side by side then read different heads' K and V: only where all of them stay in the L2 cache. An entry of the list is a
+    // byte, 256 of them fit behind the barriers.
     const int64_t kv_bytes = p.k.dim[0] * p.k.dim[1] * p.k.dim[2] * p.k.dim[3] * 4;
-    if (!duo && p.padding_mask && single > places && p.q.dim[0] * pairs <= PairSmem<128>::kMostPairs && kv_bytes <= (64 << 20)) args.order = kLongestFirst;
+    const bool uneven = kv_tiles > 1 && (pairs > 1 || args.causal || kv_tiles > 3);
+    if (!duo && p.padding_mask && single > places && uneven && p.q.dim[0] * pairs <= PairSmem<128>::kMostPairs && kv_bytes <= (64 << 20)) args.order = kLongestFirst;
     const int64_t units = args.order == kHeavyWithLight ? (pairs + 1) / 2 * heads : single;
     const unsigned grid = static_cast<unsigned>(std::min<int64_t>(units, places));
     if (plain_tiles(p)) return duo ? launch_duo<false, false>(map_q, map_k, map_v, map_o, args, grid, stream) : launch_pair<128, false, false, false>(map_q, map_k, map_v, map_o, args, grid, stream);

@@ -42,9 +42,9 @@ def test_far_below_the_maximum(batch):
         assert not bool(torch.isfinite(o[:, :4]).any()) and bool(torch.all(o[:, 4:] == 1.0))
 
 
-@pytest.mark.parametrize("tiles", [1, 31, 32, 33, 65, 128, 129, 200])
+@pytest.mark.parametrize("tiles", [1, 2, 7, 8, 9, 31, 32, 33, 65, 128, 129, 200])
 def test_any_number_of_chunks(tiles):
-    """Chunks of one key tile: groups of 32 that are full, one over and one short, and more than the first four. A probability is within
+    """Chunks of one key tile: the most that are merged eight at once and one more; groups of 32 that are full, one over and one short, and more than the first four. A probability is within
     2^-8 of its value and O is rounded once by 2^-9, with as much again for the exponentials and sums."""
     hq, block, length = 8, 64, 128 * tiles
     pages = length // block
