@@ -1509,10 +1509,11 @@ int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, cudaStrea
         if ((reinterpret_cast<uintptr_t>(tensors[i]) & 15u) != 0) return fail(kInvalidArgument, "SDPA: the tcgen05 kernel needs 16-byte aligned Q, K, V and O");
     // One SM or two per pair of query tiles: the longest list of key tiles any of them walks, times what a tile step costs (two
     // tiles in 3670 clocks on one SM, one in 1620 on each of two; the latter count for 12 % more, since they draw more and a chip that is
-    // full has to lower its clocks), and 4500 clocks a pair. A causal pair's last tile is all masked for the first query tile, which
-    // one SM skips; so it does a second query tile that does not exist.
-    //   64 pairs, 2048 causal: 37 us on one SM each, 22 on two. 96: 38 / 27. 16 x 2171 causal: 39 / 29. 8 x 32 x 2048 causal: 329 / 351.
-    //   192 x 1538 queries on 190 keys: 61 / 73.
+    // full has to lower its clocks), and 4500 clocks a pair. (3670 is from before the hand-over in halves, which takes 1.5 to 7 % off it; a padded step is
+    // 4400, and lengths are not looked at: 4 x 16 x 569 queries on up to 370 keys are 17.3 us on one SM each and 21.6 on the two they get.) A
+    // causal pair's last tile is all masked for the first query tile, which one SM skips; so it does a second query tile that does not exist.
+    //   64 pairs, 2048 causal: 35 us on one SM each, 21 on two. 96: 35 / 21. 16 x 2171 causal: 44 / 33. 8 x 32 x 2048 causal: 283 / 333 (329 / 351
+    //   once the power limit holds). 192 x 1538 queries on 190 keys: 81 / 107.
     const int64_t pairs = (p.q.dim[2] + 2 * kRows - 1) / (2 * kRows), heads = p.q.dim[0] * p.q.dim[1], kv_tiles = (p.k.dim[2] + kKeys - 1) / kKeys;
     int64_t longest = 0, all = 0;
     for (int64_t i = 0; i < pairs; ++i) {
