@@ -174,7 +174,7 @@ __device__ __forceinline__ void epilogue_barrier(int id) { asm volatile("bar.syn
 // `live`: a row that is not stored holds whatever lay behind the operands, infinities among it, and takes the short way all the same.
 template <int COUNT>   // a multiple of 4
 __device__ __forceinline__ void relu_values(float (&v)[COUNT], float lower, float upper, float slope, bool live = true) {
-    if (lower == 0.0f && slope == 0.0f && upper >= 0.0f) {
+    if (__float_as_uint(lower) == 0u && slope == 0.0f && upper > 0.0f) {   // (a negative zero below or a zero above would show in the sign of a result)
         float least[4] = {v[0], v[1], v[2], v[3]};   // (four chains)
 #pragma unroll
         for (int e = 4; e + 1 < COUNT; e += 2) asm("min.f32 %0, %0, %1, %2;" : "+f"(least[(e >> 1) & 3]) : "f"(v[e]), "f"(v[e + 1]));

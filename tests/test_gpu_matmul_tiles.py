@@ -246,3 +246,14 @@ def test_fused_operands_at_the_edges(m, k, n, first, io, operand, shift):
     assert torch.all(got[want == float("inf")] >= torch.finfo(TORCH[io]).max)
     finite = want.isfinite()
     assert torch.all((got - torch.relu(want)).abs()[finite] <= bound[finite])
+
+
+@pytest.mark.parametrize("lower,upper,negative", [(-0.0, None, -0.0), (0.0, None, 0.0), (0.0, -0.0, 0.0), (-0.0, 2.0, -0.0)])
+def test_the_sign_of_a_clipped_zero(lower, upper, negative):
+    """Below `lower` ReLU gives lower + 0 (x - lower): a negative zero where the clip is one, and never the other clip's sign."""
+    m, k, n = 40, 64, 96
+    tensors = [graphs.tensor(1, "A", [m, k], "BFLOAT16"), graphs.tensor(2, "B", [k, n], "BFLOAT16"), graphs.tensor(4, "C", [m, n], "BFLOAT16"), graphs.tensor(5, "p", [m, n], virtual=True)]
+    nodes = [graphs.matmul_node("matmul", 1, 2, 5), graphs.pointwise_node("relu", "RELU_FWD", 5, 4, lower=lower, upper=upper)]
+    buffers = {1: -torch.ones(m * k, device="cuda", dtype=torch.bfloat16), 2: torch.ones(k * n, device="cuda", dtype=torch.bfloat16)}
+    run(graphs.document("tiles", nodes, tensors, io="BFLOAT16"), buffers)
+    assert torch.all(buffers[4] == 0) and bool(torch.all(torch.signbit(buffers[4]) == (str(negative)[0] == "-")))
