@@ -3,6 +3,7 @@
 #pragma once
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 
 #include "dfgpu.h"
@@ -27,6 +28,7 @@ struct Problem {
     int64_t a_ld, b_ld, c_ld;
     bool b_mn_major;
     int in_bytes, out_bytes, out_dtype;
+    bool direct_stores;       // C's rows are off the 16-byte boundaries, or E5M2: no TMA store
     int64_t a_rows, b_rows;   // rows the maps span (pieces: three matrices on top of one another)
 };
 
@@ -65,10 +67,12 @@ struct Shape {
 // tiles of 128 x 256 on 148 SMs, three rounds and 68 tiles, which become 136 halves) and, where there are several, an epilogue of 12 bn.
 // Splitting K divides the blocks and adds an exchange that grows with the partial tile, 800 + 0.31 x rows x bn (1000 more with block
 // scales, whose six loading warps also fall behind once they have more than a block each), and shares out the epilogue, which counts
-// where it waits for a full f32 operand (`f32_operands` of them): 14 clocks for every column that a group of its warps takes.
+// for every column that a group of its warps takes: 14 clocks for a full f32 operand (`f32_operands` of them), 20 for E4M3 codes, and 300 in
+// every round where a thread stores its row element by element, as K in splits is added up and stored by neighbouring threads side by side.
 // Former costs -> these, in us: 777 x 4096 x 3072 bf16 [K, N] 26.9 (256 columns) -> 21.6 (192), 2050 x 1040 x 1040 13.0 -> 11.5, MXFP8
 // 15 x 1632 x 816 7.7 -> 6.3 (more splits). Where an exchange of 230 split K: 1 x 136 x 3648 bf16 4.0 whole, 5.0 in two. With bias, ReLU and a
-// full f32 operand, 128 x 384 x 384 f16: 6.0 in six, 7.5 whole.
+// full f32 operand, 128 x 384 x 384 f16: 6.0 in six, 7.5 whole. With rows of C off the 16-byte boundaries 128 x 512 x 1280 f16 6.9 in splits, 12.9
+// whole; FP8 128 x 1024 x 2688 to E5M2 10.2 and 29.2, 78 x 912 x 336 to E4M3 7.5 and 9.6.
 // f32 results and f32 operands (pieces) keep the former costs. Those split K more often, and an accumulator is off by 2^-24 of its value
 // for every block it takes, which a 16-bit result does not show and an f32 result does (128 x 640 x 3840 bf16 to f32: 1.7e-7 from
 // 64 bits in four splits, 5.9e-7 in one; 128 x 3328 x 1536 4.0e-7 and 6.4e-7). For pieces they are the quicker too (25 x 6312 x 6632 165 us, 196).
@@ -115,10 +119,11 @@ inline Shape choose_shape(const Problem& p, int f32_operands) {
                     const double active = static_cast<double>(std::min<int64_t>(sms, tiles * cg * splits));
                     const double rate = std::min({48.0, 6300.0 / active, in_flight / 3400.0});
                     const double block = std::max({2.3 * bn, 0.9 * (2 * rows + bn / cg + columns), (rows + columns) * kRowBytes / rate});
-                    const int box = kRowBytes / p.out_bytes, serial = std::min(bn, (bn / box + 1) / 2 * box);   // (columns that one epilogue group takes)
+                    const int box = p.direct_stores ? 32 : kRowBytes / p.out_bytes, serial = std::min(bn, (bn / box + 1) / 2 * box);   // (columns that one epilogue group takes)
                     const double exchange = splits > 1 ? 800.0 + 0.31 * std::min<double>(rows, static_cast<double>(p.M)) * bn + (scaled(p) ? 1000.0 : 0.0) : 0.0;
-                    const double operands = splits > 1 ? 0.0 : 14.0 * f32_operands * serial;
-                    clocks = rounds * (k_per_split * block + (rounds > 1.0 ? 12.0 * bn : 0.0)) + 2000.0 + exchange + operands + (scaled(p) && k_per_split > 6 ? 450.0 : 0.0) + (cg == 2 ? 1480.0 : 0.0);
+                    const double stores = p.direct_stores ? 300.0 * std::ceil(rounds) : (p.out_dtype == DFGPU_E4M3 ? 20.0 : 0.0);
+                    const double epilogue = splits > 1 ? 0.0 : (14.0 * f32_operands + stores) * serial;
+                    clocks = rounds * (k_per_split * block + (rounds > 1.0 ? 12.0 * bn : 0.0)) + 2000.0 + exchange + epilogue + (scaled(p) && k_per_split > 6 ? 450.0 : 0.0) + (cg == 2 ? 1480.0 : 0.0);
                 }
                 if (best.cg == 0 || clocks < best.clocks) best = Shape{cg, bn, splits, static_cast<int>(k_per_split), tiles, halved, clocks};
             }

@@ -984,7 +984,8 @@ int launch_kernel(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUte
 }
 
 // Everything but the epilogue's operands and the operand formats, which the callers have put into `args`.
-int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* b, void* c, cudaStream_t stream, const char* what) {
+int launch_problem(Problem p, TileArgs& args, const void* a, const void* b, void* c, cudaStream_t stream, const char* what) {
+    p.direct_stores = !on16(c) || (p.c_ld * p.out_bytes) % 16 != 0 || p.out_dtype == DFGPU_E5M2;
     int f32_operands = 0;   // full ADD operands in 32 bits
     for (int s = 0; s < args.step_count; ++s) f32_operands += args.step_kind[s] == kStepFull && args.step_dtype[s] == DFGPU_F32 ? 1 : 0;
     const Shape shape = choose_shape(p, f32_operands);
@@ -1008,7 +1009,7 @@ int launch_problem(const Problem& p, TileArgs& args, const void* a, const void* 
     args.out = c;
     args.out_ld = p.c_ld;
     args.out_dtype = p.out_dtype;
-    args.tma_store = on16(c) && (p.c_ld * p.out_bytes) % 16 == 0 && p.out_dtype != DFGPU_E5M2 ? 1 : 0;
+    args.tma_store = p.direct_stores ? 0 : 1;
     // Tensor memory: two accumulators, and with block scales 32 columns of them at the end. At bn = 256 the accumulators then
     // overlap by 32 columns, which the epilogue reads out first.
     // Pieces: an accumulator is two of bn columns (leading and lower products), so that 192 and 256 columns leave room for one: the

@@ -9,12 +9,12 @@ import numpy as np
 import pytest
 
 from deepforge_b200 import dfgpu, graphs, runtime
-from test_matmul_shape_cpu import CODES, N_MAJOR_192, SIXTEEN
+from test_matmul_shape_cpu import CODES, DIRECT, N_MAJOR_192, SIXTEEN
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
-TORCH = {"FLOAT": torch.float32, "BFLOAT16": torch.bfloat16, "HALF": torch.float16, "FP8_E4M3": torch.uint8, "FP8_E8M0": torch.uint8}
+TORCH = {"FLOAT": torch.float32, "BFLOAT16": torch.bfloat16, "HALF": torch.float16, "FP8_E4M3": torch.uint8, "FP8_E5M2": torch.uint8, "FP8_E8M0": torch.uint8}
 ROUNDING = {"FLOAT": 2.0 ** -24, "BFLOAT16": 2.0 ** -8, "HALF": 2.0 ** -11}
 # M, K, N: K and N in 16-byte rows. Single rows; edges of 128 and 256 rows; 64 / 128 / 192 / 256 columns; K of one block, less, more
 EXTENTS = [(1, 16, 16), (1, 4096, 96), (7, 144, 272), (16, 4096, 4096), (64, 8192, 512), (127, 128, 112), (128, 4096, 256), (129, 272, 128), (255, 64, 192),
@@ -98,6 +98,37 @@ def test_fp8_columns_of_three_quarters_of_a_box(m, k, n, c_type):
     assert float((a @ b).abs().max()) * (0.5 * 0.25 * 0.125) < 65504
     close(buffers[26].view(m, n), a, b, lambda p: p * (0.5 * 0.25 * 0.125), c_type, k)
     assert abs(float(buffers[27][0]) - float((a @ b).abs().max()) * 0.125) <= k * 2.0 ** -24 * float((a.abs() @ b.abs()).max())
+
+
+@pytest.mark.parametrize("m,k,n", DIRECT[SIXTEEN] + [(4097, 64, 136)])
+@pytest.mark.parametrize("io", ["BFLOAT16", "HALF"])
+@pytest.mark.parametrize("pad", [1, 5])
+def test_rows_of_c_off_the_boundaries(m, k, n, io, pad):
+    """Stored element by element, by the owners of a cluster's rows and by single CTAs; nothing between the rows is touched."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    doc = graphs.document("tiles", [graphs.matmul_node("matmul", 1, 2, 5), graphs.pointwise_node("relu", "RELU_FWD", 5, 4)], [graphs.tensor(1, "A", [m, k], io), graphs.tensor(2, "B", [k, n], io, [1, k]), graphs.tensor(4, "C", [m, n], io, [n + pad, 1]),
+                          graphs.tensor(5, "p", [m, n], virtual=True)], io=io)
+    buffers = {uid: torch.randn(count, device="cuda", generator=g).to(TORCH[io]) for uid, count in ((1, m * k), (2, k * n))}
+    buffers[4] = torch.full((m * (n + pad),), 7.0, device="cuda", dtype=TORCH[io])
+    assert [s["kernel"] for s in run(doc, buffers).steps()] == [dfgpu.MATMUL_UMMA_BF16]
+    c = buffers[4].view(m, n + pad)
+    close(c[:, :n], buffers[1].view(m, k).double(), buffers[2].view(n, k).t().double(), torch.relu, io, k)
+    assert torch.all(c[:-1, n:] == 7.0)
+
+
+@pytest.mark.parametrize("m,k,n", DIRECT[CODES] + [(2050, 256, 1040)])
+@pytest.mark.parametrize("c_type,code", [("FP8_E5M2", torch.float8_e5m2), ("FP8_E4M3", torch.float8_e4m3fn)])
+def test_codes_as_results(m, k, n, c_type, code):
+    """Whole numbers up to 2, so that sums are exact and the codes the same to the byte."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    codes = {uid: torch.randint(-2, 3, (count,), device="cuda", generator=g).float().to(torch.float8_e4m3fn) for uid, count in ((21, m * k), (22, k * n))}
+    buffers = {uid: c.view(torch.uint8) for uid, c in codes.items()}
+    buffers.update({uid: torch.full((1,), v, device="cuda") for uid, v in ((23, 0.5), (24, 0.25), (25, 0.5))})
+    doc = graphs.matmul_fp8(m, k, n, c_type, batch=(), b_k_major=True)
+    run(doc, buffers)
+    product = codes[21].float().view(m, k).double() @ codes[22].float().view(n, k).t().double()
+    assert float(product.abs().max()) / 16 < 440 and float(buffers[27][0]) == float(product.abs().max()) / 8
+    assert torch.equal(buffers[26].view(m, n), (product / 16).float().to(code).view(torch.uint8))
 
 
 @pytest.mark.parametrize("m,k,n", [(m, (k + 31) // 32 * 32, n) for m, k, n in EXTENTS if n > 64])

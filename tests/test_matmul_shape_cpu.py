@@ -6,9 +6,13 @@ from pathlib import Path
 
 import pytest
 
+from deepforge_b200.dfgpu import E4M3, E5M2
+
 ROOT = Path(__file__).resolve().parent.parent
 SIXTEEN, CODES, SCALED = 0, 1, 2
-TYPES = {"FLOAT": (0, 4), "HALF": (1, 2), "BFLOAT16": (2, 2)}
+TYPES = {"FLOAT": (0, 4), "HALF": (1, 2), "BFLOAT16": (2, 2), "E4M3": (E4M3, 1), "E5M2": (E5M2, 1)}
+# M, K, N whose K is split where C is stored element by element: in 16 bits with rows off the 16-byte boundaries, and as E5M2.
+DIRECT = {SIXTEEN: [(128, 512, 1280), (179, 336, 128), (256, 384, 128), (70, 200, 264)], CODES: [(128, 1024, 2688), (596, 528, 336), (78, 832, 2384)]}
 # M, K, N with B [K, N] that two SMs take as tiles of 192 columns, 96 of them a CTA's. The last tile has all of them, 16 (none left for the
 # second CTA), 80, 96 (the first CTA's all), 112 and 144; a second round of tiles; rows past 256 and K with a remainder throughout.
 N_MAJOR_192 = {kind: [(1030, 1040, 2112), (1030, 528, 2128), (1030, 528, 2192), (1030, 528, 2208), (1030, 528, 2224), (1030, 1040, 2064), several]
@@ -25,8 +29,9 @@ def shapes(tmp_path_factory):
 #include "matmul_shape.cuh"
 int main() {
     dfgpu::Problem p{};
-    int n_major, f32_operands;
-    while (scanf("%d %ld %ld %ld %d %d %d %d", &p.kind, &p.M, &p.K, &p.N, &n_major, &p.out_dtype, &p.out_bytes, &f32_operands) == 8) {
+    int n_major, f32_operands, direct;
+    while (scanf("%d %ld %ld %ld %d %d %d %d %d", &p.kind, &p.M, &p.K, &p.N, &n_major, &p.out_dtype, &p.out_bytes, &f32_operands, &direct) == 9) {
+        p.direct_stores = direct != 0;
         p.b_mn_major = n_major != 0;
         p.in_bytes = dfgpu::sixteen_bits(p) ? 2 : 1;
         const dfgpu::Shape s = dfgpu::choose_shape(p, f32_operands);
@@ -36,9 +41,9 @@ int main() {
 """)
     subprocess.run(["g++", "-std=c++17", "-I", str(ROOT / "include"), "-I", str(ROOT / "deepforge_b200" / "csrc"), str(source), "-o", str(folder / "shape")], check=True)
 
-    def ask(kind, m, k, n, n_major, c_type, f32_operands=0):
+    def ask(kind, m, k, n, n_major, c_type, f32_operands=0, direct=False):
         dtype, size = TYPES[c_type]
-        line = f"{kind} {m} {k} {n} {int(n_major)} {dtype} {size} {f32_operands}\n"
+        line = f"{kind} {m} {k} {n} {int(n_major)} {dtype} {size} {f32_operands} {int(direct)}\n"
         return tuple(int(v) for v in subprocess.run([str(folder / "shape")], input=line, check=True, capture_output=True, text=True).stdout.split())
     return ask
 
@@ -62,3 +67,10 @@ def test_few_blocks_are_not_worth_an_exchange(shapes, kind, m, k, n):
 
 def test_a_full_f32_operand_is_shared_out(shapes):
     assert [shapes(SIXTEEN, 128, 384, 384, True, "HALF", operands)[2] for operands in (0, 1)] == [1, 6]
+
+
+def test_stores_element_by_element_are_shared_out(shapes):
+    for kind, c_type in ((SIXTEEN, "HALF"), (CODES, "E5M2")):
+        for m, k, n in DIRECT[kind]:
+            assert shapes(kind, m, k, n, False, c_type, direct=True)[2] > 1, (m, k, n)
+    assert shapes(CODES, 78, 912, 336, True, "E4M3")[2] > 1
