@@ -67,25 +67,31 @@ struct Shape {
 // tiles of 128 x 256 on 148 SMs, three rounds and 68 tiles, which become 136 halves) and, where there are several, an epilogue of 12 bn.
 // Splitting K divides the blocks and adds an exchange that grows with the partial tile, 800 + 0.31 x rows x bn (1000 more with block
 // scales, whose six loading warps also fall behind once they have more than a block each), and shares out the epilogue, which counts
-// for every column that a group of its warps takes: 14 clocks for a full f32 operand (`f32_operands` of them), 20 for E4M3 codes, and 300 in
+// for every column that a group of its warps takes: 14 clocks for a full operand that is not loaded ahead (`operands` of them), 20 for E4M3 codes, and 300 in
 // every round where a thread stores its row element by element, as K in splits is added up and stored by neighbouring threads side by side.
 // Former costs -> these, in us: 777 x 4096 x 3072 bf16 [K, N] 26.9 (256 columns) -> 21.6 (192), 2050 x 1040 x 1040 13.0 -> 11.5, MXFP8
 // 15 x 1632 x 816 7.7 -> 6.3 (more splits). Where an exchange of 230 split K: 1 x 136 x 3648 bf16 4.0 whole, 5.0 in two. With bias, ReLU and a
-// full f32 operand, 128 x 384 x 384 f16: 6.0 in six, 7.5 whole. With rows of C off the 16-byte boundaries 128 x 512 x 1280 f16 6.9 in splits, 12.9
+// full f32 operand, 128 x 384 x 384 f16: 6.0 in six, 7.5 whole; with a bf16 one 1059 x 368 x 104 6.4 and 7.7. With rows of C off the 16-byte boundaries 128 x 512 x 1280 f16 6.9 in splits, 12.9
 // whole; FP8 128 x 1024 x 2688 to E5M2 10.2 and 29.2, 78 x 912 x 336 to E4M3 7.5 and 9.6.
 // f32 results and f32 operands (pieces) keep the former costs. Those split K more often, and an accumulator is off by 2^-24 of its value
 // for every block it takes, which a 16-bit result does not show and an f32 result does (128 x 640 x 3840 bf16 to f32: 1.7e-7 from
 // 64 bits in four splits, 5.9e-7 in one; 128 x 3328 x 1536 4.0e-7 and 6.4e-7). For pieces they are the quicker too (25 x 6312 x 6632 165 us, 196).
-inline Shape choose_shape(const Problem& p, int f32_operands) {
+// MATMUL_FP8's Amax_C is an f32 result beside a C of any type: new costs, but no accumulator of more blocks than by the former ones (956
+// products, Amax_C 5.9e-8 from 64 bits in the root mean square that way, 6.2e-8 without).
+inline Shape choose_shape(const Problem& p, int operands) {
     const int64_t blocks = (p.K * p.in_bytes + kRowBytes - 1) / kRowBytes;
     constexpr int clusters_at_once[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};   // (cudaOccupancyMaxActiveClusters, by CTAs per cluster)
     const int sms = 148;   // (a function of the shape alone: the count this library is built for)
-    const bool former = p.out_dtype == DFGPU_F32 || has_pieces(p);
-    Shape best{0, 0, 0, 0, 0, 0, 0.0};
+    const bool former_only = p.out_dtype == DFGPU_F32 || has_pieces(p), both = p.kind == kCodes && !former_only;
+    Shape best{0, 0, 0, 0, 0, 0, 0.0}, former_best = best, shapes[2 * 4 * 8];
+    int count = 0;
+    auto take = [](Shape& least, const Shape& shape) {
+        if (least.cg == 0 || shape.clocks < least.clocks) least = shape;
+    };
     for (int cg = 1; cg <= 2; ++cg)
         for (int bn = 64; bn <= 256; bn += 64) {
             const int chunk = sixteen_bits(p) ? 64 : 128;   // columns of one N-major copy
-            if (p.b_mn_major && (bn / cg) % chunk != 0 && !(cg == 2 && bn == 192 && !scaled(p) && !former)) continue;
+            if (p.b_mn_major && (bn / cg) % chunk != 0 && !(cg == 2 && bn == 192 && !scaled(p) && !former_only)) continue;
             if (p.out_dtype == DFGPU_E4M3 && bn % 128 != 0) continue;   // (whole 128-byte boxes)
             if (scaled(p) && bn % 128 != 0) continue;           // (whole chunks of column scales)
             if (cg == 2 && bn < 128) continue;
@@ -108,13 +114,16 @@ inline Shape choose_shape(const Problem& p, int f32_operands) {
                     rounds -= 0.45;
                 }
                 const double in_flight = static_cast<double>(stages_that_fit(stage_size, kSmemBudget - 2 * kStageBox)) * stage_size;
-                double clocks;
-                if (former) {
+                Shape shape{cg, bn, splits, static_cast<int>(k_per_split), tiles, halved, 0.0};
+                const bool whole_boxes = !p.b_mn_major || (bn / cg) % chunk == 0;
+                if (former_only || (both && whole_boxes)) {
                     const double products = has_pieces(p) ? 6.0 : 1.0, pieces = has_pieces(p) ? 3.0 : 1.0;
                     const double summed = in_registers(p) ? 150.0 + 2.0 * bn : (p.kind == kScaledSummed ? 250.0 + 3.0 * bn : 0.0);   // the epilogue's loads and additions of a block
                     const double block = std::max({summed, products * 2.0 * bn, (products + pieces) * (rows + bn / cg), pieces * (rows + bn / cg) * kRowBytes / std::min(48.0, in_flight / 2300.0)});
-                    clocks = rounds * (k_per_split * block) + 2000.0 + bn * 6.0 + (splits > 1 ? (scaled(p) ? 5000.0 : 2500.0) : 0.0) + (cg == 2 ? 1500.0 : 0.0);
-                } else {
+                    shape.clocks = rounds * (k_per_split * block) + 2000.0 + bn * 6.0 + (splits > 1 ? (scaled(p) ? 5000.0 : 2500.0) : 0.0) + (cg == 2 ? 1500.0 : 0.0);
+                    take(former_best, shape);
+                }
+                if (!former_only) {
                     const int columns = loaded_columns(p, bn, cg);
                     const double active = static_cast<double>(std::min<int64_t>(sms, tiles * cg * splits));
                     const double rate = std::min({48.0, 6300.0 / active, in_flight / 3400.0});
@@ -122,12 +131,16 @@ inline Shape choose_shape(const Problem& p, int f32_operands) {
                     const int box = p.direct_stores ? 32 : kRowBytes / p.out_bytes, serial = std::min(bn, (bn / box + 1) / 2 * box);   // (columns that one epilogue group takes)
                     const double exchange = splits > 1 ? 800.0 + 0.31 * std::min<double>(rows, static_cast<double>(p.M)) * bn + (scaled(p) ? 1000.0 : 0.0) : 0.0;
                     const double stores = p.direct_stores ? 300.0 * std::ceil(rounds) : (p.out_dtype == DFGPU_E4M3 ? 20.0 : 0.0);
-                    const double epilogue = splits > 1 ? 0.0 : (14.0 * f32_operands + stores) * serial;
-                    clocks = rounds * (k_per_split * block + (rounds > 1.0 ? 12.0 * bn : 0.0)) + 2000.0 + exchange + epilogue + (scaled(p) && k_per_split > 6 ? 450.0 : 0.0) + (cg == 2 ? 1480.0 : 0.0);
+                    const double epilogue = splits > 1 ? 0.0 : (14.0 * operands + stores) * serial;
+                    shape.clocks = rounds * (k_per_split * block + (rounds > 1.0 ? 12.0 * bn : 0.0)) + 2000.0 + exchange + epilogue + (scaled(p) && k_per_split > 6 ? 450.0 : 0.0) + (cg == 2 ? 1480.0 : 0.0);
+                    if (both) shapes[count++] = shape;
+                    else take(best, shape);
                 }
-                if (best.cg == 0 || clocks < best.clocks) best = Shape{cg, bn, splits, static_cast<int>(k_per_split), tiles, halved, clocks};
             }
         }
+    if (former_only) return former_best;
+    for (int i = 0; i < count; ++i)
+        if (shapes[i].k_per_split <= former_best.k_per_split) take(best, shapes[i]);
     return best;
 }
 

@@ -986,9 +986,9 @@ int launch_kernel(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUte
 // Everything but the epilogue's operands and the operand formats, which the callers have put into `args`.
 int launch_problem(Problem p, TileArgs& args, const void* a, const void* b, void* c, cudaStream_t stream, const char* what) {
     p.direct_stores = !on16(c) || (p.c_ld * p.out_bytes) % 16 != 0 || p.out_dtype == DFGPU_E5M2;
-    int f32_operands = 0;   // full ADD operands in 32 bits
-    for (int s = 0; s < args.step_count; ++s) f32_operands += args.step_kind[s] == kStepFull && args.step_dtype[s] == DFGPU_F32 ? 1 : 0;
-    const Shape shape = choose_shape(p, f32_operands);
+    int operands = 0;   // full ADD operands that are not loaded ahead
+    for (int s = 0; s < args.step_count; ++s) operands += args.step_kind[s] == kStepFull && (s > 0 || args.step_dtype[s] == DFGPU_F32 || p.kind != kSixteen) ? 1 : 0;
+    const Shape shape = choose_shape(p, operands);
     const int chunk = sixteen_bits(p) ? 64 : 128;
     args.m_total = static_cast<int>(p.M);
     args.n_total = static_cast<int>(p.N);
