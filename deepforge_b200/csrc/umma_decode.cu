@@ -36,6 +36,7 @@ struct DecodeArgs {
     int32_t table_len_k, table_len_v;
     int32_t num_pages;
     int32_t max_chunks, tiles_per_cta;
+    int32_t tile_step;        // key tiles from one of a CTA's tiles to its next: 1, or max_chunks (interleaves())
     int32_t has_left, has_right, bottom_right, padding;
     int64_t left, right, s_kv;
     float scale_log2;
@@ -173,7 +174,9 @@ sdpa_decode_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     // paying a dependent global load per tile. An id outside the container is stored as -1 (its rows read as zeros).
     int32_t* page_ids = reinterpret_cast<int32_t*>(generic_base + DecodeSmem::kPages);
     const bool is_v = threadIdx.x >= 64;
-    const int entry = threadIdx.x & 63, table_slot = chunk * args.tiles_per_cta * args.pages_per_tile + entry;
+    const int tile0 = args.tile_step == 1 ? chunk * args.tiles_per_cta : chunk;   // this CTA's key tiles: tile0, tile0 + tile_step, ...
+    const int entry = threadIdx.x & 63, entry_tile = entry >> (31 - __clz(args.pages_per_tile));   // (a power of two)
+    const int table_slot = tile0 * args.pages_per_tile + entry + entry_tile * (args.tile_step - 1) * args.pages_per_tile;
     const void* offsets = is_v ? args.offsets_v : args.offsets_k;
     const bool in_table = threadIdx.x < 128 && entry < args.tiles_per_cta * args.pages_per_tile && table_slot < (is_v ? args.table_len_v : args.table_len_k);
     int64_t page = -1;
@@ -183,10 +186,13 @@ sdpa_decode_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 
     int64_t lo, hi;
     key_window(args, batch, lo, hi);
-    const int64_t chunk_begin = static_cast<int64_t>(chunk) * args.tiles_per_cta * kTileKeys;
-    const int64_t chunk_end_all = chunk_begin + args.tiles_per_cta * kTileKeys;
+    // those of them that intersect the window: the first_tile-th and `tiles` in all
+    const int below = static_cast<int>(lo / kTileKeys) - tile0, until = static_cast<int>((hi + kTileKeys - 1) / kTileKeys) - tile0;   // from this CTA's first tile: tiles before the window, and up to its end
+    auto own_tiles = [&](int count) { return args.tile_step == 1 ? count : static_cast<int>((static_cast<unsigned>(count) + args.tile_step - 1) / static_cast<unsigned>(args.tile_step)); };
+    const int first_tile = below > 0 ? own_tiles(below) : 0;
+    const int tiles = until > 0 ? min(args.tiles_per_cta, own_tiles(until)) - first_tile : 0;
     float* my_partial = args.partial + ((batch * args.heads_q + static_cast<int64_t>(kv_head) * G) * args.max_chunks + chunk) * kPartialStride;
-    if (chunk_begin >= hi || chunk_end_all <= lo) {
+    if (tiles <= 0 || lo >= hi) {
         if (threadIdx.x < G) {
             float* p = my_partial + static_cast<int64_t>(threadIdx.x) * args.max_chunks * kPartialStride;
             p[kDim] = -INFINITY;
@@ -195,10 +201,6 @@ sdpa_decode_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         if (warp == 1) tmem_dealloc(*tmem_slot_ptr, 64);
         return;
     }
-    // tiles of this CTA that intersect the window
-    const int first_tile = lo > chunk_begin ? static_cast<int>((lo - chunk_begin) / kTileKeys) : 0;
-    const int64_t last_key = (hi < chunk_end_all ? hi : chunk_end_all) - 1;
-    const int tiles = static_cast<int>((last_key - chunk_begin) / kTileKeys) + 1 - first_tile;
 
     if (in_table && offsets && args.prefix_ok[is_v ? 1 : 0]) {
         const int64_t length = args.seq_kv[batch * args.seq_kv_stride];
@@ -322,7 +324,7 @@ sdpa_decode_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         }
         for (int j = 0; j < tiles; ++j) {
             const int b = j & 1;
-            const int64_t key = chunk_begin + static_cast<int64_t>(first_tile + j) * kTileKeys + key_lane;
+            const int64_t key = (tile0 + static_cast<int64_t>(first_tile + j) * args.tile_step) * kTileKeys + key_lane;
             // page validity of this key (an invalid page reads as zeros: score 0, no contribution to O)
             const int entry = ((first_tile + j) * kTileKeys + key_lane) / args.block;
             const bool k_page_ok = page_ids[entry] >= 0, v_page_ok = page_ids[64 + entry] >= 0;
@@ -465,8 +467,18 @@ static int tiles_per_cta(const dfgpu_sdpa_params& p) {
     while (per_cta > 1 && 2 * lists * ((tiles + per_cta - 1) / per_cta) < 3 * 148) per_cta /= 2;
     return per_cta;
 }
-int decode_umma_chunk_keys(const dfgpu_sdpa_params& p) { return tiles_per_cta(p) * kTileKeys; }
-int decode_umma_chunks(const dfgpu_sdpa_params& p) { return static_cast<int>((p.s_kv + decode_umma_chunk_keys(p) - 1) / decode_umma_chunk_keys(p)); }
+int decode_umma_chunks(const dfgpu_sdpa_params& p) {
+    const int64_t chunk_keys = static_cast<int64_t>(tiles_per_cta(p)) * kTileKeys;
+    return static_cast<int>((p.s_kv + chunk_keys - 1) / chunk_keys);
+}
+// A CTA's key tiles lie side by side where the CTAs are many: those past a sequence's end leave at once, and the others have fewer prologues and
+// partial results between them. Where all of them are on the chip together (two per SM) the tiles go round the CTAs instead, so that
+// a sequence of any length is shared out over all of its CTAs: its length is not known here, only the most it may be. 4 x 8 KV heads of up to
+// 8192 keys 17.9 -> 13.5 us, one sequence of 8 KV heads with up to 32768 20.5 -> 17.0. With four tiles a CTA or fewer a shorter walk no longer
+// pays for the prologues and the partial results (two sequences of up to 8192: 16.3 and 16.8; up to 16384 with 4 KV heads: 13.5 and 13.0).
+static bool interleaves(const dfgpu_sdpa_params& p) { return tiles_per_cta(p) == kMaxTilesPerCta && p.q.dim[0] * p.k.dim[1] * decode_umma_chunks(p) <= 2 * 148; }
+// Chunk c holds keys only where the sequence is longer than c times this.
+int decode_umma_chunk_keys(const dfgpu_sdpa_params& p) { return interleaves(p) ? kTileKeys : tiles_per_cta(p) * kTileKeys; }
 
 bool decode_umma_supported(const dfgpu_sdpa_params& p) {
     if (p.q.rank != 4 || p.k.rank != 4 || p.v.rank != 4) return false;
@@ -518,6 +530,7 @@ int launch_decode_umma(const dfgpu_sdpa_params& p, void* const* tensors, void* s
     args.num_pages = static_cast<int>(pages);
     args.max_chunks = decode_umma_chunks(p);
     args.tiles_per_cta = tiles_per_cta(p);
+    args.tile_step = interleaves(p) ? args.max_chunks : 1;
     args.has_left = p.has_left_bound;
     args.has_right = p.has_right_bound;
     args.bottom_right = p.bottom_right;

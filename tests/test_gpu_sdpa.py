@@ -472,3 +472,22 @@ def test_tma_paged_decode_long_sequences_and_windows():
                                                   128 ** -0.5, kernel, seq=([1] * batch, lengths), tables=(tk, tv), **flags)
             close_bf16(o, o_ref)
             close_f32(rows[0], rows_ref[0], 1e-3)
+
+
+@pytest.mark.parametrize("batch,hkv,block,max_len", [(14, 8, 64, 2000), (4, 2, 64, 32700), (4, 2, 16, 29000)])
+def test_paged_decode_key_tiles_that_go_round_the_ctas(batch, hkv, block, max_len):
+    """Eight key tiles a CTA and all CTAs on the chip at once: a CTA's tiles lie as many tiles apart as a sequence has CTAs. Lengths of
+    nothing, one key, one tile and one key more, one short of a round of tiles, one tile over a round and everything; windows that
+    start and end inside a round; page ids outside the container in the first and a later round."""
+    hq, pages = 4 * hkv, max_len // block + 70
+    chunks = -(-max_len // 1024)
+    assert 3 * 148 <= 2 * batch * hkv * chunks <= 4 * 148
+    lengths = ([max_len, 0, 1, 129, 128 * chunks - 1, 128 * chunks + 1] * 3)[:batch]
+    lengths, tk, tv = _paged_inputs(batch, hq, hkv, pages, block, max_len, seed=91, lengths=lengths)
+    tk[0, 1], tv[0, (128 * chunks + 130) // block] = -1, pages + 7
+    for flags in ({}, dict(has_left_bound=1, left_bound=128 * chunks + 200, bottom_right=1), dict(has_right_bound=1, right_bound=-140, bottom_right=1)):
+        info, o, o_ref, rows, rows_ref = both(BF16, [batch, hq, 1, 128], [pages, hkv, block, 128], [pages, hkv, block, 128], max_len,
+                                              128 ** -0.5, dfgpu.SDPA_PAGED_DECODE_UMMA, seq=([1] * batch, lengths), tables=(tk, tv), **flags)
+        close_bf16(o, o_ref)
+        for a, r in zip(rows, rows_ref):
+            close_f32(a, r, 1e-3)
