@@ -146,6 +146,11 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
                  ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar) : "memory");
 }
 
+// Starts the fetch of a box into the L2 cache.
+__device__ __forceinline__ void prefetch_box_4d(const CUtensorMap* map, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global [%0, {%1, %2, %3, %4}];" ::"l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
+
 // Starts the fetch of a tensor map into the TMA unit's descriptor cache; the first copy that uses the map otherwise
 // pays that global-memory round trip on the critical path of the kernel's prologue.
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {

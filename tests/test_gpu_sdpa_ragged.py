@@ -98,7 +98,7 @@ def test_strides_scale_and_misalignment():
 @pytest.mark.parametrize("b,h,hkv,sq,skv,causal,scale", [(1, 37, 37, 1000, 1000, True, None), (1, 40, 8, 700, 700, True, 1.5), (2, 60, 12, 256, 1500, False, 1.5), (1, 148, 4, 200, 129, False, None),
                                                          (1, 16, 8, 2171, 2171, True, None), (2, 96, 96, 300, 300, True, 1.5)])
 def test_several_items_per_place(io, b, h, hkv, sq, skv, causal, scale):
-    """More work items than SMs or pairs of SMs, which walk them one after another, with maxima that jump."""
+    """More work items than SMs, which walk them one after another, with maxima that jump."""
     check(b, h, hkv, sq, skv, 128, io, causal, scale=scale)
 
 
@@ -118,10 +118,24 @@ def test_padded_items_by_their_lengths(io, d, b, h, sq, causal):
     check(b, h, 1, sq, sq, d, io, causal, padding=(lengths[::-1], lengths), fine=True)
 
 
+@pytest.mark.parametrize("b,sq,causal", [(256, 500, True), (257, 500, True), (256, 500, False), (255, 512, True)])
+def test_padded_items_as_many_as_are_listed(b, sq, causal):
+    """1024 (batch, query tile)s are put in order by their lengths, 1028 are not, and 1020 are."""
+    lengths = [sq if i % 3 == 0 else (i * 97) % (sq + 1) for i in range(b)]
+    check(b, 1, 1, sq, sq, 64, "BFLOAT16", causal, padding=(lengths[::-1], lengths), fine=True)
+
+
+@pytest.mark.parametrize("b,h,s,padded", [(1, 230, 900, False), (10, 20, 1100, False), (1, 220, 1024, False), (10, 20, 1100, True), (10, 23, 900, True)])
+def test_more_keys_than_the_cache_holds(b, h, s, padded):
+    """Causal lists that stay with one head at a time, a heavy query tile and then a light one: even and odd numbers of tiles, whole tiles, lengths."""
+    lengths = ([s - 200 * (i % 4) for i in range(b)], [s - 130 * (i % 3) for i in range(b)]) if padded else None
+    check(b, h, h, s, s, 128, "BFLOAT16", True, padding=lengths, fine=s % 128 != 0)
+
+
 @pytest.mark.parametrize("io,d", [("BFLOAT16", 128), ("HALF", 128), ("BFLOAT16", 64), ("HALF", 64)])
 @pytest.mark.parametrize("b,h,hkv,sq,skv,causal", [(3, 1, 1, 17, 17, True), (5, 4, 1, 75, 89, False), (1, 37, 37, 1000, 1000, True), (2, 96, 96, 300, 300, True), (2, 60, 12, 256, 1500, False)])
 def test_probabilities_as_accurate_as_f32_ones(io, d, b, h, hkv, sq, skv, causal):
-    """On one SM and on two per pair of query tiles, short lists and long."""
+    """Short lists and long."""
     check(b, h, hkv, sq, skv, d, io, causal, fine=True)
 
 
