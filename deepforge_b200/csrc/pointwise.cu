@@ -343,12 +343,34 @@ __device__ __forceinline__ void store4<__half>(void* p, int64_t i, const float (
     *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p) + i) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
 }
 
+// Eight values of a 16-bit type.
+template <typename T>
+__device__ __forceinline__ void store8(void* p, int64_t i, const float (&v)[2][4]) {
+    uint32_t words[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float lo = v[j >> 1][2 * (j & 1)], hi = v[j >> 1][2 * (j & 1) + 1];
+        if constexpr (std::is_same_v<T, __nv_bfloat16>) {
+            const __nv_bfloat162 two = __floats2bfloat162_rn(lo, hi);
+            words[j] = *reinterpret_cast<const uint32_t*>(&two);
+        } else {
+            const __half2 two = __floats2half2_rn(lo, hi);
+            words[j] = *reinterpret_cast<const uint32_t*>(&two);
+        }
+    }
+    *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p) + i) = make_uint4(words[0], words[1], words[2], words[3]);
+}
+
 template <typename T> struct QuadsInFlight;
 template <> struct QuadsInFlight<float> { static constexpr int value = 2; };
 template <> struct QuadsInFlight<__nv_bfloat16> { static constexpr int value = 4; };
 template <> struct QuadsInFlight<__half> { static constexpr int value = 4; };
 
 constexpr int kPackedThreads = 256;
+// CTAs per SM of the dense kernel, which walk the tiles between them: with a tile each, 3072 CTAs of 4096 bf16 values and a bias took 10.2 us,
+// at most 12 or 16 per SM 9.9, 6 or 8 (all at once, in uneven shares) 10.1. In eights as well, and with the way to the mode's body
+// behind it when the kernel before ends, 9.4.
+constexpr unsigned kDenseBlocks = 16;
 
 template <typename T>
 unsigned packed_grid(int64_t total) {
@@ -364,6 +386,9 @@ __device__ __forceinline__ void packed_body(const void* a, const void* b, void* 
     constexpr int U = QuadsInFlight<T>::value;
     constexpr bool binary = input_count(MODE) == 2;
     const int64_t first = (static_cast<int64_t>(blockIdx.x) * U * kPackedThreads + threadIdx.x) * 4;
+    chain_wait();
+    a = after_chain(a);
+    b = after_chain(b);
     typename Quad<T>::type raw_x[U], raw_y[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -397,10 +422,8 @@ static_assert(DFGPU_PW_MODE_COUNT == 50, "DFGPU_PW_EVERY_MODE lists every mode")
 template <typename T, int INPUTS>
 __global__ void __launch_bounds__(kPackedThreads, (sizeof(T) == 2 && INPUTS == 2) ? 5 : 2048 / kPackedThreads)
 pointwise_general_packed_kernel(const void* a, const void* b, void* out, int mode, PointwiseScalars s, int64_t total) {
-    chain_begin();
-    a = after_chain(a);
-    b = after_chain(b);
-    switch (mode) {
+    chain_release();
+    switch (mode) {   // (each body waits for the kernel before: see dense_body())
 #define DFGPU_PW_CASE(M) case M: if constexpr (input_count(M) == INPUTS) packed_body<T, M>(a, b, out, s, total); break;
         DFGPU_PW_EVERY_MODE(DFGPU_PW_CASE)
 #undef DFGPU_PW_CASE
@@ -417,7 +440,7 @@ enum { kFull = 0, kPeriod = 1, kRepeat = 2 };
 struct DenseOperand {
     const void* data;
     int32_t kind;
-    int32_t vector;       // quads of this operand (or the value a quad repeats) may be read at once
+    int32_t vector;       // neighbouring values of this operand (or of what they repeat) that may be read at once: 8 (16-bit types), 4, or 0
     FastDivisor by;       // PERIOD: values before it starts again; REPEAT: outputs per value
 };
 
@@ -433,21 +456,53 @@ __device__ __forceinline__ uint32_t dense_index(const DenseOperand& o, uint32_t 
     const uint32_t q = fast_divide(i, o.by);
     return o.kind == kRepeat ? q : i - q * o.by.divisor;
 }
-// A quad, or the one value it repeats, as it is stored: nothing waits for it before widen_raw().
-template <typename T>
-__device__ __forceinline__ typename Quad<T>::type load_raw(const DenseOperand& o, uint32_t i) {
+// WIDTH values, or the one value they repeat, as they are stored: nothing waits for them before widen_raw().
+template <typename T, int WIDTH> struct Raw { uint32_t words[WIDTH * sizeof(T) / 4]; };
+template <typename T, int WIDTH>
+__device__ __forceinline__ Raw<T, WIDTH> load_raw(const DenseOperand& o, uint32_t i) {
+    Raw<T, WIDTH> raw{};
+    const T* p = static_cast<const T*>(o.data) + dense_index(o, i);
     if (o.kind == kRepeat) {
-        typename Quad<T>::type raw{};
-        if constexpr (sizeof(T) == 4) raw.x = __ldg(static_cast<const float*>(o.data) + dense_index(o, i));
-        else raw.x = __ldg(static_cast<const uint16_t*>(o.data) + dense_index(o, i));
-        return raw;
+        if constexpr (sizeof(T) == 4) raw.words[0] = __ldg(reinterpret_cast<const uint32_t*>(p));
+        else raw.words[0] = __ldg(reinterpret_cast<const uint16_t*>(p));
+    } else if constexpr (sizeof(raw) == 16) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+        raw.words[0] = v.x, raw.words[1] = v.y, raw.words[2] = v.z, raw.words[3] = v.w;
+    } else {
+        const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+        raw.words[0] = v.x, raw.words[1] = v.y;
     }
-    return load_quad<T>(o.data, dense_index(o, i));
+    return raw;
 }
-template <typename T>
-__device__ __forceinline__ void widen_raw(const DenseOperand& o, const typename Quad<T>::type& raw, float (&v)[4]) {
-    widen(raw, v);
-    if (o.kind == kRepeat) v[1] = v[2] = v[3] = v[0];
+// Values 4 * quad ... 4 * quad + 3 of them.
+template <typename T, int WIDTH>
+__device__ __forceinline__ void widen_raw(const DenseOperand& o, const Raw<T, WIDTH>& raw, int quad, float (&v)[4]) {
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = __uint_as_float(raw.words[j]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const uint32_t two = raw.words[2 * quad + j];
+            if constexpr (std::is_same_v<T, __nv_bfloat16>) {
+                v[2 * j] = __uint_as_float(two << 16);
+                v[2 * j + 1] = __uint_as_float(two & 0xffff0000u);
+            } else {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&two));
+                v[2 * j] = f.x;
+                v[2 * j + 1] = f.y;
+            }
+        }
+    }
+    if (o.kind == kRepeat) {
+        float one = v[0];
+        if constexpr (sizeof(T) == 2)
+            if (quad > 0) {   // (the one value lies in the first word)
+                if constexpr (std::is_same_v<T, __nv_bfloat16>) one = __uint_as_float(raw.words[0] << 16);
+                else one = __low2float(*reinterpret_cast<const __half2*>(&raw.words[0]));
+            }
+        v[0] = v[1] = v[2] = v[3] = one;
+    }
 }
 template <typename T>
 __device__ __forceinline__ void load_dense(const DenseOperand& o, uint32_t i, uint32_t total, float (&v)[4]) {
@@ -461,44 +516,65 @@ __device__ __forceinline__ void load_dense(const DenseOperand& o, uint32_t i, ui
     for (int j = 0; j < 4; ++j) v[j] = i + j < total ? one_value<T>(o.data, dense_index(o, i + j)) : 0.0f;
 }
 
-template <typename T, int MODE>
-__device__ __forceinline__ void dense_body(const DenseOperand& a, const DenseOperand& b, void* out, bool out_vector, const PointwiseScalars& s, uint32_t total) {
-    constexpr int U = QuadsInFlight<T>::value;
+template <typename T, int MODE, int WIDTH>
+__device__ __forceinline__ void dense_tile(const DenseOperand& a, const DenseOperand& b, void* out, const PointwiseScalars& s, uint32_t tile) {
+    constexpr int U = QuadsInFlight<T>::value * 4 / WIDTH;
     constexpr bool binary = input_count(MODE) == 2;
-    const uint32_t first = (blockIdx.x * U * kPackedThreads + threadIdx.x) * 4;
-    if (a.vector && (!binary || b.vector) && out_vector && (blockIdx.x + 1) * U * kPackedThreads * 4 <= total) {
-        typename Quad<T>::type raw_x[U], raw_y[U];
+    const uint32_t first = tile + threadIdx.x * WIDTH;
+    Raw<T, WIDTH> raw_x[U], raw_y[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {   // every load in flight before the first value is used
-            raw_x[u] = load_raw<T>(a, first + u * kPackedThreads * 4);
-            if (binary) raw_y[u] = load_raw<T>(b, first + u * kPackedThreads * 4);
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            float x[4], y[4] = {0.0f, 0.0f, 0.0f, 0.0f}, r[4];
-            widen_raw<T>(a, raw_x[u], x);
-            if (binary) widen_raw<T>(b, raw_y[u], y);
-            four_values<T, MODE>(x, y, s, r);
-            store4<T>(out, first + u * kPackedThreads * 4, r);
-        }
-        return;
+    for (int u = 0; u < U; ++u) {   // every load in flight before the first value is used
+        raw_x[u] = load_raw<T, WIDTH>(a, first + u * kPackedThreads * WIDTH);
+        if (binary) raw_y[u] = load_raw<T, WIDTH>(b, first + u * kPackedThreads * WIDTH);
     }
-#pragma unroll 1
+#pragma unroll
     for (int u = 0; u < U; ++u) {
-        const uint32_t i = first + u * kPackedThreads * 4;
-        if (i >= total) break;
-        float x[4], y[4] = {0.0f, 0.0f, 0.0f, 0.0f}, r[4];
-        load_dense<T>(a, i, total, x);
-        if (binary) load_dense<T>(b, i, total, y);
-        four_values<T, MODE>(x, y, s, r);
-        if (out_vector && i + 4 <= total) {
-            store4<T>(out, i, r);
-        } else {
-            for (int j = 0; j < 4; ++j) {
-                if (i + j >= total) break;
-                if constexpr (sizeof(T) == 4) static_cast<float*>(out)[i + j] = r[j];
-                else if constexpr (std::is_same_v<T, __nv_bfloat16>) static_cast<uint16_t*>(out)[i + j] = f32_to_bf16_bits(r[j]);
-                else static_cast<__half*>(out)[i + j] = __float2half_rn(r[j]);
+        float r[WIDTH / 4][4];
+#pragma unroll
+        for (int quad = 0; quad < WIDTH / 4; ++quad) {
+            float x[4], y[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            widen_raw<T, WIDTH>(a, raw_x[u], quad, x);
+            if (binary) widen_raw<T, WIDTH>(b, raw_y[u], quad, y);
+            four_values<T, MODE>(x, y, s, r[quad]);
+        }
+        if constexpr (WIDTH == 8) store8<T>(out, first + u * kPackedThreads * WIDTH, r);
+        else store4<T>(out, first + u * kPackedThreads * WIDTH, r[0]);
+    }
+}
+template <typename T, int MODE>
+__device__ __forceinline__ void dense_body(DenseOperand& a, DenseOperand& b, void* out, int out_vector, const PointwiseScalars& s, uint32_t total) {
+    constexpr int U = QuadsInFlight<T>::value;
+    constexpr uint32_t kTile = U * kPackedThreads * 4;
+    constexpr bool binary = input_count(MODE) == 2;
+    const int width = min(out_vector, min(a.vector, binary ? b.vector : 8));
+    chain_wait();   // (here, when the mode's code and the operands' forms are known)
+    a.data = after_chain(a.data);
+    b.data = after_chain(b.data);
+#pragma unroll 1
+    for (uint32_t tile = blockIdx.x * kTile; tile < total; tile += gridDim.x * kTile) {
+        if (width != 0 && tile + kTile <= total) {
+            if (sizeof(T) == 2 && width == 8) dense_tile<T, MODE, sizeof(T) == 2 ? 8 : 4>(a, b, out, s, tile);
+            else dense_tile<T, MODE, 4>(a, b, out, s, tile);
+            continue;
+        }
+        const uint32_t first = tile + threadIdx.x * 4;
+#pragma unroll 1
+        for (int u = 0; u < U; ++u) {
+            const uint32_t i = first + u * kPackedThreads * 4;
+            if (i >= total) break;
+            float x[4], y[4] = {0.0f, 0.0f, 0.0f, 0.0f}, r[4];
+            load_dense<T>(a, i, total, x);
+            if (binary) load_dense<T>(b, i, total, y);
+            four_values<T, MODE>(x, y, s, r);
+            if (out_vector && i + 4 <= total) {
+                store4<T>(out, i, r);
+            } else {
+                for (int j = 0; j < 4; ++j) {
+                    if (i + j >= total) break;
+                    if constexpr (sizeof(T) == 4) static_cast<float*>(out)[i + j] = r[j];
+                    else if constexpr (std::is_same_v<T, __nv_bfloat16>) static_cast<uint16_t*>(out)[i + j] = f32_to_bf16_bits(r[j]);
+                    else static_cast<__half*>(out)[i + j] = __float2half_rn(r[j]);
+                }
             }
         }
     }
@@ -507,11 +583,9 @@ __device__ __forceinline__ void dense_body(const DenseOperand& a, const DenseOpe
 template <typename T, int INPUTS>
 __global__ void __launch_bounds__(kPackedThreads)
 pointwise_dense_kernel(DenseOperand a, DenseOperand b, void* out, int out_vector, int mode, PointwiseScalars s, uint32_t total) {
-    chain_begin();
-    a.data = after_chain(a.data);
-    b.data = after_chain(b.data);
-    switch (mode) {
-#define DFGPU_PW_CASE(M) case M: if constexpr (input_count(M) == INPUTS) dense_body<T, M>(a, b, out, out_vector != 0, s, total); break;
+    chain_release();
+    switch (mode) {   // (each body waits for the kernel before)
+#define DFGPU_PW_CASE(M) case M: if constexpr (input_count(M) == INPUTS) dense_body<T, M>(a, b, out, out_vector, s, total); break;
         DFGPU_PW_EVERY_MODE(DFGPU_PW_CASE)
 #undef DFGPU_PW_CASE
         default: break;
@@ -532,6 +606,13 @@ bool dense_order(const dfgpu_tensor& out, int (&order)[DFGPU_MAX_RANK], int& cou
     return expected < (1ll << 31) - 65536;
 }
 
+// Values that may be read or written at once, by the pointer, and at the start of every run of `length` of them.
+int vector_of(const void* data, int bytes) {
+    const uintptr_t address = reinterpret_cast<uintptr_t>(data);
+    return bytes == 2 && address % 16 == 0 ? 8 : (address % (4 * bytes) == 0 ? 4 : 0);
+}
+int vector_in(int64_t length, int bytes) { return bytes == 2 && length % 8 == 0 ? 8 : (length % 4 == 0 ? 4 : 0); }
+
 bool dense_operand(const dfgpu_tensor& t, const dfgpu_tensor& out, const int (&order)[DFGPU_MAX_RANK], int count, const void* data, DenseOperand& o) {
     const int shift = out.rank - t.rank;
     int64_t inner = 1, own = 1, held = 1;   // outputs and own values so far, from the innermost axis; outputs per own value
@@ -551,30 +632,31 @@ bool dense_operand(const dfgpu_tensor& t, const dfgpu_tensor& out, const int (&o
         inner *= extent;
     }
     const int bytes = dtype_bytes(t.dtype);
-    const bool on_quads = reinterpret_cast<uintptr_t>(data) % (4 * bytes) == 0;
+    const int aligned = vector_of(data, bytes);
     o.data = data;
     o.by = make_fast_divisor(1);
     if (held > 1) {
         if (period != 0) return false;
         o.kind = kRepeat;
         o.by = make_fast_divisor(static_cast<uint32_t>(held));
-        o.vector = held % 4 == 0;
+        o.vector = vector_in(held, bytes);
     } else if (period != 0) {
         o.kind = kPeriod;
         o.by = make_fast_divisor(static_cast<uint32_t>(period));
-        o.vector = period % 4 == 0 && on_quads;
+        o.vector = std::min(vector_in(period, bytes), aligned);
     } else {
         o.kind = kFull;
-        o.vector = on_quads;
+        o.vector = aligned;
     }
     return true;
 }
 
 template <typename T>
 void launch_dense(int inputs, const DenseOperand& a, const DenseOperand& b, void* out, int mode, const PointwiseScalars& s, int64_t total, cudaStream_t stream) {
-    const int out_vector = reinterpret_cast<uintptr_t>(out) % (4 * sizeof(T)) == 0;
-    if (inputs == 1) launch_chained(pointwise_dense_kernel<T, 1>, dim3(packed_grid<T>(total)), dim3(kPackedThreads), 0, stream, a, b, out, out_vector, mode, s, static_cast<uint32_t>(total));
-    else launch_chained(pointwise_dense_kernel<T, 2>, dim3(packed_grid<T>(total)), dim3(kPackedThreads), 0, stream, a, b, out, out_vector, mode, s, static_cast<uint32_t>(total));
+    const int out_vector = vector_of(out, sizeof(T));
+    const unsigned grid = std::min(packed_grid<T>(total), kDenseBlocks * static_cast<unsigned>(sm_count()));
+    if (inputs == 1) launch_chained(pointwise_dense_kernel<T, 1>, dim3(grid), dim3(kPackedThreads), 0, stream, a, b, out, out_vector, mode, s, static_cast<uint32_t>(total));
+    else launch_chained(pointwise_dense_kernel<T, 2>, dim3(grid), dim3(kPackedThreads), 0, stream, a, b, out, out_vector, mode, s, static_cast<uint32_t>(total));
 }
 
 template <typename T>

@@ -38,6 +38,20 @@ def test_broadcast_counts_and_pointers(io, dims, b_dims, offset):
     assert torch.equal(out[:math.prod(dims)].view(dims), want) and bool(torch.all(out[math.prod(dims):] == 7.0))
 
 
+@pytest.mark.parametrize("io", ["FLOAT", "BFLOAT16", "HALF"])
+@pytest.mark.parametrize("dims,b_dims", [([700, 24], [1, 24]), ([700, 28], [1, 28]), ([700, 24], [700, 1]), ([700, 28], [700, 1]), ([512, 24], [1, 1]), ([2400, 4104], [1, 4104])])
+@pytest.mark.parametrize("offsets", [(0, 0, 0), (4, 0, 0), (0, 4, 0), (0, 0, 4)])
+def test_eights_fours_and_singles(io, dims, b_dims, offsets):
+    """Runs of whole eights and of a four more, pointers on eight values and on four, a last tile that is not full, several tiles a CTA."""
+    g = torch.Generator(device="cuda").manual_seed(dims[-1])
+    a, b = (torch.randn(math.prod(d) + o, device="cuda", generator=g).to(TORCH[io])[o:] for d, o in zip((dims, b_dims), offsets))
+    out = torch.full((math.prod(dims) + 8 + offsets[2],), 7.0, device="cuda").to(TORCH[io])[offsets[2]:]
+    tensors = [graphs.tensor(1, "A", dims, io), graphs.tensor(2, "B", b_dims, io), graphs.tensor(3, "O", dims, io)]
+    execute(graphs.document("dense", [graphs.pointwise_node("sub", "SUB", 1, 3, 2)], tensors, io=io), {1: a, 2: b, 3: out})
+    want = (a.view(dims).float() - b.view(b_dims).float()).to(TORCH[io])
+    assert torch.equal(out[:math.prod(dims)].view(dims), want) and bool(torch.all(out[math.prod(dims):] == 7.0))
+
+
 def test_channels_last_bias_and_first_operand_broadcast():
     n, c, h, w = 2, 24, 5, 7
     g = torch.Generator(device="cuda").manual_seed(1)
