@@ -93,6 +93,8 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t address_in(uint32_t own_address, uint32_t rank) {
     uint32_t remote;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(own_address), "r"(rank));
@@ -879,39 +881,67 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
     if (split) {
         // ---- the cluster's partial tiles: every CTA adds its share of the live rows over all ranks, in rank order ----
-        __syncthreads();
-        cluster_sync_all();
+        // (Latencies one behind the other: what does not need the other CTAs, places and the first fused operand, is fetched while they
+        // arrive, and a CTA lets the others leave as soon as their partial sums are in registers, not when its own are stored: 100 x 544 x 1008 f16 with
+        // bias and ReLU 6.15 -> 5.17 us, 128 x 4096 x 4096 bf16 11.6 -> 10.9, FP8 117 x 1040 x 416 7.3 -> 6.6, MXFP8 15 x 1632 x 816 6.1 -> 5.6.)
+        cluster_arrive();   // (all threads: this CTA's partial tile is in place)
         const Item item = item_at(args, first_item);
         const int row0 = item.m_tile * kRows, live_rows = min(kRows, args.m_total - row0);
         const int share = (live_rows + args.splits - 1) / args.splits, begin = rank * share, end = min(live_rows, begin + share);
-        const int quads = bn / 4;
+        const int quad_bits = 31 - __clz(bn >> 2), count = max(0, end - begin) << quad_bits;   // (bn is 64 or 128)
         Scalars scalars = load_scalars<kCodesOnly>(args);
+        const bool ahead = !kCodesOnly && args.step_count > 0 && args.step_kind[0] != kStepRelu && args.step_dtype[0] != DFGPU_F32;
+        uint32_t operand[2] = {};
+        auto row_of = [&](int i) { return begin + (i >> quad_bits); };
+        auto column_of = [&](int i) { return item.col0 + (i & ((1 << quad_bits) - 1)) * 4; };
+        auto fetch = [&](int i) {
+            const int col = column_of(i);
+            if (ahead && i < count && col < args.n_total)
+                load_words<4>(operand, static_cast<const uint16_t*>(args.step_data[0]) + (args.step_kind[0] == kStepBias ? 0 : (row0 + row_of(i)) * args.step_ld[0]) + col, args.n_total - col,
+                              args.step_vector[0] != 0);
+        };
+        fetch(static_cast<int>(threadIdx.x));
+        cluster_wait();
         const bool healthy = g_device_status == 0;
-        for (int i = threadIdx.x; i < (end - begin) * quads; i += blockDim.x) {
-            const int row = begin + i / quads, unit = i % quads;
-            const int col = item.col0 + unit * 4;
-            if (col >= args.n_total) continue;
+        bool left = false;
+        for (int first = warp * 32; first < count; first += static_cast<int>(blockDim.x)) {
+            const int i = first + lane, row = row_of(i), unit = i & ((1 << quad_bits) - 1), col = column_of(i);
+            const bool mine = i < count && col < args.n_total;
             const uint32_t at = smem_base + row * bn * 4 + (((unit & ~7) | ((unit ^ row) & 7)) << 4);
             constexpr int kMost = 8;
-            float4 part[kMost];
+            float v[4] = {};
+            if (mine) {
+                float4 part[kMost];
 #pragma unroll
-            for (int z = 0; z < kMost; ++z)   // every load in flight before the first sum
-                if (z < args.splits) part[z] = load_from_rank(address_in(at, z));
-            float v[4] = {part[0].x, part[0].y, part[0].z, part[0].w};
+                for (int z = 0; z < kMost; ++z)   // every load in flight before the first sum
+                    if (z < args.splits) part[z] = load_from_rank(address_in(at, z));
+                v[0] = part[0].x, v[1] = part[0].y, v[2] = part[0].z, v[3] = part[0].w;
 #pragma unroll
-            for (int z = 1; z < kMost; ++z) {
-                if (z >= args.splits) break;
-                v[0] = __fadd_rn(v[0], part[z].x);
-                v[1] = __fadd_rn(v[1], part[z].y);
-                v[2] = __fadd_rn(v[2], part[z].z);
-                v[3] = __fadd_rn(v[3], part[z].w);
+                for (int z = 1; z < kMost; ++z) {
+                    if (z >= args.splits) break;
+                    v[0] = __fadd_rn(v[0], part[z].x);
+                    v[1] = __fadd_rn(v[1], part[z].y);
+                    v[2] = __fadd_rn(v[2], part[z].z);
+                    v[3] = __fadd_rn(v[3], part[z].w);
+                }
             }
-            apply_steps<kCodesOnly, 4, 4>(args, v, row0 + row, col, true, scalars);
-            if (healthy) store_four(args, v, row0 + row, col);
+            if (first + static_cast<int>(blockDim.x) >= count) {   // this warp's last look at the others' tiles
+                asm volatile("" : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]));
+                __syncwarp();
+                cluster_arrive();
+                left = true;
+            }
+            if (mine) {
+                if (ahead) apply_steps<kCodesOnly, 4, 4>(args, v, row0 + row, col, true, scalars, &operand);
+                else apply_steps<kCodesOnly, 4, 4>(args, v, row0 + row, col, true, scalars);
+                if (healthy) store_four(args, v, row0 + row, col);
+            }
+            if (!left) fetch(i + static_cast<int>(blockDim.x));
         }
         __syncwarp();
+        if (!left) cluster_arrive();
         fold_amax<kCodesOnly>(args, scalars, lane, healthy);
-        cluster_sync_all();   // no CTA leaves while another still reads its partial tile
+        cluster_wait();   // no CTA leaves while another still reads its partial tile
     }
     tc_fence_before();
     __syncthreads();

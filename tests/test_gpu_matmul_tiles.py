@@ -41,6 +41,25 @@ def close(got, a, b, after, out_type, k):
     assert torch.all((got.double() - want).abs() <= bound), float(((got.double() - want).abs() / bound).max())
 
 
+@pytest.mark.parametrize("m,n", [(1, 99), (5, 130), (5, 66), (100, 99), (128, 128), (130, 65), (12, 1001)])
+@pytest.mark.parametrize("k", [520, 4096])
+@pytest.mark.parametrize("first", ["bias", "addend", "f32 bias", "relu"])
+def test_sums_over_a_cluster_with_their_first_operand(m, n, k, first):
+    """K shared out over a cluster: CTAs without rows of their own, columns that end inside a four, a first fused operand that is fetched
+    while the partial tiles meet (16 bits, per column or full, its rows on no boundary) and ones that are not."""
+    io = "BFLOAT16"
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    full = first == "addend"
+    tensors = [graphs.tensor(1, "A", [m, k], io), graphs.tensor(2, "B", [k, n], io, [1, k]), graphs.tensor(3, "X", [m, n] if full else [1, n], "FLOAT" if first == "f32 bias" else io),
+               graphs.tensor(4, "C", [m, n], io), graphs.tensor(5, "p", [m, n], virtual=True), graphs.tensor(6, "q", [m, n], virtual=True)]
+    add, relu = (lambda i, o: graphs.pointwise_node("add", "ADD", i, o, 3)), (lambda i, o: graphs.pointwise_node("relu", "RELU_FWD", i, o))
+    nodes = [graphs.matmul_node("matmul", 1, 2, 5)] + ([relu(5, 6), add(6, 4)] if first == "relu" else [add(5, 6), relu(6, 4)])
+    buffers = {uid: torch.randn(count, device="cuda", generator=g).to(torch.float32 if uid == 3 and first == "f32 bias" else TORCH[io]) for uid, count in ((1, m * k), (2, k * n), (3, m * n if full else n))}
+    run(graphs.document("cluster", nodes, tensors, io=io), buffers)
+    x = buffers[3].double().view(m if full else 1, n)
+    close(buffers[4].view(m, n), buffers[1].view(m, k).double(), buffers[2].view(n, k).t().double(), (lambda p: torch.relu(p) + x) if first == "relu" else (lambda p: torch.relu(p + x)), io, k)
+
+
 @pytest.mark.parametrize("m,k,n", EXTENTS)
 @pytest.mark.parametrize("io", ["BFLOAT16", "HALF"])
 @pytest.mark.parametrize("b_k_major", [False, True])
