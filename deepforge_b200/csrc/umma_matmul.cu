@@ -255,9 +255,29 @@ __device__ __forceinline__ void add_operand(float (&v)[COUNT], const void* data,
     }
 }
 
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
 struct Scalars {
     float descale_a, descale_b, scale_c;
     float magnitude;   // largest |value| of this thread so far (NaN sticks)
+    // finite de-scales: `magnitude` is that of the accumulators, which they are applied to once, at the end. (Products with them and their roundings
+    // keep the order of magnitudes, and an infinity times zero is a NaN then as it would have been.)
+    bool at_end;
 };
 template <bool CODES>
 __device__ __forceinline__ Scalars load_scalars(const TileArgs& args) {
@@ -266,13 +286,15 @@ __device__ __forceinline__ Scalars load_scalars(const TileArgs& args) {
         s.descale_a = *args.descale_a;
         s.descale_b = *args.descale_b;
         s.scale_c = *args.scale_c;
+        s.at_end = fabsf(s.descale_a) < INFINITY && fabsf(s.descale_b) < INFINITY;
     }
     return s;
 }
 template <bool CODES>
 __device__ __forceinline__ void fold_amax(const TileArgs& args, const Scalars& s, int lane, bool ok) {
     if constexpr (!CODES) return;
-    unsigned int bits = s.magnitude != s.magnitude ? 0x7fc00000u : __float_as_uint(s.magnitude);
+    const float magnitude = s.at_end ? fabsf(__fmul_rn(__fmul_rn(s.magnitude, s.descale_a), s.descale_b)) : s.magnitude;
+    unsigned int bits = magnitude != magnitude ? 0x7fc00000u : __float_as_uint(magnitude);
     bits = __reduce_max_sync(0xffffffffu, bits);
     if (lane == 0 && bits != 0u && ok) atomicMax(args.amax_bits, bits);
 }
@@ -295,15 +317,24 @@ __device__ __forceinline__ void apply_steps(const TileArgs& args, float (&v)[COU
         }
     }
     if constexpr (CODES) {
-        float top = scalars.magnitude;
+        // value = (sum + 0) * descale_a * descale_b, C = value * scale_c, each rounded by itself, two at a time. (+0.0 first: the reference's
+        // sum starts from +0.0 and so is never -0.0, the tensor core's can be.) Where an epilogue is not hidden its instructions are what a
+        // tile waits for.
+        const uint64_t by_a = pack2(scalars.descale_a, scalars.descale_a), by_b = pack2(scalars.descale_b, scalars.descale_b), by_c = pack2(scalars.scale_c, scalars.scale_c);
+        float top = 0.0f;
 #pragma unroll
-        for (int e = 0; e < COUNT; ++e) {
-            // (+0.0 first: the reference's sum starts from +0.0 and so is never -0.0, the tensor core's can be)
-            const float value = __fmul_rn(__fmul_rn(__fadd_rn(v[e], 0.0f), scalars.descale_a), scalars.descale_b);
-            if (row_live && e < live) top = maximum_nan(top, fabsf(value));
-            v[e] = __fmul_rn(value, scalars.scale_c);
+        for (int e = 0; e < COUNT; e += 2) {
+            const uint64_t value = mul2(mul2(add2(pack2(v[e], v[e + 1]), 0ull), by_a), by_b);
+            float lo = v[e], hi = v[e + 1];
+            if (!scalars.at_end) unpack2(value, lo, hi);
+            if (live < COUNT) {
+                lo = e < live ? lo : 0.0f;
+                hi = e + 1 < live ? hi : 0.0f;
+            }
+            asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(top) : "f"(lo), "f"(hi));
+            unpack2(mul2(value, by_c), v[e], v[e + 1]);
         }
-        scalars.magnitude = top;
+        if (row_live) scalars.magnitude = maximum_nan(scalars.magnitude, top);
     }
 }
 
@@ -344,6 +375,18 @@ __device__ __forceinline__ void store_four(const TileArgs& args, const float (&v
     }
     for (int i = 0; i < 4; ++i)
         if (i < live) store_from_f32(args.out, args.out_dtype, at + i, v[i]);
+}
+
+// The status word, asked for here and looked at in healthy_now() alone: some 600 clocks later, a third of an epilogue part, which a
+// comparison beside the load would wait for.
+__device__ __forceinline__ int ask_status() {
+    int status;
+    asm volatile("ld.volatile.global.s32 %0, [%1];" : "=r"(status) : "l"(__cvta_generic_to_global(&g_device_status)) : "memory");
+    return status;
+}
+__device__ __forceinline__ bool healthy_now(bool ok, int status) {
+    asm volatile("" : "+r"(status));
+    return ok && status == 0;
 }
 
 template <bool CLUSTER>
@@ -733,7 +776,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     if (ok) ok = mbar_wait(acc_full(acc), use & 1, 505 + kCode);
                     tc_fence_after();
                 }
-                const bool healthy = ok && g_device_status == 0;
+                const int status = ask_status();
                 const uint32_t columns = tmem_base + lane_base + (kInPlace<KIND> ? args.sums_column : acc * args.acc_stride);
                 const int boxes = item.width / box_columns;
                 for (int b = g; b < boxes; b += 2) {
@@ -785,7 +828,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         }
                         if (args.tma_store) {
                             uint8_t* target = generic_base + staging + row * 128;
-                            if (args.out_dtype == DFGPU_F32) {
+                            if (kInRegisters<KIND> || KIND == kScaledSummed || args.out_dtype == DFGPU_F32) {   // (those have f32 results only)
 #pragma unroll
                                 for (int j = 0; j < 8; ++j)
                                     *reinterpret_cast<float4*>(target + ((j ^ (row & 7)) << 4)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
@@ -795,13 +838,17 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                                     *reinterpret_cast<uint4*>(target + (((part * 2 + j) ^ (row & 7)) << 4)) =
                                         make_uint4(encode_four_e4m3(v + 16 * j), encode_four_e4m3(v + 16 * j + 4), encode_four_e4m3(v + 16 * j + 8), encode_four_e4m3(v + 16 * j + 12));
                             } else {
+                                auto put = [&](int dtype) {   // (one branch for all)
 #pragma unroll
-                                for (int j = 0; j < 4; ++j)
-                                    *reinterpret_cast<uint4*>(target + (((part * 4 + j) ^ (row & 7)) << 4)) =
-                                        make_uint4(narrow_pair(v[8 * j], v[8 * j + 1], args.out_dtype), narrow_pair(v[8 * j + 2], v[8 * j + 3], args.out_dtype),
-                                                   narrow_pair(v[8 * j + 4], v[8 * j + 5], args.out_dtype), narrow_pair(v[8 * j + 6], v[8 * j + 7], args.out_dtype));
+                                    for (int j = 0; j < 4; ++j)
+                                        *reinterpret_cast<uint4*>(target + (((part * 4 + j) ^ (row & 7)) << 4)) =
+                                            make_uint4(narrow_pair(v[8 * j], v[8 * j + 1], dtype), narrow_pair(v[8 * j + 2], v[8 * j + 3], dtype),
+                                                       narrow_pair(v[8 * j + 4], v[8 * j + 5], dtype), narrow_pair(v[8 * j + 6], v[8 * j + 7], dtype));
+                                };
+                                if (args.out_dtype == DFGPU_BF16) put(DFGPU_BF16);
+                                else put(DFGPU_F16);
                             }
-                        } else if (row_live && healthy) {
+                        } else if (row_live && healthy_now(ok, status)) {
                             const int64_t at = out_row * args.out_ld + col;
 #pragma unroll
                             for (int e = 0; e < 32; ++e)
@@ -812,7 +859,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         fence_async_shared();
                         epilogue_barrier(1 + g);
                         if (row == 0) {
-                            if (healthy && row0 < args.m_total && col0 < args.n_total) tma_store_2d(&map_c, smem_base + staging, col0, row0);
+                            if (healthy_now(ok, status) && row0 < args.m_total && col0 < args.n_total) tma_store_2d(&map_c, smem_base + staging, col0, row0);
                             tma_store_commit();
                         }
                         ++stored;
@@ -902,7 +949,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         };
         fetch(static_cast<int>(threadIdx.x));
         cluster_wait();
-        const bool healthy = g_device_status == 0;
+        const int status = ask_status();
         bool left = false;
         for (int first = warp * 32; first < count; first += static_cast<int>(blockDim.x)) {
             const int i = first + lane, row = row_of(i), unit = i & ((1 << quad_bits) - 1), col = column_of(i);
@@ -934,13 +981,13 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             if (mine) {
                 if (ahead) apply_steps<kCodesOnly, 4, 4>(args, v, row0 + row, col, true, scalars, &operand);
                 else apply_steps<kCodesOnly, 4, 4>(args, v, row0 + row, col, true, scalars);
-                if (healthy) store_four(args, v, row0 + row, col);
+                if (healthy_now(true, status)) store_four(args, v, row0 + row, col);
             }
             if (!left) fetch(i + static_cast<int>(blockDim.x));
         }
         __syncwarp();
         if (!left) cluster_arrive();
-        fold_amax<kCodesOnly>(args, scalars, lane, healthy);
+        fold_amax<kCodesOnly>(args, scalars, lane, healthy_now(true, status));
         cluster_wait();   // no CTA leaves while another still reads its partial tile
     }
     tc_fence_before();

@@ -13,7 +13,7 @@ import torch
 
 sys.path.insert(0, str(Path(__file__).resolve().parent.parent / "oracle"))
 import graph_oracle  # noqa: E402
-from deepforge_b200 import dfgpu, harness, runtime, synthetic, workloads  # noqa: E402
+from deepforge_b200 import dfgpu, graphs, harness, runtime, synthetic, workloads  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
@@ -142,3 +142,31 @@ def test_requesting_the_tcgen05_kernel_for_an_uncovered_shape_fails():
     with pytest.raises(dfgpu.DfgpuError) as error:
         dfgpu.query("matmul_fp8", params)
     assert error.value.code == 20
+
+
+@pytest.mark.parametrize("descale_a,descale_b", [(0.0625, 3.0), (-0.5, 1.1), (float("inf"), 1.0), (1.0, float("nan")), (0.0, 1.0), (1e30, 1e30), (1e38, 0.0), (1e-38, 1e-10), (0.0, float("inf"))])
+@pytest.mark.parametrize("m,k,n", [(130, 256, 144), (300, 2048, 2304), (5, 4096, 80)])
+@pytest.mark.parametrize("infinite", [False, True])
+def test_amax_with_any_descales(descale_a, descale_b, m, k, n, infinite):
+    """Amax_C is the largest |sum * Descale_A * Descale_B|, each product rounded: with finite de-scales taken from the largest sum, else value by
+    value. Sums of small whole numbers are exact, so C and Amax_C are compared for equality, NaN and infinities included."""
+    g = torch.Generator(device="cuda").manual_seed(k)
+    a, b = (torch.randint(-2, 3, shape, device="cuda", generator=g).float() for shape in ((m, k), (n, k)))
+    a[m // 2] = 0.0
+    if infinite:
+        a[m - 1, 3] = float("inf")   # (a row of infinities, and of NaN where B holds a zero there)
+    a_codes, b_codes = a.to(torch.float8_e5m2).view(torch.uint8), b.to(torch.float8_e4m3fn).view(torch.uint8)
+    doc = graphs.matmul_fp8(m, k, n, "FLOAT", batch=(), b_k_major=True, a_type="FP8_E5M2", b_type="FP8_E4M3")
+    one = lambda x: torch.full((1,), x, device="cuda")
+    buffers = {21: a_codes, 22: b_codes, 23: one(descale_a), 24: one(descale_b), 25: one(0.25), 26: torch.zeros(m, n, device="cuda"), 27: one(-7.0)}
+    exe = runtime.compile_graph(doc)
+    workspace = torch.empty(max(exe.workspace_size, 1), dtype=torch.uint8, device="cuda")
+    exe.execute({uid: x.data_ptr() for uid, x in buffers.items()}, workspace.data_ptr())
+    torch.cuda.synchronize()
+    assert dfgpu.device_status() == 0
+    sums = (a.double() @ b.double().t()).float() + 0.0
+    value = sums * torch.tensor(descale_a, device="cuda") * torch.tensor(descale_b, device="cuda")
+    want = float("nan") if bool(torch.isnan(value).any()) else float(value.abs().max())
+    assert torch.equal(torch.isnan(buffers[26]), torch.isnan(value)) and torch.equal(buffers[26].nan_to_num(5.0), (value * 0.25).nan_to_num(5.0))
+    got = float(buffers[27][0])
+    assert got == want or (got != got and want != want)
