@@ -36,7 +36,7 @@ struct DecodeArgs {
     int32_t table_len_k, table_len_v;
     int32_t num_pages;
     int32_t max_chunks, tiles_per_cta;
-    int32_t tile_step;        // key tiles from one of a CTA's tiles to its next: 1, or max_chunks (interleaves())
+    int32_t tile_step;        // ROUND: key tiles from one of a CTA's tiles to its next, max_chunks
     int32_t has_left, has_right, bottom_right, padding;
     int64_t left, right, s_kv;
     float scale_log2;
@@ -119,7 +119,8 @@ __device__ __forceinline__ void key_window(const DecodeArgs& a, int64_t batch, i
     if (hi < 0) hi = 0;
 }
 
-template <int G, int kRingSlots>
+// ROUND: a CTA's key tiles lie args.tile_step apart (interleaves()), else side by side. (Compiled for itself: 0.5 % of the others.)
+template <int G, int kRingSlots, bool ROUND>
 __global__ void __launch_bounds__(kDecodeThreads, kRingSlots <= 3 ? 2 : 1)
 sdpa_decode_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                         const __grid_constant__ CUtensorMap map_v, DecodeArgs args) {
@@ -174,9 +175,9 @@ sdpa_decode_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     // paying a dependent global load per tile. An id outside the container is stored as -1 (its rows read as zeros).
     int32_t* page_ids = reinterpret_cast<int32_t*>(generic_base + DecodeSmem::kPages);
     const bool is_v = threadIdx.x >= 64;
-    const int tile0 = args.tile_step == 1 ? chunk * args.tiles_per_cta : chunk;   // this CTA's key tiles: tile0, tile0 + tile_step, ...
-    const int entry = threadIdx.x & 63, entry_tile = entry >> (31 - __clz(args.pages_per_tile));   // (a power of two)
-    const int table_slot = tile0 * args.pages_per_tile + entry + entry_tile * (args.tile_step - 1) * args.pages_per_tile;
+    const int tile0 = ROUND ? chunk : chunk * args.tiles_per_cta, step = ROUND ? args.tile_step : 1;   // this CTA's key tiles: tile0, tile0 + step, ...
+    const int entry = threadIdx.x & 63;
+    const int table_slot = tile0 * args.pages_per_tile + entry + (ROUND ? (entry >> (31 - __clz(args.pages_per_tile))) * (step - 1) * args.pages_per_tile : 0);   // (pages_per_tile is a power of two)
     const void* offsets = is_v ? args.offsets_v : args.offsets_k;
     const bool in_table = threadIdx.x < 128 && entry < args.tiles_per_cta * args.pages_per_tile && table_slot < (is_v ? args.table_len_v : args.table_len_k);
     int64_t page = -1;
@@ -188,7 +189,7 @@ sdpa_decode_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     key_window(args, batch, lo, hi);
     // those of them that intersect the window: the first_tile-th and `tiles` in all
     const int below = static_cast<int>(lo / kTileKeys) - tile0, until = static_cast<int>((hi + kTileKeys - 1) / kTileKeys) - tile0;   // from this CTA's first tile: tiles before the window, and up to its end
-    auto own_tiles = [&](int count) { return args.tile_step == 1 ? count : static_cast<int>((static_cast<unsigned>(count) + args.tile_step - 1) / static_cast<unsigned>(args.tile_step)); };
+    auto own_tiles = [&](int count) { return ROUND ? static_cast<int>((static_cast<unsigned>(count) + step - 1) / static_cast<unsigned>(step)) : count; };
     const int first_tile = below > 0 ? own_tiles(below) : 0;
     const int tiles = until > 0 ? min(args.tiles_per_cta, own_tiles(until)) - first_tile : 0;
     float* my_partial = args.partial + ((batch * args.heads_q + static_cast<int64_t>(kv_head) * G) * args.max_chunks + chunk) * kPartialStride;
@@ -324,7 +325,7 @@ sdpa_decode_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         }
         for (int j = 0; j < tiles; ++j) {
             const int b = j & 1;
-            const int64_t key = (tile0 + static_cast<int64_t>(first_tile + j) * args.tile_step) * kTileKeys + key_lane;
+            const int64_t key = (tile0 + static_cast<int64_t>(first_tile + j) * step) * kTileKeys + key_lane;
             // page validity of this key (an invalid page reads as zeros: score 0, no contribution to O)
             const int entry = ((first_tile + j) * kTileKeys + key_lane) / args.block;
             const bool k_page_ok = page_ids[entry] >= 0, v_page_ok = page_ids[64 + entry] >= 0;
@@ -530,7 +531,8 @@ int launch_decode_umma(const dfgpu_sdpa_params& p, void* const* tensors, void* s
     args.num_pages = static_cast<int>(pages);
     args.max_chunks = decode_umma_chunks(p);
     args.tiles_per_cta = tiles_per_cta(p);
-    args.tile_step = interleaves(p) ? args.max_chunks : 1;
+    args.tile_step = args.max_chunks;
+    const bool round = interleaves(p);
     args.has_left = p.has_left_bound;
     args.has_right = p.has_right_bound;
     args.bottom_right = p.bottom_right;
@@ -565,7 +567,7 @@ int launch_decode_umma(const dfgpu_sdpa_params& p, void* const* tensors, void* s
         return check_launch("SDPA paged decode (tcgen05)");
     };
     // three ring slots: two CTAs per SM (about 219 KiB of shared memory together) hide each other's softmax latency
-#define DFGPU_DECODE_CASE(G_) return run(sdpa_decode_umma_kernel<G_, 3>, DecodeSmemT<3>::kDynamic)
+#define DFGPU_DECODE_CASE(G_) return round ? run(sdpa_decode_umma_kernel<G_, 3, true>, DecodeSmemT<3>::kDynamic) : run(sdpa_decode_umma_kernel<G_, 3, false>, DecodeSmemT<3>::kDynamic)
     switch (args.group) {
         case 1: DFGPU_DECODE_CASE(1);
         case 2: DFGPU_DECODE_CASE(2);
