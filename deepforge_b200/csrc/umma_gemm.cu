@@ -629,7 +629,7 @@ umma_conv_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __g
                 epilogue_barrier(1 + group);
             }
             tc_fence_after();
-            const bool healthy = ok && g_device_status == 0;
+            const int status = ask_status();
             uint8_t* tile_smem = generic_base + pargs.epi_offset + buf * pargs.epi_bytes;
 #pragma unroll 1
             for (int chunk = 0; chunk < BN / 32; ++chunk) {
@@ -705,7 +705,7 @@ umma_conv_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __g
             fence_async_shared();
             epilogue_barrier(1 + group);
             if (store_thread) {
-                if (healthy) {
+                if (healthy_now(ok, status)) {
                     auto store = [&](int box, int col0) {
                         const uint32_t source = epi_base + buf * pargs.epi_bytes + box * (kTileM * 128);
                         if constexpr (CLIPPED) tma_store_4d(&map_out, source, col0, 0, h0, image);

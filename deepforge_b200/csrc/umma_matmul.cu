@@ -377,18 +377,6 @@ __device__ __forceinline__ void store_four(const TileArgs& args, const float (&v
         if (i < live) store_from_f32(args.out, args.out_dtype, at + i, v[i]);
 }
 
-// The status word, asked for here and looked at in healthy_now() alone: some 600 clocks later, a third of an epilogue part, which a
-// comparison beside the load would wait for.
-__device__ __forceinline__ int ask_status() {
-    int status;
-    asm volatile("ld.volatile.global.s32 %0, [%1];" : "=r"(status) : "l"(__cvta_generic_to_global(&g_device_status)) : "memory");
-    return status;
-}
-__device__ __forceinline__ bool healthy_now(bool ok, int status) {
-    asm volatile("" : "+r"(status));
-    return ok && status == 0;
-}
-
 template <bool CLUSTER>
 __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, int code) {
     if constexpr (CLUSTER) return mbar_wait_warp_cluster(bar, parity, code);
