@@ -94,6 +94,8 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// ... which waits for no store of the thread's own: for threads that have only read the others' memory, and have what they read
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t address_in(uint32_t own_address, uint32_t rank) {
     uint32_t remote;
@@ -594,6 +596,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const uint32_t tmem_base = *tmem_slot_ptr;
     chain_wait();
     chain_release();
+    bool settled = !kInBlocks<KIND>;   // (CG = 2, a warp's own answer) CTA 0 has waited for every arrival that this CTA's threads sent it
 
     if (warp == 0) {
         // ---- loader: this CTA's rows of A and share of B; with CG = 2 the bytes are counted on CTA 0's barrier ----
@@ -745,7 +748,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             const int box_columns = !args.tma_store || args.out_dtype == DFGPU_F32 ? 32 : (args.out_dtype == DFGPU_E4M3 ? 128 : 64);
             Scalars scalars = load_scalars<kCodesOnly>(args);
             int stored = 0;   // boxes this group has sent off
-            int local = 0;
+            int local = 0, status = 0;
             const bool ahead = (KIND == kSixteen || KIND == kPieces) && args.step_count > 0 && args.step_kind[0] != kStepRelu && args.step_dtype[0] != DFGPU_F32;
             uint32_t first_operand[16];
             for (int i = first_item; i < args.items; i += item_step, local += kInBlocks<KIND> ? 0 : 1) {
@@ -764,7 +767,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     if (ok) ok = mbar_wait(acc_full(acc), use & 1, 505 + kCode);
                     tc_fence_after();
                 }
-                const int status = ask_status();
+                status = ask_status();
                 const uint32_t columns = tmem_base + lane_base + (kInPlace<KIND> ? args.sums_column : acc * args.acc_stride);
                 const int boxes = item.width / box_columns;
                 for (int b = g; b < boxes; b += 2) {
@@ -796,8 +799,8 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                             tc_fence_before();
                             __syncwarp();
                             if (lane == 0) {
-                                if (CG == 2) mbar_arrive_cluster(leader_bars + (overlap_free - bar_base));
-                                else mbar_arrive(overlap_free);
+                                if (CG == 2 && i + item_step < args.items) mbar_arrive_cluster(leader_bars + (overlap_free - bar_base));   // (one that nobody waits for could come when CTA 0 has left)
+                                if (CG == 1) mbar_arrive(overlap_free);
                             }
                         }
                         float v[32];
@@ -856,11 +859,12 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 tc_fence_before();
                 __syncwarp();
                 if (!kInBlocks<KIND> && lane == 0) {
-                    if (CG == 2) mbar_arrive_cluster(leader_bars + 8u * (2 * kMaxStages + 2 + acc));
-                    else mbar_arrive(acc_empty(acc));
+                    if (CG == 2 && i + item_step * (args.acc_shift + 1) < args.items) mbar_arrive_cluster(leader_bars + 8u * (2 * kMaxStages + 2 + acc));
+                    if (CG == 1) mbar_arrive(acc_empty(acc));
                 }
             }
             if (args.tma_store && row == 0) tma_store_wait_all();
+            if (CG == 2) settled = __all_sync(0xffffffffu, settled && healthy_now(ok, status)) != 0;
             __syncwarp();
             fold_amax<kCodesOnly>(args, scalars, lane, ok);
         }
@@ -917,8 +921,8 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     if (split) {
         // ---- the cluster's partial tiles: every CTA adds its share of the live rows over all ranks, in rank order ----
         // (Latencies one behind the other: what does not need the other CTAs, places and the first fused operand, is fetched while they
-        // arrive, and a CTA lets the others leave as soon as their partial sums are in registers, not when its own are stored: 100 x 544 x 1008 f16 with
-        // bias and ReLU 6.15 -> 5.17 us, 128 x 4096 x 4096 bf16 11.6 -> 10.9, FP8 117 x 1040 x 416 7.3 -> 6.6, MXFP8 15 x 1632 x 816 6.1 -> 5.6.)
+        // arrive, and the others may leave once this CTA has their partial sums, which its own stores need not be done for, as a release would wait for:
+        // 100 x 544 x 1008 f16 with bias and ReLU 6.15 -> 4.90 us, 128 x 4096 x 4096 bf16 11.6 -> 10.0, FP8 117 x 1040 x 416 7.3 -> 6.1, MXFP8 15 x 1632 x 816 6.1 -> 5.3.)
         cluster_arrive();   // (all threads: this CTA's partial tile is in place)
         const Item item = item_at(args, first_item);
         const int row0 = item.m_tile * kRows, live_rows = min(kRows, args.m_total - row0);
@@ -938,49 +942,43 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         fetch(static_cast<int>(threadIdx.x));
         cluster_wait();
         const int status = ask_status();
-        bool left = false;
-        for (int first = warp * 32; first < count; first += static_cast<int>(blockDim.x)) {
-            const int i = first + lane, row = row_of(i), unit = i & ((1 << quad_bits) - 1), col = column_of(i);
-            const bool mine = i < count && col < args.n_total;
+        for (int i = threadIdx.x; i < count; i += static_cast<int>(blockDim.x)) {
+            const int row = row_of(i), unit = i & ((1 << quad_bits) - 1), col = column_of(i);
+            if (col >= args.n_total) continue;   // (and so are this thread's further columns: its unit stays)
             const uint32_t at = smem_base + row * bn * 4 + (((unit & ~7) | ((unit ^ row) & 7)) << 4);
             constexpr int kMost = 8;
-            float v[4] = {};
-            if (mine) {
-                float4 part[kMost];
+            float4 part[kMost];
 #pragma unroll
-                for (int z = 0; z < kMost; ++z)   // every load in flight before the first sum
-                    if (z < args.splits) part[z] = load_from_rank(address_in(at, z));
-                v[0] = part[0].x, v[1] = part[0].y, v[2] = part[0].z, v[3] = part[0].w;
+            for (int z = 0; z < kMost; ++z)   // every load in flight before the first sum
+                if (z < args.splits) part[z] = load_from_rank(address_in(at, z));
+            float v[4] = {part[0].x, part[0].y, part[0].z, part[0].w};
 #pragma unroll
-                for (int z = 1; z < kMost; ++z) {
-                    if (z >= args.splits) break;
-                    v[0] = __fadd_rn(v[0], part[z].x);
-                    v[1] = __fadd_rn(v[1], part[z].y);
-                    v[2] = __fadd_rn(v[2], part[z].z);
-                    v[3] = __fadd_rn(v[3], part[z].w);
-                }
+            for (int z = 1; z < kMost; ++z) {
+                if (z >= args.splits) break;
+                v[0] = __fadd_rn(v[0], part[z].x);
+                v[1] = __fadd_rn(v[1], part[z].y);
+                v[2] = __fadd_rn(v[2], part[z].z);
+                v[3] = __fadd_rn(v[3], part[z].w);
             }
-            if (first + static_cast<int>(blockDim.x) >= count) {   // this warp's last look at the others' tiles
-                asm volatile("" : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]));
-                __syncwarp();
-                cluster_arrive();
-                left = true;
-            }
-            if (mine) {
-                if (ahead) apply_steps<kCodesOnly, 4, 4>(args, v, row0 + row, col, true, scalars, &operand);
-                else apply_steps<kCodesOnly, 4, 4>(args, v, row0 + row, col, true, scalars);
-                if (healthy_now(true, status)) store_four(args, v, row0 + row, col);
-            }
-            if (!left) fetch(i + static_cast<int>(blockDim.x));
+            if (ahead) apply_steps<kCodesOnly, 4, 4>(args, v, row0 + row, col, true, scalars, &operand);
+            else apply_steps<kCodesOnly, 4, 4>(args, v, row0 + row, col, true, scalars);
+            if (healthy_now(true, status)) store_four(args, v, row0 + row, col);
+            fetch(i + static_cast<int>(blockDim.x));
         }
         __syncwarp();
-        if (!left) cluster_arrive();
+        cluster_arrive_relaxed();
         fold_amax<kCodesOnly>(args, scalars, lane, healthy_now(true, status));
         cluster_wait();   // no CTA leaves while another still reads its partial tile
     }
     tc_fence_before();
     __syncthreads();
-    if (CG == 2) cluster_sync_all();   // ... or may still signal its barriers or read its operands
+    if (CG == 2) {   // ... or may still signal its barriers or read its operands
+        // (The stores of C go to nobody here: a release, which waits until they are done, is for the arrivals at CTA 0's barriers alone, and
+        // those that it waits for have come before the accumulator that this CTA waited for. FP8 777 x 4096 x 3072 14.4 -> 13.85 us, bf16 2048^3 15.0 -> 14.5.)
+        if (settled) cluster_arrive_relaxed();
+        else cluster_arrive();
+        cluster_wait();
+    }
     if (warp == 1) {
         tc_fence_after();
         free_columns<CG>(tmem_base);
