@@ -286,7 +286,10 @@ matmul_few_rows_kernel(const float* __restrict__ a, const float* __restrict__ b,
         for (int z = 0; z < ranks; ++z) value += cluster.map_shared_rank(&partial[0][0][0], z)[at];
         store_from_f32(c, g.c.dtype, m * g.c.stride[r - 2] + n * g.c.stride[r - 1], fused_steps(g, value, m, n, no_batch));
     }
-    cluster.sync();   // no CTA leaves while another still reads its sums
+    // No CTA leaves while another still reads its sums. (Relaxed: nothing is published with it, and a release would wait for the stores of C.)
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 struct FewRows {
