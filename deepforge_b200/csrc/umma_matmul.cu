@@ -963,6 +963,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             if (ahead) apply_steps<kCodesOnly, 4, 4>(args, v, row0 + row, col, true, scalars, &operand);
             else apply_steps<kCodesOnly, 4, 4>(args, v, row0 + row, col, true, scalars);
             if (healthy_now(true, status)) store_four(args, v, row0 + row, col);
+            else asm volatile("" : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]));   // (what is read has come before this CTA arrives, after a failure too)
             fetch(i + static_cast<int>(blockDim.x));
         }
         __syncwarp();
