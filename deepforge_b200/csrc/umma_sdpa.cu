@@ -723,7 +723,9 @@ sdpa_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
             for (int j = static_cast<int>((t0 ^ group) & 1); j < item.tiles; j += 2, ++mine_done) {
                 const uint32_t t = t0 + j, b = t % kScoreTiles;
                 const uint32_t tmem_s = tmem_base + lane_base + b * 128 + half * 64;
-                // (S(t) follows PV(t - 3): what this tile's turn of the buffers held before has been read, and no barrier below is more than one phase behind)
+                // (A wait tells a phase from its neighbours by parity alone, so the phase before must be over and the one behind it impossible. s_full(b):
+                // S(t - 3) was over when the other group passed on tile t - 3, which this group took for tile t - 2, and S(t + 3) follows PV(t), which needs
+                // this warp. passed_on: every phase is waited for, in order. pv_done(b): S(t) follows PV(t - 3), and PV(t + 1) follows PV(t).)
                 if (ok) ok = mbar_wait(s_full(b), (t / kScoreTiles) & 1, 279);
                 tc_fence_after();
                 const int last_key = !GENERAL ? q_index : (args.causal ? min(q_index, item.kv_len - 1) : item.kv_len - 1);
@@ -855,7 +857,10 @@ sdpa_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                 }
                 if (PADDED && (j + 1) * kKeys > item.kv_len && (D == 128 || half == 0)) {
                     // V rows past the batch's length are not this sequence's: cleared before the product
+                    // (the slot held V(t - 2) before, which no wait above has asked for: while it is still on its way, its barrier is a phase further behind than
+                    // the parity can tell. Once it has been multiplied, it has come. In the slot of V1 that was K1, which S(1) has read; V(t + 2) follows PV(t).)
                     const uint32_t place = v_place(t), v_slot = slot_of(place);
+                    if (ok && t >= 2) ok = mbar_wait(pv_done((t - 2) % kScoreTiles), ((t - 2) / kScoreTiles) & 1, 284);
                     if (ok) ok = mbar_wait(kv_full(v_slot), parity_of(place), 281);
                     if (j * kKeys + row >= item.kv_len) {
                         uint8_t* v_row = generic_base + Smem::kRing + v_slot * kTileBytes + half * kHalfBytes + row * 128;

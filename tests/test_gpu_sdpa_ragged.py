@@ -38,7 +38,7 @@ def attention(q, k, v, scale, causal, len_q=None, len_kv=None):
     return p @ v, p @ v.abs(), v.abs().sum(-2, keepdim=True), stats
 
 
-def check(b, h, hkv, sq, skv, d, io, causal, padding=None, scale=None, strided=False, seed=3, fine=False, amplify=1.0):
+def check(b, h, hkv, sq, skv, d, io, causal, padding=None, scale=None, strided=False, seed=3, fine=False, amplify=1.0, cold=0):
     g = torch.Generator(device="cuda").manual_seed(seed)
     scale = d ** -0.5 if scale is None else scale
     def operand(heads, length):
@@ -64,6 +64,13 @@ def check(b, h, hkv, sq, skv, d, io, causal, padding=None, scale=None, strided=F
     exe.execute({uid: x.data_ptr() for uid, x in pack.items()})
     torch.cuda.synchronize()
     assert dfgpu.device_status() == 0
+    first, first_stats = o.clone(), stats.clone()
+    for i in range(cold):   # (operands out of HBM, at another pace than out of the L2 cache: the same bits)
+        torch.full((1 << 26,), float(i), device="cuda")
+        o.fill_(float("nan")), stats.fill_(float("nan"))
+        exe.execute({uid: x.data_ptr() for uid, x in pack.items()})
+        torch.cuda.synchronize()
+        assert dfgpu.device_status() == 0 and torch.equal(o, first) and torch.equal(stats, first_stats)
     want, weight, every, want_stats = attention(q, k, v, scale, causal, len_q, len_kv)
     u = ROUNDING[io]
     bound = (amplify * 2.0 ** -14 if fine else u + 2.0 ** -12) * weight + u * want.abs() + (2.0 ** -24 * every if io == "HALF" else 0.0) + 1e-30
@@ -100,6 +107,15 @@ def test_strides_scale_and_misalignment():
 def test_several_items_per_place(io, b, h, hkv, sq, skv, causal, scale):
     """More work items than SMs, which walk them one after another, with maxima that jump."""
     check(b, h, hkv, sq, skv, 128, io, causal, scale=scale)
+
+
+@pytest.mark.parametrize("io,d", [("BFLOAT16", 128), ("HALF", 128), ("BFLOAT16", 64)])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("s,lengths", [(520, [257, 520, 272, 513, 258, 400]), (300, [16, 300, 1, 299, 129, 256]), (1100, [1100, 260, 5, 1025, 641, 130])])
+def test_few_keys_in_a_last_tile_out_of_memory(io, d, causal, s, lengths):
+    """V rows behind a batch's length (infinities) are cleared when they have come, however late the tiles before them do: a head's keys are
+    nobody else's, lists of several query tiles, tiles with one to sixteen keys whose softmax is short."""
+    check(6, 30, 30, s, s, d, io, causal, padding=(lengths, lengths), cold=6)
 
 
 @pytest.mark.parametrize("causal", [False, True])
