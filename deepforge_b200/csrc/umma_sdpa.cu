@@ -586,6 +586,9 @@ sdpa_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         while (p.live && ok) {
             const uint32_t b = p.t % kScoreTiles, place = v_place(p.t), slot = slot_of(place), d_tmem = tmem_u + o_column(p.n);
             if (p.j == 0) ok = mbar_wait_warp(o_empty(p.n), o_parity(p.n) ^ 1, 274);
+            // (V1's slot held K1, which this warp asks nothing of: the parity of V1's use could be that before K1's. The score product has read K1, and V0
+            // and the later ones follow phases that this warp has waited for or that come first.)
+            if (ok && p.t == 1) ok = mbar_wait_warp(s_full(b), 0, 277);
             if (ok) ok = mbar_wait_warp(kv_full(slot), parity_of(place), 275);
             if (ok) ok = mbar_wait_warp(p_full(b), (p.t / kScoreTiles) & 1, 276);
             tc_fence_after();

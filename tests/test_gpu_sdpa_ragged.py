@@ -118,6 +118,13 @@ def test_few_keys_in_a_last_tile_out_of_memory(io, d, causal, s, lengths):
     check(6, 30, 30, s, s, d, io, causal, padding=(lengths, lengths), cold=6)
 
 
+@pytest.mark.parametrize("io,d", [("BFLOAT16", 128), ("HALF", 128), ("BFLOAT16", 64)])
+@pytest.mark.parametrize("b,h,sq,skv,causal", [(1, 140, 128, 256, False), (3, 60, 5, 200, False), (2, 148, 128, 128, True), (1, 74, 256, 256, True), (1, 40, 129, 700, False)])
+def test_first_key_tiles_out_of_memory(io, d, b, h, sq, skv, causal):
+    """The first and second key tile of every CTA, in the ring's slots that held nothing and a K tile before: whole tiles and others, items of one key tile."""
+    check(b, h, h, sq, skv, d, io, causal, cold=6)
+
+
 @pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("h,sq,skv", [(6, 390, 400), (24, 23, 23), (12, 130, 260)])
 def test_several_padded_items_per_place(causal, h, sq, skv):
