@@ -596,7 +596,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const uint32_t tmem_base = *tmem_slot_ptr;
     chain_wait();
     chain_release();
-    bool settled = !kInBlocks<KIND>;   // (CG = 2, a warp's own answer) CTA 0 has waited for every arrival that this CTA's threads sent it
+    bool settled = !kInBlocks<KIND>;   // (CG = 2, a warp's own answer; the epilogue warps know it for the scale warps too) CTA 0 has waited for every arrival that this CTA's threads sent it
 
     if (warp == 0) {
         // ---- loader: this CTA's rows of A and share of B; with CG = 2 the bytes are counted on CTA 0's barrier ----
@@ -972,11 +972,12 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         cluster_wait();   // no CTA leaves while another still reads its partial tile
     }
     tc_fence_before();
-    __syncthreads();
+    const bool all_settled = CG == 2 && kHasScales<KIND> ? __syncthreads_and(settled) != 0 : (__syncthreads(), settled);
     if (CG == 2) {   // ... or may still signal its barriers or read its operands
         // (The stores of C go to nobody here: a release, which waits until they are done, is for the arrivals at CTA 0's barriers alone, and
-        // those that it waits for have come before the accumulator that this CTA waited for. FP8 777 x 4096 x 3072 14.4 -> 13.85 us, bf16 2048^3 15.0 -> 14.5.)
-        if (settled) cluster_arrive_relaxed();
+        // those that it waits for have come before the accumulators that the epilogue waited for. Where a wait gave up, the scale warps' last arrivals may have been
+        // waited for by nobody, and they release too. FP8 777 x 4096 x 3072 14.4 -> 13.85 us, bf16 2048^3 15.0 -> 14.5.)
+        if (all_settled) cluster_arrive_relaxed();
         else cluster_arrive();
         cluster_wait();
     }

@@ -78,6 +78,7 @@ __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, int c
             if (mbar_try_wait(bar, parity)) return true;
         if (global_timer_ns() - start > 2000000000ull) {
             atomicCAS(&g_device_status, 0, code);
+            __threadfence();   // (whoever learns of what this thread does next finds the code there)
             return false;
         }
     }
@@ -119,6 +120,7 @@ __device__ __noinline__ bool mbar_wait_cluster_slow(uint32_t bar, uint32_t parit
             if (mbar_try_wait_cluster(bar, parity)) return true;
         if (global_timer_ns() - start > 2000000000ull) {
             atomicCAS(&g_device_status, 0, code);
+            __threadfence();   // (whoever learns of what this thread does next finds the code there)
             return false;
         }
     }
