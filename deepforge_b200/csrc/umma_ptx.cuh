@@ -77,9 +77,7 @@ __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, int c
         for (int spin = 0; spin < 128; ++spin)
             if (mbar_try_wait(bar, parity)) return true;
         if (global_timer_ns() - start > 2000000000ull) {
-            atomicCAS(&g_device_status, 0, code);
-            __threadfence();   // (whoever learns of what this thread does next finds the code there)
-            return false;
+            return atomicCAS(&g_device_status, 0, code) < 0;   // (false, codes being positive, and not before the code is in place: whoever learns of what this thread does next finds it)
         }
     }
 }
@@ -119,9 +117,7 @@ __device__ __noinline__ bool mbar_wait_cluster_slow(uint32_t bar, uint32_t parit
         for (int spin = 0; spin < 128; ++spin)
             if (mbar_try_wait_cluster(bar, parity)) return true;
         if (global_timer_ns() - start > 2000000000ull) {
-            atomicCAS(&g_device_status, 0, code);
-            __threadfence();   // (whoever learns of what this thread does next finds the code there)
-            return false;
+            return atomicCAS(&g_device_status, 0, code) < 0;   // (false, codes being positive, and not before the code is in place: whoever learns of what this thread does next finds it)
         }
     }
 }
