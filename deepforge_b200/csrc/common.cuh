@@ -83,6 +83,15 @@ cudaError_t submit(const void* function, dim3 grid, dim3 block, unsigned cluster
 #ifdef __CUDACC__
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A CTA's last arrival at its cluster's barrier, after which the others may leave, behind loads from their shared memory: by every thread of a warp, with whether
+// one of the sums that it formed of them is kRareSum. A relaxed arrival orders nothing by itself, and a releasing one waits for the thread's
+// stores to global memory as well, half a microsecond. So the sums decide which of the two it is: neither can be issued before
+// the loads have come, whatever became of them otherwise. (Where a result happens to be the one it asks for the slower one does the same.)
+constexpr uint32_t kRareSum = 0x0dc00000u;   // 1.5 * 2^-100
+__device__ __forceinline__ void cluster_arrive_behind_loads(bool rare_sum_loaded) {
+    if (__any_sync(0xffffffffu, rare_sum_loaded)) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    else asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
 // The pointer again, but known only from here on: a load through a const __restrict__ pointer counts as independent of
 // memory barriers, so only a data dependence keeps the compiler from moving it above the wait. The address passes through
 // as a global one: a pointer of unknown space would make generic loads of what were global ones (22 % on the CUDA-core MATMUL).

@@ -279,16 +279,18 @@ matmul_few_rows_kernel(const float* __restrict__ a, const float* __restrict__ b,
     cluster.sync();
     const int64_t no_batch[DFGPU_MAX_RANK] = {};
     const int r = g.rank;
+    bool rare = false;
     for (int at = rank * 256 + tid; at < rows * kFewColumns; at += ranks * 256) {
         const int64_t m = m0 + at / kFewColumns, n = n0 + at % kFewColumns;
         if (n >= N) continue;
         float value = 0.0f;
         for (int z = 0; z < ranks; ++z) value += cluster.map_shared_rank(&partial[0][0][0], z)[at];
+        rare = rare || __float_as_uint(value) == kRareSum;
         store_from_f32(c, g.c.dtype, m * g.c.stride[r - 2] + n * g.c.stride[r - 1], fused_steps(g, value, m, n, no_batch));
     }
-    // No CTA leaves while another still reads its sums. (Relaxed: nothing is published with it, and a release would wait for the stores of C.)
+    // No CTA leaves while another still reads its sums. (Nothing is published with it, and a release would wait for the stores of C.)
     __syncwarp();
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    cluster_arrive_behind_loads(rare);
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 

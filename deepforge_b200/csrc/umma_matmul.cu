@@ -942,6 +942,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         fetch(static_cast<int>(threadIdx.x));
         cluster_wait();
         const int status = ask_status();
+        bool rare = false;
         for (int i = threadIdx.x; i < count; i += static_cast<int>(blockDim.x)) {
             const int row = row_of(i), unit = i & ((1 << quad_bits) - 1), col = column_of(i);
             if (col >= args.n_total) continue;   // (and so are this thread's further columns: its unit stays)
@@ -960,14 +961,14 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 v[2] = __fadd_rn(v[2], part[z].z);
                 v[3] = __fadd_rn(v[3], part[z].w);
             }
+            rare = rare || __float_as_uint(v[0]) == kRareSum;
             if (ahead) apply_steps<kCodesOnly, 4, 4>(args, v, row0 + row, col, true, scalars, &operand);
             else apply_steps<kCodesOnly, 4, 4>(args, v, row0 + row, col, true, scalars);
             if (healthy_now(true, status)) store_four(args, v, row0 + row, col);
-            else asm volatile("" : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]));   // (what is read has come before this CTA arrives, after a failure too)
             fetch(i + static_cast<int>(blockDim.x));
         }
         __syncwarp();
-        cluster_arrive_relaxed();
+        cluster_arrive_behind_loads(rare);
         fold_amax<kCodesOnly>(args, scalars, lane, healthy_now(true, status));
         cluster_wait();   // no CTA leaves while another still reads its partial tile
     }

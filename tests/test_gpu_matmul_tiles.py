@@ -60,6 +60,25 @@ def test_sums_over_a_cluster_with_their_first_operand(m, n, k, first):
     close(buffers[4].view(m, n), buffers[1].view(m, k).double(), buffers[2].view(n, k).t().double(), (lambda p: torch.relu(p) + x) if first == "relu" else (lambda p: torch.relu(p + x)), io, k)
 
 
+@pytest.mark.parametrize("m,k,n", [(1, 4096, 512), (7, 2048, 96), (16, 1024, 260), (100, 4096, 144), (128, 2048, 64)])
+@pytest.mark.parametrize("io", ["FLOAT", "BFLOAT16"])
+@pytest.mark.parametrize("b_k_major", [False, True])
+@pytest.mark.parametrize("rare", ["none", "some", "all"])
+def test_both_ways_to_leave_a_cluster(m, k, n, io, b_k_major, rare):
+    """The CTAs that share out K part by one of two arrivals, by whether a sum is 1.5 x 2^-100: none, every second column, all. Products
+    of small whole numbers and of powers of two are exact."""
+    g = torch.Generator(device="cuda").manual_seed(k + n)
+    a, b = (torch.randint(-2, 3, shape, device="cuda", generator=g).float() for shape in ((m, k), (n, k)))
+    a[:, 0], b[:, 0] = 1.5 * 2.0 ** -50, 0.0
+    columns = slice(0, 0) if rare == "none" else (slice(0, n, 2) if rare == "some" else slice(0, n))
+    b[columns] = 0.0
+    b[columns, 0] = 2.0 ** -50
+    tensors = [graphs.tensor(1, "A", [m, k], io), graphs.tensor(2, "B", [k, n], io, [1, k] if b_k_major else [n, 1]), graphs.tensor(3, "C", [m, n], io)]
+    buffers = {1: a.to(TORCH[io]), 2: (b if b_k_major else b.t().contiguous()).to(TORCH[io])}
+    run(graphs.document("leave", [graphs.matmul_node("matmul", 1, 2, 3)], tensors, io=io), buffers)
+    assert torch.equal(buffers[3].view(m, n), (a.double() @ b.double().t()).to(TORCH[io]))
+
+
 @pytest.mark.parametrize("m,k,n", EXTENTS)
 @pytest.mark.parametrize("io", ["BFLOAT16", "HALF"])
 @pytest.mark.parametrize("b_k_major", [False, True])
