@@ -367,9 +367,10 @@ template <> struct QuadsInFlight<__nv_bfloat16> { static constexpr int value = 4
 template <> struct QuadsInFlight<__half> { static constexpr int value = 4; };
 
 constexpr int kPackedThreads = 256;
-// CTAs per SM of the dense kernel, which walk the tiles between them: with a tile each, 3072 CTAs of 4096 bf16 values and a bias took 10.2 us,
-// at most 12 or 16 per SM 9.9, 6 or 8 (all at once, in uneven shares) 10.1. In eights as well, and with the way to the mode's body
-// behind it when the kernel before ends, 9.4.
+// CTAs per SM of the dense kernel that walk the tiles between them, in eights, where a CTA gets two tiles at most: 4096 x 3072 bf16 and a bias, 3072 tiles, 10.3 us
+// with a CTA each (fours), 9.1 so; RELU of 4097 x 3071 10.4 and 9.5. Beyond that the walks drift apart in memory and a CTA a tile is faster:
+// TANH of 13747 x 3007 bf16 30.4 walking, 27.2; and so it is in fours from the start: 16384 x 4100 bf16 and a bias 55 walking, 42.5, f32 TANH of
+// 13747 x 3007 54.6 and 49.2.
 constexpr unsigned kDenseBlocks = 16;
 
 template <typename T>
@@ -459,13 +460,18 @@ __device__ __forceinline__ uint32_t dense_index(const DenseOperand& o, uint32_t 
 // WIDTH values, or the one value they repeat, as they are stored: nothing waits for them before widen_raw().
 template <typename T, int WIDTH> struct Raw { uint32_t words[WIDTH * sizeof(T) / 4]; };
 template <typename T, int WIDTH>
-__device__ __forceinline__ Raw<T, WIDTH> load_raw(const DenseOperand& o, uint32_t i) {
+__device__ __forceinline__ Raw<T, WIDTH> load_one(const DenseOperand& o, uint32_t index) {
     Raw<T, WIDTH> raw{};
-    const T* p = static_cast<const T*>(o.data) + dense_index(o, i);
-    if (o.kind == kRepeat) {
-        if constexpr (sizeof(T) == 4) raw.words[0] = __ldg(reinterpret_cast<const uint32_t*>(p));
-        else raw.words[0] = __ldg(reinterpret_cast<const uint16_t*>(p));
-    } else if constexpr (sizeof(raw) == 16) {
+    const T* p = static_cast<const T*>(o.data) + index;
+    if constexpr (sizeof(T) == 4) raw.words[0] = __ldg(reinterpret_cast<const uint32_t*>(p));
+    else raw.words[0] = __ldg(reinterpret_cast<const uint16_t*>(p));
+    return raw;
+}
+template <typename T, int WIDTH>
+__device__ __forceinline__ Raw<T, WIDTH> load_run(const DenseOperand& o, uint32_t index) {
+    Raw<T, WIDTH> raw;
+    const T* p = static_cast<const T*>(o.data) + index;
+    if constexpr (sizeof(raw) == 16) {
         const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
         raw.words[0] = v.x, raw.words[1] = v.y, raw.words[2] = v.z, raw.words[3] = v.w;
     } else {
@@ -473,6 +479,11 @@ __device__ __forceinline__ Raw<T, WIDTH> load_raw(const DenseOperand& o, uint32_
         raw.words[0] = v.x, raw.words[1] = v.y;
     }
     return raw;
+}
+template <typename T, int WIDTH>
+__device__ __forceinline__ Raw<T, WIDTH> load_raw(const DenseOperand& o, uint32_t i) {
+    const uint32_t index = dense_index(o, i);
+    return o.kind == kRepeat ? load_one<T, WIDTH>(o, index) : load_run<T, WIDTH>(o, index);
 }
 // Values 4 * quad ... 4 * quad + 3 of them.
 template <typename T, int WIDTH>
@@ -522,10 +533,29 @@ __device__ __forceinline__ void dense_tile(const DenseOperand& a, const DenseOpe
     constexpr bool binary = input_count(MODE) == 2;
     const uint32_t first = tile + threadIdx.x * WIDTH;
     Raw<T, WIDTH> raw_x[U], raw_y[U];
+    // Every load is in flight before the first value is used. (In fours of 16 bits an operand's form is looked at once for all of them: with a look
+    // before each load 16384 x 4100 bf16 and a bias took 53 us for 42.5. Eights and f32 lose by it, 9.1 -> 9.9 for 4096 x 3072 and 16.4 -> 17.3.)
+    if constexpr (sizeof(T) == 2 && WIDTH == 4) {
+        auto fetch = [&](const DenseOperand& o, Raw<T, WIDTH> (&raw)[U]) {
+            if (o.kind == kRepeat) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) {   // every load in flight before the first value is used
-        raw_x[u] = load_raw<T, WIDTH>(a, first + u * kPackedThreads * WIDTH);
-        if (binary) raw_y[u] = load_raw<T, WIDTH>(b, first + u * kPackedThreads * WIDTH);
+                for (int u = 0; u < U; ++u) raw[u] = load_one<T, WIDTH>(o, fast_divide(first + u * kPackedThreads * WIDTH, o.by));
+            } else {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t i = first + u * kPackedThreads * WIDTH;
+                    raw[u] = load_run<T, WIDTH>(o, o.kind == kFull ? i : i - fast_divide(i, o.by) * o.by.divisor);
+                }
+            }
+        };
+        fetch(a, raw_x);
+        if (binary) fetch(b, raw_y);
+    } else {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            raw_x[u] = load_raw<T, WIDTH>(a, first + u * kPackedThreads * WIDTH);
+            if (binary) raw_y[u] = load_raw<T, WIDTH>(b, first + u * kPackedThreads * WIDTH);
+        }
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -541,51 +571,53 @@ __device__ __forceinline__ void dense_tile(const DenseOperand& a, const DenseOpe
         else store4<T>(out, first + u * kPackedThreads * WIDTH, r[0]);
     }
 }
-template <typename T, int MODE>
-__device__ __forceinline__ void dense_body(DenseOperand& a, DenseOperand& b, void* out, int out_vector, const PointwiseScalars& s, uint32_t total) {
+// WIDTH 8: every operand's and the output's runs are of whole eights. 4: of whole fours (`vector` kAll), or the output's only, or not even those (0).
+enum { kOutputOnly = 1, kAll = 2 };
+template <typename T, int MODE, int WIDTH, bool WALK>
+__device__ __forceinline__ void dense_body(DenseOperand& a, DenseOperand& b, void* out, int vector, const PointwiseScalars& s, uint32_t total) {
     constexpr int U = QuadsInFlight<T>::value;
     constexpr uint32_t kTile = U * kPackedThreads * 4;
     constexpr bool binary = input_count(MODE) == 2;
-    const int width = min(out_vector, min(a.vector, binary ? b.vector : 8));
     chain_wait();   // (here, when the mode's code and the operands' forms are known)
     a.data = after_chain(a.data);
     b.data = after_chain(b.data);
+    uint32_t tile = blockIdx.x * kTile;
+    if (!WALK && vector == kAll && tile + kTile <= total) return dense_tile<T, MODE, WIDTH>(a, b, out, s, tile);
+    do {
+        if (WALK && vector == kAll && tile + kTile <= total) {
+            dense_tile<T, MODE, WIDTH>(a, b, out, s, tile);
+        } else {
+            const uint32_t first = tile + threadIdx.x * 4;
 #pragma unroll 1
-    for (uint32_t tile = blockIdx.x * kTile; tile < total; tile += gridDim.x * kTile) {
-        if (width != 0 && tile + kTile <= total) {
-            if (sizeof(T) == 2 && width == 8) dense_tile<T, MODE, sizeof(T) == 2 ? 8 : 4>(a, b, out, s, tile);
-            else dense_tile<T, MODE, 4>(a, b, out, s, tile);
-            continue;
-        }
-        const uint32_t first = tile + threadIdx.x * 4;
-#pragma unroll 1
-        for (int u = 0; u < U; ++u) {
-            const uint32_t i = first + u * kPackedThreads * 4;
-            if (i >= total) break;
-            float x[4], y[4] = {0.0f, 0.0f, 0.0f, 0.0f}, r[4];
-            load_dense<T>(a, i, total, x);
-            if (binary) load_dense<T>(b, i, total, y);
-            four_values<T, MODE>(x, y, s, r);
-            if (out_vector && i + 4 <= total) {
-                store4<T>(out, i, r);
-            } else {
-                for (int j = 0; j < 4; ++j) {
-                    if (i + j >= total) break;
-                    if constexpr (sizeof(T) == 4) static_cast<float*>(out)[i + j] = r[j];
-                    else if constexpr (std::is_same_v<T, __nv_bfloat16>) static_cast<uint16_t*>(out)[i + j] = f32_to_bf16_bits(r[j]);
-                    else static_cast<__half*>(out)[i + j] = __float2half_rn(r[j]);
+            for (int u = 0; u < U; ++u) {
+                const uint32_t i = first + u * kPackedThreads * 4;
+                if (i >= total) break;
+                float x[4], y[4] = {0.0f, 0.0f, 0.0f, 0.0f}, r[4];
+                load_dense<T>(a, i, total, x);
+                if (binary) load_dense<T>(b, i, total, y);
+                four_values<T, MODE>(x, y, s, r);
+                if (vector != 0 && i + 4 <= total) {
+                    store4<T>(out, i, r);
+                } else {
+                    for (int j = 0; j < 4; ++j) {
+                        if (i + j >= total) break;
+                        if constexpr (sizeof(T) == 4) static_cast<float*>(out)[i + j] = r[j];
+                        else if constexpr (std::is_same_v<T, __nv_bfloat16>) static_cast<uint16_t*>(out)[i + j] = f32_to_bf16_bits(r[j]);
+                        else static_cast<__half*>(out)[i + j] = __float2half_rn(r[j]);
+                    }
                 }
             }
         }
-    }
+        tile += gridDim.x * kTile;
+    } while (WALK && tile < total);
 }
 
-template <typename T, int INPUTS>
+template <typename T, int INPUTS, int WIDTH, bool WALK>
 __global__ void __launch_bounds__(kPackedThreads)
-pointwise_dense_kernel(DenseOperand a, DenseOperand b, void* out, int out_vector, int mode, PointwiseScalars s, uint32_t total) {
+pointwise_dense_kernel(DenseOperand a, DenseOperand b, void* out, int vector, int mode, PointwiseScalars s, uint32_t total) {
     chain_release();
     switch (mode) {   // (each body waits for the kernel before)
-#define DFGPU_PW_CASE(M) case M: if constexpr (input_count(M) == INPUTS) dense_body<T, M>(a, b, out, out_vector, s, total); break;
+#define DFGPU_PW_CASE(M) case M: if constexpr (input_count(M) == INPUTS) dense_body<T, M, WIDTH, WALK>(a, b, out, vector, s, total); break;
         DFGPU_PW_EVERY_MODE(DFGPU_PW_CASE)
 #undef DFGPU_PW_CASE
         default: break;
@@ -653,10 +685,16 @@ bool dense_operand(const dfgpu_tensor& t, const dfgpu_tensor& out, const int (&o
 
 template <typename T>
 void launch_dense(int inputs, const DenseOperand& a, const DenseOperand& b, void* out, int mode, const PointwiseScalars& s, int64_t total, cudaStream_t stream) {
-    const int out_vector = vector_of(out, sizeof(T));
-    const unsigned grid = std::min(packed_grid<T>(total), kDenseBlocks * static_cast<unsigned>(sm_count()));
-    if (inputs == 1) launch_chained(pointwise_dense_kernel<T, 1>, dim3(grid), dim3(kPackedThreads), 0, stream, a, b, out, out_vector, mode, s, static_cast<uint32_t>(total));
-    else launch_chained(pointwise_dense_kernel<T, 2>, dim3(grid), dim3(kPackedThreads), 0, stream, a, b, out, out_vector, mode, s, static_cast<uint32_t>(total));
+    const int out_width = vector_of(out, sizeof(T)), width = std::min(out_width, std::min(a.vector, inputs == 2 ? b.vector : 8));
+    const unsigned tiles = packed_grid<T>(total), walkers = kDenseBlocks * static_cast<unsigned>(sm_count());
+    auto launch = [&](auto kernel, unsigned grid) {
+        launch_chained(kernel, dim3(grid), dim3(kPackedThreads), 0, stream, a, b, out, width != 0 ? kAll : (out_width != 0 ? kOutputOnly : 0), mode, s, static_cast<uint32_t>(total));
+    };
+    if constexpr (sizeof(T) == 2) {
+        if (width == 8 && tiles <= 2 * walkers) return launch(inputs == 1 ? pointwise_dense_kernel<T, 1, 8, true> : pointwise_dense_kernel<T, 2, 8, true>, std::min(tiles, walkers));
+        if (width == 8) return launch(inputs == 1 ? pointwise_dense_kernel<T, 1, 8, false> : pointwise_dense_kernel<T, 2, 8, false>, tiles);
+    }
+    launch(inputs == 1 ? pointwise_dense_kernel<T, 1, 4, false> : pointwise_dense_kernel<T, 2, 4, false>, tiles);
 }
 
 template <typename T>

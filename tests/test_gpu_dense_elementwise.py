@@ -52,6 +52,25 @@ def test_eights_fours_and_singles(io, dims, b_dims, offsets):
     assert torch.equal(out[:math.prod(dims)].view(dims), want) and bool(torch.all(out[math.prod(dims):] == 7.0))
 
 
+@pytest.mark.parametrize("io", ["HALF", "BFLOAT16"])
+@pytest.mark.parametrize("mode", ["SUB", "RELU_FWD"])
+@pytest.mark.parametrize("over", [0, 8, 12, 4096, 4100])
+def test_where_tiles_are_no_longer_walked(io, mode, over):
+    """32 tiles of 4096 16-bit values per SM are walked, a tile more is not: whole eights and a four more, a last tile that is full or not."""
+    count = torch.cuda.get_device_properties(0).multi_processor_count * 32 * 4096 + over
+    rows = next(r for r in range(5, 0, -1) if count % (4 * r) == 0)
+    dims = [rows, count // rows]
+    g = torch.Generator(device="cuda").manual_seed(over)
+    a, b = (torch.randn(n, device="cuda", generator=g).to(TORCH[io]) for n in (count, dims[1]))
+    out = torch.full((count + 8,), 7.0, device="cuda").to(TORCH[io])
+    binary = mode == "SUB"
+    tensors = [graphs.tensor(1, "A", dims, io), graphs.tensor(3, "O", dims, io)] + ([graphs.tensor(2, "B", [1, dims[1]], io)] if binary else [])
+    buffers = {1: a, 3: out, **({2: b} if binary else {})}
+    execute(graphs.document("dense", [graphs.pointwise_node("node", mode, 1, 3, 2 if binary else None)], tensors, io=io), buffers)
+    want = (a.view(dims).float() - b.view(1, -1).float()).to(TORCH[io]) if binary else torch.relu(a).view(dims)
+    assert torch.equal(out[:count].view(dims), want) and bool(torch.all(out[count:] == 7.0))
+
+
 def test_channels_last_bias_and_first_operand_broadcast():
     n, c, h, w = 2, 24, 5, 7
     g = torch.Generator(device="cuda").manual_seed(1)
