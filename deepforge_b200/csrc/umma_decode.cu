@@ -472,12 +472,19 @@ int decode_umma_chunks(const dfgpu_sdpa_params& p) {
     const int64_t chunk_keys = static_cast<int64_t>(tiles_per_cta(p)) * kTileKeys;
     return static_cast<int>((p.s_kv + chunk_keys - 1) / chunk_keys);
 }
-// A CTA's key tiles lie side by side where the CTAs are many: those past a sequence's end leave at once, and the others have fewer prologues and
-// partial results between them. Where all of them are on the chip together (two per SM) the tiles go round the CTAs instead, so that
-// a sequence of any length is shared out over all of its CTAs: its length is not known here, only the most it may be. 4 x 8 KV heads of up to
-// 8192 keys 17.9 -> 13.5 us, one sequence of 8 KV heads with up to 32768 20.5 -> 17.0. With four tiles a CTA or fewer a shorter walk no longer
-// pays for the prologues and the partial results (two sequences of up to 8192: 16.3 and 16.8; up to 16384 with 4 KV heads: 13.5 and 13.0).
-static bool interleaves(const dfgpu_sdpa_params& p) { return tiles_per_cta(p) == kMaxTilesPerCta && p.q.dim[0] * p.k.dim[1] * decode_umma_chunks(p) <= 2 * 148; }
+// A CTA's key tiles lie side by side: past the end of a short sequence whole CTAs have no work and leave at once, and the others have fewer prologues and
+// partial results between them. Where all CTAs are on the chip together (two per SM) with eight tiles each, the tiles go round a sequence's
+// CTAs instead if that is likely to shorten the longest walk. Either the list of tiles ends well inside its last CTA's eight: 18 sequences of 8 KV heads and up
+// to 1152 keys 21.6 -> 18.5 us, 9 of up to 3200 22.0 -> 20.2. Or the sequences are few, so that the longest of them, n / (n + 1) of what is allowed (which is
+// all that is known here) if they are spread evenly, takes 6.5 tiles a CTA: one of 8 KV heads and up to 32768 keys 24.0 -> 20.3, where it is at least half as long
+// 25.8 -> 24.2; four of up to 9216 25.1 -> 24.3 and 29.4 -> 29.8; seven of up to 3712 21.7 -> 19.8 and 24.4 -> 24.1. With more of them it only adds prologues: 9 x 4 KV heads of 4096 to 8192 27.3 -> 28.4, 37 x 2 of up to 4096
+// 23.6 -> 24.3. With four tiles a CTA or fewer a shorter walk does not pay either: two sequences of up to 8192 16.3 and 16.8.
+// (Pages out of HBM, means over three to nine draws of lengths.)
+static bool interleaves(const dfgpu_sdpa_params& p) {
+    const int64_t tiles = (p.s_kv + kTileKeys - 1) / kTileKeys, chunks = decode_umma_chunks(p), sequences = p.q.dim[0];
+    if (tiles_per_cta(p) != kMaxTilesPerCta || sequences * p.k.dim[1] * chunks > 2 * 148) return false;
+    return (tiles + chunks - 1) / chunks < kMaxTilesPerCta || 2 * tiles * sequences <= 13 * chunks * (sequences + 1);
+}
 // Chunk c holds keys only where the sequence is longer than c times this.
 int decode_umma_chunk_keys(const dfgpu_sdpa_params& p) { return interleaves(p) ? kTileKeys : tiles_per_cta(p) * kTileKeys; }
 

@@ -474,7 +474,7 @@ def test_tma_paged_decode_long_sequences_and_windows():
             close_f32(rows[0], rows_ref[0], 1e-3)
 
 
-@pytest.mark.parametrize("batch,hkv,block,max_len", [(14, 8, 64, 2000), (4, 2, 64, 32700), (4, 2, 16, 29000)])
+@pytest.mark.parametrize("batch,hkv,block,max_len", [(14, 8, 64, 2000), (4, 2, 64, 32700), (4, 2, 16, 29000), (14, 8, 64, 1700), (9, 8, 64, 3200), (5, 8, 16, 5200), (7, 8, 64, 3712)])
 def test_paged_decode_key_tiles_that_go_round_the_ctas(batch, hkv, block, max_len):
     """Eight key tiles a CTA and all CTAs on the chip at once: a CTA's tiles lie as many tiles apart as a sequence has CTAs. Lengths of
     nothing, one key, one tile and one key more, one short of a round of tiles, one tile over a round and everything; windows that
