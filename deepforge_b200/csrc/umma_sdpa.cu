@@ -312,7 +312,7 @@ __device__ __forceinline__ void batch_lengths(const SdpaUmmaArgs& args, int batc
     }
 }
 
-// The work list of a CTA, the same in every warp role; query tiles without keys are left out of it (`dead` walks only those).
+// The work list of a CTA, the same in every warp role; query tiles without keys are left out of it (`every` takes them too).
 //   kAsStored        head after head: CTA c takes items c, c + gridDim.x, ..., so that neighbours share a head's K and V in L2
 //   kHeavyWithLight  causal: unit i of a head is the heavy tile T-1-i followed by the light tile i, so that every unit walks T+1 key tiles
 //                    and equal numbers of units are equal work; neighbours share a head as above
@@ -325,7 +325,7 @@ struct ItemWalker {
     int k = 0;
     const uint16_t* list = nullptr;
     const int2* lengths = nullptr;
-    __device__ __forceinline__ bool next(const SdpaUmmaArgs& args, QueryItem& item, bool dead = false) {
+    __device__ __forceinline__ bool next(const SdpaUmmaArgs& args, QueryItem& item, bool every = false) {
         const int places = static_cast<int>(gridDim.x), place = static_cast<int>(blockIdx.x), tiles = args.q_tiles;
         for (;;) {
             int bh;
@@ -372,7 +372,7 @@ struct ItemWalker {
                 batch_lengths<PADDED>(args, item.batch, item.kv_len, item.live_q);
             }
             item.tiles = key_tiles(args, item.q_tile, item.kv_len, item.live_q);
-            if (PADDED && (item.tiles == 0) != dead) continue;
+            if (PADDED && item.tiles == 0 && !every) continue;
             return true;
         }
     }
@@ -617,7 +617,25 @@ sdpa_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         QueryItem item;
         uint32_t n = 0, t0 = 0;
         bool ok = true;
-        for (; walker.next(args, item); ++n) {   // (to the end also after a wait gave up: the warps meet at their barrier)
+        while (walker.next(args, item, true)) {   // (to the end also after a wait gave up: the warps meet at their barrier)
+            if (PADDED && item.tiles == 0) {
+                // No row of this query tile has keys: zeros and -inf, while these warps would wait for the next one's sums (a walk of its own at the end took 0.9 us,
+                // with or without such tiles; by the softmax warps, in their shadow, its code cost every tile 3 to 8 %: 6 x 32 x 1748 x 64 122 us, 131).
+                constexpr int kUnits = D / 8;   // of 16 bytes a row
+                const int rows = min(kRows, args.seq_q - item.q_tile * kRows);
+                const int64_t b64 = item.batch, h64 = item.head;
+                for (int i = row; i < rows * kUnits; i += 128) {
+                    const int64_t q64 = item.q_tile * kRows + i / kUnits;
+                    *reinterpret_cast<uint4*>(args.out + b64 * args.out_stride[0] + h64 * args.out_stride[1] + q64 * args.out_stride[2] + (i % kUnits) * 8) = make_uint4(0, 0, 0, 0);
+                }
+                if (row < rows) {
+                    const int64_t q64 = item.q_tile * kRows + row;
+                    if (args.row_max != nullptr) args.row_max[b64 * args.max_stride[0] + h64 * args.max_stride[1] + q64 * args.max_stride[2]] = -INFINITY;
+                    if (args.row_sum != nullptr) args.row_sum[b64 * args.sum_stride[0] + h64 * args.sum_stride[1] + q64 * args.sum_stride[2]] = 0.0f;
+                    if (args.stats != nullptr) args.stats[b64 * args.stats_batch_stride + h64 * args.stats_head_stride + q64 * args.stats_row_stride] = -INFINITY;
+                }
+                continue;
+            }
             const int q_index = item.q_tile * kRows + row;
             const int group = static_cast<int>((t0 + item.tiles - 1) & 1);   // of the item's last key tile, whose reference is the latest
             t0 += item.tiles;
@@ -676,25 +694,7 @@ sdpa_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                 }
                 tma_store_commit();
             }
-        }
-        if (PADDED) {
-            // query tiles none of whose rows has keys: zeros and -inf
-            ItemWalker<PADDED> rest = beginning;
-            while (rest.next(args, item, true)) {
-                constexpr int kUnits = D / 8;   // of 16 bytes a row
-                const int rows = min(kRows, args.seq_q - item.q_tile * kRows);
-                const int64_t b64 = item.batch, h64 = item.head;
-                for (int i = row; i < rows * kUnits; i += 128) {
-                    const int64_t q64 = item.q_tile * kRows + i / kUnits;
-                    *reinterpret_cast<uint4*>(args.out + b64 * args.out_stride[0] + h64 * args.out_stride[1] + q64 * args.out_stride[2] + (i % kUnits) * 8) = make_uint4(0, 0, 0, 0);
-                }
-                if (row < rows) {
-                    const int64_t q64 = item.q_tile * kRows + row;
-                    if (args.row_max != nullptr) args.row_max[b64 * args.max_stride[0] + h64 * args.max_stride[1] + q64 * args.max_stride[2]] = -INFINITY;
-                    if (args.row_sum != nullptr) args.row_sum[b64 * args.sum_stride[0] + h64 * args.sum_stride[1] + q64 * args.sum_stride[2]] = 0.0f;
-                    if (args.stats != nullptr) args.stats[b64 * args.stats_batch_stride + h64 * args.stats_head_stride + q64 * args.stats_row_stride] = -INFINITY;
-                }
-            }
+            ++n;
         }
         if (sender) tma_store_wait_all();
     } else {
@@ -868,7 +868,7 @@ sdpa_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                     if (j * kKeys + row >= item.kv_len) {
                         uint8_t* v_row = generic_base + Smem::kRing + v_slot * kTileBytes + half * kHalfBytes + row * 128;
 #pragma unroll
-                        for (int u = 0; u < 8; ++u) *reinterpret_cast<uint4*>(v_row + u * 16) = make_uint4(0, 0, 0, 0);
+                        for (int u = 0; u < 8; ++u) *reinterpret_cast<uint4*>(v_row + ((u ^ (row & 7)) << 4)) = make_uint4(0, 0, 0, 0);   // (eight rows of a warp, eight different banks)
                     }
                     fence_async_shared();
                 }

@@ -141,6 +141,15 @@ def test_padded_items_by_their_lengths(io, d, b, h, sq, causal):
     check(b, h, 1, sq, sq, d, io, causal, padding=(lengths[::-1], lengths), fine=True)
 
 
+@pytest.mark.parametrize("io,d", [("BFLOAT16", 128), ("HALF", 64)])
+@pytest.mark.parametrize("b,h,sq,skv", [(7, 24, 256, 128), (5, 40, 513, 200), (3, 80, 300, 100), (2, 9, 1300, 130)])
+def test_padded_queries_in_more_tiles_than_the_keys(io, d, b, h, sq, skv):
+    """Query tiles without keys among the others, several an SM: behind a batch's queries, of batches without keys, and rows of a tile that is not."""
+    len_q = [(sq, skv, 1, sq - 1, 128, 129, 0)[i % 7] for i in range(b)]
+    len_kv = [(skv, 1, skv - 1, 0, 128, 100, 50)[i % 7] for i in range(b)]
+    check(b, h, h, sq, skv, d, io, False, padding=(len_q, len_kv), fine=True)
+
+
 @pytest.mark.parametrize("b,sq,causal", [(256, 500, True), (257, 500, True), (256, 500, False), (255, 512, True)])
 def test_padded_items_as_many_as_are_listed(b, sq, causal):
     """1024 (batch, query tile)s are put in order by their lengths, 1028 are not, and 1020 are."""
