@@ -1010,11 +1010,13 @@ int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, cudaStrea
     // where all of them stay in the L2 cache: 8 x 32 x 2048 causal, 268 MB of them, took 452 us that way, 274 as heavy and light tiles of
     // a head (29 x 4 x 1494, 88 MB: 54 and 64 the other way round). By length where lengths can differ by much: making the list costs each CTA 1 us, which
     // two or three key tiles a query tile do not give back unless there are many of them (31 x 8 x 25 16.8 us without, 13.6 with it; 27 x 4 x 167
-    // 13.0 and 14.4; 16 x 32 x 303 x 64 35 and 32 the other way round).
+    // 13.0 and 14.4; 16 x 32 x 303 x 64 35 and 32 the other way round), or the queries take more tiles than the keys: a head's last ones are likely behind their
+    // batch's length then, and as stored, with an even number of them, half of the CTAs meet no others (16 x 16 x 512 on 128 keys x 64 21.2 without, 14.6 with it;
+    // 7 x 16 x 256 on 128 11.1 and 10.3; 7 x 16 x 640 on 256, where few are, 16.3 and 16.7).
     const int64_t items = args.q_tiles * heads;
     const bool several = items > sm_count(), in_l2 = p.k.dim[0] * p.k.dim[1] * p.k.dim[2] * p.k.dim[3] * 4 <= (96 << 20);
     args.order = args.causal && several ? (in_l2 ? kHeaviestFirst : kHeavyWithLight) : kAsStored;
-    const bool uneven = kv_tiles >= 4 || (kv_tiles >= 2 && items >= 4 * sm_count());
+    const bool uneven = kv_tiles >= 4 || (kv_tiles >= 2 && items >= 4 * sm_count()) || (!args.causal && args.q_tiles > kv_tiles);
     if (p.padding_mask && several && in_l2 && uneven && p.q.dim[0] * args.q_tiles <= kMostListed) args.order = kLongestFirst;
     const int64_t units = args.order == kHeavyWithLight ? (args.q_tiles + 1) / 2 * heads : items;
     const unsigned grid = static_cast<unsigned>(std::min<int64_t>(units, sm_count()));
