@@ -474,7 +474,7 @@ def test_tma_paged_decode_long_sequences_and_windows():
             close_f32(rows[0], rows_ref[0], 1e-3)
 
 
-@pytest.mark.parametrize("batch,hkv,block,max_len", [(14, 8, 64, 2000), (4, 2, 64, 32700), (4, 2, 16, 29000), (14, 8, 64, 1700), (9, 8, 64, 3200), (5, 8, 16, 5200), (7, 8, 64, 3712)])
+@pytest.mark.parametrize("batch,hkv,block,max_len", [(14, 8, 64, 2000), (4, 2, 64, 32700), (4, 2, 16, 29000)])
 def test_paged_decode_key_tiles_that_go_round_the_ctas(batch, hkv, block, max_len):
     """Eight key tiles a CTA and all CTAs on the chip at once: a CTA's tiles lie as many tiles apart as a sequence has CTAs. Lengths of
     nothing, one key, one tile and one key more, one short of a round of tiles, one tile over a round and everything; windows that
@@ -491,3 +491,9 @@ def test_paged_decode_key_tiles_that_go_round_the_ctas(batch, hkv, block, max_le
         close_bf16(o, o_ref)
         for a, r in zip(rows, rows_ref):
             close_f32(a, r, 1e-3)
+
+
+@pytest.mark.parametrize("batch,hkv,block,max_len", [(14, 8, 64, 1700), (9, 8, 64, 3200), (5, 8, 16, 5200), (7, 8, 64, 3712)])
+def test_paged_decode_lists_that_end_inside_a_cta_and_few_sequences(batch, hkv, block, max_len):
+    """The same where the tiles go round because the list ends inside its last CTA's eight, and at both sides of what counts as few sequences."""
+    test_paged_decode_key_tiles_that_go_round_the_ctas(batch, hkv, block, max_len)
