@@ -24,7 +24,7 @@ constexpr int kKeys = 128;      // keys per tile
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 
 struct SdpaUmmaArgs {
-    int32_t heads_q, heads_kv, seq_q, seq_kv;
+    int32_t heads_q, seq_q, seq_kv;
     int32_t causal;
     int32_t order;            // of the work list: kAsStored, kHeavyWithLight, kHeaviestFirst or kLongestFirst (see ItemWalker)
     float scale_log2;  // |attn_scale| * log2(e); a negative scale negates Q in the products
@@ -80,25 +80,6 @@ __device__ __forceinline__ float ex2_fast(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-
-// Packed pairs of f32 (one 64-bit register): Blackwell's FMA pipe takes two lanes per instruction, which
-// halves the instruction count of the scale-and-subtract and of the row sums in the softmax loop.
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-    uint64_t v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-    return v;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
 }
 
 // 2^x on the FMA and integer pipes: round x to the nearest integer n with the 1.5 * 2^23 trick, evaluate a
@@ -930,6 +911,8 @@ bool packed_rows(const dfgpu_tensor& t) {
     return t.stride[3] == 1 && t.stride[2] == t.dim[3] && t.stride[1] == t.dim[2] * t.stride[2] && t.stride[0] == t.dim[1] * t.stride[1];
 }
 // Whole 128-row tiles of packed bf16 rows of 128, no padding, a causal mask on square scores only: P V on P rounded to bf16.
+// (The kernel itself would take any number of query tiles and heads and a negative scale with Max and Sum_exp as well. Such graphs have had f32 probabilities
+// ever since they ran on tensor cores, and in here they would get 16-bit ones.)
 bool plain_tiles(const dfgpu_sdpa_params& p) {
     const int64_t sq = p.q.dim[2], skv = p.k.dim[2];
     return p.q.dtype == DFGPU_BF16 && p.q.dim[3] == 128 && !p.padding_mask && sq % kRows == 0 && skv % kKeys == 0 && (!p.has_right_bound || sq == skv) &&
@@ -953,7 +936,7 @@ bool sdpa_umma_supported(const dfgpu_sdpa_params& p) {
     if (!(p.attn_scale > -INFINITY && p.attn_scale < INFINITY)) return false;
     for (const dfgpu_tensor* row : {&p.stats, &p.max, &p.sum_exp})
         if (row->rank && row->dtype != DFGPU_F32) return false;
-    return p.q.dim[0] * p.q.dim[1] * ((sq + 2 * kRows - 1) / (2 * kRows)) < (1ll << 30);
+    return p.q.dim[0] * p.q.dim[1] * ((sq + 2 * kRows - 1) / (2 * kRows)) < (1ll << 30);   // (items, at most two for each of these, are counted in 31 bits)
 }
 
 int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, cudaStream_t stream) {
@@ -967,7 +950,6 @@ int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, cudaStrea
     if (status) return status;
     SdpaUmmaArgs args{};
     args.heads_q = static_cast<int>(p.q.dim[1]);
-    args.heads_kv = static_cast<int>(p.k.dim[1]);
     args.seq_q = static_cast<int>(p.q.dim[2]);
     args.seq_kv = static_cast<int>(p.k.dim[2]);
     args.batch_heads = static_cast<int>(p.q.dim[0] * p.q.dim[1]);
@@ -1005,7 +987,7 @@ int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, cudaStrea
     args.by_units = make_fast_divisor((args.q_tiles + 1) / 2);
     args.by_heads = make_fast_divisor(args.heads_q);
     args.by_batch_heads = make_fast_divisor(args.batch_heads);
-    args.by_group = make_fast_divisor(args.heads_q / args.heads_kv);
+    args.by_group = make_fast_divisor(args.heads_q / static_cast<int>(p.k.dim[1]));
     // The order of the list (see ItemWalker) where a CTA takes several items. Heaviest first, CTAs that run side by side read different heads' K and V, so only
     // where all of them stay in the L2 cache: 8 x 32 x 2048 causal, 268 MB of them, took 452 us that way, 274 as heavy and light tiles of
     // a head (29 x 4 x 1494, 88 MB: 54 and 64 the other way round). By length where lengths can differ by much: making the list costs each CTA 1 us, which
