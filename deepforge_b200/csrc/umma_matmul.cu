@@ -365,7 +365,7 @@ __device__ __forceinline__ void store_four(const TileArgs& args, const float (&v
 template <bool CLUSTER>
 __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, int code) {
     if constexpr (CLUSTER) return mbar_wait_warp_cluster(bar, parity, code);
-    else return mbar_wait_warp(bar, parity, code);
+    else return mbar_wait_warp<true>(bar, parity, code);
 }
 
 // kPieces: 32 columns of the products of the lower pieces onto those of the leading ones.
@@ -388,7 +388,7 @@ __device__ __forceinline__ void sum_blocks(float (&sums)[2][32], uint32_t column
                                            int lane, bool& ok) {
     for (int block = 0; block < blocks; ++block, ++local) {
         const int acc = local & 1;
-        if (ok) ok = mbar_wait_warp(acc_full + 8u * acc, (local >> 1) & 1, 585);   // (the warp stays together)
+        if (ok) ok = mbar_wait_warp<true>(acc_full + 8u * acc, (local >> 1) & 1, 585);   // (the warp stays together)
         tc_fence_after();
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -416,7 +416,7 @@ template <int KIND, int CG>
 __device__ __forceinline__ void sum_blocks_in_place(const TileArgs& args, uint32_t columns, int boxes, int g, int blocks, int& local, uint32_t acc_full, uint32_t acc_empty, int lane, bool& ok) {
     for (int block = 0; block < blocks; block += args.blocks_per_sum, ++local) {
         const int acc = local & args.acc_shift;
-        if (ok) ok = mbar_wait_warp(acc_full + 8u * acc, (local >> args.acc_shift) & 1, KIND == kPiecesSummed ? 565 : 595);
+        if (ok) ok = mbar_wait_warp<true>(acc_full + 8u * acc, (local >> args.acc_shift) & 1, KIND == kPiecesSummed ? 565 : 595);
         tc_fence_after();
         for (int box = g; box < boxes; box += 2) {
             const uint32_t own = columns + acc * args.acc_stride + box * 32, target = columns + args.sums_column + box * 32;
@@ -592,7 +592,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             const int columns = item.width / CG, boxes = (columns + args.b_box_columns - 1) / args.b_box_columns;
             const int row0 = (item.m_tile * CG + (CG == 2 ? rank : 0)) * kRows, col0 = item.col0 + (CG == 2 ? rank * columns : 0);
             for (int kb = kb_begin; kb < kb_end; ++kb) {
-                ok = mbar_wait_warp(empty_bar(stage), phase, 501 + kCode);
+                ok = mbar_wait_warp<true>(empty_bar(stage), phase, 501 + kCode);
                 if (!ok) break;
                 if (leader) {
                     const uint32_t bar = counted_on + 8u * stage;
@@ -629,7 +629,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 const uint32_t idesc_wide = args.idesc | (static_cast<uint32_t>(width >> 3) << 17);
                 if (!kInBlocks<KIND> && ok) ok = wait_warp<CG == 2>(acc_empty(acc), (use & 1) ^ 1, 502 + kCode);
                 // (where the accumulators overlap, the other one's shared columns must have been read out too)
-                if (overlapped && ok && local > 0) ok = mbar_wait_warp(overlap_free, (local - 1) & 1, 507 + kCode);
+                if (overlapped && ok && local > 0) ok = mbar_wait_warp<true>(overlap_free, (local - 1) & 1, 507 + kCode);
                 tc_fence_after();
                 uint32_t d = tmem_u + acc * args.acc_stride;
                 int in_sum = 0;
@@ -641,7 +641,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         tc_fence_after();
                         d = tmem_u + block_acc * args.acc_stride;
                     }
-                    ok = mbar_wait_warp(full_bar(stage), phase, 503 + kCode);
+                    ok = mbar_wait_warp<true>(full_bar(stage), phase, 503 + kCode);
                     if (!ok) break;   // (operands by TMA, scales by generic stores + fence.proxy.async: no tcgen05 fence needed)
                     if (leader) {
                         const uint32_t a_src = smem_base + stage * args.stage_bytes, b_src = a_src + kPieceCount * args.a_bytes;   // (with few rows the products read on into B: rows of C nobody stores)
@@ -703,7 +703,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 int local = 0;
                 sum_blocks_in_place<KIND, CG>(args, tmem_base + lane_base, bn / 32, g, kb_end - kb_begin, local, acc_full(0), acc_empty(0), lane, ok);
             } else {
-                ok = mbar_wait(acc_full(0), 0, 504 + kCode);
+                ok = mbar_wait<true>(acc_full(0), 0, 504 + kCode);
                 tc_fence_after();
             }
             uint8_t* parked = generic_base + row * bn * 4;
@@ -747,7 +747,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 } else if constexpr (kInPlace<KIND>) {
                     sum_blocks_in_place<KIND, CG>(args, tmem_base + lane_base, item.width / 32, g, kb_end - kb_begin, local, acc_full(0), leader_bars + (acc_empty(0) - bar_base), lane, ok);
                 } else {
-                    if (ok) ok = mbar_wait(acc_full(acc), use & 1, 505 + kCode);
+                    if (ok) ok = mbar_wait<true>(acc_full(acc), use & 1, 505 + kCode);
                     tc_fence_after();
                 }
                 status = ask_status();
@@ -884,7 +884,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             advance();
             more = seek();
             if (more) load();
-            if (!mbar_wait_warp(empty_bar(slot), slot_phase, 506 + kCode)) break;
+            if (!mbar_wait_warp<true>(empty_bar(slot), slot_phase, 506 + kCode)) break;
             uint8_t* scales = generic_base + slot * args.stage_bytes + args.a_bytes + bn / CG * kRowBytes + lane * 16;
             *reinterpret_cast<uint4*>(scales) = make_uint4(a_words[0], a_words[1], a_words[2], a_words[3]);
             *reinterpret_cast<uint4*>(scales + 512) = make_uint4(b_words[0][0], b_words[0][1], b_words[0][2], b_words[0][3]);

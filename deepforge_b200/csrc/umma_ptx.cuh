@@ -95,37 +95,44 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
 // Bounded wait: false after ~2 s, with `code` left in g_device_status. The common case (the phase
 // is already complete, or completes within the hardware's own suspend window) stays inline; only
 // the long wait is a call, so the hot loops do not pay a call's register save/restore.
+// IN_PLACE: not before the code is there, so that whoever learns of what this thread does next finds it. (The result depends on the atomic's
+// answer then; a fence cost FP8 products 1 %. Not for everybody: the call's registers are its callers' too, and SDPA's plain form spilled 48 bytes
+// for 28 with it, 8 x 32 x 2048 causal 327.6 us for 320.3.)
+template <bool IN_PLACE = false>
 __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, int code) {
     const uint64_t start = global_timer_ns();
     for (;;) {
         for (int spin = 0; spin < 128; ++spin)
             if (mbar_try_wait(bar, parity)) return true;
         if (global_timer_ns() - start > 2000000000ull) {
-            return atomicCAS(&g_device_status, 0, code) < 0;   // (false, codes being positive, and not before the code is in place: whoever learns of what this thread does next finds it)
+            const int before = atomicCAS(&g_device_status, 0, code);
+            return IN_PLACE && before < 0;   // (false: codes are positive)
         }
     }
 }
+template <bool IN_PLACE = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int code) {
     if (mbar_test_wait(bar, parity)) return true;
 #pragma unroll 1
     for (int spin = 0; spin < 64; ++spin)
         if (mbar_try_wait(bar, parity)) return true;
-    return mbar_wait_slow(bar, parity, code);
+    return mbar_wait_slow<IN_PLACE>(bar, parity, code);
 }
 
 // Whole-warp forms for the loader and issuing warps. Their loops run on all 32 lanes with warp-uniform
 // control flow, so addresses, descriptors and counters live in uniform registers (the operands the TMA
 // and tcgen05 instructions take) and only the asynchronous instruction itself is predicated on one
 // elected lane; a loop that runs inside `if (lane == 0)` pays a vector-to-uniform move per operand.
+template <bool IN_PLACE = false>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int code) {
     if (__all_sync(0xffffffffu, mbar_test_wait(bar, parity))) return true;
 #pragma unroll 1
     for (int spin = 0; spin < 64; ++spin)
         if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-    return __all_sync(0xffffffffu, mbar_wait_slow(bar, parity, code)) != 0;
+    return __all_sync(0xffffffffu, mbar_wait_slow<IN_PLACE>(bar, parity, code)) != 0;
 }
 // A wait for what another CTA's threads have written to shared memory: acquires at cluster scope, as mbar_arrive_cluster_release()
-// releases. Bounded like mbar_wait().
+// releases. Bounded like mbar_wait<true>().
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
     uint32_t done;
     asm volatile(
@@ -141,7 +148,7 @@ __device__ __noinline__ bool mbar_wait_cluster_slow(uint32_t bar, uint32_t parit
         for (int spin = 0; spin < 128; ++spin)
             if (mbar_try_wait_cluster(bar, parity)) return true;
         if (global_timer_ns() - start > 2000000000ull) {
-            return atomicCAS(&g_device_status, 0, code) < 0;   // (false, codes being positive, and not before the code is in place: whoever learns of what this thread does next finds it)
+            return atomicCAS(&g_device_status, 0, code) < 0;   // (false, and the code in place)
         }
     }
 }
