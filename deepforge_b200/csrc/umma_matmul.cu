@@ -905,7 +905,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         // ---- the cluster's partial tiles: every CTA adds its share of the live rows over all ranks, in rank order ----
         // (Latencies one behind the other: what does not need the other CTAs, places and the first fused operand, is fetched while they
         // arrive, and the others may leave once this CTA has their partial sums, which its own stores need not be done for, as a release would wait for:
-        // 100 x 544 x 1008 f16 with bias and ReLU 6.15 -> 4.90 us, 128 x 4096 x 4096 bf16 11.6 -> 10.0, FP8 117 x 1040 x 416 7.3 -> 6.1, MXFP8 15 x 1632 x 816 6.1 -> 5.3.)
+        // with bias and ReLU 100 x 544 x 1008 f16 6.13 -> 4.82 us, 128 x 4096 x 4096 bf16 out of HBM 13.6 -> 11.7, in L2 11.6 -> 10.0; FP8 117 x 1040 x 416 7.20 -> 6.06.)
         cluster_arrive();   // (all threads: this CTA's partial tile is in place)
         const Item item = item_at(args, first_item);
         const int row0 = item.m_tile * kRows, live_rows = min(kRows, args.m_total - row0);
@@ -960,7 +960,7 @@ umma_matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     if (CG == 2) {   // ... or may still signal its barriers or read its operands
         // (The stores of C go to nobody here: a release, which waits until they are done, is for the arrivals at CTA 0's barriers alone, and
         // those that it waits for have come before the accumulators that the epilogue waited for. Where a wait gave up, the scale warps' last arrivals may have been
-        // waited for by nobody, and they release too. FP8 777 x 4096 x 3072 14.4 -> 13.85 us, bf16 2048^3 15.0 -> 14.5.)
+        // waited for by nobody, and they release too. FP8 777 x 4096 x 3072 with the shorter waits of its epilogue 15.0 -> 14.5 us, bf16 2048^3 15.0 -> 14.5.)
         if (all_settled) cluster_arrive_relaxed();
         else cluster_arrive();
         cluster_wait();

@@ -239,9 +239,10 @@ constexpr int kProbabilityColumns = GENERAL ? 16 : 8;
 // causal or padded list was balanced to a pair of query tiles only. One warp issuing both kinds of product waited some 100 clocks before each, also
 // for what had long arrived, with the tensor pipe idle: 2000 a tile. Code counts: 16 warps run it out of a small instruction cache, and an
 // edge tile's masks compiled into the sixteens of every tile, or unrolled beside them, cost 3 to 7 %.
-//   before (the better of that kernel and one that gave two SMs a pair) -> this: 4 x 16 (4) x 1000 x 128 padded causal 28.2 -> 25.6 and 33.3 -> 30.4 us by the
-//   lengths, 32 heads of 2449 causal 114 -> 61, 21 x 8 x 796 causal 87.6 -> 51, 32 x 4096 causal 135.7 -> 117, 10 x 32 x 1895 x 64 padded 255 -> 220,
-//   11 x 32 x 69 22.6 -> 15.2, 4 heads of 126 9.8 -> 7.3, 8 x 32 x 2048 causal 273.7 -> 274.0 (323.3 -> 320.0 at the power limit).
+//   before (the better of that kernel and one that gave two SMs a pair) -> this, us a launch in a long row of them on changing operands (power limit):
+//   4 x 16 (4) x 1000 x 128 padded causal 31.8 -> 28.7 (25 to 31 by the lengths), 32 heads of 2449 causal 115 -> 79, 21 x 8 x 796 causal 89 -> 66, 32 x 4096
+//   causal 161 -> 152, 10 x 32 x 1895 x 64 padded 477 -> 434, 11 x 32 x 69 18.3 -> 10.4, 4 heads of 126 8.0 -> 6.5, 8 x 32 x 2048 causal 334 -> 329 (the first
+//   twenty 284 -> 280, one by itself 313 -> 282). Short padded lists of 64 channels lost: 7 x 16 x 187 11.3 -> 11.8.
 // GENERAL: what the kernel takes beyond whole tiles of packed bf16 rows of 128 (plain_tiles()): a batch's keys may end inside a key
 // tile (padding masks, or a key length that is no multiple of 128), and probabilities are held to f32's accuracy: O += P V runs
 // twice, on P rounded to the operands' type and on what that left over (16 or 22 bits in all), as O and Stats of these graphs are
@@ -989,7 +990,7 @@ int launch_sdpa_umma(const dfgpu_sdpa_params& p, void* const* tensors, cudaStrea
     args.by_batch_heads = make_fast_divisor(args.batch_heads);
     args.by_group = make_fast_divisor(args.heads_q / static_cast<int>(p.k.dim[1]));
     // The order of the list (see ItemWalker) where a CTA takes several items. Heaviest first, CTAs that run side by side read different heads' K and V, so only
-    // where all of them stay in the L2 cache: 8 x 32 x 2048 causal, 268 MB of them, took 452 us that way, 274 as heavy and light tiles of
+    // where all of them stay in the L2 cache: 8 x 32 x 2048 causal, 268 MB of them, took 452 us that way in a short run, 274 as heavy and light tiles of
     // a head (29 x 4 x 1494, 88 MB: 54 and 64 the other way round). By length where lengths can differ by much: making the list costs each CTA 1 us, which
     // two or three key tiles a query tile do not give back unless there are many of them (31 x 8 x 25 16.8 us without, 13.6 with it; 27 x 4 x 167
     // 13.0 and 14.4; 16 x 32 x 303 x 64 35 and 32 the other way round), or the queries take more tiles than the keys: a head's last ones are likely behind their
